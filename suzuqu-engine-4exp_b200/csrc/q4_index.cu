@@ -176,6 +176,123 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
     for (uint32_t b = n_vis + blockIdx.x * (SC_WARPS * 32u) + threadIdx.x; b < n_blocks; b += gridDim.x * SC_WARPS * 32u)
         score[(size_t)t * stride + b] = -1.0e30f;
 }
+/* ---- score for many tokens over one pool (a prompt's slice).  The scan above reads the pool once per token, 17 GB
+ * through L2 for 512 tokens x 32 768 blocks (1.67 ms).  This form is a tiled fp32 product on the FMA pipe (the
+ * result is defined as one fused multiply-add per dim in dim order, which rules the tensor cores out): 32 tokens x 4
+ * heads against 128 pooled blocks per tile, 8 x 8 chains per thread -- two tokens' four heads, so the relu sum over
+ * heads stays in the thread.  64 FMAs per 16 shared-memory words; the queries stay in shared memory while a
+ * persistent block walks pool tiles, two buffers deep.  Bound by the FMA pipe. */
+constexpr uint32_t SM_TOK = 32, SM_ROWS = SM_TOK * 4, SM_COLS = 128, SM_THREADS = 256;
+constexpr uint32_t SM_TILE_FLOATS = 128u * SC_ROW_FLOATS;
+constexpr uint32_t SM_SMEM = 3u * SM_TILE_FLOATS * sizeof(float);
+__global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q, const float *pool, float *score, uint32_t n_tok,
+                                                                 uint32_t n_blocks, uint32_t stride, uint32_t n_head,
+                                                                 uint32_t pos0, uint32_t ratio) {
+    extern __shared__ __align__(16) float sm_tiles[];   /* queries | pool tile 0 | pool tile 1, rows 132 floats apart */
+    const uint32_t tid = threadIdx.x;
+    const uint32_t ty = tid >> 4, tc = tid & 15u;       /* tokens 2 ty, 2 ty + 1; pooled blocks tc + 16 j */
+    const uint32_t col_tiles = (n_blocks + SM_COLS - 1u) / SM_COLS, tok_tiles = (n_tok + SM_TOK - 1u) / SM_TOK;
+    const uint64_t total = (uint64_t)col_tiles * tok_tiles;
+    const uint32_t first = (uint32_t)(total * blockIdx.x / gridDim.x), last = (uint32_t)(total * (blockIdx.x + 1u) / gridDim.x);
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(sm_tiles);
+    auto visible = [&](uint32_t tok) { return (pos0 + tok + 1u) / ratio; };
+    /* rows of a tile that no token of the group can see are not read: they need not exist yet */
+    auto fetch_pool = [&](uint32_t tile, uint32_t which) {
+        if (tile < last) {
+            const uint32_t t_last = min((tile / col_tiles + 1u) * SM_TOK, n_tok) - 1u, c0 = (tile % col_tiles) * SM_COLS;
+            const uint32_t lim = min(visible(t_last), n_blocks);
+            for (uint32_t i = tid; i < SM_COLS * 32u; i += SM_THREADS) {
+                const uint32_t r = i >> 5, c = i & 31u;
+                const uint32_t dst = s0 + ((1u + which) * SM_TILE_FLOATS + r * SC_ROW_FLOATS + c * 4u) * 4u;
+                if (c0 + r < lim)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(pool + (size_t)(c0 + r) * IX_HD + c * 4u) : "memory");
+                else
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dst), "r"(0u) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint32_t have = 0xffffffffu, which = 0;
+    fetch_pool(first, 0);
+    for (uint32_t tile = first; tile < last; tile++, which ^= 1u) {
+        const uint32_t group = tile / col_tiles, c0 = (tile % col_tiles) * SM_COLS;
+        if (group != have) {   /* the barrier at the end of the previous tile has released the queries */
+            for (uint32_t i = tid; i < SM_ROWS * 32u; i += SM_THREADS) {
+                const uint32_t r = i >> 5, c = i & 31u, tok = group * SM_TOK + (r >> 2), h = r & 3u;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (tok < n_tok && h < n_head) v = *reinterpret_cast<const float4 *>(q + ((size_t)tok * n_head + h) * IX_HD + c * 4u);
+                *reinterpret_cast<float4 *>(sm_tiles + r * SC_ROW_FLOATS + c * 4u) = v;
+            }
+            have = group;
+        }
+        fetch_pool(tile + 1u, which ^ 1u);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float *qa = sm_tiles + ty * 8u * SC_ROW_FLOATS, *kb = sm_tiles + (1u + which) * SM_TILE_FLOATS + tc * SC_ROW_FLOATS;
+        float acc[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+#pragma unroll 2
+        for (uint32_t d = 0; d < IX_HD; d += 4) {
+            float4 a[8], b[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(qa + i * SC_ROW_FLOATS + d);
+#pragma unroll
+            for (int j = 0; j < 8; j++) b[j] = *reinterpret_cast<const float4 *>(kb + j * 16 * SC_ROW_FLOATS + d);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].x, b[j].x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].y, b[j].y, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].z, b[j].z, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].w, b[j].w, acc[i][j]);
+        }
+        __syncthreads();   /* this pool tile, and the queries if the group changes, may be overwritten */
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t tok = group * SM_TOK + 2u * ty + u;
+            if (tok >= n_tok) continue;
+            const uint32_t n_vis = visible(tok);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const uint32_t b = c0 + tc + 16u * j;
+                /* heads that do not exist have zero queries: their relu adds exactly nothing */
+                float sc = __fadd_rn(0.f, fmaxf(acc[4 * u][j], 0.f));
+                sc = __fadd_rn(sc, fmaxf(acc[4 * u + 1][j], 0.f));
+                sc = __fadd_rn(sc, fmaxf(acc[4 * u + 2][j], 0.f));
+                sc = __fadd_rn(sc, fmaxf(acc[4 * u + 3][j], 0.f));
+                if (b < n_blocks) score[(size_t)tok * stride + b] = b < n_vis ? sc : -1.0e30f;
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+/* A tile costs 32 tokens' work however few there are; the scan costs one pass over the pool per token.  They meet at
+ * about five tokens (a 32-token tile row of the product takes as long as five passes of the scan). */
+constexpr uint32_t SM_MIN_TOK = 6;
+bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride, uint32_t n_head,
+                     uint32_t pos0, uint32_t ratio) {
+    static bool done = false;
+    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score_mt_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_SMEM),
+                            "qsa_score smem attribute"))
+        return false;
+    done = true;
+    const uint64_t tiles = (uint64_t)((n_blocks + SM_COLS - 1u) / SM_COLS) * ((n_tok + SM_TOK - 1u) / SM_TOK);
+    const uint32_t grid = (uint32_t)(tiles < (uint64_t)g_q4.sm_count ? tiles : (uint64_t)g_q4.sm_count);
+    q4_ix_score_mt_k<<<grid, SM_THREADS, SM_SMEM, g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+    return q4i_check(cudaGetLastError(), "qsa_score launch");
+}
 bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
                   uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp,
                   const float *const *pools = nullptr, const int32_t *pos_arr = nullptr) {
@@ -375,75 +492,149 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topk1_k(const float *scor
     }
 }
 
-/* ---- selection by a cluster of 8 blocks (rows of up to 65 536 pooled blocks = ctx 262 144): every
- * thread keeps its 8 keys in registers (block r, warp w, step i, lane l holds index 8192 r + 256 w +
- * 32 i + l, so (r, w, i, l) is ascending index order), the per-pass histograms are summed into block
- * 0 through distributed shared memory, every block picks the digit from that sum (copied back with one
- * load per thread: one warp reading its bins from block 0 itself was 3 us slower), and the ordered emit ranks by ballots, one scan over the warps and the other
- * blocks' counts, and writes the positions straight into the list.  One cluster barrier and three block
- * barriers per pass, one cluster barrier for the counts, none after the last remote access; 8 SMs
- * instead of one. */
-constexpr uint32_t TKC_BLOCKS = 8, TKC_KPT = 8, TKC_MAX_ROW = TKC_BLOCKS * IX_TK_THREADS * TKC_KPT;
-constexpr uint32_t TKC_CAND = 256;   /* most keys sharing a 16-bit prefix that are ranked directly */
+/* ---- selection with the keys in registers (rows of up to 65 536 pooled blocks = ctx 262 144): a cluster of
+ * NB = 1, 2, 4 or 8 blocks (8192 keys each), 8 keys per thread; block r, warp w, step i, lane l holds index
+ * 8192 r + 256 w + 32 i + l, so (r, w, i, l) is ascending index order.  Latency-bound: a token's selection is a
+ * chain of meetings, so the chain is kept short.  A first digit of 12 bits (sign, exponent, 3 mantissa bits)
+ * leaves under 1 % of a row's keys in the threshold bin; every block adds its occupied bins to EVERY block's sum
+ * (no read-back after the meeting), and pushes its keys of the threshold bin to every block, which then finishes
+ * the remaining 20 bits alone.  Two cluster meetings after the launch wait (one block: none); the four
+ * meetings and the read-backs of the earlier 8-bit form cost 14.5 us at 65 536 keys and 15.6 us at 8192. */
+constexpr uint32_t TKC_KPT = 8, TKC_KEYS = IX_TK_THREADS * TKC_KPT, TKC_MAX_ROW = 8 * TKC_KEYS;
+constexpr uint32_t TK_BINS = 4096, TK_B1 = 20, TK_B2 = 8;   /* digits: bits 31..20, 19..8, 7..0 */
+constexpr uint32_t TKC_CAND = 512, TKC_CAND_ALL = 2048;     /* most threshold-bin keys of one block / of the cluster that are pushed */
 __device__ __forceinline__ uint32_t tkc_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+template <uint32_t NB>
 __device__ __forceinline__ void tkc_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (NB == 1) __syncthreads();
+    else asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t tkc_remote(const void *p, uint32_t rank) {
     uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
-__device__ __forceinline__ uint32_t tkc_ld(uint32_t ra) {
-    uint32_t v;
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(ra) : "memory");
-    return v;
-}
 __device__ __forceinline__ void tkc_st(uint32_t ra, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ra), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t tkc_atom_add(uint32_t ra, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(ra), "r"(v) : "memory");
-    return old;
 }
 __device__ __forceinline__ void tkc_red_add(uint32_t ra, uint32_t v) {
     asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(ra), "r"(v) : "memory");
 }
+struct TkPick { uint32_t digit, above, cnt; };   /* the digit that holds the target-th key from the top, keys above it, keys in it */
+/* from TK_BINS counts, by the whole block (two block barriers); `tot` and `st` are scratch of the block */
+template <uint32_t NT>
+__device__ __forceinline__ TkPick tk_pick(const uint32_t *hist, uint32_t target, uint32_t *tot /* [32] */, TkPick *st) {
+    constexpr uint32_t PER = TK_BINS / NT;
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, top = TK_BINS - 1u - PER * threadIdx.x;
+    uint32_t c[PER], sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < PER; j++) { c[j] = hist[top - j]; sum += c[j]; }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) tot[w] = incl;
+    __syncthreads();
+    const uint32_t mine = lane < NT / 32 ? tot[lane] : 0u;   /* every warp scans the warp totals for itself */
+    uint32_t s = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= (uint32_t)o) s += y;
+    }
+    uint32_t above = __shfl_sync(0xffffffffu, s - mine, w) + incl - sum;
+    if (above < target && above + sum >= target) {   /* exactly one thread */
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++) {
+            if (above + c[j] >= target) { st->digit = top - j; st->above = above; st->cnt = c[j]; break; }
+            above += c[j];
+        }
+    }
+    __syncthreads();
+    return *st;
+}
+/* the same over 256 counts; every warp works it out for itself, no barrier */
+__device__ __forceinline__ TkPick tk_pick256(const uint32_t *hist, uint32_t target) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t c[8], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) { c[j] = hist[255 - 8 * (int)lane - j]; sum += c[j]; }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    uint32_t above = incl - sum, digit = 0, cnt = 0;
+    const bool here = above < target && incl >= target;
+    if (here) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (above + c[j] >= target) { digit = 255u - 8u * lane - (uint32_t)j; cnt = c[j]; break; }
+            above += c[j];
+        }
+    }
+    const int src = __ffs(__ballot_sync(0xffffffffu, here)) - 1;
+    return {__shfl_sync(0xffffffffu, digit, src), __shfl_sync(0xffffffffu, above, src), __shfl_sync(0xffffffffu, cnt, src)};
+}
+/* exclusive prefix sum of one value per warp over the block's warps (all lanes hold the warp's value); one block barrier */
+__device__ __forceinline__ uint32_t tk_warp_prefix(uint32_t v, uint32_t *tot /* [32] */) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    if (lane == 0) tot[w] = v;
+    __syncthreads();
+    const uint32_t mine = lane < (blockDim.x >> 5) ? tot[lane] : 0u;
+    return __reduce_add_sync(0xffffffffu, lane < w ? mine : 0u);
+}
 
+template <uint32_t NB>
+struct TkcShared {
+    __align__(16) uint32_t ha[TK_BINS];   /* this block's counts of the first digit, then the candidates' of the second */
+    __align__(16) uint32_t hb[NB > 1 ? TK_BINS : 4];   /* the cluster's counts of the first digit */
+    __align__(16) uint32_t h2[NB > 1 ? 4 : TK_BINS];   /* one block: counts of the second digit */
+    uint32_t h3[256], tot[3][32];
+    uint32_t cand[NB][TKC_CAND];          /* keys of the threshold bin, by the block that pushed them */
+    uint32_t ccnt[NB], gcnt[NB];          /* their counts; counts of the keys above that bin */
+    uint32_t cg[NB], ce[NB];              /* candidates above / at the threshold key */
+    uint32_t n_cand, n_above;
+    TkPick st[3];
+};
+template <uint32_t NB>
 __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *score, int32_t *sel, uint32_t stride,
                                                                uint32_t k_blk, uint32_t ratio, uint32_t pos0,
                                                                uint32_t width, const int32_t *pp, const int32_t *pos_arr) {
-    __shared__ uint32_t lhist[4][256];            /* this block's histogram of every pass, zeroed once */
-    __shared__ uint32_t ghist[4][256];            /* block 0's copy is the cluster-wide sum, one per pass */
-    __shared__ uint32_t cta_cnt[TKC_BLOCKS];      /* (ties << 16 | above) of every block, pushed by its owner */
-    __shared__ uint32_t warp_tot[33], st_prefix, st_hi, st_cnt;
-    __shared__ uint32_t cand[TKC_CAND], cand_n;   /* block 0's copy collects the keys that share the 16-bit prefix */
-    const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = tkc_rank();
+    extern __shared__ __align__(16) uint8_t tkc_smem[];
+    TkcShared<NB> &S = *reinterpret_cast<TkcShared<NB> *>(tkc_smem);
+    const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = NB > 1 ? tkc_rank() : 0u;
     /* The block's own shared memory is prepared, and the cluster has met once, before the launch waits for
      * the previous kernel: with programmatic dependent launch this part runs under that kernel's tail. */
-    (&lhist[0][0])[tx] = 0u;                      /* 4 x 256 words, one per thread */
-    if (rank == 0) (&ghist[0][0])[tx] = 0u;
-    static_assert(IX_TK_THREADS == 4 * 256, "one histogram word per thread");
-    if (tx == 0) { st_prefix = 0u; st_hi = 0u; cand_n = 0u; }
-    tkc_sync();   /* block 0's sums are zero before anyone adds to them */
+    constexpr uint32_t BPT = TK_BINS / IX_TK_THREADS;   /* bins per thread */
+    static_assert(BPT == 4, "one 16-byte word of counts per thread");
+    uint32_t *h2 = NB > 1 ? S.ha : S.h2;
+    reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4 *>(NB > 1 ? S.hb : S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
+    if (tx < 256) S.h3[tx] = 0u;
+    if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
+    if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
+    tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
     ix_pdl_sync();
     const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
     const float *row = score + (size_t)t * stride;
     int32_t *out = sel + (size_t)t * width;
-    const uint32_t w_per = (width + TKC_BLOCKS - 1u) / TKC_BLOCKS;
+    const uint32_t w_per = (width + NB - 1u) / NB;
     const uint32_t w0 = min(rank * w_per, width), w1 = min(w0 + w_per, width);   /* this block's slice of the list */
     if (need == n_vis) {   /* every complete block fits: the dense prefix (same decision in all blocks) */
         for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
         return;
     }
-    const uint32_t base = rank * (IX_TK_THREADS * TKC_KPT) + warp * (32u * TKC_KPT) + lane;
+    const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
     uint32_t key[TKC_KPT];
 #pragma unroll
     for (uint32_t i = 0; i < TKC_KPT; i++) {
@@ -456,95 +647,106 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         const uint32_t tail = n_vis * ratio + (w - ncs);
         out[w] = tail <= pos ? (int32_t)tail : -1;
     }
-
-    bool ranked = false;   /* the threshold came from ranking the last candidates, st_cnt holds the count above it */
-    for (int p = 0; p < 4; p++) {
-        const uint32_t sh = 24u - 8u * p, pre = st_prefix;
+#pragma unroll
+    for (uint32_t i = 0; i < TKC_KPT; i++)
+        if (base + 32u * i < n_vis) atomicAdd(&S.ha[key[i] >> TK_B1], 1u);
+    __syncthreads();
+    /* this block's counts into every block's sum; the local array is left at zero for the next digit */
+    auto spread = [&]() {
+        const uint4 c4 = reinterpret_cast<const uint4 *>(S.ha)[tx];
+        const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+        for (uint32_t j = 0; j < BPT; j++)
+            if (c[j])
+                for (uint32_t r = 0; r < NB; r++) tkc_red_add(tkc_remote(&S.hb[BPT * tx + j], r), c[j]);
+        reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+        tkc_sync<NB>();
+    };
+    if (NB > 1) spread();
+    const TkPick p1 = tk_pick<IX_TK_THREADS>(NB > 1 ? S.hb : S.ha, need, S.tot[0], &S.st[0]);
+    uint32_t thr, n_gt;      /* the need-th largest key, keys above it: n_gt < need <= n_gt + ties */
+    bool fast = p1.cnt <= TKC_CAND_ALL;
+    if (fast) {
+        /* keys of the threshold bin to every block, in any order (a key is all that the rest needs) */
+        uint32_t ng = 0;
 #pragma unroll
         for (uint32_t i = 0; i < TKC_KPT; i++) {
-            const uint32_t u = key[i];
-            const bool in = base + 32u * i < n_vis && (p == 0 || (u >> (sh + 8u)) == pre);
-            const uint32_t bin = (u >> sh) & 255u;
-            const uint32_t m = __ballot_sync(0xffffffffu, in);
-            if (m) {   /* one add per warp where the lanes agree, else one per lane */
-                const uint32_t first = __shfl_sync(0xffffffffu, bin, __ffs(m) - 1);
-                if (__all_sync(0xffffffffu, !in || bin == first)) {
-                    if (lane == (uint32_t)(__ffs(m) - 1)) atomicAdd(&lhist[p][first], (uint32_t)__popc(m));
-                } else if (in) {
-                    atomicAdd(&lhist[p][bin], 1u);
-                }
+            const bool live = base + 32u * i < n_vis;
+            ng += __popc(__ballot_sync(0xffffffffu, live && (key[i] >> TK_B1) > p1.digit));
+            if (live && (key[i] >> TK_B1) == p1.digit) {
+                const uint32_t slot = atomicAdd(&S.n_cand, 1u);
+                if (slot < TKC_CAND)
+                    for (uint32_t r = 0; r < NB; r++) {
+                        if (NB == 1) S.cand[0][slot] = key[i];
+                        else tkc_st(tkc_remote(&S.cand[rank][slot], r), key[i]);
+                    }
             }
         }
+        if (lane == 0 && ng) atomicAdd(&S.n_above, ng);
         __syncthreads();
-        if (tx < 256 && lhist[p][tx]) tkc_red_add(tkc_remote(&ghist[p][tx], 0), lhist[p][tx]);
-        tkc_sync();
-        if (tx < 256) lhist[p][tx] = tkc_ld(tkc_remote(&ghist[p][tx], 0));   /* the cluster-wide sum, one load per thread */
-        __syncthreads();
-        if (tx < 32) {
-            /* digit = the highest bin whose count, added to those above it, reaches the target: lane l owns
-             * bins 255 - 8 l .. 248 - 8 l of the cluster-wide sum */
-            const uint32_t target = need - st_hi;
-            uint32_t c[8], tot = 0;
-#pragma unroll
-            for (int j = 0; j < 8; j++) { c[j] = lhist[p][255 - 8 * (int)lane - j]; tot += c[j]; }
-            uint32_t incl = tot;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= (uint32_t)o) incl += y;
-            }
-            uint32_t above = incl - tot;
-            if (above < target && incl >= target) {   /* exactly one lane */
-                uint32_t dg = 0, cnt = 0;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    if (above + c[j] >= target) { dg = 255u - 8u * lane - (uint32_t)j; cnt = c[j]; break; }
-                    above += c[j];
-                }
-                st_hi += above;
-                st_prefix = (pre << 8) | dg;
-                st_cnt = cnt;   /* keys that share the prefix chosen so far */
+        if (tx < NB) {
+            if (NB == 1) { S.ccnt[0] = S.n_cand; S.gcnt[0] = S.n_above; }
+            else {
+                tkc_st(tkc_remote(&S.ccnt[rank], tx), S.n_cand);
+                tkc_st(tkc_remote(&S.gcnt[rank], tx), S.n_above);
             }
         }
+        tkc_sync<NB>();   /* the last access to another block's shared memory is behind this point */
+        for (uint32_t r = 0; r < NB; r++) fast = fast && S.ccnt[r] <= TKC_CAND;   /* same decision in all blocks */
+    }
+    if (fast) {
+        constexpr uint32_t CPT = (NB * TKC_CAND + IX_TK_THREADS - 1u) / IX_TK_THREADS;
+        uint32_t ck[CPT];
+        bool cl[CPT];
+#pragma unroll
+        for (uint32_t j = 0; j < CPT; j++) {
+            const uint32_t i = tx + j * IX_TK_THREADS, r = i / TKC_CAND, c = i % TKC_CAND;
+            cl[j] = i < NB * TKC_CAND && c < S.ccnt[r];
+            ck[j] = cl[j] ? S.cand[r][c] : 0u;
+            if (cl[j]) atomicAdd(&h2[(ck[j] >> TK_B2) & (TK_BINS - 1u)], 1u);
+        }
         __syncthreads();
-        if (p == 1 && st_cnt <= TKC_CAND) {
-            /* After 16 bits only a handful of keys still share the prefix (the same decision in every
-             * block: the counts are cluster-wide).  They are collected in block 0, and every block ranks
-             * them itself: the key with fewer than `target` keys above it and at least `target` at or
-             * above it is the threshold.  One cluster barrier instead of the two remaining passes. */
-            const uint32_t pre16 = st_prefix, target = need - st_hi;
+        const TkPick p2 = tk_pick<IX_TK_THREADS>(h2, need - p1.above, S.tot[1], &S.st[1]);
+        const uint32_t pre = (p1.digit << 12) | p2.digit;
+#pragma unroll
+        for (uint32_t j = 0; j < CPT; j++)
+            if (cl[j] && (ck[j] >> TK_B2) == pre) atomicAdd(&S.h3[ck[j] & 255u], 1u);
+        __syncthreads();
+        const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
+        thr = (pre << 8) | p3.digit;
+        n_gt = p1.above + p2.above + p3.above;
+#pragma unroll
+        for (uint32_t j = 0; j < CPT; j++) {
+            const uint32_t r = (tx + j * IX_TK_THREADS) / TKC_CAND;   /* the same block in all lanes of a warp */
+            const uint32_t mg = __ballot_sync(0xffffffffu, cl[j] && ck[j] > thr), me = __ballot_sync(0xffffffffu, cl[j] && ck[j] == thr);
+            if (lane == 0 && mg) atomicAdd(&S.cg[r], (uint32_t)__popc(mg));
+            if (lane == 0 && me) atomicAdd(&S.ce[r], (uint32_t)__popc(me));
+        }
+    } else {
+        /* Thousands of keys share the first digit (rows of ties): the second and third digit are counted over the
+         * rows' own keys as the first was, with a meeting to clear the sums and one to complete them. */
+        uint32_t pre = p1.digit, above = p1.above;
+#pragma unroll 1
+        for (uint32_t d = 1; d < 3; d++) {
+            const uint32_t sh = d == 1 ? TK_B2 : 0u, bits = d == 1 ? 12u : 8u;
+            __syncthreads();
+            reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+            if (NB > 1) reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
+            tkc_sync<NB>();
 #pragma unroll
             for (uint32_t i = 0; i < TKC_KPT; i++)
-                if (base + 32u * i < n_vis && (key[i] >> 16) == pre16) {
-                    const uint32_t slot = tkc_atom_add(tkc_remote(&cand_n, 0), 1u);
-                    if (slot < TKC_CAND) tkc_st(tkc_remote(&cand[slot], 0), key[i]);
-                }
-            tkc_sync();
-            const uint32_t n = st_cnt;   /* exactly the keys just collected */
-            if (rank != 0 && tx < n) cand[tx] = tkc_ld(tkc_remote(&cand[tx], 0));
+                if (base + 32u * i < n_vis && (key[i] >> (sh + bits)) == pre) atomicAdd(&S.ha[(key[i] >> sh) & ((1u << bits) - 1u)], 1u);
             __syncthreads();
-            if (tx < n) {
-                const uint32_t mine = cand[tx];
-                uint32_t gt = 0, ge = 0;
-                for (uint32_t j = 0; j < n; j++) {
-                    const uint32_t o = cand[j];
-                    gt += o > mine;
-                    ge += o >= mine;
-                }
-                if (gt < target && ge >= target) {   /* every copy of the threshold key writes the same values */
-                    st_prefix = mine;
-                    st_cnt = st_hi + gt;
-                }
-            }
-            __syncthreads();
-            ranked = true;
-            break;
+            if (NB > 1) spread();
+            const TkPick p = tk_pick<IX_TK_THREADS>(NB > 1 ? S.hb : S.ha, need - above, S.tot[d], &S.st[d]);
+            pre = (pre << bits) | p.digit;
+            above += p.above;
         }
+        thr = pre;
+        n_gt = above;
     }
-    const uint32_t thr = st_prefix, n_gt = ranked ? st_cnt : st_hi;
-
-    /* counts: per warp by ballots, per block by one scan over the warps (ties in the high half-word: a
-     * block holds at most 8192 keys), per cluster by every block pushing its pair to all the others */
+    /* counts above and at the threshold: per warp by ballots, per block by one scan over the warps (ties in the
+     * high half-word: a block holds at most 8192 keys) */
     uint32_t ng = 0, ne = 0;
 #pragma unroll
     for (uint32_t i = 0; i < TKC_KPT; i++) {
@@ -552,14 +754,21 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         ng += __popc(__ballot_sync(0xffffffffu, live && key[i] > thr));
         ne += __popc(__ballot_sync(0xffffffffu, live && key[i] == thr));
     }
-    static_assert(IX_TK_THREADS * TKC_KPT < 65536, "two counts share a word");
-    uint32_t off;
-    const uint32_t tot = block_excl_scan(lane == 0 ? (ne << 16 | ng) : 0u, off, warp_tot);
-    off = __shfl_sync(0xffffffffu, off, 0);
-    if (tx < TKC_BLOCKS) tkc_st(tkc_remote(&cta_cnt[rank], tx), tot);
-    tkc_sync();   /* the last access to another block's shared memory is behind this point */
-    for (uint32_t r = 0; r < rank; r++) off += cta_cnt[r];   /* neither half carries: at most 7 x 8192 + 8191 keys precede a thread */
+    static_assert(TKC_KEYS < 65536, "two counts share a word");
+    const uint32_t off = tk_warp_prefix(ne << 16 | ng, S.tot[2]);   /* its barrier also completes cg and ce */
     uint32_t og = off & 0xffffu, oe = off >> 16;
+    if (NB > 1) {
+        if (!fast) {   /* every block tells the others its counts */
+            uint32_t all = lane < 32u ? S.tot[2][lane] : 0u;
+            all = __reduce_add_sync(0xffffffffu, all);
+            if (tx < NB) {
+                tkc_st(tkc_remote(&S.gcnt[rank], tx), all & 0xffffu);
+                tkc_st(tkc_remote(&S.ce[rank], tx), all >> 16);
+            }
+            tkc_sync<NB>();
+        }
+        for (uint32_t r = 0; r < rank; r++) { og += S.gcnt[r] + S.cg[r]; oe += S.ce[r]; }
+    }
     /* ordered emit, straight into the list: above the threshold in index order, then ties until `need` is full */
     const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
@@ -577,29 +786,207 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     }
 }
 
-/* rows that fit the cluster kernel go there, longer ones to the single block */
+/* ---- selection for many tokens at once (a prompt's slice): one block of 512 threads per token, four blocks per
+ * SM.  The cluster form above holds 16 SMs' worth of threads per token for a dozen block barriers (409 us for 512
+ * tokens x 32 768 keys); here a token's row is read twice from L2 and the exact finish works on the few hundred
+ * keys of the threshold bin.  Keys above the bin are marked in a bitmap in index order by the ballots themselves;
+ * candidates join it one by one; the ordered emit is a prefix sum of the bitmap's population counts. */
+constexpr uint32_t TKM_THREADS = 512, TKM_CAND = 2048, TKM_BATCH = 8;
+struct TkmShared {
+    __align__(16) uint32_t hist[TK_BINS], h3[256], tot[4][32];
+    uint32_t ckey[TKM_CAND];
+    uint32_t cidx[TKM_CAND];
+    uint32_t chosen[IX_MAX_KBLK];
+    uint32_t n_cand;
+    TkPick st[2];
+};
+/* all keys of a row in steps of the block's width: f(index, key, live) with the lanes of a warp on 32 consecutive indices */
+template <typename F>
+__device__ __forceinline__ void tkm_walk(const float *row, uint32_t n, F f) {
+    for (uint32_t b0 = threadIdx.x; b0 - threadIdx.x < n; b0 += TKM_THREADS * TKM_BATCH) {
+        float x[TKM_BATCH];
+#pragma unroll
+        for (uint32_t k = 0; k < TKM_BATCH; k++) {
+            const uint32_t b = b0 + k * TKM_THREADS;
+            x[k] = b < n ? __ldcg(row + b) : 0.f;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < TKM_BATCH; k++) {
+            const uint32_t b = b0 + k * TKM_THREADS;
+            f(b, ix_key(x[k]), b < n);
+        }
+    }
+}
+__global__ void __launch_bounds__(TKM_THREADS, 4) q4_ix_topkm_k(const float *score, int32_t *sel, uint32_t stride, uint32_t k_blk,
+                                                               uint32_t ratio, uint32_t pos0, uint32_t width, uint32_t words,
+                                                               const int32_t *pp, const int32_t *pos_arr) {
+    extern __shared__ __align__(16) uint8_t tkm_smem[];
+    TkmShared &S = *reinterpret_cast<TkmShared *>(tkm_smem);
+    uint32_t *bg = reinterpret_cast<uint32_t *>(tkm_smem + sizeof(TkmShared)), *be = bg + words;   /* above / at the threshold */
+    const uint32_t t = blockIdx.x, tx = threadIdx.x, lane = tx & 31u;
+    ix_pdl_sync();
+    const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
+    const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
+    const float *row = score + (size_t)t * stride;
+    int32_t *out = sel + (size_t)t * width;
+    if (need == n_vis) {   /* every complete block fits: the dense prefix */
+        for (uint32_t w = tx; w < width; w += TKM_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
+        return;
+    }
+    const uint32_t n = min(n_vis, words * 32u);   /* the launcher sizes the bitmaps for the row */
+    auto clear = [&]() {
+        for (uint32_t i = tx; i < TK_BINS / 4; i += TKM_THREADS) reinterpret_cast<uint4 *>(S.hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+    };
+    if (tx < 256) S.h3[tx] = 0u;
+    if (tx == 0) S.n_cand = 0u;
+    for (uint32_t i = tx; i < words; i += TKM_THREADS) { bg[i] = 0u; be[i] = 0u; }
+    clear();
+    tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) { if (live) atomicAdd(&S.hist[u >> TK_B1], 1u); });
+    __syncthreads();
+    const TkPick p1 = tk_pick<TKM_THREADS>(S.hist, need, S.tot[0], &S.st[0]);
+    clear();
+    uint32_t thr, n_gt;
+    if (p1.cnt <= TKM_CAND) {
+        tkm_walk(row, n, [&](uint32_t b, uint32_t u, bool live) {
+            const uint32_t m = __ballot_sync(0xffffffffu, live && (u >> TK_B1) > p1.digit);
+            if (lane == 0 && m) bg[b >> 5] = m;
+            if (live && (u >> TK_B1) == p1.digit) {
+                const uint32_t slot = atomicAdd(&S.n_cand, 1u);
+                S.ckey[slot] = u;
+                S.cidx[slot] = b;
+                atomicAdd(&S.hist[(u >> TK_B2) & (TK_BINS - 1u)], 1u);
+            }
+        });
+        __syncthreads();
+        const TkPick p2 = tk_pick<TKM_THREADS>(S.hist, need - p1.above, S.tot[1], &S.st[1]);
+        const uint32_t pre = (p1.digit << 12) | p2.digit;
+        for (uint32_t i = tx; i < p1.cnt; i += TKM_THREADS)
+            if ((S.ckey[i] >> TK_B2) == pre) atomicAdd(&S.h3[S.ckey[i] & 255u], 1u);
+        __syncthreads();
+        const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
+        thr = (pre << 8) | p3.digit;
+        n_gt = p1.above + p2.above + p3.above;
+        for (uint32_t i = tx; i < p1.cnt; i += TKM_THREADS) {
+            const uint32_t u = S.ckey[i], b = S.cidx[i];
+            if (u > thr) atomicOr(&bg[b >> 5], 1u << (b & 31u));
+            else if (u == thr) atomicOr(&be[b >> 5], 1u << (b & 31u));
+        }
+    } else {   /* rows of ties: the second and third digit are counted over the row too */
+        tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) {
+            if (live && (u >> TK_B1) == p1.digit) atomicAdd(&S.hist[(u >> TK_B2) & (TK_BINS - 1u)], 1u);
+        });
+        __syncthreads();
+        const TkPick p2 = tk_pick<TKM_THREADS>(S.hist, need - p1.above, S.tot[1], &S.st[1]);
+        const uint32_t pre = (p1.digit << 12) | p2.digit;
+        tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) {
+            if (live && (u >> TK_B2) == pre) atomicAdd(&S.h3[u & 255u], 1u);
+        });
+        __syncthreads();
+        const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
+        thr = (pre << 8) | p3.digit;
+        n_gt = p1.above + p2.above + p3.above;
+        tkm_walk(row, n, [&](uint32_t b, uint32_t u, bool live) {
+            const uint32_t mg = __ballot_sync(0xffffffffu, live && u > thr), me = __ballot_sync(0xffffffffu, live && u == thr);
+            if (lane == 0 && mg) bg[b >> 5] = mg;
+            if (lane == 0 && me) be[b >> 5] = me;
+        });
+    }
+    __syncthreads();
+    /* ranks: every thread owns consecutive words of the bitmaps */
+    const uint32_t wpt = (words + TKM_THREADS - 1u) / TKM_THREADS, wa = min(tx * wpt, words), wb = min(wa + wpt, words);
+    uint32_t ng = 0, ne = 0;
+    for (uint32_t i = wa; i < wb; i++) { ng += __popc(bg[i]); ne += __popc(be[i]); }
+    uint32_t ig = ng, ie = ne;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t yg = __shfl_up_sync(0xffffffffu, ig, o), ye = __shfl_up_sync(0xffffffffu, ie, o);
+        if (lane >= (uint32_t)o) { ig += yg; ie += ye; }
+    }
+    uint32_t og = tk_warp_prefix(__shfl_sync(0xffffffffu, ig, 31), S.tot[2]) + ig - ng;
+    uint32_t oe = n_gt + tk_warp_prefix(__shfl_sync(0xffffffffu, ie, 31), S.tot[3]) + ie - ne;
+    for (uint32_t i = wa; i < wb; i++) {
+        for (uint32_t m = bg[i]; m; m &= m - 1u, og++)
+            if (og < need) S.chosen[og] = 32u * i + (uint32_t)__ffs(m) - 1u;
+        for (uint32_t m = be[i]; m && oe < need; m &= m - 1u, oe++) S.chosen[oe] = 32u * i + (uint32_t)__ffs(m) - 1u;
+    }
+    __syncthreads();
+    const uint32_t ncs = need * ratio;
+    for (uint32_t w = tx; w < width; w += TKM_THREADS) {
+        int32_t v;
+        if (w < ncs) {
+            const uint32_t i = w / ratio;
+            v = (int32_t)(S.chosen[i] * ratio + (w - i * ratio));
+        } else {
+            const uint32_t tail = n_vis * ratio + (w - ncs);
+            v = tail <= pos ? (int32_t)tail : -1;
+        }
+        out[w] = v;
+    }
+}
+
+template <typename K, typename... A>
+bool topk_start(K kernel, dim3 grid, uint32_t threads, size_t smem, uint32_t cluster, A... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = g_q4.stream;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = 1;
+        at[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (ix_pdl()) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "qsa_topk launch");
+}
+template <uint32_t NB>
+bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stride, uint32_t k_blk, uint32_t ratio, uint32_t pos0,
+                 uint32_t width, const int32_t *pp, const int32_t *pos_arr) {
+    static bool done = false;
+    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_topkc_k<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TkcShared<NB>)),
+                            "qsa_topk smem attribute"))
+        return false;
+    done = true;
+    return topk_start(q4_ix_topkc_k<NB>, dim3(NB, n_tok), IX_TK_THREADS, sizeof(TkcShared<NB>), NB, score, sel, stride, k_blk, ratio, pos0,
+                      width, pp, pos_arr);
+}
+/* Which form: rows of up to 8192 keys need one block either way, which keeps them in registers.  Longer rows take the
+ * cluster form while all clusters are resident at once (two blocks of 1024 threads per SM), the streaming form beyond
+ * (512 tokens x 32 768 keys), and the single block that re-reads the row behind 65 536 keys. */
 bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stride, uint32_t k_blk, uint32_t ratio,
                  uint32_t pos0, uint32_t width, const int32_t *pp, const int32_t *pos_arr = nullptr) {
-    if (stride <= TKC_MAX_ROW) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(TKC_BLOCKS, n_tok);
-        cfg.blockDim = dim3(IX_TK_THREADS);
-        cfg.stream = g_q4.stream;
-        cudaLaunchAttribute at[2];
-        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[1].val.programmaticStreamSerializationAllowed = 1;
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = TKC_BLOCKS;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = ix_pdl() ? 2 : 1;
-        return q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_topkc_k, score, sel, stride, k_blk, ratio, pos0, width, pp, pos_arr),
-                         "qsa_topk launch");
+    if (stride > TKC_MAX_ROW) {
+        q4_ix_topk1_k<<<n_tok, IX_TK_THREADS, 0, g_q4.stream>>>(score, sel, stride, k_blk, ratio, pos0, width, pp, pos_arr);
+        return q4i_check(cudaGetLastError(), "qsa_topk launch");
     }
-    q4_ix_topk1_k<<<n_tok, IX_TK_THREADS, 0, g_q4.stream>>>(score, sel, stride, k_blk, ratio, pos0, width, pp, pos_arr);
-    return q4i_check(cudaGetLastError(), "qsa_topk launch");
+    if (stride <= TKC_KEYS) return topkc_start<1>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
+    const uint32_t nb = stride <= 2 * TKC_KEYS ? 2u : stride <= 4 * TKC_KEYS ? 4u : 8u;
+    if ((uint64_t)n_tok * nb > 2ull * (uint64_t)g_q4.sm_count) {
+        static bool done = false;
+        if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_topkm_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)(sizeof(TkmShared) + 2 * TKC_MAX_ROW / 8)), "qsa_topk smem attribute"))
+            return false;
+        done = true;
+        const uint32_t words = (stride + 31u) / 32u;
+        return topk_start(q4_ix_topkm_k, dim3(n_tok), TKM_THREADS, sizeof(TkmShared) + 2u * words * 4u, 1u, score, sel, stride, k_blk, ratio,
+                          pos0, width, words, pp, pos_arr);
+    }
+    if (nb == 2) return topkc_start<2>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
+    if (nb == 4) return topkc_start<4>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
+    return topkc_start<8>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
 }
 
 }  // namespace
@@ -622,6 +1009,8 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
                                  uint32_t stride, uint32_t n_head, uint32_t hd, uint32_t pos0, uint32_t ratio) {
     if (!g_q4.ok || !q || !pool || !score || n_tok == 0 || hd != IX_HD || n_head == 0 || n_head > 4) return false;
     if (n_blocks == 0) return true;
+    if (n_tok >= SM_MIN_TOK && ratio && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0)
+        return score_mt_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr);
 }
 /* Device position (graph-captured decode): the grid covers `stride` blocks, the bound comes from the

@@ -169,3 +169,43 @@ def test_argument_checks():
     assert not L.q4_hip_qsa_score(z.data_ptr(), z.data_ptr(), z.data_ptr(), 1, 1, 1, 4, 64, 3, 4)      # hd != 128
     assert not L.q4_hip_qsa_topk(z.data_ptr(), s.data_ptr(), 1, 1, 1, 513, 4, 3, 64)                   # k_blk > 512
     assert not L.q4_hip_qsa_topk(None, s.data_ptr(), 1, 1, 1, 16, 4, 3, 64)
+
+
+@pytest.mark.parametrize("n_head,n_tok,pos0,ratio", [(4, 6, 3, 4), (4, 33, 500, 4), (3, 32, 127, 4), (1, 7, 1021, 4), (4, 70, 4099, 4),
+                                                     (2, 40, 60, 1)])
+def test_score_of_many_tokens_bit_exact(oracle, n_head, n_tok, pos0, ratio):
+    """the tiled form (6 tokens and more): edges of its 32-token x 128-block tiles, fewer heads than four, blocks that
+    only some of a tile's tokens see; nothing is written behind n_blocks, and nothing is read behind the blocks that
+    the last token sees (NaN there)"""
+    L = lib()
+    nb = (pos0 + n_tok) // ratio
+    n_blocks, stride = nb + 3, nb + 9
+    rng = np.random.default_rng(n_tok * 1000 + pos0)
+    pool = np.full((n_blocks, 128), np.nan, np.float32)
+    pool[:nb] = rng.standard_normal((nb, 128)).astype(np.float32)
+    q = rng.standard_normal((n_tok, n_head, 128)).astype(np.float32)
+    want = oracle.ix_score(q, np.nan_to_num(pool), n_tok, n_blocks, stride, n_head, pos0, ratio)
+    d_score = torch.full((n_tok, stride), 7.0, device="cuda")
+    assert L.q4_hip_qsa_score(dev(q).data_ptr(), dev(pool).data_ptr(), d_score.data_ptr(), n_tok, n_blocks, stride, n_head, 128, pos0, ratio)
+    got = host(d_score)
+    assert np.array_equal(got[:, :n_blocks].view(np.uint32), want[:, :n_blocks].view(np.uint32))
+    assert (got[:, n_blocks:] == 7.0).all()
+
+
+@pytest.mark.parametrize("n_tok,n_vis,k_blk", [(3, 8192, 512), (1, 8193, 512), (2, 16389, 512), (1, 32773, 100), (160, 8200, 512),
+                                               (80, 16390, 512), (40, 40000, 1)])
+def test_topk_forms_and_their_edges(oracle, n_tok, n_vis, k_blk):
+    """one block, clusters of 2 / 4 / 8, and the streaming form of many tokens (more clusters than fit at once), each on
+    rows whose threshold bin is small, holds thousands of keys, and is all ties"""
+    L = lib()
+    ratio, width = 4, 4 * k_blk + 3
+    pos0 = n_vis * ratio - n_tok
+    stride = n_vis + 5
+    rng = np.random.default_rng(n_vis + n_tok)
+    rows = np.maximum(rng.standard_normal((n_tok, stride)), 0).astype(np.float32)
+    rows[::3] = np.float32(1.0) + rng.integers(0, 1 << 14, rows[::3].shape).astype(np.float32) / (1 << 20)   # one 12-bit digit for all
+    rows[2::3] = np.round(rows[2::3] * 4) / 4
+    d_sel = torch.zeros(n_tok, width, dtype=torch.int32, device="cuda")
+    assert L.q4_hip_qsa_topk(dev(rows).data_ptr(), d_sel.data_ptr(), n_tok, n_vis, stride, k_blk, ratio, pos0, width)
+    want = oracle.ix_topk(rows, n_tok, stride, k_blk, ratio, pos0, width)
+    assert np.array_equal(host(d_sel), want)
