@@ -278,9 +278,14 @@ __global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
-/* A tile costs 32 tokens' work however few there are; the scan costs one pass over the pool per token.  They meet at
- * about five tokens (a 32-token tile row of the product takes as long as five passes of the scan). */
-constexpr uint32_t SM_MIN_TOK = 6;
+/* A tile takes 13.7 us however few of its 32 tokens exist; the scan takes 1.2 us per token and 8192 blocks.  The product
+ * is taken where its tiles, spread over the SMs, come out sooner (8 tokens at 65 536 blocks: 56 against 62 us; at 8192
+ * blocks the scan keeps 8 tokens with 9.4 against 15.3 us). */
+bool score_mt_wins(uint32_t n_tok, uint32_t n_blocks) {
+    const uint64_t tiles = (uint64_t)((n_blocks + SM_COLS - 1u) / SM_COLS) * ((n_tok + SM_TOK - 1u) / SM_TOK);
+    const uint64_t per_sm = (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count;
+    return n_tok > 1 && per_sm * 13700u < (uint64_t)n_tok * n_blocks * 1200u / 8192u;
+}
 bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                      uint32_t pos0, uint32_t ratio) {
     static bool done = false;
@@ -623,10 +628,15 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
     tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
     ix_pdl_sync();
+    /* the keys are requested before the position arrives: the row's storage reaches to `stride` whatever is visible */
+    const float *row = score + (size_t)t * stride;
+    const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
+    uint32_t key[TKC_KPT];
+#pragma unroll
+    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < stride ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
     const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
-    const float *row = score + (size_t)t * stride;
     int32_t *out = sel + (size_t)t * width;
     const uint32_t w_per = (width + NB - 1u) / NB;
     const uint32_t w0 = min(rank * w_per, width), w1 = min(w0 + w_per, width);   /* this block's slice of the list */
@@ -634,13 +644,8 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
         return;
     }
-    const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
-    uint32_t key[TKC_KPT];
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) {
-        const uint32_t b = base + 32u * i;
-        key[i] = b < n_vis ? ix_key(__ldcg(row + b)) : 0u;
-    }
+    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = ix_key(__uint_as_float(key[i]));
     /* the tail of the list (positions behind the last complete block) does not depend on the selection */
     const uint32_t ncs = need * ratio;
     for (uint32_t w = max(w0, ncs) + tx; w < w1; w += IX_TK_THREADS) {
@@ -667,22 +672,32 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     uint32_t thr, n_gt;      /* the need-th largest key, keys above it: n_gt < need <= n_gt + ties */
     bool fast = p1.cnt <= TKC_CAND_ALL;
     if (fast) {
-        /* keys of the threshold bin to every block, in any order (a key is all that the rest needs) */
-        uint32_t ng = 0;
+        /* keys of the threshold bin to every block, in any order (a key is all that the rest needs); one add per
+         * warp reserves its slots and counts the keys above the bin */
+        uint32_t ng = 0, ne = 0, mq[TKC_KPT];
 #pragma unroll
         for (uint32_t i = 0; i < TKC_KPT; i++) {
             const bool live = base + 32u * i < n_vis;
             ng += __popc(__ballot_sync(0xffffffffu, live && (key[i] >> TK_B1) > p1.digit));
-            if (live && (key[i] >> TK_B1) == p1.digit) {
-                const uint32_t slot = atomicAdd(&S.n_cand, 1u);
-                if (slot < TKC_CAND)
-                    for (uint32_t r = 0; r < NB; r++) {
-                        if (NB == 1) S.cand[0][slot] = key[i];
-                        else tkc_st(tkc_remote(&S.cand[rank][slot], r), key[i]);
-                    }
-            }
+            mq[i] = __ballot_sync(0xffffffffu, live && (key[i] >> TK_B1) == p1.digit);
+            ne += __popc(mq[i]);
         }
         if (lane == 0 && ng) atomicAdd(&S.n_above, ng);
+        if (ne) {
+            uint32_t slot = 0;
+            if (lane == 0) slot = atomicAdd(&S.n_cand, ne);
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+#pragma unroll
+            for (uint32_t i = 0; i < TKC_KPT; i++) {
+                const uint32_t at = slot + __popc(mq[i] & ((1u << lane) - 1u));
+                if (((mq[i] >> lane) & 1u) && at < TKC_CAND)
+                    for (uint32_t r = 0; r < NB; r++) {
+                        if (NB == 1) S.cand[0][at] = key[i];
+                        else tkc_st(tkc_remote(&S.cand[rank][at], r), key[i]);
+                    }
+                slot += __popc(mq[i]);
+            }
+        }
         __syncthreads();
         if (tx < NB) {
             if (NB == 1) { S.ccnt[0] = S.n_cand; S.gcnt[0] = S.n_above; }
@@ -708,19 +723,30 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         __syncthreads();
         const TkPick p2 = tk_pick<IX_TK_THREADS>(h2, need - p1.above, S.tot[1], &S.st[1]);
         const uint32_t pre = (p1.digit << 12) | p2.digit;
+        if (p2.cnt == 1u) {   /* 24 bits name one key: the threshold */
 #pragma unroll
-        for (uint32_t j = 0; j < CPT; j++)
-            if (cl[j] && (ck[j] >> TK_B2) == pre) atomicAdd(&S.h3[ck[j] & 255u], 1u);
-        __syncthreads();
-        const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
-        thr = (pre << 8) | p3.digit;
-        n_gt = p1.above + p2.above + p3.above;
+            for (uint32_t j = 0; j < CPT; j++)
+                if (cl[j] && (ck[j] >> TK_B2) == pre) S.h3[0] = ck[j];
+            __syncthreads();
+            thr = S.h3[0];
+            n_gt = p1.above + p2.above;
+        } else {
 #pragma unroll
-        for (uint32_t j = 0; j < CPT; j++) {
-            const uint32_t r = (tx + j * IX_TK_THREADS) / TKC_CAND;   /* the same block in all lanes of a warp */
-            const uint32_t mg = __ballot_sync(0xffffffffu, cl[j] && ck[j] > thr), me = __ballot_sync(0xffffffffu, cl[j] && ck[j] == thr);
-            if (lane == 0 && mg) atomicAdd(&S.cg[r], (uint32_t)__popc(mg));
-            if (lane == 0 && me) atomicAdd(&S.ce[r], (uint32_t)__popc(me));
+            for (uint32_t j = 0; j < CPT; j++)
+                if (cl[j] && (ck[j] >> TK_B2) == pre) atomicAdd(&S.h3[ck[j] & 255u], 1u);
+            __syncthreads();
+            const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
+            thr = (pre << 8) | p3.digit;
+            n_gt = p1.above + p2.above + p3.above;
+        }
+        if (NB > 1) {
+#pragma unroll
+            for (uint32_t j = 0; j < CPT; j++) {
+                const uint32_t r = (tx + j * IX_TK_THREADS) / TKC_CAND;   /* the same block in all lanes of a warp */
+                const uint32_t mg = __ballot_sync(0xffffffffu, cl[j] && ck[j] > thr), me = __ballot_sync(0xffffffffu, cl[j] && ck[j] == thr);
+                if (lane == 0 && mg) atomicAdd(&S.cg[r], (uint32_t)__popc(mg));
+                if (lane == 0 && me) atomicAdd(&S.ce[r], (uint32_t)__popc(me));
+            }
         }
     } else {
         /* Thousands of keys share the first digit (rows of ties): the second and third digit are counted over the
@@ -756,33 +782,41 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     }
     static_assert(TKC_KEYS < 65536, "two counts share a word");
     const uint32_t off = tk_warp_prefix(ne << 16 | ng, S.tot[2]);   /* its barrier also completes cg and ce */
-    uint32_t og = off & 0xffffu, oe = off >> 16;
+    uint32_t og = off & 0xffffu, oe = off >> 16, g0 = 0;   /* g0: the block's first place in the list */
+    const uint32_t all = __reduce_add_sync(0xffffffffu, S.tot[2][lane]);
+    const uint32_t n_own = all & 0xffffu;                  /* this block's keys above the threshold */
     if (NB > 1) {
         if (!fast) {   /* every block tells the others its counts */
-            uint32_t all = lane < 32u ? S.tot[2][lane] : 0u;
-            all = __reduce_add_sync(0xffffffffu, all);
             if (tx < NB) {
-                tkc_st(tkc_remote(&S.gcnt[rank], tx), all & 0xffffu);
+                tkc_st(tkc_remote(&S.gcnt[rank], tx), n_own);
                 tkc_st(tkc_remote(&S.ce[rank], tx), all >> 16);
             }
             tkc_sync<NB>();
         }
-        for (uint32_t r = 0; r < rank; r++) { og += S.gcnt[r] + S.cg[r]; oe += S.ce[r]; }
+        for (uint32_t r = 0; r < rank; r++) { g0 += S.gcnt[r] + S.cg[r]; oe += S.ce[r]; }
     }
-    /* ordered emit, straight into the list: above the threshold in index order, then ties until `need` is full */
+    /* ordered emit: above the threshold in index order (collected in shared memory, so that the list is written in
+     * whole lines), then ties until `need` is full */
+    uint32_t *chosen = S.ha;   /* the counts are no longer needed; n_own < need <= 512 */
     const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
     for (uint32_t i = 0; i < TKC_KPT; i++) {
         const uint32_t b = base + 32u * i;
         const bool live = b < n_vis, gt = live && key[i] > thr, eq = live && key[i] == thr;
         const uint32_t mg = __ballot_sync(0xffffffffu, gt), me = __ballot_sync(0xffffffffu, eq);
-        uint32_t at = need;
-        if (gt) at = og + __popc(mg & lt);
-        else if (eq) at = n_gt + oe + __popc(me & lt);
-        if (at < need)
-            for (uint32_t j = 0; j < ratio && at * ratio + j < width; j++) out[at * ratio + j] = (int32_t)(b * ratio + j);
+        if (gt) chosen[og + __popc(mg & lt)] = b;
+        if (me) {
+            const uint32_t at = n_gt + oe + __popc(me & lt);
+            if (eq && at < need)
+                for (uint32_t j = 0; j < ratio && at * ratio + j < width; j++) out[at * ratio + j] = (int32_t)(b * ratio + j);
+        }
         og += __popc(mg);
         oe += __popc(me);
+    }
+    __syncthreads();
+    for (uint32_t w = tx; w < n_own * ratio && g0 * ratio + w < width; w += IX_TK_THREADS) {
+        const uint32_t i = w / ratio;
+        out[g0 * ratio + w] = (int32_t)(chosen[i] * ratio + (w - i * ratio));
     }
 }
 
@@ -1009,7 +1043,7 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
                                  uint32_t stride, uint32_t n_head, uint32_t hd, uint32_t pos0, uint32_t ratio) {
     if (!g_q4.ok || !q || !pool || !score || n_tok == 0 || hd != IX_HD || n_head == 0 || n_head > 4) return false;
     if (n_blocks == 0) return true;
-    if (n_tok >= SM_MIN_TOK && ratio && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0)
+    if (ratio && score_mt_wins(n_tok, n_blocks) && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0)
         return score_mt_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr);
 }

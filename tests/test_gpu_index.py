@@ -171,10 +171,10 @@ def test_argument_checks():
     assert not L.q4_hip_qsa_topk(None, s.data_ptr(), 1, 1, 1, 16, 4, 3, 64)
 
 
-@pytest.mark.parametrize("n_head,n_tok,pos0,ratio", [(4, 6, 3, 4), (4, 33, 500, 4), (3, 32, 127, 4), (1, 7, 1021, 4), (4, 70, 4099, 4),
-                                                     (2, 40, 60, 1)])
+@pytest.mark.parametrize("n_head,n_tok,pos0,ratio", [(4, 33, 20000, 4), (3, 32, 40001, 4), (1, 97, 4003, 4), (4, 160, 2100, 4),
+                                                     (2, 65, 2300, 1), (4, 16, 20, 4)])
 def test_score_of_many_tokens_bit_exact(oracle, n_head, n_tok, pos0, ratio):
-    """the tiled form (6 tokens and more): edges of its 32-token x 128-block tiles, fewer heads than four, blocks that
+    """the tiled form (the last case: the scan): edges of its 32-token x 128-block tiles, fewer heads than four, blocks that
     only some of a tile's tokens see; nothing is written behind n_blocks, and nothing is read behind the blocks that
     the last token sees (NaN there)"""
     L = lib()
