@@ -157,4 +157,21 @@ struct Q4DecodeArgs {
 };
 bool q4i_decode(const Q4DecodeArgs &a);
 
+/* causal attention of n_tok > 1 query tokens on the tensor cores (q4_prefill.cu): hd 128 or 256 (a native q8_0 store:
+ * 128), 1..16 query heads per kv head, scale > 0, 16-byte aligned operands.  1 = enqueued, 0 = failed, -1 = the
+ * workspace would have to grow inside a capture. */
+struct Q4PrefillArgs {
+    Q4Cache cache;
+    int layout;
+    uint32_t layer, n_head, n_kvh, hd;
+    const void *q;               /* [n_tok][n_head][hd] bf16 or fp32 */
+    int q_bf16;
+    const float *gate;           /* or null */
+    void *out;                   /* bf16 or fp32 */
+    int out_bf16;
+    uint32_t n_tok, kv_base;     /* token t attends rows [0, min(kv_base + t + 1, max_kv)) */
+    float scale;
+};
+int q4i_prefill(const Q4PrefillArgs &a);
+
 #endif

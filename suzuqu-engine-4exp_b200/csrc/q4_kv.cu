@@ -255,12 +255,28 @@ extern "C" bool q4_hip_kv_append_d(void *kcache, void *vcache, const float *k, c
     return launch_append(p, ref_layout(kind));
 }
 
+constexpr uint32_t LEGACY_PREFILL_MIN_TOK = 8;
 static bool legacy_decode(const float *q, const void *kc, const void *vc, const float *gate, float *out,
                           const int32_t *idx, uint32_t width, uint32_t n_head, uint32_t n_kvh, uint32_t hd,
                           uint32_t n_tok, uint32_t kv_base, uint32_t max_kv, float scale, int kind) {
     if (!g_q4.ok || !q || !kc || !vc || !gate || !out) return false;   /* NULL gate is rejected: :7254,7312 */
     if (n_tok == 0 || hd == 0 || hd > 256 || n_head == 0 || n_kvh == 0) return false;
     if (!hd_ok(hd) || kind < 0 || kind > 2) return q4i_fail(Q4E_ARG, "decode: unsupported hd or kind");
+    /* A slice of a prompt: a contraction, on the tensor cores.  512 tokens over 2048 rows of q8_0 at 24 / 2 heads, hd
+     * 256 took 1.23 ms as one decode per token.  Few tokens stay with the decode kernel, which splits the positions
+     * finer, and so do shapes that the tensor-core tiles do not cover. */
+    if (!idx && n_tok >= LEGACY_PREFILL_MIN_TOK && (hd == 128 || hd == 256) && n_head % n_kvh == 0 && n_head / n_kvh <= 16 && scale > 0.f && max_kv &&
+        (((uintptr_t)q | (uintptr_t)gate | (uintptr_t)out | (kind == Q4K_Q8 ? 0u : (uintptr_t)kc | (uintptr_t)vc)) & 15u) == 0) {
+        Q4PrefillArgs f;
+        memset(&f, 0, sizeof(f));
+        f.cache = ref_view(kc, vc, n_kvh, hd, max_kv, kind);
+        f.layout = ref_layout(kind);
+        f.n_head = n_head; f.n_kvh = n_kvh; f.hd = hd;
+        f.q = q; f.gate = gate; f.out = out;
+        f.n_tok = n_tok; f.kv_base = kv_base; f.scale = scale;
+        const int r = q4i_prefill(f);
+        if (r >= 0) return r == 1;   /* else: its workspace may not grow inside a capture */
+    }
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));
     a.one = ref_view(kc, vc, n_kvh, hd, max_kv, kind);

@@ -1,44 +1,41 @@
 /*
- * Dense causal prefill attention over the native q8_0 store on the 5th-generation tensor cores
- * (tcgen05.mma, accumulators in tensor memory, operands brought in by TMA).  Query t of the chunk
- * attends rows [0, min(kv_base + t + 1, max_kv)) -- the semantics of gqa_prefill_k
- * (src/q4_rocm.cu:7019-7206) as launched by q4_hip_qsa_decode_n with n_tok > 1 (:7263,7286-7298);
- * the reference computes it with scalar FMAs on an fp16 tile and re-dequantises every K/V tile for
- * every query token.
+ * Dense causal attention of a chunk of query tokens on the 5th-generation tensor cores (tcgen05.mma, accumulators
+ * in tensor memory, operands brought in by bulk copies).  Query t of the chunk attends rows
+ * [0, min(kv_base + t + 1, max_kv)) -- the semantics of gqa_prefill_k (src/q4_rocm.cu:7019-7206) as launched by
+ * q4_hip_qsa_decode_n with n_tok > 1 (:7263,7286-7298); the reference computes it with scalar FMAs and
+ * re-dequantises every K/V tile for every query token.
  *
- * Two launches per call:
+ * Launches per call:
  *
- *  1. q4_pf_stage_k dequantises the rows the chunk can see, once, into two fp16 staging tensors in
- *     device memory: K as [kv head][row][128] and V transposed as [kv head][dim][row] (value =
- *     fp16(code * scale), the reference's fp16 tile).  25 MB at the benchmark shape, against
- *     1.4 TFLOP of attention that reads each of its tiles 512 times.
- *  2. q4_prefill_k: one block = one kv head x a group of query tokens whose (token, head) pairs
- *     fill the 128 rows of the MMA (16 tokens x 8 heads at the benchmark shape).  Per 64-position
- *     tile, K and V^T arrive by TMA (128-byte swizzle, two stages each) straight into the K-major
- *     operand layout, so no thread touches them:
+ *  1. q4_pf_stage_k turns the rows the chunk can see, once, into fp16 operand tiles: 32 KB images of 128 K rows x 128
+ *     dims and of V^T, already in the 128-byte-swizzled K-major layout that the tensor core reads, so that a tile
+ *     comes in with one plain bulk copy (no tensor maps).  The q8_0 caches of the reference ABI get K as two images,
+ *     fp16(code * scale) and the rest, which together are exact: that entry point always multiplied exact codes.
+ *  2. q4_prefill_k: one block = one kv head x NQ groups of query tokens whose (token, head) pairs fill the 128 rows
+ *     of the MMA each (NQ = 2: 32 tokens x 8 heads at the benchmark shape), against 128-position tiles.
  *
- *       producer warp (one thread): TMA loads, two tiles of K and of V^T in flight
- *       issuer warp (one thread): O[128 x 128] += P . V[j], 4 x tcgen05.mma (k = 16) with P as the A
- *                     operand in tensor memory, as soon as the softmax warps have published P, then
- *                     S[j+2] = Q . K[j+2]^T, 8 x tcgen05.mma, into the score buffer that held S[j]
- *                     and P[j] (two score buffers in tensor memory, so the next tile's scores are
- *                     always ready; products issued by one thread run in order, so P[j] is read
- *                     before S[j+2] lands on it)
- *       4 softmax warps: thread r owns row r: tcgen05.ld its 64 scores of tile j, causal mask,
- *                     running max with lazy rescale (the stored max only moves when it would grow
- *                     by more than 2^8, so the O accumulator in tensor memory is rarely touched),
- *                     P = exp2(..) as fp16 -> tcgen05.st into the first 32 columns of the score
- *                     buffer just read, mbarrier arrive.  Nothing here waits for the previous P . V
- *                     unless O has to be rescaled.
+ *       producer warp (one thread): bulk copies into a ring of five 32 KB slots
+ *       issuer warp (one elected lane): a sequence of units.  O += P . V of unit i as soon as the softmax warps have
+ *                     published its P (64 positions at a time), then S = Q . K^T of the unit that takes over the score
+ *                     buffer just freed (products of one thread run in order)
+ *       softmax warps: thread r owns row r: its scores out of tensor memory, causal mask, running max with lazy
+ *                     rescale, P = exp2(..) as fp16 back into the first half of the score buffer's columns.
  *
- *     The roles meet only at mbarriers (scores ready, P ready, P.V drained, tiles landed): there
- *     is no block-wide barrier inside the tile loop.  Two blocks fit on an SM (97 KB of shared
- *     memory, 256 of the 512 tensor-memory columns each).
+ *     A score buffer holds S and then P of one unit, and every group of softmax warps has two, so that the scores of
+ *     its next unit are computed under its present exponentials.  NQ = 2 (hd 128): units are (64 positions, group),
+ *     four buffers of 64 columns; both groups share every K/V tile.  NQ = 1: units are tiles of 128 positions, two
+ *     buffers of 128 columns.  Tensor memory: 256 columns of scores, NQ x hd of O.
+ *  3. Where query groups alone would leave SMs idle (a short chunk behind a long prefix), the positions are split over
+ *     blockIdx.z; the blocks write (O, m, l) and q4_pf_merge_k combines them.
  *
- * Every mbarrier wait is bounded: on expiry the thread raises a block-wide abort flag that every
- * other wait polls, the block records Q4E_CUDA in the status word, and still frees its tensor memory.
+ * Measured rates of tcgen05.mma with both operands in shared memory: 64 cycles per 128 x 128 x 16, 48 per 128 x 64 x 16
+ * (4 KB of Q and 2 KB of K at 128 B/clk).  Single score buffers of 128 columns per group (all 512 columns in use as
+ * well) make the products cheaper but leave a serial chain S -> softmax -> P . V -> Q . K^T per group: 3270 cycles per
+ * 128 positions of both groups at 8192 tokens over 16 384, the tensor core 63 % busy.
+ *
+ * Every mbarrier wait is bounded: on expiry the thread raises a block-wide abort flag that every other wait polls, the
+ * block records Q4E_CUDA in the status word, and still frees its tensor memory.
  */
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <math_constants.h>
 #include <string.h>
@@ -47,24 +44,28 @@
 
 namespace {
 
-constexpr int PF_ROWS = 128, PF_BN = 64, PF_HD = 128;
-constexpr uint32_t PF_Q_BYTES = 2 * PF_ROWS * 128, PF_K_BYTES = 2 * PF_BN * 128, PF_V_BYTES = PF_HD * 128;
-constexpr uint32_t PF_STAGES = 2;
-constexpr uint32_t PF_THREADS = PF_ROWS + 64;   /* 4 softmax warps, the tensor-core issuer, the TMA producer */
-/* Q | P | K stages | V stages | barriers in the alignment slack */
-constexpr uint32_t PF_TILE_BYTES = PF_Q_BYTES + PF_STAGES * (PF_K_BYTES + PF_V_BYTES);
-constexpr uint32_t PF_SMEM = PF_TILE_BYTES + 1024;
-constexpr uint32_t PF_TMEM_COLS = 256, PF_S_COL = 0, PF_O_COL = 128;   /* S0 at 0, S1 at 64, O at 128 */
-constexpr uint32_t PF_SPIN_LIMIT = 1u << 24;
+constexpr uint32_t PF_ROWS = 128, PF_BN = 128;              /* rows of a query group, positions of a tile */
+constexpr uint32_t PF_CHUNK = 32768, PF_RING = 5;           /* operand image bytes, ring slots */
+constexpr uint32_t PF_Q_BYTES = 65536;                      /* NQ x 128 rows x hd fp16, in every configuration at most this */
+constexpr uint32_t PF_BAR_BYTES = 256;
+constexpr uint32_t PF_SMEM = PF_Q_BYTES + PF_RING * PF_CHUNK + PF_BAR_BYTES + 1024;
+constexpr uint32_t PF_SPIN_LIMIT = 1u << 22;
+constexpr unsigned long long PF_LIMIT_NS = 2000000000ull;   /* a block that has not finished by then gives up */
 constexpr float PF_RESCALE_TAU = 8.f;
 
 struct PrefillParams {
-    uint32_t n_head, n_kvh, gqa, tpc /* tokens per block */;
-    const __nv_bfloat16 *q;
+    uint32_t n_head, n_kvh, gqa, tpc /* tokens per query group */;
+    const void *q;           /* [n_tok][n_head][hd] */
     const float *gate;
-    __nv_bfloat16 *out;
+    void *out;               /* [n_tok][n_head][hd] */
+    int q_bf16, out_bf16;
     uint32_t n_tok, kv_base, max_kv;
     float scale_log2e;
+    const uint8_t *kimg, *vimg;   /* operand images [kv head][tile][chunk][32 KB] */
+    uint32_t img_tiles;           /* tiles per kv head in the images */
+    uint32_t n_split;             /* position ranges of equal tile count; > 1: partial results */
+    float *part;                  /* [split][token][head][hd] unnormalised O */
+    float2 *part_ml;              /* [split][token][head] running max (log2 units), sum */
     uint32_t *err;
 };
 
@@ -74,35 +75,70 @@ __device__ __forceinline__ float ex2f(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+/* two fp32 in one 64-bit register pair */
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+/* x * sigmoid(g) */
+__device__ __forceinline__ float gated(float x, float g) { return __fdividef(x, 1.f + __expf(-g)); }
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
-__device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
-__device__ __forceinline__ uint32_t magic_sub(uint32_t v) { return h2u(__hsub2(u2h(v), u2h(0x64806480u))); }
-
-/* K-major operand tile, 128-byte rows, 16-byte chunks XOR-swizzled by (row & 7) inside 8-row groups */
-__device__ __forceinline__ uint32_t sw128(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
-    /* start >> 4 | LBO (unused with swizzle) = 1 | SBO = 1024 B >> 4 | version 1 | SWIZZLE_128B (2) */
+    /* K-major operand tile, 128-byte rows, 16-byte chunks XOR-swizzled by (row & 7) inside 8-row groups:
+     * start >> 4 | LBO (unused with swizzle) = 1 | SBO = 1024 B >> 4 | version 1 | SWIZZLE_128B (2) */
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+/* The issuing warp runs converged and one elected lane's predicate guards the instruction: the descriptors then stay in
+ * uniform registers.  Issued from a branch that only one lane takes, each product costs about 107 cycles of moves
+ * instead of the 64 that the tensor core needs for 128 x 128 x 16. */
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p;
+}
+__device__ __forceinline__ void umma_f16(uint32_t el, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
 }
 /* same product with the A operand in tensor memory (lane = row, one 32-bit column = two consecutive k) */
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void umma_f16_ta(uint32_t el, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t el, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        ::"r"(bar), "r"(el) : "memory");
 }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -118,6 +154,13 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t *r = reinterpret_cast<uint32_t *>(v);
@@ -147,345 +190,520 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-/* ---- TMA: 3-D tiled loads that complete on an mbarrier */
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t x, int32_t y,
-                                            int32_t z) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+
+/* Programmatic dependent launch: a block may become resident while the previous kernel of the stream drains; nothing
+ * that the stream writes is read before this point. */
+__device__ __forceinline__ void pf_pdl_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-/* ---- staging: rows [0, n) of (layer, kv head) -> fp16 K [kh][row][128] and V^T [kh][dim][n_pad].
- * Block = 64 positions of one kv head, 256 threads: thread t takes the 32-value block t & 3 of row
- * t >> 2, for K and for V; V goes through shared memory to come out position-contiguous. */
-constexpr int PF_VT_PITCH = PF_BN + 2;   /* halves per dim row of the transposition tile (odd word count) */
-__device__ __forceinline__ void dequant32(const uint8_t *codes, __half scale, uint32_t (&o)[16]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4 *>(codes)), b = __ldg(reinterpret_cast<const uint4 *>(codes) + 1);
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    const __half2 s2 = __half2half2(scale);
+/* ---- staging: rows [0, n) of (layer, kv head) -> operand images.  Per tile of 128 positions: KP * HD / 128 images of
+ * K (128 rows x 128 dims: two blocks of 64 dims, rows of 128 bytes), then HD / 128 images' worth of V^T (two blocks of
+ * 64 positions x HD dims).  Rows behind n are zero.  Block = 32 positions of one kv head, K or V (blockIdx.z); V goes
+ * through shared memory to come out position-contiguous.  Short and bound by latency, hence the small blocks: 64
+ * positions of K and V per block took 12.8 us for 2048 rows of hd 256, 2 kv heads. */
+/* dims d .. d + 7 of a row as fp32 (exact for every kind) */
+template <int LAY>
+__device__ __forceinline__ void load8(const uint8_t *row, const uint8_t *srow, uint32_t d, float (&x)[8]) {
+    if constexpr (LAY == LAY_F32) {
+        const float4 a = *reinterpret_cast<const float4 *>(row + d * 4u), b = *reinterpret_cast<const float4 *>(row + d * 4u + 16u);
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+    } else if constexpr (LAY == LAY_F16) {
+        const uint4 w = *reinterpret_cast<const uint4 *>(row + d * 2u);
+        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        /* int8 -> the fp16 numbers 1152 + code by a byte permute, minus 1152 (exact), times the scale */
-        const uint32_t x = w[i] ^ 0x80808080u;
-        o[2 * i] = h2u(__hmul2(u2h(magic_sub(__byte_perm(x, 0x64646464u, 0x4140))), s2));
-        o[2 * i + 1] = h2u(__hmul2(u2h(magic_sub(__byte_perm(x, 0x64646464u, 0x4342))), s2));
+        for (int i = 0; i < 4; i++) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u[i]));
+            x[2 * i] = f.x; x[2 * i + 1] = f.y;
+        }
+    } else {
+        uint32_t u[2];
+        float s;
+        if constexpr (LAY == LAY_Q8P) {
+            const uint2 w = *reinterpret_cast<const uint2 *>(row + d);
+            u[0] = w.x; u[1] = w.y;
+            s = __half2float(reinterpret_cast<const __half *>(srow)[d >> 5]);
+        } else {   /* 34-byte blocks {fp16 scale, 32 codes}, 2-byte aligned */
+            const uint16_t *b = reinterpret_cast<const uint16_t *>(row + (d >> 5) * 34u);
+            const uint16_t *c = b + 1 + ((d & 31u) >> 1);
+            u[0] = (uint32_t)c[0] | ((uint32_t)c[1] << 16);
+            u[1] = (uint32_t)c[2] | ((uint32_t)c[3] << 16);
+            s = __half2float(__ushort_as_half(b[0]));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = (float)(int8_t)(u[i >> 2] >> (8 * (i & 3))) * s;   /* 8 + 11 bits: exact */
     }
 }
-__global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t n_pad,
-                                                     __half *kf, __half *vt) {
-    __shared__ __half tile[PF_HD * PF_VT_PITCH];
-    const uint32_t kh = blockIdx.y, p0 = blockIdx.x * PF_BN, tid = threadIdx.x;
-    const uint32_t r = tid >> 2, qb = tid & 3u, p = p0 + r;
-    const uint8_t *kq = C.k + (uint64_t)layer * C.layer_stride + (uint64_t)kh * C.kvh_stride;
-    const uint8_t *vq = C.v + (uint64_t)layer * C.layer_stride + (uint64_t)kh * C.kvh_stride;
-    const uint8_t *sc = C.s + (uint64_t)layer * C.s_layer_stride + (uint64_t)kh * C.s_kvh_stride;
-    uint32_t o[16];
-    if (p < n) {
-        const __half *srow = reinterpret_cast<const __half *>(sc + (uint64_t)p * C.s_tok_stride);
-        dequant32(kq + (uint64_t)p * C.tok_stride + qb * 32u, __ldg(srow + qb), o);
-        uint4 *dst = reinterpret_cast<uint4 *>(kf + ((size_t)kh * n + p) * PF_HD + qb * 32u);
+template <int LAY, int HD, int KP>
+__global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
+    constexpr uint32_t PITCH = 34;   /* halves per dim row of the transposition tile (odd word count) */
+    constexpr uint32_t CK = KP * HD / 128, CV = HD / 128, PER = HD * 32u / 8u / 256u;   /* groups of 8 dims per thread */
+    __shared__ __half tile[HD * PITCH];
+    const uint32_t kh = blockIdx.y, p0 = blockIdx.x * 32u, tid = threadIdx.x;
+    pf_pdl_sync();
+    const uint8_t *sc = LAY == LAY_Q8P ? C.s + (uint64_t)layer * C.s_layer_stride + (uint64_t)kh * C.s_kvh_stride : nullptr;
+    const uint64_t base = (uint64_t)layer * C.layer_stride + (uint64_t)kh * C.kvh_stride;
+    float x[PER][8];
+    if (blockIdx.z == 0) {
+        const uint8_t *kq = C.k + base;
+        uint8_t *kt = kimg + ((size_t)kh * tiles + p0 / PF_BN) * CK * PF_CHUNK;
 #pragma unroll
-        for (int i = 0; i < 4; i++) dst[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-        dequant32(vq + (uint64_t)p * C.tok_stride + qb * 32u, __ldg(srow + 4 + qb), o);
-    } else {
+        for (uint32_t it = 0; it < PER; it++) {
+            const uint32_t i = tid + 256u * it, p = p0 + i / (HD / 8u), c = i % (HD / 8u);
 #pragma unroll
-        for (int i = 0; i < 16; i++) o[i] = 0u;
+            for (int j = 0; j < 8; j++) x[it][j] = 0.f;
+            if (p < n) load8<LAY>(kq + (uint64_t)p * C.tok_stride, sc + (uint64_t)p * C.s_tok_stride, c * 8u, x[it]);
+        }
+#pragma unroll
+        for (uint32_t it = 0; it < PER; it++) {
+            const uint32_t i = tid + 256u * it, R = p0 % PF_BN + i / (HD / 8u), c = i % (HD / 8u);
+            uint8_t *dst = kt + (c >> 4) * PF_CHUNK + ((c >> 3) & 1u) * 16384u + R * 128u + (((c & 7u) ^ (R & 7u)) << 4);
+            __half2 hi[4], lo[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                hi[j] = __floats2half2_rn(x[it][2 * j], x[it][2 * j + 1]);
+                const float2 f = __half22float2(hi[j]);
+                lo[j] = __floats2half2_rn(x[it][2 * j] - f.x, x[it][2 * j + 1] - f.y);
+            }
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(h2u(hi[0]), h2u(hi[1]), h2u(hi[2]), h2u(hi[3]));
+            if (KP == 2) *reinterpret_cast<uint4 *>(dst + (HD / 128) * PF_CHUNK) = make_uint4(h2u(lo[0]), h2u(lo[1]), h2u(lo[2]), h2u(lo[3]));
+        }
+        return;
+    }
+    const uint8_t *vq = C.v + base;
+    uint8_t *vt = vimg + ((size_t)kh * tiles + p0 / PF_BN) * CV * PF_CHUNK + ((p0 / 64u) & 1u) * (HD * 128u);
+#pragma unroll
+    for (uint32_t it = 0; it < PER; it++) {   /* lanes on consecutive rows: the 2-byte stores below do not conflict */
+        const uint32_t i = tid + 256u * it, p = p0 + (i & 31u), c = i >> 5;
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[it][j] = 0.f;
+        if (p < n) load8<LAY>(vq + (uint64_t)p * C.tok_stride, sc + (uint64_t)p * C.s_tok_stride + 2u * (HD / 32u), c * 8u, x[it]);
     }
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const __half2 h = u2h(o[i]);
-        tile[(qb * 32u + 2 * i) * PF_VT_PITCH + r] = __low2half(h);
-        tile[(qb * 32u + 2 * i + 1) * PF_VT_PITCH + r] = __high2half(h);
+    for (uint32_t it = 0; it < PER; it++) {
+        const uint32_t i = tid + 256u * it;
+#pragma unroll
+        for (int j = 0; j < 8; j++) tile[((i >> 5) * 8u + j) * PITCH + (i & 31u)] = __float2half_rn(x[it][j]);
     }
     __syncthreads();
-    /* dim d = tid >> 1, positions 32 * (tid & 1) .. + 31: 64 contiguous bytes of V^T */
-    const uint32_t d = tid >> 1, h0 = (tid & 1u) * 32u;
-    uint32_t w[16];
 #pragma unroll
-    for (int i = 0; i < 16; i++)
-        w[i] = *reinterpret_cast<const uint32_t *>(&tile[d * PF_VT_PITCH + h0 + 2 * i]);
-    uint4 *dst = reinterpret_cast<uint4 *>(vt + ((size_t)kh * PF_HD + d) * n_pad + p0 + h0);
-#pragma unroll
-    for (int i = 0; i < 4; i++) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    for (uint32_t it = 0; it < PER; it++) {
+        const uint32_t i = tid + 256u * it, d = i >> 2, c = (p0 & 63u) / 8u + (i & 3u);
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(tile + d * PITCH + (i & 3u) * 8u);
+        *reinterpret_cast<uint4 *>(vt + d * 128u + ((c ^ (d & 7u)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
 }
 
-
-__global__ void __launch_bounds__(PF_THREADS, 2) q4_prefill_k(const PrefillParams P, const __grid_constant__ CUtensorMap map_k,
-                                                              const __grid_constant__ CUtensorMap map_v) {
+/* the rest of a wait whose first test found the phase incomplete: at most two seconds from the block's start, and no
+ * longer than every other thread of the block; out of line, so that the loops around it stay short */
+__device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_abort, unsigned long long t_start) {
+    for (uint32_t i = 0; i < PF_SPIN_LIMIT; i++) {
+        if (mbar_test(bar, parity)) return true;
+        if ((i & 63u) == 63u) {
+            uint32_t a;
+            asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(a) : "r"(s_abort) : "memory");
+            if (a) return false;
+            if (global_ns() - t_start > PF_LIMIT_NS) break;
+        }
+    }
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(1u) : "memory");
+    return false;
+}
+/* HD: head size; NQ: query groups per block; KP: images per 128 dims of K (2: value and remainder) */
+template <int HD, int NQ, int KP>
+__global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillParams P) {
+    constexpr uint32_t CK = KP * HD / 128, CV = HD / 128;      /* ring slots a K / V tile takes */
+    constexpr uint32_t SW = NQ * 4;                            /* softmax warps; then the issuer, then the producer */
+    constexpr uint32_t O_COL = 256, TMEM_COLS = 512;           /* scores in the first 256 columns, O of group g at 256 + 128 g */
+    constexpr uint32_t UN = NQ == 2 ? 64 : 128, SB = 2 * NQ;   /* positions of a unit, score buffers */
+    constexpr uint32_t QG_BYTES = PF_ROWS * HD * 2;            /* one group's queries */
+    static_assert(NQ * QG_BYTES <= PF_Q_BYTES && O_COL + NQ * HD <= TMEM_COLS, "shared / tensor memory");
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     /* later token groups see more rows: launch them first so the tail of the grid is made of short blocks */
-    const uint32_t kh = blockIdx.y, t0 = (gridDim.x - 1u - blockIdx.x) * P.tpc;
+    const uint32_t kh = blockIdx.y, t0 = (gridDim.x - 1u - blockIdx.x) * (P.tpc * NQ);
 
     /* 1024-byte aligned operand tiles (the swizzle pattern is anchored to the address) */
-    const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
-    const uint32_t sQ = base, sK = sQ + PF_Q_BYTES, sV = sK + PF_STAGES * PF_K_BYTES;
-    /* barriers in the alignment slack in front of the tiles when there is room, else behind them */
-    const uint32_t bars = (base - smem_u32(smem_dyn) >= 96u) ? smem_u32(smem_dyn) : base + PF_TILE_BYTES;
-    /* bar_p: one per score buffer.  A softmax warp may publish P of tile j + 1 before a slower warp has published
-     * tile j (nothing but the score buffers holds it back), so consecutive tiles must not count on one barrier. */
-    const uint32_t full_k = bars, full_v = bars + 16, bar_s = bars + 32, bar_o = bars + 48, bar_p = bars + 72,
-                   s_tmem = bars + 64, s_abort = bars + 68;
+    const uint32_t sQ = (smem_u32(smem_dyn) + 1023u) & ~1023u, sR = sQ + PF_Q_BYTES, bars = sR + PF_RING * PF_CHUNK;
+    const uint32_t full = bars, empty = bars + 40, bar_s = bars + 80, bar_p = bars + 112, bar_o = bars + 144,
+                   s_tmem = bars + 160, s_abort = bars + 164;
 
-    /* softmax thread r < 128 owns row r = (token t0 + r / gqa, head kh*gqa + r % gqa); rows past tpc*gqa or
-     * past n_tok are padding.  Warp 4 issues the MMAs, warp 5 the TMA loads (one thread each). */
-    const bool softmax_thread = tid < PF_ROWS;
-    const uint32_t tl = tid / P.gqa, hh = tid % P.gqa, tok = t0 + tl;
-    const bool row_live = softmax_thread && tl < P.tpc && tok < P.n_tok;
-    uint32_t row_nkv = 0;                      /* this row attends positions [0, row_nkv) */
-    if (row_live) row_nkv = min(P.kv_base + tok + 1u, P.max_kv);
-    const uint32_t t_last = min(t0 + P.tpc, P.n_tok) - 1u;
+    const uint32_t inv_gqa = 65536u / P.gqa + 1u;   /* row / gqa = row * inv_gqa >> 16 for rows below 128, gqa up to 16 */
+    const uint32_t t_last = min(t0 + P.tpc * NQ, P.n_tok) - 1u;
     const uint32_t cta_nkv = min(P.kv_base + t_last + 1u, P.max_kv);
-    const uint32_t cta_min_nkv = min(P.kv_base + t0 + 1u, P.max_kv);
-    const uint32_t n_tiles = (cta_nkv + PF_BN - 1u) / PF_BN;
+    const uint32_t all_tiles = (cta_nkv + PF_BN - 1u) / PF_BN;
+    /* this block's range of tiles */
+    const uint32_t j0 = (uint32_t)((uint64_t)all_tiles * blockIdx.z / P.n_split), j1 = (uint32_t)((uint64_t)all_tiles * (blockIdx.z + 1u) / P.n_split);
+    const uint32_t n_tiles = j1 - j0;
+    /* units per group: the last tile may be needed in half only */
+    const uint32_t n_seq = NQ == 2 ? min(n_tiles * 2u, (cta_nkv - j0 * PF_BN + 63u) / 64u) : n_tiles, n_units = n_seq * NQ;
 
-    if (warp == 4) {
+    if (warp == SW) {
         if (lane == 0) {
 #pragma unroll
-            for (uint32_t s = 0; s < PF_STAGES; s++) {
-                mbar_init(full_k + 8 * s, 1);
-                mbar_init(full_v + 8 * s, 1);
+            for (uint32_t s = 0; s < PF_RING; s++) {
+                mbar_init(full + 8 * s, 1);
+                mbar_init(empty + 8 * s, 1);
+            }
+#pragma unroll
+            for (uint32_t s = 0; s < 4; s++) {
                 mbar_init(bar_s + 8 * s, 1);
+                mbar_init(bar_p + 8 * s, PF_ROWS);
             }
             mbar_init(bar_o, 1);
-            mbar_init(bar_p, PF_ROWS);
-            mbar_init(bar_p + 8, PF_ROWS);
+            mbar_init(bar_o + 8, 1);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(0u) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem),
-                     "r"(PF_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    } else if (warp < 4) {
-        /* ---- Q rows: bf16 -> fp16 (exact for normal values), K-major swizzled, 2 k-blocks of 64 dims */
-        const __nv_bfloat16 *qrow = P.q + ((size_t)tok * P.n_head + (size_t)kh * P.gqa + hh) * PF_HD;
+    }
+    pf_pdl_sync();
+    if (warp < SW) {
+        /* ---- queries as fp16 (exact for normal bf16 values), K-major swizzled, blocks of 64 dims: 8 dims per thread
+         * and step, whole rows per warp step */
+        constexpr uint32_t PER = HD / 8u, BATCH = 4u;   /* loads in flight before the first store */
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < PER; k0 += BATCH) {
+            uint4 w[BATCH][2];
 #pragma unroll
-        for (uint32_t c = 0; c < 16; c++) {
-            uint4 w = make_uint4(0u, 0u, 0u, 0u);
-            if (row_live) w = *reinterpret_cast<const uint4 *>(qrow + c * 8);
-            const uint32_t in[4] = {w.x, w.y, w.z, w.w};
-            uint32_t o[4];
+            for (uint32_t k = 0; k < BATCH; k++) {
+                const uint32_t i = tid + (k0 + k) * SW * 32u, row = i / PER, c = i % PER, g = row / PF_ROWS, r = row % PF_ROWS;
+                const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl;
+                w[k][0] = w[k][1] = make_uint4(0u, 0u, 0u, 0u);
+                if (tl < P.tpc && tok < P.n_tok) {
+                    const size_t off = ((size_t)tok * P.n_head + (size_t)kh * P.gqa + (r - tl * P.gqa)) * HD + c * 8u;
+                    if (P.q_bf16) {
+                        w[k][0] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + off);
+                    } else {
+                        w[k][0] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(P.q) + off);
+                        w[k][1] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(P.q) + off + 4);
+                    }
+                }
+            }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                o[i] = h2u(__floats2half2_rn(__uint_as_float(in[i] << 16), __uint_as_float(in[i] & 0xffff0000u)));
-            const uint32_t a = sQ + (c >> 3) * (PF_ROWS * 128) + sw128(tid, c & 7);
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+            for (uint32_t k = 0; k < BATCH; k++) {
+                const uint32_t i = tid + (k0 + k) * SW * 32u, row = i / PER, c = i % PER, g = row / PF_ROWS, r = row % PF_ROWS;
+                const uint32_t in[8] = {w[k][0].x, w[k][0].y, w[k][0].z, w[k][0].w, w[k][1].x, w[k][1].y, w[k][1].z, w[k][1].w};
+                uint32_t o[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    o[e] = P.q_bf16 ? h2u(__floats2half2_rn(__uint_as_float(in[e] << 16), __uint_as_float(in[e] & 0xffff0000u)))
+                                    : h2u(__floats2half2_rn(__uint_as_float(in[2 * e]), __uint_as_float(in[2 * e + 1])));
+                const uint32_t a = sQ + g * QG_BYTES + (c >> 3) * (PF_ROWS * 128u) + r * 128u + (((c & 7u) ^ (r & 7u)) << 4);
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+            }
         }
         fence_async_smem();
     }
     tc_fence_before();
-    __syncthreads();          /* barriers initialised, Q in place, tensor memory allocated */
+    __syncthreads();          /* barriers initialised, queries in place, tensor memory allocated */
     tc_fence_after();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(s_tmem));
 
-    constexpr uint32_t IDESC_QK = (1u << 4) | ((uint32_t)(PF_BN >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
-    constexpr uint32_t IDESC_PV = (1u << 4) | ((uint32_t)(PF_HD >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
-    /* bounded wait that also gives up when any thread of the block has given up */
-    auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        for (uint32_t i = 0; i < PF_SPIN_LIMIT; i++) {
-            if (mbar_test(bar, parity)) return true;
-            if ((i & 1023u) == 1023u) {
-                uint32_t a;
-                asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(a) : "r"(s_abort) : "memory");
-                if (a) return false;
-            }
-        }
-        asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(1u) : "memory");
-        return false;
+    constexpr uint32_t IDESC_QK = (1u << 4) | ((uint32_t)(UN >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
+    constexpr uint32_t IDESC_PV = (1u << 4) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
+    const unsigned long long t_start = global_ns();
+    auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_test(bar, parity) || pf_wait(bar, parity, s_abort, t_start); };
+    /* by a whole warp, which goes on as one; the test that succeeds at once stays in line */
+    auto all_wait = [&](uint32_t bar, uint32_t parity) -> bool {
+        if (__builtin_expect(__all_sync(0xffffffffu, mbar_test(bar, parity)), 1)) return true;
+        return __all_sync(0xffffffffu, pf_wait(bar, parity, s_abort, t_start));
     };
+    /* order of the images in the ring, that of their first use: K0 V0 K1 V1 .. where two groups share a tile, K0 K1 V0 K2
+     * V1 .. V(n-1) where units are tiles (the scores run a tile and two tiles ahead of P . V) */
     bool ok = true;
 
-    if (warp == 5) {
-        /* ================= producer: one thread keeps two tiles of K and of V^T in flight ================= */
+    if (warp == SW + 1) {
+        /* ================= producer: one thread keeps the ring full ================= */
         if (lane == 0 && n_tiles > 0) {
-            auto load_k = [&](uint32_t tile) {     /* two 64-dim boxes of 64 rows */
-                const uint32_t st = tile % PF_STAGES, bar = full_k + 8 * st, dst = sK + st * PF_K_BYTES;
-                mbar_expect_tx(bar, PF_K_BYTES);
-                tma_load_3d(dst, &map_k, bar, 0, (int32_t)(tile * PF_BN), (int32_t)kh);
-                tma_load_3d(dst + PF_BN * 128, &map_k, bar, 64, (int32_t)(tile * PF_BN), (int32_t)kh);
-            };
-            auto load_v = [&](uint32_t tile) {     /* one box: 64 positions x 128 dims of V^T */
-                const uint32_t st = tile % PF_STAGES, bar = full_v + 8 * st;
-                mbar_expect_tx(bar, PF_V_BYTES);
-                tma_load_3d(sV + st * PF_V_BYTES, &map_v, bar, (int32_t)(tile * PF_BN), 0, (int32_t)kh);
-            };
-            uint32_t k_issued = 1, v_issued = 1;
-            load_k(0);
-            load_v(0);
-            if (n_tiles > 1) {
-                load_k(1);
-                load_v(1);
-                k_issued = v_issued = 2;
-            }
-            for (uint32_t tile = 0; tile < n_tiles && ok; tile++) {
-                const uint32_t st = tile % PF_STAGES, use = (tile / PF_STAGES) & 1u;
-                /* Q.K of this tile complete: its K stage takes the tile two ahead */
-                if (tile + 2 < n_tiles) {
-                    ok = wait(bar_s + 8 * st, use);
-                    if (ok) { load_k(tile + 2); k_issued = tile + 3; }
+            uint32_t at = 0;
+            auto load = [&](const uint8_t *src, uint32_t chunks) {
+                for (uint32_t c = 0; c < chunks && ok; c++, at++) {
+                    const uint32_t s = at % PF_RING, use = at / PF_RING;
+                    if (use > 0) ok = wait(empty + 8 * s, (use - 1u) & 1u);
+                    if (ok) {
+                        mbar_expect_tx(full + 8 * s, PF_CHUNK);
+                        bulk_load(sR + s * PF_CHUNK, src + (size_t)c * PF_CHUNK, PF_CHUNK, full + 8 * s);
+                    } else {
+                        return;
+                    }
                 }
-                /* P.V of the previous tile complete: its V stage takes the tile after this one */
-                if (ok && tile > 0 && tile + 1 < n_tiles) {
-                    ok = wait(bar_o, (tile - 1u) & 1u);
-                    if (ok) { load_v(tile + 1); v_issued = tile + 2; }
-                }
+            };
+            const uint8_t *ks = P.kimg + ((size_t)kh * P.img_tiles + j0) * CK * PF_CHUNK, *vs = P.vimg + ((size_t)kh * P.img_tiles + j0) * CV * PF_CHUNK;
+            load(ks, CK);
+            if (NQ == 1 && n_tiles > 1) load(ks + (size_t)CK * PF_CHUNK, CK);
+            for (uint32_t j = 0; j < n_tiles && ok; j++) {
+                load(vs + (size_t)j * CV * PF_CHUNK, CV);
+                if (j + (3u - NQ) < n_tiles) load(ks + (size_t)(j + (3u - NQ)) * CK * PF_CHUNK, CK);
             }
-            /* Gave up somewhere: copies still in flight must land before the block's shared memory is
-             * released (bounded again; these probes ignore the abort flag; phases that completed long ago
-             * answer at once). */
-            if (!ok) {
-                for (uint32_t t = k_issued > 2 ? k_issued - 2 : 0; t < k_issued; t++)
-                    for (uint32_t i = 0; i < PF_SPIN_LIMIT && !mbar_test(full_k + 8 * (t % PF_STAGES), (t / PF_STAGES) & 1u); i++) {}
-                for (uint32_t t = v_issued > 2 ? v_issued - 2 : 0; t < v_issued; t++)
-                    for (uint32_t i = 0; i < PF_SPIN_LIMIT && !mbar_test(full_v + 8 * (t % PF_STAGES), (t / PF_STAGES) & 1u); i++) {}
-            }
+            /* Gave up somewhere: copies still in flight must land before the block's shared memory is released
+             * (bounded again; these probes ignore the abort flag; phases that completed long ago answer at once). */
+            if (!ok)
+                for (uint32_t t = at > PF_RING ? at - PF_RING : 0; t < at; t++)
+                    for (uint32_t i = 0; i < 4096u && !mbar_test(full + 8 * (t % PF_RING), (t / PF_RING) & 1u); i++) {}
         }
-    } else if (warp == 4) {
-        /* ================= tensor-core issuer: one thread ================= */
-        if (lane == 0 && n_tiles > 0) {
-            auto issue_qk = [&](uint32_t tile) {
-                const uint32_t st = tile % PF_STAGES;
-#pragma unroll
-                for (uint32_t kk = 0; kk < 8; kk++) {
-                    const uint64_t ad = umma_desc(sQ + (kk >> 2) * (PF_ROWS * 128) + (kk & 3) * 32);
-                    const uint64_t bd = umma_desc(sK + st * PF_K_BYTES + (kk >> 2) * (PF_BN * 128) + (kk & 3) * 32);
-                    umma_f16(tmem + PF_S_COL + st * PF_BN, ad, bd, IDESC_QK, kk > 0);
-                }
-                umma_commit(bar_s + 8 * st);
+    } else if (warp == SW) {
+        /* ================= tensor-core issuer: a converged warp, one elected lane ================= */
+        if (n_tiles > 0) {
+            const uint32_t el = elect_one();
+            /* the ring is consumed in order: (slot, phase) of the next image */
+            uint32_t slot = 0, phase = 0;
+            auto take = [&]() -> uint32_t {
+                const uint32_t s = slot;
+                ok = ok && all_wait(full + 8 * s, phase);
+                if (++slot == PF_RING) { slot = 0; phase ^= 1u; }
+                return s;
             };
-            /* both score buffers are filled ahead of the softmax */
-            ok = wait(full_k, 0);
-            tc_fence_after();
-            if (ok) issue_qk(0);
-            if (ok && n_tiles > 1) {
-                ok = wait(full_k + 8, 0);
-                tc_fence_after();
-                if (ok) issue_qk(1);
-            }
-            for (uint32_t tile = 0; tile < n_tiles && ok; tile++) {
-                const uint32_t st = tile % PF_STAGES, use = (tile / PF_STAGES) & 1u;
-                /* operands first (they land while the softmax runs), then the softmax's hand-over, so that
-                 * nothing but the issue itself stands between "P is ready" and the two products */
-                ok = wait(full_v + 8 * st, use);
-                if (ok && tile + 2 < n_tiles) ok = wait(full_k + 8 * st, ((tile + 2) / PF_STAGES) & 1u);
-                /* softmax of this tile done: P is in shared memory, O is rescaled, S[st] has been read */
-                ok = ok && wait(bar_p + 8 * st, use);
+            const uint64_t q_desc = umma_desc(sQ), r_desc = umma_desc(sR);   /* byte offsets / 16 are added to these */
+            auto qk_chunk = [&](uint32_t s_col, uint32_t g, uint32_t c, uint32_t s, uint32_t row0) {
+                const uint64_t qd = q_desc + ((g * QG_BYTES + (c % (HD / 128)) * (2u * PF_ROWS * 128u)) >> 4), kd = r_desc + ((s * PF_CHUNK + row0 * 128u) >> 4);
+#pragma unroll
+                for (uint32_t kk = 0; kk < 8; kk++)
+                    umma_f16(el, tmem + s_col, qd + (((kk >> 2) * (PF_ROWS * 128u) + (kk & 3) * 32u) >> 4),
+                             kd + (((kk >> 2) * (PF_BN * 128u) + (kk & 3) * 32u) >> 4), IDESC_QK, (c | kk) > 0);
+            };
+            auto pv_half = [&](uint32_t s_col, uint32_t g, uint32_t s, uint32_t half_off, bool first) {
+                const uint64_t vd = r_desc + ((s * PF_CHUNK + half_off) >> 4);
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4; kk++)
+                    umma_f16_ta(el, tmem + O_COL + g * 128u, tmem + s_col + kk * 8u, vd + kk * 2u, IDESC_PV, (first && kk == 0) ? 0u : 1u);
+            };
+            if (NQ == 2) {
+                /* per tile: its P . V for both groups and both halves, each followed by the scores that take over the buffer */
+                uint32_t ks[CK];
+#pragma unroll
+                for (uint32_t c = 0; c < CK; c++) ks[c] = take();
                 tc_fence_after();
                 if (ok) {
 #pragma unroll
-                    for (uint32_t kk = 0; kk < 4; kk++) {
-                        const uint64_t bd = umma_desc(sV + st * PF_V_BYTES + kk * 32);
-                        umma_f16_ta(tmem + PF_O_COL, tmem + PF_S_COL + st * PF_BN + kk * 8, bd, IDESC_PV,
-                                    (tile > 0 || kk > 0) ? 1u : 0u);
+                    for (uint32_t e = 0; e < 4; e++)
+                        if ((e >> 1) < n_seq) {
+#pragma unroll
+                            for (uint32_t c = 0; c < CK; c++) qk_chunk((e & 1u) * 128u + (e >> 1) * 64u, e & 1u, c, ks[c], (e >> 1) * 64u);
+                            umma_commit(el, bar_s + 8 * e);
+                        }
+#pragma unroll
+                    for (uint32_t c = 0; c < CK; c++) umma_commit(el, empty + 8 * ks[c]);
+                }
+                for (uint32_t j = 0; j < n_tiles && ok; j++) {
+                    const uint32_t sv = take();
+                    const bool more = j + 1u < n_tiles;
+                    if (more) {
+#pragma unroll
+                        for (uint32_t c = 0; c < CK; c++) ks[c] = take();
                     }
-                    umma_commit(bar_o);
-                    if (tile + 2 < n_tiles) issue_qk(tile + 2);
+#pragma unroll
+                    for (uint32_t e = 0; e < 4; e++) {   /* buffer e: half e >> 1, group e & 1 */
+                        if (2u * j + (e >> 1) >= n_seq) continue;
+                        ok = ok && all_wait(bar_p + 8 * e, j & 1u);
+                        tc_fence_after();
+                        if (!ok) break;
+                        pv_half((e & 1u) * 128u + (e >> 1) * 64u, e & 1u, sv, (e >> 1) * (HD * 128u), j == 0 && e < 2);
+                        umma_commit(el, bar_o + 8 * (e & 1u));
+                        if (e == 3) umma_commit(el, empty + 8 * sv);
+                        if (2u * (j + 1u) + (e >> 1) < n_seq) {
+#pragma unroll
+                            for (uint32_t c = 0; c < CK; c++) qk_chunk((e & 1u) * 128u + (e >> 1) * 64u, e & 1u, c, ks[c], (e >> 1) * 64u);
+                            umma_commit(el, bar_s + 8 * e);
+                        }
+                    }
+                    if (more && ok) {
+#pragma unroll
+                        for (uint32_t c = 0; c < CK; c++) umma_commit(el, empty + 8 * ks[c]);
+                    }
+                }
+            } else {
+                auto issue_qk = [&](uint32_t j) {
+                    for (uint32_t c = 0; c < CK && ok; c++) {
+                        const uint32_t s = take();
+                        tc_fence_after();
+                        if (!ok) return;
+                        qk_chunk((j & 1u) * 128u, 0u, c, s, 0u);
+                        umma_commit(el, empty + 8 * s);
+                    }
+                    umma_commit(el, bar_s + 8 * (j & 1u));
+                };
+                issue_qk(0);
+                if (ok && n_tiles > 1) issue_qk(1);
+                for (uint32_t j = 0; j < n_tiles && ok; j++) {
+                    uint32_t s = 0;
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; h++) {   /* 64 positions each; the operands land while the softmax runs */
+                        if (CV == 2 || h == 0) s = take();
+                        if (h == 0) ok = ok && all_wait(bar_p + 8 * (j & 1u), (j >> 1) & 1u);
+                        tc_fence_after();
+                        if (!ok) break;
+                        pv_half((j & 1u) * 128u + h * 32u, 0u, s, CV == 2 ? 0u : h * (HD * 128u), j == 0 && h == 0);
+                        if (CV == 2 || h == 1) umma_commit(el, empty + 8 * s);
+                    }
+                    if (ok) {
+                        umma_commit(el, bar_o);
+                        if (j + 2u < n_tiles) issue_qk(j + 2u);
+                    }
                 }
             }
         }
     } else {
-        /* ================= softmax (warps 0-3): thread r owns row r ================= */
-        const uint32_t t_lane = tmem + ((warp * 32u) << 16);   /* this warp's 32 lanes of tensor memory */
+        /* ================= softmax: thread r of group g owns row r of that group's queries ================= */
+        const uint32_t g = warp >> 2, r = tid & 127u, t_lane = tmem + (((warp & 3u) * 32u) << 16);
+        const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl, head = kh * P.gqa + r - tl * P.gqa;   /* rows past tpc * gqa or past n_tok are padding */
+        const bool row_live = tl < P.tpc && tok < P.n_tok;
+        /* this row attends positions [0, row_nkv); padding rows (queries of zeros, never stored) need no mask */
+        const uint32_t row_nkv = row_live ? min(P.kv_base + tok + 1u, P.max_kv) : 0xffffffffu;
+        const uint32_t warp_min = __reduce_min_sync(0xffffffffu, row_nkv);
         float m_ref = -CUDART_INF_F, l_run = 0.f;
-        for (uint32_t tile = 0; tile < n_tiles && ok; tile++) {
-            const uint32_t st = tile % PF_STAGES, use = (tile / PF_STAGES) & 1u;
-            ok = __all_sync(0xffffffffu, wait(bar_s + 8 * st, use));   /* a warp leaves the loop as one */
+        for (uint32_t u = 0; u < n_seq && ok; u++) {
+            const uint32_t i = u * NQ + g, b = i % SB, use = (i / SB) & 1u, p0 = j0 * PF_BN + u * UN;
+            const uint32_t t_s = t_lane + (NQ == 2 ? g * 128u + (u & 1u) * 64u : b * 128u);
+            ok = all_wait(bar_s + 8 * b, use);   /* a warp leaves the loop as one */
             tc_fence_after();
-            float s[64];
-            tmem_ld32(t_lane + PF_S_COL + st * PF_BN, *reinterpret_cast<float(*)[32]>(&s[0]));
-            tmem_ld32(t_lane + PF_S_COL + st * PF_BN + 32, *reinterpret_cast<float(*)[32]>(&s[32]));
+            float s[UN];
+#pragma unroll
+            for (int c = 0; c < (int)UN / 32; c++) tmem_ld32(t_s + 32 * c, *reinterpret_cast<float(*)[32]>(&s[32 * c]));
             tmem_wait_ld();
-            const uint32_t p0 = tile * PF_BN;
-            float mx0 = -CUDART_INF_F, mx1 = -CUDART_INF_F, mx2 = -CUDART_INF_F, mx3 = -CUDART_INF_F;
-            if (!(p0 + PF_BN <= cta_min_nkv && row_live)) {
+            if (__builtin_expect(p0 + UN > warp_min, 0)) {
 #pragma unroll
-                for (int i = 0; i < 64; i++)
-                    if (p0 + i >= row_nkv) s[i] = -CUDART_INF_F;
+                for (int k = 0; k < (int)UN; k++)
+                    if (p0 + k >= row_nkv) s[k] = -CUDART_INF_F;
+            }
+            /* P of 64 positions against the reference maximum, as fp16 pairs; sums into ls */
+            auto exps = [&](int h, float mneg, uint32_t (&pk)[32], uint64_t (&ls)[2]) {
+                const uint64_t sc2 = pack2(P.scale_log2e, P.scale_log2e), mn2 = pack2(mneg, mneg);
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    const float2 x = unpack2(fma2(pack2(s[64 * h + 2 * k], s[64 * h + 2 * k + 1]), sc2, mn2));
+                    const float e0 = ex2f(x.x), e1 = ex2f(x.y);
+                    ls[k & 1] = add2(ls[k & 1], pack2(e0, e1));
+                    pk[k] = h2u(__floats2half2_rn(e0, e1));
+                }
+            };
+            /* The exponentials start against the maximum of the units before, while this unit's own is still being
+             * formed: the reference only has to be within 2^8 of it.  Where it is not (the first unit, a large new
+             * score) the reference moves and they are taken again. */
+            float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+            uint32_t pk[UN / 64][32];
+            uint64_t ls[2] = {0ull, 0ull};
+            {
+                const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
+#pragma unroll
+                for (int h = 0; h < (int)UN / 64; h++) exps(h, mneg, pk[h], ls);
             }
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
-                mx0 = fmaxf(mx0, s[i]); mx1 = fmaxf(mx1, s[i + 1]);
-                mx2 = fmaxf(mx2, s[i + 2]); mx3 = fmaxf(mx3, s[i + 3]);
+            for (int k = 0; k < (int)UN; k += 8) {
+                mx[0] = fmaxf(fmaxf(mx[0], s[k]), s[k + 1]); mx[1] = fmaxf(fmaxf(mx[1], s[k + 2]), s[k + 3]);
+                mx[2] = fmaxf(fmaxf(mx[2], s[k + 4]), s[k + 5]); mx[3] = fmaxf(fmaxf(mx[3], s[k + 6]), s[k + 7]);
             }
-            const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * P.scale_log2e;   /* scale > 0 */
-            float alpha = 1.f;
-            const bool grow = mx > m_ref + PF_RESCALE_TAU;   /* also true on the first live tile (m_ref = -inf) */
-            if (grow) {
-                alpha = ex2f(m_ref - mx);             /* 0 on the first tile */
-                m_ref = mx;
-                l_run *= alpha;
-            }
-            const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
-            float ls0 = 0.f, ls1 = 0.f;
-            uint32_t pk[32];
+            const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * P.scale_log2e;   /* scale > 0 */
+            const bool grow = m_new > m_ref + PF_RESCALE_TAU;   /* also true on the first live unit (m_ref = -inf) */
+            if (__builtin_expect(__any_sync(0xffffffffu, grow), 0)) {
+                float alpha = 1.f;
+                if (grow) {
+                    alpha = ex2f(m_ref - m_new);             /* 0 on the first live unit */
+                    m_ref = m_new;
+                    l_run *= alpha;
+                }
+                const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
+                ls[0] = ls[1] = 0ull;
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-                const float e0 = ex2f(fmaf(s[2 * i], P.scale_log2e, mneg));
-                const float e1 = ex2f(fmaf(s[2 * i + 1], P.scale_log2e, mneg));
-                ls0 += e0;
-                ls1 += e1;
-                pk[i] = h2u(__floats2half2_rn(e0, e1));
-            }
-            l_run += ls0 + ls1;
-            /* O is rescaled only when the stored maximum moved; the previous P.V must have drained first.  P itself
-             * waits for nothing: it goes into the first 32 columns of the score buffer this thread has just read
-             * (two fp16 per column), which the tensor core reads as the A operand of P.V before the scores of the
-             * tile two ahead are written there (products issued by one thread run in order). */
-            if (tile > 0 && __any_sync(0xffffffffu, grow)) {
-                ok = __all_sync(0xffffffffu, ok && wait(bar_o, (tile - 1u) & 1u));
-                tc_fence_after();
+                for (int h = 0; h < (int)UN / 64; h++) exps(h, mneg, pk[h], ls);
+                /* O is rescaled only here; the group's previous P . V must have drained first */
+                if (u > 0) {
+                    ok = all_wait(bar_o + 8 * g, (u - 1u) & 1u) && ok;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < HD / 32; c++) {
+                        float o[32];
+                        tmem_ld32(t_lane + O_COL + g * 128u + 32 * c, o);
+                        tmem_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    float o[32];
-                    tmem_ld32(t_lane + PF_O_COL + 32 * c, o);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; i++) o[i] *= alpha;
-                    tmem_st32(t_lane + PF_O_COL + 32 * c, o);
+                        for (int k = 0; k < 32; k++) o[k] *= alpha;
+                        tmem_st32(t_lane + O_COL + g * 128u + 32 * c, o);
+                    }
                 }
             }
-            tmem_st32(t_lane + PF_S_COL + st * PF_BN, *reinterpret_cast<const float(*)[32]>(&pk[0]));
+            /* P goes into the first half of the score buffer this thread has just read (two fp16 per column) */
+#pragma unroll
+            for (int h = 0; h < (int)UN / 64; h++) tmem_st32(t_s + 32 * h, *reinterpret_cast<const float(*)[32]>(&pk[h][0]));
             tmem_wait_st();
+            /* A parity wait can tell the current phase from the one before it, no further, and bar_o's phases are not
+             * followed unit by unit.  So the phase before the last is waited for here, while the last cannot
+             * complete without this thread (that of unit n - 3 has: the scores of unit n - 1 were committed behind it). */
+            if (u > 0 && u + 1u == n_seq) ok = all_wait(bar_o + 8 * g, (u - 1u) & 1u) && ok;
             tc_fence_before();
-            mbar_arrive(bar_p + 8 * st);
+            mbar_arrive(bar_p + 8 * b);
+            const float2 l0 = unpack2(ls[0]), l1 = unpack2(ls[1]);
+            l_run += (l0.x + l0.y) + (l1.x + l1.y);
         }
-        /* The last P.V.  A parity wait can tell the current phase from the one before it, no further: this thread
-         * has not followed the phases of bar_o tile by tile, and when it gets here the product of tile n - 3 is
-         * complete (the scores of tile n - 1 were committed behind it) but perhaps not yet that of tile n - 2. */
-        if (ok && n_tiles > 1) ok = wait(bar_o, (n_tiles - 2u) & 1u);
-        if (ok && n_tiles > 0) ok = wait(bar_o, (n_tiles - 1u) & 1u);
+        if (ok && n_seq > 0) ok = wait(bar_o + 8 * g, (n_seq - 1u) & 1u);
+        ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
 
-        /* ---- epilogue: O / l * sigmoid(gate) -> bf16 */
+        /* ---- epilogue: O / l * sigmoid(gate), or the unnormalised part of a split range.  32 columns at a time go
+         * through the warp's share of the query tiles (read by no product any more), so that rows leave in whole lines */
         if (ok) {
-            const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-            const size_t off = ((size_t)tok * P.n_head + (size_t)kh * P.gqa + hh) * PF_HD;
+            const bool split = P.n_split > 1u;
+            const float inv = split ? 1.f : l_run > 0.f ? 1.f / l_run : 0.f;
+            float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + g * QG_BYTES + (warp & 3u) * (QG_BYTES / 4u));   /* [32][36] */
+            const uint32_t w_row0 = (warp & 3u) * 32u;
+            if (split && row_live)
+                P.part_ml[((size_t)blockIdx.z * P.n_tok + tok) * P.n_head + head] = make_float2(m_ref, l_run);
+            /* step q of a column block: 4 rows of 32 columns, 8 lanes each; the gates are requested a column block ahead */
+            uint32_t off[8], live = 0;   /* in 16-byte units from the chunk's first token */
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+            for (int q = 0; q < 8; q++) {
+                const uint32_t row = w_row0 + 4u * q + (lane >> 3), ti = row * inv_gqa >> 16;
+                if (ti < P.tpc && t0 + g * P.tpc + ti < P.n_tok) live |= 1u << q;
+                off[q] = ((g * P.tpc + ti) * P.n_head + kh * P.gqa + (row - ti * P.gqa)) * (HD / 4u) + (lane & 7u);
+            }
+            const size_t first = (size_t)t0 * P.n_head * (HD / 4u);
+            const bool gates = P.gate && !split;
+            float4 gt[8];
+            auto fetch_gates = [&](int c) {
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if (gates && ((live >> q) & 1u)) gt[q] = reinterpret_cast<const float4 *>(P.gate)[first + off[q] + 8u * c];
+            };
+            fetch_gates(0);
+#pragma unroll 1
+            for (int c = 0; c < HD / 32; c++) {
                 float o[32];
-                tmem_ld32(t_lane + PF_O_COL + 32 * c, o);
-                tmem_wait_ld();
-                if (row_live) {
+                if (n_tiles > 0) {
+                    tmem_ld32(t_lane + O_COL + g * 128u + 32 * c, o);
+                    tmem_wait_ld();
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint32_t w[4];
+                    for (int k = 0; k < 32; k++) o[k] = 0.f;
+                }
+                __syncwarp();
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            float x0 = o[i + 2 * j] * inv, x1 = o[i + 2 * j + 1] * inv;
-                            if (P.gate) {
-                                const float2 gt = *reinterpret_cast<const float2 *>(P.gate + off + 32 * c + i + 2 * j);
-                                x0 *= 1.f / (1.f + __expf(-gt.x));
-                                x1 *= 1.f / (1.f + __expf(-gt.y));
-                            }
-                            __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
-                            w[j] = *reinterpret_cast<uint32_t *>(&b);
-                        }
-                        *reinterpret_cast<uint4 *>(P.out + off + 32 * c + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                for (int k = 0; k < 32; k += 4)
+                    *reinterpret_cast<float4 *>(buf + lane * 36u + k) = make_float4(o[k] * inv, o[k + 1] * inv, o[k + 2] * inv, o[k + 3] * inv);
+                __syncwarp();
+                float4 x[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    x[q] = *reinterpret_cast<const float4 *>(buf + (4u * q + (lane >> 3)) * 36u + 4u * (lane & 7u));
+                    if (gates) {
+                        x[q].x = gated(x[q].x, gt[q].x); x[q].y = gated(x[q].y, gt[q].y);
+                        x[q].z = gated(x[q].z, gt[q].z); x[q].w = gated(x[q].w, gt[q].w);
+                    }
+                }
+                if (c + 1 < HD / 32) fetch_gates(c + 1);
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    if (!((live >> q) & 1u)) continue;
+                    const size_t at = first + off[q] + 8u * c;
+                    if (split) {
+                        reinterpret_cast<float4 *>(P.part)[(size_t)blockIdx.z * P.n_tok * P.n_head * (HD / 4u) + at] = x[q];
+                    } else if (P.out_bf16) {
+                        const __nv_bfloat162 b0 = __floats2bfloat162_rn(x[q].x, x[q].y), b1 = __floats2bfloat162_rn(x[q].z, x[q].w);
+                        reinterpret_cast<uint2 *>(P.out)[at] = make_uint2(*reinterpret_cast<const uint32_t *>(&b0), *reinterpret_cast<const uint32_t *>(&b1));
+                    } else {
+                        reinterpret_cast<float4 *>(P.out)[at] = x[q];
                     }
                 }
             }
@@ -494,115 +712,162 @@ __global__ void __launch_bounds__(PF_THREADS, 2) q4_prefill_k(const PrefillParam
     if (!ok && lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
     tc_fence_before();
     __syncthreads();
-    if (warp == 4)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PF_TMEM_COLS) : "memory");
+    if (warp == SW)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
-/* ---- host side: staging tensors, tensor maps, launches */
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult st;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &st) == cudaSuccess &&
-            st == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-        else
-            (void)cudaGetLastError();
+/* ---- the parts of split position ranges -> out: thread = 4 dims of one (token, head) */
+__global__ void __launch_bounds__(256) q4_pf_merge_k(const PrefillParams P, uint32_t hd, uint64_t total4) {
+    const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
+    pf_pdl_sync();
+    if (i >= total4) return;
+    const uint64_t row = i / (hd / 4u), rows = (uint64_t)P.n_tok * P.n_head;
+    float M = -CUDART_INF_F;
+    for (uint32_t s = 0; s < P.n_split; s++) M = fmaxf(M, P.part_ml[s * rows + row].x);
+    const float Mu = M == -CUDART_INF_F ? 0.f : M;
+    float L = 0.f;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t s = 0; s < P.n_split; s++) {
+        const float2 ml = P.part_ml[s * rows + row];
+        const float w = ml.y > 0.f ? ex2f(ml.x - Mu) : 0.f;
+        const float4 a = reinterpret_cast<const float4 *>(P.part)[s * total4 + i];
+        L = fmaf(w, ml.y, L);
+        x.x = fmaf(w, a.x, x.x); x.y = fmaf(w, a.y, x.y); x.z = fmaf(w, a.z, x.z); x.w = fmaf(w, a.w, x.w);
     }
-    return fn;
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
+    if (P.gate) {
+        const float4 gt = reinterpret_cast<const float4 *>(P.gate)[i];
+        x.x = gated(x.x, gt.x); x.y = gated(x.y, gt.y);
+        x.z = gated(x.z, gt.z); x.w = gated(x.w, gt.w);
+    }
+    if (P.out_bf16) {
+        const __nv_bfloat162 b0 = __floats2bfloat162_rn(x.x, x.y), b1 = __floats2bfloat162_rn(x.z, x.w);
+        reinterpret_cast<uint2 *>(P.out)[i] = make_uint2(*reinterpret_cast<const uint32_t *>(&b0), *reinterpret_cast<const uint32_t *>(&b1));
+    } else {
+        reinterpret_cast<float4 *>(P.out)[i] = x;
+    }
 }
 
-/* fp16 staging of the rows a chunk can see; grows on demand, never inside a graph capture */
-__half *g_stage = nullptr;
-size_t g_stage_halves = 0;
-bool stage_reserve(size_t halves) {
-    if (halves <= g_stage_halves) return true;
-    if (g_q4.capturing) return q4i_fail(Q4E_SCRATCH, "kv_prefill: staging buffer too small inside a capture");
+/* ---- host side: workspace, launches */
+/* operand images of the rows a chunk can see, and the parts of split ranges; grows on demand, never inside a capture */
+uint8_t *g_stage = nullptr;
+size_t g_stage_bytes = 0;
+bool stage_reserve(size_t bytes) {
+    if (bytes <= g_stage_bytes) return true;
+    if (g_q4.capturing) return false;
     if (!q4i_check(cudaStreamSynchronize(g_q4.stream), "prefill staging sync")) return false;
     if (g_stage) cudaFree(g_stage);
     g_stage = nullptr;
-    g_stage_halves = 0;
-    const size_t want = halves + halves / 4;
-    if (!q4i_check(cudaMalloc(&g_stage, want * sizeof(__half)), "prefill staging alloc")) return false;
-    g_stage_halves = want;
+    g_stage_bytes = 0;
+    const size_t want = bytes + bytes / 4;
+    if (!q4i_check(cudaMalloc(&g_stage, want), "prefill staging alloc")) return false;
+    g_stage_bytes = want;
     return true;
+}
+
+template <typename K, typename... A>
+bool pf_start(K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = g_q4.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prefill launch");
+}
+template <int HD, int NQ, int KP>
+bool attend(const PrefillParams &p, dim3 grid) {
+    static bool attr = false;
+    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
+                            "prefill smem attribute"))
+        return false;
+    attr = true;
+    return pf_start(q4_prefill_k<HD, NQ, KP>, grid, NQ * 128u + 64u, PF_SMEM, p);
+}
+template <int LAY, int HD, int KP>
+bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
+    return pf_start(q4_pf_stage_k<LAY, HD, KP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
 }
 
 }  // namespace
 
-
 void q4i_prefill_release() {
     if (g_stage) cudaFree(g_stage);
     g_stage = nullptr;
-    g_stage_halves = 0;
+    g_stage_bytes = 0;
+}
+
+int q4i_prefill(const Q4PrefillArgs &a) {
+    const uint32_t gqa = a.n_head / a.n_kvh, hd = a.hd;
+    const uint64_t n64 = (uint64_t)a.kv_base + a.n_tok;
+    const uint32_t n = (uint32_t)(n64 < a.cache.max_kv ? n64 : a.cache.max_kv), tiles = (n + PF_BN - 1u) / PF_BN;
+    /* codes times scales do not fit fp16: the exact form keeps what the first image leaves over */
+    const uint32_t kp = a.layout == LAY_Q8R ? 2u : 1u;
+    const uint32_t tpc = PF_ROWS / gqa, groups = (a.n_tok + tpc - 1u) / tpc, sms = (uint32_t)g_q4.sm_count;
+    /* Two groups per block share every K/V tile and hide one another's softmax; one group per block while that does not
+     * fill the SMs, and then the positions are split too, at least two tiles a block. */
+    const uint32_t nq = hd == 128 && groups * a.n_kvh > sms ? 2u : 1u;
+    const uint32_t blocks = (groups + nq - 1u) / nq * a.n_kvh;
+    uint32_t split = nq == 1 && blocks * 2u <= sms ? sms / blocks : 1u;
+    if (split > (tiles + 1u) / 2u) split = (tiles + 1u) / 2u;
+    if (split > 16u) split = 16u;
+    const size_t k_bytes = (size_t)a.n_kvh * tiles * kp * (hd / 128u) * PF_CHUNK, v_bytes = (size_t)a.n_kvh * tiles * (hd / 128u) * PF_CHUNK;
+    const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
+    if (!stage_reserve(k_bytes + v_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0)))
+        return g_q4.capturing ? -1 : 0;
+
+    PrefillParams p;
+    memset(&p, 0, sizeof(p));
+    p.n_head = a.n_head; p.n_kvh = a.n_kvh; p.gqa = gqa; p.tpc = tpc;
+    p.q = a.q; p.q_bf16 = a.q_bf16; p.gate = a.gate; p.out = a.out; p.out_bf16 = a.out_bf16;
+    p.n_tok = a.n_tok; p.kv_base = a.kv_base; p.max_kv = a.cache.max_kv;
+    p.scale_log2e = a.scale * 1.4426950408889634f;
+    uint8_t *kimg = g_stage, *vimg = g_stage + k_bytes;
+    p.kimg = kimg; p.vimg = vimg; p.img_tiles = tiles;
+    p.n_split = split;
+    p.part = reinterpret_cast<float *>(g_stage + k_bytes + v_bytes);
+    p.part_ml = reinterpret_cast<float2 *>(g_stage + k_bytes + v_bytes + part_bytes);
+    p.err = g_q4.err_d;
+
+    bool ok;
+    if (a.layout == LAY_Q8P) ok = stage<LAY_Q8P, 128, 1>(a, n, tiles, kimg, vimg);
+    else if (a.layout == LAY_Q8R) ok = hd == 128 ? stage<LAY_Q8R, 128, 2>(a, n, tiles, kimg, vimg) : stage<LAY_Q8R, 256, 2>(a, n, tiles, kimg, vimg);
+    else if (a.layout == LAY_F16) ok = hd == 128 ? stage<LAY_F16, 128, 1>(a, n, tiles, kimg, vimg) : stage<LAY_F16, 256, 1>(a, n, tiles, kimg, vimg);
+    else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, kimg, vimg) : stage<LAY_F32, 256, 1>(a, n, tiles, kimg, vimg);
+    if (!ok) return 0;
+    const dim3 grid((groups + nq - 1u) / nq, a.n_kvh, split);
+    if (hd == 256) ok = kp == 2 ? attend<256, 1, 2>(p, grid) : attend<256, 1, 1>(p, grid);
+    else if (nq == 2) ok = kp == 2 ? attend<128, 2, 2>(p, grid) : attend<128, 2, 1>(p, grid);
+    else ok = kp == 2 ? attend<128, 1, 2>(p, grid) : attend<128, 1, 1>(p, grid);
+    if (ok && split > 1) {
+        const uint64_t total4 = (uint64_t)rows * hd / 4u;
+        ok = pf_start(q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4);
+    }
+    return ok ? 1 : 0;
 }
 
 extern "C" bool q4_gpu_kv_prefill(const q4_gpu_kv *kv, uint32_t layer, const void *q_bf16, const float *gate,
                                   void *out_bf16, uint32_t n_head, uint32_t n_tok, uint32_t kv_base, float scale) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_prefill: library not initialised");
     Q4_REQUIRE(kv && q_bf16 && out_bf16 && n_head && n_tok && layer < kv->n_layers, "kv_prefill: bad argument");
-    Q4_REQUIRE(kv->kind == Q4K_Q8 && kv->hd == PF_HD, "kv_prefill: tensor-core path needs a q8_0 store with hd 128");
+    Q4_REQUIRE(kv->kind == Q4K_Q8 && kv->hd == 128, "kv_prefill: tensor-core path needs a q8_0 store with hd 128");
     Q4_REQUIRE(n_head % kv->n_kvh == 0 && n_head / kv->n_kvh <= 16, "kv_prefill: n_head/n_kvh must be 1..16");
     Q4_REQUIRE(scale > 0.f, "kv_prefill: scale must be positive");
     Q4_REQUIRE((uint64_t)kv_base + 1 <= kv->max_kv, "kv_prefill: kv_base beyond max_kv");
-    static bool attr = false;
-    if (!attr) {
-        if (!q4i_check(cudaFuncSetAttribute(q4_prefill_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
-                       "prefill smem attribute"))
-            return false;
-        attr = true;
-    }
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) return q4i_fail(Q4E_CUDA, "kv_prefill: cuTensorMapEncodeTiled is not available from this driver");
-
-    /* rows the chunk can see, staged as fp16: K [kvh][n][128], V^T [kvh][128][n_pad] */
-    const uint64_t n64 = (uint64_t)kv_base + n_tok;
-    const uint32_t n = (uint32_t)(n64 < kv->max_kv ? n64 : kv->max_kv);
-    const uint32_t n_pad = (n + PF_BN - 1u) / PF_BN * PF_BN;
-    const size_t k_halves = (size_t)kv->n_kvh * n * PF_HD, v_halves = (size_t)kv->n_kvh * PF_HD * n_pad;
-    const size_t k_room = (k_halves + 63) & ~(size_t)63;    /* keeps V^T 128-byte aligned */
-    if (!stage_reserve(k_room + v_halves)) return false;
-    __half *kf = g_stage, *vt = g_stage + k_room;
-    q4_pf_stage_k<<<dim3(n_pad / PF_BN, kv->n_kvh), 256, 0, g_q4.stream>>>(kv->view, layer, n, n_pad, kf, vt);
-    if (!q4i_check(cudaGetLastError(), "prefill staging launch")) return false;
-
-    CUtensorMap map_k, map_v;
-    {
-        const cuuint64_t dims[3] = {PF_HD, n, kv->n_kvh};
-        const cuuint64_t strides[2] = {PF_HD * sizeof(__half), (cuuint64_t)n * PF_HD * sizeof(__half)};
-        const cuuint32_t box[3] = {64, PF_BN, 1}, estr[3] = {1, 1, 1};
-        if (enc(&map_k, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, kf, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return q4i_fail(Q4E_CUDA, "kv_prefill: tensor map (K) rejected");
-    }
-    {
-        const cuuint64_t dims[3] = {n, PF_HD, kv->n_kvh};
-        const cuuint64_t strides[2] = {(cuuint64_t)n_pad * sizeof(__half), (cuuint64_t)PF_HD * n_pad * sizeof(__half)};
-        const cuuint32_t box[3] = {PF_BN, PF_HD, 1}, estr[3] = {1, 1, 1};
-        if (enc(&map_v, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, vt, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return q4i_fail(Q4E_CUDA, "kv_prefill: tensor map (V) rejected");
-    }
-
-    PrefillParams p;
-    memset(&p, 0, sizeof(p));
-    p.n_head = n_head;
-    p.n_kvh = kv->n_kvh;
-    p.gqa = n_head / kv->n_kvh;
-    p.tpc = PF_ROWS / p.gqa;
-    p.q = (const __nv_bfloat16 *)q_bf16;
-    p.gate = gate;
-    p.out = (__nv_bfloat16 *)out_bf16;
-    p.n_tok = n_tok;
-    p.kv_base = kv_base;
-    p.max_kv = kv->max_kv;
-    p.scale_log2e = scale * 1.4426950408889634f;
-    p.err = g_q4.err_d;
-    dim3 grid((n_tok + p.tpc - 1) / p.tpc, kv->n_kvh);
-    q4_prefill_k<<<grid, PF_THREADS, PF_SMEM, g_q4.stream>>>(p, map_k, map_v);
-    return q4i_check(cudaGetLastError(), "prefill launch");
+    Q4PrefillArgs a;
+    memset(&a, 0, sizeof(a));
+    a.cache = kv->view;
+    a.layout = LAY_Q8P;
+    a.layer = layer;
+    a.n_head = n_head; a.n_kvh = kv->n_kvh; a.hd = kv->hd;
+    a.q = q_bf16; a.q_bf16 = 1; a.gate = gate; a.out = out_bf16; a.out_bf16 = 1;
+    a.n_tok = n_tok; a.kv_base = kv_base; a.scale = scale;
+    const int r = q4i_prefill(a);
+    return r < 0 ? q4i_fail(Q4E_SCRATCH, "kv_prefill: staging buffer too small inside a capture") : r == 1;
 }

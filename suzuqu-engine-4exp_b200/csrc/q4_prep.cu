@@ -2,8 +2,15 @@
  * Q / K preparation ahead of the append and the attention: per-head RMSNorm (optional weight),
  * interleaved-pair RoPE on the first n_rot dims, and for Q the split of the packed [q | gate]
  * projection.  Restates qsa_q_prep_k / qsa_k_prep_k (src/q4_rocm.cu:6229-6294) and their launchers
- * (:6296-6343): one block per (head, token), position = pos0 + t or the device position word + t.
+ * (:6296-6343); position = pos0 + t or the device position word + t.
+ *
+ * Head sizes 64, 128 and 256: a block takes the heads of one token, one warp per head.  The rotation of a pair depends
+ * on the token alone, so its power, sine and cosine are taken once per token (one block per (head, token) took them
+ * n_head times: 72 us for 2048 tokens x 24 heads of 256, which read and write 200 MB).  Every sum keeps the order of
+ * that form, so the cache bytes quantised from the rows stay the same.  Other head sizes: one block per (head, token).
  */
+#include <string.h>
+
 #include "q4_internal.h"
 
 namespace {
@@ -59,6 +66,140 @@ __global__ void q4_k_prep_k(float *k, const float *wn, uint32_t hd, uint32_t n_r
     norm_rope(kh, kh, wn, hd, n_rot, pos, base, eps, sh);
 }
 
+
+/* ---- one warp per head */
+constexpr uint32_t PREP_WARPS = 8;
+__device__ __forceinline__ void prep_pdl_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+/* cos and sin of the token's rotation of pair p, by thread p of the block; np <= 128 */
+__device__ __forceinline__ void rope_table(float2 *cs, uint32_t np, int32_t pos, float base) {
+    const uint32_t p = threadIdx.x;
+    if (p < np) {
+        const float freq = powf(base, -(float)p / (float)np);
+        const float ang = (float)pos * freq;
+        cs[p] = make_float2(cosf(ang), sinf(ang));
+    }
+}
+/* a row as the warp holds it: register k of lane l = elements 64 k + 2 l, + 1 */
+template <int HD>
+__device__ __forceinline__ void row_load(const float *src, float2 (&v)[HD / 64]) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int k = 0; k < HD / 64; k++) v[k] = reinterpret_cast<const float2 *>(src)[32 * k + lane];
+}
+/* RMSNorm and rotation in place.  Sum of squares as 128 threads of a block would take it: thread i adds elements i and
+ * i + 128, a butterfly over each 32 threads, then the four totals in order (element 2 l + e of a register is thread
+ * 2 l + e: the butterfly's last step is the addition inside the lane). */
+template <int HD>
+__device__ __forceinline__ void row_norm_rope(float2 (&v)[HD / 64], const float *wn, const float2 *cs, uint32_t np, float eps) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float tot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < (HD / 64 < 2 ? HD / 64 : 2); k++) {
+        float a = __fmul_rn(v[k].x, v[k].x), b = __fmul_rn(v[k].y, v[k].y);
+        if (HD == 256) { a = __fmaf_rn(v[k + HD / 128].x, v[k + HD / 128].x, a); b = __fmaf_rn(v[k + HD / 128].y, v[k + HD / 128].y, b); }
+#pragma unroll
+        for (int o = 8; o; o >>= 1) {
+            a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, o));
+            b = __fadd_rn(b, __shfl_xor_sync(0xffffffffu, b, o));
+        }
+        a = __fadd_rn(a, b);
+        tot[2 * k] = __shfl_sync(0xffffffffu, a, 0);
+        tot[2 * k + 1] = __shfl_sync(0xffffffffu, a, 16);
+    }
+    const float ss = __fadd_rn(__fadd_rn(__fadd_rn(tot[0], tot[1]), tot[2]), tot[3]);
+    const float scale = 1.0f / sqrtf(ss / (float)HD + eps);
+#pragma unroll
+    for (int k = 0; k < HD / 64; k++) {
+        const uint32_t p = 32u * k + lane;
+        float x0 = v[k].x * scale * (wn ? wn[2 * p] : 1.f);
+        float x1 = v[k].y * scale * (wn ? wn[2 * p + 1] : 1.f);
+        if (p < np) {
+            const float c = cs[p].x, si = cs[p].y;
+            const float y0 = x0 * c - x1 * si, y1 = x0 * si + x1 * c;
+            x0 = y0;
+            x1 = y1;
+        }
+        v[k] = make_float2(x0, x1);
+    }
+}
+template <int HD>
+__device__ __forceinline__ void row_store(float *dst, const float2 (&v)[HD / 64]) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int k = 0; k < HD / 64; k++) reinterpret_cast<float2 *>(dst)[32 * k + lane] = v[k];
+}
+/* SPLIT: rows are [q | gate] pairs, q goes to `q` and the gate to `g`; else rows of `q` in place.  blockIdx.x: a group of
+ * `per` heads, blockIdx.y: token. */
+template <int HD, bool SPLIT>
+__global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *src, const float *wn, float *q, float *g, uint32_t n_rot,
+                                                                  int32_t pos0, float base, float eps, uint32_t n_head, uint32_t per,
+                                                                  const int32_t *pp) {
+    __shared__ float2 cs[128];
+    const uint32_t t = blockIdx.y, warp = threadIdx.x >> 5, h0 = blockIdx.x * per, h1 = min(h0 + per, n_head);
+    prep_pdl_sync();
+    rope_table(cs, n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base);
+    __syncthreads();
+    for (uint32_t h = h0 + warp; h < h1; h += PREP_WARPS) {
+        const size_t row = (size_t)t * n_head + h;
+        float2 v[HD / 64];
+        row_load<HD>(SPLIT ? src + row * 2u * HD : q + row * HD, v);
+        if (SPLIT) {
+            float2 w[HD / 64];
+            row_load<HD>(src + row * 2u * HD + HD, w);
+            row_store<HD>(g + row * HD, w);
+        }
+        row_norm_rope<HD>(v, wn, cs, n_rot / 2u, eps);
+        row_store<HD>(q + row * HD, v);
+    }
+}
+
+template <typename K, typename... A>
+bool prep_start(K kernel, dim3 grid, uint32_t threads, A... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = g_q4.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prep launch");
+}
+/* false in `done` where the head size or an address is not the warp form's */
+template <bool SPLIT>
+bool prep_rows(const float *src, const float *wn, float *q, float *g, uint32_t n_head, uint32_t hd, uint32_t n_rot, int32_t pos0, float base,
+               float eps, uint32_t n_tok, const int32_t *pp, bool &done) {
+    done = (hd == 64 || hd == 128 || hd == 256) && (((uintptr_t)src | (uintptr_t)q | (uintptr_t)g) & 7u) == 0;
+    if (!done) return false;
+    /* one token: its heads over several SMs, eight to a block; many tokens: one block each */
+    const uint32_t per = n_tok < (uint32_t)g_q4.sm_count ? PREP_WARPS : n_head;
+    const dim3 grid((n_head + per - 1u) / per, n_tok);
+    if (hd == 64) return prep_start(q4_prep_rows_k<64, SPLIT>, grid, PREP_WARPS * 32u, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp);
+    if (hd == 128) return prep_start(q4_prep_rows_k<128, SPLIT>, grid, PREP_WARPS * 32u, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp);
+    return prep_start(q4_prep_rows_k<256, SPLIT>, grid, PREP_WARPS * 32u, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp);
+}
+bool q_prep(const float *qg, const float *wn, float *q, float *g, uint32_t n_head, uint32_t hd, uint32_t n_rot, int32_t pos0, float base,
+            float eps, uint32_t n_tok, const int32_t *pp) {
+    bool done;
+    const bool ok = prep_rows<true>(qg, wn, q, g, n_head, hd, n_rot, pos0, base, eps, n_tok, pp, done);
+    if (done) return ok;
+    q4_q_prep_k<<<dim3(n_head, n_tok), 128, 0, g_q4.stream>>>(qg, wn, q, g, hd, n_rot, pos0, base, eps, n_head, pp);
+    return q4i_check(cudaGetLastError(), "q_prep launch");
+}
+bool k_prep(float *k, const float *wn, uint32_t n_kvh, uint32_t hd, uint32_t n_rot, int32_t pos0, float base, float eps, uint32_t n_tok,
+            const int32_t *pp) {
+    bool done;
+    const bool ok = prep_rows<false>(nullptr, wn, k, nullptr, n_kvh, hd, n_rot, pos0, base, eps, n_tok, pp, done);
+    if (done) return ok;
+    q4_k_prep_k<<<dim3(n_kvh, n_tok), 128, 0, g_q4.stream>>>(k, wn, hd, n_rot, pos0, base, eps, n_kvh, pp);
+    return q4i_check(cudaGetLastError(), "k_prep launch");
+}
+
 }  // namespace
 
 extern "C" bool q4_hip_qsa_q_prep_n(const float *d_qg, const float *d_wn, float *d_q, float *d_g, uint32_t n_head,
@@ -66,17 +207,13 @@ extern "C" bool q4_hip_qsa_q_prep_n(const float *d_qg, const float *d_wn, float 
                                     uint32_t n_tok) {
     if (!g_q4.ok || !d_qg || !d_q || !d_g || n_head == 0 || n_tok == 0 || hd == 0 || (hd & 1) || n_rot > hd)
         return false;
-    q4_q_prep_k<<<dim3(n_head, n_tok), 128, 0, g_q4.stream>>>(d_qg, d_wn, d_q, d_g, hd, n_rot, pos0, base, eps,
-                                                             n_head, nullptr);
-    return q4i_check(cudaGetLastError(), "q_prep launch");
+    return q_prep(d_qg, d_wn, d_q, d_g, n_head, hd, n_rot, pos0, base, eps, n_tok, nullptr);
 }
 extern "C" bool q4_hip_qsa_q_prep_d(const float *qg, const float *wn, float *q, float *g, uint32_t n_head,
                                     uint32_t hd, uint32_t n_rot, float base, float eps) {
     if (!g_q4.ok || !g_q4.pos_d || !qg || !q || !g || n_head == 0 || hd == 0 || (hd & 1) || n_rot > hd)
         return false;
-    q4_q_prep_k<<<dim3(n_head, 1), 128, 0, g_q4.stream>>>(qg, wn, q, g, hd, n_rot, 0, base, eps, n_head,
-                                                         g_q4.pos_d);
-    return q4i_check(cudaGetLastError(), "q_prep_d launch");
+    return q_prep(qg, wn, q, g, n_head, hd, n_rot, 0, base, eps, 1, g_q4.pos_d);
 }
 extern "C" bool q4_hip_qsa_q_prep(const float *d_qg, const float *d_wn, float *d_q, float *d_g, uint32_t n_head,
                                   uint32_t hd, uint32_t n_rot, int32_t pos, float base, float eps) {
@@ -85,14 +222,12 @@ extern "C" bool q4_hip_qsa_q_prep(const float *d_qg, const float *d_wn, float *d
 extern "C" bool q4_hip_qsa_k_prep_n(float *d_k, const float *d_wn, uint32_t n_kvh, uint32_t hd, uint32_t n_rot,
                                     int32_t pos0, float base, float eps, uint32_t n_tok) {
     if (!g_q4.ok || !d_k || n_kvh == 0 || n_tok == 0 || hd == 0 || (hd & 1) || n_rot > hd) return false;
-    q4_k_prep_k<<<dim3(n_kvh, n_tok), 128, 0, g_q4.stream>>>(d_k, d_wn, hd, n_rot, pos0, base, eps, n_kvh, nullptr);
-    return q4i_check(cudaGetLastError(), "k_prep launch");
+    return k_prep(d_k, d_wn, n_kvh, hd, n_rot, pos0, base, eps, n_tok, nullptr);
 }
 extern "C" bool q4_hip_qsa_k_prep_d(float *k, const float *wn, uint32_t n_kvh, uint32_t hd, uint32_t n_rot,
                                     float base, float eps) {
     if (!g_q4.ok || !g_q4.pos_d || !k || n_kvh == 0 || hd == 0 || (hd & 1) || n_rot > hd) return false;
-    q4_k_prep_k<<<dim3(n_kvh, 1), 128, 0, g_q4.stream>>>(k, wn, hd, n_rot, 0, base, eps, n_kvh, g_q4.pos_d);
-    return q4i_check(cudaGetLastError(), "k_prep_d launch");
+    return k_prep(k, wn, n_kvh, hd, n_rot, 0, base, eps, 1, g_q4.pos_d);
 }
 extern "C" bool q4_hip_qsa_k_prep(float *d_k, const float *d_wn, uint32_t n_kvh, uint32_t hd, uint32_t n_rot,
                                   int32_t pos, float base, float eps) {
@@ -118,6 +253,7 @@ struct PrepAppendParams {
     uint32_t *err;
 };
 
+/* head sizes 32 and 64: a block per (row, K or V) */
 __global__ void q4_prep_append_k(const PrepAppendParams P) {
     __shared__ float sh[4];
     __shared__ __align__(16) float row_s[256];
@@ -157,6 +293,54 @@ __global__ void q4_prep_append_k(const PrepAppendParams P) {
     }
 }
 
+/* Head sizes 128 and 256: a block per token, a warp per row (K heads, then V heads), the rotation once per token.  The row
+ * passes through the warp's part of shared memory to be quantised eight lanes per 32 values, as everywhere. */
+template <int HD>
+__global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_append_rows_k(const PrepAppendParams P) {
+    __shared__ float2 cs[128];
+    __shared__ __align__(16) float row_s[PREP_WARPS][HD];
+    const uint32_t t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    prep_pdl_sync();
+    const int32_t pos = (P.pos ? *P.pos : P.pos0) + (int32_t)t;
+    rope_table(cs, P.n_rot / 2u, pos, P.base);
+    __syncthreads();
+    if (pos < 0 || (uint32_t)pos >= P.C.max_kv) {
+        if (threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
+        return;
+    }
+    for (uint32_t r = warp; r < 2u * P.n_kvh; r += PREP_WARPS) {
+        const bool which = r >= P.n_kvh;
+        const uint32_t kh = which ? r - P.n_kvh : r;
+        float2 v[HD / 64];
+        row_load<HD>((which ? P.v : P.k) + ((size_t)t * P.n_kvh + kh) * HD, v);
+        if (!which) row_norm_rope<HD>(v, P.wn, cs, P.n_rot / 2u, P.eps);
+        __syncwarp();
+        row_store<HD>(row_s[warp], v);
+        __syncwarp();
+        uint8_t *row = const_cast<uint8_t *>(which ? P.C.v : P.C.k) + (uint64_t)P.layer * P.C.layer_stride +
+                       (uint64_t)kh * P.C.kvh_stride + (uint64_t)pos * P.C.tok_stride;
+#pragma unroll
+        for (uint32_t i = lane; i < HD / 4u; i += 32u) {
+            const float4 x = *reinterpret_cast<const float4 *>(row_s[warp] + i * 4u);
+            float d, id;
+            if (P.layout == LAY_Q8P) {
+                q4d_block_scale(x, d, id);
+                *reinterpret_cast<uint32_t *>(row + i * 4u) = q4d_quant4(x, id);
+                if ((i & 7u) == 0) {
+                    uint8_t *srow = const_cast<uint8_t *>(P.C.s) + (uint64_t)P.layer * P.C.s_layer_stride +
+                                    (uint64_t)kh * P.C.s_kvh_stride + (uint64_t)pos * P.C.s_tok_stride;
+                    reinterpret_cast<__half *>(srow)[(which ? HD / 32u : 0u) + (i >> 3)] = __float2half_rn(d);
+                }
+            } else if (P.layout == LAY_F16) {
+                const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
+                *reinterpret_cast<uint2 *>(row + i * 8u) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+            } else {
+                *reinterpret_cast<float4 *>(row + i * 16u) = x;
+            }
+        }
+    }
+}
+
 bool prep_append(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, const float *wn, uint32_t n_rot,
                  float base, float eps, const int32_t *pos_dev, int32_t pos0, uint32_t n_tok) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_prep_append: library not initialised");
@@ -167,6 +351,9 @@ bool prep_append(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, 
     p.layout = kv->kind == Q4K_Q8 ? LAY_Q8P : kv->kind == Q4K_F16 ? LAY_F16 : LAY_F32;
     p.layer = layer; p.n_kvh = kv->n_kvh; p.hd = kv->hd; p.n_rot = n_rot; p.n_tok = n_tok;
     p.k = k; p.v = v; p.wn = wn; p.pos = pos_dev; p.pos0 = pos0; p.base = base; p.eps = eps; p.err = g_q4.err_d;
+    if ((kv->hd == 128 || kv->hd == 256) && (((uintptr_t)k | (uintptr_t)v) & 7u) == 0)
+        return kv->hd == 128 ? prep_start(q4_prep_append_rows_k<128>, dim3(n_tok), PREP_WARPS * 32u, p)
+                             : prep_start(q4_prep_append_rows_k<256>, dim3(n_tok), PREP_WARPS * 32u, p);
     q4_prep_append_k<<<dim3(kv->n_kvh, n_tok, 2), 128, 0, g_q4.stream>>>(p);
     return q4i_check(cudaGetLastError(), "kv_prep_append launch");
 }

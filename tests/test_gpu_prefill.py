@@ -62,6 +62,14 @@ def test_prefill_gqa_shapes(oracle, n_head, n_kvh):
     run_case(oracle, 40, 77, n_head, n_kvh, 2000 + n_head, gate=(n_head % 2 == 0))
 
 
+@pytest.mark.parametrize("n_head,n_kvh,n_tok,kv_base", [(64, 4, 297, 0), (64, 4, 313, 700), (9, 3, 1300, 5)])
+def test_prefill_two_query_groups_per_block(oracle, n_head, n_kvh, n_tok, kv_base):
+    """enough query groups to fill the SMs: two per block, the last of them partly or wholly padding"""
+    lib()
+    run_case(oracle, n_tok, kv_base, n_head, n_kvh, 3000 + n_tok)
+    assert q4gpu.load().q4_gpu_last_error() == 0
+
+
 def test_prefill_chunk_over_existing_cache(oracle):
     """the chunked-prefill shape scaled down: 512 new tokens over a 1024-token cache, RoPE'd inputs"""
     lib()
@@ -135,3 +143,30 @@ def test_prefill_large_magnitude_queries(oracle, mode):
     ref = oracle.attn(oracle.bf16_to_f32(qb), kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, ctx, scale, 2, threads=8)
     check(host(dout.float()).reshape(n_tok, n_head, hd), ref, "prefill, %s" % mode, out_scale=max(1.0, float(np.abs(ref).max())))
     st.close()
+
+
+@pytest.mark.parametrize("kind", [2, 1, 0])
+@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base,max_kv", [
+    (24, 2, 256, 40, 0, 40), (24, 2, 256, 23, 1000, 1023), (4, 4, 256, 130, 127, 257), (16, 1, 256, 9, 640, 640),
+    (16, 2, 128, 300, 500, 800), (16, 2, 128, 8, 2000, 2008), (3, 1, 128, 129, 0, 129), (16, 2, 128, 100, 30, 90), (64, 4, 128, 301, 200, 501)])
+def test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, n_head, n_kvh, hd, n_tok, kv_base, max_kv):
+    """q4_hip_qsa_decode_n with a prompt's slice on caches in the reference layout: every kind at both head sizes, group
+    sizes that do not divide the 128-row tiles, tile edges, position ranges split over several blocks (few tokens
+    behind many rows) and rows that max_kv cuts off; the tolerance is the fp32 oracle's"""
+    from gpu_util import assert_close, dev_bytes
+    L = lib()
+    kvw = n_kvh * hd
+    seed = 7000 + n_tok + hd
+    rows = min(kv_base + n_tok, max_kv)
+    k = oracle.normal(seed, 0, rows * kvw).reshape(rows, kvw)
+    v = oracle.normal(seed, 1, rows * kvw).reshape(rows, kvw)
+    q = oracle.normal(seed, 2, n_tok * n_head * hd)
+    g = oracle.normal(seed, 3, n_tok * n_head * hd)
+    kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind)
+    out = torch.full((n_tok * n_head * hd,), float("nan"), device="cuda")
+    scale = float(1.0 / np.sqrt(hd))
+    assert L.q4_hip_qsa_decode_n(dev(q).data_ptr(), dev_bytes(kc).data_ptr(), dev_bytes(vc).data_ptr(), dev(g).data_ptr(), out.data_ptr(),
+                                 n_head, n_kvh, hd, n_tok, kv_base, max_kv, scale, kind)
+    ref = oracle.attn(q.reshape(n_tok, n_head, hd), kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, max_kv, scale, kind, threads=8)
+    assert_close(host(out).reshape(ref.shape), ref, "kind %d %d/%d/%d" % (kind, n_head, n_kvh, hd))
+    assert L.q4_gpu_last_error() == 0
