@@ -87,6 +87,7 @@ struct DecParams {
     uint32_t push_bytes;          /* > 0: the launch carries this much extra shared memory and merges by pushing */
     uint32_t push_async;          /* pushes complete an mbarrier of the receiving block (its last 16 bytes) instead of
                                    * meeting at a cluster barrier */
+    uint32_t direct;              /* host side: the cache is not aligned for asynchronous copies */
     uint32_t bulk_runs;           /* tiles of 16 consecutive positions come in by one bulk copy each (else by cp.async) */
 };
 
@@ -179,6 +180,16 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
     return v;
 }
+__device__ __forceinline__ float4 lds_f4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float2 lds_f2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                          uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -236,12 +247,21 @@ __device__ __forceinline__ float warp_sum_over_g(float v) {
     return v + __shfl_xor_sync(0xffffffffu, v, 16);
 }
 
+/* Reference q8_0 blocks come in pairs of 68 bytes, 17 aligned words: {scale 0, codes 0 1}, seven words of codes 2 .. 29,
+ * {codes 30 31, scale 1}, eight words of block 1's codes.  Word j of block b (even: the seven words, then codes 0 1 30 31
+ * put together) holds in byte i the dim: */
+__device__ __forceinline__ int q8r_dim(int b, int j, int i) {
+    if (b & 1) return 32 * b + 4 * j + i;
+    return j < 7 ? 32 * b + 2 + 4 * j + i : 32 * b + (i < 2 ? i : 28 + i);
+}
 /* Which head dimension the accumulator pair (c0,c1) / (c2,c3) of output tile mt holds for lane
  * group g.  The register-direct q8 paths interleave so that each tile stays inside one 32-wide scale
  * block; the staged path (fragments through ldmatrix) and the fp16 / fp32 rows use plain 16-dim tiles. */
-template <int LAY, bool STAGED>
+template <int LAY, bool STAGED, bool STAGED2>
 __device__ __forceinline__ int out_dim(int mt, int g, int hi) {
-    if ((LAY == LAY_Q8P || LAY == LAY_Q8R) && !STAGED) return 32 * (mt >> 1) + 4 * g + 2 * (mt & 1) + hi;
+    if (STAGED2 && LAY == LAY_F16) return 16 * mt + g + 8 * hi;
+    if (STAGED2 && LAY == LAY_Q8R) return q8r_dim(mt >> 1, g, 2 * (mt & 1) + hi);
+    if ((LAY == LAY_Q8P || LAY == LAY_Q8R) && !STAGED && !STAGED2) return 32 * (mt >> 1) + 4 * g + 2 * (mt & 1) + hi;
     return 16 * mt + 2 * g + hi;
 }
 /* Which 4 head dimensions lane t feeds to k-step ks of the QK product (same map for Q and K). */
@@ -318,8 +338,8 @@ __device__ __noinline__ void merge_records(const float *recs, uint32_t count, bo
     constexpr int REC = HD + 4;
     float *s_w = scratch, *s_l = scratch + DEC_GROUP * 16, *s_M = scratch + 2 * DEC_GROUP * 16, *s_L = s_M + 16;
     const uint32_t gqa = mo.gqa;
-    if (!global && count == DEC_WARPS && dst_rec) {
-        /* The block's own four warp records, in shared memory: every thread recomputes the four weights
+    if (!global && count <= DEC_WARPS && dst_rec) {
+        /* The block's own warp records (at most four), in shared memory: every thread recomputes the four weights
          * of its head (no shared weights, no barriers in between) and writes its 4 dims of the block
          * record.  This runs once in every block of every launch. */
         for (uint32_t i = threadIdx.x; i < gqa * (HD / 4); i += DEC_THREADS) {
@@ -328,7 +348,7 @@ __device__ __noinline__ void merge_records(const float *recs, uint32_t count, bo
             float4 x[DEC_WARPS];
 #pragma unroll
             for (int k = 0; k < DEC_WARPS; k++) {
-                const float *r = recs + ((size_t)k * HEADS + h) * REC;
+                const float *r = recs + ((size_t)min((uint32_t)k, count - 1u) * HEADS + h) * REC;
                 ml[k] = *reinterpret_cast<const float2 *>(r + HD);
                 x[k] = *reinterpret_cast<const float4 *>(r + d);
             }
@@ -340,7 +360,7 @@ __device__ __noinline__ void merge_records(const float *recs, uint32_t count, bo
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int k = 0; k < DEC_WARPS; k++) {
-                const float w = ex2(ml[k].x - Mu);
+                const float w = (uint32_t)k < count ? ex2(ml[k].x - Mu) : 0.f;
                 L = fmaf(w, ml[k].y, L);
                 A.x = fmaf(w, x[k].x, A.x); A.y = fmaf(w, x[k].y, A.y);
                 A.z = fmaf(w, x[k].z, A.z); A.w = fmaf(w, x[k].w, A.w);
@@ -835,23 +855,49 @@ constexpr int RING_STAGE_BYTES = 16 * RING_ROW + 32;        /* rows, mask word *
 constexpr int RING_BAR_BYTES = DEC_WARPS * RING_STAGES * 8; /* one mbarrier per stage, behind the rings of all warps */
 constexpr uint32_t RING_SPIN_LIMIT = 1u << 22;             /* probes of a stage's mbarrier before the block gives up */
 
-template <int LAY, int HD, int NHT>
+/* Tiles of the other layouts at hd 128 and 256 (STAGED2): 16 positions, the K rows and then the V rows as they lie in the
+ * cache, or the records of the native q8_0 store, at a pitch that keeps the fragment reads free of bank conflicts:
+ * fp16 and records: the eight 16-byte pieces of an 8x8 ldmatrix block in eight different bank groups; fp32: 16-byte reads
+ * of 2 K rows x 4 lanes, 8-byte reads of 2 V rows x 8 lanes; reference q8_0 blocks: 4-byte reads of 8 rows x 4 lanes. */
+template <int LAY, int HD>
+struct DecTile {
+    static constexpr bool REC = LAY == LAY_Q8P;
+    static constexpr int ROW = LAY == LAY_Q8P ? (2 * HD + HD / 8 + 15) / 16 * 16 : LAY == LAY_Q8R ? HD / 32 * 34 : HD * (LAY == LAY_F16 ? 2 : 4);
+    static constexpr int CH = LAY == LAY_Q8R && HD == 128 ? 8 : 16;              /* bytes per asynchronous copy: 136-byte rows are 8-byte aligned */
+    static constexpr int CPR = ROW / CH;                                         /* copies per row */
+    static constexpr int K_PITCH = LAY == LAY_Q8R ? (HD == 128 ? 144 : 272) : LAY == LAY_F32 ? ROW + 64 : ROW + 16;
+    static constexpr int V_PITCH = REC ? 0 : LAY == LAY_F32 ? ROW + 32 : K_PITCH;
+    static constexpr int V_OFF = REC ? HD : 16 * K_PITCH;
+    static constexpr int BYTES = 16 * (K_PITCH + V_PITCH);
+};
+constexpr int dec_stages(int groups_bytes) {   /* 3 blocks per SM with 2 to 4 stages, else 2 with 2, else 1 */
+    return groups_bytes * 4 <= 73728 ? 4 : groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 110592 ? 2 : groups_bytes * 2 <= 204800 ? 2 : 1;
+}
+/* DIRECT: caches whose base is not aligned for the asynchronous copies (reference ABI only) load fragments into registers */
+template <int LAY, int HD, int NHT, bool DIRECT>
 struct DecCfg {
     static constexpr bool STAGED = (LAY == LAY_Q8P && HD == 128);
+    static constexpr bool STAGED2 = !STAGED && !DIRECT && HD >= 128;
+    /* STAGED2: a warp takes 8 query heads; with more, two warps share every tile */
+    static constexpr int NW = STAGED2 ? 1 : NHT, WPT = STAGED2 ? NHT : 1, NPG = DEC_WARPS / WPT;
     static constexpr int HEADS = 8 * NHT;
     static constexpr int REC = HD + 4;          /* acc[HD], m, l, 2 pad: 16-byte aligned records */
-    static constexpr size_t EPI_BYTES = (size_t)DEC_WARPS * HEADS * REC * sizeof(float);
-    static constexpr size_t RING_BYTES = STAGED ? (size_t)DEC_WARPS * RING_STAGES * RING_STAGE_BYTES + RING_BAR_BYTES : 0;
+    static constexpr size_t EPI_BYTES = (size_t)NPG * HEADS * REC * sizeof(float);
+    static constexpr int TILE2 = STAGED2 ? DecTile<LAY, (HD < 128 ? 128 : HD)>::BYTES : 16;
+    static constexpr int ST2 = dec_stages(NPG * TILE2);
+    static constexpr size_t RING_BYTES = STAGED ? (size_t)DEC_WARPS * RING_STAGES * RING_STAGE_BYTES + RING_BAR_BYTES
+                                       : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 : 0;
     static constexpr size_t REC_BYTES = (size_t)HEADS * REC * sizeof(float);   /* the block's merged record */
     static constexpr size_t TAIL_BYTES = EPI_BYTES + REC_BYTES + MERGE_SCRATCH_FLOATS * sizeof(float);   /* after the loop */
-    static constexpr size_t SMEM = TAIL_BYTES > RING_BYTES ? TAIL_BYTES : RING_BYTES;
-    static constexpr int MIN_BLOCKS = STAGED ? (NHT == 1 ? 3 : 2) : (HD * NHT <= 128 ? 3 : 1);
+    static constexpr size_t SMEM = ((TAIL_BYTES > RING_BYTES ? TAIL_BYTES : RING_BYTES) + 15) / 16 * 16;
+    static constexpr int MIN_BLOCKS = STAGED ? (NHT == 1 ? 3 : 2) : STAGED2 ? (SMEM <= 74752 ? 3 : SMEM <= 113664 ? 2 : 1) : (HD * NHT <= 128 ? 3 : 1);
 };
 
-template <int LAY, int HD, int NHT>
-__global__ void __launch_bounds__(DEC_THREADS, (DecCfg<LAY, HD, NHT>::MIN_BLOCKS))
+template <int LAY, int HD, int NHT, bool DIRECT>
+__global__ void __launch_bounds__(DEC_THREADS, (DecCfg<LAY, HD, NHT, DIRECT>::MIN_BLOCKS))
 q4_decode_k(const DecParams P) {
-    using Cfg = DecCfg<LAY, HD, NHT>;
+    using Cfg = DecCfg<LAY, HD, NHT, DIRECT>;
+    constexpr int NW = Cfg::NW;   /* groups of 8 query heads per warp */
     constexpr int NB = HD / 32;   /* q8_0 blocks per row */
     constexpr int KS = HD / 16;   /* k-steps of the QK product */
     constexpr int MT = HD / 16;   /* 16-dim output tiles of the PV product */
@@ -874,7 +920,7 @@ q4_decode_k(const DecParams P) {
         if (P.push_async) {
             /* the barrier that the peers' pushes complete: initialised before this block announces itself */
             if (threadIdx.x == 0) {
-                ring_bar_init((uint32_t)__cvta_generic_to_shared(smem_raw + DecCfg<LAY, HD, NHT>::SMEM + P.push_bytes - 16u));
+                ring_bar_init((uint32_t)__cvta_generic_to_shared(smem_raw + DecCfg<LAY, HD, NHT, DIRECT>::SMEM + P.push_bytes - 16u));
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             }
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -920,7 +966,7 @@ q4_decode_k(const DecParams P) {
     float4 ap_x = make_float4(0.f, 0.f, 0.f, 0.f);
     bool ap_which = false, ap_live = false;
     uint32_t ap_b = 0, ap_sub = 0;
-    if constexpr (Cfg::STAGED) {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
+    if constexpr (Cfg::STAGED || Cfg::STAGED2) {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
         if (P.new_k) {
             constexpr uint32_t QL = HD / 4;
             const uint32_t tid = threadIdx.x;
@@ -948,9 +994,9 @@ q4_decode_k(const DecParams P) {
     };
 
     /* ---- Q fragments (B operand of the QK product): head nt*8+g, dims qk_dim(ks, t)..+3 */
-    uint32_t qf[NHT][KS][2];
+    uint32_t qf[NW][KS][2];   /* unused, and dropped by the compiler, where tiles are staged */
 #pragma unroll
-    for (int nt = 0; nt < NHT; nt++) {
+    for (int nt = 0; nt < NW; nt++) {
         const uint32_t hg = nt * 8 + g;
         const bool live = hg < P.gqa;
         const size_t qoff = ((size_t)u * P.n_head + (size_t)kh * P.gqa + hg) * HD;
@@ -977,9 +1023,9 @@ q4_decode_k(const DecParams P) {
         }
     }
 
-    float m_run[NHT][2], l_run[NHT][2], acc[NHT][MT][4];
+    float m_run[NW][2], l_run[NW][2], acc[NW][MT][4];
 #pragma unroll
-    for (int nt = 0; nt < NHT; nt++) {
+    for (int nt = 0; nt < NW; nt++) {
         m_run[nt][0] = m_run[nt][1] = -CUDART_INF_F;
         l_run[nt][0] = l_run[nt][1] = 0.f;
 #pragma unroll
@@ -994,26 +1040,26 @@ q4_decode_k(const DecParams P) {
                        const uint32_t (&vw)[4][NBQ], const float (&ksc)[2][NBQ], const __half (&vsc)[4][NBQ],
                        const uint8_t *const (&krow)[2], const uint8_t *const (&vrow)[4]) {
         /* ---- S^T = K . Q^T (log2 domain: scale * log2(e) folded in) */
-        float sc[NHT][4];
+        float sc[NW][4];
 #pragma unroll
-        for (int nt = 0; nt < NHT; nt++) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
+        for (int nt = 0; nt < NW; nt++) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
         if constexpr (Q8) {
 #pragma unroll
             for (int b = 0; b < NB; b++) {
-                float cb[NHT][4];
+                float cb[NW][4];
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++) cb[nt][0] = cb[nt][1] = cb[nt][2] = cb[nt][3] = 0.f;
+                for (int nt = 0; nt < NW; nt++) cb[nt][0] = cb[nt][1] = cb[nt][2] = cb[nt][3] = 0.f;
 #pragma unroll
                 for (int jj = 0; jj < 2; jj++) {
                     uint32_t a0, a1, a2, a3;
                     cvt_i8x4(jj ? kw[0][b].y : kw[0][b].x, a0, a2);
                     cvt_i8x4(jj ? kw[1][b].y : kw[1][b].x, a1, a3);
 #pragma unroll
-                    for (int nt = 0; nt < NHT; nt++)
+                    for (int nt = 0; nt < NW; nt++)
                         mma16816(cb[nt], a0, a1, a2, a3, qf[nt][2 * b + jj][0], qf[nt][2 * b + jj][1]);
                 }
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++) {
+                for (int nt = 0; nt < NW; nt++) {
                     sc[nt][0] = fmaf(ksc[0][b], cb[nt][0], sc[nt][0]);
                     sc[nt][1] = fmaf(ksc[0][b], cb[nt][1], sc[nt][1]);
                     sc[nt][2] = fmaf(ksc[1][b], cb[nt][2], sc[nt][2]);
@@ -1040,19 +1086,19 @@ q4_decode_k(const DecParams P) {
                     a[r] = lo; a[2 + r] = hi;
                 }
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++)
+                for (int nt = 0; nt < NW; nt++)
                     mma16816(sc[nt], a[0], a[1], a[2], a[3], qf[nt][ks][0], qf[nt][ks][1]);
             }
 #pragma unroll
-            for (int nt = 0; nt < NHT; nt++)
+            for (int nt = 0; nt < NW; nt++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) sc[nt][e] *= P.scale_log2e;
         }
 
         /* ---- online softmax; lanes (g, t) hold positions g / g+8 for heads 2t, 2t+1 */
-        uint32_t pb0[NHT], pb1[NHT];
+        uint32_t pb0[NW], pb1[NW];
 #pragma unroll
-        for (int nt = 0; nt < NHT; nt++) {
+        for (int nt = 0; nt < NW; nt++) {
             if (pk[0] < 0) sc[nt][0] = sc[nt][1] = -CUDART_INF_F;
             if (pk[1] < 0) sc[nt][2] = sc[nt][3] = -CUDART_INF_F;
             const float mx0 = warp_max_over_g(fmaxf(sc[nt][0], sc[nt][2]));
@@ -1084,9 +1130,9 @@ q4_decode_k(const DecParams P) {
             for (int b = 0; b < NB; b++) {
                 const __half2 s01 = __halves2half2(vsc[0][b], vsc[1][b]);
                 const __half2 s23 = __halves2half2(vsc[2][b], vsc[3][b]);
-                uint32_t bb0[NHT], bb1[NHT];
+                uint32_t bb0[NW], bb1[NW];
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++) {
+                for (int nt = 0; nt < NW; nt++) {
                     bb0[nt] = h2u(__hmul2(u2h(pb0[nt]), s01));
                     bb1[nt] = h2u(__hmul2(u2h(pb1[nt]), s23));
                 }
@@ -1096,7 +1142,7 @@ q4_decode_k(const DecParams P) {
                     const uint32_t a2 = cvt_i8_pair<0>(vw[2][b], vw[3][b]);
                     const uint32_t a3 = cvt_i8_pair<1>(vw[2][b], vw[3][b]);
 #pragma unroll
-                    for (int nt = 0; nt < NHT; nt++) mma16816(acc[nt][2 * b], a0, a1, a2, a3, bb0[nt], bb1[nt]);
+                    for (int nt = 0; nt < NW; nt++) mma16816(acc[nt][2 * b], a0, a1, a2, a3, bb0[nt], bb1[nt]);
                 }
                 {
                     const uint32_t a0 = cvt_i8_pair<2>(vw[0][b], vw[1][b]);
@@ -1104,7 +1150,7 @@ q4_decode_k(const DecParams P) {
                     const uint32_t a2 = cvt_i8_pair<2>(vw[2][b], vw[3][b]);
                     const uint32_t a3 = cvt_i8_pair<3>(vw[2][b], vw[3][b]);
 #pragma unroll
-                    for (int nt = 0; nt < NHT; nt++)
+                    for (int nt = 0; nt < NW; nt++)
                         mma16816(acc[nt][2 * b + 1], a0, a1, a2, a3, bb0[nt], bb1[nt]);
                 }
             }
@@ -1130,7 +1176,7 @@ q4_decode_k(const DecParams P) {
                 const uint32_t a0 = lo[0] | (lo[1] << 16), a1 = hi[0] | (hi[1] << 16);
                 const uint32_t a2 = lo[2] | (lo[3] << 16), a3 = hi[2] | (hi[3] << 16);
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++) mma16816(acc[nt][mt], a0, a1, a2, a3, pb0[nt], pb1[nt]);
+                for (int nt = 0; nt < NW; nt++) mma16816(acc[nt][mt], a0, a1, a2, a3, pb0[nt], pb1[nt]);
             }
         }
     };
@@ -1221,9 +1267,9 @@ q4_decode_k(const DecParams P) {
         };
         /* ---- queries: the raw values are requested now, next to the list entries, and converted after the ring
          * has been filled (lane (g, t) takes dims 16ks + 4t .. + 3 of head nt*8 + g) */
-        uint32_t qraw[NHT][KS][4];
+        uint32_t qraw[NW][KS][4];
 #pragma unroll
-        for (int nt = 0; nt < NHT; nt++) {
+        for (int nt = 0; nt < NW; nt++) {
             const uint32_t hg = nt * 8 + g;
             const bool live = hg < P.gqa;
             const size_t qoff = ((size_t)u * P.n_head + (size_t)kh * P.gqa + hg) * HD;
@@ -1273,10 +1319,10 @@ q4_decode_k(const DecParams P) {
          * k-slots 2t, 2t+1, 2t+8, 2t+9.  And,
          * per 32-wide block, -1152 * sum(q): K codes enter the MMA as the fp16 numbers 1152 + code (one byte
          * permute per pair, no subtract), so each block's partial product starts from that correction. */
-        uint32_t qs[NHT][KS][2];
-        float qcorr[NHT][NB][2];
+        uint32_t qs[NW][KS][2];
+        float qcorr[NW][NB][2];
 #pragma unroll
-        for (int nt = 0; nt < NHT; nt++) {
+        for (int nt = 0; nt < NW; nt++) {
             float bsum[NB];
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
@@ -1360,28 +1406,28 @@ q4_decode_k(const DecParams P) {
                 ksc[0][0] = a01.x; ksc[0][1] = a01.y; ksc[0][2] = a23.x; ksc[0][3] = a23.y;
                 ksc[1][0] = b01.x; ksc[1][1] = b01.y; ksc[1][2] = b23.x; ksc[1][3] = b23.y;
             }
-            float sc[NHT][4];
+            float sc[NW][4];
 #pragma unroll
-            for (int nt = 0; nt < NHT; nt++) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
+            for (int nt = 0; nt < NW; nt++) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
 #pragma unroll
             for (int b = 0; b < NB; b++) {
-                float cb[NHT][4];
+                float cb[NW][4];
                 {
                     const uint32_t a0 = __byte_perm(kf[b][0], 0x64646464u, 0x4140), a2 = __byte_perm(kf[b][0], 0x64646464u, 0x4342);
                     const uint32_t a1 = __byte_perm(kf[b][1], 0x64646464u, 0x4140), a3 = __byte_perm(kf[b][1], 0x64646464u, 0x4342);
 #pragma unroll
-                    for (int nt = 0; nt < NHT; nt++)
+                    for (int nt = 0; nt < NW; nt++)
                         mma16816_from(cb[nt], a0, a1, a2, a3, qs[nt][2 * b][0], qs[nt][2 * b][1], qcorr[nt][b][0], qcorr[nt][b][1]);
                 }
                 {
                     const uint32_t a0 = __byte_perm(kf[b][2], 0x64646464u, 0x4140), a2 = __byte_perm(kf[b][2], 0x64646464u, 0x4342);
                     const uint32_t a1 = __byte_perm(kf[b][3], 0x64646464u, 0x4140), a3 = __byte_perm(kf[b][3], 0x64646464u, 0x4342);
 #pragma unroll
-                    for (int nt = 0; nt < NHT; nt++)
+                    for (int nt = 0; nt < NW; nt++)
                         mma16816(cb[nt], a0, a1, a2, a3, qs[nt][2 * b + 1][0], qs[nt][2 * b + 1][1]);
                 }
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++) {
+                for (int nt = 0; nt < NW; nt++) {
                     sc[nt][0] = fmaf(ksc[0][b], cb[nt][0], sc[nt][0]);
                     sc[nt][1] = fmaf(ksc[0][b], cb[nt][1], sc[nt][1]);
                     sc[nt][2] = fmaf(ksc[1][b], cb[nt][2], sc[nt][2]);
@@ -1390,9 +1436,9 @@ q4_decode_k(const DecParams P) {
             }
 
             /* ---- online softmax in the log2 domain; lanes (g, t) hold positions g / g+8 for heads 2t, 2t+1 */
-            uint32_t pb0[NHT], pb1[NHT];
+            uint32_t pb0[NW], pb1[NW];
 #pragma unroll
-            for (int nt = 0; nt < NHT; nt++) {
+            for (int nt = 0; nt < NW; nt++) {
                 sc[nt][0] = kok0 ? sc[nt][0] * P.scale_log2e : -CUDART_INF_F;
                 sc[nt][1] = kok0 ? sc[nt][1] * P.scale_log2e : -CUDART_INF_F;
                 sc[nt][2] = kok1 ? sc[nt][2] * P.scale_log2e : -CUDART_INF_F;
@@ -1428,9 +1474,9 @@ q4_decode_k(const DecParams P) {
                 const uint32_t sel = (b & 1) ? 0x7632 : 0x5410;
                 const uint32_t s01 = __byte_perm(b < 2 ? vs[0].x : vs[0].y, b < 2 ? vs[1].x : vs[1].y, sel);
                 const uint32_t s23 = __byte_perm(b < 2 ? vs[2].x : vs[2].y, b < 2 ? vs[3].x : vs[3].y, sel);
-                uint32_t bb0[NHT], bb1[NHT];
+                uint32_t bb0[NW], bb1[NW];
 #pragma unroll
-                for (int nt = 0; nt < NHT; nt++) {
+                for (int nt = 0; nt < NW; nt++) {
                     bb0[nt] = h2u(__hmul2(u2h(pb0[nt]), u2h(s01)));
                     bb1[nt] = h2u(__hmul2(u2h(pb1[nt]), u2h(s23)));
                 }
@@ -1442,7 +1488,7 @@ q4_decode_k(const DecParams P) {
                     const uint32_t a2 = magic_sub(__byte_perm(v89, 0x64646464u, 0x4240));
                     const uint32_t a3 = magic_sub(__byte_perm(v89, 0x64646464u, 0x4341));
 #pragma unroll
-                    for (int nt = 0; nt < NHT; nt++) mma16816(acc[nt][2 * b + hf], a0, a1, a2, a3, bb0[nt], bb1[nt]);
+                    for (int nt = 0; nt < NW; nt++) mma16816(acc[nt][2 * b + hf], a0, a1, a2, a3, bb0[nt], bb1[nt]);
                 }
             }
         }
@@ -1454,6 +1500,324 @@ q4_decode_k(const DecParams P) {
                 for (uint32_t probes = 0; probes < (RING_SPIN_LIMIT >> 6) && !ring_bar_test(bars + s_i * 8, (par >> s_i) & 1u); probes++) {}
             if (lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
         }
+        __syncthreads();    /* the epilogue below reuses the ring memory of all warps */
+    } else if constexpr (Cfg::STAGED2) {
+        /* ---- fp16 and fp32 rows, reference q8_0 blocks, and native q8_0 records at hd 256: every position group (a warp,
+         * or two warps with 8 query heads each) owns a ring of ST2 tiles in shared memory, filled with asynchronous copies
+         * of whole rows; fragments come out of it as the products need them.  (Fragments loaded straight into registers,
+         * 2 to 16 bytes per lane and no tile ahead, kept too little in flight: 65 us for a 2051-entry list of reference
+         * blocks at hd 256, 12 heads per kv head; 29 us for 100 003 fp16 rows of hd 128.) */
+        using T = DecTile<LAY, HD>;
+        constexpr int ST = Cfg::ST2, WPT = Cfg::WPT, NPG = Cfg::NPG;
+        const uint32_t pg = warp / WPT, hg = warp % WPT;
+        const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + pg * ST * T::BYTES;
+        const uint32_t masks = (uint32_t)__cvta_generic_to_shared(smem_raw) + NPG * ST * T::BYTES + (uint32_t)warp * ST * 4;
+        const uint32_t n_my = s_begin + pg < s_end ? (s_end - s_begin - pg + NPG - 1u) / NPG : 0u;
+        const uint32_t r16 = lane & 15;
+        const bool packed = tok_stride == (uint32_t)T::ROW;   /* rows (records) of consecutive positions are consecutive */
+        auto group_sync = [&]() {
+            if (WPT == 2) asm volatile("bar.sync %0, 64;" ::"r"(pg + 1u) : "memory");
+            else __syncwarp();
+        };
+        auto my_pos = [&](uint32_t it) -> int32_t {
+            const uint32_t j = ((s_begin + pg + it * NPG) << 4) + r16;
+            if (it >= n_my || j >= n_pos) return -1;
+            return list ? list[j] : (int32_t)j;
+        };
+        auto copy = [&](uint32_t dst, const uint8_t *src, bool live) {
+            if (T::CH == 16) {
+                if (live) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+                else if (!Q8) asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dst), "r"(0u) : "memory");
+            } else if (live) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+            }
+        };
+        /* fill one stage; padding rows are zeroed (fp16 / fp32), or left as they are and masked (q8_0) */
+        auto issue = [&](uint32_t it, int32_t p) {
+            if (it < n_my) {
+                if (p >= (int32_t)bound) {
+                    atomicOr(P.err, (uint32_t)Q4E_RANGE);
+                    p = -1;
+                }
+                const uint32_t slot = it % ST, st = ring + slot * T::BYTES;
+                const uint32_t livemask = __ballot_sync(0xffffffffu, p >= 0) & 0xffffu;
+                const int32_t p0 = __shfl_sync(0xffffffffu, p, 0);
+                const bool run = packed && __all_sync(0xffffffffu, p0 >= 0 && p == p0 + (int32_t)r16);
+                constexpr int ITER = (16 * T::CPR + 32 * WPT - 1) / (32 * WPT);
+                const uint64_t run_off = (uint64_t)(uint32_t)max(p0, 0) * tok_stride;
+#pragma unroll
+                for (int plane = 0; plane < (T::REC ? 1 : 2); plane++) {
+                    const uint8_t *src = plane ? vbase : kbase;
+                    const uint32_t dst = st + (plane ? T::V_OFF : 0), pitch = plane ? T::V_PITCH : T::K_PITCH;
+#pragma unroll 4
+                    for (int i = 0; i < ITER; i++) {
+                        const uint32_t idx = lane + 32u * (i * WPT + hg), r = idx / T::CPR, c = idx % T::CPR;
+                        const bool in = 16 * T::CPR % (32 * WPT) == 0 || idx < 16u * T::CPR;
+                        if (run) {
+                            if (in) copy(dst + r * pitch + c * T::CH, src + run_off + idx * T::CH, true);
+                        } else {
+                            const int32_t pr = __shfl_sync(0xffffffffu, p, r & 15u);
+                            if (in) copy(dst + r * pitch + c * T::CH, src + (uint64_t)(uint32_t)max(pr, 0) * tok_stride + c * T::CH, pr >= 0);
+                        }
+                    }
+                }
+                if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
+            }
+            cp_async_commit();   /* one group per tile, empty or not, keeps the wait count uniform */
+        };
+        /* ---- queries, requested next to the list entries: the pairs of dims that k-step ks multiplies in lane t's slots
+         * 2t, 2t+1 (half 0) and 2t+8, 2t+9 (half 1), in the order in which the layout's K fragments carry them */
+        auto q_dim = [&](int ks, int half) -> int {
+            if (LAY == LAY_F16) return 16 * ks + 2 * t + 8 * half;
+            if (LAY == LAY_Q8R) return q8r_dim(ks >> 1, 2 * t + (ks & 1), 2 * half);
+            return 16 * ks + 4 * t + 2 * half;
+        };
+        const uint32_t head = hg * 8 + g;
+        const bool q_live = head < P.gqa;
+        const size_t qoff = ((size_t)u * P.n_head + (size_t)kh * P.gqa + head) * HD;
+        uint32_t qs[KS][2];
+        auto load_q = [&]() {
+#pragma unroll
+            for (int ks = 0; ks < KS; ks++)
+#pragma unroll
+                for (int half = 0; half < 2; half++) {
+                    float2 x = make_float2(0.f, 0.f);
+                    if (q_live) {
+                        if (P.q_bf16) {
+                            const uint32_t w = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + qoff + q_dim(ks, half));
+                            x = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+                        } else {
+                            x = *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(P.q) + qoff + q_dim(ks, half));
+                        }
+                    }
+                    qs[ks][half] = pack_h2(x.x, x.y);
+                }
+        };
+        int32_t pf[ST];
+#pragma unroll
+        for (int i = 0; i < ST; i++) pf[i] = my_pos(i);
+        int32_t pn0 = my_pos(ST), pn1 = my_pos(ST + 1), pn2 = my_pos(ST + 2);
+        /* fused append, second half (see the hd-128 path): a group whose first tiles name the newest row waits for it */
+        bool hold = false;
+        if (P.new_k) {
+#pragma unroll
+            for (int i = 0; i < ST; i++) hold = hold || pf[i] == (int32_t)newest;
+            hold = __any_sync(0xffffffffu, hold);
+        }
+        if (!hold) {
+#pragma unroll
+            for (int i = 0; i < ST; i++) issue(i, pf[i]);
+        }
+        if (LAY != LAY_Q8R && P.new_k) {
+            uint8_t *row = const_cast<uint8_t *>(ap_which ? vbase : kbase) + (uint64_t)newest * tok_stride;
+            const uint32_t at = ap_b * 32 + ap_sub * 4;
+            if (LAY == LAY_Q8P) {
+                float d, id;
+                q4d_block_scale(ap_x, d, id);
+                if (ap_live) {
+                    *reinterpret_cast<uint32_t *>(row + at) = q4d_quant4(ap_x, id);
+                    if (ap_sub == 0)
+                        reinterpret_cast<__half *>(const_cast<uint8_t *>(sbase) + (uint64_t)newest * s_tok_stride)[(ap_which ? NB : 0) + ap_b] = __float2half_rn(d);
+                }
+            } else if (ap_live) {
+                if (LAY == LAY_F16) *reinterpret_cast<uint2 *>(row + at * 2) = make_uint2(pack_h2(ap_x.x, ap_x.y), pack_h2(ap_x.z, ap_x.w));
+                else *reinterpret_cast<float4 *>(row + at * 4) = ap_x;
+            }
+            if (newest >= max_kv && threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
+            __syncthreads();
+        }
+        if (hold) {
+#pragma unroll
+            for (int i = 0; i < ST; i++) issue(i, pf[i]);
+        }
+        load_q();
+        for (uint32_t it = 0; it < n_my; it++) {
+            cp_async_wait<ST - 1>();    /* all but the newest ST - 1 tiles have landed: this warp's part of tile `it` is in */
+            group_sync();
+            const uint32_t slot = it % ST, st = ring + slot * T::BYTES, sv = st + T::V_OFF;
+            const uint32_t livemask = lds32(masks + slot * 4);
+            const bool kok0 = (livemask >> g) & 1u, kok1 = (livemask >> (g + 8)) & 1u;
+            /* ---- S^T = K . Q^T; lanes (g, t) get positions g / g + 8 for heads 2t, 2t + 1 */
+            float sc[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (LAY == LAY_F16) {
+                float s2[4] = {0.f, 0.f, 0.f, 0.f};
+                const uint32_t a0 = st + (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8) * T::K_PITCH + (uint32_t)(lane >> 4) * 16;
+#pragma unroll
+                for (int ks = 0; ks < KS; ks++) {
+                    uint32_t a[4];
+                    ldmatrix_x4(a, a0 + ks * 32);
+                    mma16816(ks & 1 ? s2 : sc, a[0], a[1], a[2], a[3], qs[ks][0], qs[ks][1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) sc[e] += s2[e];
+            } else if constexpr (LAY == LAY_F32) {
+                float s2[4] = {0.f, 0.f, 0.f, 0.f};
+                const uint32_t r0 = st + (uint32_t)g * T::K_PITCH + (uint32_t)t * 16, r1 = r0 + 8 * T::K_PITCH;
+#pragma unroll
+                for (int ks = 0; ks < KS; ks++) {
+                    const float4 x = lds_f4(r0 + ks * 64), y = lds_f4(r1 + ks * 64);
+                    mma16816(ks & 1 ? s2 : sc, pack_h2(x.x, x.y), pack_h2(y.x, y.y), pack_h2(x.z, x.w), pack_h2(y.z, y.w), qs[ks][0], qs[ks][1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) sc[e] += s2[e];
+            } else if constexpr (LAY == LAY_Q8P) {
+                const uint32_t a0 = st + (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8) * T::K_PITCH + (uint32_t)(lane >> 4) * 16;
+                __align__(16) __half h0[NB], h1[NB];
+#pragma unroll
+                for (int i = 0; i < NB / 4; i++) {
+                    reinterpret_cast<uint2 *>(h0)[i] = lds64(st + (uint32_t)g * T::K_PITCH + 2 * HD + 8 * i);
+                    reinterpret_cast<uint2 *>(h1)[i] = lds64(st + (uint32_t)(g + 8) * T::K_PITCH + 2 * HD + 8 * i);
+                }
+#pragma unroll
+                for (int b = 0; b < NB; b++) {
+                    uint32_t k[4];
+                    ldmatrix_x4(k, a0 + b * 32);
+                    float cb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t x0, x2, y0, y2;
+                        cvt_i8x4(k[2 * hf], x0, x2);
+                        cvt_i8x4(k[2 * hf + 1], y0, y2);
+                        mma16816(cb, x0, y0, x2, y2, qs[2 * b + hf][0], qs[2 * b + hf][1]);
+                    }
+                    const float f0 = __half2float(h0[b]), f1 = __half2float(h1[b]);
+                    sc[0] = fmaf(f0, cb[0], sc[0]); sc[1] = fmaf(f0, cb[1], sc[1]);
+                    sc[2] = fmaf(f1, cb[2], sc[2]); sc[3] = fmaf(f1, cb[3], sc[3]);
+                }
+            } else {
+                const uint32_t r0 = st + (uint32_t)g * T::K_PITCH, r1 = r0 + 8 * T::K_PITCH;
+#pragma unroll
+                for (int pr = 0; pr < NB / 2; pr++) {
+                    const uint32_t q0 = r0 + 68 * pr, q1 = r1 + 68 * pr;
+                    const uint32_t u0 = lds32(q0), u8 = lds32(q0 + 32), v0 = lds32(q1), v8 = lds32(q1 + 32);
+                    float cb[4] = {0.f, 0.f, 0.f, 0.f};
+                    {   /* words 1 + 2t and 2 + 2t of the even block; lane 3's second is codes 0 1 30 31 */
+                        const uint32_t xa = lds32(q0 + 4 + 8 * t), ya = lds32(q1 + 4 + 8 * t);
+                        const uint32_t xb = t == 3 ? __byte_perm(u0, u8, 0x5432) : lds32(q0 + 8 + 8 * t);
+                        const uint32_t yb = t == 3 ? __byte_perm(v0, v8, 0x5432) : lds32(q1 + 8 + 8 * t);
+                        uint32_t x0, x2, y0, y2;
+                        cvt_i8x4(xa, x0, x2); cvt_i8x4(ya, y0, y2);
+                        mma16816(cb, x0, y0, x2, y2, qs[4 * pr][0], qs[4 * pr][1]);
+                        cvt_i8x4(xb, x0, x2); cvt_i8x4(yb, y0, y2);
+                        mma16816(cb, x0, y0, x2, y2, qs[4 * pr + 1][0], qs[4 * pr + 1][1]);
+                    }
+                    float f0 = __low2float(u2h(u0)), f1 = __low2float(u2h(v0));
+                    sc[0] = fmaf(f0, cb[0], sc[0]); sc[1] = fmaf(f0, cb[1], sc[1]);
+                    sc[2] = fmaf(f1, cb[2], sc[2]); sc[3] = fmaf(f1, cb[3], sc[3]);
+                    cb[0] = cb[1] = cb[2] = cb[3] = 0.f;
+#pragma unroll
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t x0, x2, y0, y2;
+                        cvt_i8x4(lds32(q0 + 36 + 8 * t + 4 * hf), x0, x2);
+                        cvt_i8x4(lds32(q1 + 36 + 8 * t + 4 * hf), y0, y2);
+                        mma16816(cb, x0, y0, x2, y2, qs[4 * pr + 2 + hf][0], qs[4 * pr + 2 + hf][1]);
+                    }
+                    f0 = __high2float(u2h(u8)); f1 = __high2float(u2h(v8));
+                    sc[0] = fmaf(f0, cb[0], sc[0]); sc[1] = fmaf(f0, cb[1], sc[1]);
+                    sc[2] = fmaf(f1, cb[2], sc[2]); sc[3] = fmaf(f1, cb[3], sc[3]);
+                }
+            }
+            /* ---- online softmax in the log2 domain */
+            sc[0] = kok0 ? sc[0] * P.scale_log2e : -CUDART_INF_F;
+            sc[1] = kok0 ? sc[1] * P.scale_log2e : -CUDART_INF_F;
+            sc[2] = kok1 ? sc[2] * P.scale_log2e : -CUDART_INF_F;
+            sc[3] = kok1 ? sc[3] * P.scale_log2e : -CUDART_INF_F;
+            const float mn0 = fmaxf(m_run[0][0], warp_max_over_g(fmaxf(sc[0], sc[2])));
+            const float mn1 = fmaxf(m_run[0][1], warp_max_over_g(fmaxf(sc[1], sc[3])));
+            const float mu0 = mn0 == -CUDART_INF_F ? 0.f : mn0, mu1 = mn1 == -CUDART_INF_F ? 0.f : mn1;
+            const float al0 = ex2(m_run[0][0] - mu0), al1 = ex2(m_run[0][1] - mu1);
+            m_run[0][0] = mn0;
+            m_run[0][1] = mn1;
+            const __half2 h0 = __floats2half2_rn(ex2(sc[0] - mu0), ex2(sc[1] - mu1));
+            const __half2 h1 = __floats2half2_rn(ex2(sc[2] - mu0), ex2(sc[3] - mu1));
+            l_run[0][0] = fmaf(l_run[0][0], al0, __low2float(h0) + __low2float(h1));
+            l_run[0][1] = fmaf(l_run[0][1], al1, __high2float(h0) + __high2float(h1));
+            if (__any_sync(0xffffffffu, al0 != 1.f || al1 != 1.f)) {
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    acc[0][mt][0] *= al0; acc[0][mt][1] *= al1;
+                    acc[0][mt][2] *= al0; acc[0][mt][3] *= al1;
+                }
+            }
+            const uint32_t pb0 = movmatrix_t(h2u(h0)), pb1 = movmatrix_t(h2u(h1));   /* positions 2t, 2t+1 / 2t+8, 2t+9 of head g */
+
+            /* ---- O^T += V^T . P^T */
+            if constexpr (LAY == LAY_F16) {
+                const uint32_t v0 = sv + (uint32_t)((lane & 7) + (lane >> 4) * 8) * T::V_PITCH + (uint32_t)((lane >> 3) & 1) * 16;
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    uint32_t a[4];
+                    ldmatrix_x4_trans(a, v0 + mt * 32);
+                    mma16816(acc[0][mt], a[0], a[1], a[2], a[3], pb0, pb1);
+                }
+            } else if constexpr (LAY == LAY_F32) {
+                const uint32_t v0 = sv + (uint32_t)(2 * t) * T::V_PITCH + (uint32_t)g * 8;
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    float2 x[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) x[r] = lds_f2(v0 + (uint32_t)((r & 1) + 8 * (r >> 1)) * T::V_PITCH + mt * 64);
+                    mma16816(acc[0][mt], pack_h2(x[0].x, x[1].x), pack_h2(x[0].y, x[1].y), pack_h2(x[2].x, x[3].x), pack_h2(x[2].y, x[3].y), pb0, pb1);
+                }
+            } else {
+                /* V block scales go into the weights, block by block; a padding position's scale counts as zero */
+                const bool vok[4] = {(bool)((livemask >> (2 * t)) & 1u), (bool)((livemask >> (2 * t + 1)) & 1u),
+                                     (bool)((livemask >> (2 * t + 8)) & 1u), (bool)((livemask >> (2 * t + 9)) & 1u)};
+                auto products = [&](int b, const uint32_t (&w)[4], const uint32_t (&s16)[4]) {
+                    const uint32_t s01 = (vok[0] ? s16[0] & 0xffffu : 0u) | (vok[1] ? s16[1] << 16 : 0u);
+                    const uint32_t s23 = (vok[2] ? s16[2] & 0xffffu : 0u) | (vok[3] ? s16[3] << 16 : 0u);
+                    const uint32_t b0 = h2u(__hmul2(u2h(pb0), u2h(s01))), b1 = h2u(__hmul2(u2h(pb1), u2h(s23)));
+                    mma16816(acc[0][2 * b], cvt_i8_pair<0>(w[0], w[1]), cvt_i8_pair<1>(w[0], w[1]), cvt_i8_pair<0>(w[2], w[3]), cvt_i8_pair<1>(w[2], w[3]), b0, b1);
+                    mma16816(acc[0][2 * b + 1], cvt_i8_pair<2>(w[0], w[1]), cvt_i8_pair<3>(w[0], w[1]), cvt_i8_pair<2>(w[2], w[3]), cvt_i8_pair<3>(w[2], w[3]), b0, b1);
+                };
+                if constexpr (LAY == LAY_Q8P) {
+                    const uint32_t v0 = sv + (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8) * T::K_PITCH + (uint32_t)(lane >> 4) * 16;
+                    __align__(16) uint16_t vs[4][NB];
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+#pragma unroll
+                        for (int i = 0; i < NB / 4; i++)
+                            reinterpret_cast<uint2 *>(vs[r])[i] = lds64(st + (uint32_t)(2 * t + (r & 1) + 8 * (r >> 1)) * T::K_PITCH + 2 * HD + 2 * NB + 8 * i);
+#pragma unroll
+                    for (int b = 0; b < NB; b++) {
+                        /* v[i]: positions 2t, 2t+1 (+8 for odd i), 2 codes each of dims 32b + 16 (i >> 1) + 2g, + 1 */
+                        uint32_t v[4];
+                        ldmatrix_x4_trans(v, v0 + b * 32);
+                        const uint32_t s01 = (vok[0] ? vs[0][b] : 0u) | (vok[1] ? (uint32_t)vs[1][b] << 16 : 0u);
+                        const uint32_t s23 = (vok[2] ? vs[2][b] : 0u) | (vok[3] ? (uint32_t)vs[3][b] << 16 : 0u);
+                        const uint32_t b0 = h2u(__hmul2(u2h(pb0), u2h(s01))), b1 = h2u(__hmul2(u2h(pb1), u2h(s23)));
+#pragma unroll
+                        for (int hf = 0; hf < 2; hf++) {
+                            const uint32_t x = v[2 * hf] ^ 0x80808080u, y = v[2 * hf + 1] ^ 0x80808080u;
+                            mma16816(acc[0][2 * b + hf], magic_sub(__byte_perm(x, 0x64646464u, 0x4240)), magic_sub(__byte_perm(x, 0x64646464u, 0x4341)),
+                                     magic_sub(__byte_perm(y, 0x64646464u, 0x4240)), magic_sub(__byte_perm(y, 0x64646464u, 0x4341)), b0, b1);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int pr = 0; pr < NB / 2; pr++) {
+                        uint32_t w0[4], w8[4], we[4], wo[4];
+#pragma unroll
+                        for (int r = 0; r < 4; r++) {
+                            const uint32_t row = sv + (uint32_t)(2 * t + (r & 1) + 8 * (r >> 1)) * T::V_PITCH + 68 * pr;
+                            w0[r] = lds32(row);
+                            w8[r] = lds32(row + 32);
+                            we[r] = g == 7 ? __byte_perm(w0[r], w8[r], 0x5432) : lds32(row + 4 + 4 * g);
+                            wo[r] = lds32(row + 36 + 4 * g);
+                        }
+                        products(2 * pr, we, w0);
+#pragma unroll
+                        for (int r = 0; r < 4; r++) w8[r] >>= 16;
+                        products(2 * pr + 1, wo, w8);
+                    }
+                }
+            }
+            group_sync();                        /* every lane that shares the stage is done with it */
+            issue(it + ST, pn0);                 /* refill it with the tile ST ahead */
+            pn0 = pn1; pn1 = pn2;
+            pn2 = my_pos(it + ST + 3);
+        }
+        cp_async_wait<0>();
         __syncthreads();    /* the epilogue below reuses the ring memory of all warps */
     } else {
         for (uint32_t step = s_begin + warp; step < s_end; step += DEC_WARPS) {
@@ -1553,11 +1917,11 @@ q4_decode_k(const DecParams P) {
     }
 
     /* ---- block reduction of the warps' partials ------------------------------------------- */
-    float *sm = reinterpret_cast<float *>(smem_raw);   /* [DEC_WARPS][HEADS][REC] : acc[HD], m, l */
+    float *sm = reinterpret_cast<float *>(smem_raw);   /* [position group][HEADS][REC] : acc[HD], m, l */
 #pragma unroll
-    for (int nt = 0; nt < NHT; nt++) {
+    for (int nt = 0; nt < NW; nt++) {
         const float l0 = warp_sum_over_g(l_run[nt][0]), l1 = warp_sum_over_g(l_run[nt][1]);
-        float *r0 = sm + ((size_t)warp * HEADS + nt * 8 + 2 * t) * REC;
+        float *r0 = sm + ((size_t)(warp / Cfg::WPT) * HEADS + (warp % Cfg::WPT) * 8 + nt * 8 + 2 * t) * REC;
         float *r1 = r0 + REC;
         if (g == 0) {
             r0[HD] = m_run[nt][0]; r0[HD + 1] = l0;
@@ -1565,7 +1929,7 @@ q4_decode_k(const DecParams P) {
         }
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
-            const int d0 = out_dim<LAY, Cfg::STAGED>(mt, g, 0), d1 = out_dim<LAY, Cfg::STAGED>(mt, g, 1);
+            const int d0 = out_dim<LAY, Cfg::STAGED, Cfg::STAGED2>(mt, g, 0), d1 = out_dim<LAY, Cfg::STAGED, Cfg::STAGED2>(mt, g, 1);
             r0[d0] = acc[nt][mt][0]; r1[d0] = acc[nt][mt][1];
             r0[d1] = acc[nt][mt][2]; r1[d1] = acc[nt][mt][3];
         }
@@ -1581,13 +1945,13 @@ q4_decode_k(const DecParams P) {
     /* exchange mode: the unit's last merge leaves this rank's record here instead of finalising */
     float *fin = P.xchg ? reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES) : nullptr;
     if (S == 1) {
-        merge_records<HD, HEADS>(sm, DEC_WARPS, false, fin, mo, mscr);
+        merge_records<HD, HEADS>(sm, Cfg::NPG, false, fin, mo, mscr);
         if (fin) xchg_finish<HD, HEADS>(P.xchg, P.xchg_phase, (uint32_t)unit, fin, mo, P.err);
         return;
     }
     if (P.cluster) {
         float *own = reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES);
-        merge_records<HD, HEADS>(sm, DEC_WARPS, false, own, mo, mscr);
+        merge_records<HD, HEADS>(sm, Cfg::NPG, false, own, mo, mscr);
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   /* every peer block has started (arrive at entry) */
         if (P.push_bytes) {
             cluster_push_merge<HD, HEADS>(own, reinterpret_cast<const float *>(smem_raw + Cfg::SMEM), S, cluster_ctarank(), mo,
@@ -1607,7 +1971,7 @@ q4_decode_k(const DecParams P) {
     const uint32_t grp_size = min(DEC_GROUP, S - grp * DEC_GROUP);
     float *rec1 = P.scratch + (unit * (size_t)(S + n_groups)) * HEADS * REC;
     if (P.gridmerge) {
-        merge_records<HD, HEADS>(sm, DEC_WARPS, false, rec1 + (size_t)split * HEADS * REC, mo, mscr);
+        merge_records<HD, HEADS>(sm, Cfg::NPG, false, rec1 + (size_t)split * HEADS * REC, mo, mscr);
         __syncthreads();   /* the warp records in shared memory are no longer needed: their space is the scratch */
         grid_merge<HD, HEADS>(rec1, S, split, P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP), mo, sm, P.err);
         return;
@@ -1616,7 +1980,7 @@ q4_decode_k(const DecParams P) {
     uint32_t *ctr = P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP);
     /* one call site for every level keeps a single copy of the merge code in the kernel */
     const float *src = sm;
-    uint32_t count = DEC_WARPS;
+    uint32_t count = Cfg::NPG;
     bool global = false;
     float *dst = rec1 + (size_t)split * HEADS * REC;
     uint32_t *arrive = ctr + 1 + grp;
@@ -1674,17 +2038,17 @@ __global__ void q4_lse_merge_k(const float *parts, uint32_t n_parts, uint32_t n_
     }
 }
 
-template <int LAY, int HD, int NHT>
+template <int LAY, int HD, int NHT, bool DIRECT>
 bool launch(const DecParams &p_in, dim3 grid) {
-    constexpr size_t smem_base = DecCfg<LAY, HD, NHT>::SMEM;
+    constexpr size_t smem_base = DecCfg<LAY, HD, NHT, DIRECT>::SMEM;
     constexpr size_t SMEM_LIMIT = smem_base + 2u * DEC_CLUSTER_MAX * (HD + 4) * sizeof(float) + 16u;   /* ring / epilogue + the largest receive area of the push merge */
     static bool attr_done = false;
     if (!attr_done) {
-        if (!q4i_check(cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT>,
+        if (!q4i_check(cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT),
                        "decode smem attribute"))
             return false;
-        (void)cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        (void)cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
     attr_done = true;
     DecParams p = p_in;
@@ -1709,7 +2073,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
         qc.attrs = qa;
         qc.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, q4_decode_k<LAY, HD, NHT>, &qc) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&n, q4_decode_k<LAY, HD, NHT, DIRECT>, &qc) != cudaSuccess) {
             (void)cudaGetLastError();
             n = 0;
         }
@@ -1725,7 +2089,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
     if (p.gridmerge) {
         /* the blocks of a unit wait for one another: only when the whole grid is resident at once */
         static int occ = -1;
-        if (occ < 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, q4_decode_k<LAY, HD, NHT>, DEC_THREADS, smem_base) != cudaSuccess) {
+        if (occ < 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, q4_decode_k<LAY, HD, NHT, DIRECT>, DEC_THREADS, smem_base) != cudaSuccess) {
             (void)cudaGetLastError();
             occ = 0;
         }
@@ -1765,11 +2129,14 @@ bool launch(const DecParams &p_in, dim3 grid) {
     }
     cfg.attrs = at;
     cfg.numAttrs = n_at;
-    return q4i_check(cudaLaunchKernelEx(&cfg, q4_decode_k<LAY, HD, NHT>, p), "decode launch");
+    return q4i_check(cudaLaunchKernelEx(&cfg, q4_decode_k<LAY, HD, NHT, DIRECT>, p), "decode launch");
 }
 template <int LAY, int HD>
 bool launch_nht(const DecParams &p, dim3 grid) {
-    return p.gqa <= 8 ? launch<LAY, HD, 1>(p, grid) : launch<LAY, HD, 2>(p, grid);
+    if constexpr (HD >= 128 && (LAY == LAY_Q8R || LAY == LAY_F16)) {
+        if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true>(p, grid) : launch<LAY, HD, 2, true>(p, grid);
+    }
+    return p.gqa <= 8 ? launch<LAY, HD, 1, false>(p, grid) : launch<LAY, HD, 2, false>(p, grid);
 }
 template <int LAY>
 bool launch_hd(const DecParams &p, dim3 grid, uint32_t hd) {
@@ -1925,8 +2292,9 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         p.pdl = pdl ? 1u : 0u;
     }
     if (a.new_k || a.new_v)
-        Q4_REQUIRE(a.new_k && a.new_v && a.layout == LAY_Q8P && a.hd == 128,
-                   "decode: fused append needs both rows and the native q8_0 store at hd 128");
+        Q4_REQUIRE(a.new_k && a.new_v && a.layout != LAY_Q8R && a.hd >= 128,
+                   "decode: fused append needs both rows and a store at hd 128 or 256");
+    p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
     dim3 grid(S, a.n_kvh, a.n_units);
     switch (a.layout) {
     case LAY_F32: return launch_hd<LAY_F32>(p, grid, a.hd);

@@ -706,7 +706,7 @@ extern "C" bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, cons
     Q4_REQUIRE(b && b->n && k && v && q && out && b->kv[0] && layer < b->kv[0]->n_layers && n_head,
                "batch_append_decode: bad argument");
     Q4_REQUIRE(b->n_active, "batch_append_decode: no positions published (q4_gpu_batch_set_pos)");
-    const bool fused = b->kv[0]->kind == Q4K_Q8 && b->kv[0]->hd == 128;
+    const bool fused = b->kv[0]->hd >= 128;
     if (!fused && !q4_gpu_batch_append(b, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));
@@ -732,7 +732,7 @@ extern "C" bool q4_gpu_kv_append_decode_d(q4_gpu_kv *kv, uint32_t layer, const f
                                           uint32_t width, uint32_t idx_kvh_stride, float scale) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_append_decode_d: library not initialised");
     Q4_REQUIRE(kv && k && v && q && out && layer < kv->n_layers && n_head, "kv_append_decode_d: bad argument");
-    const bool fused = kv->kind == Q4K_Q8 && kv->hd == 128;
+    const bool fused = kv->hd >= 128;
     if (!fused && !q4_gpu_kv_append_d(kv, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));
