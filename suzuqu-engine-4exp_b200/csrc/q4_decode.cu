@@ -84,6 +84,7 @@ struct DecParams {
     uint32_t pdl;                 /* launched with programmatic stream serialization */
     uint32_t gridmerge;           /* long scans: every split's record goes to scratch, the unit's blocks meet at a counter,
                                    * and (head, 32-dim) slices of the merge are shared out among them */
+    uint32_t min_tiles;           /* with gridmerge: tiles that a block takes at least */
     uint32_t push_bytes;          /* > 0: the launch carries this much extra shared memory and merges by pushing */
     uint32_t push_async;          /* pushes complete an mbarrier of the receiving block (its last 16 bytes) instead of
                                    * meeting at a cluster barrier */
@@ -613,41 +614,60 @@ __device__ __noinline__ void cluster_push_merge(const float *own, const float *r
 }
 
 /* ---- merge of a long scan's records by all of the unit's blocks ---------------------------------
- * A unit with hundreds of splits (a dense scan over 262144 rows: 222 blocks per kv head) used to merge in two
- * levels, each a fence + atomic + the last block of a group reading 16 records: two serial round trips through L2
- * behind the slowest block.  Here every block writes its record, the unit's S blocks meet at a counter (they are
- * all resident: the launcher checks that the grid fits in one wave), and the first gqa * HD / 32 of them each
- * merge one (head, 32 dims) slice of all S records: the weights once per record, then 16 record lanes x 8 threads
- * of 4 dims stream the accumulators.  The wait is bounded; the last block to leave re-arms the two counters. */
+ * A unit with hundreds of splits (a dense scan over 262144 rows: 222 blocks per kv head) would merge in two levels, each a
+ * fence + atomic + the last block of a group reading 16 records: two serial round trips through L2 behind the slowest
+ * block.  Here every block writes its record, the unit's blocks meet at a counter (they are all resident: the launcher
+ * checks that the grid fits in one wave), and each merges (head, 32 dims) slices of all records.  A slice is one round trip:
+ * all (m, l) pairs and all accumulator pieces are requested at once, 16 record lanes x 8 threads of 4 dims (piece by
+ * piece in a loop they took 7 us behind the last block at 262144 rows, 16 serial round trips).
+ * `n_rec` blocks have a record; blocks without one (the launch was sized for the store's capacity, the context is short)
+ * only help to merge.  The wait is bounded; the last block to leave re-arms the two counters. */
 constexpr uint32_t GRID_SPIN_LIMIT = 1u << 22;
 template <int HD, int HEADS>
-__device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t split, uint32_t *ctr, const MergeOut mo,
+__device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t n_rec, uint32_t split, uint32_t *ctr, const MergeOut mo,
                                         float *scr /* >= 256 + 16 * 32 + 8 floats of shared memory */, uint32_t *err) {
     constexpr int REC = HD + 4, CH = HD / 32;
+    constexpr uint32_t LANES = 16, PER = DEC_MAX_SPLIT / LANES;
+    const uint32_t tasks = mo.gqa * CH, members = min(S, max(n_rec, tasks));
+    if (split >= members) return;   /* neither a record nor a slice */
     __shared__ uint32_t s_ok;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        atomicAdd(&ctr[0], 1u);
+        if (split < n_rec) atomicAdd(&ctr[0], 1u);
         uint32_t spins = 0, seen;
         do {
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
-        } while (seen < S && ++spins < GRID_SPIN_LIMIT);
-        s_ok = seen >= S ? 1u : 0u;
+        } while (seen < n_rec && ++spins < GRID_SPIN_LIMIT);
+        s_ok = seen >= n_rec ? 1u : 0u;
     }
     __syncthreads();
     const bool ok = s_ok != 0u;
     float *s_w = scr, *s_part = scr + 256, *s_red = scr + 256 + 16 * 32;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (ok)
-        for (uint32_t task = split; task < mo.gqa * CH; task += S) {
+        for (uint32_t task = split; task < tasks; task += S) {
             const uint32_t h = task / CH, d0 = (task % CH) * 32;
-            /* weights of the S records of head h (m in log2 units; an empty record has l = 0) */
-            float mloc = -CUDART_INF_F;
-            for (uint32_t r = threadIdx.x; r < S; r += DEC_THREADS) {
-                const float2 ml = __ldcg(reinterpret_cast<const float2 *>(recs + ((size_t)r * HEADS + h) * REC + HD));
-                if (ml.y > 0.f) mloc = fmaxf(mloc, ml.x);
+            const uint32_t q = threadIdx.x >> 3, dq = (threadIdx.x & 7u) * 4u;
+            float2 ml[DEC_MAX_SPLIT / DEC_THREADS];
+            float4 x[PER];
+#pragma unroll
+            for (uint32_t k = 0; k < DEC_MAX_SPLIT / DEC_THREADS; k++) {
+                const uint32_t r = threadIdx.x + k * DEC_THREADS;
+                ml[k] = make_float2(0.f, 0.f);
+                if (r < n_rec) ml[k] = __ldcg(reinterpret_cast<const float2 *>(recs + ((size_t)r * HEADS + h) * REC + HD));
             }
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) {
+                const uint32_t r = q + k * LANES;
+                x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < n_rec) x[k] = __ldcg(reinterpret_cast<const float4 *>(recs + ((size_t)r * HEADS + h) * REC + d0 + dq));
+            }
+            /* weights of the records of head h (m in log2 units; an empty record has l = 0) */
+            float mloc = -CUDART_INF_F;
+#pragma unroll
+            for (uint32_t k = 0; k < DEC_MAX_SPLIT / DEC_THREADS; k++)
+                if (ml[k].y > 0.f) mloc = fmaxf(mloc, ml[k].x);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) mloc = fmaxf(mloc, __shfl_xor_sync(0xffffffffu, mloc, o));
             if (lane == 0) s_red[warp] = mloc;
@@ -655,25 +675,22 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
             const float M = fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3]));
             const float Mu = M == -CUDART_INF_F ? 0.f : M;
             float lloc = 0.f;
-            for (uint32_t r = threadIdx.x; r < S; r += DEC_THREADS) {
-                const float2 ml = __ldcg(reinterpret_cast<const float2 *>(recs + ((size_t)r * HEADS + h) * REC + HD));
-                const float w = ml.y > 0.f ? ex2(ml.x - Mu) : 0.f;
-                s_w[r] = w;
-                lloc = fmaf(w, ml.y, lloc);
+#pragma unroll
+            for (uint32_t k = 0; k < DEC_MAX_SPLIT / DEC_THREADS; k++) {
+                const float w = ml[k].y > 0.f ? ex2(ml[k].x - Mu) : 0.f;
+                s_w[threadIdx.x + k * DEC_THREADS] = w;
+                lloc = fmaf(w, ml[k].y, lloc);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) lloc += __shfl_xor_sync(0xffffffffu, lloc, o);
-            __syncthreads();                       /* s_red read by everyone, s_w written */
             if (lane == 0) s_red[4 + warp] = lloc;
             __syncthreads();
             const float L = (s_red[4] + s_red[5]) + (s_red[6] + s_red[7]);
-            /* 16 record lanes x 8 threads of 4 dims */
-            const uint32_t q = threadIdx.x >> 3, dq = (threadIdx.x & 7u) * 4u;
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (uint32_t r = q; r < S; r += 16) {
-                const float w = s_w[r];
-                const float4 x = __ldcg(reinterpret_cast<const float4 *>(recs + ((size_t)r * HEADS + h) * REC + d0 + dq));
-                A.x = fmaf(w, x.x, A.x); A.y = fmaf(w, x.y, A.y); A.z = fmaf(w, x.z, A.z); A.w = fmaf(w, x.w, A.w);
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) {
+                const float w = s_w[q + k * LANES];
+                A.x = fmaf(w, x[k].x, A.x); A.y = fmaf(w, x[k].y, A.y); A.z = fmaf(w, x[k].z, A.z); A.w = fmaf(w, x[k].w, A.w);
             }
             *reinterpret_cast<float4 *>(s_part + q * 32 + dq) = A;
             __syncthreads();
@@ -681,8 +698,8 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
                 float4 T = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int k = 0; k < 16; k++) {
-                    const float4 x = *reinterpret_cast<const float4 *>(s_part + k * 32 + dq);
-                    T.x += x.x; T.y += x.y; T.z += x.z; T.w += x.w;
+                    const float4 y = *reinterpret_cast<const float4 *>(s_part + k * 32 + dq);
+                    T.x += y.x; T.y += y.y; T.z += y.z; T.w += y.w;
                 }
                 merge_store<HD>(nullptr, mo, h, d0 + dq, M, L, T);
             }
@@ -691,7 +708,7 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
     if (threadIdx.x == 0) {
         if (!ok) atomicOr(err, (uint32_t)Q4E_CUDA);
         __threadfence();
-        if (atomicAdd(&ctr[1], 1u) == S - 1u) {   /* everyone has passed the meeting point: ready for the next launch */
+        if (atomicAdd(&ctr[1], 1u) == members - 1u) {   /* everyone has passed the meeting point: ready for the next launch */
             ctr[1] = 0u;
             __threadfence();
             ctr[0] = 0u;
@@ -870,8 +887,8 @@ struct DecTile {
     static constexpr int V_OFF = REC ? HD : 16 * K_PITCH;
     static constexpr int BYTES = 16 * (K_PITCH + V_PITCH);
 };
-constexpr int dec_stages(int groups_bytes) {   /* 3 blocks per SM with 2 to 4 stages, else 2 with 2, else 1 */
-    return groups_bytes * 4 <= 73728 ? 4 : groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 110592 ? 2 : groups_bytes * 2 <= 204800 ? 2 : 1;
+constexpr int dec_stages(int groups_bytes) {   /* as many, up to 4, as leave room for 3 blocks per SM */
+    return groups_bytes * 4 <= 73728 ? 4 : groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 73728 ? 2 : 1;
 }
 /* DIRECT: caches whose base is not aligned for the asynchronous copies (reference ABI only) load fragments into registers */
 template <int LAY, int HD, int NHT, bool DIRECT>
@@ -944,7 +961,9 @@ q4_decode_k(const DecParams P) {
                                 : nullptr;
     const uint32_t n_pos = list ? P.width : n_kv;
     const uint32_t steps = (n_pos + 15u) >> 4;
-    const uint32_t per = (steps + S - 1u) / S;
+    /* a launch sized for the store's capacity (position from the device) uses as many of its blocks as the context needs */
+    const uint32_t S_act = P.gridmerge ? min(S, max((steps + P.min_tiles - 1u) / P.min_tiles, 1u)) : S;
+    const uint32_t per = (steps + S_act - 1u) / S_act;
     const uint32_t s_begin = split * per;
     const uint32_t s_end = min(s_begin + per, steps);
 
@@ -958,6 +977,18 @@ q4_decode_k(const DecParams P) {
     /* list entries at or beyond this are skipped and raise the range status: the rows written so far for a
      * store (rows behind them hold nothing), the capacity for a caller-owned cache of the reference ABI */
     const uint32_t bound = P.idx_bound_nkv ? n_kv : max_kv;
+
+    const size_t unit = (size_t)u * P.n_kvh + kh;
+    MergeOut mo;
+    mo.out = P.out; mo.part_out = P.part_out; mo.gate = P.gate;
+    mo.row0 = (size_t)u * P.n_head + (size_t)kh * P.gqa;
+    mo.gqa = P.gqa;
+    const uint32_t n_groups = (S + DEC_GROUP - 1u) / DEC_GROUP;
+    float *rec1 = P.scratch + (unit * (size_t)(S + n_groups)) * HEADS * REC;
+    if (P.gridmerge && split >= S_act) {
+        grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP), mo, reinterpret_cast<float *>(smem_raw), P.err);
+        return;
+    }
 
     /* ---- fused append, first half: the load of the unit's new K/V row is issued here, next to the
      * loads of the list entries below, so that the two round trips overlap; the row is quantised and
@@ -1508,7 +1539,7 @@ q4_decode_k(const DecParams P) {
          * 2 to 16 bytes per lane and no tile ahead, kept too little in flight: 65 us for a 2051-entry list of reference
          * blocks at hd 256, 12 heads per kv head; 29 us for 100 003 fp16 rows of hd 128.) */
         using T = DecTile<LAY, HD>;
-        constexpr int ST = Cfg::ST2, WPT = Cfg::WPT, NPG = Cfg::NPG;
+        constexpr int ST = Cfg::ST2, WPT = Cfg::WPT, NPG = Cfg::NPG, PLANES = T::REC ? 1 : 2;
         const uint32_t pg = warp / WPT, hg = warp % WPT;
         const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + pg * ST * T::BYTES;
         const uint32_t masks = (uint32_t)__cvta_generic_to_shared(smem_raw) + NPG * ST * T::BYTES + (uint32_t)warp * ST * 4;
@@ -1532,8 +1563,8 @@ q4_decode_k(const DecParams P) {
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
             }
         };
-        /* fill one stage; padding rows are zeroed (fp16 / fp32), or left as they are and masked (q8_0) */
-        auto issue = [&](uint32_t it, int32_t p) {
+        /* fill one stage (planes [pl0, pl1): K, V); padding rows are zeroed (fp16 / fp32), or left as they are and masked (q8_0) */
+        auto issue_planes = [&](uint32_t it, int32_t p, int pl0, int pl1) {
             if (it < n_my) {
                 if (p >= (int32_t)bound) {
                     atomicOr(P.err, (uint32_t)Q4E_RANGE);
@@ -1546,7 +1577,7 @@ q4_decode_k(const DecParams P) {
                 constexpr int ITER = (16 * T::CPR + 32 * WPT - 1) / (32 * WPT);
                 const uint64_t run_off = (uint64_t)(uint32_t)max(p0, 0) * tok_stride;
 #pragma unroll
-                for (int plane = 0; plane < (T::REC ? 1 : 2); plane++) {
+                for (int plane = pl0; plane < pl1; plane++) {
                     const uint8_t *src = plane ? vbase : kbase;
                     const uint32_t dst = st + (plane ? T::V_OFF : 0), pitch = plane ? T::V_PITCH : T::K_PITCH;
 #pragma unroll 4
@@ -1561,9 +1592,15 @@ q4_decode_k(const DecParams P) {
                         }
                     }
                 }
-                if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
+                if (pl1 == PLANES && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
             }
-            cp_async_commit();   /* one group per tile, empty or not, keeps the wait count uniform */
+            cp_async_commit();   /* one group per call, empty or not, keeps the wait count uniform */
+        };
+        /* With a single stage K and V travel as two groups: the next tile's K rows come in under this tile's P . V. */
+        constexpr bool HALVES = ST == 1 && !T::REC;
+        auto issue = [&](uint32_t it, int32_t p) {
+            if (HALVES) { issue_planes(it, p, 0, 1); issue_planes(it, p, 1, 2); }
+            else issue_planes(it, p, 0, PLANES);
         };
         /* ---- queries, requested next to the list entries: the pairs of dims that k-step ks multiplies in lane t's slots
          * 2t, 2t+1 (half 0) and 2t+8, 2t+9 (half 1), in the order in which the layout's K fragments carry them */
@@ -1632,7 +1669,7 @@ q4_decode_k(const DecParams P) {
         }
         load_q();
         for (uint32_t it = 0; it < n_my; it++) {
-            cp_async_wait<ST - 1>();    /* all but the newest ST - 1 tiles have landed: this warp's part of tile `it` is in */
+            cp_async_wait<HALVES ? 1 : ST - 1>();    /* all but the newest ST - 1 tiles (the V rows) have landed: this warp's part of tile `it` is in */
             group_sync();
             const uint32_t slot = it % ST, st = ring + slot * T::BYTES, sv = st + T::V_OFF;
             const uint32_t livemask = lds32(masks + slot * 4);
@@ -1717,6 +1754,10 @@ q4_decode_k(const DecParams P) {
                     sc[2] = fmaf(f1, cb[2], sc[2]); sc[3] = fmaf(f1, cb[3], sc[3]);
                 }
             }
+            if (HALVES) {
+                group_sync();                    /* K rows read */
+                issue_planes(it + 1, pn0, 0, 1);
+            }
             /* ---- online softmax in the log2 domain */
             sc[0] = kok0 ? sc[0] * P.scale_log2e : -CUDART_INF_F;
             sc[1] = kok0 ? sc[1] * P.scale_log2e : -CUDART_INF_F;
@@ -1741,6 +1782,10 @@ q4_decode_k(const DecParams P) {
             }
             const uint32_t pb0 = movmatrix_t(h2u(h0)), pb1 = movmatrix_t(h2u(h1));   /* positions 2t, 2t+1 / 2t+8, 2t+9 of head g */
 
+            if (HALVES) {
+                cp_async_wait<1>();
+                group_sync();                    /* V rows are in */
+            }
             /* ---- O^T += V^T . P^T */
             if constexpr (LAY == LAY_F16) {
                 const uint32_t v0 = sv + (uint32_t)((lane & 7) + (lane >> 4) * 8) * T::V_PITCH + (uint32_t)((lane >> 3) & 1) * 16;
@@ -1813,7 +1858,8 @@ q4_decode_k(const DecParams P) {
                 }
             }
             group_sync();                        /* every lane that shares the stage is done with it */
-            issue(it + ST, pn0);                 /* refill it with the tile ST ahead */
+            if (HALVES) issue_planes(it + 1, pn0, 1, 2);
+            else issue(it + ST, pn0);            /* refill it with the tile ST ahead */
             pn0 = pn1; pn1 = pn2;
             pn2 = my_pos(it + ST + 3);
         }
@@ -1936,11 +1982,6 @@ q4_decode_k(const DecParams P) {
     }
     __syncthreads();
 
-    const size_t unit = (size_t)u * P.n_kvh + kh;
-    MergeOut mo;
-    mo.out = P.out; mo.part_out = P.part_out; mo.gate = P.gate;
-    mo.row0 = (size_t)u * P.n_head + (size_t)kh * P.gqa;
-    mo.gqa = P.gqa;
     float *mscr = reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES + Cfg::REC_BYTES);   /* scratch of the merges */
     /* exchange mode: the unit's last merge leaves this rank's record here instead of finalising */
     float *fin = P.xchg ? reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES) : nullptr;
@@ -1966,14 +2007,12 @@ q4_decode_k(const DecParams P) {
     }
     /* level 1: record per block; groups of DEC_GROUP blocks are merged by their last arrival,
      * level 2: the group records are merged by the last group to finish. */
-    const uint32_t n_groups = (S + DEC_GROUP - 1u) / DEC_GROUP;
     const uint32_t grp = split / DEC_GROUP;
     const uint32_t grp_size = min(DEC_GROUP, S - grp * DEC_GROUP);
-    float *rec1 = P.scratch + (unit * (size_t)(S + n_groups)) * HEADS * REC;
     if (P.gridmerge) {
         merge_records<HD, HEADS>(sm, Cfg::NPG, false, rec1 + (size_t)split * HEADS * REC, mo, mscr);
         __syncthreads();   /* the warp records in shared memory are no longer needed: their space is the scratch */
-        grid_merge<HD, HEADS>(rec1, S, split, P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP), mo, sm, P.err);
+        grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP), mo, sm, P.err);
         return;
     }
     float *rec2 = rec1 + (size_t)S * HEADS * REC;
@@ -2281,6 +2320,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         if (gm < 0) { const char *e = getenv("Q4_DEC_GRIDMERGE"); gm = e ? atoi(e) : 1; }
         p.gridmerge = (gm && !cluster && S > DEC_GROUP && !a.xchg) ? 1u : 0u;
     }
+    p.min_tiles = 4u * DEC_WARPS;
     p.xchg = a.xchg;
     p.xchg_phase = (uint32_t)a.xchg_phase;
     p.new_k = a.new_k;
