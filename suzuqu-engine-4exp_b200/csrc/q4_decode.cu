@@ -81,13 +81,16 @@ struct DecParams {
     const Q4XchgDev *xchg;   /* sequence-sharded decode: exchange window (null otherwise) */
     uint32_t xchg_phase;
     const float *new_k, *new_v;   /* fused append of the newest row (native q8_0 store), or null */
+    uint32_t early_pos, early_rows;   /* positions / rows of a dense scan may be read before the dependent-launch wait */
     uint32_t pdl;                 /* launched with programmatic stream serialization */
     uint32_t gridmerge;           /* long scans: every split's record goes to scratch, the unit's blocks meet at a counter,
                                    * and (head, 32-dim) slices of the merge are shared out among them */
-    uint32_t min_tiles;           /* with gridmerge: tiles that a block takes at least */
+    uint32_t mid_steps, mid_splits;   /* with gridmerge: a unit of fewer tiles uses this many blocks at most */
+    uint32_t small_steps;         /* with gridmerge and clusters: a unit of at most this many tiles is left to its first cluster */
     uint32_t push_bytes;          /* > 0: the launch carries this much extra shared memory and merges by pushing */
     uint32_t push_async;          /* pushes complete an mbarrier of the receiving block (its last 16 bytes) instead of
                                    * meeting at a cluster barrier */
+    uint32_t hybrid;              /* host side: cluster size wanted for a grid merge */
     uint32_t direct;              /* host side: the cache is not aligned for asynchronous copies */
     uint32_t bulk_runs;           /* tiles of 16 consecutive positions come in by one bulk copy each (else by cp.async) */
 };
@@ -620,9 +623,11 @@ __device__ __noinline__ void cluster_push_merge(const float *own, const float *r
  * checks that the grid fits in one wave), and each merges (head, 32 dims) slices of all records.  A slice is one round trip:
  * all (m, l) pairs and all accumulator pieces are requested at once, 16 record lanes x 8 threads of 4 dims (piece by
  * piece in a loop they took 7 us behind the last block at 262144 rows, 16 serial round trips).
- * `n_rec` blocks have a record; blocks without one (the launch was sized for the store's capacity, the context is short)
- * only help to merge.  The wait is bounded; the last block to leave re-arms the two counters. */
+ * `n_rec` records; every block with a record or a slice takes part (a launch sized for the store's capacity may have more
+ * blocks than a short context needs).  The last to arrive re-arms the counter and turns the flag word, so nobody meets
+ * again on the way out.  The wait is bounded. */
 constexpr uint32_t GRID_SPIN_LIMIT = 1u << 22;
+constexpr uint32_t DEC_CTR = 2u + DEC_MAX_SPLIT / DEC_GROUP;   /* words per unit: arrivals | arrivals per group | flag of the grid merge */
 template <int HD, int HEADS>
 __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t n_rec, uint32_t split, uint32_t *ctr, const MergeOut mo,
                                         float *scr /* >= 256 + 16 * 32 + 8 floats of shared memory */, uint32_t *err) {
@@ -631,15 +636,24 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
     const uint32_t tasks = mo.gqa * CH, members = min(S, max(n_rec, tasks));
     if (split >= members) return;   /* neither a record nor a slice */
     __shared__ uint32_t s_ok;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (split < n_rec) atomicAdd(&ctr[0], 1u);
-        uint32_t spins = 0, seen;
-        do {
-            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
-        } while (seen < n_rec && ++spins < GRID_SPIN_LIMIT);
-        s_ok = seen >= n_rec ? 1u : 0u;
+        uint32_t *flag = ctr + DEC_CTR - 1u;
+        uint32_t old, seen, prev;
+        asm volatile("ld.relaxed.gpu.u32 %0, [%1];" : "=r"(old) : "l"(flag) : "memory");
+        /* the block's records are ordered before this by the barrier above */
+        asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(prev) : "l"(ctr) : "memory");
+        bool met = prev == members - 1u;
+        if (met) {
+            *ctr = 0u;
+            asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(flag), "r"(old + 1u) : "memory");
+        }
+        for (uint32_t spins = 0; !met && spins < GRID_SPIN_LIMIT; spins++) {
+            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
+            met = seen != old;
+        }
+        s_ok = met ? 1u : 0u;
+        if (!met) atomicOr(err, (uint32_t)Q4E_CUDA);
     }
     __syncthreads();
     const bool ok = s_ok != 0u;
@@ -705,15 +719,6 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
             }
             __syncthreads();
         }
-    if (threadIdx.x == 0) {
-        if (!ok) atomicOr(err, (uint32_t)Q4E_CUDA);
-        __threadfence();
-        if (atomicAdd(&ctr[1], 1u) == members - 1u) {   /* everyone has passed the meeting point: ready for the next launch */
-            ctr[1] = 0u;
-            __threadfence();
-            ctr[0] = 0u;
-        }
-    }
 }
 
 /* ---- exchange of the units' records between ranks (sequence-sharded decode) --------------------
@@ -945,16 +950,23 @@ q4_decode_k(const DecParams P) {
             asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
         }
     }
-    /* Programmatic dependent launch: the blocks of this launch may already be resident while the previous
-     * kernel of the stream drains.  Only the cache view above (written when the store was created or bound)
-     * is read before this point; positions, lists, queries and rows are read after it. */
-    if (P.pdl) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        /* the next launch of the stream may bring its blocks in as slots free up (it still waits, at its
-         * own griddepcontrol.wait, for this grid to finish before it reads anything this grid writes) */
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
+    /* Programmatic dependent launch: the blocks of this launch may already be resident while the previous kernel of the
+     * stream drains.  Before this wait only the cache view is read (written when the store was created or bound) and
+     * what the host knows to be settled: the positions, and in a dense scan the rows written by earlier launches, so that
+     * the rings fill under the previous kernel's tail.  Queries, new rows, lists, scratch and outputs come after it. */
+    auto pdl_wait = [&]() {
+        if (P.pdl) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            /* the next launch of the stream may bring its blocks in as slots free up (it still waits, at its
+             * own griddepcontrol.wait, for this grid to finish before it reads anything this grid writes) */
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        }
+    };
+    constexpr bool CAN_EARLY = Cfg::STAGED || Cfg::STAGED2;
+    const bool early = CAN_EARLY && P.early_rows;   /* the wait comes behind the ring's first tiles */
+    if (!P.early_pos) pdl_wait();
     const uint32_t newest = P.pos ? (uint32_t)P.pos[P.many ? u : 0] : P.kv_base + u;
+    if (P.early_pos && !early) pdl_wait();
     uint32_t n_kv = newest + 1u;
     if (n_kv > C.max_kv) n_kv = C.max_kv;
     const int32_t *list = P.idx ? P.idx + (size_t)u * P.idx_unit_stride + (size_t)kh * P.idx_kvh_stride
@@ -962,7 +974,10 @@ q4_decode_k(const DecParams P) {
     const uint32_t n_pos = list ? P.width : n_kv;
     const uint32_t steps = (n_pos + 15u) >> 4;
     /* a launch sized for the store's capacity (position from the device) uses as many of its blocks as the context needs */
-    const uint32_t S_act = P.gridmerge ? min(S, max((steps + P.min_tiles - 1u) / P.min_tiles, 1u)) : S;
+    uint32_t S_act = P.gridmerge ? (steps <= 4u * DEC_WARPS ? 1u : min(steps < P.mid_steps ? P.mid_splits : S, (steps + DEC_WARPS - 1u) / DEC_WARPS)) : S;
+    const bool hybrid = P.gridmerge && P.cluster;
+    const bool in_cluster = P.cluster && (!hybrid || steps <= P.small_steps);   /* the unit's splits are one cluster */
+    if (hybrid) S_act = in_cluster ? P.cluster : (S_act + P.cluster - 1u) / P.cluster * P.cluster;
     const uint32_t per = (steps + S_act - 1u) / S_act;
     const uint32_t s_begin = split * per;
     const uint32_t s_end = min(s_begin + per, steps);
@@ -986,7 +1001,10 @@ q4_decode_k(const DecParams P) {
     const uint32_t n_groups = (S + DEC_GROUP - 1u) / DEC_GROUP;
     float *rec1 = P.scratch + (unit * (size_t)(S + n_groups)) * HEADS * REC;
     if (P.gridmerge && split >= S_act) {
-        grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP), mo, reinterpret_cast<float *>(smem_raw), P.err);
+        if (early) pdl_wait();
+        if (hybrid) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (!in_cluster && S_act > 1u)
+            grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * DEC_CTR, mo, reinterpret_cast<float *>(smem_raw), P.err);
         return;
     }
 
@@ -997,7 +1015,7 @@ q4_decode_k(const DecParams P) {
     float4 ap_x = make_float4(0.f, 0.f, 0.f, 0.f);
     bool ap_which = false, ap_live = false;
     uint32_t ap_b = 0, ap_sub = 0;
-    if constexpr (Cfg::STAGED || Cfg::STAGED2) {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
+    auto load_new = [&]() {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
         if (P.new_k) {
             constexpr uint32_t QL = HD / 4;
             const uint32_t tid = threadIdx.x;
@@ -1010,6 +1028,9 @@ q4_decode_k(const DecParams P) {
                 ap_x = *reinterpret_cast<const float4 *>((ap_which ? P.new_v : P.new_k) +
                                                          ((size_t)u * P.n_kvh + kh) * HD + ap_b * 32 + ap_sub * 4);
         }
+    };
+    if constexpr (CAN_EARLY) {
+        if (!early) load_new();
     }
 
     /* position j of the list / range, or -1 (padding, out of range) */
@@ -1296,6 +1317,23 @@ q4_decode_k(const DecParams P) {
             }
             cp_async_commit();   /* one group per tile, empty or not, keeps the wait count uniform */
         };
+        int32_t pa, pb, pc, pd, pn0, pn1, pn2;
+        bool hold = false;
+        auto first_positions = [&]() {
+            pa = my_pos(0); pb = my_pos(1); pc = my_pos(2); pd = my_pos(3);
+            pn0 = my_pos(4); pn1 = my_pos(5); pn2 = my_pos(6);
+            if (P.new_k) {
+                const int32_t nw = (int32_t)newest;
+                hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
+            }
+        };
+        auto fill = [&]() { issue(0, pa); issue(1, pb); issue(2, pc); issue(3, pd); };
+        if (early) {
+            first_positions();
+            if (!hold) fill();
+            pdl_wait();
+            load_new();
+        }
         /* ---- queries: the raw values are requested now, next to the list entries, and converted after the ring
          * has been filled (lane (g, t) takes dims 16ks + 4t .. + 3 of head nt*8 + g) */
         uint32_t qraw[NW][KS][4];
@@ -1319,18 +1357,12 @@ q4_decode_k(const DecParams P) {
                 }
             }
         }
-        int32_t pa = my_pos(0), pb = my_pos(1), pc = my_pos(2), pd = my_pos(3);
-        int32_t pn0 = my_pos(4), pn1 = my_pos(5), pn2 = my_pos(6);
+        if (!early) first_positions();
         /* ---- fused append, second half.  Every split of the unit quantises and stores the unit's newest row
          * (identical bytes from every split, so no block depends on another having written); a block's own
-         * store is ordered before its later reads by the barrier.  A warp whose first tiles do not name the
+         * store is ordered before its later reads by the barrier.  A warp whose first four tiles do not name the
          * newest row fills its ring before that, so the append runs under the first copies. */
-        bool hold = false;
-        if (P.new_k) {
-            const int32_t nw = (int32_t)newest;
-            hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
-        }
-        if (!hold) { issue(0, pa); issue(1, pb); issue(2, pc); issue(3, pd); }
+        if (!early && !hold) fill();
         if (P.new_k) {
             float d, id;
             q4d_block_scale(ap_x, d, id);
@@ -1343,7 +1375,7 @@ q4_decode_k(const DecParams P) {
             if (P.bulk_runs) asm volatile("fence.proxy.async;" ::: "memory");   /* the row may be read back by the bulk-copy engine */
             __syncthreads();
         }
-        if (hold) { issue(0, pa); issue(1, pb); issue(2, pc); issue(3, pd); }
+        if (hold) fill();
 
         /* Q fragments as fp16 (exact for bf16 queries; scale * log2(e) multiplies the scores in fp32 later):
          * lane (g, t) holds dims 16ks + 4t .. + 3 of head nt*8 + g, the columns the K fragments below carry in
@@ -1630,20 +1662,28 @@ q4_decode_k(const DecParams P) {
                     qs[ks][half] = pack_h2(x.x, x.y);
                 }
         };
-        int32_t pf[ST];
-#pragma unroll
-        for (int i = 0; i < ST; i++) pf[i] = my_pos(i);
-        int32_t pn0 = my_pos(ST), pn1 = my_pos(ST + 1), pn2 = my_pos(ST + 2);
+        int32_t pf[ST], pn0, pn1, pn2;
         /* fused append, second half (see the hd-128 path): a group whose first tiles name the newest row waits for it */
         bool hold = false;
-        if (P.new_k) {
+        auto first_positions = [&]() {
 #pragma unroll
-            for (int i = 0; i < ST; i++) hold = hold || pf[i] == (int32_t)newest;
-            hold = __any_sync(0xffffffffu, hold);
-        }
-        if (!hold) {
+            for (int i = 0; i < ST; i++) pf[i] = my_pos(i);
+            pn0 = my_pos(ST); pn1 = my_pos(ST + 1); pn2 = my_pos(ST + 2);
+            if (P.new_k) {
+#pragma unroll
+                for (int i = 0; i < ST; i++) hold = hold || pf[i] == (int32_t)newest;
+                hold = __any_sync(0xffffffffu, hold);
+            }
+        };
+        auto fill = [&]() {
 #pragma unroll
             for (int i = 0; i < ST; i++) issue(i, pf[i]);
+        };
+        first_positions();
+        if (!hold) fill();
+        if (early) {
+            pdl_wait();
+            load_new();
         }
         if (LAY != LAY_Q8R && P.new_k) {
             uint8_t *row = const_cast<uint8_t *>(ap_which ? vbase : kbase) + (uint64_t)newest * tok_stride;
@@ -1663,10 +1703,7 @@ q4_decode_k(const DecParams P) {
             if (newest >= max_kv && threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
             __syncthreads();
         }
-        if (hold) {
-#pragma unroll
-            for (int i = 0; i < ST; i++) issue(i, pf[i]);
-        }
+        if (hold) fill();
         load_q();
         for (uint32_t it = 0; it < n_my; it++) {
             cp_async_wait<HALVES ? 1 : ST - 1>();    /* all but the newest ST - 1 tiles (the V rows) have landed: this warp's part of tile `it` is in */
@@ -1985,23 +2022,24 @@ q4_decode_k(const DecParams P) {
     float *mscr = reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES + Cfg::REC_BYTES);   /* scratch of the merges */
     /* exchange mode: the unit's last merge leaves this rank's record here instead of finalising */
     float *fin = P.xchg ? reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES) : nullptr;
-    if (S == 1) {
+    if (S_act == 1) {
+        if (hybrid) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         merge_records<HD, HEADS>(sm, Cfg::NPG, false, fin, mo, mscr);
         if (fin) xchg_finish<HD, HEADS>(P.xchg, P.xchg_phase, (uint32_t)unit, fin, mo, P.err);
         return;
     }
-    if (P.cluster) {
+    if (in_cluster) {
         float *own = reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES);
         merge_records<HD, HEADS>(sm, Cfg::NPG, false, own, mo, mscr);
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   /* every peer block has started (arrive at entry) */
         if (P.push_bytes) {
-            cluster_push_merge<HD, HEADS>(own, reinterpret_cast<const float *>(smem_raw + Cfg::SMEM), S, cluster_ctarank(), mo,
+            cluster_push_merge<HD, HEADS>(own, reinterpret_cast<const float *>(smem_raw + Cfg::SMEM), P.cluster, cluster_ctarank(), mo,
                                           P.push_async ? (uint32_t)__cvta_generic_to_shared(smem_raw + Cfg::SMEM + P.push_bytes - 16u) : 0u,
                                           P.err);
             return;
         }
         cluster_sync_all();
-        cluster_merge<HD, HEADS>((uint32_t)__cvta_generic_to_shared(own), S, cluster_ctarank(), mo);
+        cluster_merge<HD, HEADS>((uint32_t)__cvta_generic_to_shared(own), P.cluster, cluster_ctarank(), mo);
         cluster_sync_all();
         return;
     }
@@ -2012,11 +2050,12 @@ q4_decode_k(const DecParams P) {
     if (P.gridmerge) {
         merge_records<HD, HEADS>(sm, Cfg::NPG, false, rec1 + (size_t)split * HEADS * REC, mo, mscr);
         __syncthreads();   /* the warp records in shared memory are no longer needed: their space is the scratch */
-        grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP), mo, sm, P.err);
+        if (hybrid) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * DEC_CTR, mo, sm, P.err);
         return;
     }
     float *rec2 = rec1 + (size_t)S * HEADS * REC;
-    uint32_t *ctr = P.counters + unit * (1u + DEC_MAX_SPLIT / DEC_GROUP);
+    uint32_t *ctr = P.counters + unit * DEC_CTR;
     /* one call site for every level keeps a single copy of the merge code in the kernel */
     const float *src = sm;
     uint32_t count = Cfg::NPG;
@@ -2090,8 +2129,9 @@ bool launch(const DecParams &p_in, dim3 grid) {
         (void)cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
     attr_done = true;
+    using Cfg = DecCfg<LAY, HD, NHT, DIRECT>;
     DecParams p = p_in;
-    const uint64_t blocks = (uint64_t)grid.x * grid.y * grid.z;
+    auto n_blocks = [&]() -> uint64_t { return (uint64_t)grid.x * grid.y * grid.z; };
     /* how many clusters of this shape can be resident at once with `bytes` of dynamic shared memory per block */
     auto resident_clusters = [&](size_t bytes) -> uint64_t {
         static size_t c_bytes[4];
@@ -2101,7 +2141,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
             if (c_bytes[i] == bytes && c_cluster[i] == p.cluster) return (uint64_t)c_n[i];
         cudaLaunchConfig_t qc;
         memset(&qc, 0, sizeof(qc));
-        qc.gridDim = grid;
+        qc.gridDim = dim3(p.cluster, grid.y, grid.z);
         qc.blockDim = dim3(DEC_THREADS);
         qc.dynamicSmemBytes = bytes;
         cudaLaunchAttribute qa[1];
@@ -2123,7 +2163,23 @@ bool launch(const DecParams &p_in, dim3 grid) {
     /* The push merge needs extra shared memory; it is used only if that leaves the grid in one wave.
      * (Asking for still more shared memory, so that a shallow grid spreads one or two blocks deep over all
      * SMs instead of three deep over some, was measured: no gain at 1-8 sessions, 3 us slower at 16.) */
-    if (p.push_bytes && resident_clusters(smem_base + p.push_bytes) < blocks / p.cluster) p.push_bytes = 0;
+    if (p.gridmerge && p.hybrid) {
+        p.cluster = p.hybrid;
+        p.push_bytes = (p.gqa + p.cluster - 1u) / p.cluster * p.cluster * (HD + 4u) * (uint32_t)sizeof(float) + 16u;
+        const uint64_t n = resident_clusters(smem_base + p.push_bytes);
+        const uint32_t fit = (uint32_t)(n / (grid.y * grid.z)) * p.cluster;
+        /* only where the receive area costs no block per SM and nearly all splits fit; the first cluster takes up to four
+         * tiles per warp (three of fp32), where it meets the other form (2048 rows of q8_0: 7.0 against 7.8 us) */
+        if (n == resident_clusters(smem_base) && 4u * fit >= 3u * grid.x && Cfg::NPG == DEC_WARPS) {
+            p.push_async = 1u;
+            grid.x = min(grid.x / p.cluster * p.cluster, fit);
+            p.S = grid.x;
+            p.small_steps = (LAY == LAY_F32 ? 3u : 4u) * p.cluster * DEC_WARPS;
+        } else {
+            p.cluster = p.push_bytes = 0;
+        }
+    }
+    if (!p.gridmerge && p.push_bytes && resident_clusters(smem_base + p.push_bytes) < n_blocks() / p.cluster) p.push_bytes = 0;
     if (!p.push_bytes) p.push_async = 0;
     if (p.gridmerge) {
         /* the blocks of a unit wait for one another: only when the whole grid is resident at once */
@@ -2132,7 +2188,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
             (void)cudaGetLastError();
             occ = 0;
         }
-        if (blocks > (uint64_t)occ * (uint64_t)g_q4.sm_count) p.gridmerge = 0;
+        if (n_blocks() > (uint64_t)occ * (uint64_t)g_q4.sm_count) p.gridmerge = 0;
     }
     const size_t smem = smem_base + p.push_bytes;
     cudaLaunchConfig_t cfg;
@@ -2222,7 +2278,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         if (!a.idx && a.n_units > 1) S = S > (steps + 63u) / 64u ? S : (steps + 63u) / 64u;
         /* every warp keeps at least one tile of a list, four of a dense scan (measured at 16384 / 32768 rows:
          * 12.0 / 14.6 us per layer against 13.5 / 15.4 with one tile per warp; no difference from 49152 rows on) */
-        const uint32_t per_block = (a.idx || a.xchg) ? DEC_WARPS : 4u * DEC_WARPS;   /* the exchange form merges in two levels: finer splits serve it better (8 ranks x 32768 rows: 24.7 against 26.0 us) */
+        const uint32_t per_block = (a.idx || a.xchg) ? DEC_WARPS : (gqa > 8 ? 2u : 4u) * DEC_WARPS;   /* the exchange form merges in two levels: finer splits serve it better (8 ranks x 32768 rows: 24.7 against 26.0 us) */
         const uint32_t cap = (steps + per_block - 1u) / per_block;
         if (S > cap) S = cap;
     }
@@ -2260,7 +2316,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
     }
     const uint32_t n_groups = (S + DEC_GROUP - 1u) / DEC_GROUP;
     const size_t need_part = (size_t)units * (S + n_groups) * heads * (a.hd + 4);
-    const size_t need_ctr = (size_t)units * (1u + DEC_MAX_SPLIT / DEC_GROUP);
+    const size_t need_ctr = (size_t)units * DEC_CTR;
     float *scratch = a.scratch_part;
     uint32_t *counters = a.scratch_counters;
     if (scratch) {
@@ -2320,16 +2376,30 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         if (gm < 0) { const char *e = getenv("Q4_DEC_GRIDMERGE"); gm = e ? atoi(e) : 1; }
         p.gridmerge = (gm && !cluster && S > DEC_GROUP && !a.xchg) ? 1u : 0u;
     }
-    p.min_tiles = 4u * DEC_WARPS;
+    /* Up to 131072 rows two blocks per SM do better than three: the next launch's blocks find room and fill their rings
+     * under this one's tail (65536 / 100003 / 262144 rows of q8_0: 15.6 / 19.9 / 37.8 against 17.2 / 20.6 / 33.5 us).
+     * With two warps to a tile (more than 8 heads) three blocks are always better. */
+    p.mid_steps = gqa > 8 ? 0u : 8192u;
+    p.mid_splits = (uint32_t)g_q4.sm_count * 2u / units;
+    if (p.mid_splits > S) p.mid_splits = S;
+    if (p.mid_splits < 1u) p.mid_splits = 1u;
+    /* Where the launch is sized for a capacity and the context may be short, a grid merge's blocks come in clusters of 8, of
+     * which a short context uses the first alone, merging through distributed shared memory (777 rows in a store of 32768:
+     * 5.4 against 7.0 us).  Long scans lose 3 to 6 % by it (the next launch's blocks come in eight at a time), so large
+     * stores do without. */
+    p.hybrid = p.gridmerge && use_cluster && a.pos && !a.scratch_part && steps <= 2048u ? 8u : 0u;
     p.xchg = a.xchg;
     p.xchg_phase = (uint32_t)a.xchg_phase;
     p.new_k = a.new_k;
     p.new_v = a.new_v;
+    p.early_pos = a.early_pos ? 1u : 0u;
+    p.early_rows = p.early_pos && a.early_rows && !a.idx && a.layout != LAY_Q8R && a.hd >= 128 ? 1u : 0u;
     {
         /* Q4_DEC_PDL=0 switches programmatic dependent launch off */
         static int pdl = -1;
         if (pdl < 0) { const char *e = getenv("Q4_DEC_PDL"); pdl = e ? atoi(e) : 1; }
         p.pdl = pdl ? 1u : 0u;
+        if (!p.pdl) p.early_pos = p.early_rows = 0u;
     }
     if (a.new_k || a.new_v)
         Q4_REQUIRE(a.new_k && a.new_v && a.layout != LAY_Q8R && a.hd >= 128,
@@ -2337,10 +2407,10 @@ bool q4i_decode(const Q4DecodeArgs &a) {
     p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
     dim3 grid(S, a.n_kvh, a.n_units);
     switch (a.layout) {
-    case LAY_F32: return launch_hd<LAY_F32>(p, grid, a.hd);
-    case LAY_F16: return launch_hd<LAY_F16>(p, grid, a.hd);
-    case LAY_Q8P: return launch_hd<LAY_Q8P>(p, grid, a.hd);
-    case LAY_Q8R: return launch_hd<LAY_Q8R>(p, grid, a.hd);
+    case LAY_F32: return q4i_launched(launch_hd<LAY_F32>(p, grid, a.hd));
+    case LAY_F16: return q4i_launched(launch_hd<LAY_F16>(p, grid, a.hd));
+    case LAY_Q8P: return q4i_launched(launch_hd<LAY_Q8P>(p, grid, a.hd));
+    case LAY_Q8R: return q4i_launched(launch_hd<LAY_Q8R>(p, grid, a.hd));
     }
     return q4i_fail(Q4E_ARG, "decode: bad layout");
 }
@@ -2377,7 +2447,7 @@ extern "C" bool q4_gpu_lse_merge(const float *parts, uint32_t n_parts, uint32_t 
  * library holds these 4 MB + 272 B until the process exits.  The names below are host-side stand-ins
  * in host code; the device addresses come from cudaGetSymbolAddress, once per device. */
 constexpr size_t Q4_STATIC_PART_FLOATS = (size_t)1 << 20;   /* 4 MB of records */
-constexpr size_t Q4_STATIC_COUNTERS = 4 * (1 + DEC_MAX_SPLIT / DEC_GROUP);   /* up to 4 kv heads */
+constexpr size_t Q4_STATIC_COUNTERS = 4 * DEC_CTR;   /* up to 4 kv heads */
 static __device__ __align__(256) float q4_static_part[Q4_STATIC_PART_FLOATS];
 static __device__ __align__(256) uint32_t q4_static_counters[Q4_STATIC_COUNTERS];
 

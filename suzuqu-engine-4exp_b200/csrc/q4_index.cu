@@ -296,7 +296,7 @@ bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n
     const uint64_t tiles = (uint64_t)((n_blocks + SM_COLS - 1u) / SM_COLS) * ((n_tok + SM_TOK - 1u) / SM_TOK);
     const uint32_t grid = (uint32_t)(tiles < (uint64_t)g_q4.sm_count ? tiles : (uint64_t)g_q4.sm_count);
     q4_ix_score_mt_k<<<grid, SM_THREADS, SM_SMEM, g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
-    return q4i_check(cudaGetLastError(), "qsa_score launch");
+    return q4i_launched(q4i_check(cudaGetLastError(), "qsa_score launch"));
 }
 bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
                   uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp,
@@ -326,8 +326,8 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = ix_pdl() ? 1 : 0;
-    return q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr),
-                     "qsa_score launch");
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr),
+                     "qsa_score launch"));
 }
 
 /* ---- selection: one block per token */
@@ -984,7 +984,7 @@ bool topk_start(K kernel, dim3 grid, uint32_t threads, size_t smem, uint32_t clu
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
-    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "qsa_topk launch");
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "qsa_topk launch"));
 }
 template <uint32_t NB>
 bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stride, uint32_t k_blk, uint32_t ratio, uint32_t pos0,
@@ -1004,7 +1004,7 @@ bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
                  uint32_t pos0, uint32_t width, const int32_t *pp, const int32_t *pos_arr = nullptr) {
     if (stride > TKC_MAX_ROW) {
         q4_ix_topk1_k<<<n_tok, IX_TK_THREADS, 0, g_q4.stream>>>(score, sel, stride, k_blk, ratio, pos0, width, pp, pos_arr);
-        return q4i_check(cudaGetLastError(), "qsa_topk launch");
+        return q4i_launched(q4i_check(cudaGetLastError(), "qsa_topk launch"));
     }
     if (stride <= TKC_KEYS) return topkc_start<1>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
     const uint32_t nb = stride <= 2 * TKC_KEYS ? 2u : stride <= 4 * TKC_KEYS ? 4u : 8u;
@@ -1031,13 +1031,13 @@ extern "C" bool q4_hip_qsa_pool(const void *raw_f16, float *pool, const float *w
     if (!g_q4.ok || !raw_f16 || !pool || b1 <= b0 || hd != IX_HD || ratio == 0) return false;
     q4_ix_pool_k<<<(b1 - b0 + 3u) / 4u, 128, 0, g_q4.stream>>>((const __half *)raw_f16, pool, wn, ratio, b0, b1, n_rot,
                                                              rope_base, eps, nullptr);
-    return q4i_check(cudaGetLastError(), "qsa_pool launch");
+    return q4i_launched(q4i_check(cudaGetLastError(), "qsa_pool launch"));
 }
 extern "C" bool q4_hip_qsa_pool_d(const void *raw, float *pool, const float *wn, uint32_t hd, uint32_t ratio,
                                   uint32_t n_rot, float rope_base, float eps) {
     if (!g_q4.ok || !g_q4.pos_d || !raw || !pool || hd != IX_HD || ratio == 0) return false;
     q4_ix_pool_k<<<1, 128, 0, g_q4.stream>>>((const __half *)raw, pool, wn, ratio, 0, 0, n_rot, rope_base, eps, g_q4.pos_d);
-    return q4i_check(cudaGetLastError(), "qsa_pool_d launch");
+    return q4i_launched(q4i_check(cudaGetLastError(), "qsa_pool_d launch"));
 }
 extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks,
                                  uint32_t stride, uint32_t n_head, uint32_t hd, uint32_t pos0, uint32_t ratio) {

@@ -38,6 +38,7 @@ struct q4_gpu_kv {
     uint32_t rec_bytes;          /* bytes per (kv head, position): q8_0 record, or fp16 / fp32 row */
     Q4Cache view;                /* host copy of the kernel view */
     Q4Cache *d_view;             /* same, in device memory (for batched launches) */
+    uint64_t *written;           /* per layer: g_q4.launches when its rows were last written */
 };
 
 /* runtime state (q4_runtime.cu) */
@@ -50,6 +51,12 @@ struct Q4State {
     uint32_t *err_d;             /* device-side sticky error bits */
     uint32_t err_h;
     uint32_t last_graph_nodes;
+    /* What a kernel may read before it has waited for its predecessor in the stream (programmatic dependent launch).
+     * Every kernel of the library either starts after its predecessor has finished, or waits for that before it lets its
+     * successor start.  So what was written at least one library launch earlier is complete when a kernel starts:
+     * `launches` counts them, the position word and the rows of a store remember the count at their last write, and
+     * `unsettled` is the count at the last event behind which nothing is known (a graph launch, another stream). */
+    uint64_t launches, pos_written, unsettled;
     /* attention scratch: split-KV partial records + per-unit arrival counters */
     float *part;
     size_t part_floats;
@@ -60,6 +67,12 @@ extern Q4State g_q4;
 
 bool q4i_fail(uint32_t bit, const char *what);
 bool q4i_check(cudaError_t e, const char *what);
+inline bool q4i_launched(bool ok) {
+    if (ok) g_q4.launches++;
+    return ok;
+}
+inline bool q4i_settled(uint64_t written) { return g_q4.launches > written && g_q4.launches > g_q4.unsettled; }
+inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->written[layer] = g_q4.launches; }
 bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside capture, fails inside */
 
 #define Q4_REQUIRE(cond, what)                    \
@@ -154,6 +167,7 @@ struct Q4DecodeArgs {
     /* fused append (native q8_0 store only): the new K and V rows [unit][n_kvh*hd] (fp32) are quantised
      * and stored at each unit's position by the attention kernel itself before it reads the cache */
     const float *new_k, *new_v;
+    int early_pos, early_rows;   /* the positions / the rows of a dense scan are settled (q4i_settled) */
 };
 bool q4i_decode(const Q4DecodeArgs &a);
 

@@ -195,7 +195,7 @@ bool launch_append(const AppendParams &p, int layout) {
     case LAY_F16: q4_append_k<LAY_F16><<<grid, 256, 0, g_q4.stream>>>(p); break;
     default: q4_append_k<LAY_F32><<<grid, 256, 0, g_q4.stream>>>(p); break;
     }
-    return q4i_check(cudaGetLastError(), "append launch");
+    return q4i_launched(q4i_check(cudaGetLastError(), "append launch"));
 }
 
 }  // namespace
@@ -339,6 +339,9 @@ extern "C" q4_gpu_kv *q4_gpu_kv_create(uint32_t n_layers, uint32_t n_kvh, uint32
     }
     q4_gpu_kv *kv = (q4_gpu_kv *)calloc(1, sizeof(q4_gpu_kv));
     if (!kv) return nullptr;
+    kv->written = (uint64_t *)calloc(n_layers, sizeof(uint64_t));
+    if (!kv->written) { free(kv); return nullptr; }
+    for (uint32_t i = 0; i < n_layers; i++) q4i_kv_written(kv, i);
     kv->n_layers = n_layers; kv->n_kvh = n_kvh; kv->hd = hd; kv->max_kv = max_kv; kv->kind = kind;
     /* q8_0: one record per (kv head, position) = K codes | V codes | K scales | V scales, so a gathered
      * position is one contiguous 272-byte read (hd 128) instead of three scattered ones.  fp16 / fp32:
@@ -382,6 +385,7 @@ extern "C" void q4_gpu_kv_destroy(q4_gpu_kv *kv) {
     if (kv->k) cudaFree(kv->k);
     if (kv->v && kv->kind != Q4K_Q8) cudaFree(kv->v);   /* q8_0: v and s point into the k allocation */
     if (kv->d_view) cudaFree(kv->d_view);
+    free(kv->written);
     free(kv);
 }
 
@@ -394,7 +398,9 @@ extern "C" bool q4_gpu_kv_append(q4_gpu_kv *kv, uint32_t layer, const float *k, 
     memset(&p, 0, sizeof(p));
     p.one = kv->view; p.layer = layer; p.n_rows = n_tok; p.n_kvh = kv->n_kvh; p.hd = kv->hd;
     p.k = k; p.v = v; p.pos0 = pos0; p.err = g_q4.err_d;
-    return launch_append(p, store_layout(kv->kind));
+    const bool ok = launch_append(p, store_layout(kv->kind));
+    q4i_kv_written(kv, layer);
+    return ok;
 }
 extern "C" bool q4_gpu_kv_append_d(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_append_d: library not initialised");
@@ -403,7 +409,9 @@ extern "C" bool q4_gpu_kv_append_d(q4_gpu_kv *kv, uint32_t layer, const float *k
     memset(&p, 0, sizeof(p));
     p.one = kv->view; p.layer = layer; p.n_rows = 1; p.n_kvh = kv->n_kvh; p.hd = kv->hd;
     p.k = k; p.v = v; p.pos = g_q4.pos_d; p.err = g_q4.err_d;
-    return launch_append(p, store_layout(kv->kind));
+    const bool ok = launch_append(p, store_layout(kv->kind));
+    q4i_kv_written(kv, layer);
+    return ok;
 }
 
 template <bool TO_REF>
@@ -424,7 +432,9 @@ static bool relayout(const q4_gpu_kv *kv, uint32_t layer, int which, uint32_t to
         q4_relayout_k<LAY_F32, TO_REF><<<grid, 256, 0, g_q4.stream>>>(kv->view, layer, which, kv->n_kvh, kv->hd, tok0, n_tok, (uint8_t *)ref);
         break;
     }
-    return q4i_check(cudaGetLastError(), "kv relayout launch");
+    const bool ok = q4i_launched(q4i_check(cudaGetLastError(), "kv relayout launch"));
+    if (!TO_REF) q4i_kv_written(const_cast<q4_gpu_kv *>(kv), layer);
+    return ok;
 }
 extern "C" bool q4_gpu_kv_export(const q4_gpu_kv *kv, uint32_t layer, int which, uint32_t tok0, uint32_t n_tok, void *dst) {
     return relayout<true>(kv, layer, which, tok0, n_tok, dst);
@@ -484,6 +494,8 @@ static bool snapshot(const q4_gpu_kv *kv, uint32_t n_kv, void *buf, int host, bo
         }
         b += width * height;
     }
+    if (!save)
+        for (uint32_t i = 0; i < kv->n_layers; i++) q4i_kv_written(const_cast<q4_gpu_kv *>(kv), i);
     return true;
 }
 extern "C" bool q4_gpu_kv_save(const q4_gpu_kv *kv, uint32_t n_kv, void *buf, int host) {
@@ -525,6 +537,8 @@ static bool store_decode(const q4_gpu_kv *kv, uint32_t layer, const void *q, int
     }
     a.idx_bound_nkv = 1;
     a.scale = scale;
+    a.early_pos = !a.pos || q4i_settled(g_q4.pos_written);
+    a.early_rows = q4i_settled(kv->written[layer]);
     return q4i_decode(a);
 }
 extern "C" bool q4_gpu_kv_decode(const q4_gpu_kv *kv, uint32_t layer, const void *q, int q_bf16, const float *gate,
@@ -581,6 +595,7 @@ struct q4_gpu_batch {
     int32_t *pos_d, *pos_h;       /* pos_h: pinned ring of 8 uploads, each slot guarded by an event */
     cudaEvent_t pos_ev[8];
     uint32_t ring, max_pos;
+    uint64_t pos_written;         /* g_q4.launches when pos_d was last written */
 };
 
 extern "C" q4_gpu_batch *q4_gpu_batch_create(uint32_t max_sessions) {
@@ -645,6 +660,7 @@ extern "C" bool q4_gpu_batch_set_pos(q4_gpu_batch *b, const int32_t *pos, uint32
     }
     b->max_pos = mx;
     b->n_active = n_sessions;
+    b->pos_written = g_q4.launches;
     return q4i_check(cudaMemcpyAsync(b->pos_d, h, sizeof(int32_t) * n_sessions, cudaMemcpyHostToDevice, g_q4.stream),
                      "batch_set_pos upload") &&
            q4i_check(cudaEventRecord(b->pos_ev[slot], g_q4.stream), "batch_set_pos event");
@@ -660,8 +676,18 @@ extern "C" bool q4_gpu_batch_advance(q4_gpu_batch *b, int32_t delta) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_advance: library not initialised");
     Q4_REQUIRE(b && b->n_active, "batch_advance: no positions published (q4_gpu_batch_set_pos)");
     q4_batch_advance_k<<<(b->n_active + 127u) / 128u, 128, 0, g_q4.stream>>>(b->pos_d, b->n_active, delta);
+    b->pos_written = ++g_q4.launches;
     if (!g_q4.capturing) b->max_pos = (uint32_t)((int64_t)b->max_pos + delta < 0 ? 0 : (int64_t)b->max_pos + delta);
     return q4i_check(cudaGetLastError(), "batch_advance launch");
+}
+static void batch_written(q4_gpu_batch *b, uint32_t layer) {
+    for (uint32_t i = 0; i < b->n_active; i++)
+        if (b->kv[i]) q4i_kv_written(b->kv[i], layer);
+}
+static void batch_early(const q4_gpu_batch *b, uint32_t layer, Q4DecodeArgs &a) {
+    a.early_pos = q4i_settled(b->pos_written);
+    a.early_rows = 1;
+    for (uint32_t i = 0; i < b->n_active && a.early_rows; i++) a.early_rows = b->kv[i] && q4i_settled(b->kv[i]->written[layer]);
 }
 extern "C" bool q4_gpu_batch_append(q4_gpu_batch *b, uint32_t layer, const float *k, const float *v) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_append: library not initialised");
@@ -671,7 +697,9 @@ extern "C" bool q4_gpu_batch_append(q4_gpu_batch *b, uint32_t layer, const float
     memset(&p, 0, sizeof(p));
     p.many = b->d_views; p.layer = layer; p.n_rows = b->n_active; p.n_kvh = b->kv[0]->n_kvh; p.hd = b->kv[0]->hd;
     p.k = k; p.v = v; p.pos = b->pos_d; p.err = g_q4.err_d;
-    return launch_append(p, store_layout(b->kv[0]->kind));
+    const bool ok = launch_append(p, store_layout(b->kv[0]->kind));
+    batch_written(b, layer);
+    return ok;
 }
 extern "C" bool q4_gpu_batch_decode(q4_gpu_batch *b, uint32_t layer, const void *q, int q_bf16, const float *gate,
                                     float *out, const int32_t *idx, uint32_t width, uint32_t idx_kvh_stride,
@@ -694,6 +722,7 @@ extern "C" bool q4_gpu_batch_decode(q4_gpu_batch *b, uint32_t layer, const void 
     a.hint_rows = b->max_pos + 1;
     a.idx_bound_nkv = 1;
     a.scale = scale;
+    batch_early(b, layer, a);
     return q4i_decode(a);
 }
 
@@ -724,7 +753,10 @@ extern "C" bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, cons
     a.idx_bound_nkv = 1;
     a.scale = scale;
     if (fused) { a.new_k = k; a.new_v = v; }
-    return q4i_decode(a);
+    batch_early(b, layer, a);
+    const bool ok = q4i_decode(a);
+    if (fused) batch_written(b, layer);
+    return ok;
 }
 /* Single session, position from the device position word (graph-captured decode). */
 extern "C" bool q4_gpu_kv_append_decode_d(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, const void *q,
@@ -750,5 +782,9 @@ extern "C" bool q4_gpu_kv_append_decode_d(q4_gpu_kv *kv, uint32_t layer, const f
     a.idx_bound_nkv = 1;
     a.scale = scale;
     if (fused) { a.new_k = k; a.new_v = v; }
-    return q4i_decode(a);
+    a.early_pos = q4i_settled(g_q4.pos_written);
+    a.early_rows = q4i_settled(kv->written[layer]);
+    const bool ok = q4i_decode(a);
+    if (fused) q4i_kv_written(kv, layer);
+    return ok;
 }

@@ -779,7 +779,7 @@ bool pf_start(K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prefill launch");
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prefill launch"));
 }
 template <int HD, int NQ, int KP>
 bool attend(const PrefillParams &p, dim3 grid) {

@@ -168,7 +168,7 @@ bool prep_start(K kernel, dim3 grid, uint32_t threads, A... args) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prep launch");
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prep launch"));
 }
 /* false in `done` where the head size or an address is not the warp form's */
 template <bool SPLIT>
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_append_rows_k(const P
     }
 }
 
-bool prep_append(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, const float *wn, uint32_t n_rot,
+bool prep_append_launch(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, const float *wn, uint32_t n_rot,
                  float base, float eps, const int32_t *pos_dev, int32_t pos0, uint32_t n_tok) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_prep_append: library not initialised");
     Q4_REQUIRE(kv && k && v && n_tok && layer < kv->n_layers && n_rot <= kv->hd && !(n_rot & 1), "kv_prep_append: bad argument");
@@ -356,6 +356,13 @@ bool prep_append(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, 
                              : prep_start(q4_prep_append_rows_k<256>, dim3(n_tok), PREP_WARPS * 32u, p);
     q4_prep_append_k<<<dim3(kv->n_kvh, n_tok, 2), 128, 0, g_q4.stream>>>(p);
     return q4i_check(cudaGetLastError(), "kv_prep_append launch");
+}
+
+bool prep_append(q4_gpu_kv *kv, uint32_t layer, const float *k, const float *v, const float *wn, uint32_t n_rot,
+                 float base, float eps, const int32_t *pos_dev, int32_t pos0, uint32_t n_tok) {
+    const bool ok = prep_append_launch(kv, layer, k, v, wn, n_rot, base, eps, pos_dev, pos0, n_tok);
+    if (kv && layer < kv->n_layers) q4i_kv_written(kv, layer);
+    return ok;
 }
 
 }  // namespace

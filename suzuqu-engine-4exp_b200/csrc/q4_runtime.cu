@@ -110,6 +110,7 @@ extern "C" bool q4_gpu_set_stream(void *s) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "set_stream: library not initialised");
     if (g_q4.capturing) return q4i_fail(Q4E_ARG, "set_stream: a capture is open");
     g_q4.stream = s ? (cudaStream_t)s : g_q4.own_stream;
+    g_q4.unsettled = g_q4.launches;
     return true;
 }
 extern "C" const int32_t *q4_gpu_pos_word(void) { return g_q4.pos_d; }
@@ -228,6 +229,7 @@ __global__ void q4_set_word_k(int32_t *dst, int32_t v) { *dst = v; }
 extern "C" void q4_hip_pos_push(int32_t pos) {
     if (!g_q4.ok) return;
     q4_set_word_k<<<1, 1, 0, g_q4.stream>>>(g_q4.pos_d, pos);
+    g_q4.pos_written = ++g_q4.launches;
     (void)q4i_check(cudaGetLastError(), "pos_push launch");
 }
 extern "C" int q4_hip_capturing(void) { return g_q4.capturing; }
@@ -247,11 +249,13 @@ extern "C" int q4_hip_graph_begin(void) {
         return 0;
     }
     g_q4.capturing = 1;
+    g_q4.unsettled = g_q4.launches;
     return 1;
 }
 extern "C" void *q4_hip_graph_end(void) {
     if (!g_q4.ok || !g_q4.capturing) return nullptr;
     g_q4.capturing = 0;
+    g_q4.unsettled = g_q4.launches;
     cudaGraph_t g = nullptr;
     if (cudaStreamEndCapture(g_q4.stream, &g) != cudaSuccess || !g) {
         (void)cudaGetLastError();
@@ -276,6 +280,7 @@ extern "C" uint32_t q4_hip_graph_nodes(void *exec) {
 }
 extern "C" bool q4_hip_graph_launch(void *exec) {
     if (!g_q4.ok || !exec) return false;
+    g_q4.unsettled = g_q4.launches;
     return q4i_check(cudaGraphLaunch((cudaGraphExec_t)exec, g_q4.stream), "graph launch");
 }
 extern "C" void q4_hip_graph_free(void *exec) {
@@ -330,6 +335,7 @@ extern "C" bool q4_gpu_pipe_run(q4_gpu_pipe *p, void *graph_exec, void *dst_h, c
     Q4_REQUIRE(p && graph_exec, "pipe_run: bad argument");
     if (!q4i_check(cudaStreamWaitEvent(g_q4.stream, p->in_done, 0), "pipe_run wait")) return false;
     if (p->has_out && !q4i_check(cudaStreamWaitEvent(g_q4.stream, p->out_done, 0), "pipe_run wait")) return false;
+    g_q4.unsettled = g_q4.launches;
     if (!q4i_check(cudaGraphLaunch((cudaGraphExec_t)graph_exec, g_q4.stream), "pipe_run launch") ||
         !q4i_check(cudaEventRecord(p->run_done, g_q4.stream), "pipe_run record"))
         return false;
