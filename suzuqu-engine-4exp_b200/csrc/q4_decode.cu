@@ -1327,7 +1327,13 @@ q4_decode_k(const DecParams P) {
                 hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
             }
         };
-        auto fill = [&]() { issue(0, pa); issue(1, pb); issue(2, pc); issue(3, pd); };
+        auto fill = [&]() {   /* rolled: the kernel has this in three places, and every launch fetches its image anew */
+#pragma unroll 1
+            for (uint32_t i = 0; i < RING_STAGES; i++) {
+                issue(i, pa);
+                pa = pb; pb = pc; pc = pd;
+            }
+        };
         if (early) {
             first_positions();
             if (!hold) fill();

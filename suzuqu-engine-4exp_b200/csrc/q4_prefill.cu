@@ -96,8 +96,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-/* x * sigmoid(g) */
-__device__ __forceinline__ float gated(float x, float g) { return __fdividef(x, 1.f + __expf(-g)); }
+/* x * sigmoid(g); a gate below -126 / log2(e) gives 0 (1 / (1 + inf)) */
+__device__ __forceinline__ float gated(float x, float g) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + ex2f(g * -1.4426950408889634f)));
+    return x * r;
+}
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
     if (warp < SW) {
         /* ---- queries as fp16 (exact for normal bf16 values), K-major swizzled, blocks of 64 dims: 8 dims per thread
          * and step, whole rows per warp step */
-        constexpr uint32_t PER = HD / 8u, BATCH = 4u;   /* loads in flight before the first store */
+        constexpr uint32_t PER = HD / 8u, BATCH = 8u;   /* loads in flight before the first store */
 #pragma unroll 1
         for (uint32_t k0 = 0; k0 < PER; k0 += BATCH) {
             uint4 w[BATCH][2];
@@ -638,38 +642,38 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             const float2 l0 = unpack2(ls[0]), l1 = unpack2(ls[1]);
             l_run += (l0.x + l0.y) + (l1.x + l1.y);
         }
+        /* ---- epilogue: O / l * sigmoid(gate), or the unnormalised part of a split range.  32 columns at a time go
+         * through the warp's share of the query tiles (read by no product any more), so that rows leave in whole lines.
+         * Step q of a column block: 4 rows of 32 columns, 8 lanes each.  The gates are requested a whole column block
+         * ahead, the first ones under the last product (requested behind their use a block took 2600 cycles, most of it
+         * their latency). */
+        const bool split = P.n_split > 1u, gates = P.gate && !split;
+        const uint32_t w_row0 = (warp & 3u) * 32u;
+        uint32_t off[8], live = 0;   /* in 16-byte units from the chunk's first token */
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const uint32_t row = w_row0 + 4u * q + (lane >> 3), ti = row * inv_gqa >> 16;
+            if (ti < P.tpc && t0 + g * P.tpc + ti < P.n_tok) live |= 1u << q;
+            off[q] = ((g * P.tpc + ti) * P.n_head + kh * P.gqa + (row - ti * P.gqa)) * (HD / 4u) + (lane & 7u);
+        }
+        const size_t first = (size_t)t0 * P.n_head * (HD / 4u);
+        auto fetch_gates = [&](int c, float4 (&gt)[8]) {
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (gates && ((live >> q) & 1u)) gt[q] = reinterpret_cast<const float4 *>(P.gate)[first + off[q] + 8u * c];
+        };
+        float4 gt0[8], gt1[8];
+        fetch_gates(0, gt0);
         if (ok && n_seq > 0) ok = wait(bar_o + 8 * g, (n_seq - 1u) & 1u);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
 
-        /* ---- epilogue: O / l * sigmoid(gate), or the unnormalised part of a split range.  32 columns at a time go
-         * through the warp's share of the query tiles (read by no product any more), so that rows leave in whole lines */
         if (ok) {
-            const bool split = P.n_split > 1u;
             const float inv = split ? 1.f : l_run > 0.f ? 1.f / l_run : 0.f;
             float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + g * QG_BYTES + (warp & 3u) * (QG_BYTES / 4u));   /* [32][36] */
-            const uint32_t w_row0 = (warp & 3u) * 32u;
             if (split && row_live)
                 P.part_ml[((size_t)blockIdx.z * P.n_tok + tok) * P.n_head + head] = make_float2(m_ref, l_run);
-            /* step q of a column block: 4 rows of 32 columns, 8 lanes each; the gates are requested a column block ahead */
-            uint32_t off[8], live = 0;   /* in 16-byte units from the chunk's first token */
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const uint32_t row = w_row0 + 4u * q + (lane >> 3), ti = row * inv_gqa >> 16;
-                if (ti < P.tpc && t0 + g * P.tpc + ti < P.n_tok) live |= 1u << q;
-                off[q] = ((g * P.tpc + ti) * P.n_head + kh * P.gqa + (row - ti * P.gqa)) * (HD / 4u) + (lane & 7u);
-            }
-            const size_t first = (size_t)t0 * P.n_head * (HD / 4u);
-            const bool gates = P.gate && !split;
-            float4 gt[8];
-            auto fetch_gates = [&](int c) {
-#pragma unroll
-                for (int q = 0; q < 8; q++)
-                    if (gates && ((live >> q) & 1u)) gt[q] = reinterpret_cast<const float4 *>(P.gate)[first + off[q] + 8u * c];
-            };
-            fetch_gates(0);
-#pragma unroll 1
-            for (int c = 0; c < HD / 32; c++) {
+            auto columns = [&](int c, float4 (&gt)[8]) {
                 float o[32];
                 if (n_tiles > 0) {
                     tmem_ld32(t_lane + O_COL + g * 128u + 32 * c, o);
@@ -683,29 +687,39 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
                 for (int k = 0; k < 32; k += 4)
                     *reinterpret_cast<float4 *>(buf + lane * 36u + k) = make_float4(o[k] * inv, o[k + 1] * inv, o[k + 2] * inv, o[k + 3] * inv);
                 __syncwarp();
-                float4 x[8];
+                float4 x[8];   /* all eight at once: a step after the other is 300 cycles of latency each */
 #pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    x[q] = *reinterpret_cast<const float4 *>(buf + (4u * q + (lane >> 3)) * 36u + 4u * (lane & 7u));
-                    if (gates) {
+                for (int q = 0; q < 8; q++) x[q] = *reinterpret_cast<const float4 *>(buf + (4u * q + (lane >> 3)) * 36u + 4u * (lane & 7u));
+                if (gates) {
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
                         x[q].x = gated(x[q].x, gt[q].x); x[q].y = gated(x[q].y, gt[q].y);
                         x[q].z = gated(x[q].z, gt[q].z); x[q].w = gated(x[q].w, gt[q].w);
                     }
                 }
-                if (c + 1 < HD / 32) fetch_gates(c + 1);
+                if (split) {
 #pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    if (!((live >> q) & 1u)) continue;
-                    const size_t at = first + off[q] + 8u * c;
-                    if (split) {
-                        reinterpret_cast<float4 *>(P.part)[(size_t)blockIdx.z * P.n_tok * P.n_head * (HD / 4u) + at] = x[q];
-                    } else if (P.out_bf16) {
+                    for (int q = 0; q < 8; q++)
+                        if ((live >> q) & 1u) reinterpret_cast<float4 *>(P.part)[(size_t)blockIdx.z * P.n_tok * P.n_head * (HD / 4u) + first + off[q] + 8u * c] = x[q];
+                } else if (P.out_bf16) {
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
                         const __nv_bfloat162 b0 = __floats2bfloat162_rn(x[q].x, x[q].y), b1 = __floats2bfloat162_rn(x[q].z, x[q].w);
-                        reinterpret_cast<uint2 *>(P.out)[at] = make_uint2(*reinterpret_cast<const uint32_t *>(&b0), *reinterpret_cast<const uint32_t *>(&b1));
-                    } else {
-                        reinterpret_cast<float4 *>(P.out)[at] = x[q];
+                        if ((live >> q) & 1u)
+                            reinterpret_cast<uint2 *>(P.out)[first + off[q] + 8u * c] = make_uint2(*reinterpret_cast<const uint32_t *>(&b0), *reinterpret_cast<const uint32_t *>(&b1));
                     }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; q++)
+                        if ((live >> q) & 1u) reinterpret_cast<float4 *>(P.out)[first + off[q] + 8u * c] = x[q];
                 }
+            };
+#pragma unroll 1
+            for (int c = 0; c < HD / 32; c += 2) {
+                fetch_gates(c + 1, gt1);
+                columns(c, gt0);
+                if (c + 2 < HD / 32) fetch_gates(c + 2, gt0);
+                columns(c + 1, gt1);
             }
         }
     }
@@ -811,11 +825,12 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     const uint32_t kp = a.layout == LAY_Q8R ? 2u : 1u;
     const uint32_t tpc = PF_ROWS / gqa, groups = (a.n_tok + tpc - 1u) / tpc, sms = (uint32_t)g_q4.sm_count;
     /* Two groups per block share every K/V tile and hide one another's softmax; one group per block while that does not
-     * fill the SMs, and then the positions are split too, at least two tiles a block. */
+     * fill the SMs, and then the positions are split too, three tiles a block. */
     const uint32_t nq = hd == 128 && groups * a.n_kvh > sms ? 2u : 1u;
     const uint32_t blocks = (groups + nq - 1u) / nq * a.n_kvh;
     uint32_t split = nq == 1 && blocks * 2u <= sms ? sms / blocks : 1u;
-    if (split > (tiles + 1u) / 2u) split = (tiles + 1u) / 2u;
+    if (tiles < 6u) split = 1u;                            /* the merge costs about as much as three tiles */
+    if (split > (tiles + 2u) / 3u) split = (tiles + 2u) / 3u;
     if (split > 16u) split = 16u;
     const size_t k_bytes = (size_t)a.n_kvh * tiles * kp * (hd / 128u) * PF_CHUNK, v_bytes = (size_t)a.n_kvh * tiles * (hd / 128u) * PF_CHUNK;
     const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
