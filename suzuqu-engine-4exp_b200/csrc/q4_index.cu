@@ -179,44 +179,53 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
 /* ---- score for many tokens over one pool (a prompt's slice).  The scan above reads the pool once per token, 17 GB
  * through L2 for 512 tokens x 32 768 blocks (1.67 ms).  This form is a tiled fp32 product on the FMA pipe (the
  * result is defined as one fused multiply-add per dim in dim order, which rules the tensor cores out): 32 tokens x 4
- * heads against 128 pooled blocks per tile, 8 x 8 chains per thread -- two tokens' four heads, so the relu sum over
- * heads stays in the thread.  64 FMAs per 16 shared-memory words; the queries stay in shared memory while a
- * persistent block walks pool tiles, two buffers deep.  Bound by the FMA pipe. */
-constexpr uint32_t SM_TOK = 32, SM_ROWS = SM_TOK * 4, SM_COLS = 128, SM_THREADS = 256;
-constexpr uint32_t SM_TILE_FLOATS = 128u * SC_ROW_FLOATS;
-constexpr uint32_t SM_SMEM = 3u * SM_TILE_FLOATS * sizeof(float);
+ * heads against 16 JC pooled blocks per tile, 8 x JC chains per thread -- two tokens' four heads, so the relu sum over
+ * heads stays in the thread.  Bound by the FMA pipe if shared memory keeps up: 8 + JC reads of 16 bytes feed 32 JC
+ * multiply-adds, so JC = 16 (with JC = 8 both pipes are equally full, and 512 tokens x 32 768 blocks take 381 us).
+ * The queries stay in shared memory while a persistent block walks the tiles; the pool comes in 32 dims at a time,
+ * three buffers deep. */
+constexpr uint32_t SM_TOK = 32, SM_ROWS = SM_TOK * 4, SM_THREADS = 256, SM_CD = 32, SM_CHUNKS = IX_HD / SM_CD, SM_STAGES = 3;
+constexpr uint32_t SM_PITCH = SM_CD + 4;   /* floats: 16-byte reads of eight consecutive rows in eight bank groups */
+template <uint32_t JC>
+constexpr uint32_t sm_smem() { return (SM_ROWS * SC_ROW_FLOATS + SM_STAGES * 16u * JC * SM_PITCH) * (uint32_t)sizeof(float); }
+template <uint32_t JC>
 __global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q, const float *pool, float *score, uint32_t n_tok,
                                                                  uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                                                                  uint32_t pos0, uint32_t ratio) {
-    extern __shared__ __align__(16) float sm_tiles[];   /* queries | pool tile 0 | pool tile 1, rows 132 floats apart */
+    constexpr uint32_t COLS = 16u * JC;
+    extern __shared__ __align__(16) float sm_tiles[];   /* queries, rows 132 floats apart | pool chunks, rows 36 floats apart */
     const uint32_t tid = threadIdx.x;
     const uint32_t ty = tid >> 4, tc = tid & 15u;       /* tokens 2 ty, 2 ty + 1; pooled blocks tc + 16 j */
-    const uint32_t col_tiles = (n_blocks + SM_COLS - 1u) / SM_COLS, tok_tiles = (n_tok + SM_TOK - 1u) / SM_TOK;
+    const uint32_t col_tiles = (n_blocks + COLS - 1u) / COLS, tok_tiles = (n_tok + SM_TOK - 1u) / SM_TOK;
     const uint64_t total = (uint64_t)col_tiles * tok_tiles;
     const uint32_t first = (uint32_t)(total * blockIdx.x / gridDim.x), last = (uint32_t)(total * (blockIdx.x + 1u) / gridDim.x);
-    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(sm_tiles);
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(sm_tiles) + SM_ROWS * SC_ROW_FLOATS * 4u;
     auto visible = [&](uint32_t tok) { return (pos0 + tok + 1u) / ratio; };
     /* rows of a tile that no token of the group can see are not read: they need not exist yet */
-    auto fetch_pool = [&](uint32_t tile, uint32_t which) {
+    auto fetch = [&](uint32_t it) {
+        const uint32_t tile = first + it / SM_CHUNKS, d0 = (it % SM_CHUNKS) * SM_CD;
         if (tile < last) {
-            const uint32_t t_last = min((tile / col_tiles + 1u) * SM_TOK, n_tok) - 1u, c0 = (tile % col_tiles) * SM_COLS;
-            const uint32_t lim = min(visible(t_last), n_blocks);
-            for (uint32_t i = tid; i < SM_COLS * 32u; i += SM_THREADS) {
-                const uint32_t r = i >> 5, c = i & 31u;
-                const uint32_t dst = s0 + ((1u + which) * SM_TILE_FLOATS + r * SC_ROW_FLOATS + c * 4u) * 4u;
+            const uint32_t t_last = min((tile / col_tiles + 1u) * SM_TOK, n_tok) - 1u, c0 = (tile % col_tiles) * COLS;
+            const uint32_t lim = min(visible(t_last), n_blocks), dst0 = s0 + (it % SM_STAGES) * COLS * SM_PITCH * 4u;
+#pragma unroll
+            for (uint32_t k = 0; k < COLS * (SM_CD / 4u) / SM_THREADS; k++) {
+                const uint32_t i = tid + k * SM_THREADS, r = i / (SM_CD / 4u), c = i % (SM_CD / 4u);
+                const uint32_t dst = dst0 + (r * SM_PITCH + c * 4u) * 4u;
                 if (c0 + r < lim)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(pool + (size_t)(c0 + r) * IX_HD + c * 4u) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(pool + (size_t)(c0 + r) * IX_HD + d0 + c * 4u) : "memory");
                 else
                     asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dst), "r"(0u) : "memory");
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    uint32_t have = 0xffffffffu, which = 0;
-    fetch_pool(first, 0);
-    for (uint32_t tile = first; tile < last; tile++, which ^= 1u) {
-        const uint32_t group = tile / col_tiles, c0 = (tile % col_tiles) * SM_COLS;
-        if (group != have) {   /* the barrier at the end of the previous tile has released the queries */
+    uint32_t have = 0xffffffffu, it = 0;
+    fetch(0);
+    fetch(1);
+    for (uint32_t tile = first; tile < last; tile++) {
+        const uint32_t group = tile / col_tiles, c0 = (tile % col_tiles) * COLS;
+        if (group != have) {
+            __syncthreads();   /* everyone is done with the queries of the group before */
             for (uint32_t i = tid; i < SM_ROWS * 32u; i += SM_THREADS) {
                 const uint32_t r = i >> 5, c = i & 31u, tok = group * SM_TOK + (r >> 2), h = r & 3u;
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -225,47 +234,54 @@ __global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q
             }
             have = group;
         }
-        fetch_pool(tile + 1u, which ^ 1u);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        const float *qa = sm_tiles + ty * 8u * SC_ROW_FLOATS, *kb = sm_tiles + (1u + which) * SM_TILE_FLOATS + tc * SC_ROW_FLOATS;
-        float acc[8][8];
+        float acc[8][JC];
 #pragma unroll
         for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+            for (uint32_t j = 0; j < JC; j++) acc[i][j] = 0.f;
+#pragma unroll 1
+        for (uint32_t ch = 0; ch < SM_CHUNKS; ch++, it++) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();   /* chunk `it` is in; everyone is done with the buffer that chunk it + 2 goes to */
+            fetch(it + 2u);
+            const float *qa = sm_tiles + ty * 8u * SC_ROW_FLOATS + ch * SM_CD;
+            const float *kb = sm_tiles + SM_ROWS * SC_ROW_FLOATS + (it % SM_STAGES) * COLS * SM_PITCH + tc * SM_PITCH;
 #pragma unroll 2
-        for (uint32_t d = 0; d < IX_HD; d += 4) {
-            float4 a[8], b[8];
+            for (uint32_t d = 0; d < SM_CD; d += 4) {
+                float4 a[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(qa + i * SC_ROW_FLOATS + d);
+                for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(qa + i * SC_ROW_FLOATS + d);
 #pragma unroll
-            for (int j = 0; j < 8; j++) b[j] = *reinterpret_cast<const float4 *>(kb + j * 16 * SC_ROW_FLOATS + d);
+                for (uint32_t j0 = 0; j0 < JC; j0 += 4) {
+                    float4 b[4];
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+                    for (uint32_t j = 0; j < 4; j++) b[j] = *reinterpret_cast<const float4 *>(kb + (j0 + j) * 16u * SM_PITCH + d);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].x, b[j].x, acc[i][j]);
+                    for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].x, b[j].x, acc[i][j0 + j]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].y, b[j].y, acc[i][j]);
+                    for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].y, b[j].y, acc[i][j0 + j]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].z, b[j].z, acc[i][j]);
+                    for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].z, b[j].z, acc[i][j0 + j]);
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(a[i].w, b[j].w, acc[i][j]);
+                    for (int i = 0; i < 8; i++)
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].w, b[j].w, acc[i][j0 + j]);
+                }
+            }
         }
-        __syncthreads();   /* this pool tile, and the queries if the group changes, may be overwritten */
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const uint32_t tok = group * SM_TOK + 2u * ty + u;
             if (tok >= n_tok) continue;
             const uint32_t n_vis = visible(tok);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
+            for (uint32_t j = 0; j < JC; j++) {
                 const uint32_t b = c0 + tc + 16u * j;
                 /* heads that do not exist have zero queries: their relu adds exactly nothing */
                 float sc = __fadd_rn(0.f, fmaxf(acc[4 * u][j], 0.f));
@@ -278,24 +294,26 @@ __global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
-/* A tile takes 13.7 us however few of its 32 tokens exist; the scan takes 1.2 us per token and 8192 blocks.  The product
- * is taken where its tiles, spread over the SMs, come out sooner (8 tokens at 65 536 blocks: 56 against 62 us; at 8192
- * blocks the scan keeps 8 tokens with 9.4 against 15.3 us). */
-bool score_mt_wins(uint32_t n_tok, uint32_t n_blocks) {
-    const uint64_t tiles = (uint64_t)((n_blocks + SM_COLS - 1u) / SM_COLS) * ((n_tok + SM_TOK - 1u) / SM_TOK);
-    const uint64_t per_sm = (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count;
-    return n_tok > 1 && per_sm * 13700u < (uint64_t)n_tok * n_blocks * 1200u / 8192u;
+/* Estimated ns of the product with tiles of 16 JC blocks, and of the scan.  A tile takes a time of its own however few of
+ * its 32 tokens exist. */
+constexpr uint64_t SM_TILE_NS[2] = {13000, 18000};   /* JC = 8, 16 */
+uint64_t score_mt_ns(uint32_t n_tok, uint32_t n_blocks, uint32_t jc) {
+    const uint64_t tiles = (uint64_t)((n_blocks + 16u * jc - 1u) / (16u * jc)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
+    return (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count * SM_TILE_NS[jc == 16u];
 }
+/* (8 tokens at 65 536 blocks: the scan takes 62 us; at 8192 blocks it keeps 8 tokens with 9.4 us) */
+uint64_t score_scan_ns(uint32_t n_tok, uint32_t n_blocks) { return (uint64_t)n_tok * n_blocks * 1200u / 8192u; }
+template <uint32_t JC>
 bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                      uint32_t pos0, uint32_t ratio) {
     static bool done = false;
-    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score_mt_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_SMEM),
+    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score_mt_k<JC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_smem<JC>()),
                             "qsa_score smem attribute"))
         return false;
     done = true;
-    const uint64_t tiles = (uint64_t)((n_blocks + SM_COLS - 1u) / SM_COLS) * ((n_tok + SM_TOK - 1u) / SM_TOK);
+    const uint64_t tiles = (uint64_t)((n_blocks + 16u * JC - 1u) / (16u * JC)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
     const uint32_t grid = (uint32_t)(tiles < (uint64_t)g_q4.sm_count ? tiles : (uint64_t)g_q4.sm_count);
-    q4_ix_score_mt_k<<<grid, SM_THREADS, SM_SMEM, g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+    q4_ix_score_mt_k<JC><<<grid, SM_THREADS, sm_smem<JC>(), g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     return q4i_launched(q4i_check(cudaGetLastError(), "qsa_score launch"));
 }
 bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
@@ -1043,8 +1061,11 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
                                  uint32_t stride, uint32_t n_head, uint32_t hd, uint32_t pos0, uint32_t ratio) {
     if (!g_q4.ok || !q || !pool || !score || n_tok == 0 || hd != IX_HD || n_head == 0 || n_head > 4) return false;
     if (n_blocks == 0) return true;
-    if (ratio && score_mt_wins(n_tok, n_blocks) && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0)
-        return score_mt_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+    if (ratio && n_tok > 1 && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0) {
+        const uint64_t wide = score_mt_ns(n_tok, n_blocks, 16), narrow = score_mt_ns(n_tok, n_blocks, 8), scan = score_scan_ns(n_tok, n_blocks);
+        if (wide <= narrow && wide < scan) return score_mt_launch<16>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+        if (narrow < scan) return score_mt_launch<8>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+    }
     return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr);
 }
 /* Device position (graph-captured decode): the grid covers `stride` blocks, the bound comes from the
