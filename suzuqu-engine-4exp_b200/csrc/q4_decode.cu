@@ -336,35 +336,35 @@ __device__ __forceinline__ void merge_store(float *dst_rec, const MergeOut &mo, 
  * public record {m (natural-log units), l, acc[HD]}.  Deliberately not inlined: the kernel calls it
  * from one place for every merge level, and a small kernel image matters for launches that run each
  * instruction once. */
-template <int HD, int HEADS>
+template <int HD, int HEADS, int NREC /* a block's own records */>
 __device__ __noinline__ void merge_records(const float *recs, uint32_t count, bool global, float *dst_rec,
                                            const MergeOut mo, float *scratch /* MERGE_SCRATCH_FLOATS of shared memory */) {
     constexpr int REC = HD + 4;
     float *s_w = scratch, *s_l = scratch + DEC_GROUP * 16, *s_M = scratch + 2 * DEC_GROUP * 16, *s_L = s_M + 16;
     const uint32_t gqa = mo.gqa;
-    if (!global && count <= DEC_WARPS && dst_rec) {
+    if (!global && dst_rec) {
         /* The block's own warp records (at most four), in shared memory: every thread recomputes the four weights
          * of its head (no shared weights, no barriers in between) and writes its 4 dims of the block
          * record.  This runs once in every block of every launch. */
         for (uint32_t i = threadIdx.x; i < gqa * (HD / 4); i += DEC_THREADS) {
             const uint32_t h = i / (HD / 4), d = (i % (HD / 4)) * 4;
-            float2 ml[DEC_WARPS];
-            float4 x[DEC_WARPS];
+            float2 ml[NREC];
+            float4 x[NREC];
 #pragma unroll
-            for (int k = 0; k < DEC_WARPS; k++) {
-                const float *r = recs + ((size_t)min((uint32_t)k, count - 1u) * HEADS + h) * REC;
+            for (int k = 0; k < NREC; k++) {
+                const float *r = recs + ((size_t)k * HEADS + h) * REC;
                 ml[k] = *reinterpret_cast<const float2 *>(r + HD);
                 x[k] = *reinterpret_cast<const float4 *>(r + d);
             }
             float M = -CUDART_INF_F;
 #pragma unroll
-            for (int k = 0; k < DEC_WARPS; k++) M = fmaxf(M, ml[k].x);
+            for (int k = 0; k < NREC; k++) M = fmaxf(M, ml[k].x);
             const float Mu = M == -CUDART_INF_F ? 0.f : M;
             float L = 0.f;
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < DEC_WARPS; k++) {
-                const float w = (uint32_t)k < count ? ex2(ml[k].x - Mu) : 0.f;
+            for (int k = 0; k < NREC; k++) {
+                const float w = ex2(ml[k].x - Mu);
                 L = fmaf(w, ml[k].y, L);
                 A.x = fmaf(w, x[k].x, A.x); A.y = fmaf(w, x[k].y, A.y);
                 A.z = fmaf(w, x[k].z, A.z); A.w = fmaf(w, x[k].w, A.w);
@@ -895,8 +895,8 @@ struct DecTile {
 constexpr int dec_stages(int groups_bytes) {   /* as many, up to 4, as leave room for 3 blocks per SM */
     return groups_bytes * 4 <= 73728 ? 4 : groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 73728 ? 2 : 1;
 }
-/* DIRECT: caches whose base is not aligned for the asynchronous copies (reference ABI only) load fragments into registers */
-template <int LAY, int HD, int NHT, bool DIRECT>
+/* LIST: positions from a list (else a dense range).  DIRECT: caches whose base is not aligned for the asynchronous copies (reference ABI only) load fragments into registers */
+template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
 struct DecCfg {
     static constexpr bool STAGED = (LAY == LAY_Q8P && HD == 128);
     static constexpr bool STAGED2 = !STAGED && !DIRECT && HD >= 128;
@@ -908,17 +908,17 @@ struct DecCfg {
     static constexpr int TILE2 = STAGED2 ? DecTile<LAY, (HD < 128 ? 128 : HD)>::BYTES : 16;
     static constexpr int ST2 = dec_stages(NPG * TILE2);
     static constexpr size_t RING_BYTES = STAGED ? (size_t)DEC_WARPS * RING_STAGES * RING_STAGE_BYTES + RING_BAR_BYTES
-                                       : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 : 0;
+                                       : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 + NPG * ST2 * 16 : 0;
     static constexpr size_t REC_BYTES = (size_t)HEADS * REC * sizeof(float);   /* the block's merged record */
     static constexpr size_t TAIL_BYTES = EPI_BYTES + REC_BYTES + MERGE_SCRATCH_FLOATS * sizeof(float);   /* after the loop */
     static constexpr size_t SMEM = ((TAIL_BYTES > RING_BYTES ? TAIL_BYTES : RING_BYTES) + 15) / 16 * 16;
     static constexpr int MIN_BLOCKS = STAGED ? (NHT == 1 ? 3 : 2) : STAGED2 ? (SMEM <= 74752 ? 3 : SMEM <= 113664 ? 2 : 1) : (HD * NHT <= 128 ? 3 : 1);
 };
 
-template <int LAY, int HD, int NHT, bool DIRECT>
-__global__ void __launch_bounds__(DEC_THREADS, (DecCfg<LAY, HD, NHT, DIRECT>::MIN_BLOCKS))
+template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
+__global__ void __launch_bounds__(DEC_THREADS, (DecCfg<LAY, HD, NHT, DIRECT, LIST>::MIN_BLOCKS))
 q4_decode_k(const DecParams P) {
-    using Cfg = DecCfg<LAY, HD, NHT, DIRECT>;
+    using Cfg = DecCfg<LAY, HD, NHT, DIRECT, LIST>;
     constexpr int NW = Cfg::NW;   /* groups of 8 query heads per warp */
     constexpr int NB = HD / 32;   /* q8_0 blocks per row */
     constexpr int KS = HD / 16;   /* k-steps of the QK product */
@@ -942,7 +942,7 @@ q4_decode_k(const DecParams P) {
         if (P.push_async) {
             /* the barrier that the peers' pushes complete: initialised before this block announces itself */
             if (threadIdx.x == 0) {
-                ring_bar_init((uint32_t)__cvta_generic_to_shared(smem_raw + DecCfg<LAY, HD, NHT, DIRECT>::SMEM + P.push_bytes - 16u));
+                ring_bar_init((uint32_t)__cvta_generic_to_shared(smem_raw + DecCfg<LAY, HD, NHT, DIRECT, LIST>::SMEM + P.push_bytes - 16u));
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             }
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -962,15 +962,14 @@ q4_decode_k(const DecParams P) {
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         }
     };
-    constexpr bool CAN_EARLY = Cfg::STAGED || Cfg::STAGED2;
+    constexpr bool APPENDS = Cfg::STAGED || Cfg::STAGED2, CAN_EARLY = APPENDS && !LIST;
     const bool early = CAN_EARLY && P.early_rows;   /* the wait comes behind the ring's first tiles */
     if (!P.early_pos) pdl_wait();
     const uint32_t newest = P.pos ? (uint32_t)P.pos[P.many ? u : 0] : P.kv_base + u;
     if (P.early_pos && !early) pdl_wait();
     uint32_t n_kv = newest + 1u;
     if (n_kv > C.max_kv) n_kv = C.max_kv;
-    const int32_t *list = P.idx ? P.idx + (size_t)u * P.idx_unit_stride + (size_t)kh * P.idx_kvh_stride
-                                : nullptr;
+    const int32_t *list = LIST ? P.idx + (size_t)u * P.idx_unit_stride + (size_t)kh * P.idx_kvh_stride : nullptr;
     const uint32_t n_pos = list ? P.width : n_kv;
     const uint32_t steps = (n_pos + 15u) >> 4;
     /* a launch sized for the store's capacity (position from the device) uses as many of its blocks as the context needs */
@@ -1029,7 +1028,7 @@ q4_decode_k(const DecParams P) {
                                                          ((size_t)u * P.n_kvh + kh) * HD + ap_b * 32 + ap_sub * 4);
         }
     };
-    if constexpr (CAN_EARLY) {
+    if constexpr (APPENDS) {
         if (!early) load_new();
     }
 
@@ -1572,8 +1571,10 @@ q4_decode_k(const DecParams P) {
         __syncthreads();    /* the epilogue below reuses the ring memory of all warps */
     } else if constexpr (Cfg::STAGED2) {
         /* ---- fp16 and fp32 rows, reference q8_0 blocks, and native q8_0 records at hd 256: every position group (a warp,
-         * or two warps with 8 query heads each) owns a ring of ST2 tiles in shared memory, filled with asynchronous copies
-         * of whole rows; fragments come out of it as the products need them.  (Fragments loaded straight into registers,
+         * or two warps with 8 query heads each) owns a ring of ST2 tiles in shared memory; fragments come out of it as the
+         * products need them.  A row is one bulk copy, issued by one lane, and completes the stage's mbarrier: filling the
+         * ring with 16-byte copies, 40 instructions and their addresses per lane, held the first tile up for 6400 cycles.
+         * (Rows of reference blocks at hd 128 are only 8-byte aligned and go that way all the same.)  (Fragments loaded straight into registers,
          * 2 to 16 bytes per lane and no tile ahead, kept too little in flight: 65 us for a 2051-entry list of reference
          * blocks at hd 256, 12 heads per kv head; 29 us for 100 003 fp16 rows of hd 128.) */
         using T = DecTile<LAY, HD>;
@@ -1583,6 +1584,16 @@ q4_decode_k(const DecParams P) {
         const uint32_t masks = (uint32_t)__cvta_generic_to_shared(smem_raw) + NPG * ST * T::BYTES + (uint32_t)warp * ST * 4;
         const uint32_t n_my = s_begin + pg < s_end ? (s_end - s_begin - pg + NPG - 1u) / NPG : 0u;
         const uint32_t r16 = lane & 15;
+        constexpr bool BULK = T::CH == 16 && (LIST || T::ROW > 256);   /* a dense scan of 256-byte rows: 26.9 us for 100 003 by 16-byte copies, 30.0 by rows */
+        /* two barriers per stage: all of it, or K rows and V rows */
+        const uint32_t bars = (uint32_t)__cvta_generic_to_shared(smem_raw) + NPG * ST * T::BYTES + DEC_WARPS * ST * 4 + pg * ST * 16;
+        uint32_t spin_limit = RING_SPIN_LIMIT;   /* 1 once a copy has not arrived in time: the block reports it and computes on */
+        if (BULK) {
+            if (hg == 0 && lane < 2 * ST) ring_bar_init(bars + lane * 8);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();   /* the warps of a group share the barriers */
+        }
         const bool packed = tok_stride == (uint32_t)T::ROW;   /* rows (records) of consecutive positions are consecutive */
         auto group_sync = [&]() {
             if (WPT == 2) asm volatile("bar.sync %0, 64;" ::"r"(pg + 1u) : "memory");
@@ -1610,6 +1621,24 @@ q4_decode_k(const DecParams P) {
                 }
                 const uint32_t slot = it % ST, st = ring + slot * T::BYTES;
                 const uint32_t livemask = __ballot_sync(0xffffffffu, p >= 0) & 0xffffu;
+                if constexpr (BULK) {
+                    if (hg == 0) {   /* lanes 0-15: K rows (records), 16-31: V rows */
+                        const int plane = T::REC ? 0 : (int)(lane >> 4);
+                        const uint32_t bar = bars + slot * 16 + (pl0 ? 8 : 0);
+                        if (plane >= pl0 && plane < pl1 && (!T::REC || lane < 16)) {
+                            const uint32_t dst = st + (plane ? T::V_OFF + r16 * T::V_PITCH : r16 * T::K_PITCH);
+                            /* the stage was last read (and perhaps written) through the generic proxy */
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                            if (p >= 0)
+                                bulk_copy_g2s(dst, (plane ? vbase : kbase) + (uint64_t)(uint32_t)p * tok_stride, T::ROW, bar);
+                            else if (!Q8)
+                                for (uint32_t c = 0; c < T::ROW; c += 16) asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dst + c), "r"(0u) : "memory");
+                        }
+                        if (lane == 0) ring_bar_expect(bar, __popc(livemask) * T::ROW * (pl1 - pl0));
+                    }
+                    if (pl1 == PLANES && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
+                    return;
+                }
                 const int32_t p0 = __shfl_sync(0xffffffffu, p, 0);
                 const bool run = packed && __all_sync(0xffffffffu, p0 >= 0 && p == p0 + (int32_t)r16);
                 constexpr int ITER = (16 * T::CPR + 32 * WPT - 1) / (32 * WPT);
@@ -1632,7 +1661,7 @@ q4_decode_k(const DecParams P) {
                 }
                 if (pl1 == PLANES && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
             }
-            cp_async_commit();   /* one group per call, empty or not, keeps the wait count uniform */
+            if (!BULK) cp_async_commit();   /* one group per call, empty or not, keeps the wait count uniform */
         };
         /* With a single stage K and V travel as two groups: the next tile's K rows come in under this tile's P . V. */
         constexpr bool HALVES = ST == 1 && !T::REC;
@@ -1640,7 +1669,16 @@ q4_decode_k(const DecParams P) {
             if (HALVES) { issue_planes(it, p, 0, 1); issue_planes(it, p, 1, 2); }
             else issue_planes(it, p, 0, PLANES);
         };
-        /* ---- queries, requested next to the list entries: the pairs of dims that k-step ks multiplies in lane t's slots
+        auto landed = [&](uint32_t it, int plane) {
+            if (BULK) {
+                const uint32_t bar = bars + (it % ST) * 16 + plane * 8;
+                uint32_t probes = 0;
+                while (!ring_bar_test(bar, (it / ST) & 1u) && ++probes < spin_limit) {}
+                if (probes >= spin_limit) spin_limit = 1u;
+            } else if (plane) cp_async_wait<1>();
+            else cp_async_wait<HALVES ? 1 : ST - 1>();   /* all but the newest ST - 1 tiles (the V rows) */
+        };
+        /* ---- queries, requested ahead of the copies: the pairs of dims that k-step ks multiplies in lane t's slots
          * 2t, 2t+1 (half 0) and 2t+8, 2t+9 (half 1), in the order in which the layout's K fragments carry them */
         auto q_dim = [&](int ks, int half) -> int {
             if (LAY == LAY_F16) return 16 * ks + 2 * t + 8 * half;
@@ -1650,22 +1688,17 @@ q4_decode_k(const DecParams P) {
         const uint32_t head = hg * 8 + g;
         const bool q_live = head < P.gqa;
         const size_t qoff = ((size_t)u * P.n_head + (size_t)kh * P.gqa + head) * HD;
-        uint32_t qs[KS][2];
-        auto load_q = [&]() {
+        uint2 qraw[KS][2];
+        auto request_q = [&]() {
 #pragma unroll
             for (int ks = 0; ks < KS; ks++)
 #pragma unroll
                 for (int half = 0; half < 2; half++) {
-                    float2 x = make_float2(0.f, 0.f);
+                    qraw[ks][half] = make_uint2(0u, 0u);
                     if (q_live) {
-                        if (P.q_bf16) {
-                            const uint32_t w = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + qoff + q_dim(ks, half));
-                            x = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-                        } else {
-                            x = *reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(P.q) + qoff + q_dim(ks, half));
-                        }
+                        if (P.q_bf16) qraw[ks][half].x = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + qoff + q_dim(ks, half));
+                        else qraw[ks][half] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const float *>(P.q) + qoff + q_dim(ks, half));
                     }
-                    qs[ks][half] = pack_h2(x.x, x.y);
                 }
         };
         int32_t pf[ST], pn0, pn1, pn2;
@@ -1685,11 +1718,13 @@ q4_decode_k(const DecParams P) {
 #pragma unroll
             for (int i = 0; i < ST; i++) issue(i, pf[i]);
         };
+        if (!early) request_q();
         first_positions();
         if (!hold) fill();
         if (early) {
             pdl_wait();
             load_new();
+            request_q();
         }
         if (LAY != LAY_Q8R && P.new_k) {
             uint8_t *row = const_cast<uint8_t *>(ap_which ? vbase : kbase) + (uint64_t)newest * tok_stride;
@@ -1707,12 +1742,20 @@ q4_decode_k(const DecParams P) {
                 else *reinterpret_cast<float4 *>(row + at * 4) = ap_x;
             }
             if (newest >= max_kv && threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
+            if (BULK) asm volatile("fence.proxy.async;" ::: "memory");   /* the row may be read back by the bulk-copy engine */
             __syncthreads();
         }
         if (hold) fill();
-        load_q();
+        uint32_t qs[KS][2];
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++)
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                const uint2 w = qraw[ks][half];
+                qs[ks][half] = P.q_bf16 ? pack_h2(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u)) : pack_h2(__uint_as_float(w.x), __uint_as_float(w.y));
+            }
         for (uint32_t it = 0; it < n_my; it++) {
-            cp_async_wait<HALVES ? 1 : ST - 1>();    /* all but the newest ST - 1 tiles (the V rows) have landed: this warp's part of tile `it` is in */
+            landed(it, 0);
             group_sync();
             const uint32_t slot = it % ST, st = ring + slot * T::BYTES, sv = st + T::V_OFF;
             const uint32_t livemask = lds32(masks + slot * 4);
@@ -1826,7 +1869,7 @@ q4_decode_k(const DecParams P) {
             const uint32_t pb0 = movmatrix_t(h2u(h0)), pb1 = movmatrix_t(h2u(h1));   /* positions 2t, 2t+1 / 2t+8, 2t+9 of head g */
 
             if (HALVES) {
-                cp_async_wait<1>();
+                landed(it, 1);
                 group_sync();                    /* V rows are in */
             }
             /* ---- O^T += V^T . P^T */
@@ -1906,7 +1949,14 @@ q4_decode_k(const DecParams P) {
             pn0 = pn1; pn1 = pn2;
             pn2 = my_pos(it + ST + 3);
         }
-        cp_async_wait<0>();
+        if (BULK && spin_limit == 1u) {
+            /* copies that may still be in flight must land (bounded again) before the block leaves its shared memory */
+            for (uint32_t it = n_my > ST ? n_my - ST : 0u; it < n_my; it++)
+                for (uint32_t plane = 0; plane < (HALVES ? 2u : 1u); plane++)
+                    for (uint32_t probes = 0; probes < (RING_SPIN_LIMIT >> 6) && !ring_bar_test(bars + (it % ST) * 16 + plane * 8, (it / ST) & 1u); probes++) {}
+            if (lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
+        }
+        if (!BULK) cp_async_wait<0>();
         __syncthreads();    /* the epilogue below reuses the ring memory of all warps */
     } else {
         for (uint32_t step = s_begin + warp; step < s_end; step += DEC_WARPS) {
@@ -2030,13 +2080,13 @@ q4_decode_k(const DecParams P) {
     float *fin = P.xchg ? reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES) : nullptr;
     if (S_act == 1) {
         if (hybrid) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        merge_records<HD, HEADS>(sm, Cfg::NPG, false, fin, mo, mscr);
+        merge_records<HD, HEADS, Cfg::NPG>(sm, Cfg::NPG, false, fin, mo, mscr);
         if (fin) xchg_finish<HD, HEADS>(P.xchg, P.xchg_phase, (uint32_t)unit, fin, mo, P.err);
         return;
     }
     if (in_cluster) {
         float *own = reinterpret_cast<float *>(smem_raw + Cfg::EPI_BYTES);
-        merge_records<HD, HEADS>(sm, Cfg::NPG, false, own, mo, mscr);
+        merge_records<HD, HEADS, Cfg::NPG>(sm, Cfg::NPG, false, own, mo, mscr);
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   /* every peer block has started (arrive at entry) */
         if (P.push_bytes) {
             cluster_push_merge<HD, HEADS>(own, reinterpret_cast<const float *>(smem_raw + Cfg::SMEM), P.cluster, cluster_ctarank(), mo,
@@ -2054,7 +2104,7 @@ q4_decode_k(const DecParams P) {
     const uint32_t grp = split / DEC_GROUP;
     const uint32_t grp_size = min(DEC_GROUP, S - grp * DEC_GROUP);
     if (P.gridmerge) {
-        merge_records<HD, HEADS>(sm, Cfg::NPG, false, rec1 + (size_t)split * HEADS * REC, mo, mscr);
+        merge_records<HD, HEADS, Cfg::NPG>(sm, Cfg::NPG, false, rec1 + (size_t)split * HEADS * REC, mo, mscr);
         __syncthreads();   /* the warp records in shared memory are no longer needed: their space is the scratch */
         if (hybrid) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         grid_merge<HD, HEADS>(rec1, S, S_act, split, P.counters + unit * DEC_CTR, mo, sm, P.err);
@@ -2071,7 +2121,7 @@ q4_decode_k(const DecParams P) {
     uint32_t expected = grp_size;
     bool last = false;
     for (int level = 0;; level++) {
-        merge_records<HD, HEADS>(src, count, global, dst, mo, mscr);
+        merge_records<HD, HEADS, Cfg::NPG>(src, count, global, dst, mo, mscr);
         if (last) {                                        /* finalised, or this rank's record is complete */
             if (fin) xchg_finish<HD, HEADS>(P.xchg, P.xchg_phase, (uint32_t)unit, fin, mo, P.err);
             return;
@@ -2122,20 +2172,20 @@ __global__ void q4_lse_merge_k(const float *parts, uint32_t n_parts, uint32_t n_
     }
 }
 
-template <int LAY, int HD, int NHT, bool DIRECT>
+template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
 bool launch(const DecParams &p_in, dim3 grid) {
-    constexpr size_t smem_base = DecCfg<LAY, HD, NHT, DIRECT>::SMEM;
+    constexpr size_t smem_base = DecCfg<LAY, HD, NHT, DIRECT, LIST>::SMEM;
     constexpr size_t SMEM_LIMIT = smem_base + 2u * DEC_CLUSTER_MAX * (HD + 4) * sizeof(float) + 16u;   /* ring / epilogue + the largest receive area of the push merge */
     static bool attr_done = false;
     if (!attr_done) {
-        if (!q4i_check(cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT>,
+        if (!q4i_check(cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT, LIST>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT),
                        "decode smem attribute"))
             return false;
-        (void)cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        (void)cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT, LIST>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
     attr_done = true;
-    using Cfg = DecCfg<LAY, HD, NHT, DIRECT>;
+    using Cfg = DecCfg<LAY, HD, NHT, DIRECT, LIST>;
     DecParams p = p_in;
     auto n_blocks = [&]() -> uint64_t { return (uint64_t)grid.x * grid.y * grid.z; };
     /* how many clusters of this shape can be resident at once with `bytes` of dynamic shared memory per block */
@@ -2158,7 +2208,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
         qc.attrs = qa;
         qc.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, q4_decode_k<LAY, HD, NHT, DIRECT>, &qc) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&n, q4_decode_k<LAY, HD, NHT, DIRECT, LIST>, &qc) != cudaSuccess) {
             (void)cudaGetLastError();
             n = 0;
         }
@@ -2190,7 +2240,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
     if (p.gridmerge) {
         /* the blocks of a unit wait for one another: only when the whole grid is resident at once */
         static int occ = -1;
-        if (occ < 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, q4_decode_k<LAY, HD, NHT, DIRECT>, DEC_THREADS, smem_base) != cudaSuccess) {
+        if (occ < 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, q4_decode_k<LAY, HD, NHT, DIRECT, LIST>, DEC_THREADS, smem_base) != cudaSuccess) {
             (void)cudaGetLastError();
             occ = 0;
         }
@@ -2230,22 +2280,22 @@ bool launch(const DecParams &p_in, dim3 grid) {
     }
     cfg.attrs = at;
     cfg.numAttrs = n_at;
-    return q4i_check(cudaLaunchKernelEx(&cfg, q4_decode_k<LAY, HD, NHT, DIRECT>, p), "decode launch");
+    return q4i_check(cudaLaunchKernelEx(&cfg, q4_decode_k<LAY, HD, NHT, DIRECT, LIST>, p), "decode launch");
 }
-template <int LAY, int HD>
+template <int LAY, int HD, bool LIST>
 bool launch_nht(const DecParams &p, dim3 grid) {
     if constexpr (HD >= 128 && (LAY == LAY_Q8R || LAY == LAY_F16)) {
-        if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true>(p, grid) : launch<LAY, HD, 2, true>(p, grid);
+        if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true, LIST>(p, grid) : launch<LAY, HD, 2, true, LIST>(p, grid);
     }
-    return p.gqa <= 8 ? launch<LAY, HD, 1, false>(p, grid) : launch<LAY, HD, 2, false>(p, grid);
+    return p.gqa <= 8 ? launch<LAY, HD, 1, false, LIST>(p, grid) : launch<LAY, HD, 2, false, LIST>(p, grid);
 }
 template <int LAY>
 bool launch_hd(const DecParams &p, dim3 grid, uint32_t hd) {
     switch (hd) {
-    case 32: return launch_nht<LAY, 32>(p, grid);
-    case 64: return launch_nht<LAY, 64>(p, grid);
-    case 128: return launch_nht<LAY, 128>(p, grid);
-    case 256: return launch_nht<LAY, 256>(p, grid);
+    case 32: return p.idx ? launch_nht<LAY, 32, true>(p, grid) : launch_nht<LAY, 32, false>(p, grid);
+    case 64: return p.idx ? launch_nht<LAY, 64, true>(p, grid) : launch_nht<LAY, 64, false>(p, grid);
+    case 128: return p.idx ? launch_nht<LAY, 128, true>(p, grid) : launch_nht<LAY, 128, false>(p, grid);
+    case 256: return p.idx ? launch_nht<LAY, 256, true>(p, grid) : launch_nht<LAY, 256, false>(p, grid);
     }
     return q4i_fail(Q4E_ARG, "decode: hd must be 32, 64, 128 or 256");
 }
