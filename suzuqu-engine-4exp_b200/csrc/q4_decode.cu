@@ -908,7 +908,7 @@ struct DecCfg {
     static constexpr int TILE2 = STAGED2 ? DecTile<LAY, (HD < 128 ? 128 : HD)>::BYTES : 16;
     static constexpr int ST2 = dec_stages(NPG * TILE2);
     static constexpr size_t RING_BYTES = STAGED ? (size_t)DEC_WARPS * RING_STAGES * RING_STAGE_BYTES + RING_BAR_BYTES
-                                       : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 + NPG * ST2 * 16 : 0;
+                                       : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 : 0;
     static constexpr size_t REC_BYTES = (size_t)HEADS * REC * sizeof(float);   /* the block's merged record */
     static constexpr size_t TAIL_BYTES = EPI_BYTES + REC_BYTES + MERGE_SCRATCH_FLOATS * sizeof(float);   /* after the loop */
     static constexpr size_t SMEM = ((TAIL_BYTES > RING_BYTES ? TAIL_BYTES : RING_BYTES) + 15) / 16 * 16;
@@ -1571,12 +1571,12 @@ q4_decode_k(const DecParams P) {
         __syncthreads();    /* the epilogue below reuses the ring memory of all warps */
     } else if constexpr (Cfg::STAGED2) {
         /* ---- fp16 and fp32 rows, reference q8_0 blocks, and native q8_0 records at hd 256: every position group (a warp,
-         * or two warps with 8 query heads each) owns a ring of ST2 tiles in shared memory; fragments come out of it as the
-         * products need them.  A row is one bulk copy, issued by one lane, and completes the stage's mbarrier: filling the
-         * ring with 16-byte copies, 40 instructions and their addresses per lane, held the first tile up for 6400 cycles.
-         * (Rows of reference blocks at hd 128 are only 8-byte aligned and go that way all the same.)  (Fragments loaded straight into registers,
-         * 2 to 16 bytes per lane and no tile ahead, kept too little in flight: 65 us for a 2051-entry list of reference
-         * blocks at hd 256, 12 heads per kv head; 29 us for 100 003 fp16 rows of hd 128.) */
+         * or two warps with 8 query heads each) owns a ring of ST2 tiles in shared memory, filled with asynchronous
+         * copies; fragments come out of it as the products need them.  A copy instruction takes whole rows, or powers of
+         * two of their chunks: one shuffle and one multiply address the K and the V piece, where dividing a running index by
+         * 17 chunks held the first tile up for 6400 cycles.  (A bulk copy per row costs the issuing warp about 65 cycles a
+         * row, 2200 a tile.  Fragments loaded straight into registers, 2 to 16 bytes per lane and no tile ahead, kept too
+         * little in flight: 65 us for a 2051-entry list of reference blocks at hd 256, 12 heads per kv head.) */
         using T = DecTile<LAY, HD>;
         constexpr int ST = Cfg::ST2, WPT = Cfg::WPT, NPG = Cfg::NPG, PLANES = T::REC ? 1 : 2;
         const uint32_t pg = warp / WPT, hg = warp % WPT;
@@ -1584,17 +1584,6 @@ q4_decode_k(const DecParams P) {
         const uint32_t masks = (uint32_t)__cvta_generic_to_shared(smem_raw) + NPG * ST * T::BYTES + (uint32_t)warp * ST * 4;
         const uint32_t n_my = s_begin + pg < s_end ? (s_end - s_begin - pg + NPG - 1u) / NPG : 0u;
         const uint32_t r16 = lane & 15;
-        constexpr bool BULK = T::CH == 16 && (LIST || T::ROW > 256);   /* a dense scan of 256-byte rows: 26.9 us for 100 003 by 16-byte copies, 30.0 by rows */
-        /* two barriers per stage: all of it, or K rows and V rows */
-        const uint32_t bars = (uint32_t)__cvta_generic_to_shared(smem_raw) + NPG * ST * T::BYTES + DEC_WARPS * ST * 4 + pg * ST * 16;
-        uint32_t spin_limit = RING_SPIN_LIMIT;   /* 1 once a copy has not arrived in time: the block reports it and computes on */
-        if (BULK) {
-            if (hg == 0 && lane < 2 * ST) ring_bar_init(bars + lane * 8);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();   /* the warps of a group share the barriers */
-        }
-        const bool packed = tok_stride == (uint32_t)T::ROW;   /* rows (records) of consecutive positions are consecutive */
         auto group_sync = [&]() {
             if (WPT == 2) asm volatile("bar.sync %0, 64;" ::"r"(pg + 1u) : "memory");
             else __syncwarp();
@@ -1613,6 +1602,8 @@ q4_decode_k(const DecParams P) {
             }
         };
         /* fill one stage (planes [pl0, pl1): K, V); padding rows are zeroed (fp16 / fp32), or left as they are and masked (q8_0) */
+        constexpr int MC = T::CPR >= 64 ? 64 : T::CPR >= 32 ? 32 : 16, RC = T::CPR - MC, IPR = MC > 32 ? MC / 32 : 1, RPI = MC < 32 ? 32 / MC : 1;
+        static_assert(RC * (T::REC ? 1 : 2) <= 2, "the odd chunks of 16 rows are one copy per lane");
         auto issue_planes = [&](uint32_t it, int32_t p, int pl0, int pl1) {
             if (it < n_my) {
                 if (p >= (int32_t)bound) {
@@ -1621,47 +1612,24 @@ q4_decode_k(const DecParams P) {
                 }
                 const uint32_t slot = it % ST, st = ring + slot * T::BYTES;
                 const uint32_t livemask = __ballot_sync(0xffffffffu, p >= 0) & 0xffffu;
-                if constexpr (BULK) {
-                    if (hg == 0) {   /* lanes 0-15: K rows (records), 16-31: V rows */
-                        const int plane = T::REC ? 0 : (int)(lane >> 4);
-                        const uint32_t bar = bars + slot * 16 + (pl0 ? 8 : 0);
-                        if (plane >= pl0 && plane < pl1 && (!T::REC || lane < 16)) {
-                            const uint32_t dst = st + (plane ? T::V_OFF + r16 * T::V_PITCH : r16 * T::K_PITCH);
-                            /* the stage was last read (and perhaps written) through the generic proxy */
-                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            if (p >= 0)
-                                bulk_copy_g2s(dst, (plane ? vbase : kbase) + (uint64_t)(uint32_t)p * tok_stride, T::ROW, bar);
-                            else if (!Q8)
-                                for (uint32_t c = 0; c < T::ROW; c += 16) asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dst + c), "r"(0u) : "memory");
-                        }
-                        if (lane == 0) ring_bar_expect(bar, __popc(livemask) * T::ROW * (pl1 - pl0));
-                    }
-                    if (pl1 == PLANES && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
-                    return;
-                }
-                const int32_t p0 = __shfl_sync(0xffffffffu, p, 0);
-                const bool run = packed && __all_sync(0xffffffffu, p0 >= 0 && p == p0 + (int32_t)r16);
-                constexpr int ITER = (16 * T::CPR + 32 * WPT - 1) / (32 * WPT);
-                const uint64_t run_off = (uint64_t)(uint32_t)max(p0, 0) * tok_stride;
+                auto piece = [&](int plane, uint32_t r, uint32_t c, int32_t pr) {
+                    copy(st + (plane ? T::V_OFF + r * T::V_PITCH : r * T::K_PITCH) + c * T::CH,
+                         (plane ? vbase : kbase) + (uint64_t)(uint32_t)max(pr, 0) * tok_stride + c * T::CH, pr >= 0);
+                };
 #pragma unroll
-                for (int plane = pl0; plane < pl1; plane++) {
-                    const uint8_t *src = plane ? vbase : kbase;
-                    const uint32_t dst = st + (plane ? T::V_OFF : 0), pitch = plane ? T::V_PITCH : T::K_PITCH;
-#pragma unroll 4
-                    for (int i = 0; i < ITER; i++) {
-                        const uint32_t idx = lane + 32u * (i * WPT + hg), r = idx / T::CPR, c = idx % T::CPR;
-                        const bool in = 16 * T::CPR % (32 * WPT) == 0 || idx < 16u * T::CPR;
-                        if (run) {
-                            if (in) copy(dst + r * pitch + c * T::CH, src + run_off + idx * T::CH, true);
-                        } else {
-                            const int32_t pr = __shfl_sync(0xffffffffu, p, r & 15u);
-                            if (in) copy(dst + r * pitch + c * T::CH, src + (uint64_t)(uint32_t)max(pr, 0) * tok_stride + c * T::CH, pr >= 0);
-                        }
-                    }
+                for (int i = 0; i < 16 * IPR / RPI / WPT; i++) {
+                    const uint32_t k = i * WPT + hg, r = MC > 32 ? k / IPR : k * RPI + (RPI > 1 ? lane / MC : 0), c = MC > 32 ? lane + 32u * (k % IPR) : lane % MC;
+                    const int32_t pr = __shfl_sync(0xffffffffu, p, r);
+#pragma unroll
+                    for (int plane = pl0; plane < pl1; plane++) piece(plane, r, c, pr);
+                }
+                if (RC && hg == 0) {   /* the chunks behind the power of two: lanes 16.. take the second one, or the V rows' */
+                    const int plane = T::REC ? 0 : lane >> 4;
+                    if ((RC == 2 || !T::REC || lane < 16) && plane >= pl0 && plane < pl1) piece(plane, r16, MC + (T::REC ? lane >> 4 : 0), p);
                 }
                 if (pl1 == PLANES && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(masks + slot * 4), "r"(livemask) : "memory");
             }
-            if (!BULK) cp_async_commit();   /* one group per call, empty or not, keeps the wait count uniform */
+            cp_async_commit();   /* one group per call, empty or not, keeps the wait count uniform */
         };
         /* With a single stage K and V travel as two groups: the next tile's K rows come in under this tile's P . V. */
         constexpr bool HALVES = ST == 1 && !T::REC;
@@ -1669,37 +1637,34 @@ q4_decode_k(const DecParams P) {
             if (HALVES) { issue_planes(it, p, 0, 1); issue_planes(it, p, 1, 2); }
             else issue_planes(it, p, 0, PLANES);
         };
-        auto landed = [&](uint32_t it, int plane) {
-            if (BULK) {
-                const uint32_t bar = bars + (it % ST) * 16 + plane * 8;
-                uint32_t probes = 0;
-                while (!ring_bar_test(bar, (it / ST) & 1u) && ++probes < spin_limit) {}
-                if (probes >= spin_limit) spin_limit = 1u;
-            } else if (plane) cp_async_wait<1>();
-            else cp_async_wait<HALVES ? 1 : ST - 1>();   /* all but the newest ST - 1 tiles (the V rows) */
-        };
-        /* ---- queries, requested ahead of the copies: the pairs of dims that k-step ks multiplies in lane t's slots
-         * 2t, 2t+1 (half 0) and 2t+8, 2t+9 (half 1), in the order in which the layout's K fragments carry them */
+        /* ---- queries: requested coalesced, next to the list entries, and passed on as fp16 through the last stage before
+         * that is filled (with one stage: before any).  (Fetched lane by lane in the fragments' order they took 4000 cycles
+         * of the load pipe, 8000 in that of the reference blocks.)  Fragments: the pairs of dims that k-step ks multiplies
+         * in lane t's slots 2t, 2t+1 (half 0) and 2t+8, 2t+9 (half 1), in the order of the layout's K fragments */
         auto q_dim = [&](int ks, int half) -> int {
             if (LAY == LAY_F16) return 16 * ks + 2 * t + 8 * half;
             if (LAY == LAY_Q8R) return q8r_dim(ks >> 1, 2 * t + (ks & 1), 2 * half);
             return 16 * ks + 4 * t + 2 * half;
         };
-        const uint32_t head = hg * 8 + g;
-        const bool q_live = head < P.gqa;
-        const size_t qoff = ((size_t)u * P.n_head + (size_t)kh * P.gqa + head) * HD;
-        uint2 qraw[KS][2];
+        constexpr int QV = HEADS * HD / 4 / DEC_THREADS, Q_PITCH = 2 * HD + 16;
+        static_assert(HEADS * Q_PITCH <= T::BYTES, "the queries fit a stage");
+        const uint32_t q_at = (uint32_t)__cvta_generic_to_shared(smem_raw) + (ST - 1) * T::BYTES;
+        uint4 qv[QV];
         auto request_q = [&]() {
 #pragma unroll
-            for (int ks = 0; ks < KS; ks++)
-#pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    qraw[ks][half] = make_uint2(0u, 0u);
-                    if (q_live) {
-                        if (P.q_bf16) qraw[ks][half].x = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + qoff + q_dim(ks, half));
-                        else qraw[ks][half] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const float *>(P.q) + qoff + q_dim(ks, half));
+            for (int i = 0; i < QV; i++) {
+                const uint32_t e = threadIdx.x + i * DEC_THREADS;
+                qv[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (e / (HD / 4) < P.gqa) {
+                    const size_t off = ((size_t)u * P.n_head + (size_t)kh * P.gqa) * HD + e * 4u;
+                    if (P.q_bf16) {
+                        const uint2 w = *reinterpret_cast<const uint2 *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + off);
+                        qv[i].x = w.x; qv[i].y = w.y;
+                    } else {
+                        qv[i] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(P.q) + off);
                     }
                 }
+            }
         };
         int32_t pf[ST], pn0, pn1, pn2;
         /* fused append, second half (see the hd-128 path): a group whose first tiles name the newest row waits for it */
@@ -1714,12 +1679,17 @@ q4_decode_k(const DecParams P) {
                 hold = __any_sync(0xffffffffu, hold);
             }
         };
-        auto fill = [&]() {
+        auto fill = [&]() {   /* all stages but the last */
+#pragma unroll 1
+            for (int i = 0; i < ST - 1; i++) {
+                issue(i, pf[0]);
 #pragma unroll
-            for (int i = 0; i < ST; i++) issue(i, pf[i]);
+                for (int k = 0; k + 1 < ST; k++) pf[k] = pf[k + 1];
+            }
         };
         if (!early) request_q();
         first_positions();
+        const int32_t p_last = pf[ST - 1];
         if (!hold) fill();
         if (early) {
             pdl_wait();
@@ -1742,20 +1712,27 @@ q4_decode_k(const DecParams P) {
                 else *reinterpret_cast<float4 *>(row + at * 4) = ap_x;
             }
             if (newest >= max_kv && threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
-            if (BULK) asm volatile("fence.proxy.async;" ::: "memory");   /* the row may be read back by the bulk-copy engine */
             __syncthreads();
         }
         if (hold) fill();
+#pragma unroll
+        for (int i = 0; i < QV; i++) {
+            const uint32_t e = threadIdx.x + i * DEC_THREADS, at = q_at + e / (HD / 4) * Q_PITCH + e % (HD / 4) * 8u;
+            const uint4 w = qv[i];
+            const uint32_t lo = P.q_bf16 ? pack_h2(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u)) : pack_h2(__uint_as_float(w.x), __uint_as_float(w.y));
+            const uint32_t hi = P.q_bf16 ? pack_h2(__uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u)) : pack_h2(__uint_as_float(w.z), __uint_as_float(w.w));
+            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(at), "r"(lo), "r"(hi) : "memory");
+        }
+        __syncthreads();
         uint32_t qs[KS][2];
 #pragma unroll
         for (int ks = 0; ks < KS; ks++)
 #pragma unroll
-            for (int half = 0; half < 2; half++) {
-                const uint2 w = qraw[ks][half];
-                qs[ks][half] = P.q_bf16 ? pack_h2(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u)) : pack_h2(__uint_as_float(w.x), __uint_as_float(w.y));
-            }
+            for (int half = 0; half < 2; half++) qs[ks][half] = lds32(q_at + (hg * 8 + g) * Q_PITCH + 2 * q_dim(ks, half));
+        __syncthreads();
+        issue(ST - 1, p_last);
         for (uint32_t it = 0; it < n_my; it++) {
-            landed(it, 0);
+            cp_async_wait<HALVES ? 1 : ST - 1>();    /* all but the newest ST - 1 tiles (the V rows) have landed: this warp's part of tile `it` is in */
             group_sync();
             const uint32_t slot = it % ST, st = ring + slot * T::BYTES, sv = st + T::V_OFF;
             const uint32_t livemask = lds32(masks + slot * 4);
@@ -1869,7 +1846,7 @@ q4_decode_k(const DecParams P) {
             const uint32_t pb0 = movmatrix_t(h2u(h0)), pb1 = movmatrix_t(h2u(h1));   /* positions 2t, 2t+1 / 2t+8, 2t+9 of head g */
 
             if (HALVES) {
-                landed(it, 1);
+                cp_async_wait<1>();
                 group_sync();                    /* V rows are in */
             }
             /* ---- O^T += V^T . P^T */
@@ -1949,14 +1926,7 @@ q4_decode_k(const DecParams P) {
             pn0 = pn1; pn1 = pn2;
             pn2 = my_pos(it + ST + 3);
         }
-        if (BULK && spin_limit == 1u) {
-            /* copies that may still be in flight must land (bounded again) before the block leaves its shared memory */
-            for (uint32_t it = n_my > ST ? n_my - ST : 0u; it < n_my; it++)
-                for (uint32_t plane = 0; plane < (HALVES ? 2u : 1u); plane++)
-                    for (uint32_t probes = 0; probes < (RING_SPIN_LIMIT >> 6) && !ring_bar_test(bars + (it % ST) * 16 + plane * 8, (it / ST) & 1u); probes++) {}
-            if (lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
-        }
-        if (!BULK) cp_async_wait<0>();
+        cp_async_wait<0>();
         __syncthreads();    /* the epilogue below reuses the ring memory of all warps */
     } else {
         for (uint32_t step = s_begin + warp; step < s_end; step += DEC_WARPS) {
