@@ -1316,6 +1316,28 @@ q4_decode_k(const DecParams P) {
             }
             cp_async_commit();   /* one group per tile, empty or not, keeps the wait count uniform */
         };
+        /* ---- queries: requested coalesced, next to the list entries, and passed on as fp16 (exact for bf16 queries; scale *
+         * log2(e) multiplies the scores in fp32 later) through warp 0's last stage before that is filled */
+        constexpr int QV = HEADS * HD / 4 / DEC_THREADS, Q_PITCH = 2 * HD + 16;
+        static_assert(HEADS * Q_PITCH <= RING_STAGE_BYTES, "the queries fit a stage");
+        const uint32_t q_at = (uint32_t)__cvta_generic_to_shared(smem_raw) + (RING_STAGES - 1) * RING_STAGE_BYTES;
+        uint4 qv[QV];
+        auto request_q = [&]() {
+#pragma unroll
+            for (int i = 0; i < QV; i++) {
+                const uint32_t e = threadIdx.x + i * DEC_THREADS;
+                qv[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (e / (HD / 4) < P.gqa) {
+                    const size_t off = ((size_t)u * P.n_head + (size_t)kh * P.gqa) * HD + e * 4u;
+                    if (P.q_bf16) {
+                        const uint2 w = *reinterpret_cast<const uint2 *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + off);
+                        qv[i].x = w.x; qv[i].y = w.y;
+                    } else {
+                        qv[i] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(P.q) + off);
+                    }
+                }
+            }
+        };
         int32_t pa, pb, pc, pd, pn0, pn1, pn2;
         bool hold = false;
         auto first_positions = [&]() {
@@ -1326,48 +1348,25 @@ q4_decode_k(const DecParams P) {
                 hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
             }
         };
-        auto fill = [&]() {   /* rolled: the kernel has this in three places, and every launch fetches its image anew */
+        auto fill = [&]() {   /* all stages but the last; rolled: the kernel's image is fetched anew by every launch */
 #pragma unroll 1
-            for (uint32_t i = 0; i < RING_STAGES; i++) {
+            for (uint32_t i = 0; i < RING_STAGES - 1; i++) {
                 issue(i, pa);
-                pa = pb; pb = pc; pc = pd;
+                pa = pb; pb = pc;
             }
         };
-        if (early) {
-            first_positions();
-            if (!hold) fill();
-            pdl_wait();
-            load_new();
-        }
-        /* ---- queries: the raw values are requested now, next to the list entries, and converted after the ring
-         * has been filled (lane (g, t) takes dims 16ks + 4t .. + 3 of head nt*8 + g) */
-        uint32_t qraw[NW][KS][4];
-#pragma unroll
-        for (int nt = 0; nt < NW; nt++) {
-            const uint32_t hg = nt * 8 + g;
-            const bool live = hg < P.gqa;
-            const size_t qoff = ((size_t)u * P.n_head + (size_t)kh * P.gqa + hg) * HD;
-#pragma unroll
-            for (int ks = 0; ks < KS; ks++) {
-                qraw[nt][ks][0] = qraw[nt][ks][1] = qraw[nt][ks][2] = qraw[nt][ks][3] = 0u;
-                if (live) {
-                    const int d = 16 * ks + 4 * t;
-                    if (P.q_bf16) {
-                        const uint2 w = *reinterpret_cast<const uint2 *>(reinterpret_cast<const __nv_bfloat16 *>(P.q) + qoff + d);
-                        qraw[nt][ks][0] = w.x; qraw[nt][ks][1] = w.y;
-                    } else {
-                        const uint4 w = *reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(P.q) + qoff + d);
-                        qraw[nt][ks][0] = w.x; qraw[nt][ks][1] = w.y; qraw[nt][ks][2] = w.z; qraw[nt][ks][3] = w.w;
-                    }
-                }
-            }
-        }
-        if (!early) first_positions();
+        if (!early) request_q();
+        first_positions();
         /* ---- fused append, second half.  Every split of the unit quantises and stores the unit's newest row
          * (identical bytes from every split, so no block depends on another having written); a block's own
          * store is ordered before its later reads by the barrier.  A warp whose first four tiles do not name the
          * newest row fills its ring before that, so the append runs under the first copies. */
-        if (!early && !hold) fill();
+        if (!hold) fill();
+        if (early) {
+            pdl_wait();
+            load_new();
+            request_q();
+        }
         if (P.new_k) {
             float d, id;
             q4d_block_scale(ap_x, d, id);
@@ -1381,12 +1380,18 @@ q4_decode_k(const DecParams P) {
             __syncthreads();
         }
         if (hold) fill();
-
-        /* Q fragments as fp16 (exact for bf16 queries; scale * log2(e) multiplies the scores in fp32 later):
-         * lane (g, t) holds dims 16ks + 4t .. + 3 of head nt*8 + g, the columns the K fragments below carry in
-         * k-slots 2t, 2t+1, 2t+8, 2t+9.  And,
-         * per 32-wide block, -1152 * sum(q): K codes enter the MMA as the fp16 numbers 1152 + code (one byte
-         * permute per pair, no subtract), so each block's partial product starts from that correction. */
+#pragma unroll
+        for (int i = 0; i < QV; i++) {
+            const uint32_t e = threadIdx.x + i * DEC_THREADS, at = q_at + e / (HD / 4) * Q_PITCH + e % (HD / 4) * 8u;
+            const uint4 w = qv[i];
+            const uint32_t lo = P.q_bf16 ? pack_h2(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u)) : pack_h2(__uint_as_float(w.x), __uint_as_float(w.y));
+            const uint32_t hi = P.q_bf16 ? pack_h2(__uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u)) : pack_h2(__uint_as_float(w.z), __uint_as_float(w.w));
+            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(at), "r"(lo), "r"(hi) : "memory");
+        }
+        __syncthreads();
+        /* Q fragments: lane (g, t) holds dims 16ks + 4t .. + 3 of head nt*8 + g, the columns the K fragments below carry in
+         * k-slots 2t, 2t+1, 2t+8, 2t+9.  And, per 32-wide block, -1152 * sum(q): K codes enter the MMA as the fp16 numbers
+         * 1152 + code (one byte permute per pair, no subtract), so each block's partial product starts from that. */
         uint32_t qs[NW][KS][2];
         float qcorr[NW][NB][2];
 #pragma unroll
@@ -1394,20 +1399,10 @@ q4_decode_k(const DecParams P) {
             float bsum[NB];
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
-                float x0, x1, x2, x3;
-                if (P.q_bf16) {
-                    x0 = __uint_as_float(qraw[nt][ks][0] << 16);
-                    x1 = __uint_as_float(qraw[nt][ks][0] & 0xffff0000u);
-                    x2 = __uint_as_float(qraw[nt][ks][1] << 16);
-                    x3 = __uint_as_float(qraw[nt][ks][1] & 0xffff0000u);
-                } else {
-                    x0 = __uint_as_float(qraw[nt][ks][0]); x1 = __uint_as_float(qraw[nt][ks][1]);
-                    x2 = __uint_as_float(qraw[nt][ks][2]); x3 = __uint_as_float(qraw[nt][ks][3]);
-                }
-                const __half2 h0 = __floats2half2_rn(x0, x1);
-                const __half2 h1 = __floats2half2_rn(x2, x3);
-                qs[nt][ks][0] = h2u(h0);
-                qs[nt][ks][1] = h2u(h1);
+                const uint2 w = lds64(q_at + (nt * 8 + g) * Q_PITCH + 32 * ks + 8 * t);
+                const __half2 h0 = u2h(w.x), h1 = u2h(w.y);
+                qs[nt][ks][0] = w.x;
+                qs[nt][ks][1] = w.y;
                 const float part = (__low2float(h0) + __high2float(h0)) + (__low2float(h1) + __high2float(h1));
                 if (ks & 1) bsum[ks >> 1] += part; else bsum[ks >> 1] = part;
             }
@@ -1420,6 +1415,9 @@ q4_decode_k(const DecParams P) {
                 qcorr[nt][b][1] = -1152.f * __shfl_sync(0xffffffffu, v, (2 * t + 1) * 4);
             }
         }
+
+        __syncthreads();         /* the queries have been read */
+        issue(RING_STAGES - 1, pd);
 
         for (uint32_t it = 0; it < n_my; it++) {
             cp_async_wait<RING_STAGES - 1>();    /* all but the newest RING_STAGES - 1 tiles have landed: tile `it` is in, if gathered */
