@@ -126,20 +126,10 @@ __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void *gsrc, 
     else
         asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(smem_dst), "r"(0u) : "memory");
 }
-/* The K and the V chunk of one record (V codes follow the K codes at +HD, in the store and in a ring stage);
- * nothing is copied for a padding position. */
-template <int HD>
-__device__ __forceinline__ void cp_async16_kv(uint32_t smem_dst, const void *gsrc, int32_t pos) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ge.s32 q, %2, 0;\n\t"
-        "@q cp.async.cg.shared.global [%0], [%1], 16;\n\t"
-        "@q cp.async.cg.shared.global [%0+%3], [%1+%3], 16;\n\t}"
-        ::"r"(smem_dst), "l"(gsrc), "r"(pos), "n"(HD) : "memory");
-}
-/* 512 consecutive bytes per warp instruction: lane l copies bytes [OFF + 16 l, OFF + 16 l + 16) */
-template <int OFF>
-__device__ __forceinline__ void cp_async16_at(uint32_t smem_dst, const void *gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0+%2], [%1+%2], 16;" ::"r"(smem_dst), "l"(gsrc), "n"(OFF) : "memory");
+/* nothing is copied for a padding position */
+__device__ __forceinline__ void cp_async16_if(uint32_t smem_dst, const void *gsrc, int32_t pos) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ge.s32 q, %2, 0;\n\t@q cp.async.cg.shared.global [%0], [%1], 16;\n\t}"
+                 ::"r"(smem_dst), "l"(gsrc), "r"(pos) : "memory");
 }
 /* one record, global -> shared, through the bulk-copy engine; completion is counted in bytes on the mbarrier */
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t smem_dst, const void *gsrc, uint32_t bytes, uint32_t bar) {
@@ -1247,7 +1237,7 @@ q4_decode_k(const DecParams P) {
         const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) +
                               (uint32_t)warp * RING_STAGES * RING_STAGE_BYTES;
         const uint32_t n_my = s_begin + warp < s_end ? (s_end - s_begin - warp + DEC_WARPS - 1u) / DEC_WARPS : 0u;
-        const uint32_t r16 = lane & 15, c8 = lane & 7;
+        const uint32_t r16 = lane & 15;
         /* ldmatrix row address of this lane for block b: matrix lane / 8 = rows 8 * (that & 1) .., chunk 2b + lane / 16 */
         uint32_t moff[NB];
 #pragma unroll
@@ -1281,36 +1271,26 @@ q4_decode_k(const DecParams P) {
                 }
                 const uint32_t st = ring + (it % RING_STAGES) * RING_STAGE_BYTES;
                 const uint32_t livemask = __ballot_sync(0xffffffffu, p >= 0) & 0xffffu;
-                /* 16 consecutive positions: the tile is one contiguous span of the store */
-                const int32_t p0 = __shfl_sync(0xffffffffu, p, 0);
-                const bool run = __all_sync(0xffffffffu, p0 >= 0 && p == p0 + (int32_t)r16);
-                if (run && P.bulk_runs) {
+                if (!LIST && P.bulk_runs && livemask == 0xffffu) {
+                    /* a whole tile of a dense scan is one contiguous span of the store */
                     if (lane == 0) {
                         const uint32_t bar = bars + (it % RING_STAGES) * 8;
                         /* the stage was last read (and perhaps written) through the generic proxy */
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         ring_bar_expect(bar, 16 * RING_ROW);
-                        bulk_copy_g2s(st, kbase + (uint64_t)(uint32_t)p0 * tok_stride, 16 * RING_ROW, bar);
+                        bulk_copy_g2s(st, kbase + (uint64_t)(uint32_t)p * tok_stride, 16 * RING_ROW, bar);
                         asm volatile("st.shared.u32 [%0], %1;" ::"r"(st + RING_MASK_OFF), "r"(livemask | RING_RUN_BIT) : "memory");
                     }
                 } else {
-                    if (run) {
-                        const uint8_t *src = kbase + (uint64_t)(uint32_t)p0 * tok_stride + lane * 16;
-                        const uint32_t dst = st + lane * 16;
-                        cp_async16_at<0>(dst, src);    cp_async16_at<512>(dst, src);  cp_async16_at<1024>(dst, src);
-                        cp_async16_at<1536>(dst, src); cp_async16_at<2048>(dst, src); cp_async16_at<2560>(dst, src);
-                        cp_async16_at<3072>(dst, src); cp_async16_at<3584>(dst, src);
-                        if (lane < 16) cp_async16_at<4096>(dst, src);
-                    } else {
+                    /* two records per instruction: 16 lanes for the codes of one (K and V, 256 consecutive bytes) */
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) {
-                            const uint32_t row = 4 * j + (lane >> 3);
-                            const int32_t pr = __shfl_sync(0xffffffffu, p, row);
-                            cp_async16_kv<HD>(st + row * RING_ROW + c8 * 16, kbase + (uint64_t)(uint32_t)max(pr, 0) * tok_stride + c8 * 16, pr);
-                        }
-                        if (lane < 16)
-                            cp_async16(st + r16 * RING_ROW + 2 * HD, kbase + (uint64_t)(uint32_t)max(p, 0) * tok_stride + 2 * HD, p >= 0);
+                    for (uint32_t j = 0; j < 8; j++) {
+                        const uint32_t row = 2 * j + (lane >> 4);
+                        const int32_t pr = __shfl_sync(0xffffffffu, p, row);
+                        cp_async16_if(st + row * RING_ROW + r16 * 16, kbase + (uint64_t)(uint32_t)max(pr, 0) * tok_stride + r16 * 16, pr);
                     }
+                    if (lane < 16)
+                        cp_async16(st + r16 * RING_ROW + 2 * HD, kbase + (uint64_t)(uint32_t)max(p, 0) * tok_stride + 2 * HD, p >= 0);
                     if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(st + RING_MASK_OFF), "r"(livemask) : "memory");
                 }
             }
