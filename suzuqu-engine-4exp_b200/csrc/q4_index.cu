@@ -33,14 +33,31 @@ constexpr uint32_t IX_TK_THREADS = 1024, IX_MAX_KBLK = 512;
 /* ---- pool: one warp per block, lane l holds dims l, l+32, l+64, l+96 */
 __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *pool, const float *wn, uint32_t ratio,
                                                     uint32_t b0, uint32_t b1, uint32_t n_rot, float base, float eps,
-                                                    const int32_t *pp) {
+                                                    const int32_t *pp, bool early) {
     const uint32_t lane = threadIdx.x & 31u, w = blockIdx.x * 4u + (threadIdx.x >> 5);
+    if (!early) q4d_pdl_wait();
     if (pp) {   /* device position: the block this token completes, if any */
         const uint32_t pos = (uint32_t)*pp;
         b0 = pos / ratio;
         b1 = (pos + 1u) / ratio;
     }
     const uint32_t b = b0 + w;
+    /* the rotation depends on the block alone: a settled position's is taken under the previous kernel's tail */
+    float cs[4], sn[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const uint32_t d = lane + 32u * c;
+        cs[c] = 1.f;
+        sn[c] = 0.f;
+        if (b < b1 && (d & ~1u) < n_rot) {
+            const uint32_t p = d >> 1;
+            const float freq = powf(base, -(float)p / (float)(n_rot / 2u));
+            const float ang = (float)(b * ratio) * freq;
+            cs[c] = cosf(ang);
+            sn[c] = sinf(ang);
+        }
+    }
+    if (early) q4d_pdl_wait();
     if (b >= b1) return;
     const __half *src = raw + (size_t)b * ratio * IX_HD;
     float v[4], r[4];
@@ -66,15 +83,10 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
     for (int c = 0; c < 4; c++) {
         const uint32_t d = lane + 32u * c;
         const float other = __shfl_xor_sync(0xffffffffu, v[c], 1);
-        if ((d & ~1u) < n_rot) {
-            const uint32_t p = d >> 1;
-            const float freq = powf(base, -(float)p / (float)(n_rot / 2u));
-            const float ang = (float)(b * ratio) * freq;
-            const float cs = cosf(ang), sn = sinf(ang);
-            /* even dim: x0 * c - x1 * s; odd dim: x0 * s + x1 * c, with (x0, x1) the pair */
-            v[c] = (d & 1u) ? __fadd_rn(__fmul_rn(other, sn), __fmul_rn(v[c], cs))
-                            : __fsub_rn(__fmul_rn(v[c], cs), __fmul_rn(other, sn));
-        }
+        /* even dim: x0 * c - x1 * s; odd dim: x0 * s + x1 * c, with (x0, x1) the pair */
+        if ((d & ~1u) < n_rot)
+            v[c] = (d & 1u) ? __fadd_rn(__fmul_rn(other, sn[c]), __fmul_rn(v[c], cs[c]))
+                            : __fsub_rn(__fmul_rn(v[c], cs[c]), __fmul_rn(other, sn[c]));
         pool[(size_t)b * IX_HD + d] = v[c];
     }
 }
@@ -85,13 +97,6 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
  * fully coalesced, 16 KB in flight per warp while the previous tile is being scored -- and every lane
  * walks its own row there.  Rows are 132 floats apart: 16-byte reads of eight consecutive rows fall
  * into eight different bank groups, so the walk is conflict free; the query is read as a broadcast. */
-/* Programmatic dependent launch: the blocks of a launch may become resident while the previous kernel of
- * the stream drains; nothing the previous kernels write (position word, pool, scores, queries) is read
- * before this point.  A no-op for a launch without the attribute. */
-__device__ __forceinline__ void ix_pdl_sync() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 /* Q4_IX_PDL=0 switches it off for the score and selection launches */
 bool ix_pdl() {
     static int on = -1;
@@ -104,15 +109,16 @@ constexpr uint32_t SC_SMEM = SC_WARPS * 2u * SC_TILE_BYTES + IX_HD * sizeof(floa
 __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, const float *pool, float *score,
                                                                uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                                                                uint32_t pos0, uint32_t ratio, const int32_t *pp,
-                                                               const float *const *pools, const int32_t *pos_arr) {
+                                                               const float *const *pools, const int32_t *pos_arr, bool early) {
     extern __shared__ __align__(16) uint8_t sc_smem[];
     float4 *qs = reinterpret_cast<float4 *>(sc_smem);   /* [dim] = the 4 heads' values (0 for heads that do not exist) */
     const uint32_t t = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    ix_pdl_sync();
+    if (!early) q4d_pdl_wait();
     /* batched form: row t is session t, with its own pool and its own position */
     const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
-    if (pos_arr) pool = pools[t];
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    if (early) q4d_pdl_wait();
+    if (pos_arr) pool = pools[t];
     if (pp || pos_arr) n_blocks = min(n_vis, stride);      /* device position: the bound is derived here */
     const uint32_t buf0 = (uint32_t)__cvta_generic_to_shared(sc_smem + IX_HD * sizeof(float4)) + warp * 2u * SC_TILE_BYTES;
     const uint32_t lim = min(n_blocks, n_vis);                       /* rows to score */
@@ -344,7 +350,8 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = ix_pdl() ? 1 : 0;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr),
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr,
+                                                     !pos_arr && ix_pdl() && (!pp || q4i_settled(g_q4.pos_written))),
                      "qsa_score launch"));
 }
 
@@ -645,7 +652,7 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
     if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
     tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
-    ix_pdl_sync();
+    q4d_pdl_wait();
     /* the keys are requested before the position arrives: the row's storage reaches to `stride` whatever is visible */
     const float *row = score + (size_t)t * stride;
     const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
@@ -876,7 +883,7 @@ __global__ void __launch_bounds__(TKM_THREADS, 4) q4_ix_topkm_k(const float *sco
     TkmShared &S = *reinterpret_cast<TkmShared *>(tkm_smem);
     uint32_t *bg = reinterpret_cast<uint32_t *>(tkm_smem + sizeof(TkmShared)), *be = bg + words;   /* above / at the threshold */
     const uint32_t t = blockIdx.x, tx = threadIdx.x, lane = tx & 31u;
-    ix_pdl_sync();
+    q4d_pdl_wait();
     const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
@@ -1047,15 +1054,14 @@ bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
 extern "C" bool q4_hip_qsa_pool(const void *raw_f16, float *pool, const float *wn, uint32_t hd, uint32_t ratio,
                                 uint32_t b0, uint32_t b1, uint32_t n_rot, float rope_base, float eps) {
     if (!g_q4.ok || !raw_f16 || !pool || b1 <= b0 || hd != IX_HD || ratio == 0) return false;
-    q4_ix_pool_k<<<(b1 - b0 + 3u) / 4u, 128, 0, g_q4.stream>>>((const __half *)raw_f16, pool, wn, ratio, b0, b1, n_rot,
-                                                             rope_base, eps, nullptr);
-    return q4i_launched(q4i_check(cudaGetLastError(), "qsa_pool launch"));
+    return q4i_launch_pdl("qsa_pool launch", q4_ix_pool_k, dim3((b1 - b0 + 3u) / 4u), 128u, 0, (const __half *)raw_f16, pool, wn, ratio, b0, b1,
+                          n_rot, rope_base, eps, (const int32_t *)nullptr, true);
 }
 extern "C" bool q4_hip_qsa_pool_d(const void *raw, float *pool, const float *wn, uint32_t hd, uint32_t ratio,
                                   uint32_t n_rot, float rope_base, float eps) {
     if (!g_q4.ok || !g_q4.pos_d || !raw || !pool || hd != IX_HD || ratio == 0) return false;
-    q4_ix_pool_k<<<1, 128, 0, g_q4.stream>>>((const __half *)raw, pool, wn, ratio, 0, 0, n_rot, rope_base, eps, g_q4.pos_d);
-    return q4i_launched(q4i_check(cudaGetLastError(), "qsa_pool_d launch"));
+    return q4i_launch_pdl("qsa_pool_d launch", q4_ix_pool_k, dim3(1), 128u, 0, (const __half *)raw, pool, wn, ratio, 0u, 0u, n_rot, rope_base, eps,
+                          (const int32_t *)g_q4.pos_d, q4i_settled(g_q4.pos_written));
 }
 extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks,
                                  uint32_t stride, uint32_t n_head, uint32_t hd, uint32_t pos0, uint32_t ratio) {

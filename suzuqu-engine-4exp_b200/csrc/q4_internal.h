@@ -81,6 +81,27 @@ bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside captur
     } while (0)
 
 #ifdef __CUDACC__
+/* Programmatic dependent launch, kernel side: a block may become resident while the previous kernel of the stream drains;
+ * only what is settled (q4i_settled) is read before this.  Then the next kernel's blocks may come in. */
+__device__ __forceinline__ void q4d_pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+/* host side: a launch that may start so (the kernel calls q4d_pdl_wait in every thread) */
+template <typename K, typename... A>
+bool q4i_launch_pdl(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = g_q4.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), what));
+}
 /* ---- the q8_0 quantiser, one copy for every kernel that writes a cache row.  8 lanes share a block
  * of 32 values (4 each): d = amax / 127 and id = 1 / d as IEEE fp32 divisions, codes =
  * clamp(rint(x * id), +-127), stored scale = fp16(d) (quantize_row_q8_0's arithmetic,

@@ -27,6 +27,7 @@ struct AppendParams {
     const int32_t *pos;           /* device positions (per row if many, else one word) or null */
     uint32_t pos0;
     uint32_t *err;
+    uint32_t early;               /* the positions are settled */
 };
 
 __device__ __forceinline__ float4 load4(const float *p, bool aligned) {
@@ -36,6 +37,7 @@ __device__ __forceinline__ float4 load4(const float *p, bool aligned) {
 
 /* n floats -> n/32 reference blocks {fp16 scale, 32 x int8} at dst (2-byte aligned stores). */
 __global__ void q4_f32_to_q8_k(const float *src, uint8_t *dst, uint64_t nblocks, bool aligned) {
+    q4d_pdl_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t b = i >> 3;
     const uint32_t sub = (uint32_t)i & 7u;
@@ -54,6 +56,7 @@ __global__ void q4_f32_to_q8_k(const float *src, uint8_t *dst, uint64_t nblocks,
 
 __global__ void q4_f32_to_f16_k(const float *src, __half *dst, uint64_t n, const int32_t *pos,
                                 uint32_t stride) {
+    q4d_pdl_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pos) dst += (size_t)(uint32_t)*pos * stride;
     if (i < n) dst[i] = __float2half_rn(src[i]);
@@ -76,6 +79,7 @@ __global__ void q4_append_flat_k(uint8_t *kc, uint8_t *vc, const float *k, const
 /* Fused K+V append into a cache view.  blockIdx.y: 0 = K, 1 = V.  8 lanes per 32 values. */
 template <int LAY>
 __global__ void q4_append_k(const AppendParams P) {
+    if (!P.early) q4d_pdl_wait();
     const uint32_t nb = P.hd / 32u;
     const uint32_t per_row = P.n_kvh * nb * 8u;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -84,6 +88,9 @@ __global__ void q4_append_k(const AppendParams P) {
     const uint32_t sub = w & 7u, blk = w >> 3, kh = blk / nb, b = blk % nb;
     const bool which = blockIdx.y != 0;
     bool live = r < P.n_rows;
+    uint32_t at = P.pos0 + r;
+    if (P.pos && live) at = (uint32_t)P.pos[P.many ? r : 0] + (P.many ? 0u : r);
+    if (P.early) q4d_pdl_wait();
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (live) x = *reinterpret_cast<const float4 *>((which ? P.v : P.k) + (size_t)r * P.n_kvh * P.hd +
                                                      (size_t)blk * 32 + sub * 4);
@@ -91,7 +98,7 @@ __global__ void q4_append_k(const AppendParams P) {
     if (LAY == LAY_Q8P || LAY == LAY_Q8R) q4d_block_scale(x, d, id);
     if (!live) return;
     const Q4Cache C = P.many ? P.many[r] : P.one;
-    const uint32_t p = P.pos ? (uint32_t)P.pos[P.many ? r : 0] + (P.many ? 0u : r) : P.pos0 + r;
+    const uint32_t p = at;
     if (p >= C.max_kv) {
         if (w == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
         return;
@@ -190,12 +197,11 @@ bool launch_append(const AppendParams &p, int layout) {
     const uint64_t threads = (uint64_t)p.n_rows * p.n_kvh * (p.hd / 32u) * 8u;
     dim3 grid((unsigned)((threads + 255) / 256), 2);
     switch (layout) {
-    case LAY_Q8P: q4_append_k<LAY_Q8P><<<grid, 256, 0, g_q4.stream>>>(p); break;
-    case LAY_Q8R: q4_append_k<LAY_Q8R><<<grid, 256, 0, g_q4.stream>>>(p); break;
-    case LAY_F16: q4_append_k<LAY_F16><<<grid, 256, 0, g_q4.stream>>>(p); break;
-    default: q4_append_k<LAY_F32><<<grid, 256, 0, g_q4.stream>>>(p); break;
+    case LAY_Q8P: return q4i_launch_pdl("append launch", q4_append_k<LAY_Q8P>, grid, 256u, 0, p);
+    case LAY_Q8R: return q4i_launch_pdl("append launch", q4_append_k<LAY_Q8R>, grid, 256u, 0, p);
+    case LAY_F16: return q4i_launch_pdl("append launch", q4_append_k<LAY_F16>, grid, 256u, 0, p);
     }
-    return q4i_launched(q4i_check(cudaGetLastError(), "append launch"));
+    return q4i_launch_pdl("append launch", q4_append_k<LAY_F32>, grid, 256u, 0, p);
 }
 
 }  // namespace
@@ -206,20 +212,17 @@ extern "C" bool q4_hip_f32_to_q8(void *dst_q8, const float *src, uint64_t n) {
     if (!g_q4.ok || !dst_q8 || !src || n == 0 || (n % 32u) != 0) return false;
     const uint64_t nb = n / 32u;
     const uint64_t threads = nb * 8u;
-    q4_f32_to_q8_k<<<(unsigned)((threads + 255) / 256), 256, 0, g_q4.stream>>>(
-        src, (uint8_t *)dst_q8, nb, ((uintptr_t)src & 15u) == 0);
-    return q4i_check(cudaGetLastError(), "f32_to_q8 launch");
+    return q4i_launch_pdl("f32_to_q8 launch", q4_f32_to_q8_k, dim3((unsigned)((threads + 255) / 256)), 256u, 0, src, (uint8_t *)dst_q8, nb,
+                          ((uintptr_t)src & 15u) == 0);
 }
 extern "C" bool q4_hip_f32_to_f16(void *dst_f16, const float *src, uint64_t n) {
     if (!g_q4.ok || !dst_f16 || !src || !n) return false;
-    q4_f32_to_f16_k<<<(unsigned)((n + 255) / 256), 256, 0, g_q4.stream>>>(src, (__half *)dst_f16, n, nullptr, 0);
-    return q4i_check(cudaGetLastError(), "f32_to_f16 launch");
+    return q4i_launch_pdl("f32_to_f16 launch", q4_f32_to_f16_k, dim3((unsigned)((n + 255) / 256)), 256u, 0, src, (__half *)dst_f16, n, (const int32_t *)nullptr, 0u);
 }
 extern "C" bool q4_hip_f32_to_f16_d(void *dst_base, uint32_t stride_elems, const float *src, uint64_t n) {
     if (!g_q4.ok || !g_q4.pos_d || !dst_base || !src || !n) return false;
-    q4_f32_to_f16_k<<<(unsigned)((n + 255) / 256), 256, 0, g_q4.stream>>>(src, (__half *)dst_base, n,
-                                                                         g_q4.pos_d, stride_elems);
-    return q4i_check(cudaGetLastError(), "f32_to_f16_d launch");
+    return q4i_launch_pdl("f32_to_f16_d launch", q4_f32_to_f16_k, dim3((unsigned)((n + 255) / 256)), 256u, 0, src, (__half *)dst_base, n,
+                          (const int32_t *)g_q4.pos_d, stride_elems);
 }
 /* The reference treats the token row as n flat floats at cache + pos*bpt; as a view that is one
  * kv head of width n. */
@@ -252,6 +255,7 @@ extern "C" bool q4_hip_kv_append_d(void *kcache, void *vcache, const float *k, c
     p.v = v;
     p.pos = g_q4.pos_d;
     p.err = g_q4.err_d;
+    p.early = q4i_settled(g_q4.pos_written);
     return launch_append(p, ref_layout(kind));
 }
 
@@ -397,7 +401,7 @@ extern "C" bool q4_gpu_kv_append(q4_gpu_kv *kv, uint32_t layer, const float *k, 
     AppendParams p;
     memset(&p, 0, sizeof(p));
     p.one = kv->view; p.layer = layer; p.n_rows = n_tok; p.n_kvh = kv->n_kvh; p.hd = kv->hd;
-    p.k = k; p.v = v; p.pos0 = pos0; p.err = g_q4.err_d;
+    p.k = k; p.v = v; p.pos0 = pos0; p.err = g_q4.err_d; p.early = 1;
     const bool ok = launch_append(p, store_layout(kv->kind));
     q4i_kv_written(kv, layer);
     return ok;
@@ -408,7 +412,7 @@ extern "C" bool q4_gpu_kv_append_d(q4_gpu_kv *kv, uint32_t layer, const float *k
     AppendParams p;
     memset(&p, 0, sizeof(p));
     p.one = kv->view; p.layer = layer; p.n_rows = 1; p.n_kvh = kv->n_kvh; p.hd = kv->hd;
-    p.k = k; p.v = v; p.pos = g_q4.pos_d; p.err = g_q4.err_d;
+    p.k = k; p.v = v; p.pos = g_q4.pos_d; p.err = g_q4.err_d; p.early = q4i_settled(g_q4.pos_written);
     const bool ok = launch_append(p, store_layout(kv->kind));
     q4i_kv_written(kv, layer);
     return ok;
@@ -696,7 +700,7 @@ extern "C" bool q4_gpu_batch_append(q4_gpu_batch *b, uint32_t layer, const float
     AppendParams p;
     memset(&p, 0, sizeof(p));
     p.many = b->d_views; p.layer = layer; p.n_rows = b->n_active; p.n_kvh = b->kv[0]->n_kvh; p.hd = b->kv[0]->hd;
-    p.k = k; p.v = v; p.pos = b->pos_d; p.err = g_q4.err_d;
+    p.k = k; p.v = v; p.pos = b->pos_d; p.err = g_q4.err_d; p.early = q4i_settled(b->pos_written);
     const bool ok = launch_append(p, store_layout(b->kv[0]->kind));
     batch_written(b, layer);
     return ok;

@@ -195,13 +195,6 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 
-/* Programmatic dependent launch: a block may become resident while the previous kernel of the stream drains; nothing
- * that the stream writes is read before this point. */
-__device__ __forceinline__ void pf_pdl_sync() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 /* ---- staging: rows [0, n) of (layer, kv head) -> operand images.  Per tile of 128 positions: KP * HD / 128 images of
  * K (128 rows x 128 dims: two blocks of 64 dims, rows of 128 bytes), then HD / 128 images' worth of V^T (two blocks of
  * 64 positions x HD dims).  Rows behind n are zero.  Block = 32 positions of one kv head, K or V (blockIdx.z); V goes
@@ -245,7 +238,7 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
     constexpr uint32_t CK = KP * HD / 128, CV = HD / 128, PER = HD * 32u / 8u / 256u;   /* groups of 8 dims per thread */
     __shared__ __half tile[HD * PITCH];
     const uint32_t kh = blockIdx.y, p0 = blockIdx.x * 32u, tid = threadIdx.x;
-    pf_pdl_sync();
+    q4d_pdl_wait();
     const uint8_t *sc = LAY == LAY_Q8P ? C.s + (uint64_t)layer * C.s_layer_stride + (uint64_t)kh * C.s_kvh_stride : nullptr;
     const uint64_t base = (uint64_t)layer * C.layer_stride + (uint64_t)kh * C.kvh_stride;
     float x[PER][8];
@@ -364,7 +357,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    pf_pdl_sync();
+    q4d_pdl_wait();
     if (warp < SW) {
         /* ---- queries as fp16 (exact for normal bf16 values), K-major swizzled, blocks of 64 dims: 8 dims per thread
          * and step, whole rows per warp step */
@@ -733,7 +726,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
 /* ---- the parts of split position ranges -> out: thread = 4 dims of one (token, head) */
 __global__ void __launch_bounds__(256) q4_pf_merge_k(const PrefillParams P, uint32_t hd, uint64_t total4) {
     const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
-    pf_pdl_sync();
+    q4d_pdl_wait();
     if (i >= total4) return;
     const uint64_t row = i / (hd / 4u), rows = (uint64_t)P.n_tok * P.n_head;
     float M = -CUDART_INF_F;
@@ -780,21 +773,6 @@ bool stage_reserve(size_t bytes) {
     return true;
 }
 
-template <typename K, typename... A>
-bool pf_start(K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = g_q4.stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prefill launch"));
-}
 template <int HD, int NQ, int KP>
 bool attend(const PrefillParams &p, dim3 grid) {
     static bool attr = false;
@@ -802,11 +780,11 @@ bool attend(const PrefillParams &p, dim3 grid) {
                             "prefill smem attribute"))
         return false;
     attr = true;
-    return pf_start(q4_prefill_k<HD, NQ, KP>, grid, NQ * 128u + 64u, PF_SMEM, p);
+    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, KP>, grid, NQ * 128u + 64u, PF_SMEM, p);
 }
 template <int LAY, int HD, int KP>
 bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
-    return pf_start(q4_pf_stage_k<LAY, HD, KP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
+    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, KP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
 }
 
 }  // namespace
@@ -862,7 +840,7 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     else ok = kp == 2 ? attend<128, 1, 2>(p, grid) : attend<128, 1, 1>(p, grid);
     if (ok && split > 1) {
         const uint64_t total4 = (uint64_t)rows * hd / 4u;
-        ok = pf_start(q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4);
+        ok = q4i_launch_pdl("prefill launch", q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4);
     }
     return ok ? 1 : 0;
 }

@@ -69,10 +69,6 @@ __global__ void q4_k_prep_k(float *k, const float *wn, uint32_t hd, uint32_t n_r
 
 /* ---- one warp per head */
 constexpr uint32_t PREP_WARPS = 8;
-__device__ __forceinline__ void prep_pdl_sync() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 /* cos and sin of the token's rotation of pair p, by thread p of the block; np <= 128 */
 __device__ __forceinline__ void rope_table(float2 *cs, uint32_t np, int32_t pos, float base) {
     const uint32_t p = threadIdx.x;
@@ -136,11 +132,12 @@ __device__ __forceinline__ void row_store(float *dst, const float2 (&v)[HD / 64]
 template <int HD, bool SPLIT>
 __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *src, const float *wn, float *q, float *g, uint32_t n_rot,
                                                                   int32_t pos0, float base, float eps, uint32_t n_head, uint32_t per,
-                                                                  const int32_t *pp) {
+                                                                  const int32_t *pp, bool early) {
     __shared__ float2 cs[128];
     const uint32_t t = blockIdx.y, warp = threadIdx.x >> 5, h0 = blockIdx.x * per, h1 = min(h0 + per, n_head);
-    prep_pdl_sync();
-    rope_table(cs, n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base);
+    if (!early) q4d_pdl_wait();
+    rope_table(cs, n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base);   /* a settled position's under the previous kernel's tail */
+    if (early) q4d_pdl_wait();
     __syncthreads();
     for (uint32_t h = h0 + warp; h < h1; h += PREP_WARPS) {
         const size_t row = (size_t)t * n_head + h;
@@ -156,20 +153,6 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *s
     }
 }
 
-template <typename K, typename... A>
-bool prep_start(K kernel, dim3 grid, uint32_t threads, A... args) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.stream = g_q4.stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "prep launch"));
-}
 /* false in `done` where the head size or an address is not the warp form's */
 template <bool SPLIT>
 bool prep_rows(const float *src, const float *wn, float *q, float *g, uint32_t n_head, uint32_t hd, uint32_t n_rot, int32_t pos0, float base,
@@ -179,9 +162,10 @@ bool prep_rows(const float *src, const float *wn, float *q, float *g, uint32_t n
     /* one token: its heads over several SMs, eight to a block; many tokens: one block each */
     const uint32_t per = n_tok < (uint32_t)g_q4.sm_count ? PREP_WARPS : n_head;
     const dim3 grid((n_head + per - 1u) / per, n_tok);
-    if (hd == 64) return prep_start(q4_prep_rows_k<64, SPLIT>, grid, PREP_WARPS * 32u, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp);
-    if (hd == 128) return prep_start(q4_prep_rows_k<128, SPLIT>, grid, PREP_WARPS * 32u, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp);
-    return prep_start(q4_prep_rows_k<256, SPLIT>, grid, PREP_WARPS * 32u, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp);
+    const bool early = !pp || q4i_settled(g_q4.pos_written);
+    if (hd == 64) return q4i_launch_pdl("prep launch", q4_prep_rows_k<64, SPLIT>, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp, early);
+    if (hd == 128) return q4i_launch_pdl("prep launch", q4_prep_rows_k<128, SPLIT>, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp, early);
+    return q4i_launch_pdl("prep launch", q4_prep_rows_k<256, SPLIT>, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp, early);
 }
 bool q_prep(const float *qg, const float *wn, float *q, float *g, uint32_t n_head, uint32_t hd, uint32_t n_rot, int32_t pos0, float base,
             float eps, uint32_t n_tok, const int32_t *pp) {
@@ -251,6 +235,7 @@ struct PrepAppendParams {
     int32_t pos0;
     float base, eps;
     uint32_t *err;
+    uint32_t early;          /* the position is settled */
 };
 
 /* head sizes 32 and 64: a block per (row, K or V) */
@@ -300,9 +285,10 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_append_rows_k(const P
     __shared__ float2 cs[128];
     __shared__ __align__(16) float row_s[PREP_WARPS][HD];
     const uint32_t t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    prep_pdl_sync();
+    if (!P.early) q4d_pdl_wait();
     const int32_t pos = (P.pos ? *P.pos : P.pos0) + (int32_t)t;
     rope_table(cs, P.n_rot / 2u, pos, P.base);
+    if (P.early) q4d_pdl_wait();
     __syncthreads();
     if (pos < 0 || (uint32_t)pos >= P.C.max_kv) {
         if (threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
@@ -351,9 +337,10 @@ bool prep_append_launch(q4_gpu_kv *kv, uint32_t layer, const float *k, const flo
     p.layout = kv->kind == Q4K_Q8 ? LAY_Q8P : kv->kind == Q4K_F16 ? LAY_F16 : LAY_F32;
     p.layer = layer; p.n_kvh = kv->n_kvh; p.hd = kv->hd; p.n_rot = n_rot; p.n_tok = n_tok;
     p.k = k; p.v = v; p.wn = wn; p.pos = pos_dev; p.pos0 = pos0; p.base = base; p.eps = eps; p.err = g_q4.err_d;
+    p.early = !pos_dev || q4i_settled(g_q4.pos_written);
     if ((kv->hd == 128 || kv->hd == 256) && (((uintptr_t)k | (uintptr_t)v) & 7u) == 0)
-        return kv->hd == 128 ? prep_start(q4_prep_append_rows_k<128>, dim3(n_tok), PREP_WARPS * 32u, p)
-                             : prep_start(q4_prep_append_rows_k<256>, dim3(n_tok), PREP_WARPS * 32u, p);
+        return kv->hd == 128 ? q4i_launch_pdl("kv_prep_append launch", q4_prep_append_rows_k<128>, dim3(n_tok), PREP_WARPS * 32u, 0, p)
+                             : q4i_launch_pdl("kv_prep_append launch", q4_prep_append_rows_k<256>, dim3(n_tok), PREP_WARPS * 32u, 0, p);
     q4_prep_append_k<<<dim3(kv->n_kvh, n_tok, 2), 128, 0, g_q4.stream>>>(p);
     return q4i_check(cudaGetLastError(), "kv_prep_append launch");
 }
