@@ -106,24 +106,20 @@ bool ix_pdl() {
 constexpr uint32_t SC_ROW_FLOATS = IX_HD + 4, SC_WARPS = 2;
 constexpr uint32_t SC_TILE_BYTES = 32u * SC_ROW_FLOATS * sizeof(float);
 constexpr uint32_t SC_SMEM = SC_WARPS * 2u * SC_TILE_BYTES + IX_HD * sizeof(float4);
+/* BATCH: sessions with a pool and a position of their own.  Their tiles are counted through, and every block takes an equal
+ * share of the whole, which may end in one session and begin in the next (an equal number of blocks per session leaves
+ * most of them idle while the longest context is scanned). */
+template <bool BATCH>
 __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, const float *pool, float *score,
                                                                uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                                                                uint32_t pos0, uint32_t ratio, const int32_t *pp,
-                                                               const float *const *pools, const int32_t *pos_arr, bool early) {
+                                                               const float *const *pools, const int32_t *pos_arr, uint32_t n_sess, bool early) {
     extern __shared__ __align__(16) uint8_t sc_smem[];
     float4 *qs = reinterpret_cast<float4 *>(sc_smem);   /* [dim] = the 4 heads' values (0 for heads that do not exist) */
-    const uint32_t t = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    if (!early) q4d_pdl_wait();
-    /* batched form: row t is session t, with its own pool and its own position */
-    const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
-    const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
-    if (early) q4d_pdl_wait();
-    if (pos_arr) pool = pools[t];
-    if (pp || pos_arr) n_blocks = min(n_vis, stride);      /* device position: the bound is derived here */
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t buf0 = (uint32_t)__cvta_generic_to_shared(sc_smem + IX_HD * sizeof(float4)) + warp * 2u * SC_TILE_BYTES;
-    const uint32_t lim = min(n_blocks, n_vis);                       /* rows to score */
-    const uint32_t n_tiles = (lim + 31u) / 32u;
-    const uint32_t step = gridDim.x * SC_WARPS, first = blockIdx.x * SC_WARPS + warp;
+    /* rows [0, lim) of token t's pool, tiles of 32: first, first + step, .. below n_tiles */
+    auto scan = [&](uint32_t t, const float *pool, uint32_t lim, uint32_t first, uint32_t n_tiles, uint32_t step) {
     auto fetch = [&](uint32_t tile, uint32_t which) {
         if (tile < n_tiles) {
             const uint32_t r0 = tile * 32u, rows = min(32u, lim - r0);
@@ -178,6 +174,45 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
         __syncwarp();   /* every lane is done with this buffer before the fetch after next refills it */
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    };
+    if (BATCH) {
+        q4d_pdl_wait();
+        auto rows_of = [&](uint32_t t) -> uint32_t { return min(((uint32_t)pos_arr[t] + 1u) / ratio, stride); };
+        uint64_t total = 0;
+        for (uint32_t t0 = 0; t0 < n_sess; t0 += 32u) total += __reduce_add_sync(0xffffffffu, t0 + lane < n_sess ? (rows_of(t0 + lane) + 31u) / 32u : 0u);
+        const uint64_t share0 = total * blockIdx.x / gridDim.x, share1 = total * (blockIdx.x + 1u) / gridDim.x;
+        uint64_t at = 0;   /* tiles of the sessions before */
+        bool again = false;
+        for (uint32_t t0 = 0; t0 < n_sess && at < share1; t0 += 32u) {
+            const uint32_t rows = t0 + lane < n_sess ? rows_of(t0 + lane) : 0u, tiles = (rows + 31u) / 32u;
+            uint32_t incl = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            uint32_t mine = __ballot_sync(0xffffffffu, tiles && at + incl > share0 && at + incl - tiles < share1);
+            for (; mine; mine &= mine - 1u) {
+                const int l = __ffs(mine) - 1;
+                const uint64_t begin = at + __shfl_sync(0xffffffffu, incl - tiles, l);
+                const uint32_t n = __shfl_sync(0xffffffffu, tiles, l), lim = __shfl_sync(0xffffffffu, rows, l), t = t0 + (uint32_t)l;
+                const uint32_t first = begin < share0 ? (uint32_t)(share0 - begin) : 0u, last = begin + n > share1 ? (uint32_t)(share1 - begin) : n;
+                if (again) __syncthreads();   /* the other warp is done with the query of the session before */
+                again = true;
+                scan(t, pools[t], lim, first + warp, last, SC_WARPS);
+            }
+            at += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        return;
+    }
+    const uint32_t t = blockIdx.y;
+    if (!early) q4d_pdl_wait();
+    const uint32_t pos = (pp ? (uint32_t)*pp : pos0) + t;
+    const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    if (early) q4d_pdl_wait();
+    if (pp) n_blocks = min(n_vis, stride);      /* device position: the bound is derived here */
+    const uint32_t lim = min(n_blocks, n_vis);  /* rows to score */
+    scan(t, pool, lim, blockIdx.x * SC_WARPS + warp, (lim + 31u) / 32u, gridDim.x * SC_WARPS);
     /* blocks the token cannot see (host-position form only): -1e30 */
     for (uint32_t b = n_vis + blockIdx.x * (SC_WARPS * 32u) + threadIdx.x; b < n_blocks; b += gridDim.x * SC_WARPS * 32u)
         score[(size_t)t * stride + b] = -1.0e30f;
@@ -322,26 +357,26 @@ bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n
     q4_ix_score_mt_k<JC><<<grid, SM_THREADS, sm_smem<JC>(), g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     return q4i_launched(q4i_check(cudaGetLastError(), "qsa_score launch"));
 }
+template <bool BATCH>
 bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
-                  uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp,
-                  const float *const *pools = nullptr, const int32_t *pos_arr = nullptr) {
+                  uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, const float *const *pools, const int32_t *pos_arr) {
     static bool done = false;
     if (!done) {
-        if (!q4i_check(cudaFuncSetAttribute(q4_ix_score_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM),
+        if (!q4i_check(cudaFuncSetAttribute(q4_ix_score_k<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM),
                        "qsa_score smem attribute"))
             return false;
         done = true;
     }
-    /* persistent grid: 3 blocks of 2 warps per SM share 227 KB; fewer when the row is short */
-    const uint32_t rows = pp || pos_arr ? stride : n_blocks;
+    /* persistent grid: 3 blocks of 2 warps per SM share 227 KB; fewer when the rows are short */
+    const uint64_t rows = (uint64_t)(pp || BATCH ? stride : n_blocks) * (BATCH ? n_tok : 1u);
     uint32_t gx = (uint32_t)g_q4.sm_count * 3u;
-    const uint32_t need = (rows + SC_WARPS * 32u - 1u) / (SC_WARPS * 32u);
-    if (n_tok > 1) gx = (gx + n_tok - 1u) / n_tok;
-    if (gx > need) gx = need;
+    const uint64_t need = (rows + SC_WARPS * 32u - 1u) / (SC_WARPS * 32u);
+    if (!BATCH && n_tok > 1) gx = (gx + n_tok - 1u) / n_tok;
+    if (gx > need) gx = (uint32_t)need;
     if (gx < 1) gx = 1;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(gx, n_tok);
+    cfg.gridDim = dim3(gx, BATCH ? 1u : n_tok);
     cfg.blockDim = dim3(SC_WARPS * 32);
     cfg.dynamicSmemBytes = SC_SMEM;
     cfg.stream = g_q4.stream;
@@ -350,8 +385,8 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = ix_pdl() ? 1 : 0;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr,
-                                                     !pos_arr && ix_pdl() && (!pp || q4i_settled(g_q4.pos_written))),
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k<BATCH>, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr,
+                                                     n_tok, ix_pdl() && (!pp || q4i_settled(g_q4.pos_written))),
                      "qsa_score launch"));
 }
 
@@ -1072,7 +1107,7 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
         if (wide <= narrow && wide < scan) return score_mt_launch<16>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
         if (narrow < scan) return score_mt_launch<8>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     }
-    return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr);
+    return score_launch<false>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr, nullptr, nullptr);
 }
 /* Device position (graph-captured decode): the grid covers `stride` blocks, the bound comes from the
  * position word inside the kernel. */
@@ -1080,7 +1115,7 @@ extern "C" bool q4_hip_qsa_score_d(const float *q, const float *pool, float *sco
                                    uint32_t hd, uint32_t ratio) {
     if (!g_q4.ok || !g_q4.pos_d || !q || !pool || !score || hd != IX_HD || n_head == 0 || n_head > 4 || stride == 0)
         return false;
-    return score_launch(q, pool, score, 1, 0, stride, n_head, 0, ratio, g_q4.pos_d);
+    return score_launch<false>(q, pool, score, 1, 0, stride, n_head, 0, ratio, g_q4.pos_d, nullptr, nullptr);
 }
 extern "C" bool q4_hip_qsa_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
                                 uint32_t k_blk, uint32_t ratio, uint32_t pos0, uint32_t width) {
@@ -1106,6 +1141,6 @@ extern "C" bool q4_gpu_qsa_select_batch(const float *const *pools, const int32_t
     Q4_REQUIRE(pools && pos && q && score && sel && n_sess && stride && ratio && width, "qsa_select_batch: bad argument");
     Q4_REQUIRE(hd == IX_HD && n_head >= 1 && n_head <= 4 && k_blk >= 1 && k_blk <= IX_MAX_KBLK,
                "qsa_select_batch: unsupported shape");
-    return score_launch(q, nullptr, score, n_sess, 0, stride, n_head, 0, ratio, nullptr, pools, pos) &&
+    return score_launch<true>(q, nullptr, score, n_sess, 0, stride, n_head, 0, ratio, nullptr, pools, pos) &&
            launch_topk(score, sel, n_sess, stride, k_blk, ratio, 0, width, nullptr, pos);
 }
