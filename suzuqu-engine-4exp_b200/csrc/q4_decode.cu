@@ -2178,6 +2178,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
             p.push_async = 1u;
             grid.x = min(grid.x / p.cluster * p.cluster, fit);
             p.S = grid.x;
+            p.mid_splits = min(p.mid_splits, p.S);
             p.small_steps = (LAY == LAY_F32 ? 3u : 4u) * p.cluster * DEC_WARPS;
         } else {
             p.cluster = p.push_bytes = 0;

@@ -69,10 +69,9 @@ __global__ void q4_k_prep_k(float *k, const float *wn, uint32_t hd, uint32_t n_r
 
 /* ---- one warp per head */
 constexpr uint32_t PREP_WARPS = 8;
-/* cos and sin of the token's rotation of pair p, by thread p of the block; np <= 128 */
-__device__ __forceinline__ void rope_table(float2 *cs, uint32_t np, int32_t pos, float base) {
-    const uint32_t p = threadIdx.x;
-    if (p < np) {
+/* cos and sin of a token's rotation of pair p, by thread p of `threads`; np <= 128 */
+__device__ __forceinline__ void rope_table(float2 *cs, uint32_t np, int32_t pos, float base, uint32_t p, uint32_t threads) {
+    for (; p < np; p += threads) {
         const float freq = powf(base, -(float)p / (float)np);
         const float ang = (float)pos * freq;
         cs[p] = make_float2(cosf(ang), sinf(ang));
@@ -128,18 +127,21 @@ __device__ __forceinline__ void row_store(float *dst, const float2 (&v)[HD / 64]
     for (int k = 0; k < HD / 64; k++) reinterpret_cast<float2 *>(dst)[32 * k + lane] = v[k];
 }
 /* SPLIT: rows are [q | gate] pairs, q goes to `q` and the gate to `g`; else rows of `q` in place.  blockIdx.x: a group of
- * `per` heads, blockIdx.y: token. */
-template <int HD, bool SPLIT>
+ * `per` heads, blockIdx.y: TOK tokens (several where a token has few heads: a block with 2 rows for its 8 warps is mostly
+ * the wait for its rotation table). */
+template <int HD, bool SPLIT, uint32_t TOK>
 __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *src, const float *wn, float *q, float *g, uint32_t n_rot,
                                                                   int32_t pos0, float base, float eps, uint32_t n_head, uint32_t per,
-                                                                  const int32_t *pp, bool early) {
-    __shared__ float2 cs[128];
-    const uint32_t t = blockIdx.y, warp = threadIdx.x >> 5, h0 = blockIdx.x * per, h1 = min(h0 + per, n_head);
+                                                                  uint32_t n_tok, const int32_t *pp, bool early) {
+    __shared__ float2 cs[TOK][128];
+    constexpr uint32_t W = PREP_WARPS / TOK;   /* warps of a token */
+    const uint32_t warp = threadIdx.x >> 5, sub = warp / W, t = blockIdx.y * TOK + sub, h0 = blockIdx.x * per, h1 = min(h0 + per, n_head);
     if (!early) q4d_pdl_wait();
-    rope_table(cs, n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base);   /* a settled position's under the previous kernel's tail */
+    rope_table(cs[sub], n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base, threadIdx.x % (W * 32u), W * 32u);   /* a settled position's under the previous kernel's tail */
     if (early) q4d_pdl_wait();
     __syncthreads();
-    for (uint32_t h = h0 + warp; h < h1; h += PREP_WARPS) {
+    if (t >= n_tok) return;
+    for (uint32_t h = h0 + warp % W; h < h1; h += W) {
         const size_t row = (size_t)t * n_head + h;
         float2 v[HD / 64];
         row_load<HD>(SPLIT ? src + row * 2u * HD : q + row * HD, v);
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *s
             row_load<HD>(src + row * 2u * HD + HD, w);
             row_store<HD>(g + row * HD, w);
         }
-        row_norm_rope<HD>(v, wn, cs, n_rot / 2u, eps);
+        row_norm_rope<HD>(v, wn, cs[sub], n_rot / 2u, eps);
         row_store<HD>(q + row * HD, v);
     }
 }
@@ -159,13 +161,17 @@ bool prep_rows(const float *src, const float *wn, float *q, float *g, uint32_t n
                float eps, uint32_t n_tok, const int32_t *pp, bool &done) {
     done = (hd == 64 || hd == 128 || hd == 256) && (((uintptr_t)src | (uintptr_t)q | (uintptr_t)g) & 7u) == 0;
     if (!done) return false;
-    /* one token: its heads over several SMs, eight to a block; many tokens: one block each */
+    /* few tokens: a token's heads over several SMs, eight to a block; many: one block each, or four where heads are few */
+    const bool four = n_tok >= 2u * (uint32_t)g_q4.sm_count && n_head <= 4u;
     const uint32_t per = n_tok < (uint32_t)g_q4.sm_count ? PREP_WARPS : n_head;
-    const dim3 grid((n_head + per - 1u) / per, n_tok);
+    const dim3 grid((n_head + per - 1u) / per, four ? (n_tok + 3u) / 4u : n_tok);
     const bool early = !pp || q4i_settled(g_q4.pos_written);
-    if (hd == 64) return q4i_launch_pdl("prep launch", q4_prep_rows_k<64, SPLIT>, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp, early);
-    if (hd == 128) return q4i_launch_pdl("prep launch", q4_prep_rows_k<128, SPLIT>, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp, early);
-    return q4i_launch_pdl("prep launch", q4_prep_rows_k<256, SPLIT>, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, pp, early);
+    auto start = [&](auto kernel) {
+        return q4i_launch_pdl("prep launch", kernel, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, n_tok, pp, early);
+    };
+    if (hd == 64) return four ? start(q4_prep_rows_k<64, SPLIT, 4>) : start(q4_prep_rows_k<64, SPLIT, 1>);
+    if (hd == 128) return four ? start(q4_prep_rows_k<128, SPLIT, 4>) : start(q4_prep_rows_k<128, SPLIT, 1>);
+    return four ? start(q4_prep_rows_k<256, SPLIT, 4>) : start(q4_prep_rows_k<256, SPLIT, 1>);
 }
 bool q_prep(const float *qg, const float *wn, float *q, float *g, uint32_t n_head, uint32_t hd, uint32_t n_rot, int32_t pos0, float base,
             float eps, uint32_t n_tok, const int32_t *pp) {
@@ -278,28 +284,30 @@ __global__ void q4_prep_append_k(const PrepAppendParams P) {
     }
 }
 
-/* Head sizes 128 and 256: a block per token, a warp per row (K heads, then V heads), the rotation once per token.  The row
+/* Head sizes 128 and 256: a block per TOK tokens, a warp per row (K heads, then V heads), the rotation once per token.  The row
  * passes through the warp's part of shared memory to be quantised eight lanes per 32 values, as everywhere. */
-template <int HD>
+template <int HD, uint32_t TOK>
 __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_append_rows_k(const PrepAppendParams P) {
-    __shared__ float2 cs[128];
+    __shared__ float2 cs[TOK][128];
+    constexpr uint32_t W = PREP_WARPS / TOK;   /* warps of a token */
     __shared__ __align__(16) float row_s[PREP_WARPS][HD];
-    const uint32_t t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, sub = warp / W, t = blockIdx.x * TOK + sub;
     if (!P.early) q4d_pdl_wait();
     const int32_t pos = (P.pos ? *P.pos : P.pos0) + (int32_t)t;
-    rope_table(cs, P.n_rot / 2u, pos, P.base);
+    rope_table(cs[sub], P.n_rot / 2u, pos, P.base, threadIdx.x % (W * 32u), W * 32u);
     if (P.early) q4d_pdl_wait();
     __syncthreads();
+    if (t >= P.n_tok) return;
     if (pos < 0 || (uint32_t)pos >= P.C.max_kv) {
-        if (threadIdx.x == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
+        if (lane == 0) atomicOr(P.err, (uint32_t)Q4E_RANGE);
         return;
     }
-    for (uint32_t r = warp; r < 2u * P.n_kvh; r += PREP_WARPS) {
+    for (uint32_t r = warp % W; r < 2u * P.n_kvh; r += W) {
         const bool which = r >= P.n_kvh;
         const uint32_t kh = which ? r - P.n_kvh : r;
         float2 v[HD / 64];
         row_load<HD>((which ? P.v : P.k) + ((size_t)t * P.n_kvh + kh) * HD, v);
-        if (!which) row_norm_rope<HD>(v, P.wn, cs, P.n_rot / 2u, P.eps);
+        if (!which) row_norm_rope<HD>(v, P.wn, cs[sub], P.n_rot / 2u, P.eps);
         __syncwarp();
         row_store<HD>(row_s[warp], v);
         __syncwarp();
@@ -339,8 +347,13 @@ bool prep_append_launch(q4_gpu_kv *kv, uint32_t layer, const float *k, const flo
     p.k = k; p.v = v; p.wn = wn; p.pos = pos_dev; p.pos0 = pos0; p.base = base; p.eps = eps; p.err = g_q4.err_d;
     p.early = !pos_dev || q4i_settled(g_q4.pos_written);
     if ((kv->hd == 128 || kv->hd == 256) && (((uintptr_t)k | (uintptr_t)v) & 7u) == 0)
-        return kv->hd == 128 ? q4i_launch_pdl("kv_prep_append launch", q4_prep_append_rows_k<128>, dim3(n_tok), PREP_WARPS * 32u, 0, p)
-                             : q4i_launch_pdl("kv_prep_append launch", q4_prep_append_rows_k<256>, dim3(n_tok), PREP_WARPS * 32u, 0, p);
+    {
+        const bool two = n_tok >= 2u * (uint32_t)g_q4.sm_count && kv->n_kvh <= 2u;   /* 4 rows a token: two tokens for 8 warps */
+        const dim3 grid(two ? (n_tok + 1u) / 2u : n_tok);
+        auto start = [&](auto kernel) { return q4i_launch_pdl("kv_prep_append launch", kernel, grid, PREP_WARPS * 32u, 0, p); };
+        if (kv->hd == 128) return two ? start(q4_prep_append_rows_k<128, 2>) : start(q4_prep_append_rows_k<128, 1>);
+        return two ? start(q4_prep_append_rows_k<256, 2>) : start(q4_prep_append_rows_k<256, 1>);
+    }
     q4_prep_append_k<<<dim3(kv->n_kvh, n_tok, 2), 128, 0, g_q4.stream>>>(p);
     return q4i_check(cudaGetLastError(), "kv_prep_append launch");
 }

@@ -508,3 +508,59 @@ def test_large_magnitude_queries(oracle, mode, q_bf16):
     ref = oracle.attn(q, kc, vc, gate, n_head, n_kvh, hd, 1, ctx - 1, ctx, scale, 2)[0]
     assert_close(host(out).reshape(n_head, hd), ref, "dense, %s" % mode)
     st.close()
+
+
+@pytest.mark.parametrize("kind,n_head,hd", [(2, 16, 128), (1, 16, 128), (0, 16, 128), (2, 24, 256), (1, 24, 256)])
+@pytest.mark.parametrize("max_kv,rows", [(20000, [1, 63, 64, 65, 250, 257, 1777, 2047, 2049, 2560, 19999]), (12007, [9000, 12007]), (40009, [300, 33000])])
+def test_dense_at_the_position_word_in_larger_stores(oracle, kind, n_head, hd, max_kv, rows):
+    """a launch is sized for the store's capacity and reads the position on the device: contexts that need one block, the
+    first cluster alone, some of the blocks and all of them, in capacities whose split counts are no multiple of the
+    cluster, right after the position was pushed and again with everything settled (rows read ahead of the launch wait)"""
+    L = lib()
+    n_kvh, n = 2, max(rows)
+    kvw = n_kvh * hd
+    k = oracle.normal(77 + hd, 0, n * kvw).reshape(n, kvw)
+    v = oracle.normal(77 + hd, 1, n * kvw).reshape(n, kvw)
+    q = oracle.normal(77, 2, n_head * hd)
+    st = q4gpu.KVStore(1, n_kvh, hd, max_kv, kind)
+    st.append(0, dev(k), dev(v), 0, n)
+    kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind)
+    dq = dev(q)
+    scale = float(1.0 / np.sqrt(hd))
+    for r in rows:
+        outs = [torch.full((n_head * hd,), float("nan"), device="cuda") for _ in range(3)]
+        L.q4_hip_pos_push(r - 1)
+        for o in outs:
+            st.decode(0, dq, o, n_head, scale)
+        ref = oracle.attn(q.reshape(1, n_head, hd), kc, vc, None, n_head, n_kvh, hd, 1, r - 1, max_kv, scale, kind, threads=8)[0]
+        for o in outs:
+            assert_close(host(o).reshape(ref.shape), ref, "kind %d hd %d: %d of %d rows" % (kind, hd, r, max_kv))
+    assert L.q4_gpu_last_error() == 0
+    st.close()
+
+
+@pytest.mark.parametrize("kind", [2, 1])
+def test_batched_dense_sessions_of_unequal_length_against_the_oracle(oracle, kind):
+    """one launch over sessions of which some need one block and others dozens"""
+    lib()
+    n_head, n_kvh, hd, lens = 16, 2, 128, [9000, 12000, 5, 700]
+    kvw = n_kvh * hd
+    stores, refs, qs = [], [], oracle.normal(5150, 9, len(lens) * n_head * hd).reshape(len(lens), n_head, hd)
+    for s, n in enumerate(lens):
+        k = oracle.normal(5150 + s, 0, n * kvw).reshape(n, kvw)
+        v = oracle.normal(5150 + s, 1, n * kvw).reshape(n, kvw)
+        st = q4gpu.KVStore(1, n_kvh, hd, n + 3, kind)
+        st.append(0, dev(k), dev(v), 0, n)
+        stores.append(st)
+        refs.append(oracle.attn(qs[s][None], oracle.kv_write(k, kind), oracle.kv_write(v, kind), None, n_head, n_kvh, hd, 1, n - 1, n + 3,
+                                0.0884, kind, threads=8)[0])
+    b = q4gpu.Batch(stores)
+    b.set_pos([n - 1 for n in lens])
+    out = torch.zeros(len(lens), n_head, hd, device="cuda")
+    for _ in range(2):
+        b.decode(0, dev(qs), out, n_head, 0.0884)
+        for s in range(len(lens)):
+            assert_close(host(out[s]), refs[s], "session of %d rows" % lens[s])
+    b.close()
+    for st in stores:
+        st.close()

@@ -209,3 +209,30 @@ def test_topk_forms_and_their_edges(oracle, n_tok, n_vis, k_blk):
     assert L.q4_hip_qsa_topk(dev(rows).data_ptr(), d_sel.data_ptr(), n_tok, n_vis, stride, k_blk, ratio, pos0, width)
     want = oracle.ix_topk(rows, n_tok, stride, k_blk, ratio, pos0, width)
     assert np.array_equal(host(d_sel), want)
+
+
+def test_batched_scores_of_many_uneven_sessions(oracle):
+    """the sessions' tiles are shared equally among the blocks: 70 sessions (more than one warp's worth), some without a
+    visible block, some of one row, one much longer than the others"""
+    L = lib()
+    n_head, ratio = 4, RATIO
+    rng = np.random.default_rng(70)
+    positions = [int(x) for x in rng.integers(0, 700, 70)]
+    positions[0], positions[3], positions[33], positions[69], positions[40] = 0, 2, 3, 4099, 60003
+    stride = max(positions) // ratio + 2
+    q = rng.standard_normal((70, n_head, 128)).astype(np.float32)
+    pools = [rng.standard_normal(((p + 1) // ratio + 1, 128)).astype(np.float32) for p in positions]
+    d_pools = [dev(p) for p in pools]
+    ptrs = torch.tensor([t.data_ptr() for t in d_pools], dtype=torch.int64, device="cuda")
+    d_pos = torch.tensor(positions, dtype=torch.int32, device="cuda")
+    d_score = torch.full((70, stride), 7.0, device="cuda")
+    d_sel = torch.zeros(70, 67, dtype=torch.int32, device="cuda")
+    assert L.q4_gpu_qsa_select_batch(ptrs.data_ptr(), d_pos.data_ptr(), dev(q).data_ptr(), d_score.data_ptr(), d_sel.data_ptr(), 70, stride,
+                                     n_head, 128, 16, ratio, 67)
+    got, sel = host(d_score), host(d_sel)
+    for t, pos in enumerate(positions):
+        nb = (pos + 1) // ratio
+        want = oracle.ix_score(q[t:t + 1], pools[t], 1, nb, stride, n_head, pos, ratio) if nb else np.zeros((1, stride), np.float32)
+        assert np.array_equal(got[t, :nb].view(np.uint32), want[0, :nb].view(np.uint32)), t
+        assert (got[t, nb:] == 7.0).all(), t
+        assert np.array_equal(sel[t], oracle.ix_topk(want, 1, stride, 16, ratio, pos, 67)[0]), t

@@ -323,3 +323,32 @@ def test_fused_prep_append_equals_two_launches(oracle, kind, hd, n_rot):
         assert torch.equal(xa, xc)
     for s in (a, b, c):
         s.close()
+
+
+@pytest.mark.parametrize("hd,n_rot,n_kvh", [(128, 128, 2), (128, 64, 3), (256, 64, 1), (256, 256, 2)])
+def test_prep_of_many_tokens_equals_token_by_token(oracle, hd, n_rot, n_kvh):
+    """from some hundred tokens on, blocks take several tokens each (an odd number of tokens here): rows and cache bytes equal
+    those of the same tokens one call at a time, for which a block has one token"""
+    L = lib()
+    n, pos0 = 603, 1000
+    kvw = n_kvh * hd
+    k = oracle.normal(91 + hd, 0, n * kvw).reshape(n, kvw)
+    v = oracle.normal(91 + hd, 1, n * kvw).reshape(n, kvw)
+    wn = (1.0 + 0.1 * oracle.normal(91, 2, hd)).astype(np.float32)
+    dk, dv, dw = dev(k), dev(v), dev(wn)
+    many, one = dk.clone(), dk.clone()
+    assert L.q4_hip_qsa_k_prep_n(many.data_ptr(), dw.data_ptr(), n_kvh, hd, n_rot, pos0, 1e7, 1e-6, n)
+    for t in (0, 1, 2, 3, 4, 301, 600, 601, 602):
+        assert L.q4_hip_qsa_k_prep_n(one[t].data_ptr(), dw.data_ptr(), n_kvh, hd, n_rot, pos0 + t, 1e7, 1e-6, 1)
+        assert np.array_equal(host(many[t]).view(np.uint32), host(one[t]).view(np.uint32)), t
+    a, b = q4gpu.KVStore(1, n_kvh, hd, pos0 + n, 2), q4gpu.KVStore(1, n_kvh, hd, pos0 + n, 2)
+    assert L.q4_gpu_kv_prep_append(a.h, 0, dk.data_ptr(), dv.data_ptr(), dw.data_ptr(), n_rot, 1e7, 1e-6, pos0, n)
+    b.append(0, many, dv, pos0, n)
+    for which in (0, 1):
+        x = torch.empty(n * a.token_bytes, dtype=torch.uint8, device="cuda")
+        y = torch.empty_like(x)
+        a.export(0, which, pos0, n, x)
+        b.export(0, which, pos0, n, y)
+        assert np.array_equal(host(x), host(y)), which
+    a.close()
+    b.close()
