@@ -10,17 +10,19 @@
  * Shape of the kernel.  The path is bound by HBM, and with 8 query heads sharing each K/V byte the
  * scalar FMA pipe cannot keep up with B200's memory system (8 FMA per int8 byte at ~23 B/clk/SM
  * is more than the 128 FMA/clk an SM has), so the two contractions run on the tensor cores with
- * warp-level MMA.  Every byte of the cache is read from global memory once.  For the native q8_0
- * store at hd 128 each warp owns a 4-stage ring of 16-position tiles in shared memory (the tile's
- * records as they lie in the store, 272 bytes apart).  A tile of 16 consecutive positions is one
- * contiguous span of the store: it comes in with fully coalesced 16-byte cp.async copies, or, in a
- * dense scan, with one 4352-byte bulk copy (cp.async.bulk, completion on the stage's mbarrier); any
- * other tile is gathered row by row with 16-byte cp.async copies.  Per tile the warp unloads the
- * stage into MMA fragments (ldmatrix for the K rows, transposing ldmatrix for the V rows), refills
- * the stage at once with the tile four ahead, and then computes from registers, so four tiles per
- * warp are in flight all the time; there is no block barrier in the main loop, warps stream
- * independently.  The other layouts load fragments straight into registers with sector-aligned
- * 4/8/16-byte loads.
+ * warp-level MMA.  Every byte of the cache is read from global memory once.  At hd 128 and 256 every warp (or, with more
+ * than 8 query heads per kv head, two warps that share it) owns a ring of 16-position tiles in shared memory, up to four
+ * deep, filled with asynchronous copies of whole rows or records; in a dense scan of the native q8_0 store at hd 128 a
+ * tile is one contiguous span and one 4352-byte bulk copy (cp.async.bulk, completion on the stage's mbarrier).  That
+ * layout's warps unload a stage into MMA fragments (ldmatrix for the K rows, transposing ldmatrix for the V rows),
+ * refill it at once with the tile four ahead and compute from registers; the others read fragments from the stage as the
+ * products need them and refill it then.  No block barrier in the main loop.  Queries are requested coalesced ahead of
+ * the copies and passed to the fragments as fp16 through a stage that is not filled yet.  Head sizes 32 and 64, and
+ * caches that are not aligned for the copies, load fragments straight into registers.
+ *
+ * Launches overlap (programmatic dependent launch): what the host knows to be complete -- positions, and in a dense scan
+ * the rows that earlier launches wrote -- is read before a block waits for the previous kernel, so that the rings fill
+ * under its tail (777 dense rows 6.6 -> 5.4 us per layer, 32768 rows 14.5 -> 12.4).
  *
  *   one warp-step = 16 positions:
  *     S^T[16 pos x 8 heads]  = K[16 x hd] . Q^T        (m16n8k16, K rows are the A operand)
@@ -38,8 +40,10 @@
  * 16 splits form one thread-block cluster and merge through distributed shared memory (no scratch, no
  * atomics: every block pushes the heads of its record to the blocks that own them, and the pushes
  * complete an mbarrier there).  More splits write (acc, m, l) records to scratch; when the whole grid
- * is resident the unit's blocks meet at a counter and share out (head, 32-dim) slices of the merge,
- * otherwise -- and in the sequence-sharded exchange, whose last block must hold the rank's record --
+ * is resident the unit's blocks meet at a counter and share out (head, 32-dim) slices of the merge.  A launch whose
+ * position is on the device is sized for the store's capacity; each unit then uses as many of its blocks as its context
+ * needs, and in stores of up to 32768 rows, launched in clusters, a short context its first cluster alone.
+ * Otherwise -- and in the sequence-sharded exchange, whose last block must hold the rank's record --
  * the last block to arrive per group of 16 merges, two levels at most.  Either way the layer is one
  * launch.
  */

@@ -357,7 +357,9 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    q4d_pdl_wait();
+    /* Queries and gates are older than the staging launch before this one, and that lets this grid start only after it has
+     * waited for everything older: they need no wait.  The images do. */
+    if (warp >= SW) q4d_pdl_wait();
     if (warp < SW) {
         /* ---- queries as fp16 (exact for normal bf16 values), K-major swizzled, blocks of 64 dims: 8 dims per thread
          * and step, whole rows per warp step */
@@ -394,6 +396,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             }
         }
         fence_async_smem();
+        q4d_pdl_wait();
     }
     tc_fence_before();
     __syncthreads();          /* barriers initialised, queries in place, tensor memory allocated */
@@ -584,7 +587,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
             uint32_t pk[UN / 64][32];
             uint64_t ls[2] = {0ull, 0ull};
-            {
+            if (NQ == 2 || u > 0) {   /* a short chunk's first unit is a good part of it */
                 const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
 #pragma unroll
                 for (int h = 0; h < (int)UN / 64; h++) exps(h, mneg, pk[h], ls);
@@ -596,7 +599,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             }
             const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * P.scale_log2e;   /* scale > 0 */
             const bool grow = m_new > m_ref + PF_RESCALE_TAU;   /* also true on the first live unit (m_ref = -inf) */
-            if (__builtin_expect(__any_sync(0xffffffffu, grow), 0)) {
+            if (__builtin_expect((NQ == 1 && u == 0) || __any_sync(0xffffffffu, grow), 0)) {
                 float alpha = 1.f;
                 if (grow) {
                     alpha = ex2f(m_ref - m_new);             /* 0 on the first live unit */
@@ -650,13 +653,15 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             off[q] = ((g * P.tpc + ti) * P.n_head + kh * P.gqa + (row - ti * P.gqa)) * (HD / 4u) + (lane & 7u);
         }
         const size_t first = (size_t)t0 * P.n_head * (HD / 4u);
-        auto fetch_gates = [&](int c, float4 (&gt)[8]) {
+        auto fetch_gates = [&](int c, float4 (&to)[8]) {
 #pragma unroll
             for (int q = 0; q < 8; q++)
-                if (gates && ((live >> q) & 1u)) gt[q] = reinterpret_cast<const float4 *>(P.gate)[first + off[q] + 8u * c];
+                if (gates && ((live >> q) & 1u)) to[q] = reinterpret_cast<const float4 *>(P.gate)[first + off[q] + 8u * c];
         };
-        float4 gt0[8], gt1[8];
-        fetch_gates(0, gt0);
+        constexpr int GA = NQ == 2 ? 2 : 4;   /* column blocks whose gates are on their way: as registers allow */
+        float4 gt[GA][8];
+#pragma unroll
+        for (int c = 0; c < GA - 1; c++) fetch_gates(c, gt[c]);
         if (ok && n_seq > 0) ok = wait(bar_o + 8 * g, (n_seq - 1u) & 1u);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
@@ -666,7 +671,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + g * QG_BYTES + (warp & 3u) * (QG_BYTES / 4u));   /* [32][36] */
             if (split && row_live)
                 P.part_ml[((size_t)blockIdx.z * P.n_tok + tok) * P.n_head + head] = make_float2(m_ref, l_run);
-            auto columns = [&](int c, float4 (&gt)[8]) {
+            auto columns = [&](int c, float4 (&gs)[8]) {
                 float o[32];
                 if (n_tiles > 0) {
                     tmem_ld32(t_lane + O_COL + g * 128u + 32 * c, o);
@@ -686,8 +691,8 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
                 if (gates) {
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
-                        x[q].x = gated(x[q].x, gt[q].x); x[q].y = gated(x[q].y, gt[q].y);
-                        x[q].z = gated(x[q].z, gt[q].z); x[q].w = gated(x[q].w, gt[q].w);
+                        x[q].x = gated(x[q].x, gs[q].x); x[q].y = gated(x[q].y, gs[q].y);
+                        x[q].z = gated(x[q].z, gs[q].z); x[q].w = gated(x[q].w, gs[q].w);
                     }
                 }
                 if (split) {
@@ -708,12 +713,12 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
                 }
             };
 #pragma unroll 1
-            for (int c = 0; c < HD / 32; c += 2) {
-                fetch_gates(c + 1, gt1);
-                columns(c, gt0);
-                if (c + 2 < HD / 32) fetch_gates(c + 2, gt0);
-                columns(c + 1, gt1);
-            }
+            for (int c = 0; c < HD / 32; c += GA)
+#pragma unroll
+                for (int e = 0; e < GA; e++) {
+                    if (c + e + GA - 1 < HD / 32) fetch_gates(c + e + GA - 1, gt[(e + GA - 1) % GA]);
+                    columns(c + e, gt[e]);
+                }
         }
     }
     if (!ok && lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
