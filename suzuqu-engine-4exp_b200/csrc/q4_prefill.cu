@@ -47,7 +47,8 @@ namespace {
 constexpr uint32_t PF_ROWS = 128, PF_BN = 128;              /* rows of a query group, positions of a tile */
 constexpr uint32_t PF_CHUNK = 32768, PF_RING = 5;           /* operand image bytes, ring slots */
 constexpr uint32_t PF_Q_BYTES = 65536;                      /* NQ x 128 rows x hd fp16, in every configuration at most this */
-constexpr uint32_t PF_BAR_BYTES = 256;
+constexpr uint32_t PF_BAR_BYTES = 256 + 1024;               /* barriers and words; one float per softmax thread */
+constexpr uint32_t PF_THREADS = 320;                        /* 8 softmax warps, the issuer, the producer */
 constexpr uint32_t PF_SMEM = PF_Q_BYTES + PF_RING * PF_CHUNK + PF_BAR_BYTES + 1024;
 constexpr uint32_t PF_SPIN_LIMIT = 1u << 22;
 constexpr unsigned long long PF_LIMIT_NS = 2000000000ull;   /* a block that has not finished by then gives up */
@@ -309,11 +310,12 @@ __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_a
 }
 /* HD: head size; NQ: query groups per block; KP: images per 128 dims of K (2: value and remainder) */
 template <int HD, int NQ, int KP>
-__global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillParams P) {
+__global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParams P) {
     constexpr uint32_t CK = KP * HD / 128, CV = HD / 128;      /* ring slots a K / V tile takes */
-    constexpr uint32_t SW = NQ * 4;                            /* softmax warps; then the issuer, then the producer */
+    constexpr uint32_t SW = 8;                                 /* softmax warps; then the issuer, then the producer */
     constexpr uint32_t O_COL = 256, TMEM_COLS = 512;           /* scores in the first 256 columns, O of group g at 256 + 128 g */
     constexpr uint32_t UN = NQ == 2 ? 64 : 128, SB = 2 * NQ;   /* positions of a unit, score buffers */
+    constexpr uint32_t TU = 64;                                /* of them, those of one softmax thread */
     constexpr uint32_t QG_BYTES = PF_ROWS * HD * 2;            /* one group's queries */
     static_assert(NQ * QG_BYTES <= PF_Q_BYTES && O_COL + NQ * HD <= TMEM_COLS, "shared / tensor memory");
     extern __shared__ uint8_t smem_dyn[];
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
     /* 1024-byte aligned operand tiles (the swizzle pattern is anchored to the address) */
     const uint32_t sQ = (smem_u32(smem_dyn) + 1023u) & ~1023u, sR = sQ + PF_Q_BYTES, bars = sR + PF_RING * PF_CHUNK;
     const uint32_t full = bars, empty = bars + 40, bar_s = bars + 80, bar_p = bars + 112, bar_o = bars + 144,
-                   s_tmem = bars + 160, s_abort = bars + 164;
+                   s_tmem = bars + 160, s_abort = bars + 164, s_xch = bars + 256;
 
     const uint32_t inv_gqa = 65536u / P.gqa + 1u;   /* row / gqa = row * inv_gqa >> 16 for rows below 128, gqa up to 16 */
     const uint32_t t_last = min(t0 + P.tpc * NQ, P.n_tok) - 1u;
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
 #pragma unroll
             for (uint32_t s = 0; s < 4; s++) {
                 mbar_init(bar_s + 8 * s, 1);
-                mbar_init(bar_p + 8 * s, PF_ROWS);
+                mbar_init(bar_p + 8 * s, SW * 32u / NQ);
             }
             mbar_init(bar_o, 1);
             mbar_init(bar_o + 8, 1);
@@ -363,9 +365,9 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
     if (warp < SW) {
         /* ---- queries as fp16 (exact for normal bf16 values), K-major swizzled, blocks of 64 dims: 8 dims per thread
          * and step, whole rows per warp step */
-        constexpr uint32_t PER = HD / 8u, BATCH = 8u;   /* loads in flight before the first store */
+        constexpr uint32_t PER = HD / 8u, STEPS = NQ * PF_ROWS * PER / (SW * 32u), BATCH = 8u;   /* loads in flight before the first store */
 #pragma unroll 1
-        for (uint32_t k0 = 0; k0 < PER; k0 += BATCH) {
+        for (uint32_t k0 = 0; k0 < STEPS; k0 += BATCH) {
             uint4 w[BATCH][2];
 #pragma unroll
             for (uint32_t k = 0; k < BATCH; k++) {
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
                         if (h == 0) ok = ok && all_wait(bar_p + 8 * (j & 1u), (j >> 1) & 1u);
                         tc_fence_after();
                         if (!ok) break;
-                        pv_half((j & 1u) * 128u + h * 32u, 0u, s, CV == 2 ? 0u : h * (HD * 128u), j == 0 && h == 0);
+                        pv_half((j & 1u) * 128u + h * 64u, 0u, s, CV == 2 ? 0u : h * (HD * 128u), j == 0 && h == 0);
                         if (CV == 2 || h == 1) umma_commit(el, empty + 8 * s);
                     }
                     if (ok) {
@@ -548,34 +550,62 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             }
         }
     } else {
-        /* ================= softmax: thread r of group g owns row r of that group's queries ================= */
-        const uint32_t g = warp >> 2, r = tid & 127u, t_lane = tmem + (((warp & 3u) * 32u) << 16);
+        /* ================= softmax: thread r of group g owns row r of that group's queries; with one group, thread r of
+         * half h owns 64 of a unit's positions of row r ================= */
+        const uint32_t g = NQ == 2 ? warp >> 2 : 0u, h = NQ == 2 ? 0u : warp >> 2, r = tid & 127u, t_lane = tmem + (((warp & 3u) * 32u) << 16);
         const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl, head = kh * P.gqa + r - tl * P.gqa;   /* rows past tpc * gqa or past n_tok are padding */
         const bool row_live = tl < P.tpc && tok < P.n_tok;
         /* this row attends positions [0, row_nkv); padding rows (queries of zeros, never stored) need no mask */
         const uint32_t row_nkv = row_live ? min(P.kv_base + tok + 1u, P.max_kv) : 0xffffffffu;
         const uint32_t warp_min = __reduce_min_sync(0xffffffffu, row_nkv);
+        /* the two warps of the same 32 rows (one group): all meetings are unconditional, so that they also end where one
+         * of the two has given up */
+        auto pair_sync = [&]() {
+            __syncwarp();
+            asm volatile("bar.sync %0, 64;" ::"r"(1u + (warp & 3u)) : "memory");
+        };
+        auto pair_any = [&](bool x) -> bool {
+            uint32_t any;
+            __syncwarp();
+            asm volatile("{ .reg .pred p, q; setp.ne.u32 q, %1, 0; bar.red.or.pred p, %2, 64, q; selp.u32 %0, 1, 0, p; }"
+                         : "=r"(any) : "r"((uint32_t)x), "r"(1u + (warp & 3u)) : "memory");
+            return any != 0u;
+        };
+        auto partner = [&](float x) -> float {   /* the other half's value of this row; a meeting lies between two calls */
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(s_xch + 4u * tid), "f"(x) : "memory");
+            pair_sync();
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(s_xch + 4u * (tid ^ 128u)) : "memory");
+            return x;
+        };
         float m_ref = -CUDART_INF_F, l_run = 0.f;
-        for (uint32_t u = 0; u < n_seq && ok; u++) {
-            const uint32_t i = u * NQ + g, b = i % SB, use = (i / SB) & 1u, p0 = j0 * PF_BN + u * UN;
-            const uint32_t t_s = t_lane + (NQ == 2 ? g * 128u + (u & 1u) * 64u : b * 128u);
-            ok = all_wait(bar_s + 8 * b, use);   /* a warp leaves the loop as one */
+        for (uint32_t u = 0; u < n_seq && (NQ == 1 || ok); u++) {
+            const uint32_t i = u * NQ + g, b = i % SB, use = (i / SB) & 1u, p0 = j0 * PF_BN + u * UN + h * TU;
+            const uint32_t t_s = t_lane + (NQ == 2 ? g * 128u + (u & 1u) * 64u : b * 128u + h * TU);
+            ok = ok && all_wait(bar_s + 8 * b, use);   /* a warp goes on as one */
+            if (NQ == 1 && !ok) {
+                if (u == 0 || pair_any(false)) partner(0.f);
+                continue;
+            }
             tc_fence_after();
-            float s[UN];
+            float s[TU];
 #pragma unroll
-            for (int c = 0; c < (int)UN / 32; c++) tmem_ld32(t_s + 32 * c, *reinterpret_cast<float(*)[32]>(&s[32 * c]));
+            for (int c = 0; c < (int)TU / 32; c++) tmem_ld32(t_s + 32 * c, *reinterpret_cast<float(*)[32]>(&s[32 * c]));
             tmem_wait_ld();
-            if (__builtin_expect(p0 + UN > warp_min, 0)) {
+            if (__builtin_expect(p0 + TU > warp_min, 0)) {
 #pragma unroll
-                for (int k = 0; k < (int)UN; k++)
+                for (int k = 0; k < (int)TU; k++)
                     if (p0 + k >= row_nkv) s[k] = -CUDART_INF_F;
             }
-            /* P of 64 positions against the reference maximum, as fp16 pairs; sums into ls */
-            auto exps = [&](int h, float mneg, uint32_t (&pk)[32], uint64_t (&ls)[2]) {
+            /* P against the reference maximum, as fp16 pairs; sums into ls */
+            uint32_t pk[TU / 2];
+            uint64_t ls[2];
+            auto exps = [&]() {
+                const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
                 const uint64_t sc2 = pack2(P.scale_log2e, P.scale_log2e), mn2 = pack2(mneg, mneg);
+                ls[0] = ls[1] = 0ull;
 #pragma unroll
-                for (int k = 0; k < 32; k++) {
-                    const float2 x = unpack2(fma2(pack2(s[64 * h + 2 * k], s[64 * h + 2 * k + 1]), sc2, mn2));
+                for (int k = 0; k < (int)TU / 2; k++) {
+                    const float2 x = unpack2(fma2(pack2(s[2 * k], s[2 * k + 1]), sc2, mn2));
                     const float e0 = ex2f(x.x), e1 = ex2f(x.y);
                     ls[k & 1] = add2(ls[k & 1], pack2(e0, e1));
                     pk[k] = h2u(__floats2half2_rn(e0, e1));
@@ -584,38 +614,35 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             /* The exponentials start against the maximum of the units before, while this unit's own is still being
              * formed: the reference only has to be within 2^8 of it.  Where it is not (the first unit, a large new
              * score) the reference moves and they are taken again. */
+            if (NQ == 2 || u > 0) exps();   /* of a short chunk the first unit is a good part */
             float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-            uint32_t pk[UN / 64][32];
-            uint64_t ls[2] = {0ull, 0ull};
-            if (NQ == 2 || u > 0) {   /* a short chunk's first unit is a good part of it */
-                const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
 #pragma unroll
-                for (int h = 0; h < (int)UN / 64; h++) exps(h, mneg, pk[h], ls);
-            }
-#pragma unroll
-            for (int k = 0; k < (int)UN; k += 8) {
+            for (int k = 0; k < (int)TU; k += 8) {
                 mx[0] = fmaxf(fmaxf(mx[0], s[k]), s[k + 1]); mx[1] = fmaxf(fmaxf(mx[1], s[k + 2]), s[k + 3]);
                 mx[2] = fmaxf(fmaxf(mx[2], s[k + 4]), s[k + 5]); mx[3] = fmaxf(fmaxf(mx[3], s[k + 6]), s[k + 7]);
             }
-            const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * P.scale_log2e;   /* scale > 0 */
-            const bool grow = m_new > m_ref + PF_RESCALE_TAU;   /* also true on the first live unit (m_ref = -inf) */
-            if (__builtin_expect((NQ == 1 && u == 0) || __any_sync(0xffffffffu, grow), 0)) {
+            float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * P.scale_log2e;   /* scale > 0 */
+            bool grow = m_new > m_ref + PF_RESCALE_TAU;   /* also true on the first live unit (m_ref = -inf) */
+            const bool any = NQ == 2 ? __any_sync(0xffffffffu, grow) : u == 0 || pair_any(grow);
+            if (__builtin_expect(any, 0)) {
+                if (NQ == 1) {   /* both halves of a row keep one reference: they share its O */
+                    m_new = fmaxf(m_new, partner(m_new));
+                    grow = m_new > m_ref + PF_RESCALE_TAU;
+                }
                 float alpha = 1.f;
                 if (grow) {
                     alpha = ex2f(m_ref - m_new);             /* 0 on the first live unit */
                     m_ref = m_new;
                     l_run *= alpha;
                 }
-                const float mneg = m_ref == -CUDART_INF_F ? 0.f : -m_ref;
-                ls[0] = ls[1] = 0ull;
-#pragma unroll
-                for (int h = 0; h < (int)UN / 64; h++) exps(h, mneg, pk[h], ls);
-                /* O is rescaled only here; the group's previous P . V must have drained first */
+                exps();
+                /* O is rescaled only here (one group: half of its columns by each half); the group's previous P . V must
+                 * have drained first */
                 if (u > 0) {
                     ok = all_wait(bar_o + 8 * g, (u - 1u) & 1u) && ok;
                     tc_fence_after();
 #pragma unroll 1
-                    for (int c = 0; c < HD / 32; c++) {
+                    for (uint32_t c = h * (HD / 64); c < (NQ == 2 ? HD / 32 : (h + 1u) * (HD / 64)); c++) {
                         float o[32];
                         tmem_ld32(t_lane + O_COL + g * 128u + 32 * c, o);
                         tmem_wait_ld();
@@ -625,9 +652,8 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
                     }
                 }
             }
-            /* P goes into the first half of the score buffer this thread has just read (two fp16 per column) */
-#pragma unroll
-            for (int h = 0; h < (int)UN / 64; h++) tmem_st32(t_s + 32 * h, *reinterpret_cast<const float(*)[32]>(&pk[h][0]));
+            /* P goes into the first half of the columns this thread has just read (two fp16 per column) */
+            tmem_st32(t_s, *reinterpret_cast<const float(*)[32]>(&pk[0]));
             tmem_wait_st();
             /* A parity wait can tell the current phase from the one before it, no further, and bar_o's phases are not
              * followed unit by unit.  So the phase before the last is waited for here, while the last cannot
@@ -638,11 +664,16 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             const float2 l0 = unpack2(ls[0]), l1 = unpack2(ls[1]);
             l_run += (l0.x + l0.y) + (l1.x + l1.y);
         }
+        if (NQ == 1) {
+            pair_sync();
+            l_run += partner(l_run);
+        }
         /* ---- epilogue: O / l * sigmoid(gate), or the unnormalised part of a split range.  32 columns at a time go
          * through the warp's share of the query tiles (read by no product any more), so that rows leave in whole lines.
          * Step q of a column block: 4 rows of 32 columns, 8 lanes each.  The gates are requested a whole column block
          * ahead, the first ones under the last product (requested behind their use a block took 2600 cycles, most of it
-         * their latency). */
+         * their latency).  One group: each half takes half of the columns (a warp alone is held up in turn by its
+         * special-function steps, 700 cycles a block, and its stores, 450). */
         const bool split = P.n_split > 1u, gates = P.gate && !split;
         const uint32_t w_row0 = (warp & 3u) * 32u;
         uint32_t off[8], live = 0;   /* in 16-byte units from the chunk's first token */
@@ -658,18 +689,18 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
             for (int q = 0; q < 8; q++)
                 if (gates && ((live >> q) & 1u)) to[q] = reinterpret_cast<const float4 *>(P.gate)[first + off[q] + 8u * c];
         };
-        constexpr int GA = NQ == 2 ? 2 : 4;   /* column blocks whose gates are on their way: as registers allow */
-        float4 gt[GA][8];
-#pragma unroll
-        for (int c = 0; c < GA - 1; c++) fetch_gates(c, gt[c]);
+        constexpr int NC = NQ == 2 ? HD / 32 : HD / 64;   /* column blocks of this warp */
+        const int c0 = h * NC;
+        float4 gt0[8], gt1[8];
+        fetch_gates(c0, gt0);
         if (ok && n_seq > 0) ok = wait(bar_o + 8 * g, (n_seq - 1u) & 1u);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
 
         if (ok) {
             const float inv = split ? 1.f : l_run > 0.f ? 1.f / l_run : 0.f;
-            float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + g * QG_BYTES + (warp & 3u) * (QG_BYTES / 4u));   /* [32][36] */
-            if (split && row_live)
+            float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + warp * (PF_Q_BYTES / SW));   /* [32][36] */
+            if (split && row_live && h == 0)
                 P.part_ml[((size_t)blockIdx.z * P.n_tok + tok) * P.n_head + head] = make_float2(m_ref, l_run);
             auto columns = [&](int c, float4 (&gs)[8]) {
                 float o[32];
@@ -713,12 +744,12 @@ __global__ void __launch_bounds__(NQ * 128 + 64, 1) q4_prefill_k(const PrefillPa
                 }
             };
 #pragma unroll 1
-            for (int c = 0; c < HD / 32; c += GA)
-#pragma unroll
-                for (int e = 0; e < GA; e++) {
-                    if (c + e + GA - 1 < HD / 32) fetch_gates(c + e + GA - 1, gt[(e + GA - 1) % GA]);
-                    columns(c + e, gt[e]);
-                }
+            for (int c = c0; c < c0 + NC; c += 2) {
+                fetch_gates(c + 1, gt1);
+                columns(c, gt0);
+                if (c + 2 < c0 + NC) fetch_gates(c + 2, gt0);
+                columns(c + 1, gt1);
+            }
         }
     }
     if (!ok && lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
@@ -785,7 +816,7 @@ bool attend(const PrefillParams &p, dim3 grid) {
                             "prefill smem attribute"))
         return false;
     attr = true;
-    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, KP>, grid, NQ * 128u + 64u, PF_SMEM, p);
+    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, KP>, grid, PF_THREADS, PF_SMEM, p);
 }
 template <int LAY, int HD, int KP>
 bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
