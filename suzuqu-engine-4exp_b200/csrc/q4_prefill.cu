@@ -823,6 +823,27 @@ bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, ui
     return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, KP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
 }
 
+/* Ranges of positions that a chunk's blocks of one query group are split into: the count with the least estimated time,
+ * waves x (tiles of a range + what a block takes besides) + the merge with its traffic.  In ns, from chunks of 33 to 1500
+ * tokens over 0 to 16 384: a tile 1.0 us at hd 128, 1.8 at 256 with both images of K; a block 4 and 6 us besides; the merge
+ * 1.2 us, 0.2 per range, and 7 KB per ns.  600 tokens over 16 384 (76 blocks): 146 us in one range, 112 in three. */
+uint32_t best_split(uint32_t blocks, uint32_t sms, uint32_t tiles, uint64_t rows, uint32_t hd, uint32_t kp) {
+    const uint64_t tile = 640u + 190u * (hd / 128u) * (kp + 1u), block = 2000u + 2000u * (hd / 128u);
+    uint64_t best = 0;
+    uint32_t split = 1;
+    for (uint32_t s = 1; s <= 16u && s <= tiles; s++) {
+        const uint64_t waves = ((uint64_t)blocks * s + sms - 1u) / sms;
+        uint64_t t = waves * ((tiles + s - 1u) / s * tile + block);
+        if (s > 1) t += 1200u + 200u * s + rows * hd * s * 8u / 7000u;
+        if (s == 1) best = t - t / 16u;   /* one range needs no merge: left for a clear gain only (causal chunks have less work) */
+        else if (t < best) {
+            best = t;
+            split = s;
+        }
+    }
+    return split;
+}
+
 }  // namespace
 
 void q4i_prefill_release() {
@@ -838,14 +859,12 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     /* codes times scales do not fit fp16: the exact form keeps what the first image leaves over */
     const uint32_t kp = a.layout == LAY_Q8R ? 2u : 1u;
     const uint32_t tpc = PF_ROWS / gqa, groups = (a.n_tok + tpc - 1u) / tpc, sms = (uint32_t)g_q4.sm_count;
-    /* Two groups per block share every K/V tile and hide one another's softmax; one group per block while that does not
-     * fill the SMs, and then the positions are split too, three tiles a block. */
-    const uint32_t nq = hd == 128 && groups * a.n_kvh > sms ? 2u : 1u;
+    /* Two groups per block share every K/V tile and hide one another's softmax; one group per block while that takes few
+     * waves: 1000 tokens over 4000 (126 blocks) 52 against 83 us, 2500 over 16 384 (314) 450 against 505, 3600 (450) 643
+     * against 591; between 300 and 400 it depends on the depth. */
+    const uint32_t nq = hd == 128 && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
     const uint32_t blocks = (groups + nq - 1u) / nq * a.n_kvh;
-    uint32_t split = nq == 1 && blocks * 2u <= sms ? sms / blocks : 1u;
-    if (tiles < 6u) split = 1u;                            /* the merge costs about as much as three tiles */
-    if (split > (tiles + 2u) / 3u) split = (tiles + 2u) / 3u;
-    if (split > 16u) split = 16u;
+    uint32_t split = nq == 1 ? best_split(blocks, sms, tiles, (uint64_t)a.n_tok * a.n_head, hd, kp) : 1u;
     const size_t k_bytes = (size_t)a.n_kvh * tiles * kp * (hd / 128u) * PF_CHUNK, v_bytes = (size_t)a.n_kvh * tiles * (hd / 128u) * PF_CHUNK;
     const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
     if (!stage_reserve(k_bytes + v_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0)))

@@ -70,6 +70,15 @@ def test_prefill_two_query_groups_per_block(oracle, n_head, n_kvh, n_tok, kv_bas
     assert q4gpu.load().q4_gpu_last_error() == 0
 
 
+@pytest.mark.parametrize("n_head,n_kvh,n_tok,kv_base", [(64, 4, 745, 0), (64, 4, 761, 130), (64, 4, 299, 3001), (16, 2, 37, 2950)])
+def test_prefill_waves_and_ranges(oracle, n_head, n_kvh, n_tok, kv_base):
+    """two query groups per block (above two and a half waves of one), and one group with its positions in ranges:
+    several waves of blocks, and more ranges than tiles of one"""
+    lib()
+    run_case(oracle, n_tok, kv_base, n_head, n_kvh, 4000 + n_tok)
+    assert q4gpu.load().q4_gpu_last_error() == 0
+
+
 def test_prefill_chunk_over_existing_cache(oracle):
     """the chunked-prefill shape scaled down: 512 new tokens over a 1024-token cache, RoPE'd inputs"""
     lib()
