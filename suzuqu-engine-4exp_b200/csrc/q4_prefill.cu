@@ -18,15 +18,17 @@
  *       issuer warp (one elected lane): a sequence of units.  O += P . V of unit i as soon as the softmax warps have
  *                     published its P (64 positions at a time), then S = Q . K^T of the unit that takes over the score
  *                     buffer just freed (products of one thread run in order)
- *       softmax warps: thread r owns row r: its scores out of tensor memory, causal mask, running max with lazy
- *                     rescale, P = exp2(..) as fp16 back into the first half of the score buffer's columns.
+ *       softmax warps: thread r owns row r (NQ = 1: two threads, half of the unit's positions each): its scores out of
+ *                     tensor memory, causal mask, running max with lazy rescale, P = exp2(..) as fp16 back into the
+ *                     first half of the columns it came from.
  *
  *     A score buffer holds S and then P of one unit, and every group of softmax warps has two, so that the scores of
  *     its next unit are computed under its present exponentials.  NQ = 2 (hd 128): units are (64 positions, group),
  *     four buffers of 64 columns; both groups share every K/V tile.  NQ = 1: units are tiles of 128 positions, two
- *     buffers of 128 columns.  Tensor memory: 256 columns of scores, NQ x hd of O.
- *  3. Where query groups alone would leave SMs idle (a short chunk behind a long prefix), the positions are split over
- *     blockIdx.z; the blocks write (O, m, l) and q4_pf_merge_k combines them.
+ *     buffers of 128 columns; two warps per 32 rows instead of one take the 2048-token prefill of the reference's host
+ *     (24 / 2 heads of 256) from 2591 to 2340 us.  Tensor memory: 256 columns of scores, NQ x hd of O.
+ *  3. Where blocks of one query group leave much of the last wave of SMs idle (a short chunk behind a long prefix), the
+ *     positions are split over blockIdx.z; the blocks write (O, m, l) and q4_pf_merge_k combines them.
  *
  * Measured rates of tcgen05.mma with both operands in shared memory: 64 cycles per 128 x 128 x 16, 48 per 128 x 64 x 16
  * (4 KB of Q and 2 KB of K at 128 B/clk).  Single score buffers of 128 columns per group (all 512 columns in use as
