@@ -889,7 +889,8 @@ struct DecTile {
 constexpr int dec_stages(int groups_bytes) {   /* as many, up to 4, as leave room for 3 blocks per SM */
     return groups_bytes * 4 <= 73728 ? 4 : groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 73728 ? 2 : 1;
 }
-/* LIST: positions from a list (else a dense range).  DIRECT: caches whose base is not aligned for the asynchronous copies (reference ABI only) load fragments into registers */
+/* LIST: positions from a list (else a dense range; with DIRECT, where there is no list).  DIRECT: fragments are loaded straight
+ * into registers, from caches whose base is not aligned for the asynchronous copies (reference ABI only) and in long fp32 scans */
 template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
 struct DecCfg {
     static constexpr bool STAGED = (LAY == LAY_Q8P && HD == 128);
@@ -963,7 +964,7 @@ q4_decode_k(const DecParams P) {
     if (P.early_pos && !early) pdl_wait();
     uint32_t n_kv = newest + 1u;
     if (n_kv > C.max_kv) n_kv = C.max_kv;
-    const int32_t *list = LIST ? P.idx + (size_t)u * P.idx_unit_stride + (size_t)kh * P.idx_kvh_stride : nullptr;
+    const int32_t *list = LIST && (!DIRECT || P.idx) ? P.idx + (size_t)u * P.idx_unit_stride + (size_t)kh * P.idx_kvh_stride : nullptr;
     const uint32_t n_pos = list ? P.width : n_kv;
     const uint32_t steps = (n_pos + 15u) >> 4;
     /* a launch sized for the store's capacity (position from the device) uses as many of its blocks as the context needs */
@@ -2237,6 +2238,9 @@ bool launch(const DecParams &p_in, dim3 grid) {
 }
 template <int LAY, int HD, bool LIST>
 bool launch_nht(const DecParams &p, dim3 grid) {
+    if constexpr (HD == 128 && LAY == LAY_F32 && !LIST) {   /* the list a run-time choice: compiled for dense ranges alone it spills */
+        if (p.direct) return launch<LAY, HD, 1, true, true>(p, grid);
+    }
     if constexpr (HD >= 128 && (LAY == LAY_Q8R || LAY == LAY_F16)) {
         if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true, LIST>(p, grid) : launch<LAY, HD, 2, true, LIST>(p, grid);
     }
@@ -2388,7 +2392,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
     /* Up to 131072 rows two blocks per SM do better than three: the next launch's blocks find room and fill their rings
      * under this one's tail (65536 / 100003 / 262144 rows of q8_0: 15.6 / 19.9 / 37.8 against 17.2 / 20.6 / 33.5 us).
      * With two warps to a tile (more than 8 heads) three blocks are always better. */
-    p.mid_steps = gqa > 8 ? 0u : 8192u;
+    p.mid_steps = gqa > 8 || a.layout == LAY_F32 ? 0u : 8192u;   /* fp32 tiles leave no second stage: all blocks (65536 rows 37.0 -> 33.2) */
     p.mid_splits = (uint32_t)g_q4.sm_count * 2u / units;
     if (p.mid_splits > S) p.mid_splits = S;
     if (p.mid_splits < 1u) p.mid_splits = 1u;
@@ -2414,6 +2418,8 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         Q4_REQUIRE(a.new_k && a.new_v && a.layout != LAY_Q8R && a.hd >= 128,
                    "decode: fused append needs both rows and a store at hd 128 or 256");
     p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
+    /* long scans of fp32 rows at hd 128 as well: Q4_F32_RING_ROWS */
+    if (a.layout == LAY_F32) p.direct = !a.idx && a.hd == 128 && gqa <= 8 && a.n_units == 1 && !a.new_k && rows > Q4_F32_RING_ROWS ? 1u : 0u;
     dim3 grid(S, a.n_kvh, a.n_units);
     switch (a.layout) {
     case LAY_F32: return q4i_launched(launch_hd<LAY_F32>(p, grid, a.hd));

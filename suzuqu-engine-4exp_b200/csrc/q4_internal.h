@@ -41,6 +41,11 @@ struct q4_gpu_kv {
     uint64_t *written;           /* per layer: g_q4.launches when its rows were last written */
 };
 
+/* Dense scans of more fp32 rows than this at hd 128 (up to 8 query heads per kv head) load straight into registers, behind an
+ * append of its own: through the ring every byte crosses the load/store pipe twice, which holds 536 MB at 5.2 TB/s
+ * (262144 rows 102.9 -> 83.8 us, 65536 37.2 -> 26.5; 16384 rows take 11.7 us through the ring, 15.7 without). */
+constexpr uint32_t Q4_F32_RING_ROWS = 24576;
+
 /* runtime state (q4_runtime.cu) */
 struct Q4State {
     bool ok;

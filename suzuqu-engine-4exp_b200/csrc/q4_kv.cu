@@ -768,7 +768,7 @@ extern "C" bool q4_gpu_kv_append_decode_d(q4_gpu_kv *kv, uint32_t layer, const f
                                           uint32_t width, uint32_t idx_kvh_stride, float scale) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_append_decode_d: library not initialised");
     Q4_REQUIRE(kv && k && v && q && out && layer < kv->n_layers && n_head, "kv_append_decode_d: bad argument");
-    const bool fused = kv->hd >= 128;
+    const bool fused = kv->hd >= 128 && (idx || kv->kind != Q4K_F32 || kv->hd != 128 || n_head > 8u * kv->n_kvh || kv->max_kv <= Q4_F32_RING_ROWS);
     if (!fused && !q4_gpu_kv_append_d(kv, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));

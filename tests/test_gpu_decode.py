@@ -539,6 +539,27 @@ def test_dense_at_the_position_word_in_larger_stores(oracle, kind, n_head, hd, m
     st.close()
 
 
+@pytest.mark.parametrize("n_head,n_kvh,max_kv", [(16, 2, 24576), (16, 2, 24577), (3, 3, 24590), (12, 1, 24577)])
+def test_append_and_dense_scan_of_fp32_rows_on_both_sides_of_the_ring(oracle, n_head, n_kvh, max_kv):
+    """fp32 rows at hd 128: through the ring with the append fused up to 24576 rows of capacity and above 8 query heads per kv
+    head, else straight into registers behind an append of its own; the last rows come from the appending call"""
+    L = lib()
+    hd, kvw, n = 128, n_kvh * 128, max_kv
+    k, v = (oracle.normal(78, i, n * kvw).reshape(n, kvw) for i in (0, 1))
+    q = oracle.normal(78, 2, n_head * hd)
+    st, dq, out = q4gpu.KVStore(1, n_kvh, hd, max_kv, 0), dev(q), torch.zeros(n_head * hd, device="cuda")
+    kc, vc = oracle.kv_write(k, 0), oracle.kv_write(v, 0)
+    for r in (1, 17, 600, max_kv):
+        if r > 1:
+            st.append(0, dev(k[:r - 1]), dev(v[:r - 1]), 0, r - 1)
+        L.q4_hip_pos_push(r - 1)
+        st.append_decode_d(0, dev(k[r - 1]), dev(v[r - 1]), dq, out, n_head, 0.0884)
+        ref = oracle.attn(q.reshape(1, n_head, hd), kc, vc, None, n_head, n_kvh, hd, 1, r - 1, max_kv, 0.0884, 0, threads=8)[0]
+        assert_close(host(out).reshape(ref.shape), ref, "%d of %d rows" % (r, max_kv))
+    assert L.q4_gpu_last_error() == 0
+    st.close()
+
+
 @pytest.mark.parametrize("kind", [2, 1])
 def test_batched_dense_sessions_of_unequal_length_against_the_oracle(oracle, kind):
     """one launch over sessions of which some need one block and others dozens"""
