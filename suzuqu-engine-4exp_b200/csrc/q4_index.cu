@@ -672,7 +672,7 @@ struct TkcShared {
 template <uint32_t NB>
 __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *score, int32_t *sel, uint32_t stride,
                                                                uint32_t k_blk, uint32_t ratio, uint32_t pos0,
-                                                               uint32_t width, const int32_t *pp, const int32_t *pos_arr) {
+                                                               uint32_t width, const int32_t *pp, const int32_t *pos_arr, bool early) {
     extern __shared__ __align__(16) uint8_t tkc_smem[];
     TkcShared<NB> &S = *reinterpret_cast<TkcShared<NB> *>(tkc_smem);
     const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = NB > 1 ? tkc_rank() : 0u;
@@ -687,14 +687,20 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
     if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
     tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
-    q4d_pdl_wait();
-    /* the keys are requested before the position arrives: the row's storage reaches to `stride` whatever is visible */
+    /* Only visible keys are read: a caller's last row need not reach to `stride`.  The position comes from the launch, or, if
+     * settled, from its word before the launch waits, so that the keys do not wait for it.  Rows of a batch are `stride`
+     * floats by its interface: their keys are requested before the position, which is a caller's array, arrives. */
+    uint32_t pos = pos0 + t;
+    if (!early) q4d_pdl_wait();
+    if (pp) pos = (uint32_t)*pp + t;
+    if (early) q4d_pdl_wait();
     const float *row = score + (size_t)t * stride;
     const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
+    const uint32_t n_read = pos_arr ? stride : min(stride, ratio ? (pos + 1u) / ratio : 0u);
     uint32_t key[TKC_KPT];
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < stride ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
-    const uint32_t pos = pos_arr ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
+    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
+    if (pos_arr) pos = (uint32_t)pos_arr[t];
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
     int32_t *out = sel + (size_t)t * width;
@@ -1055,7 +1061,7 @@ bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
         return false;
     done = true;
     return topk_start(q4_ix_topkc_k<NB>, dim3(NB, n_tok), IX_TK_THREADS, sizeof(TkcShared<NB>), NB, score, sel, stride, k_blk, ratio, pos0,
-                      width, pp, pos_arr);
+                      width, pp, pos_arr, ix_pdl() && !pos_arr && (!pp || q4i_settled(g_q4.pos_written)));
 }
 /* Which form: rows of up to 8192 keys need one block either way, which keeps them in registers.  Longer rows take the
  * cluster form while all clusters are resident at once (two blocks of 1024 threads per SM), the streaming form beyond

@@ -236,3 +236,35 @@ def test_batched_scores_of_many_uneven_sessions(oracle):
         assert np.array_equal(got[t, :nb].view(np.uint32), want[0, :nb].view(np.uint32)), t
         assert (got[t, nb:] == 7.0).all(), t
         assert np.array_equal(sel[t], oracle.ix_topk(want, 1, stride, 16, ratio, pos, 67)[0]), t
+
+
+@pytest.mark.parametrize("n_vis,slack", [(700, 2000), (8192, 1), (9000, 7000), (20000, 9000), (33000, 30000)])
+@pytest.mark.parametrize("form", ["host", "host_3", "word", "word_settled"])
+def test_topk_reads_visible_scores_only(oracle, n_vis, slack, form):
+    """rows reach to `stride`, but of the last one only the visible scores exist: it ends with its allocation, as a host may lay
+    it out that has sized its buffer for the blocks it has"""
+    L = lib()
+    n_tok = 3 if form == "host_3" else 1
+    stride, pos0 = n_vis + slack, n_vis * RATIO
+    n = (n_tok - 1) * stride + n_vis
+    size = (4 * n + (2 << 20) - 1) // (2 << 20) * (2 << 20)          # whole pages of the device's memory
+    base = L.q4_hip_malloc(size)
+    score = base + size - 4 * n
+    rng = np.random.default_rng(n_vis)
+    rows = np.zeros((n_tok, stride), np.float32)
+    rows[:, :n_vis] = np.maximum(rng.standard_normal((n_tok, n_vis)), 0)
+    flat = np.ascontiguousarray(rows.reshape(-1)[:n])
+    assert L.q4_hip_h2d(score, flat.ctypes.data, 4 * n)
+    d_sel = torch.zeros(n_tok, 2051, dtype=torch.int32, device="cuda")
+    if form.startswith("word"):
+        L.q4_hip_pos_push(pos0)
+        if form == "word_settled":
+            d_copy = torch.empty(256, device="cuda")
+            assert L.q4_hip_fill(d_copy.data_ptr(), 0.0, 256)
+            assert L.q4_hip_qsa_topk_d(score, d_sel.data_ptr(), stride, 512, RATIO, 2051)
+        assert L.q4_hip_qsa_topk_d(score, d_sel.data_ptr(), stride, 512, RATIO, 2051)
+    else:
+        assert L.q4_hip_qsa_topk(score, d_sel.data_ptr(), n_tok, n_vis, stride, 512, RATIO, pos0, 2051)
+    want = oracle.ix_topk(rows, n_tok, stride, 512, RATIO, pos0, 2051)
+    assert np.array_equal(host(d_sel), want)
+    L.q4_hip_free(base)
