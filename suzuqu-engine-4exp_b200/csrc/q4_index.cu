@@ -106,10 +106,12 @@ bool ix_pdl() {
 constexpr uint32_t SC_ROW_FLOATS = IX_HD + 4, SC_WARPS = 2;
 constexpr uint32_t SC_TILE_BYTES = 32u * SC_ROW_FLOATS * sizeof(float);
 constexpr uint32_t SC_SMEM = SC_WARPS * 2u * SC_TILE_BYTES + IX_HD * sizeof(float4);
-/* BATCH: sessions with a pool and a position of their own.  Their tiles are counted through, and every block takes an equal
- * share of the whole, which may end in one session and begin in the next (an equal number of blocks per session leaves
- * most of them idle while the longest context is scanned). */
-template <bool BATCH>
+/* SC_SHARED, SC_EACH: sessions with a pool and a position of their own.  SC_SHARED: their tiles are counted through, and every
+ * block takes an equal share of the whole, which may end in one session and begin in the next (an equal number of blocks per
+ * session leaves most of them idle while the longest context is scanned).  SC_EACH, while there is room for a block per two
+ * tiles of every session: nothing to count (select of 2 sessions of 512 blocks, shared out 7.6 us, 5.5 so). */
+enum { SC_ONE, SC_SHARED, SC_EACH };
+template <int FORM>
 __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, const float *pool, float *score,
                                                                uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                                                                uint32_t pos0, uint32_t ratio, const int32_t *pp,
@@ -175,16 +177,18 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     };
-    if (BATCH) {
+    if (FORM == SC_SHARED) {
         q4d_pdl_wait();
         auto rows_of = [&](uint32_t t) -> uint32_t { return min(((uint32_t)pos_arr[t] + 1u) / ratio, stride); };
-        uint64_t total = 0;
-        for (uint32_t t0 = 0; t0 < n_sess; t0 += 32u) total += __reduce_add_sync(0xffffffffu, t0 + lane < n_sess ? (rows_of(t0 + lane) + 31u) / 32u : 0u);
+        uint32_t rows = lane < n_sess ? rows_of(lane) : 0u;   /* the first 32 sessions' are kept for the walk below */
+        uint64_t total = __reduce_add_sync(0xffffffffu, (rows + 31u) / 32u);
+        for (uint32_t t0 = 32u; t0 < n_sess; t0 += 32u) total += __reduce_add_sync(0xffffffffu, t0 + lane < n_sess ? (rows_of(t0 + lane) + 31u) / 32u : 0u);
         const uint64_t share0 = total * blockIdx.x / gridDim.x, share1 = total * (blockIdx.x + 1u) / gridDim.x;
         uint64_t at = 0;   /* tiles of the sessions before */
         bool again = false;
         for (uint32_t t0 = 0; t0 < n_sess && at < share1; t0 += 32u) {
-            const uint32_t rows = t0 + lane < n_sess ? rows_of(t0 + lane) : 0u, tiles = (rows + 31u) / 32u;
+            if (t0) rows = t0 + lane < n_sess ? rows_of(t0 + lane) : 0u;
+            const uint32_t tiles = (rows + 31u) / 32u;
             uint32_t incl = tiles;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -207,10 +211,11 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
     }
     const uint32_t t = blockIdx.y;
     if (!early) q4d_pdl_wait();
-    const uint32_t pos = (pp ? (uint32_t)*pp : pos0) + t;
+    const uint32_t pos = FORM == SC_EACH ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
     if (early) q4d_pdl_wait();
-    if (pp) n_blocks = min(n_vis, stride);      /* device position: the bound is derived here */
+    if (FORM == SC_EACH) pool = pools[t];
+    if (FORM == SC_EACH || pp) n_blocks = min(n_vis, stride);      /* device position: the bound is derived here */
     const uint32_t lim = min(n_blocks, n_vis);  /* rows to score */
     scan(t, pool, lim, blockIdx.x * SC_WARPS + warp, (lim + 31u) / 32u, gridDim.x * SC_WARPS);
     /* blocks the token cannot see (host-position form only): -1e30 */
@@ -357,26 +362,19 @@ bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n
     q4_ix_score_mt_k<JC><<<grid, SM_THREADS, sm_smem<JC>(), g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     return q4i_launched(q4i_check(cudaGetLastError(), "qsa_score launch"));
 }
-template <bool BATCH>
-bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
-                  uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, const float *const *pools, const int32_t *pos_arr) {
+template <int FORM>
+bool score_start(dim3 grid, const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
+                 uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, const float *const *pools, const int32_t *pos_arr) {
     static bool done = false;
     if (!done) {
-        if (!q4i_check(cudaFuncSetAttribute(q4_ix_score_k<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM),
+        if (!q4i_check(cudaFuncSetAttribute(q4_ix_score_k<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM),
                        "qsa_score smem attribute"))
             return false;
         done = true;
     }
-    /* persistent grid: 3 blocks of 2 warps per SM share 227 KB; fewer when the rows are short */
-    const uint64_t rows = (uint64_t)(pp || BATCH ? stride : n_blocks) * (BATCH ? n_tok : 1u);
-    uint32_t gx = (uint32_t)g_q4.sm_count * 3u;
-    const uint64_t need = (rows + SC_WARPS * 32u - 1u) / (SC_WARPS * 32u);
-    if (!BATCH && n_tok > 1) gx = (gx + n_tok - 1u) / n_tok;
-    if (gx > need) gx = (uint32_t)need;
-    if (gx < 1) gx = 1;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(gx, BATCH ? 1u : n_tok);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(SC_WARPS * 32);
     cfg.dynamicSmemBytes = SC_SMEM;
     cfg.stream = g_q4.stream;
@@ -385,9 +383,21 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = ix_pdl() ? 1 : 0;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k<BATCH>, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr,
-                                                     n_tok, ix_pdl() && (!pp || q4i_settled(g_q4.pos_written))),
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k<FORM>, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr,
+                                                     n_tok, FORM == SC_ONE && ix_pdl() && (!pp || q4i_settled(g_q4.pos_written))),
                      "qsa_score launch"));
+}
+/* persistent grid: 3 blocks of 2 warps per SM share 227 KB; fewer when the rows are short */
+bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
+                  uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, const float *const *pools, const int32_t *pos_arr) {
+    const uint32_t all = (uint32_t)g_q4.sm_count * 3u, need = ((pp || pools ? stride : n_blocks) + SC_WARPS * 32u - 1u) / (SC_WARPS * 32u);
+    if (pools && (uint64_t)need * n_tok > all)
+        return score_start<SC_SHARED>(dim3(all), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr);
+    if (pools) return score_start<SC_EACH>(dim3(need, n_tok), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr);
+    uint32_t gx = n_tok > 1 ? (all + n_tok - 1u) / n_tok : all;
+    if (gx > need) gx = need;
+    if (gx < 1) gx = 1;
+    return score_start<SC_ONE>(dim3(gx, n_tok), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, nullptr, nullptr);
 }
 
 /* ---- selection: one block per token */
@@ -676,6 +686,28 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     extern __shared__ __align__(16) uint8_t tkc_smem[];
     TkcShared<NB> &S = *reinterpret_cast<TkcShared<NB> *>(tkc_smem);
     const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = NB > 1 ? tkc_rank() : 0u;
+    int32_t *out = sel + (size_t)t * width;
+    const uint32_t w_per = (width + NB - 1u) / NB;
+    const uint32_t w0 = min(rank * w_per, width), w1 = min(w0 + w_per, width);   /* this block's slice of the list */
+    /* The position comes from the launch, or, if settled, from its word before the launch waits: a short context's list (every
+     * complete block fits: the dense prefix) is then known before anything is prepared (one token, 512 blocks: 2.9 -> 2.4 us). */
+    uint32_t pos = pos0 + t, n_vis = 0, need = 0;
+    auto visible = [&]() {
+        n_vis = ratio ? (pos + 1u) / ratio : 0u;
+        need = n_vis < k_blk ? n_vis : k_blk;
+    };
+    auto prefix = [&]() {
+        for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
+    };
+    if (early) {
+        if (pp) pos = (uint32_t)*pp + t;
+        visible();
+        if (need == n_vis) {   /* the same decision in all blocks */
+            q4d_pdl_wait();
+            prefix();
+            return;
+        }
+    }
     /* The block's own shared memory is prepared, and the cluster has met once, before the launch waits for
      * the previous kernel: with programmatic dependent launch this part runs under that kernel's tail. */
     constexpr uint32_t BPT = TK_BINS / IX_TK_THREADS;   /* bins per thread */
@@ -687,27 +719,24 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
     if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
     tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
-    /* Only visible keys are read: a caller's last row need not reach to `stride`.  The position comes from the launch, or, if
-     * settled, from its word before the launch waits, so that the keys do not wait for it.  Rows of a batch are `stride`
-     * floats by its interface: their keys are requested before the position, which is a caller's array, arrives. */
-    uint32_t pos = pos0 + t;
-    if (!early) q4d_pdl_wait();
-    if (pp) pos = (uint32_t)*pp + t;
-    if (early) q4d_pdl_wait();
+    q4d_pdl_wait();
+    /* Only visible keys are read: a caller's last row need not reach to `stride`.  Rows of a batch are `stride` floats by its
+     * interface: their keys are requested before the position, which is a caller's array, arrives. */
+    if (!early && pp) pos = (uint32_t)*pp + t;
+    if (!early && !pos_arr) visible();
+    const uint32_t pos_of_batch = pos_arr ? (uint32_t)pos_arr[t] : 0u;
     const float *row = score + (size_t)t * stride;
     const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
-    const uint32_t n_read = pos_arr ? stride : min(stride, ratio ? (pos + 1u) / ratio : 0u);
+    const uint32_t n_read = pos_arr ? stride : min(stride, n_vis);
     uint32_t key[TKC_KPT];
 #pragma unroll
     for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
-    if (pos_arr) pos = (uint32_t)pos_arr[t];
-    const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
-    const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
-    int32_t *out = sel + (size_t)t * width;
-    const uint32_t w_per = (width + NB - 1u) / NB;
-    const uint32_t w0 = min(rank * w_per, width), w1 = min(w0 + w_per, width);   /* this block's slice of the list */
-    if (need == n_vis) {   /* every complete block fits: the dense prefix (same decision in all blocks) */
-        for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
+    if (pos_arr) {
+        pos = pos_of_batch;
+        visible();
+    }
+    if (need == n_vis) {
+        prefix();
         return;
     }
 #pragma unroll
@@ -1113,7 +1142,7 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
         if (wide <= narrow && wide < scan) return score_mt_launch<16>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
         if (narrow < scan) return score_mt_launch<8>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     }
-    return score_launch<false>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr, nullptr, nullptr);
+    return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr, nullptr, nullptr);
 }
 /* Device position (graph-captured decode): the grid covers `stride` blocks, the bound comes from the
  * position word inside the kernel. */
@@ -1121,7 +1150,7 @@ extern "C" bool q4_hip_qsa_score_d(const float *q, const float *pool, float *sco
                                    uint32_t hd, uint32_t ratio) {
     if (!g_q4.ok || !g_q4.pos_d || !q || !pool || !score || hd != IX_HD || n_head == 0 || n_head > 4 || stride == 0)
         return false;
-    return score_launch<false>(q, pool, score, 1, 0, stride, n_head, 0, ratio, g_q4.pos_d, nullptr, nullptr);
+    return score_launch(q, pool, score, 1, 0, stride, n_head, 0, ratio, g_q4.pos_d, nullptr, nullptr);
 }
 extern "C" bool q4_hip_qsa_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
                                 uint32_t k_blk, uint32_t ratio, uint32_t pos0, uint32_t width) {
@@ -1147,6 +1176,6 @@ extern "C" bool q4_gpu_qsa_select_batch(const float *const *pools, const int32_t
     Q4_REQUIRE(pools && pos && q && score && sel && n_sess && stride && ratio && width, "qsa_select_batch: bad argument");
     Q4_REQUIRE(hd == IX_HD && n_head >= 1 && n_head <= 4 && k_blk >= 1 && k_blk <= IX_MAX_KBLK,
                "qsa_select_batch: unsupported shape");
-    return score_launch<true>(q, nullptr, score, n_sess, 0, stride, n_head, 0, ratio, nullptr, pools, pos) &&
+    return score_launch(q, nullptr, score, n_sess, 0, stride, n_head, 0, ratio, nullptr, pools, pos) &&
            launch_topk(score, sel, n_sess, stride, k_blk, ratio, 0, width, nullptr, pos);
 }

@@ -268,3 +268,29 @@ def test_topk_reads_visible_scores_only(oracle, n_vis, slack, form):
     want = oracle.ix_topk(rows, n_tok, stride, 512, RATIO, pos0, 2051)
     assert np.array_equal(host(d_sel), want)
     L.q4_hip_free(base)
+
+
+@pytest.mark.parametrize("n_sess,positions", [(6, [4031 * 4 + 2, 3, 2, 255, 256, 4032 * 4 + 1]), (7, [4031 * 4 + 2, 3, 2, 255, 256, 4032 * 4 + 1, 700]),
+                                              (1, [63]), (2, [64 * 4 - 1, 64 * 4 + 3])])
+def test_batched_scores_with_and_without_a_block_for_every_two_tiles(oracle, n_sess, positions):
+    """both sides of the line between a grid that gives every session its own blocks and one that shares all tiles out
+    (6 sessions of 64 block pairs fit 444 blocks, 7 do not)"""
+    L = lib()
+    rng = np.random.default_rng(n_sess)
+    stride = 4033 if n_sess > 2 else 65
+    q = rng.standard_normal((n_sess, 4, 128)).astype(np.float32)
+    pools = [rng.standard_normal((max((p + 1) // RATIO, 1), 128)).astype(np.float32) for p in positions]
+    d_pools = [dev(p) for p in pools]
+    ptrs = torch.tensor([t.data_ptr() for t in d_pools], dtype=torch.int64, device="cuda")
+    d_pos = torch.tensor(positions, dtype=torch.int32, device="cuda")
+    d_score = torch.full((n_sess, stride), 7.0, device="cuda")
+    d_sel = torch.zeros(n_sess, 67, dtype=torch.int32, device="cuda")
+    assert L.q4_gpu_qsa_select_batch(ptrs.data_ptr(), d_pos.data_ptr(), dev(q).data_ptr(), d_score.data_ptr(), d_sel.data_ptr(), n_sess, stride,
+                                     4, 128, 16, RATIO, 67)
+    got, sel = host(d_score), host(d_sel)
+    for t, pos in enumerate(positions):
+        nb = (pos + 1) // RATIO
+        want = oracle.ix_score(q[t:t + 1], pools[t], 1, nb, stride, 4, pos, RATIO) if nb else np.zeros((1, stride), np.float32)
+        assert np.array_equal(got[t, :nb].view(np.uint32), want[0, :nb].view(np.uint32)), t
+        assert (got[t, nb:] == 7.0).all(), t
+        assert np.array_equal(sel[t], oracle.ix_topk(want, 1, stride, 16, RATIO, pos, 67)[0]), t
