@@ -340,15 +340,22 @@ __global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
-/* Estimated ns of the product with tiles of 16 JC blocks, and of the scan.  A tile takes a time of its own however few of
- * its 32 tokens exist. */
-constexpr uint64_t SM_TILE_NS[2] = {13000, 18000};   /* JC = 8, 16 */
+/* Estimated ns of the product with tiles of 16 JC blocks, and of the scan; fitted to 1 .. 512 tokens over 16 .. 65 536 blocks,
+ * within 10 % where the two are close.  Product: a tile takes a time of its own however few of its 32 tokens exist (us,
+ * narrow / wide tiles: 32 tokens over 8192 blocks 18.0 / -, 32 over 32 768 - / 29.1, 512 over 65 536 - / 726). */
 uint64_t score_mt_ns(uint32_t n_tok, uint32_t n_blocks, uint32_t jc) {
     const uint64_t tiles = (uint64_t)((n_blocks + 16u * jc - 1u) / (16u * jc)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
-    return (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count * SM_TILE_NS[jc == 16u];
+    return 3500u + (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count * (jc == 16u ? 26200u : 13200u);
 }
-/* (8 tokens at 65 536 blocks: the scan takes 62 us; at 8192 blocks it keeps 8 tokens with 9.4 us) */
-uint64_t score_scan_ns(uint32_t n_tok, uint32_t n_blocks) { return (uint64_t)n_tok * n_blocks * 1200u / 8192u; }
+/* Scan: tiles of 32 blocks a warp takes one after the other, and again (with the card nearly to itself) where the tokens'
+ * grids do not fit at once: 4 tokens over 65 536 blocks 25.0 us, 5 (445 blocks of 444) 40.3, 8 62.7, 12 62.5. */
+uint64_t score_scan_ns(uint32_t n_tok, uint32_t n_blocks) {
+    const uint32_t all = (uint32_t)g_q4.sm_count * 3u, need = (n_blocks + SC_WARPS * 32u - 1u) / (SC_WARPS * 32u);
+    uint32_t gx = (all + n_tok - 1u) / n_tok;
+    if (gx > need) gx = need;
+    const uint64_t per_warp = ((n_blocks + 31u) / 32u + gx * SC_WARPS - 1u) / (gx * SC_WARPS), waves = ((uint64_t)gx * n_tok + all - 1u) / all;
+    return 3000u + per_warp * (2150u + (waves - 1u) * 1250u);
+}
 template <uint32_t JC>
 bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                      uint32_t pos0, uint32_t ratio) {

@@ -294,3 +294,18 @@ def test_batched_scores_with_and_without_a_block_for_every_two_tiles(oracle, n_s
         assert np.array_equal(got[t, :nb].view(np.uint32), want[0, :nb].view(np.uint32)), t
         assert (got[t, nb:] == 7.0).all(), t
         assert np.array_equal(sel[t], oracle.ix_topk(want, 1, stride, 16, RATIO, pos, 67)[0]), t
+
+
+@pytest.mark.parametrize("n_tok,blocks", [(4, 32768), (5, 65536), (8, 65536), (12, 8192), (12, 16384), (16, 8192)])
+def test_scores_of_a_few_tokens_on_both_sides_of_the_product(n_tok, blocks):
+    """whichever form the estimate picks, every token's row has the bits of a call of its own"""
+    L = lib()
+    g = torch.Generator(device="cuda").manual_seed(blocks + n_tok)
+    pool = torch.randn(blocks, 128, device="cuda", generator=g)
+    q = torch.randn(n_tok, 4, 128, device="cuda", generator=g)
+    pos0 = blocks * RATIO - n_tok
+    a, b = torch.zeros(n_tok, blocks, device="cuda"), torch.zeros(n_tok, blocks, device="cuda")
+    assert L.q4_hip_qsa_score(q.data_ptr(), pool.data_ptr(), a.data_ptr(), n_tok, blocks, blocks, 4, 128, pos0, RATIO)
+    for t in range(n_tok):
+        assert L.q4_hip_qsa_score(q[t].data_ptr(), pool.data_ptr(), b[t].data_ptr(), 1, blocks, blocks, 4, 128, pos0 + t, RATIO)
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
