@@ -689,61 +689,54 @@ struct TkcShared {
 template <uint32_t NB>
 __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *score, int32_t *sel, uint32_t stride,
                                                                uint32_t k_blk, uint32_t ratio, uint32_t pos0,
-                                                               uint32_t width, const int32_t *pp, const int32_t *pos_arr, bool early) {
+                                                               uint32_t width, const int32_t *pp, const int32_t *pos_arr, uint32_t last_read, bool early) {
     extern __shared__ __align__(16) uint8_t tkc_smem[];
     TkcShared<NB> &S = *reinterpret_cast<TkcShared<NB> *>(tkc_smem);
     const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = NB > 1 ? tkc_rank() : 0u;
-    int32_t *out = sel + (size_t)t * width;
-    const uint32_t w_per = (width + NB - 1u) / NB;
-    const uint32_t w0 = min(rank * w_per, width), w1 = min(w0 + w_per, width);   /* this block's slice of the list */
-    /* The position comes from the launch, or, if settled, from its word before the launch waits: a short context's list (every
-     * complete block fits: the dense prefix) is then known before anything is prepared (one token, 512 blocks: 2.9 -> 2.4 us). */
-    uint32_t pos = pos0 + t, n_vis = 0, need = 0;
-    auto visible = [&]() {
-        n_vis = ratio ? (pos + 1u) / ratio : 0u;
-        need = n_vis < k_blk ? n_vis : k_blk;
-    };
-    auto prefix = [&]() {
-        for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
-    };
+    /* A position that comes with the launch or is settled in its word tells before anything is prepared whether every complete
+     * block fits, the list of a short context (one token, 512 blocks: 2.9 -> 2.4 us). */
+    uint32_t pos = pos0 + t, n_read = t + 1u < gridDim.y ? stride : last_read;
+    bool fits = false;
     if (early) {
-        if (pp) pos = (uint32_t)*pp + t;
-        visible();
-        if (need == n_vis) {   /* the same decision in all blocks */
-            q4d_pdl_wait();
-            prefix();
-            return;
-        }
+        if (pp) pos = (uint32_t)*pp;
+        fits = (pos + 1u) < (k_blk + 1u) * ratio;
+        if (pp) n_read = min(stride, (pos + 1u) / ratio);
     }
     /* The block's own shared memory is prepared, and the cluster has met once, before the launch waits for
      * the previous kernel: with programmatic dependent launch this part runs under that kernel's tail. */
     constexpr uint32_t BPT = TK_BINS / IX_TK_THREADS;   /* bins per thread */
     static_assert(BPT == 4, "one 16-byte word of counts per thread");
     uint32_t *h2 = NB > 1 ? S.ha : S.h2;
-    reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
-    reinterpret_cast<uint4 *>(NB > 1 ? S.hb : S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
-    if (tx < 256) S.h3[tx] = 0u;
-    if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
-    if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
-    tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
+    if (!fits) {
+        reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+        reinterpret_cast<uint4 *>(NB > 1 ? S.hb : S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
+        if (tx < 256) S.h3[tx] = 0u;
+        if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
+        if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
+        tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
+    }
     q4d_pdl_wait();
-    /* Only visible keys are read: a caller's last row need not reach to `stride`.  Rows of a batch are `stride` floats by its
-     * interface: their keys are requested before the position, which is a caller's array, arrives. */
-    if (!early && pp) pos = (uint32_t)*pp + t;
-    if (!early && !pos_arr) visible();
-    const uint32_t pos_of_batch = pos_arr ? (uint32_t)pos_arr[t] : 0u;
+    /* The keys are requested before a position that has yet to be read arrives.  Only visible ones of the last row: a host's
+     * need not reach to `stride` (those of a batch do by its interface, and there the last row has stride too). */
+    if (!early && pp) {
+        pos = (uint32_t)*pp;
+        n_read = min(stride, (pos + 1u) / ratio);
+    }
     const float *row = score + (size_t)t * stride;
     const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
-    const uint32_t n_read = pos_arr ? stride : min(stride, n_vis);
     uint32_t key[TKC_KPT];
+    if (!fits) {
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
-    if (pos_arr) {
-        pos = pos_of_batch;
-        visible();
+        for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
     }
-    if (need == n_vis) {
-        prefix();
+    if (pos_arr) pos = (uint32_t)pos_arr[t];
+    const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
+    int32_t *out = sel + (size_t)t * width;
+    const uint32_t w_per = (width + NB - 1u) / NB;
+    const uint32_t w0 = min(rank * w_per, width), w1 = min(w0 + w_per, width);   /* this block's slice of the list */
+    if (need == n_vis) {   /* every complete block fits: the dense prefix (same decision in all blocks) */
+        for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
         return;
     }
 #pragma unroll
@@ -1096,8 +1089,9 @@ bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
                             "qsa_topk smem attribute"))
         return false;
     done = true;
+    const uint32_t vis = ratio ? (pos0 + n_tok) / ratio : 0u;   /* of the last token, where the host gives the position */
     return topk_start(q4_ix_topkc_k<NB>, dim3(NB, n_tok), IX_TK_THREADS, sizeof(TkcShared<NB>), NB, score, sel, stride, k_blk, ratio, pos0,
-                      width, pp, pos_arr, ix_pdl() && !pos_arr && (!pp || q4i_settled(g_q4.pos_written)));
+                      width, pp, pos_arr, pos_arr || vis > stride ? stride : vis, ix_pdl() && ratio && !pos_arr && (!pp || q4i_settled(g_q4.pos_written)));
 }
 /* Which form: rows of up to 8192 keys need one block either way, which keeps them in registers.  Longer rows take the
  * cluster form while all clusters are resident at once (two blocks of 1024 threads per SM), the streaming form beyond
