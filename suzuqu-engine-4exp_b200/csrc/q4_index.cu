@@ -694,12 +694,15 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     TkcShared<NB> &S = *reinterpret_cast<TkcShared<NB> *>(tkc_smem);
     const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = NB > 1 ? tkc_rank() : 0u;
     /* A position that comes with the launch or is settled in its word tells before anything is prepared whether every complete
-     * block fits, the list of a short context (one token, 512 blocks: 2.9 -> 2.4 us). */
+     * block fits, the list of a short context (one token, 512 blocks: 2.9 -> 2.4 us; costs the others 0.3 of 7.5). */
     uint32_t pos = pos0 + t, n_read = t + 1u < gridDim.y ? stride : last_read;
-    bool fits = false;
     if (early) {
         if (pp) pos = (uint32_t)*pp;
-        fits = (pos + 1u) < (k_blk + 1u) * ratio;
+        if (pos + 1u < (k_blk + 1u) * ratio) {   /* the same decision in all blocks */
+            q4d_pdl_wait();
+            for (uint32_t w = rank * IX_TK_THREADS + tx; w < width; w += NB * IX_TK_THREADS) sel[(size_t)t * width + w] = w <= pos ? (int32_t)w : -1;
+            return;
+        }
         if (pp) n_read = min(stride, (pos + 1u) / ratio);
     }
     /* The block's own shared memory is prepared, and the cluster has met once, before the launch waits for
@@ -707,14 +710,12 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     constexpr uint32_t BPT = TK_BINS / IX_TK_THREADS;   /* bins per thread */
     static_assert(BPT == 4, "one 16-byte word of counts per thread");
     uint32_t *h2 = NB > 1 ? S.ha : S.h2;
-    if (!fits) {
-        reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
-        reinterpret_cast<uint4 *>(NB > 1 ? S.hb : S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
-        if (tx < 256) S.h3[tx] = 0u;
-        if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
-        if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
-        tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
-    }
+    reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4 *>(NB > 1 ? S.hb : S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
+    if (tx < 256) S.h3[tx] = 0u;
+    if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
+    if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
+    tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
     q4d_pdl_wait();
     /* The keys are requested before a position that has yet to be read arrives.  Only visible ones of the last row: a host's
      * need not reach to `stride` (those of a batch do by its interface, and there the last row has stride too). */
@@ -725,10 +726,8 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     const float *row = score + (size_t)t * stride;
     const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
     uint32_t key[TKC_KPT];
-    if (!fits) {
 #pragma unroll
-        for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
-    }
+    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
     if (pos_arr) pos = (uint32_t)pos_arr[t];
     const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
