@@ -198,8 +198,8 @@ struct Q4DecodeArgs {
 bool q4i_decode(const Q4DecodeArgs &a);
 
 /* causal attention of n_tok > 1 query tokens on the tensor cores (q4_prefill.cu): hd 128 or 256 (a native q8_0 store:
- * 128), 1..16 query heads per kv head, scale > 0, 16-byte aligned operands.  1 = enqueued, 0 = failed, -1 = the
- * workspace would have to grow inside a capture. */
+ * 128), 1..16 query heads per kv head, scale > 0, 16-byte aligned operands.  1 = enqueued, 0 = failed, -1 = its
+ * workspace is not to be had (it may not grow inside a capture, or no memory is left). */
 struct Q4PrefillArgs {
     Q4Cache cache;
     int layout;

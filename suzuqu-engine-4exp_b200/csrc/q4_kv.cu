@@ -279,7 +279,7 @@ static bool legacy_decode(const float *q, const void *kc, const void *vc, const 
         f.q = q; f.gate = gate; f.out = out;
         f.n_tok = n_tok; f.kv_base = kv_base; f.scale = scale;
         const int r = q4i_prefill(f);
-        if (r >= 0) return r == 1;   /* else: its workspace may not grow inside a capture */
+        if (r >= 0) return r == 1;   /* else: no workspace; the decode kernel needs no operand images */
     }
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));

@@ -798,17 +798,26 @@ __global__ void __launch_bounds__(256) q4_pf_merge_k(const PrefillParams P, uint
 /* operand images of the rows a chunk can see, and the parts of split ranges; grows on demand, never inside a capture */
 uint8_t *g_stage = nullptr;
 size_t g_stage_bytes = 0;
-bool stage_reserve(size_t bytes) {
-    if (bytes <= g_stage_bytes) return true;
-    if (g_q4.capturing) return false;
-    if (!q4i_check(cudaStreamSynchronize(g_q4.stream), "prefill staging sync")) return false;
+/* 1 = there, 0 = an error, -1 = not to be had: inside a capture, or no memory is left for it */
+int stage_reserve(size_t bytes) {
+    if (bytes <= g_stage_bytes) return 1;
+    if (g_q4.capturing) return -1;
+    if (!q4i_check(cudaStreamSynchronize(g_q4.stream), "prefill staging sync")) return 0;
     if (g_stage) cudaFree(g_stage);
     g_stage = nullptr;
     g_stage_bytes = 0;
-    const size_t want = bytes + bytes / 4;
-    if (!q4i_check(cudaMalloc(&g_stage, want), "prefill staging alloc")) return false;
-    g_stage_bytes = want;
-    return true;
+    const size_t wants[2] = {bytes + bytes / 4, bytes};   /* with room to grow, if that can be had */
+    for (size_t want : wants) {
+        const cudaError_t e = cudaMalloc(&g_stage, want);
+        if (e == cudaSuccess) {
+            g_stage_bytes = want;
+            return 1;
+        }
+        g_stage = nullptr;
+        if (e != cudaErrorMemoryAllocation) return q4i_check(e, "prefill staging alloc");
+        (void)cudaGetLastError();
+    }
+    return -1;
 }
 
 template <int HD, int NQ, int KP>
@@ -869,8 +878,8 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     uint32_t split = nq == 1 ? best_split(blocks, sms, tiles, (uint64_t)a.n_tok * a.n_head, hd, kp) : 1u;
     const size_t k_bytes = (size_t)a.n_kvh * tiles * kp * (hd / 128u) * PF_CHUNK, v_bytes = (size_t)a.n_kvh * tiles * (hd / 128u) * PF_CHUNK;
     const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
-    if (!stage_reserve(k_bytes + v_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0)))
-        return g_q4.capturing ? -1 : 0;
+    const int room = stage_reserve(k_bytes + v_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0));
+    if (room != 1) return room;
 
     PrefillParams p;
     memset(&p, 0, sizeof(p));
@@ -919,5 +928,8 @@ extern "C" bool q4_gpu_kv_prefill(const q4_gpu_kv *kv, uint32_t layer, const voi
     a.q = q_bf16; a.q_bf16 = 1; a.gate = gate; a.out = out_bf16; a.out_bf16 = 1;
     a.n_tok = n_tok; a.kv_base = kv_base; a.scale = scale;
     const int r = q4i_prefill(a);
-    return r < 0 ? q4i_fail(Q4E_SCRATCH, "kv_prefill: staging buffer too small inside a capture") : r == 1;
+    if (r < 0)
+        return g_q4.capturing ? q4i_fail(Q4E_SCRATCH, "kv_prefill: staging buffer too small inside a capture")
+                              : q4i_fail(Q4E_CUDA, "kv_prefill: no device memory for the staging buffer");
+    return r == 1;
 }

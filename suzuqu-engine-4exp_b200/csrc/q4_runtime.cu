@@ -17,6 +17,7 @@ bool q4i_fail(uint32_t bit, const char *what) {
 }
 bool q4i_check(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return true;
+    (void)cudaGetLastError();   /* reported here: the next launch's check is not to find it again */
     g_q4.err_h |= Q4E_CUDA;
     fprintf(stderr, "q4 gpu: %s: %s\n", what, cudaGetErrorString(e));
     return false;

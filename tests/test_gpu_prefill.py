@@ -179,3 +179,68 @@ def test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, n_head, n_kvh, h
     ref = oracle.attn(q.reshape(n_tok, n_head, hd), kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, max_kv, scale, kind, threads=8)
     assert_close(host(out).reshape(ref.shape), ref, "kind %d %d/%d/%d" % (kind, n_head, n_kvh, hd))
     assert L.q4_gpu_last_error() == 0
+
+
+def chunk_caches(L, seed, rows, kvw, kind=2):
+    """caches of N(0,1) rows in the reference layout, quantised on the device"""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    bpt = {2: kvw // 32 * 34, 1: kvw * 2}[kind]
+    out = []
+    for _ in range(2):
+        c = torch.empty(rows * bpt, dtype=torch.uint8, device="cuda")
+        for p in range(0, rows, 65536):
+            m = min(65536, rows - p)
+            x = torch.randn(m * kvw, device="cuda", generator=g)
+            f = L.q4_hip_f32_to_q8 if kind == 2 else L.q4_hip_f32_to_f16
+            assert f(c.data_ptr() + p * bpt, x.data_ptr(), m * kvw)
+        torch.cuda.synchronize()
+        out.append(c)
+    return out
+
+
+def test_reference_abi_chunk_where_no_memory_is_left_for_operand_images():
+    """12 tokens over 262144 rows want 1 GB of operand images: with 0.4 GB left on the card they are answered without, by the
+    decode kernel, with no status bit, and the next launch is not taken for a failed one"""
+    from gpu_util import assert_close
+    L = lib()
+    L.q4_hip_shutdown()                       # gives back what other tests made it reserve
+    L = lib()
+    n_head, n_kvh, hd, rows, n_tok = 24, 2, 256, 262144, 12
+    kc, vc = chunk_caches(L, 11, rows, n_kvh * hd)
+    g = torch.Generator(device="cuda").manual_seed(12)
+    q, gate = torch.randn(n_tok, n_head, hd, device="cuda", generator=g), torch.randn(n_tok, n_head, hd, device="cuda", generator=g)
+    out, want = torch.full_like(q, float("nan")), torch.empty_like(q)
+    scale = 1.0 / 16.0
+    for t in range(n_tok):
+        assert L.q4_hip_qsa_decode_n(q[t].data_ptr(), kc.data_ptr(), vc.data_ptr(), gate[t].data_ptr(), want[t].data_ptr(), n_head, n_kvh, hd, 1,
+                                     rows - n_tok + t, rows, scale, 2)
+    # the chunk kernels, loaded while there is room
+    assert L.q4_hip_qsa_decode_n(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), gate.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, n_tok, 0, 2048, scale, 2)
+    row = torch.randn(n_kvh * hd + 4, device="cuda", generator=g)
+    kf, vf = torch.zeros(4 * n_kvh * hd, device="cuda"), torch.zeros(4 * n_kvh * hd, device="cuda")
+    L.q4_hip_pos_push(1)
+    odd = (row.data_ptr() + 4, row.data_ptr() + 4, n_kvh * hd, 4 * n_kvh * hd, 0)
+    assert L.q4_hip_kv_append_d(kf.data_ptr(), vf.data_ptr(), *odd)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = L.q4_hip_malloc(torch.cuda.mem_get_info()[0] - (400 << 20))
+    assert hog
+    out.fill_(float("nan"))
+    ok = L.q4_hip_qsa_decode_n(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), gate.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, n_tok, rows - n_tok, rows,
+                               scale, 2)
+    nxt = L.q4_hip_kv_append_d(kf.data_ptr(), vf.data_ptr(), *odd)
+    got, err = host(out), L.q4_gpu_last_error()
+    L.q4_hip_free(hog)
+    assert ok and nxt and err == 0
+    assert_close(got, host(want), "chunk without operand images")
+    # the store's own prefill has no other form: refused, reported, and the next launch is sound
+    st = q4gpu.KVStore(1, 2, 128, 262144, 2)
+    bq = torch.zeros(8 * 16 * 128, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    hog = L.q4_hip_malloc(torch.cuda.mem_get_info()[0] - (100 << 20))
+    bad = L.q4_gpu_kv_prefill(st.h, 0, bq.data_ptr(), None, bq.data_ptr(), 16, 8, 262144 - 8, 0.1)
+    nxt = L.q4_hip_kv_append_d(kf.data_ptr(), vf.data_ptr(), *odd)
+    torch.cuda.synchronize()
+    L.q4_hip_free(hog)
+    assert not bad and nxt and L.q4_gpu_last_error() & 2
+    st.close()
