@@ -46,6 +46,8 @@ struct q4_gpu_kv {
  * (262144 rows 102.9 -> 83.8 us, 65536 37.2 -> 26.5; 16384 rows take 11.7 us through the ring, 15.7 without). */
 constexpr uint32_t Q4_F32_RING_ROWS = 24576;
 
+struct Q4PtrList { void **p; uint32_t n; };
+
 /* runtime state (q4_runtime.cu) */
 struct Q4State {
     bool ok;
@@ -67,6 +69,11 @@ struct Q4State {
     size_t part_floats;
     uint32_t *counters;
     size_t n_counters;
+    /* An instantiated graph keeps the addresses its launches were captured with.  A workspace that a capture has used and
+     * that then grows is kept until no graph is left (sizes grow by a quarter at least, so what is kept stays below four
+     * times what is in use). */
+    bool part_captured, counters_captured, stage_captured;
+    Q4PtrList graphs, kept;      /* instantiated and not yet freed; workspaces that one of them may use */
 };
 extern Q4State g_q4;
 
@@ -79,6 +86,7 @@ inline bool q4i_launched(bool ok) {
 inline bool q4i_settled(uint64_t written) { return g_q4.launches > written && g_q4.launches > g_q4.unsettled; }
 inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->written[layer] = g_q4.launches; }
 bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside capture, fails inside */
+void q4i_give_back(void *p, bool captured);              /* cudaFree, now or with the last graph */
 
 #define Q4_REQUIRE(cond, what)                    \
     do {                                          \

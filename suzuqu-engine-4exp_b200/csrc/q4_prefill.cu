@@ -800,12 +800,16 @@ uint8_t *g_stage = nullptr;
 size_t g_stage_bytes = 0;
 /* 1 = there, 0 = an error, -1 = not to be had: inside a capture, or no memory is left for it */
 int stage_reserve(size_t bytes) {
-    if (bytes <= g_stage_bytes) return 1;
+    if (bytes <= g_stage_bytes) {
+        g_q4.stage_captured = g_q4.stage_captured || g_q4.capturing;
+        return 1;
+    }
     if (g_q4.capturing) return -1;
     if (!q4i_check(cudaStreamSynchronize(g_q4.stream), "prefill staging sync")) return 0;
-    if (g_stage) cudaFree(g_stage);
+    q4i_give_back(g_stage, g_q4.stage_captured);
     g_stage = nullptr;
     g_stage_bytes = 0;
+    g_q4.stage_captured = false;
     const size_t wants[2] = {bytes + bytes / 4, bytes};   /* with room to grow, if that can be had */
     for (size_t want : wants) {
         const cudaError_t e = cudaMalloc(&g_stage, want);

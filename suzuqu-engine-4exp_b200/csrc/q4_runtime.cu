@@ -23,6 +23,28 @@ bool q4i_check(cudaError_t e, const char *what) {
     return false;
 }
 
+static bool list_add(Q4PtrList &l, void *p) {
+    void **q = (void **)realloc(l.p, (l.n + 1u) * sizeof(void *));
+    if (!q) return false;
+    l.p = q;
+    l.p[l.n++] = p;
+    return true;
+}
+static void list_clear(Q4PtrList &l) {
+    free(l.p);
+    l.p = nullptr;
+    l.n = 0;
+}
+static void free_kept() {
+    for (uint32_t i = 0; i < g_q4.kept.n; i++) cudaFree(g_q4.kept.p[i]);
+    list_clear(g_q4.kept);
+}
+void q4i_give_back(void *p, bool captured) {
+    if (!p) return;
+    if (!captured || !g_q4.graphs.n) cudaFree(p);
+    else (void)list_add(g_q4.kept, p);   /* where the host has no memory left it is lost rather than pulled from under a graph */
+}
+
 /* Scratch for the split-KV records and arrival counters.  Grows only outside capture (an
  * allocation would invalidate the capture, src/q4_rocm.cu:55-57); counters start at zero and every
  * kernel leaves them at zero. */
@@ -30,9 +52,10 @@ bool q4i_scratch(size_t part_floats, size_t n_counters) {
     if (part_floats > g_q4.part_floats) {
         if (g_q4.capturing) return q4i_fail(Q4E_SCRATCH, "attention scratch too small inside a capture");
         if (!q4i_check(cudaStreamSynchronize(g_q4.stream), "scratch sync")) return false;
-        if (g_q4.part) cudaFree(g_q4.part);
+        q4i_give_back(g_q4.part, g_q4.part_captured);
         g_q4.part = nullptr;
         g_q4.part_floats = 0;
+        g_q4.part_captured = false;
         size_t want = part_floats + part_floats / 4;
         if (!q4i_check(cudaMalloc(&g_q4.part, want * sizeof(float)), "scratch alloc")) return false;
         g_q4.part_floats = want;
@@ -40,13 +63,18 @@ bool q4i_scratch(size_t part_floats, size_t n_counters) {
     if (n_counters > g_q4.n_counters) {
         if (g_q4.capturing) return q4i_fail(Q4E_SCRATCH, "attention counters too small inside a capture");
         if (!q4i_check(cudaStreamSynchronize(g_q4.stream), "scratch sync")) return false;
-        if (g_q4.counters) cudaFree(g_q4.counters);
+        q4i_give_back(g_q4.counters, g_q4.counters_captured);
         g_q4.counters = nullptr;
         g_q4.n_counters = 0;
+        g_q4.counters_captured = false;
         size_t want = n_counters * 2;
         if (!q4i_check(cudaMalloc(&g_q4.counters, want * sizeof(uint32_t)), "counter alloc")) return false;
         if (!q4i_check(cudaMemset(g_q4.counters, 0, want * sizeof(uint32_t)), "counter clear")) return false;
         g_q4.n_counters = want;
+    }
+    if (g_q4.capturing) {
+        g_q4.part_captured = g_q4.part_captured || part_floats;
+        g_q4.counters_captured = g_q4.counters_captured || n_counters;
     }
     return true;
 }
@@ -91,6 +119,8 @@ extern "C" bool q4_hip_init(void) {
 extern "C" void q4_hip_shutdown(void) {
     if (!g_q4.ok) return;
     cudaDeviceSynchronize();
+    free_kept();
+    list_clear(g_q4.graphs);
     if (g_q4.part) cudaFree(g_q4.part);
     if (g_q4.counters) cudaFree(g_q4.counters);
     if (g_q4.pos_d) cudaFree(g_q4.pos_d);
@@ -272,6 +302,10 @@ extern "C" void *q4_hip_graph_end(void) {
         (void)cudaGetLastError();
         return nullptr;
     }
+    if (!list_add(g_q4.graphs, ex)) {
+        (void)cudaGraphExecDestroy(ex);
+        return nullptr;
+    }
     (void)cudaGraphUpload(ex, g_q4.stream);
     return (void *)ex;
 }
@@ -285,7 +319,15 @@ extern "C" bool q4_hip_graph_launch(void *exec) {
     return q4i_check(cudaGraphLaunch((cudaGraphExec_t)exec, g_q4.stream), "graph launch");
 }
 extern "C" void q4_hip_graph_free(void *exec) {
-    if (exec) (void)cudaGraphExecDestroy((cudaGraphExec_t)exec);
+    if (!exec) return;
+    (void)cudaGraphExecDestroy((cudaGraphExec_t)exec);
+    Q4PtrList &l = g_q4.graphs;
+    for (uint32_t i = 0; i < l.n; i++)
+        if (l.p[i] == exec) {
+            l.p[i] = l.p[--l.n];
+            if (l.n == 0) free_kept();   /* cudaFree waits for a launch that is still running */
+            break;
+        }
 }
 
 /* ---- a pipelined step loop over one set of step buffers -------------------------------------------

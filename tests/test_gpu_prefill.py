@@ -244,3 +244,51 @@ def test_reference_abi_chunk_where_no_memory_is_left_for_operand_images():
     L.q4_hip_free(hog)
     assert not bad and nxt and L.q4_gpu_last_error() & 2
     st.close()
+
+
+def test_captured_chunk_keeps_its_workspace_when_that_grows():
+    """a captured slice, then a longer one that makes the operand images grow, memory of the old size taken by others, and the
+    graph again; the same for a captured scan whose records lie in scratch.  With the last graph the old workspaces go back."""
+    L = lib()
+    L.q4_gpu_set_stream(None)                 # captures need a created stream
+    L.q4_hip_shutdown()
+    L = q4gpu.init()
+    with torch.cuda.stream(torch.cuda.ExternalStream(L.q4_gpu_stream())):
+        n_head, n_kvh, hd, n_tok, rows, more = 24, 2, 256, 16, 2048, 40000
+        kc, vc = chunk_caches(L, 21, more, n_kvh * hd, 1)
+        g = torch.Generator(device="cuda").manual_seed(22)
+        q, gate = torch.randn(n_tok, n_head, hd, device="cuda", generator=g), torch.randn(n_tok, n_head, hd, device="cuda", generator=g)
+        out, one = torch.empty_like(q), torch.empty(n_head, hd, device="cuda")
+
+        def chunk(n, to):
+            assert L.q4_hip_qsa_decode_n(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), gate.data_ptr(), to.data_ptr(), n_head, n_kvh, hd, n_tok, n - n_tok, n,
+                                         1.0 / 16.0, 1)
+
+        def scan():
+            assert L.q4_hip_qsa_decode_n(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), gate.data_ptr(), one.data_ptr(), n_head, n_kvh, hd, 1, more - 1, more,
+                                         1.0 / 16.0, 1)
+        chunk(rows, out)
+        scan()
+        want, want_one = out.clone(), one.clone()
+        assert L.q4_hip_graph_begin()
+        chunk(rows, out)
+        scan()
+        graph = L.q4_hip_graph_end()
+        assert graph
+        chunk(more, torch.empty_like(out))    # operand images grow
+        assert L.q4_hip_qsa_topk_alloc()      # scratch grows
+        others = [torch.full((s << 20,), 0xff, dtype=torch.uint8, device="cuda") for s in (1, 2, 4, 8, 16, 32, 64)]
+        out.zero_()
+        one.zero_()
+        for _ in range(3):
+            assert L.q4_hip_graph_launch(graph)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and torch.equal(one, want_one)
+        assert all(bool((o == 0xff).all()) for o in others)
+        assert L.q4_gpu_last_error() == 0
+        del others
+        torch.cuda.empty_cache()
+        before = torch.cuda.mem_get_info()[0]
+        L.q4_hip_graph_free(graph)
+        assert torch.cuda.mem_get_info()[0] > before
+    torch.cuda.synchronize()
