@@ -409,7 +409,9 @@ bool q4_gpu_comm_allgather_merge(q4_gpu_comm *c, const float *part, float *parts
 typedef struct q4_gpu_batch q4_gpu_batch;
 q4_gpu_batch *q4_gpu_batch_create(uint32_t max_sessions);
 void q4_gpu_batch_destroy(q4_gpu_batch *b);
-/* Bind session slot s to a store (all stores of a batch share n_layers, n_kvh, hd and kind). */
+/* Bind session slot s to a store (all stores of a batch share n_layers, n_kvh, hd and kind).  A bound store may be
+ * destroyed (its session has ended) while the batch goes on, as long as its published position is -1: nothing of it is read or
+ * written then, and an append reports the skipped row in the range status.  Bind the slot again before a position >= 0. */
 bool q4_gpu_batch_bind(q4_gpu_batch *b, uint32_t slot, q4_gpu_kv *kv);
 /* Publish the decode positions of sessions [0, n_sessions) (host array of n_sessions int32),
  * stream-ordered like q4_hip_pos_push.  n_sessions may be smaller than the number of bound slots: every

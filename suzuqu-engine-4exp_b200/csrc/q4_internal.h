@@ -30,6 +30,10 @@ struct Q4Cache {
     uint32_t max_kv, pad;
 };
 
+/* Per layer of a store: g_q4.launches when its rows were last written.  Shared by the store and the batches it is bound to:
+ * a batch may outlive a store of a session that has ended. */
+struct Q4Writes { uint32_t refs; uint64_t *at; };
+
 struct q4_gpu_kv {
     uint32_t n_layers, n_kvh, hd, max_kv;
     int kind;
@@ -38,7 +42,7 @@ struct q4_gpu_kv {
     uint32_t rec_bytes;          /* bytes per (kv head, position): q8_0 record, or fp16 / fp32 row */
     Q4Cache view;                /* host copy of the kernel view */
     Q4Cache *d_view;             /* same, in device memory (for batched launches) */
-    uint64_t *written;           /* per layer: g_q4.launches when its rows were last written */
+    Q4Writes *writes;
 };
 
 /* Dense scans of more fp32 rows than this at hd 128 (up to 8 query heads per kv head) load straight into registers, behind an
@@ -84,7 +88,7 @@ inline bool q4i_launched(bool ok) {
     return ok;
 }
 inline bool q4i_settled(uint64_t written) { return g_q4.launches > written && g_q4.launches > g_q4.unsettled; }
-inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->written[layer] = g_q4.launches; }
+inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->writes->at[layer] = g_q4.launches; }
 bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside capture, fails inside */
 void q4i_give_back(void *p, bool captured);              /* cudaFree, now or with the last graph */
 

@@ -335,6 +335,19 @@ extern "C" uint64_t q4_gpu_kv_bytes(uint32_t n_layers, uint32_t n_kvh, uint32_t 
     return (uint64_t)n_layers * max_kv * 2ull * n_kvh * hd * (kind == Q4K_F16 ? 2u : 4u);
 }
 
+static Q4Writes *writes_new(uint32_t n_layers) {
+    Q4Writes *w = (Q4Writes *)calloc(1, sizeof(Q4Writes));
+    if (!w) return nullptr;
+    w->at = (uint64_t *)calloc(n_layers, sizeof(uint64_t));
+    if (!w->at) { free(w); return nullptr; }
+    w->refs = 1;
+    return w;
+}
+static void writes_release(Q4Writes *w) {
+    if (!w || --w->refs) return;
+    free(w->at);
+    free(w);
+}
 extern "C" q4_gpu_kv *q4_gpu_kv_create(uint32_t n_layers, uint32_t n_kvh, uint32_t hd, uint32_t max_kv, int kind) {
     if (!g_q4.ok) { q4i_fail(Q4E_INIT, "kv_create: library not initialised"); return nullptr; }
     if (!n_layers || !n_kvh || !hd_ok(hd) || !max_kv || kind < 0 || kind > 2) {
@@ -343,8 +356,8 @@ extern "C" q4_gpu_kv *q4_gpu_kv_create(uint32_t n_layers, uint32_t n_kvh, uint32
     }
     q4_gpu_kv *kv = (q4_gpu_kv *)calloc(1, sizeof(q4_gpu_kv));
     if (!kv) return nullptr;
-    kv->written = (uint64_t *)calloc(n_layers, sizeof(uint64_t));
-    if (!kv->written) { free(kv); return nullptr; }
+    kv->writes = writes_new(n_layers);
+    if (!kv->writes) { free(kv); return nullptr; }
     for (uint32_t i = 0; i < n_layers; i++) q4i_kv_written(kv, i);
     kv->n_layers = n_layers; kv->n_kvh = n_kvh; kv->hd = hd; kv->max_kv = max_kv; kv->kind = kind;
     /* q8_0: one record per (kv head, position) = K codes | V codes | K scales | V scales, so a gathered
@@ -389,7 +402,7 @@ extern "C" void q4_gpu_kv_destroy(q4_gpu_kv *kv) {
     if (kv->k) cudaFree(kv->k);
     if (kv->v && kv->kind != Q4K_Q8) cudaFree(kv->v);   /* q8_0: v and s point into the k allocation */
     if (kv->d_view) cudaFree(kv->d_view);
-    free(kv->written);
+    writes_release(kv->writes);
     free(kv);
 }
 
@@ -542,7 +555,7 @@ static bool store_decode(const q4_gpu_kv *kv, uint32_t layer, const void *q, int
     a.idx_bound_nkv = 1;
     a.scale = scale;
     a.early_pos = !a.pos || q4i_settled(g_q4.pos_written);
-    a.early_rows = q4i_settled(kv->written[layer]);
+    a.early_rows = q4i_settled(kv->writes->at[layer]);
     return q4i_decode(a);
 }
 extern "C" bool q4_gpu_kv_decode(const q4_gpu_kv *kv, uint32_t layer, const void *q, int q_bf16, const float *gate,
@@ -594,7 +607,9 @@ extern "C" bool q4_gpu_kv_decode_idx_n(const q4_gpu_kv *kv, uint32_t layer, cons
 struct q4_gpu_batch {
     uint32_t max_sessions, n;
     uint32_t n_active;            /* sessions of the latest q4_gpu_batch_set_pos: what every batch launch covers */
-    q4_gpu_kv **kv;
+    uint32_t n_layers, n_kvh, hd; /* of every store in it */
+    int kind;
+    Q4Writes **writes;            /* the bound stores' write counts, null where none is bound; no pointer to a store is kept */
     Q4Cache *d_views;             /* device array of the bound stores' views (one load, no pointer chase) */
     int32_t *pos_d, *pos_h;       /* pos_h: pinned ring of 8 uploads, each slot guarded by an event */
     cudaEvent_t pos_ev[8];
@@ -607,8 +622,8 @@ extern "C" q4_gpu_batch *q4_gpu_batch_create(uint32_t max_sessions) {
     q4_gpu_batch *b = (q4_gpu_batch *)calloc(1, sizeof(q4_gpu_batch));
     if (!b) return nullptr;
     b->max_sessions = max_sessions;
-    b->kv = (q4_gpu_kv **)calloc(max_sessions, sizeof(q4_gpu_kv *));
-    bool ok = b->kv && cudaMalloc(&b->d_views, sizeof(Q4Cache) * max_sessions) == cudaSuccess &&
+    b->writes = (Q4Writes **)calloc(max_sessions, sizeof(Q4Writes *));
+    bool ok = b->writes && cudaMalloc(&b->d_views, sizeof(Q4Cache) * max_sessions) == cudaSuccess &&
               cudaMalloc(&b->pos_d, sizeof(int32_t) * max_sessions) == cudaSuccess &&
               cudaMallocHost(&b->pos_h, sizeof(int32_t) * max_sessions * 8) == cudaSuccess;
     if (ok) ok = cudaMemset(b->pos_d, 0, sizeof(int32_t) * max_sessions) == cudaSuccess;
@@ -630,19 +645,20 @@ extern "C" void q4_gpu_batch_destroy(q4_gpu_batch *b) {
     if (b->pos_h) cudaFreeHost(b->pos_h);
     for (int i = 0; i < 8; i++)
         if (b->pos_ev[i]) cudaEventDestroy(b->pos_ev[i]);
-    free(b->kv);
+    for (uint32_t i = 0; b->writes && i < b->n; i++) writes_release(b->writes[i]);
+    free(b->writes);
     free(b);
 }
 extern "C" bool q4_gpu_batch_bind(q4_gpu_batch *b, uint32_t slot, q4_gpu_kv *kv) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_bind: library not initialised");
     Q4_REQUIRE(b && kv && slot < b->max_sessions && !g_q4.capturing, "batch_bind: bad argument");
-    if (b->n) {
-        const q4_gpu_kv *f = nullptr;
-        for (uint32_t i = 0; i < b->n && !f; i++) f = b->kv[i];
-        if (f) Q4_REQUIRE(f->n_layers == kv->n_layers && f->n_kvh == kv->n_kvh && f->hd == kv->hd && f->kind == kv->kind,
-                          "batch_bind: stores of one batch must share shape and kind");
-    }
-    b->kv[slot] = kv;
+    if (b->n)
+        Q4_REQUIRE(b->n_layers == kv->n_layers && b->n_kvh == kv->n_kvh && b->hd == kv->hd && b->kind == kv->kind,
+                   "batch_bind: stores of one batch must share shape and kind");
+    b->n_layers = kv->n_layers; b->n_kvh = kv->n_kvh; b->hd = kv->hd; b->kind = kv->kind;
+    kv->writes->refs++;
+    writes_release(b->writes[slot]);
+    b->writes[slot] = kv->writes;
     if (slot + 1 > b->n) b->n = slot + 1;
     /* device-to-device from the store's own device copy of its view: no host buffer to keep alive */
     if (!q4i_check(cudaMemcpyAsync(b->d_views + slot, kv->d_view, sizeof(Q4Cache), cudaMemcpyDeviceToDevice, g_q4.stream),
@@ -686,22 +702,22 @@ extern "C" bool q4_gpu_batch_advance(q4_gpu_batch *b, int32_t delta) {
 }
 static void batch_written(q4_gpu_batch *b, uint32_t layer) {
     for (uint32_t i = 0; i < b->n_active; i++)
-        if (b->kv[i]) q4i_kv_written(b->kv[i], layer);
+        if (b->writes[i]) b->writes[i]->at[layer] = g_q4.launches;
 }
 static void batch_early(const q4_gpu_batch *b, uint32_t layer, Q4DecodeArgs &a) {
     a.early_pos = q4i_settled(b->pos_written);
     a.early_rows = 1;
-    for (uint32_t i = 0; i < b->n_active && a.early_rows; i++) a.early_rows = b->kv[i] && q4i_settled(b->kv[i]->written[layer]);
+    for (uint32_t i = 0; i < b->n_active && a.early_rows; i++) a.early_rows = b->writes[i] && q4i_settled(b->writes[i]->at[layer]);
 }
 extern "C" bool q4_gpu_batch_append(q4_gpu_batch *b, uint32_t layer, const float *k, const float *v) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_append: library not initialised");
-    Q4_REQUIRE(b && b->n && k && v && b->kv[0] && layer < b->kv[0]->n_layers, "batch_append: bad argument");
+    Q4_REQUIRE(b && b->n && k && v && b->writes[0] && layer < b->n_layers, "batch_append: bad argument");
     Q4_REQUIRE(b->n_active, "batch_append: no positions published (q4_gpu_batch_set_pos)");
     AppendParams p;
     memset(&p, 0, sizeof(p));
-    p.many = b->d_views; p.layer = layer; p.n_rows = b->n_active; p.n_kvh = b->kv[0]->n_kvh; p.hd = b->kv[0]->hd;
+    p.many = b->d_views; p.layer = layer; p.n_rows = b->n_active; p.n_kvh = b->n_kvh; p.hd = b->hd;
     p.k = k; p.v = v; p.pos = b->pos_d; p.err = g_q4.err_d; p.early = q4i_settled(b->pos_written);
-    const bool ok = launch_append(p, store_layout(b->kv[0]->kind));
+    const bool ok = launch_append(p, store_layout(b->kind));
     batch_written(b, layer);
     return ok;
 }
@@ -709,17 +725,17 @@ extern "C" bool q4_gpu_batch_decode(q4_gpu_batch *b, uint32_t layer, const void 
                                     float *out, const int32_t *idx, uint32_t width, uint32_t idx_kvh_stride,
                                     uint32_t idx_sess_stride, uint32_t n_head, float scale) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_decode: library not initialised");
-    Q4_REQUIRE(b && b->n && q && out && b->kv[0] && layer < b->kv[0]->n_layers && n_head, "batch_decode: bad argument");
+    Q4_REQUIRE(b && b->n && q && out && b->writes[0] && layer < b->n_layers && n_head, "batch_decode: bad argument");
     Q4_REQUIRE(b->n_active, "batch_decode: no positions published (q4_gpu_batch_set_pos)");
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));
     a.many = b->d_views;
-    a.layout = store_layout(b->kv[0]->kind);
+    a.layout = store_layout(b->kind);
     a.layer = layer;
     a.n_units = b->n_active;
     a.n_head = n_head;
-    a.n_kvh = b->kv[0]->n_kvh;
-    a.hd = b->kv[0]->hd;
+    a.n_kvh = b->n_kvh;
+    a.hd = b->hd;
     a.q = q; a.q_bf16 = q_bf16; a.gate = gate; a.out = out;
     a.idx = idx; a.width = width; a.idx_kvh_stride = idx_kvh_stride; a.idx_unit_stride = idx_sess_stride;
     a.pos = b->pos_d;
@@ -736,20 +752,20 @@ extern "C" bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, cons
                                            int q_bf16, const float *gate, float *out, const int32_t *idx, uint32_t width,
                                            uint32_t idx_kvh_stride, uint32_t idx_sess_stride, uint32_t n_head, float scale) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_append_decode: library not initialised");
-    Q4_REQUIRE(b && b->n && k && v && q && out && b->kv[0] && layer < b->kv[0]->n_layers && n_head,
+    Q4_REQUIRE(b && b->n && k && v && q && out && b->writes[0] && layer < b->n_layers && n_head,
                "batch_append_decode: bad argument");
     Q4_REQUIRE(b->n_active, "batch_append_decode: no positions published (q4_gpu_batch_set_pos)");
-    const bool fused = b->kv[0]->hd >= 128;
+    const bool fused = b->hd >= 128;
     if (!fused && !q4_gpu_batch_append(b, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));
     a.many = b->d_views;
-    a.layout = store_layout(b->kv[0]->kind);
+    a.layout = store_layout(b->kind);
     a.layer = layer;
     a.n_units = b->n_active;
     a.n_head = n_head;
-    a.n_kvh = b->kv[0]->n_kvh;
-    a.hd = b->kv[0]->hd;
+    a.n_kvh = b->n_kvh;
+    a.hd = b->hd;
     a.q = q; a.q_bf16 = q_bf16; a.gate = gate; a.out = out;
     a.idx = idx; a.width = width; a.idx_kvh_stride = idx_kvh_stride; a.idx_unit_stride = idx_sess_stride;
     a.pos = b->pos_d;
@@ -787,7 +803,7 @@ extern "C" bool q4_gpu_kv_append_decode_d(q4_gpu_kv *kv, uint32_t layer, const f
     a.scale = scale;
     if (fused) { a.new_k = k; a.new_v = v; }
     a.early_pos = q4i_settled(g_q4.pos_written);
-    a.early_rows = q4i_settled(kv->written[layer]);
+    a.early_rows = q4i_settled(kv->writes->at[layer]);
     const bool ok = q4i_decode(a);
     if (fused) q4i_kv_written(kv, layer);
     return ok;

@@ -264,3 +264,49 @@ def test_pipelined_steps_over_two_buffer_sets():
         L.q4_hip_graph_free(g)
         L.q4_gpu_pipe_destroy(pipe)
     q4gpu.use_torch_stream()
+
+
+@pytest.mark.parametrize("kind,gone", [(2, 1), (1, 0), (0, 2)])
+def test_batch_outlives_the_store_of_a_session_that_has_ended(oracle, kind, gone):
+    """a store is destroyed while its slot is still covered, at position -1: the others go on, and the host memory that the
+    store has left, taken by the next allocations of its sizes, is not written"""
+    L = lib()
+    n_layers, n_kvh, hd, n_head, n = 5, 2, 128, 16, 40
+    kvw = n_kvh * hd
+    libc = ctypes.CDLL(None)
+    libc.calloc.restype = ctypes.c_void_p
+    libc.calloc.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
+    libc.free.argtypes = [ctypes.c_void_p]
+    stores = [q4gpu.KVStore(n_layers, n_kvh, hd, 64, kind) for _ in range(3)]
+    k, v = oracle.normal(31, 0, n * kvw).reshape(n, kvw), oracle.normal(31, 1, n * kvw).reshape(n, kvw)
+    for st in stores:
+        for layer in range(n_layers):
+            st.append(layer, dev(k[:-1]), dev(v[:-1]), 0, n - 1)
+    b = q4gpu.Batch(stores)
+    q = oracle.normal(31, 2, 3 * n_head * hd)
+    nk, nv = np.stack([k[-1]] * 3), np.stack([v[-1]] * 3)
+    pos = [n - 1] * 3
+    pos[gone] = -1
+    torch.cuda.synchronize()
+    stores[gone].close()
+    taken = [libc.calloc(1, 8 * n_layers) for _ in range(8)]
+    out = torch.full((3, n_head, hd), float("nan"), device="cuda")
+    b.set_pos(pos)
+    scale = float(1.0 / np.sqrt(hd))
+    for layer in range(n_layers):
+        b.append_decode(layer, dev(nk), dev(nv), dev(q), out, n_head, scale)
+        b.append(layer, dev(nk), dev(nv))
+        b.decode(layer, dev(q), out, n_head, scale)
+    got = host(out)
+    assert L.q4_gpu_last_error() == 4                # the ended session's rows were not appended
+    assert all(ctypes.string_at(p, 8 * n_layers) == bytes(8 * n_layers) for p in taken)
+    for p in taken:
+        libc.free(p)
+    for s in range(3):
+        if s == gone:
+            assert not got[s].any()
+            continue
+        ref = oracle.attn(q.reshape(3, n_head, hd)[s:s + 1], oracle.kv_write(k, kind), oracle.kv_write(v, kind), None, n_head, n_kvh, hd, 1, n - 1, n,
+                          scale, kind)
+        assert_close(got[s], ref[0], "session %d" % s)
+    b.close()
