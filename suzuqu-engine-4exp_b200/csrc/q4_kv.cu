@@ -610,6 +610,7 @@ struct q4_gpu_batch {
     uint32_t n_layers, n_kvh, hd; /* of every store in it */
     int kind;
     Q4Writes **writes;            /* the bound stores' write counts, null where none is bound; no pointer to a store is kept */
+    int twice;                    /* 1: a store is bound to more than one slot, -1: to be found out */
     Q4Cache *d_views;             /* device array of the bound stores' views (one load, no pointer chase) */
     int32_t *pos_d, *pos_h;       /* pos_h: pinned ring of 8 uploads, each slot guarded by an event */
     cudaEvent_t pos_ev[8];
@@ -659,6 +660,7 @@ extern "C" bool q4_gpu_batch_bind(q4_gpu_batch *b, uint32_t slot, q4_gpu_kv *kv)
     kv->writes->refs++;
     writes_release(b->writes[slot]);
     b->writes[slot] = kv->writes;
+    b->twice = -1;
     if (slot + 1 > b->n) b->n = slot + 1;
     /* device-to-device from the store's own device copy of its view: no host buffer to keep alive */
     if (!q4i_check(cudaMemcpyAsync(b->d_views + slot, kv->d_view, sizeof(Q4Cache), cudaMemcpyDeviceToDevice, g_q4.stream),
@@ -746,8 +748,17 @@ extern "C" bool q4_gpu_batch_decode(q4_gpu_batch *b, uint32_t layer, const void 
     return q4i_decode(a);
 }
 
-/* Append + attend in one call.  On the native q8_0 store this is ONE launch per layer: the attention
- * kernel quantises and stores the newest rows itself; other kinds run the append kernel first. */
+/* Append + attend in one call: at hd 128 and 256 ONE launch per layer, the attention kernel stores the newest rows itself.
+ * Not where a store is bound to several slots (draft tokens of one session): a slot's new row is then another's context, and
+ * the blocks of one launch do not wait for each other's rows. */
+static bool bound_twice(q4_gpu_batch *b) {
+    if (b->twice < 0) {
+        b->twice = 0;
+        for (uint32_t i = 0; i < b->n && !b->twice; i++)
+            for (uint32_t j = 0; j < i && !b->twice; j++) b->twice = b->writes[i] && b->writes[i] == b->writes[j];
+    }
+    return b->twice != 0;
+}
 extern "C" bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, const float *k, const float *v, const void *q,
                                            int q_bf16, const float *gate, float *out, const int32_t *idx, uint32_t width,
                                            uint32_t idx_kvh_stride, uint32_t idx_sess_stride, uint32_t n_head, float scale) {
@@ -755,7 +766,7 @@ extern "C" bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, cons
     Q4_REQUIRE(b && b->n && k && v && q && out && b->writes[0] && layer < b->n_layers && n_head,
                "batch_append_decode: bad argument");
     Q4_REQUIRE(b->n_active, "batch_append_decode: no positions published (q4_gpu_batch_set_pos)");
-    const bool fused = b->hd >= 128;
+    const bool fused = b->hd >= 128 && !bound_twice(b);
     if (!fused && !q4_gpu_batch_append(b, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));

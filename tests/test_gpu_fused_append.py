@@ -125,3 +125,28 @@ def test_position_beyond_the_store_is_reported():
     assert L.q4_gpu_last_error() & 4
     b.close()
     st.close()
+
+
+@pytest.mark.parametrize("kind", [2, 1, 0])
+def test_draft_tokens_of_one_session_see_each_other(oracle, kind):
+    """one store bound to several slots, consecutive positions: every row is in place before any slot attends"""
+    L = lib()
+    n_kvh, hd, n_head, n, drafts = 2, 128, 16, 3000, 6
+    kvw = n_kvh * hd
+    k, v = oracle.normal(91, 0, (n + drafts) * kvw).reshape(-1, kvw), oracle.normal(91, 1, (n + drafts) * kvw).reshape(-1, kvw)
+    st = q4gpu.KVStore(1, n_kvh, hd, n + drafts, kind)
+    st.append(0, dev(k[:n]), dev(v[:n]), 0, n)
+    b = q4gpu.Batch([st] * drafts)
+    q = oracle.normal(91, 2, drafts * n_head * hd).reshape(drafts, n_head, hd)
+    out = torch.empty(drafts, n_head, hd, device="cuda")
+    scale = float(1.0 / np.sqrt(hd))
+    b.set_pos([n + drafts - 1 - i for i in range(drafts)])
+    b.append_decode(0, dev(k[n:][::-1]), dev(v[n:][::-1]), dev(q), out, n_head, scale)
+    got = host(out)
+    kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind)
+    for i in range(drafts):
+        ref = oracle.attn(q[i:i + 1], kc, vc, None, n_head, n_kvh, hd, 1, n + drafts - 1 - i, n + drafts, scale, kind)
+        assert_close(got[i], ref[0], "slot %d" % i)
+    assert L.q4_gpu_last_error() == 0
+    b.close()
+    st.close()
