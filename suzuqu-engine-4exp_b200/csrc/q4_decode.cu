@@ -2238,8 +2238,8 @@ bool launch(const DecParams &p_in, dim3 grid) {
 }
 template <int LAY, int HD, bool LIST>
 bool launch_nht(const DecParams &p, dim3 grid) {
-    if constexpr (HD == 128 && LAY == LAY_F32 && !LIST) {   /* the list a run-time choice: compiled for dense ranges alone it spills */
-        if (p.direct) return launch<LAY, HD, 1, true, true>(p, grid);
+    if constexpr (HD >= 128 && LAY == LAY_F32) {   /* the list a run-time choice: compiled for dense ranges alone it spills */
+        if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true, true>(p, grid) : launch<LAY, HD, 2, true, true>(p, grid);
     }
     if constexpr (HD >= 128 && (LAY == LAY_Q8R || LAY == LAY_F16)) {
         if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true, LIST>(p, grid) : launch<LAY, HD, 2, true, LIST>(p, grid);
@@ -2419,7 +2419,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
                    "decode: fused append needs both rows and a store at hd 128 or 256");
     p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
     /* long scans of fp32 rows at hd 128 as well: Q4_F32_RING_ROWS */
-    if (a.layout == LAY_F32) p.direct = !a.idx && a.hd == 128 && gqa <= 8 && a.n_units == 1 && !a.new_k && rows > Q4_F32_RING_ROWS ? 1u : 0u;
+    if (a.layout == LAY_F32 && !a.idx && a.hd == 128 && gqa <= 8 && a.n_units == 1 && !a.new_k && rows > Q4_F32_RING_ROWS) p.direct = 1u;
     dim3 grid(S, a.n_kvh, a.n_units);
     switch (a.layout) {
     case LAY_F32: return q4i_launched(launch_hd<LAY_F32>(p, grid, a.hd));

@@ -585,3 +585,30 @@ def test_batched_dense_sessions_of_unequal_length_against_the_oracle(oracle, kin
     b.close()
     for st in stores:
         st.close()
+
+
+@pytest.mark.parametrize("kind,off_k,off_v", [(0, 0, 8), (1, 8, 4), (2, 2, 6)])
+@pytest.mark.parametrize("n_head,n_kvh,hd", [(16, 2, 128), (12, 1, 128), (8, 2, 256), (24, 2, 256), (8, 2, 64)])
+def test_reference_abi_caches_of_the_least_alignment(oracle, kind, off_k, off_v, n_head, n_kvh, hd):
+    """caches that start off a 16-byte boundary, as far as every kind has always allowed: dense, and over a list"""
+    L = lib()
+    n, kvw = 400, n_kvh * hd
+    k, v = oracle.normal(71, hd, n * kvw).reshape(n, kvw), oracle.normal(72, hd, n * kvw).reshape(n, kvw)
+    q, g = oracle.normal(73, hd, n_head * hd), oracle.normal(74, hd, n_head * hd)
+    kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind)
+
+    def at(off, a):
+        t = torch.zeros(a.nbytes + 32, dtype=torch.uint8, device="cuda")
+        t[off:off + a.nbytes] = torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1)).cuda()
+        return t, t.data_ptr() + off
+    (tk, pk), (tv, pv) = at(off_k, kc), at(off_v, vc)
+    out = torch.empty(n_head * hd, device="cuda")
+    scale = float(1.0 / np.sqrt(hd))
+    assert L.q4_hip_qsa_decode(dev(q).data_ptr(), pk, pv, dev(g).data_ptr(), out.data_ptr(), n_head, n_kvh, hd, n, n, scale, kind)
+    ref = oracle.attn(q.reshape(1, n_head, hd), kc, vc, g, n_head, n_kvh, hd, 1, n - 1, n, scale, kind)
+    assert_close(host(out).reshape(ref[0].shape), ref[0], "dense")
+    idx = np.sort(np.random.default_rng(5).permutation(n)[:99]).astype(np.int32)
+    assert L.q4_hip_qsa_decode_idx(dev(q).data_ptr(), pk, pv, dev(g).data_ptr(), out.data_ptr(), dev(idx).data_ptr(), 99, n_head, n_kvh, hd, 1, n, scale, kind)
+    ref = oracle.attn(q.reshape(1, n_head, hd), kc, vc, g, n_head, n_kvh, hd, 1, 0, n, scale, kind, idx=idx, width=99)
+    assert_close(host(out).reshape(ref[0].shape), ref[0], "list")
+    assert L.q4_gpu_last_error() == 0
