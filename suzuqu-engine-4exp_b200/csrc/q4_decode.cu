@@ -2418,8 +2418,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         Q4_REQUIRE(a.new_k && a.new_v && a.layout != LAY_Q8R && a.hd >= 128,
                    "decode: fused append needs both rows and a store at hd 128 or 256");
     p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
-    /* long scans of fp32 rows at hd 128 as well: Q4_F32_RING_ROWS */
-    if (a.layout == LAY_F32 && !a.idx && a.hd == 128 && gqa <= 8 && a.n_units == 1 && !a.new_k && rows > Q4_F32_RING_ROWS) p.direct = 1u;
+    if (!a.new_k && q4i_f32_direct(a.layout == LAY_F32 ? Q4K_F32 : -1, a.hd, a.n_head, a.n_kvh, a.n_units, rows)) p.direct = 1u;
     dim3 grid(S, a.n_kvh, a.n_units);
     switch (a.layout) {
     case LAY_F32: return q4i_launched(launch_hd<LAY_F32>(p, grid, a.hd));

@@ -45,10 +45,17 @@ struct q4_gpu_kv {
     Q4Writes *writes;
 };
 
-/* Dense scans of more fp32 rows than this at hd 128 (up to 8 query heads per kv head) load straight into registers, behind an
- * append of its own: through the ring every byte crosses the load/store pipe twice, which holds 536 MB at 5.2 TB/s
- * (262144 rows 102.9 -> 83.8 us, 65536 37.2 -> 26.5; 16384 rows take 11.7 us through the ring, 15.7 without). */
-constexpr uint32_t Q4_F32_RING_ROWS = 24576;
+/* fp32 rows at hd 128 come through rings in shared memory while the launch is bound by latency, and straight into registers,
+ * behind an append of its own, beyond this many rows of all units and kv heads together: through the ring every byte crosses
+ * the load/store pipe twice.  us per launch, ring / registers, 2 kv heads: one unit of 24 576 rows 17.5 / 18.1, of 32 768
+ * 21.7 / 19.2, of 262 144 103.7 / 85.7; 8 lists of 2051 11.8 / 14.0, 32 33.7 / 30.9; 8 sessions of 24 000 rows 90.5 / 74.
+ * With more than 8 query heads per kv head the ring holds out longer, for one unit always (262 144 rows 103.7 / 123.0;
+ * 4 sessions of 32 768 59.5 / 74.5, 8 of 24 000 122.3 / 79.8, 512 lists 353 / 315). */
+constexpr uint64_t Q4_F32_RING_ROWS = 49152, Q4_F32_RING_ROWS_WIDE = 327680;
+inline bool q4i_f32_direct(int kind, uint32_t hd, uint32_t n_head, uint32_t n_kvh, uint64_t units, uint32_t rows) {
+    if (kind != Q4K_F32 || hd != 128) return false;
+    return units * n_kvh * rows > Q4_F32_RING_ROWS && (n_head <= 8u * n_kvh || (units > 1 && units * n_kvh * rows > Q4_F32_RING_ROWS_WIDE));
+}
 
 struct Q4PtrList { void **p; uint32_t n; };
 

@@ -766,7 +766,7 @@ extern "C" bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, cons
     Q4_REQUIRE(b && b->n && k && v && q && out && b->writes[0] && layer < b->n_layers && n_head,
                "batch_append_decode: bad argument");
     Q4_REQUIRE(b->n_active, "batch_append_decode: no positions published (q4_gpu_batch_set_pos)");
-    const bool fused = b->hd >= 128 && !bound_twice(b);
+    const bool fused = b->hd >= 128 && !bound_twice(b) && !q4i_f32_direct(b->kind, b->hd, n_head, b->n_kvh, b->n_active, idx ? width : b->max_pos + 1u);
     if (!fused && !q4_gpu_batch_append(b, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));
@@ -795,7 +795,7 @@ extern "C" bool q4_gpu_kv_append_decode_d(q4_gpu_kv *kv, uint32_t layer, const f
                                           uint32_t width, uint32_t idx_kvh_stride, float scale) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "kv_append_decode_d: library not initialised");
     Q4_REQUIRE(kv && k && v && q && out && layer < kv->n_layers && n_head, "kv_append_decode_d: bad argument");
-    const bool fused = kv->hd >= 128 && (idx || kv->kind != Q4K_F32 || kv->hd != 128 || n_head > 8u * kv->n_kvh || kv->max_kv <= Q4_F32_RING_ROWS);
+    const bool fused = kv->hd >= 128 && !q4i_f32_direct(kv->kind, kv->hd, n_head, kv->n_kvh, 1, idx ? width : kv->max_kv);
     if (!fused && !q4_gpu_kv_append_d(kv, layer, k, v)) return false;
     Q4DecodeArgs a;
     memset(&a, 0, sizeof(a));

@@ -612,3 +612,44 @@ def test_reference_abi_caches_of_the_least_alignment(oracle, kind, off_k, off_v,
     ref = oracle.attn(q.reshape(1, n_head, hd), kc, vc, g, n_head, n_kvh, hd, 1, 0, n, scale, kind, idx=idx, width=99)
     assert_close(host(out).reshape(ref[0].shape), ref[0], "list")
     assert L.q4_gpu_last_error() == 0
+
+
+@pytest.mark.parametrize("n_head,n_kvh,sessions,rows", [(16, 2, 3, 8192), (16, 2, 3, 8193), (16, 2, 24, 1024), (16, 2, 25, 1024), (32, 2, 20, 8192), (32, 2, 21, 8192)])
+def test_batches_of_fp32_stores_on_both_sides_of_the_ring(oracle, n_head, n_kvh, sessions, rows):
+    """append + dense scan, and lists, of several fp32 sessions: through the rings, and straight into registers behind an append
+    (more than 49152 rows of all units and kv heads; 327680 with 16 heads per kv head)"""
+    L = lib()
+    hd = 128
+    kvw = n_kvh * hd
+    k, v = oracle.normal(81, rows, rows * kvw).reshape(rows, kvw), oracle.normal(82, rows, rows * kvw).reshape(rows, kvw)
+    ctx = [rows if i < 2 else 5 + 37 * i for i in range(sessions)]
+    dk, dv = dev(k), dev(v)
+    stores = [q4gpu.KVStore(1, n_kvh, hd, c, 0) for c in ctx]
+    for st, c in zip(stores, ctx):
+        if c > 1:
+            st.append(0, dk[:c - 1], dv[:c - 1], 0, c - 1)
+    b = q4gpu.Batch(stores)
+    b.set_pos([c - 1 for c in ctx])
+    last = torch.tensor([c - 1 for c in ctx], device="cuda")
+    q = oracle.normal(83, 0, sessions * n_head * hd).reshape(sessions, n_head, hd)
+    out = torch.empty(sessions, n_head, hd, device="cuda")
+    scale = float(1.0 / np.sqrt(hd))
+    b.append_decode(0, dk[last].contiguous(), dv[last].contiguous(), dev(q), out, n_head, scale)
+    got = host(out).copy()
+    width = 2051
+    idx = np.full((sessions, width), -1, np.int32)
+    for i, c in enumerate(ctx):
+        pick = np.sort(np.random.default_rng(i).permutation(c)[:width])
+        idx[i, :len(pick)] = pick
+    b.append_decode(0, dk[last].contiguous(), dv[last].contiguous(), dev(q), out, n_head, scale, idx=dev(idx), width=width, idx_sess_stride=width)
+    lst = host(out)
+    for i in (0, 1, 2, sessions - 1):
+        c = ctx[i]
+        ref = oracle.attn(q[i:i + 1], k[:c], v[:c], None, n_head, n_kvh, hd, 1, c - 1, c, scale, 0, threads=8)
+        assert_close(got[i], ref[0], "dense, session %d" % i)
+        ref = oracle.attn(q[i:i + 1], k[:c], v[:c], None, n_head, n_kvh, hd, 1, 0, c, scale, 0, idx=idx[i], width=width, threads=8)
+        assert_close(lst[i], ref[0], "list, session %d" % i)
+    assert L.q4_gpu_last_error() == 0
+    b.close()
+    for st in stores:
+        st.close()
