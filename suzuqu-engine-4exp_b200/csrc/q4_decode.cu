@@ -2284,14 +2284,15 @@ bool q4i_decode(const Q4DecodeArgs &a) {
     const uint32_t units = a.n_units * a.n_kvh;
     uint32_t S = split_override();
     if (!S) {
-        /* one wave of 3 resident blocks per SM */
-        const uint32_t target = (uint32_t)g_q4.sm_count * 3u;
+        /* one wave of 3 resident blocks per SM; 2 where records of hd 128 are read for more than 8 heads (a wave and a half
+         * merges in two levels and ends late: 32768 rows of q8_0, 32 / 2 heads 23.4 us against 11.9) */
+        const uint32_t target = (uint32_t)g_q4.sm_count * (a.layout == LAY_Q8P && a.hd == 128 && gqa > 8 ? 2u : 3u);
         S = target / units;
         /* several units of unequal length (dense batch): finer slices so the block scheduler can balance */
         if (!a.idx && a.n_units > 1) S = S > (steps + 63u) / 64u ? S : (steps + 63u) / 64u;
         /* every warp keeps at least one tile of a list, four of a dense scan (measured at 16384 / 32768 rows:
          * 12.0 / 14.6 us per layer against 13.5 / 15.4 with one tile per warp; no difference from 49152 rows on) */
-        const uint32_t per_block = (a.idx || a.xchg) ? DEC_WARPS : (gqa > 8 ? 2u : 4u) * DEC_WARPS;   /* the exchange form merges in two levels: finer splits serve it better (8 ranks x 32768 rows: 24.7 against 26.0 us) */
+        const uint32_t per_block = (a.idx || a.xchg) ? DEC_WARPS : (gqa > 8 && steps > 4u * DEC_WARPS ? 2u : 4u) * DEC_WARPS;   /* the exchange form merges in two levels: finer splits serve it better (8 ranks x 32768 rows: 24.7 against 26.0 us) */
         const uint32_t cap = (steps + per_block - 1u) / per_block;
         if (S > cap) S = cap;
     }

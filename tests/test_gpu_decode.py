@@ -653,3 +653,11 @@ def test_batches_of_fp32_stores_on_both_sides_of_the_ring(oracle, n_head, n_kvh,
     b.close()
     for st in stores:
         st.close()
+
+
+@pytest.mark.parametrize("kind", [2, 1])
+@pytest.mark.parametrize("max_kv,rows", [(256, [1, 64, 256]), (257, [257]), (20000, [1, 2047, 2560, 19999]), (40009, [300, 33000, 40009])])
+def test_dense_scans_with_sixteen_heads_per_kv_head(oracle, kind, max_kv, rows):
+    """two resident blocks per SM for q8_0 records (one wave of them), two warps to a tile for the others; a short store is one
+    block's"""
+    test_dense_at_the_position_word_in_larger_stores(oracle, kind, 32, 128, max_kv, rows)
