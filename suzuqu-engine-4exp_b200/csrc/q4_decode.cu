@@ -2292,7 +2292,7 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         if (!a.idx && a.n_units > 1) S = S > (steps + 63u) / 64u ? S : (steps + 63u) / 64u;
         /* every warp keeps at least one tile of a list, four of a dense scan (measured at 16384 / 32768 rows:
          * 12.0 / 14.6 us per layer against 13.5 / 15.4 with one tile per warp; no difference from 49152 rows on) */
-        const uint32_t per_block = (a.idx || a.xchg) ? DEC_WARPS : (gqa > 8 && steps > 4u * DEC_WARPS ? 2u : 4u) * DEC_WARPS;   /* the exchange form merges in two levels: finer splits serve it better (8 ranks x 32768 rows: 24.7 against 26.0 us) */
+        const uint32_t per_block = (a.idx || a.xchg) ? DEC_WARPS : (gqa > 8 && (steps > 4u * DEC_WARPS || a.layout != LAY_Q8P || a.hd != 128) ? 2u : 4u) * DEC_WARPS;   /* the exchange form merges in two levels: finer splits serve it better (8 ranks x 32768 rows: 24.7 against 26.0 us) */
         const uint32_t cap = (steps + per_block - 1u) / per_block;
         if (S > cap) S = cap;
     }
@@ -2390,17 +2390,22 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         if (gm < 0) { const char *e = getenv("Q4_DEC_GRIDMERGE"); gm = e ? atoi(e) : 1; }
         p.gridmerge = (gm && !cluster && S > DEC_GROUP && !a.xchg) ? 1u : 0u;
     }
-    /* Up to 131072 rows two blocks per SM do better than three: the next launch's blocks find room and fill their rings
-     * under this one's tail (65536 / 100003 / 262144 rows of q8_0: 15.6 / 19.9 / 37.8 against 17.2 / 20.6 / 33.5 us).
-     * With two warps to a tile (more than 8 heads) three blocks are always better. */
-    p.mid_steps = gqa > 8 || a.layout == LAY_F32 ? 0u : 8192u;   /* fp32 tiles leave no second stage: all blocks (65536 rows 37.0 -> 33.2) */
+    /* A step's dense scan of one session, up to 65536 rows of q8_0 or 49152 of fp16: two blocks per SM do better than three, the
+     * next launch's blocks find room and fill their rings under this one's tail (append + scan of 16384 rows in a store of 65536
+     * 11.3 -> 10.5 us in q8_0, 10.4 -> 9.5 in fp16; 65536 rows 17.5 -> 17.1, but 19.4 -> 20.2 in fp16; 80000 rows 18.3 -> 18.9 in
+     * q8_0, 120000 21.7 -> 23.5).  Not where two warps share a tile (more than 8 heads), not for several sessions (3 of 65536
+     * rows 26.3 -> 32.7), not at head sizes without a ring (64: 65536 rows 13.7 -> 15.3), not where the host gives the row count,
+     * as for partial results (65536 rows 13.9 -> 14.8, fp16 14.4 -> 16.4); fp32 tiles leave no second stage (33.2 -> 37.0). */
+    p.mid_steps = gqa > 8 || a.layout == LAY_F32 || a.n_units > 1 || a.hd < 128 || !a.pos ? 0u : a.layout == LAY_F16 ? 3073u : 4097u;
     p.mid_splits = (uint32_t)g_q4.sm_count * 2u / units;
     if (p.mid_splits > S) p.mid_splits = S;
     if (p.mid_splits < 1u) p.mid_splits = 1u;
     /* Where the launch is sized for a capacity and the context may be short, a grid merge's blocks come in clusters of 8, of
      * which a short context uses the first alone, merging through distributed shared memory (777 rows in a store of 32768:
-     * 5.4 against 7.0 us).  Long scans lose 3 to 6 % by it (the next launch's blocks come in eight at a time), so large
-     * stores do without. */
+     * 5.4 against 7.0 us; 512 rows in one of 262144 5.3 against 7.5).  Long scans lose 3 to 10 % by it, the next launch's blocks
+     * come in eight at a time (16384 rows in a store of 65536 10.5 -> 10.9 us, of 262144 10.5 -> 11.1; 131072 rows at hd 64
+     * 19.3 -> 20.6, 262144 at hd 128 33.2 -> 35.5): a store opened for more than 32768 rows is taken to be filled beyond the
+     * few thousand to which the first cluster gains. */
     p.hybrid = p.gridmerge && use_cluster && a.pos && !a.scratch_part && steps <= 2048u ? 8u : 0u;
     p.xchg = a.xchg;
     p.xchg_phase = (uint32_t)a.xchg_phase;
