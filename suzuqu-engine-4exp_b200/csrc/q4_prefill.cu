@@ -9,8 +9,11 @@
  *
  *  1. q4_pf_stage_k turns the rows the chunk can see, once, into fp16 operand tiles: 32 KB images of 128 K rows x 128
  *     dims and of V^T, already in the 128-byte-swizzled K-major layout that the tensor core reads, so that a tile
- *     comes in with one plain bulk copy (no tensor maps).  The q8_0 caches of the reference ABI get K as two images,
- *     fp16(code * scale) and the rest, which together are exact: that entry point always multiplied exact codes.
+ *     comes in with one plain bulk copy (no tensor maps).  The q8_0 caches of the reference ABI get two images of both,
+ *     fp16(code * scale) and the rest, which together are exact: that entry point always multiplied exact codes.  (A code
+ *     times its scale is a multiple of 2^-24, like the scale: the rest is one too and has 8 bits at most.)  With one image
+ *     of V the outputs' error against 64 bits was 13 to 24 % above that of the decode form, six times on a token that
+ *     attends one row; the second costs the 2048-token prompt of the reference's host 2340 -> 2755 us.
  *  2. q4_prefill_k: one block = one kv head x NQ groups of query tokens whose (token, head) pairs fill the 128 rows
  *     of the MMA each (NQ = 2: 32 tokens x 8 heads at the benchmark shape), against 128-position tiles.
  *
@@ -198,8 +201,8 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 
-/* ---- staging: rows [0, n) of (layer, kv head) -> operand images.  Per tile of 128 positions: KP * HD / 128 images of
- * K (128 rows x 128 dims: two blocks of 64 dims, rows of 128 bytes), then HD / 128 images' worth of V^T (two blocks of
+/* ---- staging: rows [0, n) of (layer, kv head) -> operand images.  Per tile of 128 positions: NP * HD / 128 images of
+ * K (128 rows x 128 dims: two blocks of 64 dims, rows of 128 bytes) and as many images' worth of V^T (two blocks of
  * 64 positions x HD dims).  Rows behind n are zero.  Block = 32 positions of one kv head, K or V (blockIdx.z); V goes
  * through shared memory to come out position-contiguous.  Short and bound by latency, hence the small blocks: 64
  * positions of K and V per block took 12.8 us for 2048 rows of hd 256, 2 kv heads. */
@@ -235,11 +238,11 @@ __device__ __forceinline__ void load8(const uint8_t *row, const uint8_t *srow, u
         for (int i = 0; i < 8; i++) x[i] = (float)(int8_t)(u[i >> 2] >> (8 * (i & 3))) * s;   /* 8 + 11 bits: exact */
     }
 }
-template <int LAY, int HD, int KP>
+template <int LAY, int HD, int NP>
 __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
     constexpr uint32_t PITCH = 34;   /* halves per dim row of the transposition tile (odd word count) */
-    constexpr uint32_t CK = KP * HD / 128, CV = HD / 128, PER = HD * 32u / 8u / 256u;   /* groups of 8 dims per thread */
-    __shared__ __half tile[HD * PITCH];
+    constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128, PER = HD * 32u / 8u / 256u;   /* groups of 8 dims per thread */
+    __shared__ __half tile[NP][HD * PITCH];
     const uint32_t kh = blockIdx.y, p0 = blockIdx.x * 32u, tid = threadIdx.x;
     q4d_pdl_wait();
     const uint8_t *sc = LAY == LAY_Q8P ? C.s + (uint64_t)layer * C.s_layer_stride + (uint64_t)kh * C.s_kvh_stride : nullptr;
@@ -267,12 +270,14 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
                 lo[j] = __floats2half2_rn(x[it][2 * j] - f.x, x[it][2 * j + 1] - f.y);
             }
             *reinterpret_cast<uint4 *>(dst) = make_uint4(h2u(hi[0]), h2u(hi[1]), h2u(hi[2]), h2u(hi[3]));
-            if (KP == 2) *reinterpret_cast<uint4 *>(dst + (HD / 128) * PF_CHUNK) = make_uint4(h2u(lo[0]), h2u(lo[1]), h2u(lo[2]), h2u(lo[3]));
+            if (NP == 2) *reinterpret_cast<uint4 *>(dst + (HD / 128) * PF_CHUNK) = make_uint4(h2u(lo[0]), h2u(lo[1]), h2u(lo[2]), h2u(lo[3]));
         }
         return;
     }
     const uint8_t *vq = C.v + base;
-    uint8_t *vt = vimg + ((size_t)kh * tiles + p0 / PF_BN) * CV * PF_CHUNK + ((p0 / 64u) & 1u) * (HD * 128u);
+    /* a tile's images in the order of their use: hd 256 {value, rest} of its first 64 positions, then of the others; hd 128
+     * value, rest, both halves in each */
+    uint8_t *vt = vimg + ((size_t)kh * tiles + p0 / PF_BN) * CV * PF_CHUNK + ((p0 / 64u) & 1u) * (HD * 128u) * (HD == 256 ? NP : 1);
 #pragma unroll
     for (uint32_t it = 0; it < PER; it++) {   /* lanes on consecutive rows: the 2-byte stores below do not conflict */
         const uint32_t i = tid + 256u * it, p = p0 + (i & 31u), c = i >> 5;
@@ -284,15 +289,21 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
     for (uint32_t it = 0; it < PER; it++) {
         const uint32_t i = tid + 256u * it;
 #pragma unroll
-        for (int j = 0; j < 8; j++) tile[((i >> 5) * 8u + j) * PITCH + (i & 31u)] = __float2half_rn(x[it][j]);
+        for (int j = 0; j < 8; j++) {
+            const __half h = __float2half_rn(x[it][j]);
+            tile[0][((i >> 5) * 8u + j) * PITCH + (i & 31u)] = h;
+            if (NP == 2) tile[NP - 1][((i >> 5) * 8u + j) * PITCH + (i & 31u)] = __float2half_rn(x[it][j] - __half2float(h));
+        }
     }
     __syncthreads();
 #pragma unroll
-    for (uint32_t it = 0; it < PER; it++) {
-        const uint32_t i = tid + 256u * it, d = i >> 2, c = (p0 & 63u) / 8u + (i & 3u);
-        const uint32_t *w = reinterpret_cast<const uint32_t *>(tile + d * PITCH + (i & 3u) * 8u);
-        *reinterpret_cast<uint4 *>(vt + d * 128u + ((c ^ (d & 7u)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+    for (int im = 0; im < NP; im++)
+#pragma unroll
+        for (uint32_t it = 0; it < PER; it++) {
+            const uint32_t i = tid + 256u * it, d = i >> 2, c = (p0 & 63u) / 8u + (i & 3u);
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(tile[im] + d * PITCH + (i & 3u) * 8u);
+            *reinterpret_cast<uint4 *>(vt + im * PF_CHUNK + d * 128u + ((c ^ (d & 7u)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
 }
 
 /* the rest of a wait whose first test found the phase incomplete: at most two seconds from the block's start, and no
@@ -310,10 +321,11 @@ __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_a
     asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(1u) : "memory");
     return false;
 }
-/* HD: head size; NQ: query groups per block; KP: images per 128 dims of K (2: value and remainder) */
-template <int HD, int NQ, int KP>
+/* HD: head size; NQ: query groups per block; NP: images per 128 dims of K and V (2: value and remainder) */
+template <int HD, int NQ, int NP>
 __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParams P) {
-    constexpr uint32_t CK = KP * HD / 128, CV = HD / 128;      /* ring slots a K / V tile takes */
+    constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128;   /* ring slots a K / V tile takes */
+    static_assert(NQ == 1 || NP == 1, "two groups hold a tile's V and the next one's K at once: both images of them leave the ring no slack");
     constexpr uint32_t SW = 8;                                 /* softmax warps; then the issuer, then the producer */
     constexpr uint32_t O_COL = 256, TMEM_COLS = 512;           /* scores in the first 256 columns, O of group g at 256 + 128 g */
     constexpr uint32_t UN = NQ == 2 ? 64 : 128, SB = 2 * NQ;   /* positions of a unit, score buffers */
@@ -534,15 +546,22 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
                 issue_qk(0);
                 if (ok && n_tiles > 1) issue_qk(1);
                 for (uint32_t j = 0; j < n_tiles && ok; j++) {
-                    uint32_t s = 0;
+                    uint32_t sv[NP];
 #pragma unroll
                     for (uint32_t h = 0; h < 2; h++) {   /* 64 positions each; the operands land while the softmax runs */
-                        if (CV == 2 || h == 0) s = take();
+                        if (HD == 256 || h == 0) {
+#pragma unroll
+                            for (int im = 0; im < NP; im++) sv[im] = take();
+                        }
                         if (h == 0) ok = ok && all_wait(bar_p + 8 * (j & 1u), (j >> 1) & 1u);
                         tc_fence_after();
                         if (!ok) break;
-                        pv_half((j & 1u) * 128u + h * 64u, 0u, s, CV == 2 ? 0u : h * (HD * 128u), j == 0 && h == 0);
-                        if (CV == 2 || h == 1) umma_commit(el, empty + 8 * s);
+#pragma unroll
+                        for (int im = 0; im < NP; im++) pv_half((j & 1u) * 128u + h * 64u, 0u, sv[im], HD == 256 ? 0u : h * (HD * 128u), j == 0 && h == 0 && im == 0);
+                        if (HD == 256 || h == 1) {
+#pragma unroll
+                            for (int im = 0; im < NP; im++) umma_commit(el, empty + 8 * sv[im]);
+                        }
                     }
                     if (ok) {
                         umma_commit(el, bar_o);
@@ -824,26 +843,26 @@ int stage_reserve(size_t bytes) {
     return -1;
 }
 
-template <int HD, int NQ, int KP>
+template <int HD, int NQ, int NP>
 bool attend(const PrefillParams &p, dim3 grid) {
     static bool attr = false;
-    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
+    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
                             "prefill smem attribute"))
         return false;
     attr = true;
-    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, KP>, grid, PF_THREADS, PF_SMEM, p);
+    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP>, grid, PF_THREADS, PF_SMEM, p);
 }
-template <int LAY, int HD, int KP>
+template <int LAY, int HD, int NP>
 bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
-    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, KP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
+    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, NP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
 }
 
 /* Ranges of positions that a chunk's blocks of one query group are split into: the count with the least estimated time,
  * waves x (tiles of a range + what a block takes besides) + the merge with its traffic.  In ns, from chunks of 33 to 1500
- * tokens over 0 to 16 384: a tile 1.0 us at hd 128, 1.8 at 256 with both images of K; a block 4 and 6 us besides; the merge
+ * tokens over 0 to 16 384: a tile 1.0 us at hd 128, 2.2 at 256 with both images; a block 4 and 6 us besides; the merge
  * 1.2 us, 0.2 per range, and 7 KB per ns.  600 tokens over 16 384 (76 blocks): 146 us in one range, 112 in three. */
-uint32_t best_split(uint32_t blocks, uint32_t sms, uint32_t tiles, uint64_t rows, uint32_t hd, uint32_t kp) {
-    const uint64_t tile = 640u + 190u * (hd / 128u) * (kp + 1u), block = 2000u + 2000u * (hd / 128u);
+uint32_t best_split(uint32_t blocks, uint32_t sms, uint32_t tiles, uint64_t rows, uint32_t hd, uint32_t np) {
+    const uint64_t tile = 640u + 190u * (hd / 128u) * 2u * np, block = 2000u + 2000u * (hd / 128u);
     uint64_t best = 0;
     uint32_t split = 1;
     for (uint32_t s = 1; s <= 16u && s <= tiles; s++) {
@@ -871,16 +890,16 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     const uint32_t gqa = a.n_head / a.n_kvh, hd = a.hd;
     const uint64_t n64 = (uint64_t)a.kv_base + a.n_tok;
     const uint32_t n = (uint32_t)(n64 < a.cache.max_kv ? n64 : a.cache.max_kv), tiles = (n + PF_BN - 1u) / PF_BN;
-    /* codes times scales do not fit fp16: the exact form keeps what the first image leaves over */
-    const uint32_t kp = a.layout == LAY_Q8R ? 2u : 1u;
+    /* a code times its scale has 19 bits: the reference ABI's q8_0 caches keep what the first image leaves over */
+    const uint32_t np = a.layout == LAY_Q8R ? 2u : 1u;
     const uint32_t tpc = PF_ROWS / gqa, groups = (a.n_tok + tpc - 1u) / tpc, sms = (uint32_t)g_q4.sm_count;
     /* Two groups per block share every K/V tile and hide one another's softmax; one group per block while that takes few
      * waves: 1000 tokens over 4000 (126 blocks) 52 against 83 us, 2500 over 16 384 (314) 450 against 505, 3600 (450) 643
      * against 591; between 300 and 400 it depends on the depth. */
-    const uint32_t nq = hd == 128 && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
+    const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
     const uint32_t blocks = (groups + nq - 1u) / nq * a.n_kvh;
-    uint32_t split = nq == 1 ? best_split(blocks, sms, tiles, (uint64_t)a.n_tok * a.n_head, hd, kp) : 1u;
-    const size_t k_bytes = (size_t)a.n_kvh * tiles * kp * (hd / 128u) * PF_CHUNK, v_bytes = (size_t)a.n_kvh * tiles * (hd / 128u) * PF_CHUNK;
+    uint32_t split = nq == 1 ? best_split(blocks, sms, tiles, (uint64_t)a.n_tok * a.n_head, hd, np) : 1u;
+    const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes;
     const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
     const int room = stage_reserve(k_bytes + v_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0));
     if (room != 1) return room;
@@ -905,9 +924,9 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, kimg, vimg) : stage<LAY_F32, 256, 1>(a, n, tiles, kimg, vimg);
     if (!ok) return 0;
     const dim3 grid((groups + nq - 1u) / nq, a.n_kvh, split);
-    if (hd == 256) ok = kp == 2 ? attend<256, 1, 2>(p, grid) : attend<256, 1, 1>(p, grid);
-    else if (nq == 2) ok = kp == 2 ? attend<128, 2, 2>(p, grid) : attend<128, 2, 1>(p, grid);
-    else ok = kp == 2 ? attend<128, 1, 2>(p, grid) : attend<128, 1, 1>(p, grid);
+    if (hd == 256) ok = np == 2 ? attend<256, 1, 2>(p, grid) : attend<256, 1, 1>(p, grid);
+    else if (nq == 2) ok = attend<128, 2, 1>(p, grid);
+    else ok = np == 2 ? attend<128, 1, 2>(p, grid) : attend<128, 1, 1>(p, grid);
     if (ok && split > 1) {
         const uint64_t total4 = (uint64_t)rows * hd / 4u;
         ok = q4i_launch_pdl("prefill launch", q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4);

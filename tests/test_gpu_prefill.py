@@ -292,3 +292,28 @@ def test_captured_chunk_keeps_its_workspace_when_that_grows():
         L.q4_hip_graph_free(graph)
         assert torch.cuda.mem_get_info()[0] > before
     torch.cuda.synchronize()
+
+
+def run_chunk(L, q, kc, vc, gate, n_head, n_kvh, hd, kv_base, max_kv, scale, kind):
+    from gpu_util import dev_bytes
+    n_tok = q.shape[0]
+    out = torch.full((n_tok, n_head, hd), float("nan"), device="cuda")
+    assert L.q4_hip_qsa_decode_n(dev(q).data_ptr(), dev_bytes(kc).data_ptr(), dev_bytes(vc).data_ptr(), dev(gate).data_ptr(), out.data_ptr(), n_head, n_kvh,
+                                 hd, n_tok, kv_base, max_kv, scale, kind)
+    return host(out)
+
+
+@pytest.mark.parametrize("n_head,n_kvh,hd", [(24, 2, 256), (16, 2, 128)])
+def test_first_token_of_a_reference_abi_chunk_is_its_value_row(oracle, n_head, n_kvh, hd):
+    """a token that attends one row has weight 1 and gets codes x scales x sigmoid(gate) with no rounding to 16 bits: what is
+    left is the gate's (2^-20); the values have 19 bits, a single fp16 image of them would be off by 2^-12"""
+    L = lib()
+    n, kvw = 128, n_kvh * hd          # 128 tokens: on the tensor cores in every rule
+    k, v = oracle.normal(41, 0, n * kvw).reshape(n, kvw), oracle.normal(41, 1, n * kvw).reshape(n, kvw)
+    q, g = oracle.normal(41, 2, n * n_head * hd).reshape(n, n_head, hd), oracle.normal(41, 3, n * n_head * hd).reshape(n, n_head, hd)
+    kc, vc = oracle.kv_write(k, 2), oracle.kv_write(v, 2)
+    got = run_chunk(L, q, kc, vc, g, n_head, n_kvh, hd, 0, n, float(1.0 / np.sqrt(hd)), 2)[0].astype(np.float64)
+    blocks = vc.reshape(n, n_kvh, hd // 32, 34)[0]
+    rows = blocks[..., 2:].copy().view(np.int8).astype(np.float64) * blocks[..., :2].copy().view(np.float16).astype(np.float64)
+    want = np.repeat(rows.reshape(n_kvh, hd), n_head // n_kvh, 0) / (1.0 + np.exp(-g[0].astype(np.float64)))
+    assert (np.abs(got - want) <= 4e-6 * np.abs(want)).all(), np.abs(got / want - 1)[want != 0].max()
