@@ -59,6 +59,8 @@ constexpr uint32_t PF_SPIN_LIMIT = 1u << 22;
 constexpr unsigned long long PF_LIMIT_NS = 2000000000ull;   /* a block that has not finished by then gives up */
 constexpr float PF_RESCALE_TAU = 8.f;
 
+struct __align__(16) PfMark { float k, v; uint32_t bad_rows, pad; };   /* factors of 32 staged rows, V rows that are not finite */
+
 struct PrefillParams {
     uint32_t n_head, n_kvh, gqa, tpc /* tokens per query group */;
     const void *q;           /* [n_tok][n_head][hd] */
@@ -72,6 +74,7 @@ struct PrefillParams {
     uint32_t n_split;             /* position ranges of equal tile count; > 1: partial results */
     float *part;                  /* [split][token][head][hd] unnormalised O */
     float2 *part_ml;              /* [split][token][head] running max (log2 units), sum */
+    const PfMark *marks;          /* [kv head][32 positions], of caches that are not the library's */
     uint32_t *err;
 };
 
@@ -238,16 +241,37 @@ __device__ __forceinline__ void load8(const uint8_t *row, const uint8_t *srow, u
         for (int i = 0; i < 8; i++) x[i] = (float)(int8_t)(u[i >> 2] >> (8 * (i & 3))) * s;   /* 8 + 11 bits: exact */
     }
 }
+/* A caller's cache may hold what fp16 does not: a code times its scale reaches 8.3e6, and rows may hold infinities or NaN.  A
+ * group of 32 rows with a value beyond fp16 is staged by 2^-7, and its mark says so (K: scores are multiplied by it, V:
+ * weights; both exact).  A V row with a value that is still not finite has that value staged as 0, or a token that does not
+ * attend the row would get 0 x infinity, and its bit set: tokens that do attend it get NaN. */
+constexpr float PF_HALF_END = 65520.f, PF_DOWN = 1.f / 128.f;   /* the least magnitude that rounds to an fp16 infinity */
 template <int LAY, int HD, int NP>
-__global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
+__global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg, PfMark *marks) {
+    constexpr bool MARKS = LAY != LAY_Q8P;
     constexpr uint32_t PITCH = 34;   /* halves per dim row of the transposition tile (odd word count) */
     constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128, PER = HD * 32u / 8u / 256u;   /* groups of 8 dims per thread */
     __shared__ __half tile[NP][HD * PITCH];
+    __shared__ uint32_t bad_rows;
     const uint32_t kh = blockIdx.y, p0 = blockIdx.x * 32u, tid = threadIdx.x;
     q4d_pdl_wait();
     const uint8_t *sc = LAY == LAY_Q8P ? C.s + (uint64_t)layer * C.s_layer_stride + (uint64_t)kh * C.s_kvh_stride : nullptr;
     const uint64_t base = (uint64_t)layer * C.layer_stride + (uint64_t)kh * C.kvh_stride;
     float x[PER][8];
+    auto fit = [&]() -> float {   /* the group's factor; all threads */
+        bool over = false;
+#pragma unroll
+        for (uint32_t it = 0; it < PER; it++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) over = over || (fabsf(x[it][j]) >= PF_HALF_END && fabsf(x[it][j]) < PF_HALF_END / PF_DOWN);
+        if (!__syncthreads_or(over)) return 1.f;
+#pragma unroll
+        for (uint32_t it = 0; it < PER; it++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[it][j] *= PF_DOWN;
+        return 1.f / PF_DOWN;
+    };
+    PfMark *mark = marks + (size_t)kh * tiles * (PF_BN / 32u) + blockIdx.x;
     if (blockIdx.z == 0) {
         const uint8_t *kq = C.k + base;
         uint8_t *kt = kimg + ((size_t)kh * tiles + p0 / PF_BN) * CK * PF_CHUNK;
@@ -257,6 +281,10 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
 #pragma unroll
             for (int j = 0; j < 8; j++) x[it][j] = 0.f;
             if (p < n) load8<LAY>(kq + (uint64_t)p * C.tok_stride, sc + (uint64_t)p * C.s_tok_stride, c * 8u, x[it]);
+        }
+        if (MARKS) {
+            const float f = fit();
+            if (tid == 0) mark->k = f;
         }
 #pragma unroll
         for (uint32_t it = 0; it < PER; it++) {
@@ -278,6 +306,7 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
     /* a tile's images in the order of their use: hd 256 {value, rest} of its first 64 positions, then of the others; hd 128
      * value, rest, both halves in each */
     uint8_t *vt = vimg + ((size_t)kh * tiles + p0 / PF_BN) * CV * PF_CHUNK + ((p0 / 64u) & 1u) * (HD * 128u) * (HD == 256 ? NP : 1);
+    if (MARKS && tid == 0) bad_rows = 0u;
 #pragma unroll
     for (uint32_t it = 0; it < PER; it++) {   /* lanes on consecutive rows: the 2-byte stores below do not conflict */
         const uint32_t i = tid + 256u * it, p = p0 + (i & 31u), c = i >> 5;
@@ -285,17 +314,31 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
         for (int j = 0; j < 8; j++) x[it][j] = 0.f;
         if (p < n) load8<LAY>(vq + (uint64_t)p * C.tok_stride, sc + (uint64_t)p * C.s_tok_stride + 2u * (HD / 32u), c * 8u, x[it]);
     }
+    float f = 1.f;
+    if (MARKS) f = fit();
+    uint32_t bad = 0;
 #pragma unroll
     for (uint32_t it = 0; it < PER; it++) {
         const uint32_t i = tid + 256u * it;
+        bool finite = true;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
+            if (MARKS && !(fabsf(x[it][j]) < PF_HALF_END)) {
+                finite = false;
+                x[it][j] = 0.f;
+            }
             const __half h = __float2half_rn(x[it][j]);
             tile[0][((i >> 5) * 8u + j) * PITCH + (i & 31u)] = h;
             if (NP == 2) tile[NP - 1][((i >> 5) * 8u + j) * PITCH + (i & 31u)] = __float2half_rn(x[it][j] - __half2float(h));
         }
+        if (MARKS) bad |= __ballot_sync(0xffffffffu, !finite);
     }
+    if (MARKS && bad && (tid & 31u) == 0u) atomicOr(&bad_rows, bad);
     __syncthreads();
+    if (MARKS && tid == 0) {
+        mark->v = f;
+        mark->bad_rows = bad_rows;
+    }
 #pragma unroll
     for (int im = 0; im < NP; im++)
 #pragma unroll
@@ -321,8 +364,9 @@ __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_a
     asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(1u) : "memory");
     return false;
 }
-/* HD: head size; NQ: query groups per block; NP: images per 128 dims of K and V (2: value and remainder) */
-template <int HD, int NQ, int NP>
+/* HD: head size; NQ: query groups per block; NP: images per 128 dims of K and V (2: value and remainder); MARKS: rows may
+ * have been scaled or not be finite */
+template <int HD, int NQ, int NP, bool MARKS>
 __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParams P) {
     constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128;   /* ring slots a K / V tile takes */
     static_assert(NQ == 1 || NP == 1, "two groups hold a tile's V and the next one's K at once: both images of them leave the ring no slack");
@@ -602,6 +646,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
         for (uint32_t u = 0; u < n_seq && (NQ == 1 || ok); u++) {
             const uint32_t i = u * NQ + g, b = i % SB, use = (i / SB) & 1u, p0 = j0 * PF_BN + u * UN + h * TU;
             const uint32_t t_s = t_lane + (NQ == 2 ? g * 128u + (u & 1u) * 64u : b * 128u + h * TU);
+            PfMark mk[2];
+            bool marked = false;
+            if (MARKS) {   /* the same in all lanes; requested ahead of the scores */
+#pragma unroll
+                for (int i2 = 0; i2 < 2; i2++) mk[i2] = P.marks[(size_t)kh * P.img_tiles * (PF_BN / 32u) + p0 / 32u + i2];
+                marked = mk[0].k != 1.f || mk[1].k != 1.f || mk[0].v != 1.f || mk[1].v != 1.f || (mk[0].bad_rows | mk[1].bad_rows) != 0u;
+            }
             ok = ok && all_wait(bar_s + 8 * b, use);   /* a warp goes on as one */
             if (NQ == 1 && !ok) {
                 if (u == 0 || pair_any(false)) partner(0.f);
@@ -612,6 +663,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
 #pragma unroll
             for (int c = 0; c < (int)TU / 32; c++) tmem_ld32(t_s + 32 * c, *reinterpret_cast<float(*)[32]>(&s[32 * c]));
             tmem_wait_ld();
+            if (MARKS && __builtin_expect(marked, 0)) {
+#pragma unroll
+                for (int k = 0; k < (int)TU; k++) s[k] = (mk[k / 32].bad_rows >> (k & 31)) & 1u ? CUDART_NAN_F : s[k] * mk[k / 32].k;
+            }
             if (__builtin_expect(p0 + TU > warp_min, 0)) {
 #pragma unroll
                 for (int k = 0; k < (int)TU; k++)
@@ -671,6 +726,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
                         for (int k = 0; k < 32; k++) o[k] *= alpha;
                         tmem_st32(t_lane + O_COL + g * 128u + 32 * c, o);
                     }
+                }
+            }
+            if (MARKS && __builtin_expect(marked, 0)) {   /* up to 2^8 x 2^7 */
+#pragma unroll
+                for (int k = 0; k < (int)TU / 2; k++) {
+                    const __half2 f = __float2half2_rn(mk[k / 16].v);
+                    pk[k] = h2u(__hmul2(*reinterpret_cast<const __half2 *>(&pk[k]), f));
                 }
             }
             /* P goes into the first half of the columns this thread has just read (two fp16 per column) */
@@ -843,18 +905,18 @@ int stage_reserve(size_t bytes) {
     return -1;
 }
 
-template <int HD, int NQ, int NP>
+template <int HD, int NQ, int NP, bool MARKS>
 bool attend(const PrefillParams &p, dim3 grid) {
     static bool attr = false;
-    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
+    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP, MARKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
                             "prefill smem attribute"))
         return false;
     attr = true;
-    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP>, grid, PF_THREADS, PF_SMEM, p);
+    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP, MARKS>, grid, PF_THREADS, PF_SMEM, p);
 }
 template <int LAY, int HD, int NP>
-bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg) {
-    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, NP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg);
+bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg, PfMark *marks) {
+    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, NP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg, marks);
 }
 
 /* Ranges of positions that a chunk's blocks of one query group are split into: the count with the least estimated time,
@@ -899,9 +961,9 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
     const uint32_t blocks = (groups + nq - 1u) / nq * a.n_kvh;
     uint32_t split = nq == 1 ? best_split(blocks, sms, tiles, (uint64_t)a.n_tok * a.n_head, hd, np) : 1u;
-    const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes;
+    const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes, m_bytes = (size_t)a.n_kvh * tiles * (PF_BN / 32u) * sizeof(PfMark);
     const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
-    const int room = stage_reserve(k_bytes + v_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0));
+    const int room = stage_reserve(k_bytes + v_bytes + m_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0));
     if (room != 1) return room;
 
     PrefillParams p;
@@ -913,20 +975,23 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     uint8_t *kimg = g_stage, *vimg = g_stage + k_bytes;
     p.kimg = kimg; p.vimg = vimg; p.img_tiles = tiles;
     p.n_split = split;
-    p.part = reinterpret_cast<float *>(g_stage + k_bytes + v_bytes);
-    p.part_ml = reinterpret_cast<float2 *>(g_stage + k_bytes + v_bytes + part_bytes);
+    PfMark *marks = reinterpret_cast<PfMark *>(g_stage + k_bytes + v_bytes);
+    p.marks = marks;
+    p.part = reinterpret_cast<float *>(g_stage + k_bytes + v_bytes + m_bytes);
+    p.part_ml = reinterpret_cast<float2 *>(g_stage + k_bytes + v_bytes + m_bytes + part_bytes);
     p.err = g_q4.err_d;
 
     bool ok;
-    if (a.layout == LAY_Q8P) ok = stage<LAY_Q8P, 128, 1>(a, n, tiles, kimg, vimg);
-    else if (a.layout == LAY_Q8R) ok = hd == 128 ? stage<LAY_Q8R, 128, 2>(a, n, tiles, kimg, vimg) : stage<LAY_Q8R, 256, 2>(a, n, tiles, kimg, vimg);
-    else if (a.layout == LAY_F16) ok = hd == 128 ? stage<LAY_F16, 128, 1>(a, n, tiles, kimg, vimg) : stage<LAY_F16, 256, 1>(a, n, tiles, kimg, vimg);
-    else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, kimg, vimg) : stage<LAY_F32, 256, 1>(a, n, tiles, kimg, vimg);
+    if (a.layout == LAY_Q8P) ok = stage<LAY_Q8P, 128, 1>(a, n, tiles, kimg, vimg, marks);
+    else if (a.layout == LAY_Q8R) ok = hd == 128 ? stage<LAY_Q8R, 128, 2>(a, n, tiles, kimg, vimg, marks) : stage<LAY_Q8R, 256, 2>(a, n, tiles, kimg, vimg, marks);
+    else if (a.layout == LAY_F16) ok = hd == 128 ? stage<LAY_F16, 128, 1>(a, n, tiles, kimg, vimg, marks) : stage<LAY_F16, 256, 1>(a, n, tiles, kimg, vimg, marks);
+    else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, kimg, vimg, marks) : stage<LAY_F32, 256, 1>(a, n, tiles, kimg, vimg, marks);
     if (!ok) return 0;
     const dim3 grid((groups + nq - 1u) / nq, a.n_kvh, split);
-    if (hd == 256) ok = np == 2 ? attend<256, 1, 2>(p, grid) : attend<256, 1, 1>(p, grid);
-    else if (nq == 2) ok = attend<128, 2, 1>(p, grid);
-    else ok = np == 2 ? attend<128, 1, 2>(p, grid) : attend<128, 1, 1>(p, grid);
+    const bool own = a.layout == LAY_Q8P;
+    if (hd == 256) ok = np == 2 ? attend<256, 1, 2, true>(p, grid) : attend<256, 1, 1, true>(p, grid);
+    else if (nq == 2) ok = own ? attend<128, 2, 1, false>(p, grid) : attend<128, 2, 1, true>(p, grid);
+    else ok = np == 2 ? attend<128, 1, 2, true>(p, grid) : own ? attend<128, 1, 1, false>(p, grid) : attend<128, 1, 1, true>(p, grid);
     if (ok && split > 1) {
         const uint64_t total4 = (uint64_t)rows * hd / 4u;
         ok = q4i_launch_pdl("prefill launch", q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4);

@@ -317,3 +317,64 @@ def test_first_token_of_a_reference_abi_chunk_is_its_value_row(oracle, n_head, n
     rows = blocks[..., 2:].copy().view(np.int8).astype(np.float64) * blocks[..., :2].copy().view(np.float16).astype(np.float64)
     want = np.repeat(rows.reshape(n_kvh, hd), n_head // n_kvh, 0) / (1.0 + np.exp(-g[0].astype(np.float64)))
     assert (np.abs(got - want) <= 4e-6 * np.abs(want)).all(), np.abs(got / want - 1)[want != 0].max()
+
+
+@pytest.mark.parametrize("kind,big", [(2, 900.0), (0, 1.0e5)])
+@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base", [(24, 2, 256, 7, 300), (24, 2, 256, 40, 300), (16, 2, 128, 7, 300), (16, 2, 128, 140, 300)])
+def test_reference_abi_chunk_of_rows_beyond_fp16(oracle, kind, big, n_head, n_kvh, hd, n_tok, kv_base):
+    """values beyond 65504 in some rows of K and of V (q8_0: a block scale of 900 is a legal fp16; fp32: magnitudes of 1e5, in
+    one dim that the queries leave out, since the decode form rounds fp32 rows to fp16): finite and right for few tokens and for
+    many.  The rows of K with large values are turned away from the queries, those of V have ordinary keys.  An output is the
+    large value times its weight, so its error is the weight's: 2^-11 from its own rounding, inside the 1e-3; queries, and the
+    fp32 rows, are fp16 numbers here, or their rounding would move the scores by up to 1e-3 more (3.5 sigma of 2e-4)."""
+    from gpu_util import assert_close
+    L = lib()
+    n, kvw = kv_base + n_tok, n_kvh * hd
+    k, v = oracle.normal(51, 0, n * kvw).reshape(n, kvw).copy(), oracle.normal(51, 1, n * kvw).reshape(n, kvw).copy()
+    q, g = oracle.normal(51, 2, n_tok * n_head * hd).reshape(n_tok, n_head, hd), oracle.normal(51, 3, n_tok * n_head * hd).reshape(n_tok, n_head, hd)
+    q, k, v = (x.astype(np.float16).astype(np.float32) for x in (q, k, v))
+    if kind == 2:
+        q[..., :32] = np.abs(q[..., :32])
+        for r in (3, 130, 290):
+            k[r].reshape(n_kvh, hd)[:, :32] = -big * 127 * np.linspace(0.5, 1.0, 32, dtype=np.float32)
+        v[100].reshape(n_kvh, hd)[:, 32:64] = big * 127 * np.linspace(-1.0, 1.0, 32, dtype=np.float32)
+        kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind)
+    else:
+        q[..., 5] = 0.0
+        if n_tok < 8:
+            pytest.skip("the decode form rounds fp32 rows to fp16")
+        k[130].reshape(n_kvh, hd)[:, 5] = big
+        v[100].reshape(n_kvh, hd)[:, 40] = -big
+        kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind)
+    scale = float(1.0 / np.sqrt(hd))
+    got = run_chunk(L, q, kc, vc, g, n_head, n_kvh, hd, kv_base, n, scale, kind)
+    ref = oracle.attn(q, kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, n, scale, kind, threads=8)
+    assert_close(got, ref, "kind %d" % kind)
+    assert L.q4_gpu_last_error() == 0
+
+
+@pytest.mark.parametrize("kind", [2, 1, 0])
+@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok", [(24, 2, 256, 40), (16, 2, 128, 140)])
+def test_reference_abi_chunk_with_value_rows_that_are_not_finite(oracle, kind, n_head, n_kvh, hd, n_tok):
+    """a token's output depends on the rows up to its own: those before a row with an infinity or NaN in V stay as they are, the
+    others get NaN"""
+    from gpu_util import assert_close
+    L = lib()
+    kv_base, at, kvw = 200, 17, n_kvh * hd
+    n = kv_base + n_tok
+    k, v = oracle.normal(61, 0, n * kvw).reshape(n, kvw), oracle.normal(61, 1, n * kvw).reshape(n, kvw).copy()
+    q, g = oracle.normal(61, 2, n_tok * n_head * hd).reshape(n_tok, n_head, hd), oracle.normal(61, 3, n_tok * n_head * hd).reshape(n_tok, n_head, hd)
+    kc, vc = oracle.kv_write(k, kind), oracle.kv_write(v, kind).copy()
+    scale = float(1.0 / np.sqrt(hd))
+    ref = oracle.attn(q, kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, n, scale, kind, threads=8)
+    row = vc.reshape(n, -1)[kv_base + at]
+    if kind == 2:
+        row.view(np.uint16)[17 * 1] = 0x7C00                     # the second block's scale: infinity
+    elif kind == 1:
+        row.view(np.float16)[9] = np.inf
+    else:
+        row.view(np.float32)[9] = np.nan
+    got = run_chunk(L, q, kc, vc, g, n_head, n_kvh, hd, kv_base, n, scale, kind)
+    assert_close(got[:at], ref[:at], "tokens before the row")
+    assert np.isnan(got[at:, :n_head // n_kvh]).any(axis=(1, 2)).all()
+    assert_close(got[at:, n_head // n_kvh:], ref[at:, n_head // n_kvh:], "the other kv head")
