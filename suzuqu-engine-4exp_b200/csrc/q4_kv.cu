@@ -259,17 +259,25 @@ extern "C" bool q4_hip_kv_append_d(void *kcache, void *vcache, const float *k, c
     return launch_append(p, ref_layout(kind));
 }
 
+/* A slice of a prompt: a contraction, on the tensor cores.  512 tokens over 2048 rows of q8_0 at 24 / 2 heads, hd 256, took
+ * 1.23 ms as one decode per token.  Few tokens stay with the decode kernel, which splits the positions finer, and at hd 128
+ * those over few rows, where the chunk's three launches are most of its time: us as decode / as chunk at 16 / 2 heads, fp16, 8
+ * tokens over 2048 rows 8.7 / 11.8, 16 10.8 / 13.1, 24 11.3 / 13.0; 32 over 512 8.9 / 11.0, 64 12.7 / 12.0; 12 over 8192
+ * 20.2 / 19.2; q8_0 16 over 2048 10.3 / 13.7, 24 14.9 / 14.0.  (fp32 takes 16.7 us as decode for 8 over 512, 10.0 as a chunk; hd
+ * 256, 12 heads per kv head, q8_0 17.1 and 13.8.) */
 constexpr uint32_t LEGACY_PREFILL_MIN_TOK = 8;
+constexpr uint64_t LEGACY_PREFILL_MIN_WORK = 81920;   /* tokens x kv heads x rows */
+static bool as_chunk(uint32_t n_tok, uint32_t n_kvh, uint32_t hd, uint32_t kv_base, uint32_t max_kv, int kind) {
+    const uint64_t seen = (uint64_t)kv_base + n_tok, rows = seen < max_kv ? seen : max_kv;
+    return n_tok >= LEGACY_PREFILL_MIN_TOK && (hd == 256 || (hd == 128 && (kind == Q4K_F32 || (uint64_t)n_tok * n_kvh * rows > LEGACY_PREFILL_MIN_WORK)));
+}
 static bool legacy_decode(const float *q, const void *kc, const void *vc, const float *gate, float *out,
                           const int32_t *idx, uint32_t width, uint32_t n_head, uint32_t n_kvh, uint32_t hd,
                           uint32_t n_tok, uint32_t kv_base, uint32_t max_kv, float scale, int kind) {
     if (!g_q4.ok || !q || !kc || !vc || !gate || !out) return false;   /* NULL gate is rejected: :7254,7312 */
     if (n_tok == 0 || hd == 0 || hd > 256 || n_head == 0 || n_kvh == 0) return false;
     if (!hd_ok(hd) || kind < 0 || kind > 2) return q4i_fail(Q4E_ARG, "decode: unsupported hd or kind");
-    /* A slice of a prompt: a contraction, on the tensor cores.  512 tokens over 2048 rows of q8_0 at 24 / 2 heads, hd
-     * 256 took 1.23 ms as one decode per token.  Few tokens stay with the decode kernel, which splits the positions
-     * finer, and so do shapes that the tensor-core tiles do not cover. */
-    if (!idx && n_tok >= LEGACY_PREFILL_MIN_TOK && (hd == 128 || hd == 256) && n_head % n_kvh == 0 && n_head / n_kvh <= 16 && scale > 0.f && max_kv &&
+    if (!idx && as_chunk(n_tok, n_kvh, hd, kv_base, max_kv, kind) && n_head % n_kvh == 0 && n_head / n_kvh <= 16 && scale > 0.f && max_kv &&
         (((uintptr_t)q | (uintptr_t)gate | (uintptr_t)out | (kind == Q4K_Q8 ? 0u : (uintptr_t)kc | (uintptr_t)vc)) & 15u) == 0) {
         Q4PrefillArgs f;
         memset(&f, 0, sizeof(f));

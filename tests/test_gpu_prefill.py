@@ -308,7 +308,7 @@ def test_first_token_of_a_reference_abi_chunk_is_its_value_row(oracle, n_head, n
     """a token that attends one row has weight 1 and gets codes x scales x sigmoid(gate) with no rounding to 16 bits: what is
     left is the gate's (2^-20); the values have 19 bits, a single fp16 image of them would be off by 2^-12"""
     L = lib()
-    n, kvw = 128, n_kvh * hd          # 128 tokens: on the tensor cores in every rule
+    n, kvw = 208, n_kvh * hd          # tokens x rows x kv heads: on the tensor cores at both head sizes
     k, v = oracle.normal(41, 0, n * kvw).reshape(n, kvw), oracle.normal(41, 1, n * kvw).reshape(n, kvw)
     q, g = oracle.normal(41, 2, n * n_head * hd).reshape(n, n_head, hd), oracle.normal(41, 3, n * n_head * hd).reshape(n, n_head, hd)
     kc, vc = oracle.kv_write(k, 2), oracle.kv_write(v, 2)
@@ -378,3 +378,10 @@ def test_reference_abi_chunk_with_value_rows_that_are_not_finite(oracle, kind, n
     assert_close(got[:at], ref[:at], "tokens before the row")
     assert np.isnan(got[at:, :n_head // n_kvh]).any(axis=(1, 2)).all()
     assert_close(got[at:, n_head // n_kvh:], ref[at:, n_head // n_kvh:], "the other kv head")
+
+
+@pytest.mark.parametrize("kind", [2, 1, 0])
+@pytest.mark.parametrize("n_tok,rows", [(20, 2048), (20, 2049), (7, 8000), (8, 8000), (208, 208)])
+def test_reference_abi_chunks_on_both_sides_of_the_decode_form(oracle, kind, n_tok, rows):
+    """few tokens, and at hd 128 few tokens over few rows, are the decode kernel's; more are a chunk"""
+    test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, 16, 2, 128, n_tok, rows - n_tok, rows)
