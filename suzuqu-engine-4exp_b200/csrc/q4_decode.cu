@@ -84,7 +84,7 @@ struct DecParams {
     uint32_t *err;
     const Q4XchgDev *xchg;   /* sequence-sharded decode: exchange window (null otherwise) */
     uint32_t xchg_phase;
-    const float *new_k, *new_v;   /* fused append of the newest row (native q8_0 store), or null */
+    const float *new_k, *new_v;   /* fused append of the newest row (stores at hd 128 and 256), or null */
     uint32_t early_pos, early_rows;   /* positions / rows of a dense scan may be read before the dependent-launch wait */
     uint32_t pdl;                 /* launched with programmatic stream serialization */
     uint32_t gridmerge;           /* long scans: every split's record goes to scratch, the unit's blocks meet at a counter,
@@ -96,7 +96,7 @@ struct DecParams {
                                    * meeting at a cluster barrier */
     uint32_t hybrid;              /* host side: cluster size wanted for a grid merge */
     uint32_t direct;              /* host side: the cache is not aligned for asynchronous copies */
-    uint32_t bulk_runs;           /* tiles of 16 consecutive positions come in by one bulk copy each (else by cp.async) */
+    uint32_t bulk_runs;           /* whole tiles of a dense scan come in by one bulk copy each (else by cp.async) */
 };
 
 /* ---- small device helpers ---------------------------------------------------------------- */
@@ -2385,13 +2385,12 @@ bool q4i_decode(const Q4DecodeArgs &a) {
     p.counters = counters;
     p.err = g_q4.err_d;
     {
-        /* Bulk copies for runs of consecutive positions pay off on dense scans (every tile is a run: one copy
-         * instruction per tile instead of nine); in a gathered list they are slower than coalesced cp.async
-         * (measured: 64-session batch 27.4 vs 26.6 us, single session 8.3 vs 7.9 us).  Q4_DEC_BULK=0 / 1 forces
-         * the choice. */
-        static int bulk = -2;
-        if (bulk == -2) { const char *e = getenv("Q4_DEC_BULK"); bulk = e ? atoi(e) : -1; }
-        p.bulk_runs = bulk >= 0 ? (bulk ? 1u : 0u) : (a.idx ? 0u : 1u);
+        /* Tiles of a dense scan, runs of consecutive positions, come in by one bulk copy each instead of nine instructions;
+         * Q4_DEC_BULK=0: by asynchronous copies.  (Runs inside a gathered list by bulk copy were slower than by coalesced
+         * asynchronous copies: 64-session batch 27.4 against 26.6 us, single session 8.3 against 7.9.) */
+        static int bulk = -1;
+        if (bulk < 0) { const char *e = getenv("Q4_DEC_BULK"); bulk = e ? atoi(e) != 0 : 1; }
+        p.bulk_runs = bulk && !a.idx ? 1u : 0u;
     }
     {
         /* Q4_DEC_GRIDMERGE=0: long scans merge in two levels, each by the last block of a group to arrive */

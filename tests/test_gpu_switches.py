@@ -1,8 +1,8 @@
 """The decode kernel's alternative paths, each forced by its environment switch in a child process (the switches
 are read once per process): the merge through global scratch instead of a cluster, the cluster merge that meets
 at a cluster barrier instead of completing the receiver's mbarrier, launches without programmatic dependent
-launch, the driver's default cluster placement, bulk copies forced on for selection lists and off for dense
-scans, the reference's split-count knob, and the two-level merge of long scans instead of the merge by all of the
+launch, the driver's default cluster placement, bulk copies on (the default: dense scans, never lists) and off,
+the reference's split-count knob, and the two-level merge of long scans instead of the merge by all of the
 unit's blocks.  Every child runs the same parity tests against the oracle."""
 import os
 import subprocess
