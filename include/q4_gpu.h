@@ -432,9 +432,9 @@ bool q4_gpu_batch_decode(q4_gpu_batch *b, uint32_t layer, const void *q, int q_b
                          const float *gate, float *out, const int32_t *idx, uint32_t width,
                          uint32_t idx_kvh_stride, uint32_t idx_sess_stride, uint32_t n_head,
                          float scale);
-/* q4_gpu_batch_append then q4_gpu_batch_decode as one call; on a q8_0 store at hd 128 it is one launch per layer
- * (the attention kernel quantises and stores each session's newest K/V row itself, same bytes as the
- * append).  k, v: [n_sessions][n_kvh*hd] fp32.  Replaces the pair src/q4_fwd.c:891 + :922. */
+/* q4_gpu_batch_append then q4_gpu_batch_decode as one call; at hd 128 and 256 it is one launch per layer
+ * (the attention kernel quantises or converts each session's newest K/V row itself, same bytes as the append),
+ * except where a store is bound to several slots and for the larger fp32 scans at hd 128.  k, v: [n_sessions][n_kvh*hd] fp32.  Replaces the pair src/q4_fwd.c:891 + :922. */
 bool q4_gpu_batch_append_decode(q4_gpu_batch *b, uint32_t layer, const float *k, const float *v, const void *q,
                                 int q_bf16, const float *gate, float *out, const int32_t *idx, uint32_t width,
                                 uint32_t idx_kvh_stride, uint32_t idx_sess_stride, uint32_t n_head, float scale);

@@ -14,11 +14,12 @@
  * per dim in dim order (four heads = four independent chains per thread), and the selection is an
  * exact radix select followed by an index-ordered compaction.  What changes is the mapping: a warp
  * per pooled block with the tree in shuffles, a thread per pooled block for the scan with each warp's
- * 32 rows staged in shared memory by coalesced asynchronous copies, and ONE launch per token for the
- * whole selection instead of the reference's 12: a cluster of 8 blocks with the keys in registers, the
- * histograms summed through distributed shared memory, the digit picked by a warp scan, ballot ranks
- * and scans over warps and blocks for the ordered emit (rows longer than 65 536 blocks: one block that
- * re-reads the row, 16 independent loads at a time).
+ * 32 rows staged in shared memory by coalesced asynchronous copies (many tokens: a tiled product with the
+ * same chains), and ONE launch for the whole selection instead of the reference's 12 per token, in one of
+ * three forms: a cluster of 1, 2, 4 or 8 blocks per token with the keys in registers, the counts of a
+ * 12-bit digit summed through distributed shared memory and the threshold bin's keys pushed to every
+ * block; many tokens at once, a block each that streams its row twice into an index-ordered bitmap; rows
+ * longer than 65 536 blocks, one block that re-reads the row, 16 independent loads at a time.
  */
 #include <math_constants.h>
 #include <string.h>

@@ -209,7 +209,7 @@ struct Q4DecodeArgs {
      * (XCHG_FUSED) wait for theirs and write the merged output; null = single-rank decode */
     const Q4XchgDev *xchg;
     int xchg_phase;
-    /* fused append (native q8_0 store only): the new K and V rows [unit][n_kvh*hd] (fp32) are quantised
+    /* fused append (stores at hd 128 and 256): the new K and V rows [unit][n_kvh*hd] (fp32) are quantised or converted
      * and stored at each unit's position by the attention kernel itself before it reads the cache */
     const float *new_k, *new_v;
     int early_pos, early_rows;   /* the positions / the rows of a dense scan are settled (q4i_settled) */

@@ -374,7 +374,7 @@ class Batch:
 
     def append_decode(self, layer, k, v, q, out, n_head, scale, gate=None, idx=None, width=0, idx_kvh_stride=0,
                       idx_sess_stride=0, q_bf16=False):
-        """append + decode in one call (one launch per layer on a q8_0 store at hd 128)"""
+        """append + decode in one call (one launch per layer at hd 128 and 256)"""
         check(self.L.q4_gpu_batch_append_decode(self.h, layer, _ptr(k), _ptr(v), _ptr(q), int(q_bf16), _ptr(gate),
                                                 _ptr(out), _ptr(idx), width, idx_kvh_stride, idx_sess_stride,
                                                 n_head, scale), "q4_gpu_batch_append_decode")
