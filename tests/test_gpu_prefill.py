@@ -385,3 +385,36 @@ def test_reference_abi_chunk_with_value_rows_that_are_not_finite(oracle, kind, n
 def test_reference_abi_chunks_on_both_sides_of_the_decode_form(oracle, kind, n_tok, rows):
     """few tokens, and at hd 128 few tokens over few rows, are the decode kernel's; more are a chunk"""
     test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, 16, 2, 128, n_tok, rows - n_tok, rows)
+
+
+def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle):
+    """operand images may not grow inside a capture: a chunk that was never run outside one is captured as decode launches"""
+    from gpu_util import assert_close, dev_bytes
+    L = lib()
+    L.q4_gpu_set_stream(None)
+    L.q4_hip_shutdown()                       # gives back what other tests made it reserve
+    L = q4gpu.init()
+    with torch.cuda.stream(torch.cuda.ExternalStream(L.q4_gpu_stream())):
+        assert L.q4_hip_qsa_topk_alloc()
+        n_head, n_kvh, hd, n_tok, kv_base = 24, 2, 256, 20, 300
+        n, kvw = kv_base + n_tok, n_kvh * hd
+        k, v = oracle.normal(95, 0, n * kvw).reshape(n, kvw), oracle.normal(95, 1, n * kvw).reshape(n, kvw)
+        q, g = oracle.normal(95, 2, n_tok * n_head * hd).reshape(n_tok, n_head, hd), oracle.normal(95, 3, n_tok * n_head * hd)
+        kc, vc = oracle.kv_write(k, 2), oracle.kv_write(v, 2)
+        dq, dk, dv, dg = dev(q), dev_bytes(kc), dev_bytes(vc), dev(g)
+        out = torch.full((n_tok, n_head, hd), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+
+        def call(m):
+            return L.q4_hip_qsa_decode_n(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, m, kv_base, n, 1.0 / 16.0, 2)
+        assert call(7)                        # the decode kernel, loaded outside the capture
+        out.fill_(float("nan"))
+        assert L.q4_hip_graph_begin()
+        ok = call(n_tok)
+        graph = L.q4_hip_graph_end()
+        assert ok and graph and L.q4_hip_graph_launch(graph)
+        got = host(out)
+        L.q4_hip_graph_free(graph)
+    ref = oracle.attn(q, kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, n, 1.0 / 16.0, 2, threads=8)
+    assert_close(got, ref, "captured chunk")
+    assert L.q4_gpu_last_error() == 0
