@@ -2279,6 +2279,7 @@ uint32_t split_override() {
 
 }  // namespace
 
+bool q4i_decode_counters(uint64_t units) { return q4i_scratch(0, (size_t)units * DEC_CTR); }
 bool q4i_decode(const Q4DecodeArgs &a) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "decode: library not initialised");
     Q4_REQUIRE(a.q && (a.out || a.part_out) && a.n_units && a.n_head && a.n_kvh, "decode: null/zero argument");

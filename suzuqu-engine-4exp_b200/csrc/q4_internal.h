@@ -215,6 +215,7 @@ struct Q4DecodeArgs {
     int early_pos, early_rows;   /* the positions / the rows of a dense scan are settled (q4i_settled) */
 };
 bool q4i_decode(const Q4DecodeArgs &a);
+bool q4i_decode_counters(uint64_t units);   /* the arrival counters that a decode of so many units x kv heads needs */
 
 /* causal attention of n_tok > 1 query tokens on the tensor cores (q4_prefill.cu): hd 128 or 256 (a native q8_0 store:
  * 128), 1..16 query heads per kv head, scale > 0, 16-byte aligned operands.  1 = enqueued, 0 = failed, -1 = its

@@ -301,6 +301,8 @@ static bool legacy_decode(const float *q, const void *kc, const void *vc, const 
         f.n_head = n_head; f.n_kvh = n_kvh; f.hd = hd;
         f.q = q; f.gate = gate; f.out = out;
         f.n_tok = n_tok; f.kv_base = kv_base; f.scale = scale;
+        /* a longer chunk may be captured after this one and find its images too small: its decode form then needs its counters */
+        if (!g_q4.capturing && !q4i_decode_counters((uint64_t)n_tok * n_kvh)) return false;
         const int r = q4i_prefill(f);
         if (r >= 0) return r == 1;   /* else: no workspace; the decode kernel needs no operand images */
     }

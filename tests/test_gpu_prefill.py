@@ -387,15 +387,18 @@ def test_reference_abi_chunks_on_both_sides_of_the_decode_form(oracle, kind, n_t
     test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, 16, 2, 128, n_tok, rows - n_tok, rows)
 
 
-def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle):
-    """operand images may not grow inside a capture: a chunk that was never run outside one is captured as decode launches"""
+@pytest.mark.parametrize("sized_by", ["topk_alloc", "shorter_chunk"])
+def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle, sized_by):
+    """operand images may not grow inside a capture: a chunk that was never run outside one, or only over fewer rows, is captured
+    as decode launches"""
     from gpu_util import assert_close, dev_bytes
     L = lib()
     L.q4_gpu_set_stream(None)
     L.q4_hip_shutdown()                       # gives back what other tests made it reserve
     L = q4gpu.init()
     with torch.cuda.stream(torch.cuda.ExternalStream(L.q4_gpu_stream())):
-        assert L.q4_hip_qsa_topk_alloc()
+        if sized_by == "topk_alloc":
+            assert L.q4_hip_qsa_topk_alloc()
         n_head, n_kvh, hd, n_tok, kv_base = 24, 2, 256, 20, 300
         n, kvw = kv_base + n_tok, n_kvh * hd
         k, v = oracle.normal(95, 0, n * kvw).reshape(n, kvw), oracle.normal(95, 1, n * kvw).reshape(n, kvw)
@@ -405,9 +408,11 @@ def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle):
         out = torch.full((n_tok, n_head, hd), float("nan"), device="cuda")
         torch.cuda.synchronize()
 
-        def call(m):
-            return L.q4_hip_qsa_decode_n(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, m, kv_base, n, 1.0 / 16.0, 2)
+        def call(m, base=kv_base):
+            return L.q4_hip_qsa_decode_n(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, m, base, n, 1.0 / 16.0, 2)
         assert call(7)                        # the decode kernel, loaded outside the capture
+        if sized_by == "shorter_chunk":
+            assert call(n_tok, 100)
         out.fill_(float("nan"))
         assert L.q4_hip_graph_begin()
         ok = call(n_tok)
