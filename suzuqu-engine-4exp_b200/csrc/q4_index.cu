@@ -104,6 +104,32 @@ bool ix_pdl() {
     if (on < 0) { const char *e = getenv("Q4_IX_PDL"); on = e ? atoi(e) : 1; }
     return on != 0;
 }
+template <typename K, typename... A>
+bool ix_start(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, uint32_t cluster, A... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = g_q4.stream;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = 1;
+        at[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (ix_pdl()) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), what));
+}
 constexpr uint32_t SC_ROW_FLOATS = IX_HD + 4, SC_WARPS = 2;
 constexpr uint32_t SC_TILE_BYTES = 32u * SC_ROW_FLOATS * sizeof(float);
 constexpr uint32_t SC_SMEM = SC_WARPS * 2u * SC_TILE_BYTES + IX_HD * sizeof(float4);
@@ -226,127 +252,178 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
 /* ---- score for many tokens over one pool (a prompt's slice).  The scan above reads the pool once per token, 17 GB
  * through L2 for 512 tokens x 32 768 blocks (1.67 ms).  This form is a tiled fp32 product on the FMA pipe (the
  * result is defined as one fused multiply-add per dim in dim order, which rules the tensor cores out): 32 tokens x 4
- * heads against 16 JC pooled blocks per tile, 8 x JC chains per thread -- two tokens' four heads, so the relu sum over
- * heads stays in the thread.  Bound by the FMA pipe if shared memory keeps up: 8 + JC reads of 16 bytes feed 32 JC
- * multiply-adds, so JC = 16 (with JC = 8 both pipes are equally full, and 512 tokens x 32 768 blocks take 381 us).
- * The queries stay in shared memory while a persistent block walks the tiles; the pool comes in 32 dims at a time,
- * three buffers deep. */
-constexpr uint32_t SM_TOK = 32, SM_ROWS = SM_TOK * 4, SM_THREADS = 256, SM_CD = 32, SM_CHUNKS = IX_HD / SM_CD, SM_STAGES = 3;
-constexpr uint32_t SM_PITCH = SM_CD + 4;   /* floats: 16-byte reads of eight consecutive rows in eight bank groups */
-template <uint32_t JC>
-constexpr uint32_t sm_smem() { return (SM_ROWS * SC_ROW_FLOATS + SM_STAGES * 16u * JC * SM_PITCH) * (uint32_t)sizeof(float); }
-template <uint32_t JC>
+ * heads against 64 M pooled blocks per tile, 8 x 4 M chains per thread -- two tokens' four heads, so the relu sum over
+ * heads stays in the thread.  Both operands lie dim by dim in shared memory (a chunk of 32 dims is transposed on its way
+ * in, through registers; the columns of dim group c are stored at column ^ 4 (c & 7), so that neither the four-byte stores
+ * nor the 16-byte reads meet in a bank), two neighbouring blocks' chains share an instruction (fma.rn.f32x2, one rounding
+ * per chain), and the fragments of the next dim are requested under the products of this one, all 32 dims in line.
+ * 512 tokens x 32 768 blocks, us, all with the same bits:
+ *   one chain per instruction, rows of 4 dims from both operands, cp.async            370  (the FMA pipe 66 % busy: 0.44
+ *                                              warps per issue held up in dispatch, by the register file's ports)
+ *   two chains per instruction, dim by dim, requested in the order of the rows        347  (16 bytes of 32 rows per request)
+ *   requested in whole 128-byte pieces of four rows                                   331
+ *   every dim in line (4 dims in line 324, 8 321), half a chunk in registers at once  294
+ * The FMA pipe alone takes 268 (64.1 TFLOP/s of such products out of registers).  Reading the queries as pairs ready in shared
+ * memory instead of doubling them by moves: 407, bound by what shared memory returns.  Two blocks of 128 threads: 314. */
+constexpr uint32_t SM_TOK = 32, SM_ROWS = SM_TOK * 4, SM_THREADS = 256, SM_CD = 32, SM_CHUNKS = IX_HD / SM_CD;
+template <uint32_t M>
+constexpr uint32_t sm_smem() { return ((IX_HD + 1u) * SM_ROWS + 2u * (SM_CD + 1u) * 64u * M) * (uint32_t)sizeof(float); }   /* a row more each: read ahead, not used */
+__device__ __forceinline__ uint64_t ix_pair(float a, float b) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ float2 ix_unpair(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ uint64_t ix_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+template <uint32_t M>
 __global__ void __launch_bounds__(SM_THREADS, 1) q4_ix_score_mt_k(const float *q, const float *pool, float *score, uint32_t n_tok,
                                                                  uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                                                                  uint32_t pos0, uint32_t ratio) {
-    constexpr uint32_t COLS = 16u * JC;
-    extern __shared__ __align__(16) float sm_tiles[];   /* queries, rows 132 floats apart | pool chunks, rows 36 floats apart */
+    constexpr uint32_t COLS = 64u * M, BUF = (SM_CD + 1u) * COLS;
+    extern __shared__ __align__(16) float sm_tiles[];   /* queries [dim][row] | pool, two chunks [dim][column ^ 4 (dim / 4 % 8)] */
+    float *sk = sm_tiles + (IX_HD + 1u) * SM_ROWS;
     const uint32_t tid = threadIdx.x;
-    const uint32_t ty = tid >> 4, tc = tid & 15u;       /* tokens 2 ty, 2 ty + 1; pooled blocks tc + 16 j */
+    const uint32_t ty = tid >> 4, tc = tid & 15u;       /* tokens 2 ty, 2 ty + 1; pooled blocks 4 tc + 64 m .. + 3 */
+    const uint32_t lr = tid >> 3, lc = tid & 7u;        /* staging: rows lr + 32 k, dims 4 lc .. + 3 of a chunk */
     const uint32_t col_tiles = (n_blocks + COLS - 1u) / COLS, tok_tiles = (n_tok + SM_TOK - 1u) / SM_TOK;
     const uint64_t total = (uint64_t)col_tiles * tok_tiles;
     const uint32_t first = (uint32_t)(total * blockIdx.x / gridDim.x), last = (uint32_t)(total * (blockIdx.x + 1u) / gridDim.x);
-    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(sm_tiles) + SM_ROWS * SC_ROW_FLOATS * 4u;
+    const bool vec = ((uintptr_t)score & 15u) == 0u && (stride & 3u) == 0u;
     auto visible = [&](uint32_t tok) { return (pos0 + tok + 1u) / ratio; };
+    float4 stage[M];
     /* rows of a tile that no token of the group can see are not read: they need not exist yet */
-    auto fetch = [&](uint32_t it) {
-        const uint32_t tile = first + it / SM_CHUNKS, d0 = (it % SM_CHUNKS) * SM_CD;
+    auto request = [&](uint32_t it, uint32_t half) {
+        const uint32_t tile = first + it / SM_CHUNKS;
+        uint32_t lim = 0, c0 = 0;
         if (tile < last) {
-            const uint32_t t_last = min((tile / col_tiles + 1u) * SM_TOK, n_tok) - 1u, c0 = (tile % col_tiles) * COLS;
-            const uint32_t lim = min(visible(t_last), n_blocks), dst0 = s0 + (it % SM_STAGES) * COLS * SM_PITCH * 4u;
-#pragma unroll
-            for (uint32_t k = 0; k < COLS * (SM_CD / 4u) / SM_THREADS; k++) {
-                const uint32_t i = tid + k * SM_THREADS, r = i / (SM_CD / 4u), c = i % (SM_CD / 4u);
-                const uint32_t dst = dst0 + (r * SM_PITCH + c * 4u) * 4u;
-                if (c0 + r < lim)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(pool + (size_t)(c0 + r) * IX_HD + d0 + c * 4u) : "memory");
-                else
-                    asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dst), "r"(0u) : "memory");
-            }
+            c0 = (tile % col_tiles) * COLS + half * (COLS / 2u);
+            lim = min(visible(min((tile / col_tiles + 1u) * SM_TOK, n_tok) - 1u), n_blocks);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float *src = pool + (size_t)(c0 + lr) * IX_HD + (it % SM_CHUNKS) * SM_CD + 4u * lc;
+#pragma unroll
+        for (uint32_t k = 0; k < M; k++) {
+            stage[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c0 + lr + 32u * k < lim) stage[k] = *reinterpret_cast<const float4 *>(src + (size_t)(32u * k) * IX_HD);
+        }
     };
+    auto put = [&](uint32_t it, uint32_t half) {
+        float *dst = sk + (it & 1u) * BUF + 4u * lc * COLS + half * (COLS / 2u) + (lr ^ (4u * lc));
+#pragma unroll
+        for (uint32_t k = 0; k < M; k++) {
+            dst[32u * k] = stage[k].x;
+            dst[COLS + 32u * k] = stage[k].y;
+            dst[2u * COLS + 32u * k] = stage[k].z;
+            dst[3u * COLS + 32u * k] = stage[k].w;
+        }
+    };
+    q4d_pdl_wait();
     uint32_t have = 0xffffffffu, it = 0;
-    fetch(0);
-    fetch(1);
+    request(0, 0);
+    put(0, 0);
+    request(0, 1);
+    put(0, 1);
     for (uint32_t tile = first; tile < last; tile++) {
         const uint32_t group = tile / col_tiles, c0 = (tile % col_tiles) * COLS;
         if (group != have) {
             __syncthreads();   /* everyone is done with the queries of the group before */
             for (uint32_t i = tid; i < SM_ROWS * 32u; i += SM_THREADS) {
-                const uint32_t r = i >> 5, c = i & 31u, tok = group * SM_TOK + (r >> 2), h = r & 3u;
+                const uint32_t r = i % SM_ROWS, c = i / SM_ROWS, tok = group * SM_TOK + (r >> 2), h = r & 3u;
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (tok < n_tok && h < n_head) v = *reinterpret_cast<const float4 *>(q + ((size_t)tok * n_head + h) * IX_HD + c * 4u);
-                *reinterpret_cast<float4 *>(sm_tiles + r * SC_ROW_FLOATS + c * 4u) = v;
+                float *dst = sm_tiles + 4u * c * SM_ROWS + r;
+                dst[0] = v.x; dst[SM_ROWS] = v.y; dst[2u * SM_ROWS] = v.z; dst[3u * SM_ROWS] = v.w;
             }
             have = group;
         }
-        float acc[8][JC];
+        uint64_t acc[8][2 * M];
 #pragma unroll
         for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (uint32_t j = 0; j < JC; j++) acc[i][j] = 0.f;
+            for (uint32_t j = 0; j < 2 * M; j++) acc[i][j] = 0ull;
 #pragma unroll 1
         for (uint32_t ch = 0; ch < SM_CHUNKS; ch++, it++) {
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncthreads();   /* chunk `it` is in; everyone is done with the buffer that chunk it + 2 goes to */
-            fetch(it + 2u);
-            const float *qa = sm_tiles + ty * 8u * SC_ROW_FLOATS + ch * SM_CD;
-            const float *kb = sm_tiles + SM_ROWS * SC_ROW_FLOATS + (it % SM_STAGES) * COLS * SM_PITCH + tc * SM_PITCH;
-#pragma unroll 2
-            for (uint32_t d = 0; d < SM_CD; d += 4) {
-                float4 a[8];
+            __syncthreads();   /* chunk `it` is in; everyone is done with the buffer that chunk it + 1 goes to */
+            request(it + 1u, 0);
+            const float *qa = sm_tiles + ch * SM_CD * SM_ROWS + ty * 8u, *kb = sk + (it & 1u) * BUF;
+            float4 an[2], bn[M];
+            an[0] = *reinterpret_cast<const float4 *>(qa);
+            an[1] = *reinterpret_cast<const float4 *>(qa + 4);
 #pragma unroll
-                for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(qa + i * SC_ROW_FLOATS + d);
+            for (uint32_t m = 0; m < M; m++) bn[m] = *reinterpret_cast<const float4 *>(kb + 64u * m + 4u * tc);
 #pragma unroll
-                for (uint32_t j0 = 0; j0 < JC; j0 += 4) {
-                    float4 b[4];
+            for (uint32_t d = 0; d < SM_CD; d++) {
+                const float a[8] = {an[0].x, an[0].y, an[0].z, an[0].w, an[1].x, an[1].y, an[1].z, an[1].w};
+                uint64_t b[2 * M];
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; j++) b[j] = *reinterpret_cast<const float4 *>(kb + (j0 + j) * 16u * SM_PITCH + d);
+                for (uint32_t m = 0; m < M; m++) {
+                    b[2 * m] = ix_pair(bn[m].x, bn[m].y);
+                    b[2 * m + 1] = ix_pair(bn[m].z, bn[m].w);
+                }
+                an[0] = *reinterpret_cast<const float4 *>(qa + (d + 1u) * SM_ROWS);
+                an[1] = *reinterpret_cast<const float4 *>(qa + (d + 1u) * SM_ROWS + 4);
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
+                for (uint32_t m = 0; m < M; m++)
+                    bn[m] = *reinterpret_cast<const float4 *>(kb + (d + 1u) * COLS + 64u * m + ((4u * tc) ^ ((d + 1u) & 28u)));
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].x, b[j].x, acc[i][j0 + j]);
+                for (int i = 0; i < 8; i++) {
+                    const uint64_t x = ix_pair(a[i], a[i]);
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-#pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].y, b[j].y, acc[i][j0 + j]);
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-#pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].z, b[j].z, acc[i][j0 + j]);
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-#pragma unroll
-                        for (uint32_t j = 0; j < 4; j++) acc[i][j0 + j] = __fmaf_rn(a[i].w, b[j].w, acc[i][j0 + j]);
+                    for (uint32_t j = 0; j < 2 * M; j++) acc[i][j] = ix_fma2(x, b[j], acc[i][j]);
+                }
+                if (d == SM_CD / 2u) {
+                    put(it + 1u, 0);
+                    request(it + 1u, 1);
                 }
             }
+            put(it + 1u, 1);
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const uint32_t tok = group * SM_TOK + 2u * ty + u;
             if (tok >= n_tok) continue;
             const uint32_t n_vis = visible(tok);
+            float *row = score + (size_t)tok * stride;
 #pragma unroll
-            for (uint32_t j = 0; j < JC; j++) {
-                const uint32_t b = c0 + tc + 16u * j;
-                /* heads that do not exist have zero queries: their relu adds exactly nothing */
-                float sc = __fadd_rn(0.f, fmaxf(acc[4 * u][j], 0.f));
-                sc = __fadd_rn(sc, fmaxf(acc[4 * u + 1][j], 0.f));
-                sc = __fadd_rn(sc, fmaxf(acc[4 * u + 2][j], 0.f));
-                sc = __fadd_rn(sc, fmaxf(acc[4 * u + 3][j], 0.f));
-                if (b < n_blocks) score[(size_t)tok * stride + b] = b < n_vis ? sc : -1.0e30f;
+            for (uint32_t m = 0; m < M; m++) {
+                const uint32_t c = c0 + 4u * tc + 64u * m;
+                float sc[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    /* heads that do not exist have zero queries: their relu adds exactly nothing */
+                    float v = 0.f;
+#pragma unroll
+                    for (int h = 0; h < 4; h++) {
+                        const float2 f = ix_unpair(acc[4 * u + h][2 * m + (e >> 1)]);
+                        v = __fadd_rn(v, fmaxf(e & 1 ? f.y : f.x, 0.f));
+                    }
+                    sc[e] = c + e < n_vis ? v : -1.0e30f;
+                }
+                if (vec && c + 3u < n_blocks) {
+                    *reinterpret_cast<float4 *>(row + c) = make_float4(sc[0], sc[1], sc[2], sc[3]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (c + e < n_blocks) row[c + e] = sc[e];
+                }
             }
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
-/* Estimated ns of the product with tiles of 16 JC blocks, and of the scan; fitted to 1 .. 512 tokens over 16 .. 65 536 blocks,
- * within 10 % where the two are close.  Product: a tile takes a time of its own however few of its 32 tokens exist (us,
- * narrow / wide tiles: 32 tokens over 8192 blocks 18.0 / -, 32 over 32 768 - / 29.1, 512 over 65 536 - / 726). */
-uint64_t score_mt_ns(uint32_t n_tok, uint32_t n_blocks, uint32_t jc) {
-    const uint64_t tiles = (uint64_t)((n_blocks + 16u * jc - 1u) / (16u * jc)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
-    return 3500u + (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count * (jc == 16u ? 26200u : 13200u);
+/* Estimated ns of the product with tiles of 64 M blocks, and of the scan; fitted to 2 .. 512 tokens over 64 .. 65 536 blocks,
+ * within 10 % where the forms are close.  Product: a tile takes a time of its own however few of its 32 tokens exist (us,
+ * narrow / wide tiles: 32 tokens over 8192 blocks 16.6 / 25.6, 33 over 16 384 28.5 / 26.3, 512 over 65 536 667 / 602; with
+ * tiles of the earlier form 18.7, 31.0 and 726). */
+uint64_t score_mt_ns(uint32_t n_tok, uint32_t n_blocks, uint32_t m) {
+    const uint64_t tiles = (uint64_t)((n_blocks + 64u * m - 1u) / (64u * m)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
+    return (m == 4u ? 4300u : 5000u) + (tiles + (uint64_t)g_q4.sm_count - 1u) / (uint64_t)g_q4.sm_count * (m == 4u ? 21000u : 11750u);
 }
 /* Scan: tiles of 32 blocks a warp takes one after the other, and again (with the card nearly to itself) where the tokens'
  * grids do not fit at once: 4 tokens over 65 536 blocks 25.0 us, 5 (445 blocks of 444) 40.3, 8 62.7, 12 62.5. */
@@ -357,18 +434,18 @@ uint64_t score_scan_ns(uint32_t n_tok, uint32_t n_blocks) {
     const uint64_t per_warp = ((n_blocks + 31u) / 32u + gx * SC_WARPS - 1u) / (gx * SC_WARPS), waves = ((uint64_t)gx * n_tok + all - 1u) / all;
     return 3000u + per_warp * (2150u + (waves - 1u) * 1250u);
 }
-template <uint32_t JC>
+template <uint32_t M>
 bool score_mt_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride, uint32_t n_head,
                      uint32_t pos0, uint32_t ratio) {
     static bool done = false;
-    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score_mt_k<JC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_smem<JC>()),
+    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score_mt_k<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_smem<M>()),
                             "qsa_score smem attribute"))
         return false;
     done = true;
-    const uint64_t tiles = (uint64_t)((n_blocks + 16u * JC - 1u) / (16u * JC)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
+    const uint64_t tiles = (uint64_t)((n_blocks + 64u * M - 1u) / (64u * M)) * ((n_tok + SM_TOK - 1u) / SM_TOK);
     const uint32_t grid = (uint32_t)(tiles < (uint64_t)g_q4.sm_count ? tiles : (uint64_t)g_q4.sm_count);
-    q4_ix_score_mt_k<JC><<<grid, SM_THREADS, sm_smem<JC>(), g_q4.stream>>>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
-    return q4i_launched(q4i_check(cudaGetLastError(), "qsa_score launch"));
+    return ix_start("qsa_score launch", q4_ix_score_mt_k<M>, dim3(grid), SM_THREADS, sm_smem<M>(), 1u, q, pool, score, n_tok, n_blocks, stride,
+                    n_head, pos0, ratio);
 }
 template <int FORM>
 bool score_start(dim3 grid, const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
@@ -380,20 +457,8 @@ bool score_start(dim3 grid, const float *q, const float *pool, float *score, uin
             return false;
         done = true;
     }
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(SC_WARPS * 32);
-    cfg.dynamicSmemBytes = SC_SMEM;
-    cfg.stream = g_q4.stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = ix_pdl() ? 1 : 0;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, q4_ix_score_k<FORM>, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr,
-                                                     n_tok, FORM == SC_ONE && ix_pdl() && (!pp || q4i_settled(g_q4.pos_written))),
-                     "qsa_score launch"));
+    return ix_start("qsa_score launch", q4_ix_score_k<FORM>, grid, SC_WARPS * 32u, SC_SMEM, 1u, q, pool, score, n_blocks, stride, n_head, pos0, ratio, pp,
+                    pools, pos_arr, n_tok, FORM == SC_ONE && ix_pdl() && (!pp || q4i_settled(g_q4.pos_written)));
 }
 /* persistent grid: 3 blocks of 2 warps per SM share 227 KB; fewer when the rows are short */
 bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
@@ -1055,32 +1120,6 @@ __global__ void __launch_bounds__(TKM_THREADS, 4) q4_ix_topkm_k(const float *sco
     }
 }
 
-template <typename K, typename... A>
-bool topk_start(K kernel, dim3 grid, uint32_t threads, size_t smem, uint32_t cluster, A... args) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = g_q4.stream;
-    cudaLaunchAttribute at[2];
-    unsigned n = 0;
-    if (cluster > 1) {
-        at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = cluster;
-        at[n].val.clusterDim.y = 1;
-        at[n].val.clusterDim.z = 1;
-        n++;
-    }
-    if (ix_pdl()) {
-        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[n].val.programmaticStreamSerializationAllowed = 1;
-        n++;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = n;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), "qsa_topk launch"));
-}
 template <uint32_t NB>
 bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stride, uint32_t k_blk, uint32_t ratio, uint32_t pos0,
                  uint32_t width, const int32_t *pp, const int32_t *pos_arr) {
@@ -1090,7 +1129,7 @@ bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
         return false;
     done = true;
     const uint32_t vis = ratio ? (pos0 + n_tok) / ratio : 0u;   /* of the last token, where the host gives the position */
-    return topk_start(q4_ix_topkc_k<NB>, dim3(NB, n_tok), IX_TK_THREADS, sizeof(TkcShared<NB>), NB, score, sel, stride, k_blk, ratio, pos0,
+    return ix_start("qsa_topk launch", q4_ix_topkc_k<NB>, dim3(NB, n_tok), IX_TK_THREADS, sizeof(TkcShared<NB>), NB, score, sel, stride, k_blk, ratio, pos0,
                       width, pp, pos_arr, pos_arr || vis > stride ? stride : vis, ix_pdl() && ratio && !pos_arr && (!pp || q4i_settled(g_q4.pos_written)));
 }
 /* Which form: rows of up to 8192 keys need one block either way, which keeps them in registers.  Longer rows take the
@@ -1111,7 +1150,7 @@ bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
             return false;
         done = true;
         const uint32_t words = (stride + 31u) / 32u;
-        return topk_start(q4_ix_topkm_k, dim3(n_tok), TKM_THREADS, sizeof(TkmShared) + 2u * words * 4u, 1u, score, sel, stride, k_blk, ratio,
+        return ix_start("qsa_topk launch", q4_ix_topkm_k, dim3(n_tok), TKM_THREADS, sizeof(TkmShared) + 2u * words * 4u, 1u, score, sel, stride, k_blk, ratio,
                           pos0, width, words, pp, pos_arr);
     }
     if (nb == 2) return topkc_start<2>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
@@ -1139,9 +1178,9 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
     if (!g_q4.ok || !q || !pool || !score || n_tok == 0 || hd != IX_HD || n_head == 0 || n_head > 4) return false;
     if (n_blocks == 0) return true;
     if (ratio && n_tok > 1 && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0) {
-        const uint64_t wide = score_mt_ns(n_tok, n_blocks, 16), narrow = score_mt_ns(n_tok, n_blocks, 8), scan = score_scan_ns(n_tok, n_blocks);
-        if (wide <= narrow && wide < scan) return score_mt_launch<16>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
-        if (narrow < scan) return score_mt_launch<8>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+        const uint64_t wide = score_mt_ns(n_tok, n_blocks, 4), narrow = score_mt_ns(n_tok, n_blocks, 2), scan = score_scan_ns(n_tok, n_blocks);
+        if (wide <= narrow && wide < scan) return score_mt_launch<4>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+        if (narrow < scan) return score_mt_launch<2>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     }
     return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr, nullptr, nullptr);
 }

@@ -309,3 +309,25 @@ def test_scores_of_a_few_tokens_on_both_sides_of_the_product(n_tok, blocks):
     for t in range(n_tok):
         assert L.q4_hip_qsa_score(q[t].data_ptr(), pool.data_ptr(), b[t].data_ptr(), 1, blocks, blocks, 4, 128, pos0 + t, RATIO)
     assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("n_tok,n_head,blocks,slack", [(33, 4, 16389, 3), (40, 4, 16389, 0), (33, 3, 8193, 7), (64, 4, 4095, 1), (47, 2, 4098, 2), (130, 4, 16450, 2)])
+def test_product_tiles_have_the_bits_of_the_scan(n_tok, n_head, blocks, slack):
+    """wide (64 M = 256) and narrow (128) tiles: last columns of one to four blocks, rows that are stored 16 bytes at a time (stride
+    a multiple of 4) and not, fewer heads than four, infinities, NaN, subnormals and negative zeros in the pool"""
+    L = lib()
+    g = torch.Generator(device="cuda").manual_seed(blocks + n_tok)
+    pool = torch.randn(blocks, 128, device="cuda", generator=g)
+    flat = pool.view(-1)
+    for i, x in enumerate((float("inf"), float("-inf"), float("nan"), 1e-41, -0.0, 3e38)):
+        flat[torch.randint(0, flat.numel(), (50,), device="cuda", generator=g)] = x
+    pool[-1, 127] = float("inf")
+    q = torch.randn(n_tok, n_head, 128, device="cuda", generator=g)
+    q[1, 0, 5] = 0.0
+    q[2, 0] = 1e-30
+    pos0, stride = blocks * RATIO - n_tok, blocks + slack
+    a, b = torch.full((n_tok, stride), 7.0, device="cuda"), torch.full((n_tok, stride), 7.0, device="cuda")
+    assert L.q4_hip_qsa_score(q.data_ptr(), pool.data_ptr(), a.data_ptr(), n_tok, blocks, stride, n_head, 128, pos0, RATIO)
+    for t in range(n_tok):
+        assert L.q4_hip_qsa_score(q[t].data_ptr(), pool.data_ptr(), b[t].data_ptr(), 1, blocks, stride, n_head, 128, pos0 + t, RATIO)
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
