@@ -678,9 +678,14 @@ template <uint32_t NT>
 __device__ __forceinline__ TkPick tk_pick(const uint32_t *hist, uint32_t target, uint32_t *tot /* [32] */, TkPick *st) {
     constexpr uint32_t PER = TK_BINS / NT;
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, top = TK_BINS - 1u - PER * threadIdx.x;
+    static_assert(PER % 4 == 0, "whole 16-byte words of counts per thread: a count at a time they met in PER-way bank conflicts");
     uint32_t c[PER], sum = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < PER; j++) { c[j] = hist[top - j]; sum += c[j]; }
+    for (uint32_t j = 0; j < PER; j += 4) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(hist + top - j - 3u);
+        c[j] = x.w; c[j + 1] = x.z; c[j + 2] = x.y; c[j + 3] = x.x;
+        sum += (x.x + x.y) + (x.z + x.w);
+    }
     uint32_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
