@@ -331,3 +331,33 @@ def test_product_tiles_have_the_bits_of_the_scan(n_tok, n_head, blocks, slack):
     for t in range(n_tok):
         assert L.q4_hip_qsa_score(q[t].data_ptr(), pool.data_ptr(), b[t].data_ptr(), 1, blocks, stride, n_head, 128, pos0 + t, RATIO)
     assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("n_vis,stride,k_blk", [(16385, 16387, 512), (20000, 20000, 512), (32768, 32768, 512), (33001, 33004, 7), (65536, 65536, 512)])
+def test_sampled_selection_of_many_tokens(oracle, n_vis, stride, k_blk):
+    """rows long enough for a sample: ordinary ones, rows whose largest keys are exactly the sampled ones (the pivot is too
+    high), rows whose sampled keys are the smallest, rows of ties and of zeros, large keys in one run, infinities; a row start
+    on every 4-byte boundary"""
+    L = lib()
+    n_tok = 160
+    rng = np.random.default_rng(n_vis)
+    step = n_vis // 2048
+    i = np.arange((n_vis + step - 1) // step, dtype=np.uint64)
+    at = np.minimum(i * step + ((i * 0x9E3779B1 % 2**32) >> 16) % step, n_vis - 1)
+    sc = np.zeros((n_tok, stride), np.float32)
+    sc[:] = np.abs(rng.standard_normal((n_tok, stride))).astype(np.float32)
+    sc[1::8, at] += 100
+    sc[2::8, at] = 0
+    sc[3::8] = np.round(sc[3::8] * 2)
+    sc[4::8, 100:2000] += 7
+    sc[5::8] = 50 + sc[5::8] * 1e-4
+    sc[6::8, rng.integers(0, n_vis, 300)] = np.inf
+    sc[7::8] = 0
+    sc[15::16] = -1
+    pos0, width = n_vis * RATIO - n_tok, k_blk * RATIO + 3
+    d = torch.from_numpy(sc).cuda()
+    d_sel = torch.full((n_tok, width), -7, dtype=torch.int32, device="cuda")
+    assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), n_tok, n_vis, stride, k_blk, RATIO, pos0, width)
+    got = host(d_sel)
+    for t in list(range(16)) + [n_tok - 1]:
+        assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, stride, k_blk, RATIO, pos0 + t, width)[0]), t
