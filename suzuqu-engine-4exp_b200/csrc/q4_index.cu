@@ -249,6 +249,95 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
     for (uint32_t b = n_vis + blockIdx.x * (SC_WARPS * 32u) + threadIdx.x; b < n_blocks; b += gridDim.x * SC_WARPS * 32u)
         score[(size_t)t * stride + b] = -1.0e30f;
 }
+/* ---- score of one token over as many rows as one block per SM holds at once (66 304 on 148 SMs: every context of the
+ * engine's).  The form above has two parts per warp and three blocks per SM, so of 65 536 rows the last third waits for
+ * parts to be walked (1.2 us), and reading shared memory takes longer than HBM: a 16-byte read costs four cycles of what it
+ * returns to a warp, the query's broadcasts too, 5 of them per 4 dims of 32 rows.  Here every warp requests all it will need
+ * at once, and where a block has more than SC1_SHORT rows a lane walks two (6 reads per 4 dims of 64 rows).  Chunk c of row r
+ * lies at c ^ (r & 7): 16-byte reads of eight consecutive rows fall into eight different bank groups, without the padding
+ * that would not fit.  Eight steps in line, not 32: the kernel's image is fetched anew by every launch.
+ * us, the form above / here: 64 rows 2.57 / 2.4, 4096 2.66 / 2.66, 16 384 4.28 / 4.1, 32 768 6.66 / 5.2, 65 536 9.3 / 8.5. */
+constexpr uint32_t SC1_WARPS = 7, SC1_ROWS = SC1_WARPS * 64, SC1_SHORT = 128, SC1_SMEM = IX_HD * (uint32_t)sizeof(float4) + SC1_ROWS * IX_HD * (uint32_t)sizeof(float);
+/* rows at .. at + 32 R - 1, below r1, by one warp */
+template <int R>
+__device__ __forceinline__ void sc1_fetch(uint32_t buf, const float *pool, uint32_t at, uint32_t r1) {
+    const uint32_t lane = threadIdx.x & 31u, rows = at < r1 ? min(32u * R, r1 - at) : 0u;
+    const float *src = pool + (size_t)at * IX_HD + lane * 4u;
+    for (uint32_t r = 0; r < rows; r++)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buf + r * (IX_HD * 4u) + ((lane ^ (r & 7u)) << 4)), "l"(src + (size_t)r * IX_HD) : "memory");
+}
+template <int R>
+__device__ __forceinline__ void sc1_walk(uint32_t buf, const float4 *qs, float *score, uint32_t at, uint32_t r1, uint32_t n_head) {
+    const uint32_t lane = threadIdx.x & 31u, row = buf + lane * (IX_HD * 4u), x = lane & 7u;
+    auto chunk = [&](uint32_t i, float4 (&k)[R]) {   /* rows lane, lane + 32; stale bytes behind r1 are walked and not stored */
+#pragma unroll
+        for (int u = 0; u < R; u++)
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(k[u].x), "=f"(k[u].y), "=f"(k[u].z), "=f"(k[u].w)
+                         : "r"(row + ((i ^ x) << 4) + u * (32u * IX_HD * 4u)) : "memory");
+    };
+    float d[R][4];
+#pragma unroll
+    for (int u = 0; u < R; u++) d[u][0] = d[u][1] = d[u][2] = d[u][3] = 0.f;
+    float4 k[4][R];   /* a row is read two steps ahead of the multiply-adds that use it */
+    chunk(0, k[0]);
+    chunk(1, k[1]);
+#pragma unroll 8
+    for (uint32_t i = 0; i < IX_HD / 4; i++) {
+        if (i < IX_HD / 4 - 2) chunk(i + 2u, k[(i + 2u) & 3u]);
+        const float4 q0 = qs[4 * i], q1 = qs[4 * i + 1], q2 = qs[4 * i + 2], q3 = qs[4 * i + 3];
+        auto step = [&](const float4 qd, float kd, float (&a)[4]) {
+            a[0] = __fmaf_rn(qd.x, kd, a[0]); a[1] = __fmaf_rn(qd.y, kd, a[1]); a[2] = __fmaf_rn(qd.z, kd, a[2]); a[3] = __fmaf_rn(qd.w, kd, a[3]);
+        };
+#pragma unroll
+        for (int u = 0; u < R; u++) step(q0, k[i & 3u][u].x, d[u]);
+#pragma unroll
+        for (int u = 0; u < R; u++) step(q1, k[i & 3u][u].y, d[u]);
+#pragma unroll
+        for (int u = 0; u < R; u++) step(q2, k[i & 3u][u].z, d[u]);
+#pragma unroll
+        for (int u = 0; u < R; u++) step(q3, k[i & 3u][u].w, d[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        float sc = __fadd_rn(0.f, fmaxf(d[u][0], 0.f));          /* s = 0; s += relu(dot_h) in head order */
+        if (n_head > 1) sc = __fadd_rn(sc, fmaxf(d[u][1], 0.f));
+        if (n_head > 2) sc = __fadd_rn(sc, fmaxf(d[u][2], 0.f));
+        if (n_head > 3) sc = __fadd_rn(sc, fmaxf(d[u][3], 0.f));
+        if (at + lane + 32u * u < r1) score[at + lane + 32u * u] = sc;
+    }
+}
+__global__ void __launch_bounds__(SC1_WARPS * 32) q4_ix_score1_k(const float *q, const float *pool, float *score, uint32_t n_blocks, uint32_t stride,
+                                                                 uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, bool early) {
+    extern __shared__ __align__(16) uint8_t sc_smem[];
+    float4 *qs = reinterpret_cast<float4 *>(sc_smem);   /* [dim] = the 4 heads' values (0 for heads that do not exist) */
+    const uint32_t warp = threadIdx.x >> 5;
+    if (!early) q4d_pdl_wait();
+    const uint32_t pos = pp ? (uint32_t)*pp : pos0, n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    if (pp) n_blocks = min(n_vis, stride);      /* device position: the bound is derived here */
+    const uint32_t lim = min(n_blocks, n_vis), per = (lim + gridDim.x - 1u) / gridDim.x;   /* at most SC1_ROWS */
+    const uint32_t r0 = min(blockIdx.x * per, lim), r1 = min(r0 + per, lim);
+    const bool two = per > SC1_SHORT;
+    const uint32_t at = r0 + warp * (two ? 64u : 32u);
+    const uint32_t buf = (uint32_t)__cvta_generic_to_shared(sc_smem + IX_HD * sizeof(float4)) + warp * (64u * IX_HD * 4u);
+    if (early) q4d_pdl_wait();
+    if (two) sc1_fetch<2>(buf, pool, at, r1);
+    else sc1_fetch<1>(buf, pool, at, r1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    /* the query is staged while the rows are in flight */
+    if (threadIdx.x < IX_HD) {
+        const float *qt = q + threadIdx.x;
+        qs[threadIdx.x] = make_float4(qt[0], n_head > 1 ? qt[IX_HD] : 0.f, n_head > 2 ? qt[2 * IX_HD] : 0.f, n_head > 3 ? qt[3 * IX_HD] : 0.f);
+    }
+    __syncthreads();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    if (at < r1) {
+        if (two) sc1_walk<2>(buf, qs, score, at, r1, n_head);
+        else sc1_walk<1>(buf, qs, score, at, r1, n_head);
+    }
+    /* blocks the token cannot see (host-position form only): -1e30 */
+    for (uint32_t b = n_vis + blockIdx.x * blockDim.x + threadIdx.x; b < n_blocks; b += gridDim.x * blockDim.x) score[b] = -1.0e30f;
+}
 /* ---- score for many tokens over one pool (a prompt's slice).  The scan above reads the pool once per token, 17 GB
  * through L2 for 512 tokens x 32 768 blocks (1.67 ms).  This form is a tiled fp32 product on the FMA pipe (the
  * result is defined as one fused multiply-add per dim in dim order, which rules the tensor cores out): 32 tokens x 4
@@ -467,6 +556,16 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
     if (pools && (uint64_t)need * n_tok > all)
         return score_start<SC_SHARED>(dim3(all), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr);
     if (pools) return score_start<SC_EACH>(dim3(need, n_tok), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr);
+    const uint32_t rows = pp ? stride : n_blocks;
+    if (n_tok == 1 && rows <= (uint32_t)g_q4.sm_count * SC1_ROWS) {
+        static bool done = false;
+        if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score1_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC1_SMEM), "qsa_score smem attribute"))
+            return false;
+        done = true;
+        const uint32_t fill = (rows + 31u) / 32u, grid = fill < (uint32_t)g_q4.sm_count ? (fill ? fill : 1u) : (uint32_t)g_q4.sm_count;
+        return ix_start("qsa_score launch", q4_ix_score1_k, dim3(grid), SC1_WARPS * 32u, SC1_SMEM, 1u, q, pool, score, n_blocks, stride, n_head, pos0, ratio,
+                        pp, ix_pdl() && (!pp || q4i_settled(g_q4.pos_written)));
+    }
     uint32_t gx = n_tok > 1 ? (all + n_tok - 1u) / n_tok : all;
     if (gx > need) gx = need;
     if (gx < 1) gx = 1;

@@ -361,3 +361,26 @@ def test_sampled_selection_of_many_tokens(oracle, n_vis, stride, k_blk):
     got = host(d_sel)
     for t in list(range(16)) + [n_tok - 1]:
         assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, stride, k_blk, RATIO, pos0 + t, width)[0]), t
+
+
+@pytest.mark.parametrize("per,more", [(0, 1), (0, 33), (1, 0), (32, -1), (32, 1), (128, 0), (128, 1), (224, 1), (448, 0), (448, 1)])
+@pytest.mark.parametrize("n_head", [4, 3])
+def test_scores_of_one_token_at_the_edges_of_a_blocks_share(oracle, per, more, n_head):
+    """a block's share of the rows around one warp's, the line between one and two rows per lane, the last row that fits, and one
+    more; host position with hidden blocks behind, and the position word over a longer pool; NaN behind the visible rows"""
+    L = lib()
+    rows = per * torch.cuda.get_device_properties(0).multi_processor_count + more
+    rng = np.random.default_rng(rows)
+    pool = np.full((rows + 5, 128), np.nan, np.float32)
+    pool[:rows] = rng.standard_normal((rows, 128)).astype(np.float32)
+    q = rng.standard_normal((1, n_head, 128)).astype(np.float32)
+    pos = rows * RATIO + 2
+    want = oracle.ix_score(q, np.nan_to_num(pool), 1, rows + 3, rows + 5, n_head, pos, RATIO)[0]
+    d_q, d_pool = dev(q), dev(pool)
+    a, b = torch.full((rows + 5,), 7.0, device="cuda"), torch.full((rows + 5,), 7.0, device="cuda")
+    assert L.q4_hip_qsa_score(d_q.data_ptr(), d_pool.data_ptr(), a.data_ptr(), 1, rows + 3, rows + 5, n_head, 128, pos, RATIO)
+    L.q4_hip_pos_push(pos)
+    assert L.q4_hip_qsa_score_d(d_q.data_ptr(), d_pool.data_ptr(), b.data_ptr(), rows + 5, n_head, 128, RATIO)
+    a, b = host(a), host(b)
+    assert np.array_equal(a[:rows + 3].view(np.uint32), want[:rows + 3].view(np.uint32)) and (a[rows + 3:] == 7.0).all()
+    assert np.array_equal(b[:rows].view(np.uint32), want[:rows].view(np.uint32)) and (b[rows:] == 7.0).all()
