@@ -2435,11 +2435,26 @@ bool q4i_decode(const Q4DecodeArgs &a) {
     p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
     if (!a.new_k && q4i_f32_direct(a.layout == LAY_F32 ? Q4K_F32 : -1, a.hd, a.n_head, a.n_kvh, a.n_units, rows)) p.direct = 1u;
     dim3 grid(S, a.n_kvh, a.n_units);
+    Q4Touch t = {};
+    if (!a.many && !a.xchg && !a.scratch_part) {
+        const uint64_t heads_all = (uint64_t)a.n_units * a.n_head * a.hd, cache = a.one.layer_stride || a.new_k ? 0u : (uint64_t)a.one.max_kv * a.one.tok_stride;
+        t.reads(a.q, heads_all * (a.q_bf16 ? 2u : 4u));
+        t.reads(a.gate, heads_all * 4u);
+        t.reads(a.idx, ((uint64_t)(a.n_units - 1u) * a.idx_unit_stride + (uint64_t)(a.n_kvh - 1u) * a.idx_kvh_stride + a.width) * 4u);
+        t.add(a.one.k, cache, a.new_k != nullptr);   /* a store's planes end with their allocations */
+        t.add(a.one.v, cache, a.new_k != nullptr);
+        t.reads(a.new_k, (uint64_t)a.n_units * a.n_kvh * a.hd * 4u);
+        t.reads(a.new_v, (uint64_t)a.n_units * a.n_kvh * a.hd * 4u);
+        t.reads(a.pos, 4);
+        t.writes(a.out, heads_all * 4u);
+        t.writes(a.part_out, heads_all / a.hd * (a.hd + 2u) * 4u);
+    }
+    const Q4Touch *told = t.n ? &t : nullptr;
     switch (a.layout) {
-    case LAY_F32: return q4i_launched(launch_hd<LAY_F32>(p, grid, a.hd));
-    case LAY_F16: return q4i_launched(launch_hd<LAY_F16>(p, grid, a.hd));
-    case LAY_Q8P: return q4i_launched(launch_hd<LAY_Q8P>(p, grid, a.hd));
-    case LAY_Q8R: return q4i_launched(launch_hd<LAY_Q8R>(p, grid, a.hd));
+    case LAY_F32: return q4i_launched(launch_hd<LAY_F32>(p, grid, a.hd), told);
+    case LAY_F16: return q4i_launched(launch_hd<LAY_F16>(p, grid, a.hd), told);
+    case LAY_Q8P: return q4i_launched(launch_hd<LAY_Q8P>(p, grid, a.hd), told);
+    case LAY_Q8R: return q4i_launched(launch_hd<LAY_Q8R>(p, grid, a.hd), told);
     }
     return q4i_fail(Q4E_ARG, "decode: bad layout");
 }

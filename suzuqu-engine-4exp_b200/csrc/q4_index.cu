@@ -34,9 +34,10 @@ constexpr uint32_t IX_TK_THREADS = 1024, IX_MAX_KBLK = 512;
 /* ---- pool: one warp per block, lane l holds dims l, l+32, l+64, l+96 */
 __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *pool, const float *wn, uint32_t ratio,
                                                     uint32_t b0, uint32_t b1, uint32_t n_rot, float base, float eps,
-                                                    const int32_t *pp, bool early) {
+                                                    const int32_t *pp, bool early, bool apart) {
     const uint32_t lane = threadIdx.x & 31u, w = blockIdx.x * 4u + (threadIdx.x >> 5);
-    if (!early) q4d_pdl_wait();
+    if (apart) q4d_apart_begin();
+    else if (!early) q4d_pdl_wait();
     if (pp) {   /* device position: the block this token completes, if any */
         const uint32_t pos = (uint32_t)*pp;
         b0 = pos / ratio;
@@ -58,14 +59,17 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
             sn[c] = sinf(ang);
         }
     }
-    if (early) q4d_pdl_wait();
-    if (b >= b1) return;
+    if (early && !apart) q4d_pdl_wait();
+    if (b >= b1) {
+        if (apart) q4d_apart_end();
+        return;
+    }
     const __half *src = raw + (size_t)b * ratio * IX_HD;
     float v[4], r[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         float s = 0.f;
-        for (uint32_t j = 0; j < ratio; j++) s += __half2float(src[(size_t)j * IX_HD + lane + 32u * c]);
+        for (uint32_t j = 0; j < ratio; j++) s += __half2float(__ldcg(src + (size_t)j * IX_HD + lane + 32u * c));
         v[c] = __fdiv_rn(s, (float)ratio);
         r[c] = __fmul_rn(v[c], v[c]);
     }
@@ -90,6 +94,7 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
                             : __fsub_rn(__fmul_rn(v[c], cs[c]), __fmul_rn(other, sn[c]));
         pool[(size_t)b * IX_HD + d] = v[c];
     }
+    if (apart) q4d_apart_end();
 }
 
 /* ---- score: one thread per pooled block, 4 heads = 4 fused-multiply-add chains in dim order.
@@ -1343,20 +1348,36 @@ bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
     return topkc_start<8>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
 }
 
+bool pool_start(const char *what, uint32_t grid, const void *raw, float *pool, const float *wn, uint32_t ratio, uint32_t b0, uint32_t b1, uint32_t n_rot,
+                float base, float eps, const int32_t *pp) {
+    Q4Touch t = {};
+    const uint64_t row = (uint64_t)IX_HD * 2u * ratio;
+    if (pp) {
+        t.reads(raw, 0);
+        t.writes(pool, 0);
+    } else {
+        t.reads((const __half *)raw + (size_t)b0 * ratio * IX_HD, (b1 - b0) * row);
+        t.writes(pool + (size_t)b0 * IX_HD, (uint64_t)(b1 - b0) * IX_HD * 4u);
+    }
+    t.reads(wn, IX_HD * 4u);
+    t.reads(pp, 4);
+    const bool early = !pp || q4i_settled(g_q4.pos_written), apart = early && q4i_apart(t);
+    return q4i_launched(q4i_launch_dep(what, q4_ix_pool_k, dim3(grid), 128u, 0, (const __half *)raw, pool, wn, ratio, b0, b1, n_rot, base, eps, pp, early,
+                                       apart), &t, apart);
+}
+
 }  // namespace
 
 /* ======================================================================= reference ABI ===== */
 extern "C" bool q4_hip_qsa_pool(const void *raw_f16, float *pool, const float *wn, uint32_t hd, uint32_t ratio,
                                 uint32_t b0, uint32_t b1, uint32_t n_rot, float rope_base, float eps) {
     if (!g_q4.ok || !raw_f16 || !pool || b1 <= b0 || hd != IX_HD || ratio == 0) return false;
-    return q4i_launch_pdl("qsa_pool launch", q4_ix_pool_k, dim3((b1 - b0 + 3u) / 4u), 128u, 0, (const __half *)raw_f16, pool, wn, ratio, b0, b1,
-                          n_rot, rope_base, eps, (const int32_t *)nullptr, true);
+    return pool_start("qsa_pool launch", (b1 - b0 + 3u) / 4u, raw_f16, pool, wn, ratio, b0, b1, n_rot, rope_base, eps, nullptr);
 }
 extern "C" bool q4_hip_qsa_pool_d(const void *raw, float *pool, const float *wn, uint32_t hd, uint32_t ratio,
                                   uint32_t n_rot, float rope_base, float eps) {
     if (!g_q4.ok || !g_q4.pos_d || !raw || !pool || hd != IX_HD || ratio == 0) return false;
-    return q4i_launch_pdl("qsa_pool_d launch", q4_ix_pool_k, dim3(1), 128u, 0, (const __half *)raw, pool, wn, ratio, 0u, 0u, n_rot, rope_base, eps,
-                          (const int32_t *)g_q4.pos_d, q4i_settled(g_q4.pos_written));
+    return pool_start("qsa_pool_d launch", 1u, raw, pool, wn, ratio, 0u, 0u, n_rot, rope_base, eps, g_q4.pos_d);
 }
 extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks,
                                  uint32_t stride, uint32_t n_head, uint32_t hd, uint32_t pos0, uint32_t ratio) {

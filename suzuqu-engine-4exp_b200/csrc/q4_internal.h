@@ -59,6 +59,20 @@ inline bool q4i_f32_direct(int kind, uint32_t hd, uint32_t n_head, uint32_t n_kv
 
 struct Q4PtrList { void **p; uint32_t n; };
 
+/* Device memory that a launch reads and writes.  bytes == 0: to the end of p's allocation (a row whose place the device
+ * knows).  The status word, which launches only or bits into, and the library's scratch are left out. */
+struct Q4Touch {
+    struct { const void *p; uint64_t bytes; bool write; } r[12];
+    uint32_t n;
+    void reads(const void *p, uint64_t bytes) { add(p, bytes, false); }
+    void writes(const void *p, uint64_t bytes) { add(p, bytes, true); }
+    void add(const void *p, uint64_t bytes, bool write) {
+        if (!p) return;
+        r[n].p = p; r[n].bytes = bytes; r[n].write = write;
+        n++;
+    }
+};
+
 /* runtime state (q4_runtime.cu) */
 struct Q4State {
     bool ok;
@@ -73,8 +87,15 @@ struct Q4State {
      * Every kernel of the library either starts after its predecessor has finished, or waits for that before it lets its
      * successor start.  So what was written at least one library launch earlier is complete when a kernel starts:
      * `launches` counts them, the position word and the rows of a store remember the count at their last write, and
-     * `unsettled` is the count at the last event behind which nothing is known (a graph launch, another stream). */
-    uint64_t launches, pos_written, unsettled;
+     * `unsettled` is the count at the last event behind which nothing is known (a graph launch, another stream).
+     * A launch that runs apart (q4i_apart) is the exception: its successor may start before its predecessor has finished.
+     * `settled` is the count at the last launch that did not: what was written before that one is complete. */
+    uint64_t launches, settled, pos_written, unsettled;
+    /* in a capture: what the launches since may still be at (those numbered `settled` and up), and the node that the last of
+     * them left as the stream's only dependency */
+    struct { uint64_t number; Q4Touch touch; } flight[4];
+    uint32_t n_flight;
+    cudaGraphNode_t last_node;
     /* attention scratch: split-KV partial records + per-unit arrival counters */
     float *part;
     size_t part_floats;
@@ -90,11 +111,20 @@ extern Q4State g_q4;
 
 bool q4i_fail(uint32_t bit, const char *what);
 bool q4i_check(cudaError_t e, const char *what);
-inline bool q4i_launched(bool ok) {
-    if (ok) g_q4.launches++;
-    return ok;
+void q4i_in_capture(const Q4Touch *touch);
+inline bool q4i_launched(bool ok, const Q4Touch *touch = nullptr, bool apart = false) {
+    if (!ok) return false;
+    g_q4.launches++;
+    if (!apart) g_q4.settled = g_q4.launches;
+    if (g_q4.capturing) q4i_in_capture(touch);
+    return true;
 }
-inline bool q4i_settled(uint64_t written) { return g_q4.launches > written && g_q4.launches > g_q4.unsettled; }
+inline bool q4i_settled(uint64_t written) { return g_q4.settled > written && g_q4.settled > g_q4.unsettled; }
+/* Whether the next launch, which will touch `touch`, may run beside the ones before it: it is captured right behind them, and
+ * nothing that it writes is touched, and nothing that it reads is written, by any that may not have finished when it starts.
+ * Such a kernel lets its successor start at once, does its work, and waits for its predecessor before it ends
+ * (q4d_apart_begin / _end): whoever waits for it has waited for everything before it, as ever. */
+bool q4i_apart(const Q4Touch &touch);
 inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->writes->at[layer] = g_q4.launches; }
 bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside capture, fails inside */
 void q4i_give_back(void *p, bool captured);              /* cudaFree, now or with the last graph */
@@ -111,9 +141,13 @@ __device__ __forceinline__ void q4d_pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+/* A kernel that runs beside its predecessor (q4i_apart), in every thread, begin first and end last.  What it reads may have been
+ * written by the launch before last: by loads that do not look into L1. */
+__device__ __forceinline__ void q4d_apart_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void q4d_apart_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 /* host side: a launch that may start so (the kernel calls q4d_pdl_wait in every thread) */
 template <typename K, typename... A>
-bool q4i_launch_pdl(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
+bool q4i_launch_dep(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -124,7 +158,11 @@ bool q4i_launch_pdl(const char *what, K kernel, dim3 grid, uint32_t threads, siz
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return q4i_launched(q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), what));
+    return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), what);
+}
+template <typename K, typename... A>
+bool q4i_launch_pdl(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
+    return q4i_launched(q4i_launch_dep(what, kernel, grid, threads, smem, args...));
 }
 /* ---- the q8_0 quantiser, one copy for every kernel that writes a cache row.  8 lanes share a block
  * of 32 values (4 each): d = amax / 127 and id = 1 / d as IEEE fp32 divisions, codes =

@@ -57,11 +57,13 @@ __global__ void q4_f32_to_q8_k(const float *src, uint8_t *dst, uint64_t nblocks,
 
 template <bool DEP>
 __global__ void q4_f32_to_f16_k(const float *src, __half *dst, uint64_t n, const int32_t *pos,
-                                uint32_t stride) {
-    if (DEP) q4d_pdl_wait();
+                                uint32_t stride, bool apart) {
+    if (apart) q4d_apart_begin();
+    else if (DEP) q4d_pdl_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pos) dst += (size_t)(uint32_t)*pos * stride;
-    if (i < n) dst[i] = __float2half_rn(src[i]);
+    if (i < n) dst[i] = __float2half_rn(__ldcg(src + i));
+    if (apart) q4d_apart_end();
 }
 
 /* fp16 / fp32 rows of any length and alignment at the slot held in the device position word (the
@@ -198,12 +200,22 @@ inline int ref_layout(int kind) { return kind == Q4K_Q8 ? LAY_Q8R : kind == Q4K_
 bool launch_append(const AppendParams &p, int layout) {
     const uint64_t threads = (uint64_t)p.n_rows * p.n_kvh * (p.hd / 32u) * 8u;
     dim3 grid((unsigned)((threads + 255) / 256), 2);
-    switch (layout) {
-    case LAY_Q8P: return q4i_launch_pdl("append launch", q4_append_k<LAY_Q8P>, grid, 256u, 0, p);
-    case LAY_Q8R: return q4i_launch_pdl("append launch", q4_append_k<LAY_Q8R>, grid, 256u, 0, p);
-    case LAY_F16: return q4i_launch_pdl("append launch", q4_append_k<LAY_F16>, grid, 256u, 0, p);
+    Q4Touch t = {};
+    if (!p.many) {
+        const uint64_t in = (uint64_t)p.n_rows * p.n_kvh * p.hd * 4u;
+        t.reads(p.k, in);
+        t.reads(p.v, in);
+        t.reads(p.pos, 4);
+        t.writes(p.one.k, 0);
+        t.writes(p.one.v, 0);
     }
-    return q4i_launch_pdl("append launch", q4_append_k<LAY_F32>, grid, 256u, 0, p);
+    const Q4Touch *told = p.many ? nullptr : &t;
+    switch (layout) {
+    case LAY_Q8P: return q4i_launched(q4i_launch_dep("append launch", q4_append_k<LAY_Q8P>, grid, 256u, 0, p), told);
+    case LAY_Q8R: return q4i_launched(q4i_launch_dep("append launch", q4_append_k<LAY_Q8R>, grid, 256u, 0, p), told);
+    case LAY_F16: return q4i_launched(q4i_launch_dep("append launch", q4_append_k<LAY_F16>, grid, 256u, 0, p), told);
+    }
+    return q4i_launched(q4i_launch_dep("append launch", q4_append_k<LAY_F32>, grid, 256u, 0, p), told);
 }
 
 }  // namespace
@@ -229,15 +241,20 @@ extern "C" bool q4_hip_f32_to_f16(void *dst_f16, const float *src, uint64_t n) {
     if (!g_q4.ok || !dst_f16 || !src || !n) return false;
     const unsigned grid = (unsigned)((n + 255) / 256);
     if (grid > CONV_DEP_BLOCKS * (unsigned)g_q4.sm_count) {
-        q4_f32_to_f16_k<false><<<grid, 256, 0, g_q4.stream>>>(src, (__half *)dst_f16, n, nullptr, 0);
+        q4_f32_to_f16_k<false><<<grid, 256, 0, g_q4.stream>>>(src, (__half *)dst_f16, n, nullptr, 0, false);
         return q4i_launched(q4i_check(cudaGetLastError(), "f32_to_f16 launch"));
     }
-    return q4i_launch_pdl("f32_to_f16 launch", q4_f32_to_f16_k<true>, dim3(grid), 256u, 0, src, (__half *)dst_f16, n, (const int32_t *)nullptr, 0u);
+    return q4i_launch_pdl("f32_to_f16 launch", q4_f32_to_f16_k<true>, dim3(grid), 256u, 0, src, (__half *)dst_f16, n, (const int32_t *)nullptr, 0u, false);
 }
 extern "C" bool q4_hip_f32_to_f16_d(void *dst_base, uint32_t stride_elems, const float *src, uint64_t n) {
     if (!g_q4.ok || !g_q4.pos_d || !dst_base || !src || !n) return false;
-    return q4i_launch_pdl("f32_to_f16_d launch", q4_f32_to_f16_k<true>, dim3((unsigned)((n + 255) / 256)), 256u, 0, src, (__half *)dst_base, n,
-                          (const int32_t *)g_q4.pos_d, stride_elems);
+    Q4Touch t = {};
+    t.reads(src, n * 4u);
+    t.reads(g_q4.pos_d, 4);
+    t.writes(dst_base, 0);
+    const bool apart = q4i_settled(g_q4.pos_written) && q4i_apart(t);
+    return q4i_launched(q4i_launch_dep("f32_to_f16_d launch", q4_f32_to_f16_k<true>, dim3((unsigned)((n + 255) / 256)), 256u, 0, src, (__half *)dst_base, n,
+                                       (const int32_t *)g_q4.pos_d, stride_elems, apart), &t, apart);
 }
 /* The reference treats the token row as n flat floats at cache + pos*bpt; as a view that is one
  * kv head of width n. */
@@ -723,7 +740,8 @@ extern "C" bool q4_gpu_batch_advance(q4_gpu_batch *b, int32_t delta) {
     if (!g_q4.ok) return q4i_fail(Q4E_INIT, "batch_advance: library not initialised");
     Q4_REQUIRE(b && b->n_active, "batch_advance: no positions published (q4_gpu_batch_set_pos)");
     q4_batch_advance_k<<<(b->n_active + 127u) / 128u, 128, 0, g_q4.stream>>>(b->pos_d, b->n_active, delta);
-    b->pos_written = ++g_q4.launches;
+    (void)q4i_launched(true);
+    b->pos_written = g_q4.launches;
     if (!g_q4.capturing) b->max_pos = (uint32_t)((int64_t)b->max_pos + delta < 0 ? 0 : (int64_t)b->max_pos + delta);
     return q4i_check(cudaGetLastError(), "batch_advance launch");
 }

@@ -82,7 +82,7 @@ template <int HD>
 __device__ __forceinline__ void row_load(const float *src, float2 (&v)[HD / 64]) {
     const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
-    for (int k = 0; k < HD / 64; k++) v[k] = reinterpret_cast<const float2 *>(src)[32 * k + lane];
+    for (int k = 0; k < HD / 64; k++) v[k] = __ldcg(reinterpret_cast<const float2 *>(src) + 32 * k + lane);
 }
 /* RMSNorm and rotation in place.  Sum of squares as 128 threads of a block would take it: thread i adds elements i and
  * i + 128, a butterfly over each 32 threads, then the four totals in order (element 2 l + e of a register is thread
@@ -132,16 +132,16 @@ __device__ __forceinline__ void row_store(float *dst, const float2 (&v)[HD / 64]
 template <int HD, bool SPLIT, uint32_t TOK>
 __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *src, const float *wn, float *q, float *g, uint32_t n_rot,
                                                                   int32_t pos0, float base, float eps, uint32_t n_head, uint32_t per,
-                                                                  uint32_t n_tok, const int32_t *pp, bool early) {
+                                                                  uint32_t n_tok, const int32_t *pp, bool early, bool apart) {
     __shared__ float2 cs[TOK][128];
     constexpr uint32_t W = PREP_WARPS / TOK;   /* warps of a token */
     const uint32_t warp = threadIdx.x >> 5, sub = warp / W, t = blockIdx.y * TOK + sub, h0 = blockIdx.x * per, h1 = min(h0 + per, n_head);
-    if (!early) q4d_pdl_wait();
+    if (apart) q4d_apart_begin();
+    else if (!early) q4d_pdl_wait();
     rope_table(cs[sub], n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base, threadIdx.x % (W * 32u), W * 32u);   /* a settled position's under the previous kernel's tail */
-    if (early) q4d_pdl_wait();
+    if (early && !apart) q4d_pdl_wait();
     __syncthreads();
-    if (t >= n_tok) return;
-    for (uint32_t h = h0 + warp % W; h < h1; h += W) {
+    for (uint32_t h = h0 + warp % W; h < h1 && t < n_tok; h += W) {
         const size_t row = (size_t)t * n_head + h;
         float2 v[HD / 64];
         row_load<HD>(SPLIT ? src + row * 2u * HD : q + row * HD, v);
@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *s
         row_norm_rope<HD>(v, wn, cs[sub], n_rot / 2u, eps);
         row_store<HD>(q + row * HD, v);
     }
+    if (apart) q4d_apart_end();
 }
 
 /* false in `done` where the head size or an address is not the warp form's */
@@ -166,8 +167,17 @@ bool prep_rows(const float *src, const float *wn, float *q, float *g, uint32_t n
     const uint32_t per = n_tok < (uint32_t)g_q4.sm_count ? PREP_WARPS : n_head;
     const dim3 grid((n_head + per - 1u) / per, four ? (n_tok + 3u) / 4u : n_tok);
     const bool early = !pp || q4i_settled(g_q4.pos_written);
+    Q4Touch touch = {};
+    const uint64_t rows = (uint64_t)n_tok * n_head * hd * 4u;
+    touch.reads(src, 2u * rows);
+    touch.reads(wn, hd * 4u);
+    touch.reads(pp, 4);
+    touch.writes(q, rows);
+    touch.writes(g, rows);
+    const bool apart = early && q4i_apart(touch);
     auto start = [&](auto kernel) {
-        return q4i_launch_pdl("prep launch", kernel, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, n_tok, pp, early);
+        return q4i_launched(q4i_launch_dep("prep launch", kernel, grid, PREP_WARPS * 32u, 0, src, wn, q, g, n_rot, pos0, base, eps, n_head, per, n_tok, pp,
+                                           early, apart), &touch, apart);
     };
     if (hd == 64) return four ? start(q4_prep_rows_k<64, SPLIT, 4>) : start(q4_prep_rows_k<64, SPLIT, 1>);
     if (hd == 128) return four ? start(q4_prep_rows_k<128, SPLIT, 4>) : start(q4_prep_rows_k<128, SPLIT, 1>);
