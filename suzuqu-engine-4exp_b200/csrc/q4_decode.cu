@@ -629,6 +629,7 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
     constexpr uint32_t LANES = 16, PER = DEC_MAX_SPLIT / LANES;
     const uint32_t tasks = mo.gqa * CH, members = min(S, max(n_rec, tasks));
     if (split >= members) return;   /* neither a record nor a slice */
+    const bool slice = split < tasks;
     __shared__ uint32_t s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -642,13 +643,14 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
             *ctr = 0u;
             asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(flag), "r"(old + 1u) : "memory");
         }
-        for (uint32_t spins = 0; !met && spins < GRID_SPIN_LIMIT; spins++) {
+        for (uint32_t spins = 0; slice && !met && spins < GRID_SPIN_LIMIT; spins++) {
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
             met = seen != old;
         }
         s_ok = met ? 1u : 0u;
-        if (!met) atomicOr(err, (uint32_t)Q4E_CUDA);
+        if (slice && !met) atomicOr(err, (uint32_t)Q4E_CUDA);
     }
+    if (!slice) return;   /* its place is the next launch's */
     __syncthreads();
     const bool ok = s_ok != 0u;
     float *s_w = scr, *s_part = scr + 256, *s_red = scr + 256 + 16 * 32;
@@ -1009,8 +1011,11 @@ q4_decode_k(const DecParams P) {
     float4 ap_x = make_float4(0.f, 0.f, 0.f, 0.f);
     bool ap_which = false, ap_live = false;
     uint32_t ap_b = 0, ap_sub = 0;
+    /* A dense scan's newest row is in one split's slice, and only that one stores it: 222 blocks that wrote the same two lines
+     * held one another up behind the fence (262144 rows: a block's first tile 2.6 us after the wait, xx with one). */
+    const bool appends = APPENDS && P.new_k && (list || (newest < max_kv ? newest >> 4 >= s_begin && newest >> 4 < s_end : split == 0u));
     auto load_new = [&]() {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
-        if (P.new_k) {
+        if (appends) {
             constexpr uint32_t QL = HD / 4;
             const uint32_t tid = threadIdx.x;
             ap_which = tid >= QL;
@@ -1337,7 +1342,7 @@ q4_decode_k(const DecParams P) {
         auto first_positions = [&]() {
             pa = my_pos(0); pb = my_pos(1); pc = my_pos(2); pd = my_pos(3);
             pn0 = my_pos(4); pn1 = my_pos(5); pn2 = my_pos(6);
-            if (P.new_k) {
+            if (appends) {
                 const int32_t nw = (int32_t)newest;
                 hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
             }
@@ -1361,7 +1366,7 @@ q4_decode_k(const DecParams P) {
             load_new();
             request_q();
         }
-        if (P.new_k) {
+        if (appends) {
             float d, id;
             q4d_block_scale(ap_x, d, id);
             if (ap_live) {
@@ -1665,7 +1670,7 @@ q4_decode_k(const DecParams P) {
 #pragma unroll
             for (int i = 0; i < ST; i++) pf[i] = my_pos(i);
             pn0 = my_pos(ST); pn1 = my_pos(ST + 1); pn2 = my_pos(ST + 2);
-            if (P.new_k) {
+            if (appends) {
 #pragma unroll
                 for (int i = 0; i < ST; i++) hold = hold || pf[i] == (int32_t)newest;
                 hold = __any_sync(0xffffffffu, hold);
@@ -1688,7 +1693,7 @@ q4_decode_k(const DecParams P) {
             load_new();
             request_q();
         }
-        if (LAY != LAY_Q8R && P.new_k) {
+        if (LAY != LAY_Q8R && appends) {
             uint8_t *row = const_cast<uint8_t *>(ap_which ? vbase : kbase) + (uint64_t)newest * tok_stride;
             const uint32_t at = ap_b * 32 + ap_sub * 4;
             if (LAY == LAY_Q8P) {
