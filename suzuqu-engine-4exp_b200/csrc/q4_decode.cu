@@ -618,10 +618,11 @@ __device__ __noinline__ void cluster_push_merge(const float *own, const float *r
  * all (m, l) pairs and all accumulator pieces are requested at once, 16 record lanes x 8 threads of 4 dims (piece by
  * piece in a loop they took 7 us behind the last block at 262144 rows, 16 serial round trips).
  * `n_rec` records; every block with a record or a slice takes part (a launch sized for the store's capacity may have more
- * blocks than a short context needs).  The last to arrive re-arms the counter and turns the flag word, so nobody meets
- * again on the way out.  The wait is bounded. */
+ * blocks than a short context needs).  Arrivals are counted through from launch to launch, behind a word that holds the count
+ * before this one: nobody resets it, and only who has a slice waits (with a counter that the last to arrive reset, and a flag
+ * that it turned for the others, the records were met 2.2 to 4 us behind the last loop's end).  The wait is bounded. */
 constexpr uint32_t GRID_SPIN_LIMIT = 1u << 22;
-constexpr uint32_t DEC_CTR = 2u + DEC_MAX_SPLIT / DEC_GROUP;   /* words per unit: arrivals | arrivals per group | flag of the grid merge */
+constexpr uint32_t DEC_CTR = 3u + DEC_MAX_SPLIT / DEC_GROUP;   /* words per unit: arrivals | arrivals per group | the grid merge's arrivals before this launch, with it */
 template <int HD, int HEADS>
 __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t n_rec, uint32_t split, uint32_t *ctr, const MergeOut mo,
                                         float *scr /* >= 256 + 16 * 32 + 8 floats of shared memory */, uint32_t *err) {
@@ -632,20 +633,16 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
     const bool slice = split < tasks;
     __shared__ uint32_t s_ok;
     __syncthreads();
+    uint32_t before = 0;
     if (threadIdx.x == 0) {
-        uint32_t *flag = ctr + DEC_CTR - 1u;
-        uint32_t old, seen, prev;
-        asm volatile("ld.relaxed.gpu.u32 %0, [%1];" : "=r"(old) : "l"(flag) : "memory");
-        /* the block's records are ordered before this by the barrier above */
-        asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(prev) : "l"(ctr) : "memory");
-        bool met = prev == members - 1u;
-        if (met) {
-            *ctr = 0u;
-            asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(flag), "r"(old + 1u) : "memory");
-        }
+        uint32_t seen;
+        if (slice) asm volatile("ld.relaxed.gpu.u32 %0, [%1];" : "=r"(before) : "l"(ctr + DEC_CTR - 2u) : "memory");
+        /* the block's records are ordered before this by the barrier above, the load by the release */
+        asm volatile("red.release.gpu.add.u32 [%0], 1;" ::"l"(ctr + DEC_CTR - 1u) : "memory");
+        bool met = false;
         for (uint32_t spins = 0; slice && !met && spins < GRID_SPIN_LIMIT; spins++) {
-            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
-            met = seen != old;
+            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(ctr + DEC_CTR - 1u) : "memory");
+            met = seen - before == members;
         }
         s_ok = met ? 1u : 0u;
         if (slice && !met) atomicOr(err, (uint32_t)Q4E_CUDA);
@@ -715,6 +712,7 @@ __device__ __noinline__ void grid_merge(const float *recs, uint32_t S, uint32_t 
             }
             __syncthreads();
         }
+    if (split == 0u && threadIdx.x == 0) ctr[DEC_CTR - 2u] = before + members;   /* all have arrived: nobody reads it any more */
 }
 
 /* ---- exchange of the units' records between ranks (sequence-sharded decode) --------------------
@@ -1012,8 +1010,8 @@ q4_decode_k(const DecParams P) {
     bool ap_which = false, ap_live = false;
     uint32_t ap_b = 0, ap_sub = 0;
     /* A dense scan's newest row is in one split's slice, and only that one stores it: 222 blocks that wrote the same two lines
-     * held one another up behind the fence (262144 rows: a block's first tile 2.6 us after the wait, xx with one). */
-    const bool appends = APPENDS && P.new_k && (list || (newest < max_kv ? newest >> 4 >= s_begin && newest >> 4 < s_end : split == 0u));
+     * held one another up behind the fence (262144 rows: a block's loop began 2.6 us after the wait, 1.1 with one). */
+    const bool appends = APPENDS && P.new_k && (LIST || (newest < max_kv ? newest >> 4 >= s_begin && newest >> 4 < s_end : split == 0u));
     auto load_new = [&]() {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
         if (appends) {
             constexpr uint32_t QL = HD / 4;
