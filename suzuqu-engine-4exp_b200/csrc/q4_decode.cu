@@ -2491,7 +2491,7 @@ extern "C" bool q4_gpu_lse_merge(const float *parts, uint32_t n_parts, uint32_t 
 
 /* ---- decode without any allocation ------------------------------------------------------------
  * Scratch for the split-KV records lives in the library image itself: every GPU that loads the
- * library holds these 4 MB + 272 B until the process exits.  The names below are host-side stand-ins
+ * library holds these 4 MB + 304 B until the process exits.  The names below are host-side stand-ins
  * in host code; the device addresses come from cudaGetSymbolAddress, once per device. */
 constexpr size_t Q4_STATIC_PART_FLOATS = (size_t)1 << 20;   /* 4 MB of records */
 constexpr size_t Q4_STATIC_COUNTERS = 4 * DEC_CTR;   /* up to 4 kv heads */

@@ -30,8 +30,8 @@
  *     four buffers of 64 columns; both groups share every K/V tile.  NQ = 1: units are tiles of 128 positions, two
  *     buffers of 128 columns; two warps per 32 rows instead of one take the 2048-token prefill of the reference's host
  *     (24 / 2 heads of 256) from 2591 to 2340 us.  Tensor memory: 256 columns of scores, NQ x hd of O.
- *  3. Where blocks of one query group leave much of the last wave of SMs idle (a short chunk behind a long prefix), the
- *     positions are split over blockIdx.z; the blocks write (O, m, l) and q4_pf_merge_k combines them.
+ *  3. Where the last wave of blocks leaves much of the SMs idle, the positions of its blocks, or of all, are split over
+ *     several; those write (O, m, l) and q4_pf_merge_k combines them.
  *
  * Measured rates of tcgen05.mma with both operands in shared memory: 64 cycles per 128 x 128 x 16, 48 per 128 x 64 x 16
  * (4 KB of Q and 2 KB of K at 128 B/clk).  Single score buffers of 128 columns per group (all 512 columns in use as
@@ -71,7 +71,10 @@ struct PrefillParams {
     float scale_log2e;
     const uint8_t *kimg, *vimg;   /* operand images [kv head][tile][chunk][32 KB] */
     uint32_t img_tiles;           /* tiles per kv head in the images */
-    uint32_t n_split;             /* position ranges of equal tile count; > 1: partial results */
+    uint32_t n_groups;            /* blocks' worth of query groups per kv head; work items: kv head by kv head, last tokens first */
+    uint32_t n_whole, n_late, n_split;   /* items that are one block each; later ones, n_split blocks each, ranges of equal tile count */
+    uint32_t inv_groups, inv_late;       /* ceil(2^32 / n_groups), ceil(2^32 / n_late) */
+    uint32_t part_tok;            /* tokens below this may have parts */
     float *part;                  /* [split][token][head][hd] unnormalised O */
     float2 *part_ml;              /* [split][token][head] running max (log2 units), sum */
     const PfMark *marks;          /* [kv head][32 positions], of caches that are not the library's */
@@ -372,8 +375,10 @@ __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_a
     return false;
 }
 /* HD: head size; NQ: query groups per block; NP: images per 128 dims of K and V (2: value and remainder); MARKS: rows may
- * have been scaled or not be finite */
-template <int HD, int NQ, int NP, bool MARKS>
+ * have been scaled or not be finite; TAIL: the grid is a list of items, the last ones in ranges, else (groups, kv heads, ranges):
+ * where a block learns only when it runs whether it writes parts, one group's epilogue takes 0.6 us more (333 tokens 10.6 -> 11.2
+ * us), two groups' no more */
+template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
 __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParams P) {
     constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128;   /* ring slots a K / V tile takes */
     static_assert(NQ == 1 || NP == 1, "two groups hold a tile's V and the next one's K at once: both images of them leave the ring no slack");
@@ -386,19 +391,31 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     /* later token groups see more rows: launch them first so the tail of the grid is made of short blocks */
-    const uint32_t kh = blockIdx.y, t0 = (gridDim.x - 1u - blockIdx.x) * (P.tpc * NQ);
+    uint32_t kh = blockIdx.y, at = blockIdx.x, range = blockIdx.z, ranges = P.n_split;
+    if (TAIL) {
+        const bool late = blockIdx.x >= P.n_whole;
+        const uint32_t later = blockIdx.x - P.n_whole;
+        /* range by range: what runs at once reads the same tiles */
+        range = !late ? 0u : P.n_late == 1u ? later : __umulhi(later, P.inv_late);
+        ranges = late ? P.n_split : 1u;
+        const uint32_t item = late ? P.n_whole + later - range * P.n_late : blockIdx.x;
+        kh = P.n_groups == 1u ? item : __umulhi(item, P.inv_groups);
+        at = item - kh * P.n_groups;
+    }
+    const bool split = TAIL ? ranges > 1u : P.n_split > 1u;
+    const uint32_t t0 = (P.n_groups - 1u - at) * (P.tpc * NQ);
 
     /* 1024-byte aligned operand tiles (the swizzle pattern is anchored to the address) */
     const uint32_t sQ = (smem_u32(smem_dyn) + 1023u) & ~1023u, sR = sQ + PF_Q_BYTES, bars = sR + PF_RING * PF_CHUNK;
     const uint32_t full = bars, empty = bars + 40, bar_s = bars + 80, bar_p = bars + 112, bar_o = bars + 144,
-                   s_tmem = bars + 160, s_abort = bars + 164, s_xch = bars + 256;
+                   s_tmem = bars + 160, s_abort = bars + 164, s_item = bars + 176, s_xch = bars + 256;
 
     const uint32_t inv_gqa = 65536u / P.gqa + 1u;   /* row / gqa = row * inv_gqa >> 16 for rows below 128, gqa up to 16 */
     const uint32_t t_last = min(t0 + P.tpc * NQ, P.n_tok) - 1u;
     const uint32_t cta_nkv = min(P.kv_base + t_last + 1u, P.max_kv);
     const uint32_t all_tiles = (cta_nkv + PF_BN - 1u) / PF_BN;
     /* this block's range of tiles */
-    const uint32_t j0 = (uint32_t)((uint64_t)all_tiles * blockIdx.z / P.n_split), j1 = (uint32_t)((uint64_t)all_tiles * (blockIdx.z + 1u) / P.n_split);
+    const uint32_t j0 = all_tiles * range / ranges, j1 = all_tiles * (range + 1u) / ranges;   /* at most 2^25 tiles, 16 ranges */
     const uint32_t n_tiles = j1 - j0;
     /* units per group: the last tile may be needed in half only */
     const uint32_t n_seq = NQ == 2 ? min(n_tiles * 2u, (cta_nkv - j0 * PF_BN + 63u) / 64u) : n_tiles, n_units = n_seq * NQ;
@@ -418,6 +435,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
             mbar_init(bar_o, 1);
             mbar_init(bar_o + 8, 1);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(0u) : "memory");
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_item), "r"(t0), "r"(kh), "r"(range), "r"((uint32_t)split) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncwarp();
@@ -625,7 +643,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
         /* ================= softmax: thread r of group g owns row r of that group's queries; with one group, thread r of
          * half h owns 64 of a unit's positions of row r ================= */
         const uint32_t g = NQ == 2 ? warp >> 2 : 0u, h = NQ == 2 ? 0u : warp >> 2, r = tid & 127u, t_lane = tmem + (((warp & 3u) * 32u) << 16);
-        const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl, head = kh * P.gqa + r - tl * P.gqa;   /* rows past tpc * gqa or past n_tok are padding */
+        const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl;   /* rows past tpc * gqa or past n_tok are padding */
         const bool row_live = tl < P.tpc && tok < P.n_tok;
         /* this row attends positions [0, row_nkv); padding rows (queries of zeros, never stored) need no mask */
         const uint32_t row_nkv = row_live ? min(P.kv_base + tok + 1u, P.max_kv) : 0xffffffffu;
@@ -771,16 +789,21 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
          * ahead, the first ones under the last product (requested behind their use a block took 2600 cycles, most of it
          * their latency).  One group: each half takes half of the columns (a warp alone is held up in turn by its
          * special-function steps, 700 cycles a block, and its stores, 450). */
-        const bool split = P.n_split > 1u, gates = P.gate && !split;
+        /* two groups: which item this is was left in shared memory (kept in registers through the loop above it cost the softmax 4
+         * to 8 %; one group has registers to spare) */
+        uint32_t e_t0 = t0, e_kh = kh, e_range = range, e_split = split;
+        if (NQ == 2)
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(e_t0), "=r"(e_kh), "=r"(e_range), "=r"(e_split) : "r"(s_item) : "memory");
+        const bool parts = TAIL ? e_split != 0u : P.n_split > 1u, gates = P.gate && !parts;
         const uint32_t w_row0 = (warp & 3u) * 32u;
         uint32_t off[8], live = 0;   /* in 16-byte units from the chunk's first token */
 #pragma unroll
         for (int q = 0; q < 8; q++) {
             const uint32_t row = w_row0 + 4u * q + (lane >> 3), ti = row * inv_gqa >> 16;
-            if (ti < P.tpc && t0 + g * P.tpc + ti < P.n_tok) live |= 1u << q;
-            off[q] = ((g * P.tpc + ti) * P.n_head + kh * P.gqa + (row - ti * P.gqa)) * (HD / 4u) + (lane & 7u);
+            if (ti < P.tpc && e_t0 + g * P.tpc + ti < P.n_tok) live |= 1u << q;
+            off[q] = ((g * P.tpc + ti) * P.n_head + e_kh * P.gqa + (row - ti * P.gqa)) * (HD / 4u) + (lane & 7u);
         }
-        const size_t first = (size_t)t0 * P.n_head * (HD / 4u);
+        const size_t first = (size_t)e_t0 * P.n_head * (HD / 4u);
         auto fetch_gates = [&](int c, float4 (&to)[8]) {
 #pragma unroll
             for (int q = 0; q < 8; q++)
@@ -795,10 +818,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
         tc_fence_after();
 
         if (ok) {
-            const float inv = split ? 1.f : l_run > 0.f ? 1.f / l_run : 0.f;
+            const float inv = parts ? 1.f : l_run > 0.f ? 1.f / l_run : 0.f;
             float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + warp * (PF_Q_BYTES / SW));   /* [32][36] */
-            if (split && row_live && h == 0)
-                P.part_ml[((size_t)blockIdx.z * P.n_tok + tok) * P.n_head + head] = make_float2(m_ref, l_run);
+            const uint32_t etl = r * inv_gqa >> 16, etok = e_t0 + g * P.tpc + etl;
+            if (parts && etl < P.tpc && etok < P.n_tok && h == 0)
+                P.part_ml[((size_t)e_range * P.part_tok + etok) * P.n_head + e_kh * P.gqa + (r - etl * P.gqa)] = make_float2(m_ref, l_run);
             auto columns = [&](int c, float4 (&gs)[8]) {
                 float o[32];
                 if (n_tiles > 0) {
@@ -823,10 +847,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
                         x[q].z = gated(x[q].z, gs[q].z); x[q].w = gated(x[q].w, gs[q].w);
                     }
                 }
-                if (split) {
+                if (parts) {
 #pragma unroll
                     for (int q = 0; q < 8; q++)
-                        if ((live >> q) & 1u) reinterpret_cast<float4 *>(P.part)[(size_t)blockIdx.z * P.n_tok * P.n_head * (HD / 4u) + first + off[q] + 8u * c] = x[q];
+                        if ((live >> q) & 1u) reinterpret_cast<float4 *>(P.part)[(size_t)e_range * P.part_tok * P.n_head * (HD / 4u) + first + off[q] + 8u * c] = x[q];
                 } else if (P.out_bf16) {
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
@@ -857,11 +881,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
 }
 
 /* ---- the parts of split position ranges -> out: thread = 4 dims of one (token, head) */
-__global__ void __launch_bounds__(256) q4_pf_merge_k(const PrefillParams P, uint32_t hd, uint64_t total4) {
+__global__ void __launch_bounds__(256) q4_pf_merge_k(const PrefillParams P, uint32_t hd, uint64_t total4, uint32_t tok_per_group) {
     const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
     q4d_pdl_wait();
     if (i >= total4) return;
-    const uint64_t row = i / (hd / 4u), rows = (uint64_t)P.n_tok * P.n_head;
+    const uint64_t row = i / (hd / 4u), rows = (uint64_t)P.part_tok * P.n_head;
+    const uint32_t tok = (uint32_t)(row / P.n_head), head = (uint32_t)(row % P.n_head);
+    if (head / P.gqa * P.n_groups + (P.n_groups - 1u - tok / tok_per_group) < P.n_whole) return;   /* one block's, finished */
     float M = -CUDART_INF_F;
     for (uint32_t s = 0; s < P.n_split; s++) M = fmaxf(M, P.part_ml[s * rows + row].x);
     const float Mu = M == -CUDART_INF_F ? 0.f : M;
@@ -919,39 +945,60 @@ int stage_reserve(size_t bytes) {
     return -1;
 }
 
-template <int HD, int NQ, int NP, bool MARKS>
+template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
 bool attend(const PrefillParams &p, dim3 grid) {
     static bool attr = false;
-    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP, MARKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
+    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
                             "prefill smem attribute"))
         return false;
     attr = true;
-    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP, MARKS>, grid, PF_THREADS, PF_SMEM, p);
+    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, grid, PF_THREADS, PF_SMEM, p);
+}
+template <int HD, int NP, bool MARKS>
+bool attend_one(const PrefillParams &p, uint32_t n_kvh) {
+    if (p.n_whole && p.n_late) return attend<HD, 1, NP, MARKS, true>(p, dim3(p.n_whole + p.n_late * p.n_split));
+    return attend<HD, 1, NP, MARKS, false>(p, dim3(p.n_groups, n_kvh, p.n_split));
 }
 template <int LAY, int HD, int NP>
 bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg, PfMark *marks, uint8_t *flags) {
     return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, NP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg, marks, flags);
 }
 
-/* Ranges of positions that a chunk's blocks of one query group are split into: the count with the least estimated time,
- * waves x (tiles of a range + what a block takes besides) + the merge with its traffic.  In ns, from chunks of 33 to 1500
+/* Which blocks' positions are split, and into how many ranges: the choice with the least estimated time, waves x (tiles of a
+ * range + what a block takes besides) + the merge with its traffic.  In ns, one group per block, from chunks of 33 to 1500
  * tokens over 0 to 16 384: a tile 1.0 us at hd 128, 2.2 at 256 with both images; a block 4 and 6 us besides; the merge
- * 1.2 us, 0.2 per range, and 7 KB per ns.  600 tokens over 16 384 (76 blocks): 146 us in one range, 112 in three. */
-uint32_t best_split(uint32_t blocks, uint32_t sms, uint32_t tiles, uint64_t rows, uint32_t hd, uint32_t np) {
-    const uint64_t tile = 640u + 190u * (hd / 128u) * 2u * np, block = 2000u + 2000u * (hd / 128u);
-    uint64_t best = 0;
-    uint32_t split = 1;
-    for (uint32_t s = 1; s <= 16u && s <= tiles; s++) {
-        const uint64_t waves = ((uint64_t)blocks * s + sms - 1u) / sms;
-        uint64_t t = waves * ((tiles + s - 1u) / s * tile + block);
-        if (s > 1) t += 1200u + 200u * s + rows * hd * s * 8u / 7000u;
-        if (s == 1) best = t - t / 16u;   /* one range needs no merge: left for a clear gain only (causal chunks have less work) */
-        else if (t < best) {
-            best = t;
-            split = s;
+ * 1.2 us, 0.2 per range, and 7 KB per ns.  600 tokens over 16 384 (76 blocks): 146 us in one range, 112 in three.
+ * Two groups per block: a tile 1.8 us, a block 5.  There, and with more blocks than SMs, only those of the last wave are split,
+ * the shortest of the chunk: 8192 tokens over 16 384 are 512 blocks, 444 and 68 x 2. */
+struct PfSplit { uint32_t whole, ranges; };
+PfSplit best_split(uint32_t groups, uint32_t n_kvh, uint32_t sms, uint32_t kv_base, uint32_t tok_per_group, uint32_t tiles, uint32_t rows_per_group, uint32_t hd,
+                   uint32_t np, uint32_t nq) {
+    const uint32_t blocks = groups * n_kvh, waves = blocks / sms, rest = blocks % sms;
+    const uint64_t tile = nq == 2 ? 1800u : 640u + 190u * (hd / 128u) * 2u * np, block = nq == 2 ? 5000u : 2000u + 2000u * (hd / 128u);
+    auto merge = [&](uint32_t items, uint32_t s) -> uint64_t { return 1200u + 200u * s + (uint64_t)items * rows_per_group * hd * s * 8u / 7000u; };
+    PfSplit r = {blocks, 1u};
+    const uint64_t whole = (waves + (rest != 0u)) * (tiles * tile + block);
+    uint64_t best = whole - whole / 16u;   /* whole blocks need no merge: left for a clear gain only (causal chunks have less work) */
+    for (uint32_t s = 2; s <= 16u && s <= tiles; s++) {
+        if (nq == 1) {
+            const uint64_t t = ((uint64_t)blocks * s + sms - 1u) / sms * ((tiles + s - 1u) / s * tile + block) + merge(blocks, s);
+            if (t < best) {
+                best = t;
+                r = {0u, s};
+            }
+        }
+        /* The last wave's blocks are the last kv head's first tokens.  Where they are much shorter than the chunk's last tokens', as
+         * without a prefix, the blocks before them end so far apart that they fill the gaps (8192 tokens over none 240 us, split 255). */
+        const uint32_t seen = (kv_base + (rest < groups ? rest : groups) * tok_per_group + PF_BN - 1u) / PF_BN, n = seen < tiles ? seen : tiles;
+        if (waves && rest && rest * s <= sms && n >= 2u * (tiles - kv_base / PF_BN)) {
+            const uint64_t t = waves * (tiles * tile + block) + (n + s - 1u) / s * tile + block + merge(rest, s), now = waves * (tiles * tile + block) + n * tile + block;
+            if (t < best && t < now) {
+                best = t;
+                r = {blocks - rest, s};
+            }
         }
     }
-    return split;
+    return r;
 }
 
 }  // namespace
@@ -973,12 +1020,24 @@ int q4i_prefill(const Q4PrefillArgs &a) {
      * waves: 1000 tokens over 4000 (126 blocks) 52 against 83 us, 2500 over 16 384 (314) 450 against 505, 3600 (450) 643
      * against 591; between 300 and 400 it depends on the depth. */
     const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
-    const uint32_t blocks = (groups + nq - 1u) / nq * a.n_kvh;
-    uint32_t split = nq == 1 ? best_split(blocks, sms, tiles, (uint64_t)a.n_tok * a.n_head, hd, np) : 1u;
+    const uint32_t n_groups = (groups + nq - 1u) / nq, tok_per_group = tpc * nq, blocks = n_groups * a.n_kvh;
     const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes, m_bytes = (size_t)a.n_kvh * tiles * (PF_BN / 32u) * (sizeof(PfMark) + 4u);   /* marks, flags (two bytes used per mark) */
-    const size_t rows = (size_t)a.n_tok * a.n_head, part_bytes = split > 1 ? split * rows * hd * sizeof(float) : 0;
-    const int room = stage_reserve(k_bytes + v_bytes + m_bytes + part_bytes + (split > 1 ? split * rows * sizeof(float2) : 0));
+    PfSplit sp = best_split(n_groups, a.n_kvh, sms, a.kv_base, tok_per_group, tiles, tok_per_group * gqa, hd, np, nq);
+    uint32_t part_tok;
+    size_t rows, part_bytes;
+    int room;
+    for (;; sp = {blocks, 1u}) {
+        /* tokens that parts are kept for: those of the groups at the end of the order */
+        const uint32_t late = blocks - sp.whole;
+        const uint64_t late_tok = (uint64_t)(late < n_groups ? late : n_groups) * tok_per_group;
+        part_tok = (uint32_t)(late_tok < a.n_tok ? late_tok : a.n_tok);
+        rows = (size_t)part_tok * a.n_head;
+        part_bytes = sp.ranges * rows * hd * sizeof(float);
+        room = stage_reserve(k_bytes + v_bytes + m_bytes + part_bytes + sp.ranges * rows * sizeof(float2));
+        if (room != -1 || sp.ranges == 1u) break;   /* no room for parts: whole blocks need none */
+    }
     if (room != 1) return room;
+    const uint32_t split = sp.ranges;
 
     PrefillParams p;
     memset(&p, 0, sizeof(p));
@@ -988,7 +1047,10 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     p.scale_log2e = a.scale * 1.4426950408889634f;
     uint8_t *kimg = g_stage, *vimg = g_stage + k_bytes;
     p.kimg = kimg; p.vimg = vimg; p.img_tiles = tiles;
-    p.n_split = split;
+    p.n_groups = n_groups; p.n_whole = sp.whole; p.n_late = blocks - sp.whole; p.n_split = split; p.part_tok = part_tok;
+    auto inverse = [](uint32_t n) { return n ? (uint32_t)((0x100000000ull + n - 1u) / n) : 0u; };   /* quotients of x are exact while x n < 2^32 */
+    p.inv_groups = inverse(n_groups);
+    p.inv_late = inverse(p.n_late);
     PfMark *marks = reinterpret_cast<PfMark *>(g_stage + k_bytes + v_bytes);
     uint8_t *flags = reinterpret_cast<uint8_t *>(marks + (size_t)a.n_kvh * tiles * (PF_BN / 32u));
     p.marks = marks;
@@ -1003,14 +1065,18 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     else if (a.layout == LAY_F16) ok = hd == 128 ? stage<LAY_F16, 128, 1>(a, n, tiles, kimg, vimg, marks, flags) : stage<LAY_F16, 256, 1>(a, n, tiles, kimg, vimg, marks, flags);
     else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, kimg, vimg, marks, flags) : stage<LAY_F32, 256, 1>(a, n, tiles, kimg, vimg, marks, flags);
     if (!ok) return 0;
-    const dim3 grid((groups + nq - 1u) / nq, a.n_kvh, split);
     const bool own = a.layout == LAY_Q8P;
-    if (hd == 256) ok = np == 2 ? attend<256, 1, 2, true>(p, grid) : attend<256, 1, 1, true>(p, grid);
-    else if (nq == 2) ok = own ? attend<128, 2, 1, false>(p, grid) : attend<128, 2, 1, true>(p, grid);
-    else ok = np == 2 ? attend<128, 1, 2, true>(p, grid) : own ? attend<128, 1, 1, false>(p, grid) : attend<128, 1, 1, true>(p, grid);
+    if (nq == 2) {
+        const dim3 grid(p.n_whole + p.n_late * split);
+        ok = own ? attend<128, 2, 1, false, true>(p, grid) : attend<128, 2, 1, true, true>(p, grid);
+    } else if (hd == 256) {
+        ok = np == 2 ? attend_one<256, 2, true>(p, a.n_kvh) : attend_one<256, 1, true>(p, a.n_kvh);
+    } else {
+        ok = np == 2 ? attend_one<128, 2, true>(p, a.n_kvh) : own ? attend_one<128, 1, false>(p, a.n_kvh) : attend_one<128, 1, true>(p, a.n_kvh);
+    }
     if (ok && split > 1) {
         const uint64_t total4 = (uint64_t)rows * hd / 4u;
-        ok = q4i_launch_pdl("prefill launch", q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4);
+        ok = q4i_launch_pdl("prefill launch", q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4, tok_per_group);
     }
     return ok ? 1 : 0;
 }

@@ -485,8 +485,8 @@ extern "C" bool q4_gpu_pipe_sync(q4_gpu_pipe *p) {
 
 extern "C" bool q4_hip_qsa_topk_alloc(void) {
     if (!g_q4.ok) return false;
-    /* 32 MB of records + 64 Ki counters: one session at the largest supported shape (4 kv heads x
+    /* 32 MB of records + 72 Ki counters (19 per unit and kv head): one session at the largest supported shape (4 kv heads x
      * 272 records x 16 heads x 258 floats) or a batch of a few hundred sessions at the usual one;
      * the same role as g_attn_part, src/q4_rocm.cu:7705-7706 */
-    return q4i_scratch((size_t)8 << 20, (size_t)64 << 10);
+    return q4i_scratch((size_t)8 << 20, (size_t)72 << 10);
 }

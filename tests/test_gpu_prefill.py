@@ -423,3 +423,27 @@ def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle, size
     ref = oracle.attn(q, kc, vc, g, n_head, n_kvh, hd, n_tok, kv_base, n, 1.0 / 16.0, 2, threads=8)
     assert_close(got, ref, "captured chunk")
     assert L.q4_gpu_last_error() == 0
+
+
+@pytest.mark.parametrize("n_head,n_kvh,n_tok,kv_base", [(16, 2, 3000, 0), (16, 2, 3000, 2100), (16, 2, 5003, 37), (16, 2, 1300, 1500), (16, 1, 4900, 300), (9, 3, 2600, 900),
+                                                        (64, 4, 1205, 500)])
+def test_last_wave_in_ranges_of_positions(n_head, n_kvh, n_tok, kv_base):
+    """chunks of one to three waves of blocks and a remainder, whose blocks are split; against chunks of 200 tokens, which are
+    other blocks in other ranges, each within the tolerance of the oracle's tests.  And as many bytes again behind the output."""
+    L = lib()
+    hd, ctx = 128, kv_base + n_tok
+    g = torch.Generator(device="cuda").manual_seed(n_tok)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    st = q4gpu.KVStore(1, n_kvh, hd, ctx, 2)
+    st.append(0, rn(ctx, n_kvh * hd), rn(ctx, n_kvh * hd), 0, ctx)
+    q, gate = rn(n_tok, n_head, hd).bfloat16(), rn(n_tok, n_head, hd)
+    out = torch.full((2 * n_tok, n_head, hd), 7.0, dtype=torch.bfloat16, device="cuda")
+    ref = torch.empty(n_tok, n_head, hd, dtype=torch.bfloat16, device="cuda")
+    st.prefill(0, q, out, n_head, n_tok, kv_base, 1 / np.sqrt(hd), gate=gate)
+    for t in range(0, n_tok, 200):
+        m = min(200, n_tok - t)
+        st.prefill(0, q[t:], ref[t:], n_head, m, kv_base + t, 1 / np.sqrt(hd), gate=gate[t:])
+    got = host(out.float())
+    check(got[:n_tok], host(ref.float()), "tail %d over %d" % (n_tok, kv_base))
+    assert (got[n_tok:] == 7.0).all() and L.q4_gpu_last_error() == 0
+    st.close()
