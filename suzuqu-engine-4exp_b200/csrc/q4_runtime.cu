@@ -50,7 +50,7 @@ void q4i_give_back(void *p, bool captured) {
  * launches, so there alone they are looked at.  With pooling, the fp16 key, and the second of two neighbouring norms apart from
  * the launch before them: the reference host's token at 32768 390 -> 371 us per 12 layers, a 262144-token step with selection
  * 341 -> 315. */
-/* the end of the allocation that p points into; none where it is mapped piece by piece or not the driver's at all */
+/* the end of the allocation that p points into; none where it is mapped piece by piece or not device memory at all */
 static uintptr_t allocation_end(const void *p) {
     typedef int (*GetRange)(unsigned long long *, size_t *, unsigned long long);
     typedef int (*Retain)(unsigned long long *, void *);
