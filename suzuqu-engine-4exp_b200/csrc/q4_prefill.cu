@@ -73,7 +73,6 @@ struct PrefillParams {
     uint32_t img_tiles;           /* tiles per kv head in the images */
     uint32_t n_groups;            /* blocks' worth of query groups per kv head; work items: kv head by kv head, last tokens first */
     uint32_t n_whole, n_late, n_split;   /* items that are one block each; later ones, n_split blocks each, ranges of equal tile count */
-    uint32_t inv_groups, inv_late;       /* ceil(2^32 / n_groups), ceil(2^32 / n_late) */
     uint32_t part_tok;            /* tokens below this may have parts */
     float *part;                  /* [split][token][head][hd] unnormalised O */
     float2 *part_ml;              /* [split][token][head] running max (log2 units), sum */
@@ -393,14 +392,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
     /* later token groups see more rows: launch them first so the tail of the grid is made of short blocks */
     uint32_t kh = blockIdx.y, at = blockIdx.x, range = blockIdx.z, ranges = P.n_split;
     if (TAIL) {
-        const bool late = blockIdx.x >= P.n_whole;
-        const uint32_t later = blockIdx.x - P.n_whole;
-        /* range by range: what runs at once reads the same tiles */
-        range = !late ? 0u : P.n_late == 1u ? later : __umulhi(later, P.inv_late);
-        ranges = late ? P.n_split : 1u;
-        const uint32_t item = late ? P.n_whole + later - range * P.n_late : blockIdx.x;
-        kh = P.n_groups == 1u ? item : __umulhi(item, P.inv_groups);
-        at = item - kh * P.n_groups;
+        const Q4PfItem it = q4i_pf_item(blockIdx.x, P.n_groups, P.n_whole, P.n_late, P.n_split);
+        kh = it.kh;
+        at = it.group;
+        range = it.range;
+        ranges = it.ranges;
     }
     const bool split = TAIL ? ranges > 1u : P.n_split > 1u;
     const uint32_t t0 = (P.n_groups - 1u - at) * (P.tpc * NQ);
@@ -1048,9 +1044,6 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     uint8_t *kimg = g_stage, *vimg = g_stage + k_bytes;
     p.kimg = kimg; p.vimg = vimg; p.img_tiles = tiles;
     p.n_groups = n_groups; p.n_whole = sp.whole; p.n_late = blocks - sp.whole; p.n_split = split; p.part_tok = part_tok;
-    auto inverse = [](uint32_t n) { return n ? (uint32_t)((0x100000000ull + n - 1u) / n) : 0u; };   /* quotients of x are exact while x n < 2^32 */
-    p.inv_groups = inverse(n_groups);
-    p.inv_late = inverse(p.n_late);
     PfMark *marks = reinterpret_cast<PfMark *>(g_stage + k_bytes + v_bytes);
     uint8_t *flags = reinterpret_cast<uint8_t *>(marks + (size_t)a.n_kvh * tiles * (PF_BN / 32u));
     p.marks = marks;
