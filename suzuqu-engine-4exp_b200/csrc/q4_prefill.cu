@@ -44,6 +44,7 @@
 #include <cuda_bf16.h>
 #include <math_constants.h>
 #include <string.h>
+#include <type_traits>
 
 #include "q4_internal.h"
 
@@ -71,14 +72,17 @@ struct PrefillParams {
     float scale_log2e;
     const uint8_t *kimg, *vimg;   /* operand images [kv head][tile][chunk][32 KB] */
     uint32_t img_tiles;           /* tiles per kv head in the images */
-    uint32_t n_groups;            /* blocks' worth of query groups per kv head; work items: kv head by kv head, last tokens first */
-    uint32_t n_whole, n_late, n_split;   /* items that are one block each; later ones, n_split blocks each, ranges of equal tile count */
-    uint32_t part_tok;            /* tokens below this may have parts */
+    uint32_t n_split;             /* position ranges of equal tile count of the items that are split; > 1: partial results */
     float *part;                  /* [split][token][head][hd] unnormalised O */
     float2 *part_ml;              /* [split][token][head] running max (log2 units), sum */
     const PfMark *marks;          /* [kv head][32 positions], of caches that are not the library's */
     const uint32_t *flags;        /* [kv head][64 positions]: bytes that are not zero where K or V of 32 of them is marked */
     uint32_t *err;
+};
+struct PrefillTail : PrefillParams {
+    uint32_t n_groups;            /* blocks' worth of query groups per kv head; work items: kv head by kv head, last tokens first */
+    uint32_t n_whole, n_late;     /* items that are one block each; later ones, n_split blocks each */
+    uint32_t part_tok;            /* tokens below this may have parts */
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -376,9 +380,10 @@ __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_a
 /* HD: head size; NQ: query groups per block; NP: images per 128 dims of K and V (2: value and remainder); MARKS: rows may
  * have been scaled or not be finite; TAIL: the grid is a list of items, the last ones in ranges, else (groups, kv heads, ranges):
  * where a block learns only when it runs whether it writes parts, one group's epilogue takes 0.6 us more (333 tokens 10.6 -> 11.2
- * us), two groups' no more */
+ * us), two groups' no more.  Only the list's launches carry its numbers: with 16 bytes more of parameters the other forms were
+ * compiled to 1 to 6 % slower code (24 / 2 heads of 256, fp16, 1500 tokens 62.5 -> 65.4 us). */
 template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
-__global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParams P) {
+__global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditional_t<TAIL, PrefillTail, PrefillParams> P) {
     constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128;   /* ring slots a K / V tile takes */
     static_assert(NQ == 1 || NP == 1, "two groups hold a tile's V and the next one's K at once: both images of them leave the ring no slack");
     constexpr uint32_t SW = 8;                                 /* softmax warps; then the issuer, then the producer */
@@ -390,16 +395,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     /* later token groups see more rows: launch them first so the tail of the grid is made of short blocks */
-    uint32_t kh = blockIdx.y, at = blockIdx.x, range = blockIdx.z, ranges = P.n_split;
-    if (TAIL) {
+    uint32_t kh = blockIdx.y, t0 = (gridDim.x - 1u - blockIdx.x) * (P.tpc * NQ), range = 0, ranges = 1;
+    if constexpr (TAIL) {
         const Q4PfItem it = q4i_pf_item(blockIdx.x, P.n_groups, P.n_whole, P.n_late, P.n_split);
         kh = it.kh;
-        at = it.group;
+        t0 = (P.n_groups - 1u - it.group) * (P.tpc * NQ);
         range = it.range;
         ranges = it.ranges;
     }
-    const bool split = TAIL ? ranges > 1u : P.n_split > 1u;
-    const uint32_t t0 = (P.n_groups - 1u - at) * (P.tpc * NQ);
 
     /* 1024-byte aligned operand tiles (the swizzle pattern is anchored to the address) */
     const uint32_t sQ = (smem_u32(smem_dyn) + 1023u) & ~1023u, sR = sQ + PF_Q_BYTES, bars = sR + PF_RING * PF_CHUNK;
@@ -411,7 +414,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
     const uint32_t cta_nkv = min(P.kv_base + t_last + 1u, P.max_kv);
     const uint32_t all_tiles = (cta_nkv + PF_BN - 1u) / PF_BN;
     /* this block's range of tiles */
-    const uint32_t j0 = all_tiles * range / ranges, j1 = all_tiles * (range + 1u) / ranges;   /* at most 2^25 tiles, 16 ranges */
+    const uint32_t j0 = TAIL ? all_tiles * range / ranges : (uint32_t)((uint64_t)all_tiles * blockIdx.z / P.n_split);   /* at most 2^25 tiles, 16 ranges */
+    const uint32_t j1 = TAIL ? all_tiles * (range + 1u) / ranges : (uint32_t)((uint64_t)all_tiles * (blockIdx.z + 1u) / P.n_split);
     const uint32_t n_tiles = j1 - j0;
     /* units per group: the last tile may be needed in half only */
     const uint32_t n_seq = NQ == 2 ? min(n_tiles * 2u, (cta_nkv - j0 * PF_BN + 63u) / 64u) : n_tiles, n_units = n_seq * NQ;
@@ -431,7 +435,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
             mbar_init(bar_o, 1);
             mbar_init(bar_o + 8, 1);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(s_abort), "r"(0u) : "memory");
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_item), "r"(t0), "r"(kh), "r"(range), "r"((uint32_t)split) : "memory");
+            if (TAIL) asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(s_item), "r"(t0), "r"(kh), "r"(range), "r"((uint32_t)(ranges > 1u)) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncwarp();
@@ -639,7 +643,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
         /* ================= softmax: thread r of group g owns row r of that group's queries; with one group, thread r of
          * half h owns 64 of a unit's positions of row r ================= */
         const uint32_t g = NQ == 2 ? warp >> 2 : 0u, h = NQ == 2 ? 0u : warp >> 2, r = tid & 127u, t_lane = tmem + (((warp & 3u) * 32u) << 16);
-        const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl;   /* rows past tpc * gqa or past n_tok are padding */
+        const uint32_t tl = r * inv_gqa >> 16, tok = t0 + g * P.tpc + tl, head = kh * P.gqa + r - tl * P.gqa;   /* rows past tpc * gqa or past n_tok are padding */
         const bool row_live = tl < P.tpc && tok < P.n_tok;
         /* this row attends positions [0, row_nkv); padding rows (queries of zeros, never stored) need no mask */
         const uint32_t row_nkv = row_live ? min(P.kv_base + tok + 1u, P.max_kv) : 0xffffffffu;
@@ -787,7 +791,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
          * special-function steps, 700 cycles a block, and its stores, 450). */
         /* two groups: which item this is was left in shared memory (kept in registers through the loop above it cost the softmax 4
          * to 8 %; one group has registers to spare) */
-        uint32_t e_t0 = t0, e_kh = kh, e_range = range, e_split = split;
+        uint32_t e_t0 = t0, e_kh = kh, e_range = TAIL ? range : blockIdx.z, e_split = ranges > 1u;
         if (NQ == 2)
             asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(e_t0), "=r"(e_kh), "=r"(e_range), "=r"(e_split) : "r"(s_item) : "memory");
         const bool parts = TAIL ? e_split != 0u : P.n_split > 1u, gates = P.gate && !parts;
@@ -816,9 +820,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
         if (ok) {
             const float inv = parts ? 1.f : l_run > 0.f ? 1.f / l_run : 0.f;
             float *buf = reinterpret_cast<float *>(smem_dyn + (sQ - smem_u32(smem_dyn)) + warp * (PF_Q_BYTES / SW));   /* [32][36] */
-            const uint32_t etl = r * inv_gqa >> 16, etok = e_t0 + g * P.tpc + etl;
-            if (parts && etl < P.tpc && etok < P.n_tok && h == 0)
-                P.part_ml[((size_t)e_range * P.part_tok + etok) * P.n_head + e_kh * P.gqa + (r - etl * P.gqa)] = make_float2(m_ref, l_run);
+            uint32_t part_tok = P.n_tok;
+            if constexpr (TAIL) part_tok = P.part_tok;
+            const uint32_t etl = TAIL ? r * inv_gqa >> 16 : tl, etok = TAIL ? e_t0 + g * P.tpc + etl : tok, ehead = TAIL ? e_kh * P.gqa + (r - etl * P.gqa) : head;
+            if (parts && (TAIL ? etl < P.tpc && etok < P.n_tok : row_live) && h == 0)
+                P.part_ml[((size_t)e_range * part_tok + etok) * P.n_head + ehead] = make_float2(m_ref, l_run);
             auto columns = [&](int c, float4 (&gs)[8]) {
                 float o[32];
                 if (n_tiles > 0) {
@@ -846,7 +852,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
                 if (parts) {
 #pragma unroll
                     for (int q = 0; q < 8; q++)
-                        if ((live >> q) & 1u) reinterpret_cast<float4 *>(P.part)[(size_t)e_range * P.part_tok * P.n_head * (HD / 4u) + first + off[q] + 8u * c] = x[q];
+                        if ((live >> q) & 1u) reinterpret_cast<float4 *>(P.part)[(size_t)e_range * part_tok * P.n_head * (HD / 4u) + first + off[q] + 8u * c] = x[q];
                 } else if (P.out_bf16) {
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
@@ -876,14 +882,19 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const PrefillParam
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
-/* ---- the parts of split position ranges -> out: thread = 4 dims of one (token, head) */
-__global__ void __launch_bounds__(256) q4_pf_merge_k(const PrefillParams P, uint32_t hd, uint64_t total4, uint32_t tok_per_group) {
+/* ---- the parts of split position ranges -> out: thread = 4 dims of one (token, head); TAIL: only some items have parts */
+template <bool TAIL>
+__global__ void __launch_bounds__(256) q4_pf_merge_k(const std::conditional_t<TAIL, PrefillTail, PrefillParams> P, uint32_t hd, uint64_t total4, uint32_t tok_per_group) {
     const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
     q4d_pdl_wait();
     if (i >= total4) return;
-    const uint64_t row = i / (hd / 4u), rows = (uint64_t)P.part_tok * P.n_head;
-    const uint32_t tok = (uint32_t)(row / P.n_head), head = (uint32_t)(row % P.n_head);
-    if (head / P.gqa * P.n_groups + (P.n_groups - 1u - tok / tok_per_group) < P.n_whole) return;   /* one block's, finished */
+    const uint64_t row = i / (hd / 4u);
+    uint64_t rows = (uint64_t)P.n_tok * P.n_head;
+    if constexpr (TAIL) {   /* at most a block's rows per SM; where all items have parts these divisions took 0.5 us */
+        const uint32_t tok = (uint32_t)row / P.n_head, head = (uint32_t)row % P.n_head;
+        if (head / P.gqa * P.n_groups + (P.n_groups - 1u - tok / tok_per_group) < P.n_whole) return;   /* one block's, finished */
+        rows = (uint64_t)P.part_tok * P.n_head;
+    }
     float M = -CUDART_INF_F;
     for (uint32_t s = 0; s < P.n_split; s++) M = fmaxf(M, P.part_ml[s * rows + row].x);
     const float Mu = M == -CUDART_INF_F ? 0.f : M;
@@ -942,16 +953,16 @@ int stage_reserve(size_t bytes) {
 }
 
 template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
-bool attend(const PrefillParams &p, dim3 grid) {
+bool attend(const PrefillTail &p, dim3 grid) {
     static bool attr = false;
     if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
                             "prefill smem attribute"))
         return false;
     attr = true;
-    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, grid, PF_THREADS, PF_SMEM, p);
+    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, grid, PF_THREADS, PF_SMEM, static_cast<const std::conditional_t<TAIL, PrefillTail, PrefillParams> &>(p));
 }
 template <int HD, int NP, bool MARKS>
-bool attend_one(const PrefillParams &p, uint32_t n_kvh) {
+bool attend_one(const PrefillTail &p, uint32_t n_kvh) {
     if (p.n_whole && p.n_late) return attend<HD, 1, NP, MARKS, true>(p, dim3(p.n_whole + p.n_late * p.n_split));
     return attend<HD, 1, NP, MARKS, false>(p, dim3(p.n_groups, n_kvh, p.n_split));
 }
@@ -967,17 +978,17 @@ bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, ui
  * Two groups per block: a tile 1.8 us, a block 5.  There, and with more blocks than SMs, only those of the last wave are split,
  * the shortest of the chunk: 8192 tokens over 16 384 are 512 blocks, 444 and 68 x 2. */
 struct PfSplit { uint32_t whole, ranges; };
-PfSplit best_split(uint32_t groups, uint32_t n_kvh, uint32_t sms, uint32_t kv_base, uint32_t tok_per_group, uint32_t tiles, uint32_t rows_per_group, uint32_t hd,
+PfSplit best_split(uint32_t groups, uint32_t n_kvh, uint32_t sms, uint32_t kv_base, uint32_t tok_per_group, uint32_t tiles, uint64_t rows, uint32_t rows_per_group, uint32_t hd,
                    uint32_t np, uint32_t nq) {
     const uint32_t blocks = groups * n_kvh, waves = blocks / sms, rest = blocks % sms;
     const uint64_t tile = nq == 2 ? 1800u : 640u + 190u * (hd / 128u) * 2u * np, block = nq == 2 ? 5000u : 2000u + 2000u * (hd / 128u);
-    auto merge = [&](uint32_t items, uint32_t s) -> uint64_t { return 1200u + 200u * s + (uint64_t)items * rows_per_group * hd * s * 8u / 7000u; };
+    auto merge = [&](uint64_t n, uint32_t s) -> uint64_t { return 1200u + 200u * s + n * hd * s * 8u / 7000u; };
     PfSplit r = {blocks, 1u};
     const uint64_t whole = (waves + (rest != 0u)) * (tiles * tile + block);
     uint64_t best = whole - whole / 16u;   /* whole blocks need no merge: left for a clear gain only (causal chunks have less work) */
     for (uint32_t s = 2; s <= 16u && s <= tiles; s++) {
         if (nq == 1) {
-            const uint64_t t = ((uint64_t)blocks * s + sms - 1u) / sms * ((tiles + s - 1u) / s * tile + block) + merge(blocks, s);
+            const uint64_t t = ((uint64_t)blocks * s + sms - 1u) / sms * ((tiles + s - 1u) / s * tile + block) + merge(rows, s);
             if (t < best) {
                 best = t;
                 r = {0u, s};
@@ -987,7 +998,7 @@ PfSplit best_split(uint32_t groups, uint32_t n_kvh, uint32_t sms, uint32_t kv_ba
          * without a prefix, the blocks before them end so far apart that they fill the gaps (8192 tokens over none 240 us, split 255). */
         const uint32_t seen = (kv_base + (rest < groups ? rest : groups) * tok_per_group + PF_BN - 1u) / PF_BN, n = seen < tiles ? seen : tiles;
         if (waves && rest && rest * s <= sms && n >= 2u * (tiles - kv_base / PF_BN)) {
-            const uint64_t t = waves * (tiles * tile + block) + (n + s - 1u) / s * tile + block + merge(rest, s), now = waves * (tiles * tile + block) + n * tile + block;
+            const uint64_t t = waves * (tiles * tile + block) + (n + s - 1u) / s * tile + block + merge((uint64_t)rest * rows_per_group, s), now = waves * (tiles * tile + block) + n * tile + block;
             if (t < best && t < now) {
                 best = t;
                 r = {blocks - rest, s};
@@ -1018,7 +1029,7 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
     const uint32_t n_groups = (groups + nq - 1u) / nq, tok_per_group = tpc * nq, blocks = n_groups * a.n_kvh;
     const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes, m_bytes = (size_t)a.n_kvh * tiles * (PF_BN / 32u) * (sizeof(PfMark) + 4u);   /* marks, flags (two bytes used per mark) */
-    PfSplit sp = best_split(n_groups, a.n_kvh, sms, a.kv_base, tok_per_group, tiles, tok_per_group * gqa, hd, np, nq);
+    PfSplit sp = best_split(n_groups, a.n_kvh, sms, a.kv_base, tok_per_group, tiles, (uint64_t)a.n_tok * a.n_head, tok_per_group * gqa, hd, np, nq);
     uint32_t part_tok;
     size_t rows, part_bytes;
     int room;
@@ -1035,7 +1046,7 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     if (room != 1) return room;
     const uint32_t split = sp.ranges;
 
-    PrefillParams p;
+    PrefillTail p;
     memset(&p, 0, sizeof(p));
     p.n_head = a.n_head; p.n_kvh = a.n_kvh; p.gqa = gqa; p.tpc = tpc;
     p.q = a.q; p.q_bf16 = a.q_bf16; p.gate = a.gate; p.out = a.out; p.out_bf16 = a.out_bf16;
@@ -1069,7 +1080,9 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     }
     if (ok && split > 1) {
         const uint64_t total4 = (uint64_t)rows * hd / 4u;
-        ok = q4i_launch_pdl("prefill launch", q4_pf_merge_k, dim3((unsigned)((total4 + 255u) / 256u)), 256u, 0, p, hd, total4, tok_per_group);
+        const dim3 grid((unsigned)((total4 + 255u) / 256u));
+        ok = sp.whole ? q4i_launch_pdl("prefill launch", q4_pf_merge_k<true>, grid, 256u, 0, p, hd, total4, tok_per_group)
+                      : q4i_launch_pdl("prefill launch", q4_pf_merge_k<false>, grid, 256u, 0, static_cast<const PrefillParams &>(p), hd, total4, tok_per_group);
     }
     return ok ? 1 : 0;
 }
