@@ -1095,11 +1095,15 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
  * keys of the threshold bin, and the exact finish works on those.  Chosen keys are marked in a bitmap in index order; the
  * ordered emit is a prefix sum of its population counts.
  * Counting every key's digit in shared memory costs more than reading it, because most keys of a row share few leading
- * digits.  So the first pass over a long row is a sample of 2048 keys: it gives a pivot which `need` keys of the row fall short of
- * by five standard deviations, and the second collects the keys that reach it.  Where the sample misled (fewer keys than
- * needed, or more than there is room for: rows of ties) the row is counted in full.  512 tokens, us, counted / sampled:
- * 65 536 keys 86.0 / 72.6, 32 768 43.8 / 35.6, 16 384 28.0 / 27.8, 12 000 23.8 / 25.5, 8196 19.8 / 23.7. */
-constexpr uint32_t TKM_THREADS = 512, TKM_CAND = 2048, TKM_BATCH = 8, TKM_SAMPLE = 2048, TKM_SAMPLED_FROM = 16384;   /* keys */
+ * digits.  So the first pass over a long row is a sample of 2048 keys: it gives a pivot, 24 bits of a key, which `need` keys of the
+ * row fall short of by five standard deviations.  The second collects the keys above the pivot's bin and counts, by their last 8
+ * bits, those in it: where the first are too few (rows of ties, whose pivot is the threshold itself) the threshold is known by
+ * then, and a third pass marks the row.  Where the sample misled the row is counted in full.  Only with more than one block per
+ * SM: a block that has an SM to itself waits for the sample longer than it saves.
+ * us, counted / sampled: 512 tokens x 65 536 keys 86.7 / 73.7, 32 768 44.2 / 35.4, 24 576 35.5 / 30.3; 200 tokens x 32 768 24.4 /
+ * 22.3, 24 576 20.0 / 19.3, rounded keys 20.5 / 21.9; 100 x 32 768 17.3 / 19.5; 512 x 32 768 zeros 68.6 / 65.2 (111 where all keys
+ * that reach the pivot are collected, until the room ends). */
+constexpr uint32_t TKM_THREADS = 512, TKM_CAND = 2048, TKM_BATCH = 8, TKM_SAMPLE = 2048, TKM_SAMPLED_FROM = 24576;   /* keys */
 struct TkmShared {
     __align__(16) uint32_t hist[TK_BINS], h3[256], tot[4][32];
     uint32_t ckey[TKM_CAND];
@@ -1108,18 +1112,20 @@ struct TkmShared {
     uint32_t n_cand;
     TkPick st[2];
 };
-/* keys that reach the pivot, in any order; the count goes on where the room ends */
+/* keys above the pivot's bin of 256, in any order (the count goes on where the room ends), and how many lie where in the bin */
 __device__ __forceinline__ void tkm_collect(TkmShared &S, const float *row, uint32_t n, uint32_t pivot) {
     const float pf = __uint_as_float(pivot & 0x80000000u ? pivot & 0x7fffffffu : ~pivot);   /* ix_key's inverse */
     auto one = [&](uint32_t b, float x) {
         if (!(x < pf)) {   /* and NaN, which ix_key orders by its sign */
             const uint32_t u = ix_key(x);
-            if (u >= pivot) {
+            if (u > (pivot | 255u)) {
                 const uint32_t slot = atomicAdd(&S.n_cand, 1u);
                 if (slot < TKM_CAND) {
                     S.ckey[slot] = u;
                     S.cidx[slot] = b;
                 }
+            } else if (u >= pivot) {
+                atomicAdd(&S.h3[u & 255u], 1u);
             }
         }
     };
@@ -1159,6 +1165,7 @@ __device__ __forceinline__ void tkm_walk(const float *row, uint32_t n, F f) {
         }
     }
 }
+template <bool SAMPLED>
 __global__ void __launch_bounds__(TKM_THREADS, 4) q4_ix_topkm_k(const float *score, int32_t *sel, uint32_t stride, uint32_t k_blk,
                                                                uint32_t ratio, uint32_t pos0, uint32_t width, uint32_t words,
                                                                const int32_t *pp, const int32_t *pos_arr) {
@@ -1185,9 +1192,9 @@ __global__ void __launch_bounds__(TKM_THREADS, 4) q4_ix_topkm_k(const float *sco
     if (tx == 0) S.n_cand = 0u;
     for (uint32_t i = tx; i < words; i += TKM_THREADS) { bg[i] = 0u; be[i] = 0u; }
     clear();
-    uint32_t n_cand = 0;
-    bool sampled = n > TKM_SAMPLED_FROM;
-    if (sampled) {
+    uint32_t n_cand = 0, thr = 0, n_gt = 0;
+    bool sampled = false, known = false, mark = false;   /* candidates from the sampled pivot; threshold known already; the row is marked by walking it */
+    if (SAMPLED && n > TKM_SAMPLED_FROM) {
         /* the pivot: 24 bits of a key */
         constexpr uint32_t PER = TKM_SAMPLE * 9u / 8u / TKM_THREADS + 1u;
         const uint32_t step = n / TKM_SAMPLE, n_s = (n + step - 1u) / step;
@@ -1211,72 +1218,84 @@ __global__ void __launch_bounds__(TKM_THREADS, 4) q4_ix_topkm_k(const float *sco
         __syncthreads();
         const TkPick s2 = tk_pick<TKM_THREADS>(S.hist, target - s1.above, S.tot[1], &S.st[1]);
         clear();
-        tkm_collect(S, row, n, (s1.digit << TK_B1) | (s2.digit << TK_B2));
+        const uint32_t pivot = (s1.digit << TK_B1) | (s2.digit << TK_B2);
+        tkm_collect(S, row, n, pivot);
         __syncthreads();
         n_cand = S.n_cand;
         sampled = n_cand >= need && n_cand <= TKM_CAND;
+        if (n_cand < need) {   /* the threshold lies in the pivot's bin, if that has enough keys */
+            const TkPick p3 = tk_pick256(S.h3, need - n_cand);
+            thr = pivot | p3.digit;
+            n_gt = n_cand + p3.above;
+            known = mark = p3.cnt != 0u;
+        }
+        __syncthreads();
+        if (tx < 256) S.h3[tx] = 0u;
     }
-    if (sampled) {
-        for (uint32_t i = tx; i < n_cand; i += TKM_THREADS) atomicAdd(&S.hist[S.ckey[i] >> TK_B1], 1u);
-    } else {
-        tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) { if (live) atomicAdd(&S.hist[u >> TK_B1], 1u); });
-    }
-    __syncthreads();
-    const TkPick p1 = tk_pick<TKM_THREADS>(S.hist, need, S.tot[0], &S.st[0]);
-    if (tx == 0) S.n_cand = 0u;   /* everyone has read it */
-    clear();
-    uint32_t thr, n_gt;
-    if (sampled || p1.cnt <= TKM_CAND) {
+    if (!known) {
         if (sampled) {
-            for (uint32_t i = tx; i < n_cand; i += TKM_THREADS)
-                if ((S.ckey[i] >> TK_B1) == p1.digit) atomicAdd(&S.hist[(S.ckey[i] >> TK_B2) & (TK_BINS - 1u)], 1u);
+            for (uint32_t i = tx; i < n_cand; i += TKM_THREADS) atomicAdd(&S.hist[S.ckey[i] >> TK_B1], 1u);
         } else {
-            n_cand = p1.cnt;
-            tkm_walk(row, n, [&](uint32_t b, uint32_t u, bool live) {
-                const uint32_t m = __ballot_sync(0xffffffffu, live && (u >> TK_B1) > p1.digit);
-                if (lane == 0 && m) bg[b >> 5] = m;
-                if (live && (u >> TK_B1) == p1.digit) {
-                    const uint32_t slot = atomicAdd(&S.n_cand, 1u);
-                    S.ckey[slot] = u;
-                    S.cidx[slot] = b;
-                    atomicAdd(&S.hist[(u >> TK_B2) & (TK_BINS - 1u)], 1u);
-                }
+            tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) { if (live) atomicAdd(&S.hist[u >> TK_B1], 1u); });
+        }
+        __syncthreads();
+        const TkPick p1 = tk_pick<TKM_THREADS>(S.hist, need, S.tot[0], &S.st[0]);
+        if (tx == 0) S.n_cand = 0u;   /* everyone has read it */
+        clear();
+        if (sampled || p1.cnt <= TKM_CAND) {
+            if (sampled) {
+                for (uint32_t i = tx; i < n_cand; i += TKM_THREADS)
+                    if ((S.ckey[i] >> TK_B1) == p1.digit) atomicAdd(&S.hist[(S.ckey[i] >> TK_B2) & (TK_BINS - 1u)], 1u);
+            } else {
+                n_cand = p1.cnt;
+                tkm_walk(row, n, [&](uint32_t b, uint32_t u, bool live) {
+                    const uint32_t m = __ballot_sync(0xffffffffu, live && (u >> TK_B1) > p1.digit);
+                    if (lane == 0 && m) bg[b >> 5] = m;
+                    if (live && (u >> TK_B1) == p1.digit) {
+                        const uint32_t slot = atomicAdd(&S.n_cand, 1u);
+                        S.ckey[slot] = u;
+                        S.cidx[slot] = b;
+                        atomicAdd(&S.hist[(u >> TK_B2) & (TK_BINS - 1u)], 1u);
+                    }
+                });
+            }
+            __syncthreads();
+            const TkPick p2 = tk_pick<TKM_THREADS>(S.hist, need - p1.above, S.tot[1], &S.st[1]);
+            const uint32_t pre = (p1.digit << 12) | p2.digit;
+            for (uint32_t i = tx; i < n_cand; i += TKM_THREADS)
+                if ((S.ckey[i] >> TK_B2) == pre) atomicAdd(&S.h3[S.ckey[i] & 255u], 1u);
+            __syncthreads();
+            const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
+            thr = (pre << 8) | p3.digit;
+            n_gt = p1.above + p2.above + p3.above;
+            for (uint32_t i = tx; i < n_cand; i += TKM_THREADS) {
+                const uint32_t u = S.ckey[i], b = S.cidx[i];
+                if (u > thr) atomicOr(&bg[b >> 5], 1u << (b & 31u));
+                else if (u == thr) atomicOr(&be[b >> 5], 1u << (b & 31u));
+            }
+        } else {   /* rows of ties: the second and third digit are counted over the row too */
+            tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) {
+                if (live && (u >> TK_B1) == p1.digit) atomicAdd(&S.hist[(u >> TK_B2) & (TK_BINS - 1u)], 1u);
             });
+            __syncthreads();
+            const TkPick p2 = tk_pick<TKM_THREADS>(S.hist, need - p1.above, S.tot[1], &S.st[1]);
+            const uint32_t pre = (p1.digit << 12) | p2.digit;
+            tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) {
+                if (live && (u >> TK_B2) == pre) atomicAdd(&S.h3[u & 255u], 1u);
+            });
+            __syncthreads();
+            const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
+            thr = (pre << 8) | p3.digit;
+            n_gt = p1.above + p2.above + p3.above;
+            mark = true;
         }
-        __syncthreads();
-        const TkPick p2 = tk_pick<TKM_THREADS>(S.hist, need - p1.above, S.tot[1], &S.st[1]);
-        const uint32_t pre = (p1.digit << 12) | p2.digit;
-        for (uint32_t i = tx; i < n_cand; i += TKM_THREADS)
-            if ((S.ckey[i] >> TK_B2) == pre) atomicAdd(&S.h3[S.ckey[i] & 255u], 1u);
-        __syncthreads();
-        const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
-        thr = (pre << 8) | p3.digit;
-        n_gt = p1.above + p2.above + p3.above;
-        for (uint32_t i = tx; i < n_cand; i += TKM_THREADS) {
-            const uint32_t u = S.ckey[i], b = S.cidx[i];
-            if (u > thr) atomicOr(&bg[b >> 5], 1u << (b & 31u));
-            else if (u == thr) atomicOr(&be[b >> 5], 1u << (b & 31u));
-        }
-    } else {   /* rows of ties: the second and third digit are counted over the row too */
-        tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) {
-            if (live && (u >> TK_B1) == p1.digit) atomicAdd(&S.hist[(u >> TK_B2) & (TK_BINS - 1u)], 1u);
-        });
-        __syncthreads();
-        const TkPick p2 = tk_pick<TKM_THREADS>(S.hist, need - p1.above, S.tot[1], &S.st[1]);
-        const uint32_t pre = (p1.digit << 12) | p2.digit;
-        tkm_walk(row, n, [&](uint32_t, uint32_t u, bool live) {
-            if (live && (u >> TK_B2) == pre) atomicAdd(&S.h3[u & 255u], 1u);
-        });
-        __syncthreads();
-        const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
-        thr = (pre << 8) | p3.digit;
-        n_gt = p1.above + p2.above + p3.above;
+    }
+    if (mark)
         tkm_walk(row, n, [&](uint32_t b, uint32_t u, bool live) {
             const uint32_t mg = __ballot_sync(0xffffffffu, live && u > thr), me = __ballot_sync(0xffffffffu, live && u == thr);
             if (lane == 0 && mg) bg[b >> 5] = mg;
             if (lane == 0 && me) be[b >> 5] = me;
         });
-    }
     __syncthreads();
     /* ranks: every thread owns consecutive words of the bitmaps */
     const uint32_t wpt = (words + TKM_THREADS - 1u) / TKM_THREADS, wa = min(tx * wpt, words), wb = min(wa + wpt, words);
@@ -1322,6 +1341,18 @@ bool topkc_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
     return ix_start("qsa_topk launch", q4_ix_topkc_k<NB>, dim3(NB, n_tok), IX_TK_THREADS, sizeof(TkcShared<NB>), NB, score, sel, stride, k_blk, ratio, pos0,
                       width, pp, pos_arr, pos_arr || vis > stride ? stride : vis, ix_pdl() && ratio && !pos_arr && (!pp || q4i_settled(g_q4.pos_written)));
 }
+template <bool SAMPLED>
+bool topkm_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stride, uint32_t k_blk, uint32_t ratio, uint32_t pos0,
+                 uint32_t width, const int32_t *pp, const int32_t *pos_arr) {
+    static bool done = false;
+    if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_topkm_k<SAMPLED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)(sizeof(TkmShared) + 2 * TKC_MAX_ROW / 8)), "qsa_topk smem attribute"))
+        return false;
+    done = true;
+    const uint32_t words = (stride + 31u) / 32u;
+    return ix_start("qsa_topk launch", q4_ix_topkm_k<SAMPLED>, dim3(n_tok), TKM_THREADS, sizeof(TkmShared) + 2u * words * 4u, 1u, score, sel, stride, k_blk,
+                    ratio, pos0, width, words, pp, pos_arr);
+}
 /* Which form: rows of up to 8192 keys need one block either way, which keeps them in registers.  Longer rows take the
  * cluster form while all clusters are resident at once (two blocks of 1024 threads per SM), the streaming form beyond
  * (512 tokens x 32 768 keys), and the single block that re-reads the row behind 65 536 keys. */
@@ -1334,14 +1365,9 @@ bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
     if (stride <= TKC_KEYS) return topkc_start<1>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
     const uint32_t nb = stride <= 2 * TKC_KEYS ? 2u : stride <= 4 * TKC_KEYS ? 4u : 8u;
     if ((uint64_t)n_tok * nb > 2ull * (uint64_t)g_q4.sm_count) {
-        static bool done = false;
-        if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_topkm_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)(sizeof(TkmShared) + 2 * TKC_MAX_ROW / 8)), "qsa_topk smem attribute"))
-            return false;
-        done = true;
-        const uint32_t words = (stride + 31u) / 32u;
-        return ix_start("qsa_topk launch", q4_ix_topkm_k, dim3(n_tok), TKM_THREADS, sizeof(TkmShared) + 2u * words * 4u, 1u, score, sel, stride, k_blk, ratio,
-                          pos0, width, words, pp, pos_arr);
+        const uint32_t rows = pp || pos_arr || !ratio ? stride : (pos0 + n_tok) / ratio;   /* the last token's, at most */
+        return n_tok > (uint32_t)g_q4.sm_count && rows > TKM_SAMPLED_FROM ? topkm_start<true>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr)
+                                                                          : topkm_start<false>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
     }
     if (nb == 2) return topkc_start<2>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
     if (nb == 4) return topkc_start<4>(score, sel, n_tok, stride, k_blk, ratio, pos0, width, pp, pos_arr);
