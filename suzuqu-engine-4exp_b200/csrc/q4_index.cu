@@ -1411,8 +1411,9 @@ extern "C" bool q4_hip_qsa_score(const float *q, const float *pool, float *score
     if (n_blocks == 0) return true;
     if (ratio && n_tok > 1 && (((uintptr_t)q | (uintptr_t)pool) & 15u) == 0) {
         const uint64_t wide = score_mt_ns(n_tok, n_blocks, 4), narrow = score_mt_ns(n_tok, n_blocks, 2), scan = score_scan_ns(n_tok, n_blocks);
-        if (wide <= narrow && wide < scan) return score_mt_launch<4>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
-        if (narrow < scan) return score_mt_launch<2>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+        const uint64_t below = scan - scan / 16u;   /* of 8 tokens over 24 576 blocks: 23.2 us where 26.8 are estimated, the product takes 24.3 */
+        if (wide <= narrow && wide < below) return score_mt_launch<4>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
+        if (narrow < below) return score_mt_launch<2>(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio);
     }
     return score_launch(q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, nullptr, nullptr, nullptr);
 }
