@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
     if (apart) q4d_apart_begin();
     else if (!early) q4d_pdl_wait();
     if (pp) {   /* device position: the block this token completes, if any */
-        const uint32_t pos = (uint32_t)*pp;
+        const uint32_t pos = (uint32_t)__ldcg(pp);
         b0 = pos / ratio;
         b1 = (pos + 1u) / ratio;
     }
@@ -65,7 +65,11 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
         return;
     }
     const __half *src = raw + (size_t)b * ratio * IX_HD;
-    float v[4], r[4];
+    float v[4], r[4], g[4] = {1.f, 1.f, 1.f, 1.f};
+    if (wn) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) g[c] = __ldcg(wn + lane + 32u * c);
+    }
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         float s = 0.f;
@@ -80,10 +84,7 @@ __global__ void __launch_bounds__(128) q4_ix_pool_k(const __half *raw, float *po
     const float tot = __shfl_sync(0xffffffffu, a, 0);
     const float inv = rsqrtf(__fadd_rn(__fdiv_rn(tot, (float)IX_HD), eps));
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const uint32_t d = lane + 32u * c;
-        v[c] = __fmul_rn(__fmul_rn(v[c], inv), wn ? wn[d] : 1.f);
-    }
+    for (int c = 0; c < 4; c++) v[c] = __fmul_rn(__fmul_rn(v[c], inv), g[c]);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         const uint32_t d = lane + 32u * c;

@@ -141,8 +141,8 @@ __device__ __forceinline__ void q4d_pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-/* A kernel that runs beside its predecessor (q4i_apart), in every thread, begin first and end last.  What it reads may have been
- * written by the launch before last: by loads that do not look into L1. */
+/* A kernel that runs beside its predecessor (q4i_apart), in every thread, begin first and end last.  What it reads, the position
+ * word and weights too, may have been written by the launch before last: by loads that do not look into L1. */
 __device__ __forceinline__ void q4d_apart_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void q4d_apart_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 /* host side: a launch that may start so (the kernel calls q4d_pdl_wait in every thread) */

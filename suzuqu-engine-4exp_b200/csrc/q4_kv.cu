@@ -61,7 +61,7 @@ __global__ void q4_f32_to_f16_k(const float *src, __half *dst, uint64_t n, const
     if (apart) q4d_apart_begin();
     else if (DEP) q4d_pdl_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos) dst += (size_t)(uint32_t)*pos * stride;
+    if (pos) dst += (size_t)(uint32_t)__ldcg(pos) * stride;
     if (i < n) dst[i] = __float2half_rn(__ldcg(src + i));
     if (apart) q4d_apart_end();
 }

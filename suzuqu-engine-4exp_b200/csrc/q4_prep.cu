@@ -84,11 +84,22 @@ __device__ __forceinline__ void row_load(const float *src, float2 (&v)[HD / 64])
 #pragma unroll
     for (int k = 0; k < HD / 64; k++) v[k] = __ldcg(reinterpret_cast<const float2 *>(src) + 32 * k + lane);
 }
+/* the weights of those elements; l2: the launch before last may have written them (q4d_apart_begin).  A launch of few rows asks
+ * for them beside the row: behind its sums they came a trip to L2 later. */
+template <int HD>
+__device__ __forceinline__ void row_weights(const float *wn, float2 (&w)[HD / 64], bool l2) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int k = 0; k < HD / 64; k++) {
+        const float *p = wn + 64 * k + 2 * lane;
+        w[k] = !wn ? make_float2(1.f, 1.f) : l2 ? make_float2(__ldcg(p), __ldcg(p + 1)) : make_float2(p[0], p[1]);
+    }
+}
 /* RMSNorm and rotation in place.  Sum of squares as 128 threads of a block would take it: thread i adds elements i and
  * i + 128, a butterfly over each 32 threads, then the four totals in order (element 2 l + e of a register is thread
  * 2 l + e: the butterfly's last step is the addition inside the lane). */
 template <int HD>
-__device__ __forceinline__ void row_norm_rope(float2 (&v)[HD / 64], const float *wn, const float2 *cs, uint32_t np, float eps) {
+__device__ __forceinline__ void row_norm_rope(float2 (&v)[HD / 64], const float2 (&w)[HD / 64], const float2 *cs, uint32_t np, float eps) {
     const uint32_t lane = threadIdx.x & 31u;
     float tot[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -109,8 +120,7 @@ __device__ __forceinline__ void row_norm_rope(float2 (&v)[HD / 64], const float 
 #pragma unroll
     for (int k = 0; k < HD / 64; k++) {
         const uint32_t p = 32u * k + lane;
-        float x0 = v[k].x * scale * (wn ? wn[2 * p] : 1.f);
-        float x1 = v[k].y * scale * (wn ? wn[2 * p + 1] : 1.f);
+        float x0 = v[k].x * scale * w[k].x, x1 = v[k].y * scale * w[k].y;
         if (p < np) {
             const float c = cs[p].x, si = cs[p].y;
             const float y0 = x0 * c - x1 * si, y1 = x0 * si + x1 * c;
@@ -138,19 +148,20 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_rows_k(const float *s
     const uint32_t warp = threadIdx.x >> 5, sub = warp / W, t = blockIdx.y * TOK + sub, h0 = blockIdx.x * per, h1 = min(h0 + per, n_head);
     if (apart) q4d_apart_begin();
     else if (!early) q4d_pdl_wait();
-    rope_table(cs[sub], n_rot / 2u, (pp ? *pp : pos0) + (int32_t)t, base, threadIdx.x % (W * 32u), W * 32u);   /* a settled position's under the previous kernel's tail */
+    rope_table(cs[sub], n_rot / 2u, (pp ? __ldcg(pp) : pos0) + (int32_t)t, base, threadIdx.x % (W * 32u), W * 32u);   /* a settled position's under the previous kernel's tail */
     if (early && !apart) q4d_pdl_wait();
     __syncthreads();
     for (uint32_t h = h0 + warp % W; h < h1 && t < n_tok; h += W) {
         const size_t row = (size_t)t * n_head + h;
-        float2 v[HD / 64];
+        float2 v[HD / 64], wt[HD / 64];
+        row_weights<HD>(wn, wt, apart);
         row_load<HD>(SPLIT ? src + row * 2u * HD : q + row * HD, v);
         if (SPLIT) {
             float2 w[HD / 64];
             row_load<HD>(src + row * 2u * HD + HD, w);
             row_store<HD>(g + row * HD, w);
         }
-        row_norm_rope<HD>(v, wn, cs[sub], n_rot / 2u, eps);
+        row_norm_rope<HD>(v, wt, cs[sub], n_rot / 2u, eps);
         row_store<HD>(q + row * HD, v);
     }
     if (apart) q4d_apart_end();
@@ -317,7 +328,11 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) q4_prep_append_rows_k(const P
         const uint32_t kh = which ? r - P.n_kvh : r;
         float2 v[HD / 64];
         row_load<HD>((which ? P.v : P.k) + ((size_t)t * P.n_kvh + kh) * HD, v);
-        if (!which) row_norm_rope<HD>(v, P.wn, cs[sub], P.n_rot / 2u, P.eps);
+        if (!which) {
+            float2 wt[HD / 64];
+            row_weights<HD>(P.wn, wt, false);
+            row_norm_rope<HD>(v, wt, cs[sub], P.n_rot / 2u, P.eps);
+        }
         __syncwarp();
         row_store<HD>(row_s[warp], v);
         __syncwarp();
