@@ -1010,10 +1010,11 @@ q4_decode_k(const DecParams P) {
     bool ap_which = false, ap_live = false;
     uint32_t ap_b = 0, ap_sub = 0;
     /* A dense scan's newest row is in one split's slice, and only that one stores it: 222 blocks that wrote the same two lines
-     * held one another up behind the fence (262144 rows: a block's loop began 2.6 us after the wait, 1.1 with one). */
-    const bool appends = APPENDS && P.new_k && (LIST || (newest < max_kv ? newest >> 4 >= s_begin && newest >> 4 < s_end : split == 0u));
+     * held one another up behind the fence (262144 rows: a block's loop began 2.6 us after the wait, 1.1 with one).  Decided
+     * where it is stored. */
+    auto appends = [&]() { return P.new_k && (LIST || (newest < max_kv ? newest >> 4 >= s_begin && newest >> 4 < s_end : split == 0u)); };
     auto load_new = [&]() {   /* rows are read with cp.async (coherent at L2), never through the read-only path */
-        if (appends) {
+        if (P.new_k) {
             constexpr uint32_t QL = HD / 4;
             const uint32_t tid = threadIdx.x;
             ap_which = tid >= QL;
@@ -1340,7 +1341,7 @@ q4_decode_k(const DecParams P) {
         auto first_positions = [&]() {
             pa = my_pos(0); pb = my_pos(1); pc = my_pos(2); pd = my_pos(3);
             pn0 = my_pos(4); pn1 = my_pos(5); pn2 = my_pos(6);
-            if (appends) {
+            if (P.new_k) {
                 const int32_t nw = (int32_t)newest;
                 hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
             }
@@ -1364,7 +1365,7 @@ q4_decode_k(const DecParams P) {
             load_new();
             request_q();
         }
-        if (appends) {
+        if (appends()) {
             float d, id;
             q4d_block_scale(ap_x, d, id);
             if (ap_live) {
@@ -1668,7 +1669,7 @@ q4_decode_k(const DecParams P) {
 #pragma unroll
             for (int i = 0; i < ST; i++) pf[i] = my_pos(i);
             pn0 = my_pos(ST); pn1 = my_pos(ST + 1); pn2 = my_pos(ST + 2);
-            if (appends) {
+            if (P.new_k) {
 #pragma unroll
                 for (int i = 0; i < ST; i++) hold = hold || pf[i] == (int32_t)newest;
                 hold = __any_sync(0xffffffffu, hold);
@@ -1691,7 +1692,7 @@ q4_decode_k(const DecParams P) {
             load_new();
             request_q();
         }
-        if (LAY != LAY_Q8R && appends) {
+        if (LAY != LAY_Q8R && appends()) {
             uint8_t *row = const_cast<uint8_t *>(ap_which ? vbase : kbase) + (uint64_t)newest * tok_stride;
             const uint32_t at = ap_b * 32 + ap_sub * 4;
             if (LAY == LAY_Q8P) {
