@@ -580,7 +580,9 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
 
 /* ---- selection: one block per token */
 __device__ __forceinline__ uint32_t ix_key(float f) {   /* order-preserving uint of a float (:7464-7467) */
-    const uint32_t u = __float_as_uint(f);
+    uint32_t u;
+    /* bits out of the compiler's sight: it turned a conversion's  u | sign  into -|f|, which leaves a NaN its sign */
+    asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 /* exclusive prefix sum of one value per thread over the block; returns the block total */

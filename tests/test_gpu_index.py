@@ -384,3 +384,29 @@ def test_scores_of_one_token_at_the_edges_of_a_blocks_share(oracle, per, more, n
     a, b = host(a), host(b)
     assert np.array_equal(a[:rows + 3].view(np.uint32), want[:rows + 3].view(np.uint32)) and (a[rows + 3:] == 7.0).all()
     assert np.array_equal(b[:rows].view(np.uint32), want[:rows].view(np.uint32)) and (b[rows:] == 7.0).all()
+
+
+@pytest.mark.parametrize("n_tok,n_vis", [(3, 700), (3, 8192), (1, 9000), (2, 20000), (1, 40000), (1, 66000), (160, 8200), (160, 20000), (160, 33000), (300, 65536)])
+def test_scores_that_are_not_numbers_are_ordered_by_their_bits(oracle, n_tok, n_vis):
+    """every form: NaN above all numbers, NaN with a sign below them, infinities and zeros of both signs"""
+    L = lib()
+    rng = np.random.default_rng(n_vis)
+    k_blk = 512 if n_vis > 4000 else 64
+    sc = rng.standard_normal((n_tok, n_vis)).astype(np.float32)
+    for t in range(n_tok):
+        some, n = rng.permutation(n_vis), n_vis // 60 if n_vis < 16000 else 300
+        sc[t, some[:n]] = np.nan
+        sc[t, some[n:2 * n]] = -np.float32(np.nan)
+        sc[t, some[2 * n:2 * n + 5]] = np.inf
+        sc[t, some[2 * n + 5:3 * n]] = -np.inf
+        sc[t, some[3 * n:5 * n]] = 0.0
+        sc[t, some[5 * n:6 * n]] = -0.0
+        if t % 3 == 2:
+            sc[t] = np.minimum(sc[t], 0.0)   # keeps NaN
+    pos0, width = n_vis * RATIO - n_tok, k_blk * RATIO + 3
+    d = torch.from_numpy(sc).cuda()
+    d_sel = torch.full((n_tok, width), -7, dtype=torch.int32, device="cuda")
+    assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), n_tok, n_vis, n_vis, k_blk, RATIO, pos0, width)
+    got = host(d_sel)
+    for t in list(range(min(n_tok, 6))) + [n_tok - 1]:
+        assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, n_vis, k_blk, RATIO, pos0 + t, width)[0]), t
