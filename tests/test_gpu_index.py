@@ -410,3 +410,42 @@ def test_scores_that_are_not_numbers_are_ordered_by_their_bits(oracle, n_tok, n_
     got = host(d_sel)
     for t in list(range(min(n_tok, 6))) + [n_tok - 1]:
         assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, n_vis, k_blk, RATIO, pos0 + t, width)[0]), t
+
+
+@pytest.mark.parametrize("n_tok,n_vis", [(149, 24576), (149, 24577), (148, 40001), (300, 40001)])
+def test_selection_where_many_keys_share_leading_bits(oracle, n_tok, n_vis):
+    """on both sides of the sampled form's rule: rows whose threshold lies in the pivot's bin of 256 keys, whose last 8 bits then
+    decide; exactly as many keys above the bin as are needed, one fewer, as many as there is room for, one more; a bin with too
+    few keys behind it; NaN of both signs"""
+    L = lib()
+    k_blk, stride = 512, n_vis + 3
+    rng = np.random.default_rng(n_vis + n_tok)
+    step = n_vis // 2048
+    i = np.arange(200, dtype=np.uint64)
+    at = np.minimum(i * step + ((i * 0x9E3779B1 % 2**32) >> 16) % step, n_vis - 1)
+    sc = np.zeros((n_tok, stride), np.float32)
+
+    def near(x, n):   # one value's leading 24 bits, any last 8
+        return (np.full(n, x, np.float32).view(np.uint32) & ~np.uint32(255) | rng.integers(0, 256, n, dtype=np.uint32)).view(np.float32)
+    for t in range(n_tok):
+        kind, some = t % 10, rng.permutation(n_vis)
+        sc[t] = near(1.0, stride) if kind in (0, 1, 2) else 0.0
+        if kind in (1, 2, 3, 4, 5, 6):
+            above = {1: 511, 2: 512, 3: 511, 4: 512, 5: 2048, 6: 2049}[kind]
+            sc[t, some[:above]] = 3 + rng.random(above)
+        if kind == 7:
+            sc[t] = np.abs(rng.standard_normal(stride)) * 0.1
+            sc[t, at] = near(9.0, 200)
+        if kind == 8:
+            sc[t, some[:300]] = np.nan
+            sc[t, some[300:600]] = -np.float32(np.nan)
+            sc[t, some[600:2000]] = -0.0
+        if kind == 9:
+            sc[t] = near(-2.0, stride)
+    pos0, width = n_vis * RATIO - n_tok, k_blk * RATIO + 3
+    d = torch.from_numpy(sc).cuda()
+    d_sel = torch.full((n_tok, width), -7, dtype=torch.int32, device="cuda")
+    assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), n_tok, n_vis, stride, k_blk, RATIO, pos0, width)
+    got = host(d_sel)
+    for t in list(range(10)) + [n_tok - 1]:
+        assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, stride, k_blk, RATIO, pos0 + t, width)[0]), t
