@@ -150,3 +150,36 @@ def test_draft_tokens_of_one_session_see_each_other(oracle, kind):
     assert L.q4_gpu_last_error() == 0
     b.close()
     st.close()
+
+
+@pytest.mark.parametrize("kind,n_head,hd", [(2, 16, 128), (1, 16, 128), (2, 24, 256), (1, 24, 256), (0, 24, 256)])
+def test_dense_append_is_stored_by_the_split_that_holds_the_row(kind, n_head, hd):
+    """launches sized for a long store, whose blocks meet over the grid: the new row at the edges of 16-row tiles, in the last block
+    that is used and in the last of all; every byte of the store as append_d leaves it; a position beyond the store is reported
+    and stores nothing"""
+    L = lib()
+    n_kvh, cap = 2, 60000
+    kvw = n_kvh * hd
+    g = torch.Generator(device="cuda").manual_seed(hd + kind)
+    a, b = q4gpu.KVStore(1, n_kvh, hd, cap, kind), q4gpu.KVStore(1, n_kvh, hd, cap, kind)
+    k, v = torch.randn(cap, kvw, device="cuda", generator=g), torch.randn(cap, kvw, device="cuda", generator=g)
+    a.append(0, k, v, 0, cap)
+    b.append(0, k, v, 0, cap)
+    q = torch.randn(n_head * hd, device="cuda", generator=g)
+    oa, ob = torch.zeros(n_head * hd, device="cuda"), torch.zeros(n_head * hd, device="cuda")
+    for pos in (0, 15, 16, 2047, 2048, 30000, 32767, 45003, cap - 17, cap - 16, cap - 1, cap, cap + 40):
+        nk, nv = torch.randn(kvw, device="cuda", generator=g), torch.randn(kvw, device="cuda", generator=g)
+        L.q4_hip_pos_push(pos)
+        b.append_decode_d(0, nk, nv, q, ob, n_head, 0.0884)
+        torch.cuda.synchronize()
+        if pos >= cap:
+            assert L.q4_gpu_last_error() == 4, pos
+        else:
+            a.append_d(0, nk, nv)
+            a.decode(0, q, oa, n_head, 0.0884)
+            assert_close(host(ob), host(oa), "position %d" % pos)
+            assert L.q4_gpu_last_error() == 0, pos
+        for which in (0, 1):
+            assert np.array_equal(ref_bytes(a, 0, which, 0, cap), ref_bytes(b, 0, which, 0, cap)), (pos, which)
+    a.close()
+    b.close()
