@@ -96,6 +96,7 @@ struct Q4State {
     struct { uint64_t number; Q4Touch touch; } flight[4];
     uint32_t n_flight;
     cudaGraphNode_t last_node;
+    uint32_t n_apart, last_graph_apart;   /* launches apart in this capture, in the last finished one */
     /* attention scratch: split-KV partial records + per-unit arrival counters */
     float *part;
     size_t part_floats;
@@ -115,7 +116,8 @@ void q4i_in_capture(const Q4Touch *touch);
 inline bool q4i_launched(bool ok, const Q4Touch *touch = nullptr, bool apart = false) {
     if (!ok) return false;
     g_q4.launches++;
-    if (!apart) g_q4.settled = g_q4.launches;
+    if (apart) g_q4.n_apart++;
+    else g_q4.settled = g_q4.launches;
     if (g_q4.capturing) q4i_in_capture(touch);
     return true;
 }

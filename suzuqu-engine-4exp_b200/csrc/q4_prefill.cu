@@ -926,6 +926,7 @@ __global__ void __launch_bounds__(256) q4_pf_merge_k(const std::conditional_t<TA
 /* operand images of the rows a chunk can see, and the parts of split ranges; grows on demand, never inside a capture */
 uint8_t *g_stage = nullptr;
 size_t g_stage_bytes = 0;
+uint32_t g_layout[3] = {};   /* of the last chunk: whole items, split ones, their ranges */
 /* 1 = there, 0 = an error, -1 = not to be had: inside a capture, or no memory is left for it */
 int stage_reserve(size_t bytes) {
     if (bytes <= g_stage_bytes) {
@@ -1016,6 +1017,12 @@ void q4i_prefill_release() {
     g_stage_bytes = 0;
 }
 
+extern "C" void q4_gpu_prefill_layout(uint32_t *whole, uint32_t *split, uint32_t *ranges) {
+    if (whole) *whole = g_layout[0];
+    if (split) *split = g_layout[1];
+    if (ranges) *ranges = g_layout[2];
+}
+
 int q4i_prefill(const Q4PrefillArgs &a) {
     const uint32_t gqa = a.n_head / a.n_kvh, hd = a.hd;
     const uint64_t n64 = (uint64_t)a.kv_base + a.n_tok;
@@ -1045,6 +1052,7 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     }
     if (room != 1) return room;
     const uint32_t split = sp.ranges;
+    g_layout[0] = sp.whole; g_layout[1] = blocks - sp.whole; g_layout[2] = split;
 
     PrefillTail p;
     memset(&p, 0, sizeof(p));

@@ -364,6 +364,7 @@ extern "C" int q4_hip_graph_begin(void) {
     g_q4.unsettled = g_q4.launches;
     g_q4.n_flight = 0;
     g_q4.last_node = nullptr;
+    g_q4.n_apart = 0;
     return 1;
 }
 extern "C" void *q4_hip_graph_end(void) {
@@ -372,6 +373,7 @@ extern "C" void *q4_hip_graph_end(void) {
     g_q4.unsettled = g_q4.launches;
     g_q4.n_flight = 0;
     g_q4.last_node = nullptr;
+    g_q4.last_graph_apart = g_q4.n_apart;
     cudaGraph_t g = nullptr;
     if (cudaStreamEndCapture(g_q4.stream, &g) != cudaSuccess || !g) {
         (void)cudaGetLastError();
@@ -398,6 +400,7 @@ extern "C" uint32_t q4_hip_graph_nodes(void *exec) {
     (void)exec;
     return g_q4.last_graph_nodes;
 }
+extern "C" uint32_t q4_gpu_graph_apart(void) { return g_q4.last_graph_apart; }
 extern "C" bool q4_hip_graph_launch(void *exec) {
     if (!g_q4.ok || !exec) return false;
     g_q4.unsettled = g_q4.launches;

@@ -149,3 +149,129 @@ def test_foreign_work_in_a_capture_is_waited_for():
         assert np.array_equal(row, (src[-HD:] * 2).half().cpu().numpy()), i
     L.q4_hip_graph_free(graph)
     b.free()
+
+
+def captured(L, calls, launches=1, before=None):
+    """the calls as one graph, launched; how many of them may run beside their predecessor"""
+    assert L.q4_hip_graph_begin() == 1
+    for c in calls:
+        assert c() in (True, None)
+    graph = L.q4_hip_graph_end()
+    assert graph
+    n = L.q4_gpu_graph_apart()
+    for _ in range(launches):
+        if before:
+            before()
+        assert L.q4_hip_graph_launch(graph) and L.q4_hip_stream_sync()
+    L.q4_hip_graph_free(graph)
+    return n
+
+
+def test_which_neighbours_run_apart():
+    """independent neighbours do, up to four behind one that did not; every kind of conflict, foreign work and a position that is
+    written meanwhile keep the order"""
+    L = q4gpu.init()
+    assert L.q4_gpu_set_stream(None)
+    sizes = {"wn": HD * 4, "arena": 4 * KVW * 4 + 64}
+    for i in "0123456":
+        sizes.update({"k" + i: KVW * 4, "raw" + i: ROWS * HD * 2, "pool" + i: ROWS // 4 * HD * 4})
+    b = Buffers(L, sizes, 5)
+    b.reset()
+    p = b.p
+    L.q4_hip_pos_push(7)
+    k_prep = lambda k: lambda: L.q4_hip_qsa_k_prep_d(k, p["wn"], N_KVH, HD, 64, 1e4, 1e-6)
+    f16 = lambda raw, src: lambda: L.q4_hip_f32_to_f16_d(raw, HD, src, HD)
+    pool = lambda raw, out: lambda: L.q4_hip_qsa_pool_d(raw, out, p["wn"], HD, 4, 64, 1e4, 1e-6)
+    copy = lambda d, s: lambda: L.q4_hip_copy(d, s, HD)
+    arena = p["arena"]
+    assert captured(L, [k_prep(p["k0"]), f16(p["raw0"], p["k1"])]) == 1
+    assert captured(L, [f16(p["raw0"], p["k1"]), pool(p["raw1"], p["pool0"])]) == 1
+    assert captured(L, [k_prep(p["k0"]), f16(p["raw0"], p["k0"])]) == 0                                  # read after write
+    assert captured(L, [f16(p["raw0"], p["k0"]), pool(p["raw0"], p["pool0"])]) == 0
+    assert captured(L, [f16(p["raw0"], p["k0"]), k_prep(p["k0"])]) == 0                                  # write after read
+    assert captured(L, [k_prep(p["k0"]), k_prep(p["k0"])]) == 0                                          # write after write
+    assert captured(L, [k_prep(p["k0"]), k_prep(p["k1"]), f16(p["raw0"], p["k0"])]) == 1   # with the launch before last
+    assert captured(L, [k_prep(p["k0"]), copy(p["k2"], p["k3"]), f16(p["raw0"], p["k1"])]) == 0          # another node between
+    assert captured(L, [k_prep(p["k0"]), lambda: L.q4_hip_pos_push(7), f16(p["raw0"], p["k1"])]) == 0
+    # rows of one allocation: next to each other, and one float of overlap
+    assert captured(L, [k_prep(arena), k_prep(arena + KVW * 4)]) == 1
+    assert captured(L, [k_prep(arena), k_prep(arena + KVW * 4 - 8)]) == 0
+    assert captured(L, [k_prep(arena + KVW * 4), k_prep(arena + 8)]) == 0
+    # a row whose place the device knows is taken to reach to the end of its allocation
+    assert captured(L, [k_prep(arena + 2 * KVW * 4), f16(arena, p["k0"])]) == 0
+    assert captured(L, [k_prep(arena), f16(arena + 2 * KVW * 4, p["k0"])]) == 1
+    assert captured(L, [f16(p["raw" + i], p["k" + i]) for i in "012345"]) == 4                           # the sixth waits
+    assert captured(L, [f16(p["raw" + i], p["k" + i]) for i in "0123456"]) == 5
+    b.free()
+    assert L.q4_gpu_last_error() == 0
+
+
+def test_weights_and_position_written_by_the_launch_before_last():
+    """read on every SM, written, a launch that is waited for, and then a launch apart that reads them"""
+    L = q4gpu.init()
+    assert L.q4_gpu_set_stream(None)
+    wide = 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    b = Buffers(L, {"wn": HD * 4, "q0": wide * HD * 4, "q1": wide * HD * 4, "q2": wide * HD * 4, "k0": KVW * 4, "k1": KVW * 4}, 6)
+    p = b.p
+
+    def ops(pos):
+        return [lambda: L.q4_hip_qsa_k_prep_d(p["q0"], p["wn"], wide, HD, 64, 1e4, 1e-6),
+                lambda: L.q4_hip_qsa_k_prep_d(p["wn"], None, 1, HD, 64, 1e4, 1e-6),
+                lambda: L.q4_hip_qsa_k_prep_d(p["k0"], p["wn"], N_KVH, HD, 64, 1e4, 1e-6),
+                lambda: L.q4_hip_qsa_k_prep_d(p["q1"], p["wn"], wide, HD, 64, 1e4, 1e-6),
+                lambda: L.q4_hip_pos_push(pos),
+                lambda: L.q4_hip_qsa_k_prep_d(p["k1"], p["wn"], N_KVH, HD, 64, 1e4, 1e-6),
+                lambda: L.q4_hip_qsa_k_prep_d(p["q2"], p["wn"], wide, HD, 64, 1e4, 1e-6)]
+
+    b.reset()
+    L.q4_hip_pos_push(11)
+    for op in ops(5000):
+        assert op() in (True, None) and L.q4_hip_stream_sync()
+    want = b.read()
+    results = []
+
+    def before():
+        results.append(b.read())
+        b.reset()
+        L.q4_hip_pos_push(11)
+    assert captured(L, ops(5000), launches=12, before=before) == 2
+    results.append(b.read())
+    for got in results[1:]:
+        for n in want:
+            assert np.array_equal(got[n], want[n]), n
+    b.free()
+    assert L.q4_gpu_last_error() == 0
+
+
+@pytest.mark.parametrize("dependent", [False, True])
+def test_launch_behind_a_long_attention(dependent):
+    """pooling runs beside a store's append + attention; the norm of the attention's output waits for it, long as that is"""
+    L = q4gpu.init()
+    assert L.q4_gpu_set_stream(None) and L.q4_hip_qsa_topk_alloc()
+    rows = 60000
+    b = Buffers(L, {"raw0": rows * HD * 2, "pool0": rows // 4 * HD * 4, "wn": HD * 4, "out0": QW * 4}, 7)
+    p = b.p
+    with torch.cuda.stream(torch.cuda.ExternalStream(L.q4_gpu_stream())):
+        g = torch.Generator(device="cuda").manual_seed(3)
+        st = q4gpu.KVStore(1, N_KVH, HD, rows, 2)
+        st.append(0, torch.randn(rows - 1, KVW, device="cuda", generator=g), torch.randn(rows - 1, KVW, device="cuda", generator=g), 0, rows - 1)
+        k, v, q = (torch.randn(n, device="cuda", generator=g) for n in (KVW, KVW, QW))
+        L.q4_hip_pos_push(rows - 1)
+
+        def attend():
+            return L.q4_gpu_kv_append_decode_d(st.h, 0, k.data_ptr(), v.data_ptr(), q.data_ptr(), 0, None, p["out0"], N_HEAD, None, 0, 0, 0.09)
+
+        def behind():
+            if dependent:
+                return L.q4_hip_qsa_k_prep_d(p["out0"], p["wn"], N_HEAD, HD, 64, 1e4, 1e-6)
+            return L.q4_hip_qsa_pool_d(p["raw0"], p["pool0"], p["wn"], HD, 4, 64, 1e4, 1e-6)
+        b.reset()
+        assert attend() and L.q4_hip_stream_sync() and behind() and L.q4_hip_stream_sync()
+        want = b.read()
+        for _ in range(4):
+            assert captured(L, [attend, behind], before=b.reset) == (0 if dependent else 1)
+            got = b.read()
+            assert all(np.array_equal(got[n], want[n]) for n in want)
+        st.close()
+    b.free()
+    assert L.q4_gpu_last_error() == 0

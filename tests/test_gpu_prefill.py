@@ -1,6 +1,8 @@
 """GPU parity of the tensor-core (tcgen05) causal prefill attention against the CPU oracle.
 Outputs are bf16 by contract, so the comparison allows one bf16 rounding of the result on top of
 the stated 2e-3 max-abs / 1e-3 relative tolerance."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -427,9 +429,10 @@ def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle, size
 
 @pytest.mark.parametrize("n_head,n_kvh,n_tok,kv_base", [(16, 2, 3000, 0), (16, 2, 3000, 2100), (16, 2, 5003, 37), (16, 2, 1300, 1500), (16, 1, 4900, 300), (9, 3, 2600, 900),
                                                         (64, 4, 1205, 500)])
-def test_last_wave_in_ranges_of_positions(n_head, n_kvh, n_tok, kv_base):
-    """chunks of one to three waves of blocks and a remainder, whose blocks are split; against chunks of 200 tokens, which are
-    other blocks in other ranges, each within the tolerance of the oracle's tests.  And as many bytes again behind the output."""
+def test_last_wave_of_whole_blocks(n_head, n_kvh, n_tok, kv_base):
+    """chunks of one to three waves of blocks and a remainder, over prefixes too short for the last wave to be split (it is in
+    test_last_wave_split_over_positions); against chunks of 200 tokens, which are other blocks in other ranges, each within the
+    tolerance of the oracle's tests.  And as many bytes again behind the output."""
     L = lib()
     hd, ctx = 128, kv_base + n_tok
     g = torch.Generator(device="cuda").manual_seed(n_tok)
@@ -447,3 +450,101 @@ def test_last_wave_in_ranges_of_positions(n_head, n_kvh, n_tok, kv_base):
     check(got[:n_tok], host(ref.float()), "tail %d over %d" % (n_tok, kv_base))
     assert (got[n_tok:] == 7.0).all() and L.q4_gpu_last_error() == 0
     st.close()
+
+
+def exact_attention(q, k, v, gate, n_head, n_kvh, kv_base, scale):
+    """all tokens of a chunk, 64 bits; k and v are [row][kv head][hd]"""
+    n, rows = q.shape[0], k.shape[0]
+    ref = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    for t in range(0, n, 1000):
+        m = min(1000, n - t)
+        hidden = torch.arange(rows, device="cuda")[None, :] > (kv_base + t + torch.arange(m, device="cuda"))[:, None]
+        for h in range(n_head):
+            s = (q[t:t + m, h].double() @ k[:, h // (n_head // n_kvh)].T * scale).masked_fill(hidden, float("-inf"))
+            ref[t:t + m, h] = torch.softmax(s, -1) @ v[:, h // (n_head // n_kvh)]
+    return host(ref * torch.sigmoid(gate.double()))
+
+
+def rows_of(raw, n, n_kvh, hd, kind):
+    """bytes in the reference's layout -> their values"""
+    if kind == 2:
+        b = raw.view(n, n_kvh, hd // 32, 34)
+        return (b[..., 2:].contiguous().view(torch.int8).double() * b[..., :2].contiguous().view(torch.float16).double()).reshape(n, n_kvh, hd)
+    return raw.view(torch.float16 if kind == 1 else torch.float32).view(n, n_kvh, hd).double()
+
+
+def layout(L):
+    a = (ctypes.c_uint32 * 3)()
+    L.q4_gpu_prefill_layout(ctypes.byref(a, 0), ctypes.byref(a, 4), ctypes.byref(a, 8))
+    return tuple(a)
+
+
+on_148_sms = pytest.mark.skipif(torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148,
+                                reason="how a chunk is split depends on the number of SMs")
+
+
+@on_148_sms
+@pytest.mark.parametrize("n_head,n_kvh,n_tok,kv_base,want", [
+    (16, 2, 3000, 6000, (148, 40, 3)), (64, 4, 766, 1000, (148, 44, 3)), (64, 4, 803, 2000, (148, 56, 2)), (64, 4, 1205, 3000, (296, 8, 9)),
+    (16, 1, 4900, 12000, (296, 11, 12)), (9, 3, 2600, 6000, (148, 38, 3)),   # groups of tokens that do not fill their rows
+    (16, 2, 1300, 4000, (148, 16, 9)),                                       # one query group per block
+    (24, 8, 903, 8000, (148, 28, 5)),                                        # a last wave over the end of a kv head
+    (16, 2, 3000, 2100, (188, 0, 1))])                                       # too short a prefix
+def test_last_wave_split_over_positions(n_head, n_kvh, n_tok, kv_base, want):
+    """the blocks of a chunk's last wave are split; all tokens against 64 bits, twice the same, and nothing is written behind the output"""
+    L = lib()
+    hd, ctx = 128, kv_base + n_tok
+    g = torch.Generator(device="cuda").manual_seed(n_tok)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    st = q4gpu.KVStore(1, n_kvh, hd, ctx, 2)
+    st.append(0, rn(ctx, n_kvh * hd), rn(ctx, n_kvh * hd), 0, ctx)
+    q, gate = rn(n_tok, n_head, hd).bfloat16(), rn(n_tok, n_head, hd)
+    outs = []
+    for _ in range(2):
+        out = torch.full((n_tok + 64, n_head, hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        st.prefill(0, q, out, n_head, n_tok, kv_base, 1 / np.sqrt(hd), gate=gate)
+        assert layout(L) == want
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and (outs[0][n_tok:] == 7.0).all()
+    raw = [torch.empty(ctx * st.token_bytes, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    for which in (0, 1):
+        st.export(0, which, 0, ctx, raw[which])
+    k, v = (rows_of(r, ctx, n_kvh, hd, 2) for r in raw)
+    check(host(outs[0][:n_tok].float()), exact_attention(q, k, v, gate, n_head, n_kvh, kv_base, 1 / np.sqrt(hd)), "%d over %d" % (n_tok, kv_base))
+    assert L.q4_gpu_last_error() == 0
+    st.close()
+
+
+@on_148_sms
+@pytest.mark.parametrize("kind,n_head,hd,n_tok,kv_base,want", [
+    (2, 24, 256, 800, 2048, (148, 12, 9)), (1, 24, 256, 800, 2048, (148, 12, 6)), (0, 24, 256, 1000, 4000, (148, 52, 2)),
+    (2, 24, 256, 1000, 4000, (148, 52, 2)),
+    (2, 16, 128, 1300, 4000, (148, 16, 9)),                                       # value and remainder
+    (0, 16, 128, 1500, 4000, (148, 40, 3)), (1, 16, 128, 3000, 6000, (148, 40, 3))])   # one and two query groups per block, marks
+def test_last_wave_split_over_positions_of_a_callers_cache(kind, n_head, hd, n_tok, kv_base, want):
+    from gpu_util import assert_close
+    L = lib()
+    n_kvh, ctx = 2, kv_base + n_tok
+    g = torch.Generator(device="cuda").manual_seed(n_tok + kind)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    raw = []
+    for _ in range(2):
+        x = rn(ctx, n_kvh * hd)
+        r = torch.empty(ctx * n_kvh * {2: hd // 32 * 34, 1: hd * 2, 0: hd * 4}[kind], dtype=torch.uint8, device="cuda")
+        if kind == 0:
+            r.copy_(x.view(torch.uint8).view(-1))
+        else:
+            assert (L.q4_hip_f32_to_q8 if kind == 2 else L.q4_hip_f32_to_f16)(r.data_ptr(), x.data_ptr(), x.numel())
+        raw.append(r)
+    q, gate = rn(n_tok, n_head, hd), rn(n_tok, n_head, hd)
+    scale = float(1 / np.sqrt(hd))
+    outs = []
+    for _ in range(2):
+        out = torch.full((n_tok + 64, n_head, hd), 7.0, device="cuda")
+        assert L.q4_hip_qsa_decode_n(q.data_ptr(), raw[0].data_ptr(), raw[1].data_ptr(), gate.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, n_tok, kv_base, ctx, scale, kind)
+        assert layout(L) == want
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and (outs[0][n_tok:] == 7.0).all()
+    k, v = (rows_of(r, ctx, n_kvh, hd, kind) for r in raw)
+    assert_close(host(outs[0][:n_tok]), exact_attention(q, k, v, gate, n_head, n_kvh, kv_base, scale), "%d over %d" % (n_tok, kv_base))
+    assert L.q4_gpu_last_error() == 0
