@@ -429,7 +429,7 @@ def test_chunk_captured_without_its_workspace_is_the_decode_kernels(oracle, size
 
 @pytest.mark.parametrize("n_head,n_kvh,n_tok,kv_base", [(16, 2, 3000, 0), (16, 2, 3000, 2100), (16, 2, 5003, 37), (16, 2, 1300, 1500), (16, 1, 4900, 300), (9, 3, 2600, 900),
                                                         (64, 4, 1205, 500)])
-def test_last_wave_of_whole_blocks(n_head, n_kvh, n_tok, kv_base):
+def test_last_wave_in_ranges_of_positions(n_head, n_kvh, n_tok, kv_base):
     """chunks of one to three waves of blocks and a remainder, over prefixes too short for the last wave to be split (it is in
     test_last_wave_split_over_positions); against chunks of 200 tokens, which are other blocks in other ranges, each within the
     tolerance of the oracle's tests.  And as many bytes again behind the output."""
