@@ -1355,9 +1355,9 @@ q4_decode_k(const DecParams P) {
         };
         if (!early) request_q();
         first_positions();
-        /* ---- fused append, second half.  Every split of the unit quantises and stores the unit's newest row
-         * (identical bytes from every split, so no block depends on another having written); a block's own
-         * store is ordered before its later reads by the barrier.  A warp whose first four tiles do not name the
+        /* ---- fused append, second half.  Over a list every split of the unit quantises and stores the unit's newest row
+         * (identical bytes from every split, so no block depends on another having written), in a dense scan the split
+         * that reads it; a block's own store is ordered before its later reads by the barrier.  A warp whose first four tiles do not name the
          * newest row fills its ring before that, so the append runs under the first copies. */
         if (!hold) fill();
         if (early) {

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
  * at once, and where a block has more than SC1_SHORT rows a lane walks two (6 reads per 4 dims of 64 rows).  Chunk c of row r
  * lies at c ^ (r & 7): 16-byte reads of eight consecutive rows fall into eight different bank groups, without the padding
  * that would not fit.  Eight steps in line, not 32: the kernel's image is fetched anew by every launch.
- * us, the form above / here: 64 rows 2.57 / 2.4, 4096 2.66 / 2.66, 16 384 4.28 / 4.1, 32 768 6.66 / 5.2, 65 536 9.3 / 8.5. */
+ * us, the form above / here: 64 rows 2.57 / 2.4, 4096 2.66 / 2.14, 16 384 4.28 / 4.1, 32 768 6.66 / 5.2, 65 536 9.3 / 8.5. */
 constexpr uint32_t SC1_WARPS = 7, SC1_ROWS = SC1_WARPS * 64, SC1_SHORT = 128, SC1_SMEM = IX_HD * (uint32_t)sizeof(float4) + SC1_ROWS * IX_HD * (uint32_t)sizeof(float);
 /* rows at .. at + 32 R - 1, below r1, by one warp */
 template <int R>

@@ -126,8 +126,9 @@ bool q4i_apart(const Q4Touch &touch) {
 }
 
 /* Scratch for the split-KV records and arrival counters.  Grows only outside capture (an
- * allocation would invalidate the capture, src/q4_rocm.cu:55-57); counters start at zero and every
- * kernel leaves them at zero. */
+ * allocation would invalidate the capture, src/q4_rocm.cu:55-57).  Counters start at zero.  At rest the arrival words of a unit
+ * are zero, and the two of its grid merge, which count on from launch to launch, are equal: every user of the array has the same
+ * words per unit (DEC_CTR). */
 bool q4i_scratch(size_t part_floats, size_t n_counters) {
     if (part_floats > g_q4.part_floats) {
         if (g_q4.capturing) return q4i_fail(Q4E_SCRATCH, "attention scratch too small inside a capture");
