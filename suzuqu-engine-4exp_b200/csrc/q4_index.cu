@@ -16,8 +16,8 @@
  * per pooled block with the tree in shuffles, a thread per pooled block for the scan with each warp's
  * 32 rows staged in shared memory by coalesced asynchronous copies (many tokens: a tiled product with the
  * same chains), and ONE launch for the whole selection instead of the reference's 12 per token, in one of
- * three forms: a cluster of 1, 2, 4 or 8 blocks per token with the keys in registers, the counts of a
- * 12-bit digit summed through distributed shared memory and the threshold bin's keys pushed to every
+ * three forms: a cluster of 1, 2, 4 or 8 blocks per token with the keys in registers, a pivot from the
+ * threads' maxima summed through distributed shared memory and the keys that reach it pushed to every
  * block; many tokens at once, a block each that streams its row twice into an index-ordered bitmap; rows
  * longer than 65 536 blocks, one block that re-reads the row, 16 independent loads at a time.
  */
@@ -748,16 +748,24 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topk1_k(const float *scor
 }
 
 /* ---- selection with the keys in registers (rows of up to 65 536 pooled blocks = ctx 262 144): a cluster of
- * NB = 1, 2, 4 or 8 blocks (8192 keys each), 8 keys per thread; block r, warp w, step i, lane l holds index
- * 8192 r + 256 w + 32 i + l, so (r, w, i, l) is ascending index order.  Latency-bound: a token's selection is a
- * chain of meetings, so the chain is kept short.  A first digit of 12 bits (sign, exponent, 3 mantissa bits)
- * leaves under 1 % of a row's keys in the threshold bin; every block adds its occupied bins to EVERY block's sum
- * (no read-back after the meeting), and pushes its keys of the threshold bin to every block, which then finishes
- * the remaining 20 bits alone.  Two cluster meetings after the launch wait (one block: none); the four
- * meetings and the read-backs of the earlier 8-bit form cost 14.5 us at 65 536 keys and 15.6 us at 8192. */
+ * NB = 1, 2, 4 or 8 blocks (8192 keys each), 8 keys per thread; block r, step i, thread t holds index 8192 r + 1024 i + t.
+ * Bound by latency and by issue: 32 warps share an SM's four schedulers, so every instruction per key is paid for eight times,
+ * and what keeps the chain short is that all keys are looked at twice only.
+ *   pivot    the digit (12 bits: sign, exponent, 3 mantissa bits) of the need-th largest among the threads' own maxima: at least
+ *            `need` keys reach it, and not many more than that do (8192 normal scores: 820 for 512).  A thread's keys are 1024
+ *            apart, so that a run of high scores is many threads' maxima.  One count per thread instead of eight.  In a cluster
+ *            every block adds its occupied bins to EVERY block's sum: no read-back after the meeting.
+ *   collect  the keys that reach it into shared memory; in a cluster to every block, which then finishes alone.
+ *   finish   one count of the collected keys by the next 12 bits (bins of 2^12 from the pivot's edge on), and the few in the
+ *            threshold's bin against one another.  Two cluster meetings after the launch wait (one block: none).
+ *   emit     every chosen key finds its place in the list from a bitmap of the block's keys.
+ * With the first digit counted over all keys, the threshold bin's keys collected by ballots, and two more passes of ballots
+ * over all keys for the list, a selection took 6.9 us of one block (8192 normal keys, a chain of such launches) and 9.5 of eight
+ * (65 536); now 5.4 and 6.9.  Rows of ties (all zeros 8.1 and 10.9 us, now 8.1 and 10.5) are counted digit by digit as before. */
 constexpr uint32_t TKC_KPT = 8, TKC_KEYS = IX_TK_THREADS * TKC_KPT, TKC_MAX_ROW = 8 * TKC_KEYS;
 constexpr uint32_t TK_BINS = 4096, TK_B1 = 20, TK_B2 = 8;   /* digits: bits 31..20, 19..8, 7..0 */
-constexpr uint32_t TKC_CAND = 512, TKC_CAND_ALL = 2048;     /* most threshold-bin keys of one block / of the cluster that are pushed */
+constexpr uint32_t TK_B2F = 12;   /* bits of a bin of collected keys */
+constexpr uint32_t TKC_NEAR = 32;                          /* keys of the threshold's bin that are compared with one another */
 __device__ __forceinline__ uint32_t tkc_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -793,27 +801,25 @@ __device__ __forceinline__ TkPick tk_pick(const uint32_t *hist, uint32_t target,
         c[j] = x.w; c[j + 1] = x.z; c[j + 2] = x.y; c[j + 3] = x.x;
         sum += (x.x + x.y) + (x.z + x.w);
     }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += y;
-    }
-    if (lane == 31) tot[w] = incl;
+    const uint32_t of_warp = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) tot[w] = of_warp;
     __syncthreads();
-    const uint32_t mine = lane < NT / 32 ? tot[lane] : 0u;   /* every warp scans the warp totals for itself */
-    uint32_t s = mine;
+    const uint32_t mine = lane < NT / 32 ? tot[lane] : 0u;
+    uint32_t above = __reduce_add_sync(0xffffffffu, lane < w ? mine : 0u);
+    if (above < target && above + of_warp >= target) {   /* one warp, which alone works out where in its bins */
+        uint32_t incl = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= (uint32_t)o) s += y;
-    }
-    uint32_t above = __shfl_sync(0xffffffffu, s - mine, w) + incl - sum;
-    if (above < target && above + sum >= target) {   /* exactly one thread */
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        above += incl - sum;
+        if (above < target && above + sum >= target) {   /* one thread */
 #pragma unroll
-        for (uint32_t j = 0; j < PER; j++) {
-            if (above + c[j] >= target) { st->digit = top - j; st->above = above; st->cnt = c[j]; break; }
-            above += c[j];
+            for (uint32_t j = 0; j < PER; j++) {
+                if (above + c[j] >= target) { st->digit = top - j; st->above = above; st->cnt = c[j]; break; }
+                above += c[j];
+            }
         }
     }
     __syncthreads();
@@ -854,14 +860,17 @@ __device__ __forceinline__ uint32_t tk_warp_prefix(uint32_t v, uint32_t *tot /* 
 
 template <uint32_t NB>
 struct TkcShared {
-    __align__(16) uint32_t ha[TK_BINS];   /* this block's counts of the first digit, then the candidates' of the second */
+    static constexpr uint32_t CAP = NB > 1 ? IX_TK_THREADS : 2u * IX_TK_THREADS;   /* collected keys of a block, at most */
+    __align__(16) uint32_t ha[TK_BINS];   /* this block's counts of the first digit; cluster: the collected keys' */
     __align__(16) uint32_t hb[NB > 1 ? TK_BINS : 4];   /* the cluster's counts of the first digit */
-    __align__(16) uint32_t h2[NB > 1 ? 4 : TK_BINS];   /* one block: counts of the second digit */
-    uint32_t h3[256], tot[3][32];
-    uint32_t cand[NB][TKC_CAND];          /* keys of the threshold bin, by the block that pushed them */
-    uint32_t ccnt[NB], gcnt[NB];          /* their counts; counts of the keys above that bin */
-    uint32_t cg[NB], ce[NB];              /* candidates above / at the threshold key */
-    uint32_t n_cand, n_above;
+    __align__(16) uint32_t h2[TK_BINS];   /* one block: the collected keys' counts; cluster: its counts of the second digit (rows of ties) */
+    __align__(16) uint32_t h3[256];       /* its counts of the third */
+    uint32_t bg[TKC_KEYS / 32], be[TKC_KEYS / 32], before[TKC_KEYS / 32];   /* this block's keys above / at the threshold, a bit each; those of earlier words */
+    uint32_t tot[4][32];
+    uint32_t cand[NB][CAP], idx[CAP];     /* the keys that each block has collected; this block's indices */
+    uint32_t ccnt[NB], gcnt[NB];          /* their counts; keys above the pivot's digit or the threshold (rows of ties) */
+    uint32_t n_own, n_near, n_above, low, n_tie;   /* low, n_tie: keys above (low half-word) and at the threshold of earlier blocks / of this one */
+    uint32_t near[TKC_NEAR], thr, n_gt;
     TkPick st[3];
 };
 template <uint32_t NB>
@@ -873,7 +882,7 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     const uint32_t t = blockIdx.y, tx = threadIdx.x, lane = tx & 31u, warp = tx >> 5, rank = NB > 1 ? tkc_rank() : 0u;
     /* A position that comes with the launch or is settled in its word tells before anything is prepared whether every complete
      * block fits, the list of a short context (one token, 512 blocks: 2.9 -> 2.4 us; costs the others 0.3 of 7.5). */
-    uint32_t pos = pos0 + t, n_read = t + 1u < gridDim.y ? stride : last_read;
+    uint32_t pos = pos0 + t, n_read = t + 1u < gridDim.y ? stride : last_read, n_vis = 0u;
     if (early) {
         if (pp) pos = (uint32_t)*pp;
         if (pos + 1u < (k_blk + 1u) * ratio) {   /* the same decision in all blocks */
@@ -881,18 +890,19 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
             for (uint32_t w = rank * IX_TK_THREADS + tx; w < width; w += NB * IX_TK_THREADS) sel[(size_t)t * width + w] = w <= pos ? (int32_t)w : -1;
             return;
         }
-        if (pp) n_read = min(stride, (pos + 1u) / ratio);
+        n_vis = (pos + 1u) / ratio;
+        if (pp) n_read = min(stride, n_vis);
     }
     /* The block's own shared memory is prepared, and the cluster has met once, before the launch waits for
      * the previous kernel: with programmatic dependent launch this part runs under that kernel's tail. */
     constexpr uint32_t BPT = TK_BINS / IX_TK_THREADS;   /* bins per thread */
     static_assert(BPT == 4, "one 16-byte word of counts per thread");
-    uint32_t *h2 = NB > 1 ? S.ha : S.h2;
+    uint32_t *hist = NB > 1 ? S.ha : S.h2;
     reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
-    reinterpret_cast<uint4 *>(NB > 1 ? S.hb : S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
-    if (tx < 256) S.h3[tx] = 0u;
-    if (tx < NB) { S.cg[tx] = 0u; S.ce[tx] = 0u; }
-    if (tx == 0) { S.n_cand = 0u; S.n_above = 0u; }
+    reinterpret_cast<uint4 *>(S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
+    if (NB > 1) reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
+    if (tx < 256) S.h3[tx] = S.bg[tx] = S.be[tx] = 0u;
+    if (tx == 0) S.n_own = S.n_near = S.n_above = S.low = S.n_tie = 0u;
     tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
     q4d_pdl_wait();
     /* The keys are requested before a position that has yet to be read arrives.  Only visible ones of the last row: a host's
@@ -902,12 +912,14 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         n_read = min(stride, (pos + 1u) / ratio);
     }
     const float *row = score + (size_t)t * stride;
-    const uint32_t base = rank * TKC_KEYS + warp * (32u * TKC_KPT) + lane;
+    const uint32_t base = rank * TKC_KEYS + tx;
     uint32_t key[TKC_KPT];
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + 32u * i < n_read ? __float_as_uint(__ldcg(row + base + 32u * i)) : 0u;
-    if (pos_arr) pos = (uint32_t)pos_arr[t];
-    const uint32_t n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = base + IX_TK_THREADS * i < n_read ? __float_as_uint(__ldcg(row + base + IX_TK_THREADS * i)) : 0u;
+    if (!early) {
+        if (pos_arr) pos = (uint32_t)pos_arr[t];
+        n_vis = ratio ? (pos + 1u) / ratio : 0u;
+    }
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
     int32_t *out = sel + (size_t)t * width;
     const uint32_t w_per = (width + NB - 1u) / NB;
@@ -916,179 +928,250 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         for (uint32_t w = w0 + tx; w < w1; w += IX_TK_THREADS) out[w] = w <= pos ? (int32_t)w : -1;
         return;
     }
+    /* ---- pivot: at least min(n_vis, 1024) threads have a key, which is `need` or more */
+    auto live = [&](uint32_t i) { return base + IX_TK_THREADS * i < n_vis; };
+    uint32_t most = 0u;
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) key[i] = ix_key(__uint_as_float(key[i]));
+    for (uint32_t i = 0; i < TKC_KPT; i++) {
+        key[i] = live(i) ? ix_key(__uint_as_float(key[i])) : 0u;
+        most = max(most, key[i]);
+    }
+    if (live(0)) atomicAdd(&S.ha[most >> TK_B1], 1u);
     /* the tail of the list (positions behind the last complete block) does not depend on the selection */
     const uint32_t ncs = need * ratio;
     for (uint32_t w = max(w0, ncs) + tx; w < w1; w += IX_TK_THREADS) {
         const uint32_t tail = n_vis * ratio + (w - ncs);
         out[w] = tail <= pos ? (int32_t)tail : -1;
     }
-#pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++)
-        if (base + 32u * i < n_vis) atomicAdd(&S.ha[key[i] >> TK_B1], 1u);
     __syncthreads();
     /* this block's counts into every block's sum; the local array is left at zero for the next digit */
-    auto spread = [&]() {
-        const uint4 c4 = reinterpret_cast<const uint4 *>(S.ha)[tx];
-        const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+    auto spread = [&](uint32_t *sum, uint32_t bins) {
 #pragma unroll
-        for (uint32_t j = 0; j < BPT; j++)
-            if (c[j])
-                for (uint32_t r = 0; r < NB; r++) tkc_red_add(tkc_remote(&S.hb[BPT * tx + j], r), c[j]);
-        reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t j = 0; j < BPT; j++) {   /* occupied bins are neighbours: one per thread */
+            const uint32_t at = tx + j * IX_TK_THREADS, c = at < bins ? S.ha[at] : 0u;
+            if (c) {
+#pragma unroll
+                for (uint32_t r = 0; r < NB; r++) tkc_red_add(tkc_remote(&sum[at], r), c);
+                S.ha[at] = 0u;
+            }
+        }
         tkc_sync<NB>();
     };
-    if (NB > 1) spread();
+    if (NB > 1) spread(S.hb, TK_BINS);
     const TkPick p1 = tk_pick<IX_TK_THREADS>(NB > 1 ? S.hb : S.ha, need, S.tot[0], &S.st[0]);
-    uint32_t thr, n_gt;      /* the need-th largest key, keys above it: n_gt < need <= n_gt + ties */
-    bool fast = p1.cnt <= TKC_CAND_ALL;
+    const uint32_t digit = p1.digit, edge = digit << TK_B1;
+    /* Where so many threads' maxima reach the pivot the keys are ties, and more than there is room for: of 8 keys per thread an
+     * eighth (a quarter, one block) are some among 11 (15) threads of 16.  (And a pivot of 0 could not be told from no key.) */
+    bool fast = digit != 0u && (n_vis <= S.CAP || (p1.above + p1.cnt) * 16u < (n_vis / TKC_KEYS * IX_TK_THREADS + min(n_vis % TKC_KEYS, IX_TK_THREADS)) * (NB > 1 ? 11u : 15u));
     if (fast) {
-        /* keys of the threshold bin to every block, in any order (a key is all that the rest needs); one add per
-         * warp reserves its slots and counts the keys above the bin */
-        uint32_t ng = 0, ne = 0, mq[TKC_KPT];
+        /* ---- collect, in any order: one add per warp */
+        uint32_t n = 0;
 #pragma unroll
-        for (uint32_t i = 0; i < TKC_KPT; i++) {
-            const bool live = base + 32u * i < n_vis;
-            ng += __popc(__ballot_sync(0xffffffffu, live && (key[i] >> TK_B1) > p1.digit));
-            mq[i] = __ballot_sync(0xffffffffu, live && (key[i] >> TK_B1) == p1.digit);
-            ne += __popc(mq[i]);
+        for (uint32_t i = 0; i < TKC_KPT; i++) n += key[i] >= edge;
+        uint32_t at = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= (uint32_t)o) at += y;
         }
-        if (lane == 0 && ng) atomicAdd(&S.n_above, ng);
-        if (ne) {
-            uint32_t slot = 0;
-            if (lane == 0) slot = atomicAdd(&S.n_cand, ne);
-            slot = __shfl_sync(0xffffffffu, slot, 0);
+        uint32_t slot = 0;
+        if (lane == 31 && at) slot = atomicAdd(&S.n_own, at);
+        at += __shfl_sync(0xffffffffu, slot, 31) - n;
 #pragma unroll
-            for (uint32_t i = 0; i < TKC_KPT; i++) {
-                const uint32_t at = slot + __popc(mq[i] & ((1u << lane) - 1u));
-                if (((mq[i] >> lane) & 1u) && at < TKC_CAND)
-                    for (uint32_t r = 0; r < NB; r++) {
-                        if (NB == 1) S.cand[0][at] = key[i];
-                        else tkc_st(tkc_remote(&S.cand[rank][at], r), key[i]);
-                    }
-                slot += __popc(mq[i]);
+        for (uint32_t i = 0; i < TKC_KPT; i++)
+            if (key[i] >= edge) {
+                if (at < S.CAP) {
+                    S.cand[rank][at] = key[i];
+                    S.idx[at] = IX_TK_THREADS * i + tx;
+                }
+                at++;
             }
-        }
         __syncthreads();
-        if (tx < NB) {
-            if (NB == 1) { S.ccnt[0] = S.n_cand; S.gcnt[0] = S.n_above; }
-            else {
-                tkc_st(tkc_remote(&S.ccnt[rank], tx), S.n_cand);
-                tkc_st(tkc_remote(&S.gcnt[rank], tx), S.n_above);
+        const uint32_t n_own = S.n_own;
+        if (NB > 1) {
+            if (tx < n_own && n_own <= S.CAP) {
+                const uint32_t k = S.cand[rank][tx];
+#pragma unroll
+                for (uint32_t r = 0; r < NB; r++)
+                    if (r != rank) tkc_st(tkc_remote(&S.cand[rank][tx], r), k);
             }
+            if (tx < NB) tkc_st(tkc_remote(&S.ccnt[rank], tx), n_own);
+            tkc_sync<NB>();   /* the last access to another block's shared memory, but for rows of ties */
+            for (uint32_t r = 0; r < NB; r++) fast = fast && S.ccnt[r] <= S.CAP;   /* same decision in all blocks */
+        } else {
+            fast = n_own <= S.CAP;
         }
-        tkc_sync<NB>();   /* the last access to another block's shared memory is behind this point */
-        for (uint32_t r = 0; r < NB; r++) fast = fast && S.ccnt[r] <= TKC_CAND;   /* same decision in all blocks */
     }
+    uint32_t thr = 0, n_gt = 0, low = 0;   /* the need-th largest key, keys above it: n_gt < need <= n_gt + ties; of earlier blocks, and their ties << 16 */
     if (fast) {
-        constexpr uint32_t CPT = (NB * TKC_CAND + IX_TK_THREADS - 1u) / IX_TK_THREADS;
-        uint32_t ck[CPT];
-        bool cl[CPT];
+        /* ---- finish: all collected keys, a warp's lanes at one block's; every block's begin at other warps, for they are a
+         * hundred or two each */
+        constexpr uint32_t CPT = NB > 1 ? NB : 2u;
+        uint32_t ck[CPT];   /* 0: none */
+        auto place = [&](uint32_t j) { return NB > 1 ? (tx - 128u * j) % IX_TK_THREADS : tx + j * IX_TK_THREADS; };
 #pragma unroll
         for (uint32_t j = 0; j < CPT; j++) {
-            const uint32_t i = tx + j * IX_TK_THREADS, r = i / TKC_CAND, c = i % TKC_CAND;
-            cl[j] = i < NB * TKC_CAND && c < S.ccnt[r];
-            ck[j] = cl[j] ? S.cand[r][c] : 0u;
-            if (cl[j]) atomicAdd(&h2[(ck[j] >> TK_B2) & (TK_BINS - 1u)], 1u);
+            const uint32_t c = place(j);
+            ck[j] = c < (NB > 1 ? S.ccnt[j % NB] : S.n_own) ? S.cand[j % NB][c] : 0u;
+            if (ck[j]) atomicAdd(&hist[min((ck[j] - edge) >> TK_B2F, TK_BINS - 1u)], 1u);
         }
         __syncthreads();
-        const TkPick p2 = tk_pick<IX_TK_THREADS>(h2, need - p1.above, S.tot[1], &S.st[1]);
-        const uint32_t pre = (p1.digit << 12) | p2.digit;
-        if (p2.cnt == 1u) {   /* 24 bits name one key: the threshold */
+        const TkPick p2 = tk_pick<IX_TK_THREADS>(hist, need, S.tot[1], &S.st[1]);
+        fast = p2.digit < TK_BINS - 1u;   /* else what reaches beyond the bins, four times the pivot */
+        if (!fast) n_gt = 0xffffffffu;
+        if (fast) {
+            const uint32_t left = need - p2.above;
+            if (p2.cnt <= TKC_NEAR) {   /* mostly one to three */
 #pragma unroll
-            for (uint32_t j = 0; j < CPT; j++)
-                if (cl[j] && (ck[j] >> TK_B2) == pre) S.h3[0] = ck[j];
-            __syncthreads();
-            thr = S.h3[0];
-            n_gt = p1.above + p2.above;
-        } else {
+                for (uint32_t j = 0; j < CPT; j++)
+                    if (ck[j] && (ck[j] - edge) >> TK_B2F == p2.digit) S.near[atomicAdd(&S.n_near, 1u)] = ck[j];
+                __syncthreads();
+                if (tx < p2.cnt) {
+                    const uint32_t k = S.near[tx];
+                    uint32_t more = 0, same = 0;
+                    for (uint32_t j = 0; j < p2.cnt; j++) {
+                        more += S.near[j] > k;
+                        same += S.near[j] == k;
+                    }
+                    if (more < left && left <= more + same) {
+                        S.thr = k;
+                        S.n_gt = p2.above + more;
+                    }
+                }
+            } else {   /* many keys share 24 bits */
+                uint32_t *h = NB > 1 ? S.hb : S.ha;
+                reinterpret_cast<uint4 *>(h)[tx] = make_uint4(0u, 0u, 0u, 0u);
+                __syncthreads();
 #pragma unroll
-            for (uint32_t j = 0; j < CPT; j++)
-                if (cl[j] && (ck[j] >> TK_B2) == pre) atomicAdd(&S.h3[ck[j] & 255u], 1u);
-            __syncthreads();
-            const TkPick p3 = tk_pick256(S.h3, need - p1.above - p2.above);
-            thr = (pre << 8) | p3.digit;
-            n_gt = p1.above + p2.above + p3.above;
-        }
-        if (NB > 1) {
-#pragma unroll
-            for (uint32_t j = 0; j < CPT; j++) {
-                const uint32_t r = (tx + j * IX_TK_THREADS) / TKC_CAND;   /* the same block in all lanes of a warp */
-                const uint32_t mg = __ballot_sync(0xffffffffu, cl[j] && ck[j] > thr), me = __ballot_sync(0xffffffffu, cl[j] && ck[j] == thr);
-                if (lane == 0 && mg) atomicAdd(&S.cg[r], (uint32_t)__popc(mg));
-                if (lane == 0 && me) atomicAdd(&S.ce[r], (uint32_t)__popc(me));
+                for (uint32_t j = 0; j < CPT; j++)
+                    if (ck[j] && (ck[j] - edge) >> TK_B2F == p2.digit) atomicAdd(&h[(ck[j] - edge) & (TK_BINS - 1u)], 1u);
+                __syncthreads();
+                const TkPick p3 = tk_pick<IX_TK_THREADS>(h, left, S.tot[2], &S.st[2]);
+                if (tx == 0) {
+                    S.thr = edge + (p2.digit << TK_B2F) + p3.digit;
+                    S.n_gt = p2.above + p3.above;
+                }
             }
-        }
-    } else {
-        /* Thousands of keys share the first digit (rows of ties): the second and third digit are counted over the
-         * rows' own keys as the first was, with a meeting to clear the sums and one to complete them. */
-        uint32_t pre = p1.digit, above = p1.above;
-#pragma unroll 1
-        for (uint32_t d = 1; d < 3; d++) {
-            const uint32_t sh = d == 1 ? TK_B2 : 0u, bits = d == 1 ? 12u : 8u;
             __syncthreads();
-            reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
-            if (NB > 1) reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
-            tkc_sync<NB>();
+            thr = S.thr;
+            n_gt = S.n_gt;
+#pragma unroll
+            for (uint32_t j = 0; j < CPT; j++)
+                if (ck[j] >= thr) {
+                    if (NB > 1 && j != rank) {
+                        if (j < rank) atomicAdd(&S.low, ck[j] > thr ? 1u : 1u << 16);
+                    } else {
+                        const uint32_t i = S.idx[place(j)];
+                        atomicOr(ck[j] > thr ? &S.bg[i >> 5] : &S.be[i >> 5], 1u << (i & 31u));
+                    }
+                }
+            __syncthreads();
+            low = S.low;
+        }
+    }
+    if (!fast) {
+        /* ---- Rows of ties: thousands of keys reach the pivot.  Where fewer than `need` are above its digit, that is the
+         * threshold's: the second digit is counted while the blocks tell one another how many those are.  Else the first digit
+         * is counted over all keys, after a meeting to clear the sums.  Then the third. */
+        auto sum = [&](uint32_t v, uint32_t *to) -> uint32_t {   /* over the block */
+            v = __reduce_add_sync(0xffffffffu, v);
+            if (lane == 0 && v) atomicAdd(to, v);
+            __syncthreads();
+            return *to;
+        };
+        const bool counted = NB == 1 || n_gt == 0xffffffffu;   /* the counts are not zero */
+        uint32_t n = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < TKC_KPT; i++) n += (key[i] >> TK_B1) > digit;
+        uint32_t above = sum(n, &S.n_above), pre = digit, d = 1;
+        if (NB > 1 && tx < NB) tkc_st(tkc_remote(&S.gcnt[rank], tx), above);
+        bool first = true;
+#pragma unroll 1
+        while (d < 3) {
+            const uint32_t sh = d == 0 ? TK_B1 : d == 1 ? TK_B2 : 0u, bits = d < 2 ? 12u : 8u;
+            if (NB == 1 || (first && counted)) {   /* in a cluster they are left at zero */
+                __syncthreads();
+                reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+                __syncthreads();
+            }
+            if (NB > 1 && d == 0) {
+                reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
+                reinterpret_cast<uint4 *>(S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
+                tkc_sync<NB>();
+            }
 #pragma unroll
             for (uint32_t i = 0; i < TKC_KPT; i++)
-                if (base + 32u * i < n_vis && (key[i] >> (sh + bits)) == pre) atomicAdd(&S.ha[(key[i] >> sh) & ((1u << bits) - 1u)], 1u);
+                if (live(i) && (d == 0 || (key[i] >> (sh + bits)) == pre)) atomicAdd(&S.ha[(key[i] >> sh) & ((1u << bits) - 1u)], 1u);
             __syncthreads();
-            if (NB > 1) spread();
-            const TkPick p = tk_pick<IX_TK_THREADS>(NB > 1 ? S.hb : S.ha, need - above, S.tot[d], &S.st[d]);
-            pre = (pre << bits) | p.digit;
+            uint32_t *h = NB == 1 ? S.ha : d == 0 ? S.hb : d == 1 ? S.h2 : S.h3;
+            if (NB > 1) spread(h, 1u << bits);
+            if (first) {
+                first = false;
+                if (NB > 1) {
+                    above = 0;
+                    for (uint32_t r = 0; r < NB; r++) above += S.gcnt[r];
+                }
+                if (above >= need) {
+                    d = 0;
+                    above = 0;
+                    continue;
+                }
+            }
+            const TkPick p = d == 2 ? tk_pick256(h, need - above) : tk_pick<IX_TK_THREADS>(h, need - above, S.tot[2], &S.st[2]);
+            pre = d == 0 ? p.digit : (pre << bits) | p.digit;
             above += p.above;
+            d++;
         }
         thr = pre;
         n_gt = above;
-    }
-    /* counts above and at the threshold: per warp by ballots, per block by one scan over the warps (ties in the
-     * high half-word: a block holds at most 8192 keys) */
-    uint32_t ng = 0, ne = 0;
+        n = 0;
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) {
-        const bool live = base + 32u * i < n_vis;
-        ng += __popc(__ballot_sync(0xffffffffu, live && key[i] > thr));
-        ne += __popc(__ballot_sync(0xffffffffu, live && key[i] == thr));
-    }
-    static_assert(TKC_KEYS < 65536, "two counts share a word");
-    const uint32_t off = tk_warp_prefix(ne << 16 | ng, S.tot[2]);   /* its barrier also completes cg and ce */
-    uint32_t og = off & 0xffffu, oe = off >> 16, g0 = 0;   /* g0: the block's first place in the list */
-    const uint32_t all = __reduce_add_sync(0xffffffffu, S.tot[2][lane]);
-    const uint32_t n_own = all & 0xffffu;                  /* this block's keys above the threshold */
-    if (NB > 1) {
-        if (!fast) {   /* every block tells the others its counts */
-            if (tx < NB) {
-                tkc_st(tkc_remote(&S.gcnt[rank], tx), n_own);
-                tkc_st(tkc_remote(&S.ce[rank], tx), all >> 16);
-            }
+        for (uint32_t i = 0; i < TKC_KPT; i++) {
+            const bool gt = live(i) && key[i] > thr, eq = live(i) && key[i] == thr;
+            const uint32_t mg = __ballot_sync(0xffffffffu, gt), me = __ballot_sync(0xffffffffu, eq);
+            if (lane == 0) { S.bg[32u * i + warp] = mg; S.be[32u * i + warp] = me; }
+            n += gt ? 1u : eq ? 1u << 16 : 0u;
+        }
+        static_assert(TKC_KEYS < 65536, "two counts share a word");
+        n = sum(n, &S.n_tie);
+        if (NB > 1) {   /* every block tells the others its counts */
+            if (tx < NB) tkc_st(tkc_remote(&S.gcnt[rank], tx), n);
             tkc_sync<NB>();
+            for (uint32_t r = 0; r < rank; r++) low += S.gcnt[r];
         }
-        for (uint32_t r = 0; r < rank; r++) { g0 += S.gcnt[r] + S.cg[r]; oe += S.ce[r]; }
     }
-    /* ordered emit: above the threshold in index order (collected in shared memory, so that the list is written in
-     * whole lines), then ties until `need` is full */
-    uint32_t *chosen = S.ha;   /* the counts are no longer needed; n_own < need <= 512 */
-    const uint32_t lt = (1u << lane) - 1u;
+    /* ---- ordered emit: above the threshold in index order, then ties until `need` is full */
+    if (tx < TKC_KEYS / 32u) {
+        const uint32_t v = __popc(S.bg[tx]) | __popc(S.be[tx]) << 16;
+        uint32_t at = v;
 #pragma unroll
-    for (uint32_t i = 0; i < TKC_KPT; i++) {
-        const uint32_t b = base + 32u * i;
-        const bool live = b < n_vis, gt = live && key[i] > thr, eq = live && key[i] == thr;
-        const uint32_t mg = __ballot_sync(0xffffffffu, gt), me = __ballot_sync(0xffffffffu, eq);
-        if (gt) chosen[og + __popc(mg & lt)] = b;
-        if (me) {
-            const uint32_t at = n_gt + oe + __popc(me & lt);
-            if (eq && at < need)
-                for (uint32_t j = 0; j < ratio && at * ratio + j < width; j++) out[at * ratio + j] = (int32_t)(b * ratio + j);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= (uint32_t)o) at += y;
         }
-        og += __popc(mg);
-        oe += __popc(me);
+        if (lane == 31) S.tot[3][warp] = at;
+        asm volatile("bar.sync 1, %0;" ::"n"(TKC_KEYS / 32u) : "memory");
+        S.before[tx] = at - v + __reduce_add_sync(0xffffffffu, lane < warp ? S.tot[3][lane] : 0u);
     }
     __syncthreads();
-    for (uint32_t w = tx; w < n_own * ratio && g0 * ratio + w < width; w += IX_TK_THREADS) {
-        const uint32_t i = w / ratio;
-        out[g0 * ratio + w] = (int32_t)(chosen[i] * ratio + (w - i * ratio));
+    auto put = [&](uint32_t k, uint32_t i) {   /* key i of the block's, which reaches the threshold */
+        const uint32_t w = i >> 5, below = (1u << (i & 31u)) - 1u, all = S.before[w] + low, b = rank * TKC_KEYS + i;
+        uint32_t at = k > thr ? all & 0xffffu : n_gt + (all >> 16);
+        if (at >= need) return;
+        at += __popc((k > thr ? S.bg[w] : S.be[w]) & below);
+        if (at < need)
+            for (uint32_t j = 0; j < ratio && at * ratio + j < width; j++) out[at * ratio + j] = (int32_t)(b * ratio + j);
+    };
+    if (fast) {
+#pragma unroll
+        for (uint32_t j = 0; j < S.CAP / IX_TK_THREADS; j++) {
+            const uint32_t c = tx + j * IX_TK_THREADS;
+            if (c < S.n_own && S.cand[rank][c] >= thr) put(S.cand[rank][c], S.idx[c]);
+        }
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < TKC_KPT; i++)
+            if (live(i) && key[i] >= thr) put(key[i], IX_TK_THREADS * i + tx);
     }
 }
 

@@ -449,3 +449,37 @@ def test_selection_where_many_keys_share_leading_bits(oracle, n_tok, n_vis):
     got = host(d_sel)
     for t in list(range(10)) + [n_tok - 1]:
         assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, stride, k_blk, RATIO, pos0 + t, width)[0]), t
+
+
+@pytest.mark.parametrize("n_vis", [513, 1025, 2049, 8192, 8193, 16500, 40000, 65536])
+def test_selection_from_the_threads_maxima(oracle, n_vis):
+    """one block and clusters of 2, 4 and 8; rows whose pivot is negative, whose highest keys are a few threads' or one run, reach
+    beyond the bins behind the pivot, share 24 bits with the threshold, are two values, or mostly NaN with a sign (a pivot of 0)"""
+    L = lib()
+    k_blk, kinds = 512, 10
+    rng = np.random.default_rng(n_vis)
+    sc = np.abs(rng.standard_normal((kinds, n_vis))).astype(np.float32)
+    i = np.arange(n_vis)
+    sc[1] = -1 - sc[1]
+    sc[2] = np.exp(6 * rng.standard_normal(n_vis))
+    sc[3, i % 1024 < 40] += 100
+    sc[4, n_vis // 3:n_vis // 3 + 700] += 6
+    some = rng.permutation(n_vis)
+    sc[5], sc[5, some[:511]] = 0.25, 2 + rng.random(511)   # one short of ties
+    sc[6, some[:480]] = 7 + rng.random(480)                 # the threshold among 40, then among 60 keys of the same 24 bits
+    near = np.full(100, 5.0, np.float32).view(np.uint32) + rng.integers(0, 256, 100, dtype=np.uint32)
+    sc[6, some[480:][:40]] = near.view(np.float32)[:len(some[480:][:40])]
+    sc[7] = sc[6]
+    sc[7, some[480:][:60]] = near.view(np.float32)[40:40 + len(some[480:][:60])]
+    sc[8] = np.where(rng.random(n_vis) < 0.5, np.float32(-0.0), np.float32(0.0))
+    sc[9, some[400:]] = (0xffffffff - rng.integers(0, 1 << 19, n_vis - 400, dtype=np.uint32)).view(np.float32)
+    pos0, width = n_vis * RATIO - kinds, k_blk * RATIO + 3
+    got = np.zeros((kinds, width), np.int32)
+    for t in range(kinds):
+        d, d_sel = torch.from_numpy(sc[t]).cuda(), torch.full((width,), -7, dtype=torch.int32, device="cuda")
+        assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), 1, n_vis, n_vis, k_blk, RATIO, pos0 + t, width)
+        got[t] = host(d_sel)
+        assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, n_vis, k_blk, RATIO, pos0 + t, width)[0]), t
+    d, d_sel = torch.from_numpy(sc).cuda(), torch.full((kinds, width), -7, dtype=torch.int32, device="cuda")
+    assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), kinds, n_vis, n_vis, k_blk, RATIO, pos0, width)
+    assert np.array_equal(host(d_sel), got)
