@@ -183,9 +183,10 @@ void *q4_gpu_download_stream(void);
 bool q4_gpu_set_stream(void *cuda_stream);
 int q4_gpu_device(void);
 /* How launches were laid out, for tests and profiles (no counterpart in the reference).  Of the last finished capture: the launches
- * that may run beside the one before them.  Of the last tensor-core chunk: the blocks' worth of work that are one block each, and
+ * that may run beside the one before them, and those that read pooled keys ahead of their wait for it.  Of the last tensor-core chunk: the blocks' worth of work that are one block each, and
  * those behind them that are `ranges` blocks each. */
 uint32_t q4_gpu_graph_apart(void);
+uint32_t q4_gpu_graph_ahead(void);
 void q4_gpu_prefill_layout(uint32_t *whole, uint32_t *split, uint32_t *ranges);
 /* A pipelined step loop over one set of step buffers (no counterpart in the reference, whose decode step
  * uploads, computes and reads back on one stream).  A host that decodes step after step from host buffers

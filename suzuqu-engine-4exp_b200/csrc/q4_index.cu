@@ -262,7 +262,9 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
  * at once, and where a block has more than SC1_SHORT rows a lane walks two (6 reads per 4 dims of 64 rows).  Chunk c of row r
  * lies at c ^ (r & 7): 16-byte reads of eight consecutive rows fall into eight different bank groups, without the padding
  * that would not fit.  Eight steps in line, not 32: the kernel's image is fetched anew by every launch.
- * us, the form above / here: 64 rows 2.57 / 2.4, 4096 2.66 / 2.14, 16 384 4.28 / 4.1, 32 768 6.66 / 5.2, 65 536 9.3 / 8.5. */
+ * us, the form above / here: 64 rows 2.57 / 2.4, 4096 2.66 / 2.14, 16 384 4.28 / 4.1, 32 768 6.66 / 5.2, 65 536 9.3 / 8.5.
+ * ahead: all blocks but the newest are requested before the wait (q4i_blocks_ahead), under whatever this launch's pooling still
+ * waits for: a 262144-token select step 298.5 -> 255 us, the reference host's token 361 -> 345. */
 constexpr uint32_t SC1_WARPS = 7, SC1_ROWS = SC1_WARPS * 64, SC1_SHORT = 128, SC1_SMEM = IX_HD * (uint32_t)sizeof(float4) + SC1_ROWS * IX_HD * (uint32_t)sizeof(float);
 /* rows at .. at + 32 R - 1, below r1, by one warp */
 template <int R>
@@ -313,7 +315,7 @@ __device__ __forceinline__ void sc1_walk(uint32_t buf, const float4 *qs, float *
     }
 }
 __global__ void __launch_bounds__(SC1_WARPS * 32) q4_ix_score1_k(const float *q, const float *pool, float *score, uint32_t n_blocks, uint32_t stride,
-                                                                 uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, bool early) {
+                                                                 uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, bool early, bool ahead) {
     extern __shared__ __align__(16) uint8_t sc_smem[];
     float4 *qs = reinterpret_cast<float4 *>(sc_smem);   /* [dim] = the 4 heads' values (0 for heads that do not exist) */
     const uint32_t warp = threadIdx.x >> 5;
@@ -325,9 +327,17 @@ __global__ void __launch_bounds__(SC1_WARPS * 32) q4_ix_score1_k(const float *q,
     const bool two = per > SC1_SHORT;
     const uint32_t at = r0 + warp * (two ? 64u : 32u);
     const uint32_t buf = (uint32_t)__cvta_generic_to_shared(sc_smem + IX_HD * sizeof(float4)) + warp * (64u * IX_HD * 4u);
-    if (early) q4d_pdl_wait();
-    if (two) sc1_fetch<2>(buf, pool, at, r1);
-    else sc1_fetch<1>(buf, pool, at, r1);
+    if (early && !ahead) q4d_pdl_wait();
+    const uint32_t newest = n_vis ? n_vis - 1u : 0u, old = ahead ? min(r1, newest) : r1;
+    if (two) sc1_fetch<2>(buf, pool, at, old);
+    else sc1_fetch<1>(buf, pool, at, old);
+    if (ahead) {
+        q4d_pdl_wait();
+        if (newest >= at && newest < min(r1, at + (two ? 64u : 32u))) {
+            const uint32_t r = newest - at, lane = threadIdx.x & 31u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buf + r * (IX_HD * 4u) + ((lane ^ (r & 7u)) << 4)), "l"(pool + (size_t)newest * IX_HD + lane * 4u) : "memory");
+        }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
     /* the query is staged while the rows are in flight */
     if (threadIdx.x < IX_HD) {
@@ -568,9 +578,12 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
         if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score1_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC1_SMEM), "qsa_score smem attribute"))
             return false;
         done = true;
+        const bool early = ix_pdl() && (!pp || q4i_settled(g_q4.pos_written));
         const uint32_t fill = (rows + 31u) / 32u, grid = fill < (uint32_t)g_q4.sm_count ? (fill ? fill : 1u) : (uint32_t)g_q4.sm_count;
+        const bool ahead = early && q4i_blocks_ahead(pool, (uint64_t)rows * IX_HD * 4u, ratio);
+        g_q4.n_ahead += ahead;
         return ix_start("qsa_score launch", q4_ix_score1_k, dim3(grid), SC1_WARPS * 32u, SC1_SMEM, 1u, q, pool, score, n_blocks, stride, n_head, pos0, ratio,
-                        pp, ix_pdl() && (!pp || q4i_settled(g_q4.pos_written)));
+                        pp, early, ahead);
     }
     uint32_t gx = n_tok > 1 ? (all + n_tok - 1u) / n_tok : all;
     if (gx > need) gx = need;
@@ -903,7 +916,10 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     if (NB > 1) reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
     if (tx < 256) S.h3[tx] = S.bg[tx] = S.be[tx] = 0u;
     if (tx == 0) S.n_own = S.n_near = S.n_above = S.low = S.n_tie = 0u;
-    tkc_sync<NB>();   /* the sums are zero before anyone adds to them */
+    /* the sums are zero before anyone adds to them; a cluster meets while the keys are on their way (8
+     * sessions' step, met before the wait 416 us, so 411.5: its blocks find room late) */
+    if (NB == 1) __syncthreads();
+    else asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     q4d_pdl_wait();
     /* The keys are requested before a position that has yet to be read arrives.  Only visible ones of the last row: a host's
      * need not reach to `stride` (those of a batch do by its interface, and there the last row has stride too). */
@@ -920,6 +936,7 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         if (pos_arr) pos = (uint32_t)pos_arr[t];
         n_vis = ratio ? (pos + 1u) / ratio : 0u;
     }
+    if (NB > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const uint32_t need = n_vis < k_blk ? n_vis : k_blk;
     int32_t *out = sel + (size_t)t * width;
     const uint32_t w_per = (width + NB - 1u) / NB;
@@ -1467,6 +1484,7 @@ bool pool_start(const char *what, uint32_t grid, const void *raw, float *pool, c
     if (pp) {
         t.reads(raw, 0);
         t.writes(pool, 0);
+        t.r[t.n - 1u].newest = ratio;
     } else {
         t.reads((const __half *)raw + (size_t)b0 * ratio * IX_HD, (b1 - b0) * row);
         t.writes(pool + (size_t)b0 * IX_HD, (uint64_t)(b1 - b0) * IX_HD * 4u);

@@ -62,13 +62,13 @@ struct Q4PtrList { void **p; uint32_t n; };
 /* Device memory that a launch reads and writes.  bytes == 0: to the end of p's allocation (a row whose place the device
  * knows).  The status word, which launches only or bits into, and the library's scratch are left out. */
 struct Q4Touch {
-    struct { const void *p; uint64_t bytes; bool write; } r[12];
+    struct { const void *p; uint64_t bytes; bool write; uint32_t newest; } r[12];   /* newest: of the rows at p the pooled block that the position word completes alone, of so many tokens */
     uint32_t n;
     void reads(const void *p, uint64_t bytes) { add(p, bytes, false); }
     void writes(const void *p, uint64_t bytes) { add(p, bytes, true); }
     void add(const void *p, uint64_t bytes, bool write) {
         if (!p) return;
-        r[n].p = p; r[n].bytes = bytes; r[n].write = write;
+        r[n].p = p; r[n].bytes = bytes; r[n].write = write; r[n].newest = 0;
         n++;
     }
 };
@@ -96,7 +96,7 @@ struct Q4State {
     struct { uint64_t number; Q4Touch touch; } flight[4];
     uint32_t n_flight;
     cudaGraphNode_t last_node;
-    uint32_t n_apart, last_graph_apart;   /* launches apart in this capture, in the last finished one */
+    uint32_t n_apart, last_graph_apart, n_ahead, last_graph_ahead;   /* launches apart, and with blocks read ahead, in this capture, in the last finished one */
     /* attention scratch: split-KV partial records + per-unit arrival counters */
     float *part;
     size_t part_floats;
@@ -127,6 +127,10 @@ inline bool q4i_settled(uint64_t written) { return g_q4.settled > written && g_q
  * Such a kernel lets its successor start at once, does its work, and waits for its predecessor before it ends
  * (q4d_apart_begin / _end): whoever waits for it has waited for everything before it, as ever. */
 bool q4i_apart(const Q4Touch &touch);
+/* Whether the next launch may read the pooled blocks (of `ratio` tokens each) at p before it waits for the ones before it, but for
+ * the block that the position word completes: captured likewise, and nothing else in those bytes is written by any that may not
+ * have finished when it starts. */
+bool q4i_blocks_ahead(const void *p, uint64_t bytes, uint32_t ratio);
 inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->writes->at[layer] = g_q4.launches; }
 bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside capture, fails inside */
 void q4i_give_back(void *p, bool captured);              /* cudaFree, now or with the last graph */

@@ -105,14 +105,20 @@ void q4i_in_capture(const Q4Touch *touch) {
         if (!touch->r[i].bytes) g_q4.flight[keep].touch.r[i].bytes = allocation_end(touch->r[i].p) - (uintptr_t)touch->r[i].p;
     g_q4.n_flight = keep + 1u;
 }
-bool q4i_apart(const Q4Touch &touch) {
+/* whether every launch that may still run when the next one starts is known, and `clear` of all of them */
+template <typename F>
+static bool flight_clear(F clear) {
     if (!g_q4.capturing || !g_q4.last_node || capture_tail() != g_q4.last_node) return false;
     /* a record for every launch that may still run: those numbered from `settled` on */
     uint64_t at = g_q4.settled;
     for (uint32_t i = 0; i < g_q4.n_flight; i++) {
         if (g_q4.flight[i].number < g_q4.settled) continue;
-        if (g_q4.flight[i].number != at++) return false;
-        const Q4Touch &f = g_q4.flight[i].touch;
+        if (g_q4.flight[i].number != at++ || !clear(g_q4.flight[i].touch)) return false;
+    }
+    return at == g_q4.launches + 1u && g_q4.settled > g_q4.unsettled;
+}
+bool q4i_apart(const Q4Touch &touch) {
+    return flight_clear([&](const Q4Touch &f) {
         for (uint32_t a = 0; a < touch.n; a++) {
             const uintptr_t a0 = (uintptr_t)touch.r[a].p;
             for (uint32_t b = 0; b < f.n; b++) {
@@ -121,8 +127,18 @@ bool q4i_apart(const Q4Touch &touch) {
                 if (a0 < b0 + f.r[b].bytes && b0 < a1) return false;
             }
         }
-    }
-    return at == g_q4.launches + 1u && g_q4.settled > g_q4.unsettled;
+        return true;
+    });
+}
+bool q4i_blocks_ahead(const void *p, uint64_t bytes, uint32_t ratio) {
+    return flight_clear([&](const Q4Touch &f) {
+        for (uint32_t b = 0; b < f.n; b++) {
+            const uintptr_t b0 = (uintptr_t)f.r[b].p;
+            if (!f.r[b].write || (f.r[b].p == p && f.r[b].newest == ratio)) continue;
+            if ((uintptr_t)p < b0 + f.r[b].bytes && b0 < (uintptr_t)p + bytes) return false;
+        }
+        return true;
+    });
 }
 
 /* Scratch for the split-KV records and arrival counters.  Grows only outside capture (an
@@ -365,7 +381,7 @@ extern "C" int q4_hip_graph_begin(void) {
     g_q4.unsettled = g_q4.launches;
     g_q4.n_flight = 0;
     g_q4.last_node = nullptr;
-    g_q4.n_apart = 0;
+    g_q4.n_apart = g_q4.n_ahead = 0;
     return 1;
 }
 extern "C" void *q4_hip_graph_end(void) {
@@ -375,6 +391,7 @@ extern "C" void *q4_hip_graph_end(void) {
     g_q4.n_flight = 0;
     g_q4.last_node = nullptr;
     g_q4.last_graph_apart = g_q4.n_apart;
+    g_q4.last_graph_ahead = g_q4.n_ahead;
     cudaGraph_t g = nullptr;
     if (cudaStreamEndCapture(g_q4.stream, &g) != cudaSuccess || !g) {
         (void)cudaGetLastError();
@@ -402,6 +419,7 @@ extern "C" uint32_t q4_hip_graph_nodes(void *exec) {
     return g_q4.last_graph_nodes;
 }
 extern "C" uint32_t q4_gpu_graph_apart(void) { return g_q4.last_graph_apart; }
+extern "C" uint32_t q4_gpu_graph_ahead(void) { return g_q4.last_graph_ahead; }
 extern "C" bool q4_hip_graph_launch(void *exec) {
     if (!g_q4.ok || !exec) return false;
     g_q4.unsettled = g_q4.launches;

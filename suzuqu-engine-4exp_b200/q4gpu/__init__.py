@@ -27,7 +27,7 @@ SIGNATURES = {
     "q4_hip_stream_sync": (_b, []),
     "q4_hip_copy_h2d": (_b, [_v, _v, _sz]), "q4_hip_copy_wait": (None, []), "q4_gpu_copy_stream": (_v, []),
     "q4_gpu_copy_d2h": (_b, [_v, _v, _sz]), "q4_gpu_download_stream": (_v, []),
-    "q4_gpu_graph_apart": (_u32, []), "q4_gpu_prefill_layout": (None, [_v, _v, _v]),
+    "q4_gpu_graph_apart": (_u32, []), "q4_gpu_graph_ahead": (_u32, []), "q4_gpu_prefill_layout": (None, [_v, _v, _v]),
     "q4_gpu_pipe_create": (_v, []), "q4_gpu_pipe_destroy": (None, [_v]),
     "q4_gpu_pipe_upload": (_b, [_v, _v, _v, _sz]), "q4_gpu_pipe_run": (_b, [_v, _v, _v, _v, _sz]),
     "q4_gpu_pipe_sync": (_b, [_v]),

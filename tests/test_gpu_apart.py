@@ -275,3 +275,48 @@ def test_launch_behind_a_long_attention(dependent):
         st.close()
     b.free()
     assert L.q4_gpu_last_error() == 0
+
+
+def test_scores_that_read_their_blocks_ahead():
+    """the score of a captured step requests all blocks but the newest before it waits: not where a launch that may still run
+    writes an older one, and the block that pooling completes in the same step is waited for"""
+    L = q4gpu.init()
+    assert L.q4_gpu_set_stream(None) and L.q4_hip_qsa_topk_alloc()
+    blocks = 9001
+    b = Buffers(L, {"raw0": 4 * blocks * HD * 2, "raw1": 4 * blocks * HD * 2, "arena": 2 * blocks * HD * 4, "wn": HD * 4, "q0": 4 * HD * 4, "q1": 4 * HD * 4, "score": blocks * 4,
+                    "k0": KVW * 4}, 8)
+    p = b.p
+    other = p["arena"] + blocks * HD * 4
+    pool = lambda to, ratio=4: lambda: L.q4_hip_qsa_pool_d(p["raw0"], to, p["wn"], HD, ratio, 64, 1e4, 1e-6)
+    score = lambda: L.q4_hip_qsa_score_d(p["q0"], p["arena"], p["score"], blocks, 4, HD, 4)
+    norm = lambda x, heads: lambda: L.q4_hip_qsa_k_prep_d(x, p["wn"], heads, HD, 64, 1e4, 1e-6)
+    many = lambda: L.q4_hip_qsa_pool(p["raw1"], p["arena"], p["wn"], HD, 4, 0, blocks, 64, 1e4, 1e-6)
+    last = lambda: L.q4_hip_qsa_pool(p["raw1"], p["arena"], p["wn"], HD, 4, blocks - 1, blocks, 64, 1e4, 1e-6)
+    old = lambda: L.q4_hip_copy(p["arena"], other, 64 * HD)
+    row = lambda: L.q4_hip_qsa_k_prep_d(p["arena"] + 77 * HD * 4, p["wn"], 1, HD, 64, 1e4, 1e-6)
+    for case, (calls, ahead) in enumerate([([norm(p["k0"], 2), pool(p["arena"]), score], 1),
+                         ([norm(p["k0"], 2), pool(p["arena"]), norm(p["q0"], 4), score], 1),
+                         ([pool(p["arena"]), norm(p["q0"], 4), score, pool(p["arena"]), score], 2),
+                         ([score], 0),                                                    # nothing is known of what was before
+                         ([norm(p["k0"], 2), pool(other), score], 1),                     # another layer's block, to the end of the allocation
+                         ([norm(p["k0"], 2), pool(p["arena"], 2), score], 0),             # a block of other tokens
+                         ([norm(p["k0"], 2), many, score], 0),
+                         ([norm(p["k0"], 2), last, score], 0),
+                         ([norm(p["k0"], 2), pool(p["arena"]), old, score], 0),           # a copy
+                         ([norm(p["k0"], 2), row, score], 0),
+                         ([row, norm(p["q0"], 4), score], 0),                             # the norm does not wait for the first
+                         ([row, norm(p["q0"], 4), pool(p["arena"]), score], 1),           # pooling does: it writes there too
+                         ([row, norm(p["q0"], 4), score, pool(p["arena"]), score], 1)]):
+        for pos in (4 * blocks - 1, 4 * blocks - 2, 4 * 8192 - 1, 3):
+            b.reset()
+            L.q4_hip_pos_push(pos)
+            for call in calls:
+                assert call() and L.q4_hip_stream_sync()
+            want = b.read()
+            captured(L, calls, before=b.reset)
+            assert L.q4_gpu_graph_ahead() == ahead, case
+            got = b.read()
+            for n in want:
+                assert np.array_equal(got[n], want[n]), (n, pos, case)
+    b.free()
+    assert L.q4_gpu_last_error() == 0
