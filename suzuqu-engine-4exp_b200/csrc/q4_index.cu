@@ -139,11 +139,10 @@ bool ix_start(const char *what, K kernel, dim3 grid, uint32_t threads, size_t sm
 constexpr uint32_t SC_ROW_FLOATS = IX_HD + 4, SC_WARPS = 2;
 constexpr uint32_t SC_TILE_BYTES = 32u * SC_ROW_FLOATS * sizeof(float);
 constexpr uint32_t SC_SMEM = SC_WARPS * 2u * SC_TILE_BYTES + IX_HD * sizeof(float4);
-/* SC_SHARED, SC_EACH: sessions with a pool and a position of their own.  SC_SHARED: their tiles are counted through, and every
- * block takes an equal share of the whole, which may end in one session and begin in the next (an equal number of blocks per
- * session leaves most of them idle while the longest context is scanned).  SC_EACH, while there is room for a block per two
- * tiles of every session: nothing to count (select of 2 sessions of 512 blocks, shared out 7.6 us, 5.5 so). */
-enum { SC_ONE, SC_SHARED, SC_EACH };
+/* SC_EACH: sessions with a pool and a position of their own, while there is room for a block per two tiles of every session; more
+ * rows share the blocks (q4_ix_score_batch_k), which costs some counting (select of 2 sessions of 512 blocks, shared out 7.6 us,
+ * 5.5 so). */
+enum { SC_ONE, SC_EACH };
 template <int FORM>
 __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, const float *pool, float *score,
                                                                uint32_t n_blocks, uint32_t stride, uint32_t n_head,
@@ -210,38 +209,6 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     };
-    if (FORM == SC_SHARED) {
-        q4d_pdl_wait();
-        auto rows_of = [&](uint32_t t) -> uint32_t { return min(((uint32_t)pos_arr[t] + 1u) / ratio, stride); };
-        uint32_t rows = lane < n_sess ? rows_of(lane) : 0u;   /* the first 32 sessions' are kept for the walk below */
-        uint64_t total = __reduce_add_sync(0xffffffffu, (rows + 31u) / 32u);
-        for (uint32_t t0 = 32u; t0 < n_sess; t0 += 32u) total += __reduce_add_sync(0xffffffffu, t0 + lane < n_sess ? (rows_of(t0 + lane) + 31u) / 32u : 0u);
-        const uint64_t share0 = total * blockIdx.x / gridDim.x, share1 = total * (blockIdx.x + 1u) / gridDim.x;
-        uint64_t at = 0;   /* tiles of the sessions before */
-        bool again = false;
-        for (uint32_t t0 = 0; t0 < n_sess && at < share1; t0 += 32u) {
-            if (t0) rows = t0 + lane < n_sess ? rows_of(t0 + lane) : 0u;
-            const uint32_t tiles = (rows + 31u) / 32u;
-            uint32_t incl = tiles;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= (uint32_t)o) incl += y;
-            }
-            uint32_t mine = __ballot_sync(0xffffffffu, tiles && at + incl > share0 && at + incl - tiles < share1);
-            for (; mine; mine &= mine - 1u) {
-                const int l = __ffs(mine) - 1;
-                const uint64_t begin = at + __shfl_sync(0xffffffffu, incl - tiles, l);
-                const uint32_t n = __shfl_sync(0xffffffffu, tiles, l), lim = __shfl_sync(0xffffffffu, rows, l), t = t0 + (uint32_t)l;
-                const uint32_t first = begin < share0 ? (uint32_t)(share0 - begin) : 0u, last = begin + n > share1 ? (uint32_t)(share1 - begin) : n;
-                if (again) __syncthreads();   /* the other warp is done with the query of the session before */
-                again = true;
-                scan(t, pools[t], lim, first + warp, last, SC_WARPS);
-            }
-            at += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        return;
-    }
     const uint32_t t = blockIdx.y;
     if (!early) q4d_pdl_wait();
     const uint32_t pos = FORM == SC_EACH ? (uint32_t)pos_arr[t] : (pp ? (uint32_t)*pp : pos0) + t;
@@ -353,6 +320,146 @@ __global__ void __launch_bounds__(SC1_WARPS * 32) q4_ix_score1_k(const float *q,
     }
     /* blocks the token cannot see (host-position form only): -1e30 */
     for (uint32_t b = n_vis + blockIdx.x * blockDim.x + threadIdx.x; b < n_blocks; b += gridDim.x * blockDim.x) score[b] = -1.0e30f;
+}
+/* ---- scores of many sessions, one token and one pool each.  The sessions' rows are counted through and every warp takes an equal
+ * share of the whole, which may end in one session and begin in the next.  Bound by HBM as long as shared memory keeps up: a
+ * 16-byte read costs four cycles of what it returns to a warp, so a lane walks two rows (six reads per 4 dims of 64 rows; with one
+ * row per lane, 32-row tiles in two buffers and six warps per SM, ten, and 71 MB of pools took 16.7 us of a layer's 34).  A stage is
+ * 64 rows x 32 dims, 128 bytes of each row, so that five can be in flight per warp behind the one that is read; chunk c of row r
+ * lies at c ^ (r & 7).  Score + select, us, in two buffers / here: 8 sessions up to 131 072 22.1 / 20.6, of 262 144 59.3 / 54.7,
+ * 64 up to 131 072 114.6 / 109.9, of 8000 19.3 / 17.8, 33 up to 30 000 19.8 / 19.8; 2 up to 131 072 13.5 / 14.0. */
+constexpr uint32_t SB_WARPS = 4, SB_STAGES = 6, SB_ROWS = 64, SB_CD = 32, SB_STAGE = SB_ROWS * SB_CD * 4u;
+constexpr uint32_t SB_SMEM = SB_WARPS * (SB_STAGES * SB_STAGE + IX_HD * (uint32_t)sizeof(float4));
+struct SbAt { uint32_t t, row, end, left; const float *pool; };   /* session, rows [row, end) of it, rows of later sessions */
+__global__ void __launch_bounds__(SB_WARPS * 32, 1) q4_ix_score_batch_k(const float *q, float *score, uint32_t stride, uint32_t n_head, uint32_t ratio,
+                                                                        const float *const *pools, const int32_t *pos_arr, uint32_t n_sess) {
+    extern __shared__ __align__(128) uint8_t sc_smem[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t buf = (uint32_t)__cvta_generic_to_shared(sc_smem) + warp * (SB_STAGES * SB_STAGE);
+    float4 *qs = reinterpret_cast<float4 *>(sc_smem + SB_WARPS * SB_STAGES * SB_STAGE) + warp * IX_HD;   /* [dim] = the 4 heads' values */
+    q4d_pdl_wait();
+    auto rows_of = [&](uint32_t t) -> uint32_t { return min(((uint32_t)pos_arr[t] + 1u) / ratio, stride); };
+    /* the first 32 sessions' rows and pools are kept for the search below */
+    uint32_t rows = lane < n_sess ? rows_of(lane) : 0u;
+    const float *pool = lane < n_sess ? pools[lane] : nullptr;
+    uint64_t total = __reduce_add_sync(0xffffffffu, rows);
+    for (uint32_t t0 = 32u; t0 < n_sess; t0 += 32u) total += __reduce_add_sync(0xffffffffu, t0 + lane < n_sess ? rows_of(t0 + lane) : 0u);
+    const uint32_t w = blockIdx.x * SB_WARPS + warp, n_w = gridDim.x * SB_WARPS;
+    const uint64_t share0 = total * w / n_w, share1 = total * (w + 1u) / n_w;
+    if (share0 == share1) return;
+    /* the session that the share begins in */
+    SbAt at = {0u, 0u, 0u, 0u, nullptr};
+    uint64_t before = 0;
+    for (uint32_t t0 = 0;; t0 += 32u) {
+        if (t0) {
+            rows = t0 + lane < n_sess ? rows_of(t0 + lane) : 0u;
+            pool = t0 + lane < n_sess ? pools[t0 + lane] : nullptr;
+        }
+        uint32_t incl = rows;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        const uint32_t here = __ballot_sync(0xffffffffu, before + incl > share0);
+        if (here) {
+            const int l = __ffs(here) - 1;
+            at.t = t0 + (uint32_t)l;
+            at.row = (uint32_t)(share0 - before) - __shfl_sync(0xffffffffu, incl - rows, l);
+            at.end = min(__shfl_sync(0xffffffffu, rows, l), at.row + (uint32_t)(share1 - share0));
+            at.left = (uint32_t)(share1 - share0) - (at.end - at.row);
+            at.pool = reinterpret_cast<const float *>(__shfl_sync(0xffffffffu, (unsigned long long)pool, l));
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    auto next = [&](SbAt &a) {   /* the tile after; row == end: none */
+        a.row = min(a.row + SB_ROWS, a.end);
+        while (a.row == a.end && a.left) {
+            a.t++;
+            a.row = 0;
+            a.end = min(rows_of(a.t), a.left);
+            a.left -= a.end;
+            a.pool = pools[a.t];
+        }
+    };
+    SbAt ahead = at;
+    uint32_t chunk = 0, fill = 0;
+    auto fetch = [&]() {
+        const uint32_t rows = min(SB_ROWS, ahead.end - ahead.row), r0 = lane >> 3, c = lane & 7u;
+        const float *src = ahead.pool + (size_t)(ahead.row + r0) * IX_HD + chunk * SB_CD + c * 4u;
+        const uint32_t dst = buf + fill * SB_STAGE + r0 * (SB_CD * 4u);
+#pragma unroll
+        for (uint32_t j = 0; j < SB_ROWS / 4u; j++)
+            if (4u * j + r0 < rows)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * (SB_CD * 16u) + ((c ^ ((4u * j + r0) & 7u)) << 4)), "l"(src + (size_t)j * (4u * IX_HD)) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");   /* one group per call keeps the wait count uniform */
+        if (++fill == SB_STAGES) fill = 0;
+        if (++chunk == IX_HD / SB_CD) {
+            chunk = 0;
+            next(ahead);
+        }
+    };
+#pragma unroll 1
+    for (uint32_t i = 0; i < SB_STAGES - 1u; i++) fetch();
+    uint32_t stage = 0, of = 0xffffffffu;
+    while (at.row < at.end) {
+        if (at.t != of) {   /* another query */
+            of = at.t;
+            __syncwarp();
+            const float *qt = q + (size_t)of * n_head * IX_HD;
+            for (uint32_t d = lane; d < IX_HD; d += 32u)
+                qs[d] = make_float4(qt[d], n_head > 1 ? qt[IX_HD + d] : 0.f, n_head > 2 ? qt[2 * IX_HD + d] : 0.f, n_head > 3 ? qt[3 * IX_HD + d] : 0.f);
+        }
+        float d[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; u++) d[u][0] = d[u][1] = d[u][2] = d[u][3] = 0.f;
+#pragma unroll 1
+        for (uint32_t c = 0; c < IX_HD / SB_CD; c++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(SB_STAGES - 2u) : "memory");
+            __syncwarp();   /* this stage has landed, and every lane is done with the one before, which is filled again */
+            fetch();
+            const uint32_t row = buf + stage * SB_STAGE + lane * (SB_CD * 4u), x = lane & 7u;
+            if (++stage == SB_STAGES) stage = 0;
+            auto read = [&](uint32_t i, float4 (&k)[2]) {   /* rows lane, lane + 32; stale bytes behind the end are walked and not stored */
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(k[u].x), "=f"(k[u].y), "=f"(k[u].z), "=f"(k[u].w)
+                                 : "r"(row + ((i ^ x) << 4) + u * (32u * SB_CD * 4u)));   /* no clobber: the query's reads may go ahead */
+            };
+            float4 k[3][2];
+            read(0, k[0]);
+            read(1, k[1]);
+            const float4 *qc = qs + c * SB_CD;
+#pragma unroll
+            for (uint32_t i = 0; i < SB_CD / 4u; i++) {
+                if (i + 2u < SB_CD / 4u) read(i + 2u, k[(i + 2u) % 3u]);
+                const float4 q0 = qc[4 * i], q1 = qc[4 * i + 1], q2 = qc[4 * i + 2], q3 = qc[4 * i + 3];
+                auto step = [&](const float4 qd, float kd, float (&a)[4]) {
+                    a[0] = __fmaf_rn(qd.x, kd, a[0]); a[1] = __fmaf_rn(qd.y, kd, a[1]); a[2] = __fmaf_rn(qd.z, kd, a[2]); a[3] = __fmaf_rn(qd.w, kd, a[3]);
+                };
+#pragma unroll
+                for (int u = 0; u < 2; u++) step(q0, k[i % 3u][u].x, d[u]);
+#pragma unroll
+                for (int u = 0; u < 2; u++) step(q1, k[i % 3u][u].y, d[u]);
+#pragma unroll
+                for (int u = 0; u < 2; u++) step(q2, k[i % 3u][u].z, d[u]);
+#pragma unroll
+                for (int u = 0; u < 2; u++) step(q3, k[i % 3u][u].w, d[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            float sc = __fadd_rn(0.f, fmaxf(d[u][0], 0.f));          /* s = 0; s += relu(dot_h) in head order */
+            if (n_head > 1) sc = __fadd_rn(sc, fmaxf(d[u][1], 0.f));
+            if (n_head > 2) sc = __fadd_rn(sc, fmaxf(d[u][2], 0.f));
+            if (n_head > 3) sc = __fadd_rn(sc, fmaxf(d[u][3], 0.f));
+            const uint32_t b = at.row + lane + 32u * u;
+            if (b < at.end) score[(size_t)at.t * stride + b] = sc;
+        }
+        next(at);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 /* ---- score for many tokens over one pool (a prompt's slice).  The scan above reads the pool once per token, 17 GB
  * through L2 for 512 tokens x 32 768 blocks (1.67 ms).  This form is a tiled fp32 product on the FMA pipe (the
@@ -569,8 +676,12 @@ bool score_start(dim3 grid, const float *q, const float *pool, float *score, uin
 bool score_launch(const float *q, const float *pool, float *score, uint32_t n_tok, uint32_t n_blocks, uint32_t stride,
                   uint32_t n_head, uint32_t pos0, uint32_t ratio, const int32_t *pp, const float *const *pools, const int32_t *pos_arr) {
     const uint32_t all = (uint32_t)g_q4.sm_count * 3u, need = ((pp || pools ? stride : n_blocks) + SC_WARPS * 32u - 1u) / (SC_WARPS * 32u);
-    if (pools && (uint64_t)need * n_tok > all)
-        return score_start<SC_SHARED>(dim3(all), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr);
+    if (pools && (uint64_t)need * n_tok > all) {
+        static bool done = false;
+        if (!done && !q4i_check(cudaFuncSetAttribute(q4_ix_score_batch_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SB_SMEM), "qsa_score smem attribute")) return false;
+        done = true;
+        return ix_start("qsa_score launch", q4_ix_score_batch_k, dim3((unsigned)g_q4.sm_count), SB_WARPS * 32u, SB_SMEM, 1u, q, score, stride, n_head, ratio, pools, pos_arr, n_tok);
+    }
     if (pools) return score_start<SC_EACH>(dim3(need, n_tok), q, pool, score, n_tok, n_blocks, stride, n_head, pos0, ratio, pp, pools, pos_arr);
     const uint32_t rows = pp ? stride : n_blocks;
     if (n_tok == 1 && rows <= (uint32_t)g_q4.sm_count * SC1_ROWS) {
