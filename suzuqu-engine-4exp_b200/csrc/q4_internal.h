@@ -151,20 +151,27 @@ __device__ __forceinline__ void q4d_pdl_wait() {
  * word and weights too, may have been written by the launch before last: by loads that do not look into L1. */
 __device__ __forceinline__ void q4d_apart_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void q4d_apart_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-/* host side: a launch that may start so (the kernel calls q4d_pdl_wait in every thread) */
-template <typename K, typename... A>
-bool q4i_launch_dep(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
+/* host side: a launch that may start so (the kernel calls q4d_pdl_wait in every thread), in clusters of CLUSTER blocks */
+template <uint32_t CLUSTER, typename K, typename... A>
+bool q4i_launch_dep_in(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = g_q4.stream;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = CLUSTER;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = CLUSTER > 1u ? 2 : 1;
     return q4i_check(cudaLaunchKernelEx(&cfg, kernel, args...), what);
+}
+template <typename K, typename... A>
+bool q4i_launch_dep(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {
+    return q4i_launch_dep_in<1>(what, kernel, grid, threads, smem, args...);
 }
 template <typename K, typename... A>
 bool q4i_launch_pdl(const char *what, K kernel, dim3 grid, uint32_t threads, size_t smem, A... args) {

@@ -30,6 +30,12 @@
  *     four buffers of 64 columns; both groups share every K/V tile.  NQ = 1: units are tiles of 128 positions, two
  *     buffers of 128 columns; two warps per 32 rows instead of one take the 2048-token prefill of the reference's host
  *     (24 / 2 heads of 256) from 2591 to 2340 us.  Tensor memory: 256 columns of scores, NQ x hd of O.
+ *     PAIR: behind a prefix two blocks on neighbouring SMs form one product of 256 rows (cta_group::2): each has queries,
+ *     scores, weights and outputs of its own and half of every K and V image, which the tensor cores read from both.  The first
+ *     block issues; the second tells it what has landed.  Half the images' traffic from L2, and Q . K^T at the tensor core's
+ *     pace: 128 positions of hd 256 with both images 4650 -> 4130 cycles (4096 of products), of two groups at hd 128 3370 -> 3170.
+ *     What is told across is an arrival without cluster scope (1000 cycles each with it, and slower than one block): the data
+ *     are the asynchronous proxy's or the tensor core's, ordered by the barriers of the block they lie in.
  *  3. Where the last wave of blocks leaves much of the SMs idle, the positions of its blocks, or of all, are split over
  *     several; those write (O, m, l) and q4_pf_merge_k combines them.
  *
@@ -53,7 +59,7 @@ namespace {
 constexpr uint32_t PF_ROWS = 128, PF_BN = 128;              /* rows of a query group, positions of a tile */
 constexpr uint32_t PF_CHUNK = 32768, PF_RING = 5;           /* operand image bytes, ring slots */
 constexpr uint32_t PF_Q_BYTES = 65536;                      /* NQ x 128 rows x hd fp16, in every configuration at most this */
-constexpr uint32_t PF_BAR_BYTES = 256 + 1024;               /* barriers and words; one float per softmax thread */
+constexpr uint32_t PF_BAR_BYTES = 288 + 1024;               /* barriers and words; one float per softmax thread */
 constexpr uint32_t PF_THREADS = 320;                        /* 8 softmax warps, the issuer, the producer */
 constexpr uint32_t PF_SMEM = PF_Q_BYTES + PF_RING * PF_CHUNK + PF_BAR_BYTES + 1024;
 constexpr uint32_t PF_SPIN_LIMIT = 1u << 22;
@@ -80,7 +86,7 @@ struct PrefillParams {
     uint32_t *err;
 };
 struct PrefillTail : PrefillParams {
-    uint32_t n_groups;            /* blocks' worth of query groups per kv head; work items: kv head by kv head, last tokens first */
+    uint32_t n_groups;            /* items, of a block's or a pair's query groups, per kv head; work items: kv head by kv head, last tokens first */
     uint32_t n_whole, n_late;     /* items that are one block each; later ones, n_split blocks each */
     uint32_t part_tok;            /* tokens below this may have parts */
 };
@@ -139,26 +145,48 @@ __device__ __forceinline__ uint32_t elect_one() {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
     return p;
 }
+template <bool PAIR>
 __device__ __forceinline__ void umma_f16(uint32_t el, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+            "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+            "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
 }
 /* same product with the A operand in tensor memory (lane = row, one 32-bit column = two consecutive k) */
+template <bool PAIR>
 __device__ __forceinline__ void umma_f16_ta(uint32_t el, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+            "@e tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+            "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el) : "memory");
 }
+/* of a pair: on the barrier at that place in both blocks */
+template <bool PAIR>
 __device__ __forceinline__ void umma_commit(uint32_t el, uint32_t bar) {
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(bar), "r"(el) : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+            "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t}"
+            ::"r"(bar), "r"(el), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+            "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+            ::"r"(bar), "r"(el) : "memory");
 }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -172,6 +200,13 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0u;
 }
+/* on the barrier at that place in the first block of the pair */
+__device__ __forceinline__ void mbar_arrive_first(uint32_t bar) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
+                 ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -254,7 +289,7 @@ __device__ __forceinline__ void load8(const uint8_t *row, const uint8_t *srow, u
  * attend the row would get 0 x infinity, and its bit set: tokens that do attend it get NaN. */
 constexpr float PF_HALF_END = 65520.f, PF_DOWN = 1.f / 128.f;   /* the least magnitude that rounds to an fp16 infinity */
 template <int LAY, int HD, int NP>
-__global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg, PfMark *marks,
+__global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t layer, uint32_t n, uint32_t tiles, uint32_t unit, uint8_t *kimg, uint8_t *vimg, PfMark *marks,
                                                      uint8_t *flags) {
     constexpr bool MARKS = LAY != LAY_Q8P;
     constexpr uint32_t PITCH = 34;   /* halves per dim row of the transposition tile (odd word count) */
@@ -284,6 +319,10 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
     if (blockIdx.z == 0) {
         const uint8_t *kq = C.k + base;
         uint8_t *kt = kimg + ((size_t)kh * tiles + p0 / PF_BN) * CK * PF_CHUNK;
+        /* of a pair each block holds half of every unit's rows */
+        const uint32_t in = p0 % PF_BN, second = unit ? in >> (unit - 1u) & 1u : 0u, dims64 = unit ? 8192u : 16384u;   /* unit: log2 of its positions */
+        const uint32_t row0 = unit ? (in >> unit << (unit - 1u)) + (in & ((1u << (unit - 1u)) - 1u)) : in;
+        kt += second * (PF_CHUNK / 2u);
 #pragma unroll
         for (uint32_t it = 0; it < PER; it++) {
             const uint32_t i = tid + 256u * it, p = p0 + i / (HD / 8u), c = i % (HD / 8u);
@@ -300,8 +339,8 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
         }
 #pragma unroll
         for (uint32_t it = 0; it < PER; it++) {
-            const uint32_t i = tid + 256u * it, R = p0 % PF_BN + i / (HD / 8u), c = i % (HD / 8u);
-            uint8_t *dst = kt + (c >> 4) * PF_CHUNK + ((c >> 3) & 1u) * 16384u + R * 128u + (((c & 7u) ^ (R & 7u)) << 4);
+            const uint32_t i = tid + 256u * it, R = row0 + i / (HD / 8u), c = i % (HD / 8u);
+            uint8_t *dst = kt + (c >> 4) * PF_CHUNK + ((c >> 3) & 1u) * dims64 + R * 128u + (((c & 7u) ^ (R & 7u)) << 4);
             __half2 hi[4], lo[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -317,7 +356,8 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
     const uint8_t *vq = C.v + base;
     /* a tile's images in the order of their use: hd 256 {value, rest} of its first 64 positions, then of the others; hd 128
      * value, rest, both halves in each */
-    uint8_t *vt = vimg + ((size_t)kh * tiles + p0 / PF_BN) * CV * PF_CHUNK + ((p0 / 64u) & 1u) * (HD * 128u) * (HD == 256 ? NP : 1);
+    const uint32_t half = (p0 / 64u) & 1u;
+    uint8_t *vt = vimg + ((size_t)kh * tiles + p0 / PF_BN) * CV * PF_CHUNK + (HD == 256 ? half * NP * PF_CHUNK : half * (unit ? HD * 64u : HD * 128u));
     if (MARKS && tid == 0) bad_rows = 0u;
 #pragma unroll
     for (uint32_t it = 0; it < PER; it++) {   /* lanes on consecutive rows: the 2-byte stores below do not conflict */
@@ -356,9 +396,9 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
     for (int im = 0; im < NP; im++)
 #pragma unroll
         for (uint32_t it = 0; it < PER; it++) {
-            const uint32_t i = tid + 256u * it, d = i >> 2, c = (p0 & 63u) / 8u + (i & 3u);
+            const uint32_t i = tid + 256u * it, d = i >> 2, c = (p0 & 63u) / 8u + (i & 3u), second = unit && HD == 128 ? d >> 6 : 0u;   /* hd 256: halves lie behind one another anyway */
             const uint32_t *w = reinterpret_cast<const uint32_t *>(tile[im] + d * PITCH + (i & 3u) * 8u);
-            *reinterpret_cast<uint4 *>(vt + im * PF_CHUNK + d * 128u + ((c ^ (d & 7u)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4 *>(vt + im * PF_CHUNK + second * 8192u + d * 128u + ((c ^ (d & 7u)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
 }
 
@@ -378,11 +418,11 @@ __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_a
     return false;
 }
 /* HD: head size; NQ: query groups per block; NP: images per 128 dims of K and V (2: value and remainder); MARKS: rows may
- * have been scaled or not be finite; TAIL: the grid is a list of items, the last ones in ranges, else (groups, kv heads, ranges):
+ * have been scaled or not be finite; PAIR: two blocks per item; TAIL: the grid is a list of items, the last ones in ranges, else (groups, kv heads, ranges):
  * where a block learns only when it runs whether it writes parts, one group's epilogue takes 0.6 us more (333 tokens 10.6 -> 11.2
  * us), two groups' no more.  Only the list's launches carry its numbers: with 16 bytes more of parameters the other forms were
  * compiled to 1 to 6 % slower code (24 / 2 heads of 256, fp16, 1500 tokens 62.5 -> 65.4 us). */
-template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
+template <int HD, int NQ, int NP, bool MARKS, bool TAIL, bool PAIR>
 __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditional_t<TAIL, PrefillTail, PrefillParams> P) {
     constexpr uint32_t CK = NP * HD / 128, CV = NP * HD / 128;   /* ring slots a K / V tile takes */
     static_assert(NQ == 1 || NP == 1, "two groups hold a tile's V and the next one's K at once: both images of them leave the ring no slack");
@@ -391,26 +431,29 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
     constexpr uint32_t UN = NQ == 2 ? 64 : 128, SB = 2 * NQ;   /* positions of a unit, score buffers */
     constexpr uint32_t TU = 64;                                /* of them, those of one softmax thread */
     constexpr uint32_t QG_BYTES = PF_ROWS * HD * 2;            /* one group's queries */
+    constexpr uint32_t CTAS = PAIR ? 2 : 1, SLOTS = PF_RING * CTAS, PIECE = PF_CHUNK / CTAS;   /* a pair's blocks hold half of each image */
     static_assert(NQ * QG_BYTES <= PF_Q_BYTES && O_COL + NQ * HD <= TMEM_COLS, "shared / tensor memory");
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     /* later token groups see more rows: launch them first so the tail of the grid is made of short blocks */
-    uint32_t kh = blockIdx.y, t0 = (gridDim.x - 1u - blockIdx.x) * (P.tpc * NQ), range = 0, ranges = 1;
+    const uint32_t rank = PAIR ? blockIdx.x & 1u : 0u, work = blockIdx.x / CTAS;
+    uint32_t kh = blockIdx.y, t0 = (gridDim.x / CTAS - 1u - work) * (P.tpc * NQ * CTAS), range = 0, ranges = 1;
     if constexpr (TAIL) {
-        const Q4PfItem it = q4i_pf_item(blockIdx.x, P.n_groups, P.n_whole, P.n_late, P.n_split);
+        const Q4PfItem it = q4i_pf_item(work, P.n_groups, P.n_whole, P.n_late, P.n_split);
         kh = it.kh;
-        t0 = (P.n_groups - 1u - it.group) * (P.tpc * NQ);
+        t0 = (P.n_groups - 1u - it.group) * (P.tpc * NQ * CTAS);
         range = it.range;
         ranges = it.ranges;
     }
+    const uint32_t t_last = min(t0 + P.tpc * NQ * CTAS, P.n_tok) - 1u;
+    t0 += rank * (P.tpc * NQ);   /* a pair's second block may have no tokens left: rows of zeros, none stored */
 
     /* 1024-byte aligned operand tiles (the swizzle pattern is anchored to the address) */
     const uint32_t sQ = (smem_u32(smem_dyn) + 1023u) & ~1023u, sR = sQ + PF_Q_BYTES, bars = sR + PF_RING * PF_CHUNK;
-    const uint32_t full = bars, empty = bars + 40, bar_s = bars + 80, bar_p = bars + 112, bar_o = bars + 144,
-                   s_tmem = bars + 160, s_abort = bars + 164, s_item = bars + 176, s_xch = bars + 256;
+    const uint32_t full = bars, empty = bars + 80, bar_s = bars + 160, bar_p = bars + 192, bar_o = bars + 224,
+                   s_tmem = bars + 240, s_abort = bars + 244, s_item = bars + 256, s_xch = bars + 288;
 
     const uint32_t inv_gqa = 65536u / P.gqa + 1u;   /* row / gqa = row * inv_gqa >> 16 for rows below 128, gqa up to 16 */
-    const uint32_t t_last = min(t0 + P.tpc * NQ, P.n_tok) - 1u;
     const uint32_t cta_nkv = min(P.kv_base + t_last + 1u, P.max_kv);
     const uint32_t all_tiles = (cta_nkv + PF_BN - 1u) / PF_BN;
     /* this block's range of tiles */
@@ -418,19 +461,19 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
     const uint32_t j1 = TAIL ? all_tiles * (range + 1u) / ranges : (uint32_t)((uint64_t)all_tiles * (blockIdx.z + 1u) / P.n_split);
     const uint32_t n_tiles = j1 - j0;
     /* units per group: the last tile may be needed in half only */
-    const uint32_t n_seq = NQ == 2 ? min(n_tiles * 2u, (cta_nkv - j0 * PF_BN + 63u) / 64u) : n_tiles, n_units = n_seq * NQ;
+    const uint32_t n_seq = NQ == 2 ? min(n_tiles * 2u, (cta_nkv - j0 * PF_BN + 63u) / 64u) : n_tiles;
 
     if (warp == SW) {
         if (lane == 0) {
 #pragma unroll
-            for (uint32_t s = 0; s < PF_RING; s++) {
-                mbar_init(full + 8 * s, 1);
+            for (uint32_t s = 0; s < SLOTS; s++) {
+                mbar_init(full + 8 * s, PAIR && rank == 0u ? 2 : 1);   /* the other block's half counts too */
                 mbar_init(empty + 8 * s, 1);
             }
 #pragma unroll
             for (uint32_t s = 0; s < 4; s++) {
                 mbar_init(bar_s + 8 * s, 1);
-                mbar_init(bar_p + 8 * s, SW * 32u / NQ);
+                mbar_init(bar_p + 8 * s, PAIR ? 2u * SW / NQ : SW * 32u / NQ);
             }
             mbar_init(bar_o, 1);
             mbar_init(bar_o + 8, 1);
@@ -439,8 +482,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     /* Queries and gates are older than the staging launch before this one, and that lets this grid start only after it has
      * waited for everything older: they need no wait.  The images do. */
@@ -484,13 +532,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
         q4d_pdl_wait();
     }
     tc_fence_before();
-    __syncthreads();          /* barriers initialised, queries in place, tensor memory allocated */
+    if (PAIR) {               /* barriers initialised, queries in place, tensor memory allocated */
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
     tc_fence_after();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(s_tmem));
 
-    constexpr uint32_t IDESC_QK = (1u << 4) | ((uint32_t)(UN >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
-    constexpr uint32_t IDESC_PV = (1u << 4) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
+    constexpr uint32_t IDESC_QK = (1u << 4) | ((uint32_t)(UN >> 3) << 17) | ((uint32_t)(PF_ROWS * CTAS >> 4) << 24);
+    constexpr uint32_t IDESC_PV = (1u << 4) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(PF_ROWS * CTAS >> 4) << 24);
     const unsigned long long t_start = global_ns();
     auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_test(bar, parity) || pf_wait(bar, parity, s_abort, t_start); };
     /* by a whole warp, which goes on as one; the test that succeeds at once stays in line */
@@ -508,11 +561,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
             uint32_t at = 0;
             auto load = [&](const uint8_t *src, uint32_t chunks) {
                 for (uint32_t c = 0; c < chunks && ok; c++, at++) {
-                    const uint32_t s = at % PF_RING, use = at / PF_RING;
+                    const uint32_t s = at % SLOTS, use = at / SLOTS;
                     if (use > 0) ok = wait(empty + 8 * s, (use - 1u) & 1u);
                     if (ok) {
-                        mbar_expect_tx(full + 8 * s, PF_CHUNK);
-                        bulk_load(sR + s * PF_CHUNK, src + (size_t)c * PF_CHUNK, PF_CHUNK, full + 8 * s);
+                        mbar_expect_tx(full + 8 * s, PIECE);
+                        bulk_load(sR + s * PIECE, src + (size_t)c * PF_CHUNK + rank * PIECE, PIECE, full + 8 * s);
                     } else {
                         return;
                     }
@@ -528,9 +581,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
             /* Gave up somewhere: copies still in flight must land before the block's shared memory is released
              * (bounded again; these probes ignore the abort flag; phases that completed long ago answer at once). */
             if (!ok)
-                for (uint32_t t = at > PF_RING ? at - PF_RING : 0; t < at; t++)
-                    for (uint32_t i = 0; i < 4096u && !mbar_test(full + 8 * (t % PF_RING), (t / PF_RING) & 1u); i++) {}
+                for (uint32_t t = at > SLOTS ? at - SLOTS : 0; t < at; t++)
+                    for (uint32_t i = 0; i < 4096u && !mbar_test(full + 8 * (t % SLOTS), (t / SLOTS) & 1u); i++) {}
         }
+    } else if (PAIR && warp == SW && rank != 0u) {
+        /* ================= second block of a pair: the products are issued in the first, which learns here what has landed ====== */
+        if (lane == 0)
+            for (uint32_t at = 0; at < n_tiles * (CK + CV); at++) {
+                ok = wait(full + 8 * (at % SLOTS), (at / SLOTS) & 1u);
+                if (!ok) break;
+                mbar_arrive_first(full + 8 * (at % SLOTS));
+            }
     } else if (warp == SW) {
         /* ================= tensor-core issuer: a converged warp, one elected lane ================= */
         if (n_tiles > 0) {
@@ -540,22 +601,22 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
             auto take = [&]() -> uint32_t {
                 const uint32_t s = slot;
                 ok = ok && all_wait(full + 8 * s, phase);
-                if (++slot == PF_RING) { slot = 0; phase ^= 1u; }
+                if (++slot == SLOTS) { slot = 0; phase ^= 1u; }
                 return s;
             };
             const uint64_t q_desc = umma_desc(sQ), r_desc = umma_desc(sR);   /* byte offsets / 16 are added to these */
             auto qk_chunk = [&](uint32_t s_col, uint32_t g, uint32_t c, uint32_t s, uint32_t row0) {
-                const uint64_t qd = q_desc + ((g * QG_BYTES + (c % (HD / 128)) * (2u * PF_ROWS * 128u)) >> 4), kd = r_desc + ((s * PF_CHUNK + row0 * 128u) >> 4);
+                const uint64_t qd = q_desc + ((g * QG_BYTES + (c % (HD / 128)) * (2u * PF_ROWS * 128u)) >> 4), kd = r_desc + ((s * PIECE + row0 * 128u / CTAS) >> 4);
 #pragma unroll
                 for (uint32_t kk = 0; kk < 8; kk++)
-                    umma_f16(el, tmem + s_col, qd + (((kk >> 2) * (PF_ROWS * 128u) + (kk & 3) * 32u) >> 4),
-                             kd + (((kk >> 2) * (PF_BN * 128u) + (kk & 3) * 32u) >> 4), IDESC_QK, (c | kk) > 0);
+                    umma_f16<PAIR>(el, tmem + s_col, qd + (((kk >> 2) * (PF_ROWS * 128u) + (kk & 3) * 32u) >> 4),
+                                   kd + (((kk >> 2) * (PF_BN / CTAS * 128u) + (kk & 3) * 32u) >> 4), IDESC_QK, (c | kk) > 0);
             };
             auto pv_half = [&](uint32_t s_col, uint32_t g, uint32_t s, uint32_t half_off, bool first) {
-                const uint64_t vd = r_desc + ((s * PF_CHUNK + half_off) >> 4);
+                const uint64_t vd = r_desc + ((s * PIECE + half_off / CTAS) >> 4);
 #pragma unroll
                 for (uint32_t kk = 0; kk < 4; kk++)
-                    umma_f16_ta(el, tmem + O_COL + g * 128u, tmem + s_col + kk * 8u, vd + kk * 2u, IDESC_PV, (first && kk == 0) ? 0u : 1u);
+                    umma_f16_ta<PAIR>(el, tmem + O_COL + g * 128u, tmem + s_col + kk * 8u, vd + kk * 2u, IDESC_PV, (first && kk == 0) ? 0u : 1u);
             };
             if (NQ == 2) {
                 /* per tile: its P . V for both groups and both halves, each followed by the scores that take over the buffer */
@@ -569,10 +630,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
                         if ((e >> 1) < n_seq) {
 #pragma unroll
                             for (uint32_t c = 0; c < CK; c++) qk_chunk((e & 1u) * 128u + (e >> 1) * 64u, e & 1u, c, ks[c], (e >> 1) * 64u);
-                            umma_commit(el, bar_s + 8 * e);
+                            umma_commit<PAIR>(el, bar_s + 8 * e);
                         }
 #pragma unroll
-                    for (uint32_t c = 0; c < CK; c++) umma_commit(el, empty + 8 * ks[c]);
+                    for (uint32_t c = 0; c < CK; c++) umma_commit<PAIR>(el, empty + 8 * ks[c]);
                 }
                 for (uint32_t j = 0; j < n_tiles && ok; j++) {
                     const uint32_t sv = take();
@@ -588,17 +649,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
                         tc_fence_after();
                         if (!ok) break;
                         pv_half((e & 1u) * 128u + (e >> 1) * 64u, e & 1u, sv, (e >> 1) * (HD * 128u), j == 0 && e < 2);
-                        umma_commit(el, bar_o + 8 * (e & 1u));
-                        if (e == 3) umma_commit(el, empty + 8 * sv);
+                        umma_commit<PAIR>(el, bar_o + 8 * (e & 1u));
+                        if (e == 3) umma_commit<PAIR>(el, empty + 8 * sv);
                         if (2u * (j + 1u) + (e >> 1) < n_seq) {
 #pragma unroll
                             for (uint32_t c = 0; c < CK; c++) qk_chunk((e & 1u) * 128u + (e >> 1) * 64u, e & 1u, c, ks[c], (e >> 1) * 64u);
-                            umma_commit(el, bar_s + 8 * e);
+                            umma_commit<PAIR>(el, bar_s + 8 * e);
                         }
                     }
                     if (more && ok) {
 #pragma unroll
-                        for (uint32_t c = 0; c < CK; c++) umma_commit(el, empty + 8 * ks[c]);
+                        for (uint32_t c = 0; c < CK; c++) umma_commit<PAIR>(el, empty + 8 * ks[c]);
                     }
                 }
             } else {
@@ -608,9 +669,9 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
                         tc_fence_after();
                         if (!ok) return;
                         qk_chunk((j & 1u) * 128u, 0u, c, s, 0u);
-                        umma_commit(el, empty + 8 * s);
+                        umma_commit<PAIR>(el, empty + 8 * s);
                     }
-                    umma_commit(el, bar_s + 8 * (j & 1u));
+                    umma_commit<PAIR>(el, bar_s + 8 * (j & 1u));
                 };
                 issue_qk(0);
                 if (ok && n_tiles > 1) issue_qk(1);
@@ -629,11 +690,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
                         for (int im = 0; im < NP; im++) pv_half((j & 1u) * 128u + h * 64u, 0u, sv[im], HD == 256 ? 0u : h * (HD * 128u), j == 0 && h == 0 && im == 0);
                         if (HD == 256 || h == 1) {
 #pragma unroll
-                            for (int im = 0; im < NP; im++) umma_commit(el, empty + 8 * sv[im]);
+                            for (int im = 0; im < NP; im++) umma_commit<PAIR>(el, empty + 8 * sv[im]);
                         }
                     }
                     if (ok) {
-                        umma_commit(el, bar_o);
+                        umma_commit<PAIR>(el, bar_o);
                         if (j + 2u < n_tiles) issue_qk(j + 2u);
                     }
                 }
@@ -775,7 +836,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
              * complete without this thread (that of unit n - 3 has: the scores of unit n - 1 were committed behind it). */
             if (u > 0 && u + 1u == n_seq) ok = all_wait(bar_o + 8 * g, (u - 1u) & 1u) && ok;
             tc_fence_before();
-            mbar_arrive(bar_p + 8 * b);
+            if (PAIR) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_first(bar_p + 8 * b);
+            } else {
+                mbar_arrive(bar_p + 8 * b);
+            }
             const float2 l0 = unpack2(ls[0]), l1 = unpack2(ls[1]);
             l_run += (l0.x + l0.y) + (l1.x + l1.y);
         }
@@ -877,9 +943,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
     }
     if (!ok && lane == 0) atomicOr(P.err, (uint32_t)Q4E_CUDA);
     tc_fence_before();
-    __syncthreads();
-    if (warp == SW)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    if (PAIR) {   /* neither block leaves while products read its memory or the other arrives on its barriers */
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
+    if (warp == SW) {
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
 }
 
 /* ---- the parts of split position ranges -> out: thread = 4 dims of one (token, head); TAIL: only some items have parts */
@@ -953,26 +1027,32 @@ int stage_reserve(size_t bytes) {
     return -1;
 }
 
-template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
+template <int HD, int NQ, int NP, bool MARKS, bool TAIL, bool PAIR>
 bool attend(const PrefillTail &p, dim3 grid) {
     static bool attr = false;
-    if (!attr && !q4i_check(cudaFuncSetAttribute(q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM),
-                            "prefill smem attribute"))
-        return false;
+    const auto kernel = q4_prefill_k<HD, NQ, NP, MARKS, TAIL, PAIR>;
+    if (!attr && !q4i_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM), "prefill smem attribute")) return false;
     attr = true;
-    return q4i_launch_pdl("prefill launch", q4_prefill_k<HD, NQ, NP, MARKS, TAIL>, grid, PF_THREADS, PF_SMEM, static_cast<const std::conditional_t<TAIL, PrefillTail, PrefillParams> &>(p));
+    grid.x *= PAIR ? 2u : 1u;
+    return q4i_launched(q4i_launch_dep_in<PAIR ? 2u : 1u>("prefill launch", kernel, grid, PF_THREADS, PF_SMEM, static_cast<const std::conditional_t<TAIL, PrefillTail, PrefillParams> &>(p)));
+}
+template <int HD, int NQ, int NP, bool MARKS, bool TAIL>
+bool attend(const PrefillTail &p, dim3 grid, bool pair) {
+    if constexpr (NP == 2 || HD == 256 || (NQ == 2 && !MARKS))
+        if (pair) return attend<HD, NQ, NP, MARKS, TAIL, true>(p, grid);
+    return attend<HD, NQ, NP, MARKS, TAIL, false>(p, grid);
 }
 template <int HD, int NP, bool MARKS>
-bool attend_one(const PrefillTail &p, uint32_t n_kvh) {
-    if (p.n_whole && p.n_late) return attend<HD, 1, NP, MARKS, true>(p, dim3(p.n_whole + p.n_late * p.n_split));
-    return attend<HD, 1, NP, MARKS, false>(p, dim3(p.n_groups, n_kvh, p.n_split));
+bool attend_one(const PrefillTail &p, uint32_t n_kvh, bool pair) {
+    if (p.n_whole && p.n_late) return attend<HD, 1, NP, MARKS, true>(p, dim3(p.n_whole + p.n_late * p.n_split), pair);
+    return attend<HD, 1, NP, MARKS, false>(p, dim3(p.n_groups, n_kvh, p.n_split), pair);
 }
 template <int LAY, int HD, int NP>
-bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint8_t *kimg, uint8_t *vimg, PfMark *marks, uint8_t *flags) {
-    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, NP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, kimg, vimg, marks, flags);
+bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint32_t unit, uint8_t *kimg, uint8_t *vimg, PfMark *marks, uint8_t *flags) {
+    return q4i_launch_pdl("prefill launch", q4_pf_stage_k<LAY, HD, NP>, dim3(tiles * (PF_BN / 32u), a.n_kvh, 2), 256u, 0, a.cache, a.layer, n, tiles, unit, kimg, vimg, marks, flags);
 }
 
-/* Which blocks' positions are split, and into how many ranges: the choice with the least estimated time, waves x (tiles of a
+/* Which blocks' (pairs') positions are split, and into how many ranges: the choice with the least estimated time, waves x (tiles of a
  * range + what a block takes besides) + the merge with its traffic.  In ns, one group per block, from chunks of 33 to 1500
  * tokens over 0 to 16 384: a tile 1.0 us at hd 128, 2.2 at 256 with both images; a block 4 and 6 us besides; the merge
  * 1.2 us, 0.2 per range, and 7 KB per ns.  600 tokens over 16 384 (76 blocks): 146 us in one range, 112 in three.
@@ -1034,9 +1114,17 @@ int q4i_prefill(const Q4PrefillArgs &a) {
      * waves: 1000 tokens over 4000 (126 blocks) 52 against 83 us, 2500 over 16 384 (314) 450 against 505, 3600 (450) 643
      * against 591; between 300 and 400 it depends on the depth. */
     const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
-    const uint32_t n_groups = (groups + nq - 1u) / nq, tok_per_group = tpc * nq, blocks = n_groups * a.n_kvh;
+    const uint32_t prefix = a.kv_base / PF_BN;
+    const bool pair = groups * a.n_kvh >= 48u && (np == 2u ? prefix >= 4u : hd == 256u ? prefix >= 16u : nq == 2u && a.layout == LAY_Q8P && prefix >= 112u);
+    const uint32_t ctas = pair ? 2u : 1u, unit = pair ? (nq == 2u ? 6u : 7u) : 0u;
+    /* Pairs of blocks behind a prefix: their products are the tensor core's 64 cycles per 128 x 128 x 16 where one block's wait for
+     * shared memory, and meeting costs a microsecond.  us, one block / pairs.  Both images: 512 tokens over 512 at hd 256 39.5 / 37.8,
+     * 2048 over 4000 392 / 361, at hd 128 144 / 128 (2048 over none 120 / 121).  One image at hd 256: 512 over 512 24.8 / 25.4, 2048 over
+     * 4000 227 / 212.  Two groups per block: 8192 over 5000 515 / 514, 16 384 1159 / 1130, 40 000 2463 / 2389; with marks 8192 over 8000
+     * 758 / 760; one group at hd 128 600 over 16 384 115 / 121.  And not for a few blocks in ranges (100 over 4000 39.6 / 40.2). */
+    const uint32_t n_groups = (groups + nq * ctas - 1u) / (nq * ctas), tok_per_group = tpc * nq * ctas, blocks = n_groups * a.n_kvh;
     const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes, m_bytes = (size_t)a.n_kvh * tiles * (PF_BN / 32u) * (sizeof(PfMark) + 4u);   /* marks, flags (two bytes used per mark) */
-    PfSplit sp = best_split(n_groups, a.n_kvh, sms, a.kv_base, tok_per_group, tiles, (uint64_t)a.n_tok * a.n_head, tok_per_group * gqa, hd, np, nq);
+    PfSplit sp = best_split(n_groups, a.n_kvh, sms / ctas, a.kv_base, tok_per_group, tiles, (uint64_t)a.n_tok * a.n_head, tok_per_group * gqa, hd, np, nq);
     uint32_t part_tok;
     size_t rows, part_bytes;
     int room;
@@ -1052,7 +1140,7 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     }
     if (room != 1) return room;
     const uint32_t split = sp.ranges;
-    g_layout[0] = sp.whole; g_layout[1] = blocks - sp.whole; g_layout[2] = split;
+    g_layout[0] = sp.whole * ctas; g_layout[1] = (blocks - sp.whole) * ctas; g_layout[2] = split;
 
     PrefillTail p;
     memset(&p, 0, sizeof(p));
@@ -1072,19 +1160,19 @@ int q4i_prefill(const Q4PrefillArgs &a) {
     p.err = g_q4.err_d;
 
     bool ok;
-    if (a.layout == LAY_Q8P) ok = stage<LAY_Q8P, 128, 1>(a, n, tiles, kimg, vimg, marks, flags);
-    else if (a.layout == LAY_Q8R) ok = hd == 128 ? stage<LAY_Q8R, 128, 2>(a, n, tiles, kimg, vimg, marks, flags) : stage<LAY_Q8R, 256, 2>(a, n, tiles, kimg, vimg, marks, flags);
-    else if (a.layout == LAY_F16) ok = hd == 128 ? stage<LAY_F16, 128, 1>(a, n, tiles, kimg, vimg, marks, flags) : stage<LAY_F16, 256, 1>(a, n, tiles, kimg, vimg, marks, flags);
-    else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, kimg, vimg, marks, flags) : stage<LAY_F32, 256, 1>(a, n, tiles, kimg, vimg, marks, flags);
+    if (a.layout == LAY_Q8P) ok = stage<LAY_Q8P, 128, 1>(a, n, tiles, unit, kimg, vimg, marks, flags);
+    else if (a.layout == LAY_Q8R) ok = hd == 128 ? stage<LAY_Q8R, 128, 2>(a, n, tiles, unit, kimg, vimg, marks, flags) : stage<LAY_Q8R, 256, 2>(a, n, tiles, unit, kimg, vimg, marks, flags);
+    else if (a.layout == LAY_F16) ok = hd == 128 ? stage<LAY_F16, 128, 1>(a, n, tiles, unit, kimg, vimg, marks, flags) : stage<LAY_F16, 256, 1>(a, n, tiles, unit, kimg, vimg, marks, flags);
+    else ok = hd == 128 ? stage<LAY_F32, 128, 1>(a, n, tiles, unit, kimg, vimg, marks, flags) : stage<LAY_F32, 256, 1>(a, n, tiles, unit, kimg, vimg, marks, flags);
     if (!ok) return 0;
     const bool own = a.layout == LAY_Q8P;
     if (nq == 2) {
         const dim3 grid(p.n_whole + p.n_late * split);
-        ok = own ? attend<128, 2, 1, false, true>(p, grid) : attend<128, 2, 1, true, true>(p, grid);
+        ok = own ? attend<128, 2, 1, false, true>(p, grid, pair) : attend<128, 2, 1, true, true>(p, grid, pair);
     } else if (hd == 256) {
-        ok = np == 2 ? attend_one<256, 2, true>(p, a.n_kvh) : attend_one<256, 1, true>(p, a.n_kvh);
+        ok = np == 2 ? attend_one<256, 2, true>(p, a.n_kvh, pair) : attend_one<256, 1, true>(p, a.n_kvh, pair);
     } else {
-        ok = np == 2 ? attend_one<128, 2, true>(p, a.n_kvh) : own ? attend_one<128, 1, false>(p, a.n_kvh) : attend_one<128, 1, true>(p, a.n_kvh);
+        ok = np == 2 ? attend_one<128, 2, true>(p, a.n_kvh, pair) : own ? attend_one<128, 1, false>(p, a.n_kvh, pair) : attend_one<128, 1, true>(p, a.n_kvh, pair);
     }
     if (ok && split > 1) {
         const uint64_t total4 = (uint64_t)rows * hd / 4u;

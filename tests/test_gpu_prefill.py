@@ -548,3 +548,57 @@ def test_last_wave_split_over_positions_of_a_callers_cache(kind, n_head, hd, n_t
     k, v = (rows_of(r, ctx, n_kvh, hd, kind) for r in raw)
     assert_close(host(outs[0][:n_tok]), exact_attention(q, k, v, gate, n_head, n_kvh, kv_base, scale), "%d over %d" % (n_tok, kv_base))
     assert L.q4_gpu_last_error() == 0
+
+
+@pytest.mark.parametrize("kind,n_head,n_kvh,hd,n_tok,kv_base,blocks", [
+    (2, 24, 2, 256, 241, 512, 52), (2, 24, 2, 256, 241, 511, 50),            # 25 groups of 10 tokens, the last pair's second one empty; one block each
+    (2, 24, 2, 256, 250, 1000, 52), (2, 32, 2, 256, 199, 700, 52),           # full groups; 16 query heads per kv head
+    (2, 16, 2, 128, 391, 640, 52), (2, 16, 2, 128, 384, 5000, 48), (2, 9, 3, 128, 673, 513, 54), (2, 1, 1, 128, 6100, 512, 48),
+    (1, 24, 2, 256, 241, 2048, 52), (1, 24, 2, 256, 241, 2047, 50), (0, 24, 2, 256, 250, 2100, 52), (0, 4, 1, 256, 1537, 2049, 50),
+    (-1, 16, 2, 128, 3010, 14336, 192), (-1, 16, 2, 128, 3010, 14335, 190), (-1, 32, 2, 128, 1510, 15000, 192)])   # the library's store: two groups per block
+def test_pairs_of_blocks(kind, n_head, n_kvh, hd, n_tok, kv_base, blocks):
+    """chunks behind a prefix on both sides of the line from which two blocks form one product: all tokens against 64 bits, twice the
+    same, nothing written behind the output, and the number of blocks (of a pair both count)"""
+    from gpu_util import assert_close
+    L = lib()
+    ctx = kv_base + n_tok
+    g = torch.Generator(device="cuda").manual_seed(n_tok + kind)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    scale = float(1 / np.sqrt(hd))
+    q, gate = rn(n_tok, n_head, hd), rn(n_tok, n_head, hd)
+    raw = []
+    if kind < 0:
+        q, dtype = q.bfloat16(), torch.bfloat16
+        st = q4gpu.KVStore(1, n_kvh, hd, ctx, 2)
+        st.append(0, rn(ctx, n_kvh * hd), rn(ctx, n_kvh * hd), 0, ctx)
+        for which in (0, 1):
+            raw.append(torch.empty(ctx * st.token_bytes, dtype=torch.uint8, device="cuda"))
+            st.export(0, which, 0, ctx, raw[which])
+        run = lambda out: st.prefill(0, q, out, n_head, n_tok, kv_base, scale, gate=gate)
+    else:
+        dtype = torch.float32
+        for _ in range(2):
+            x = rn(ctx, n_kvh * hd)
+            r = torch.empty(ctx * n_kvh * {2: hd // 32 * 34, 1: hd * 2, 0: hd * 4}[kind], dtype=torch.uint8, device="cuda")
+            if kind == 0:
+                r.copy_(x.view(torch.uint8).view(-1))
+            else:
+                assert (L.q4_hip_f32_to_q8 if kind == 2 else L.q4_hip_f32_to_f16)(r.data_ptr(), x.data_ptr(), x.numel())
+            raw.append(r)
+
+        def run(out):
+            assert L.q4_hip_qsa_decode_n(q.data_ptr(), raw[0].data_ptr(), raw[1].data_ptr(), gate.data_ptr(), out.data_ptr(), n_head, n_kvh, hd, n_tok, kv_base, ctx, scale, kind)
+    outs = []
+    for _ in range(2):
+        out = torch.full((n_tok + 64, n_head, hd), 7.0, dtype=dtype, device="cuda")
+        run(out)
+        whole, late, _ = layout(L)
+        assert whole + late == blocks
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and (outs[0][n_tok:] == 7.0).all()
+    k, v = (rows_of(r, ctx, n_kvh, hd, 2 if kind < 0 else kind) for r in raw)
+    ref = exact_attention(q, k, v, gate, n_head, n_kvh, kv_base, scale)
+    (check if kind < 0 else assert_close)(host(outs[0][:n_tok].float()), ref, "%d over %d" % (n_tok, kv_base))
+    assert L.q4_gpu_last_error() == 0
+    if kind < 0:
+        st.close()
