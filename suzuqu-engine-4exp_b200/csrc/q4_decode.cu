@@ -11,13 +11,13 @@
  * scalar FMA pipe cannot keep up with B200's memory system (8 FMA per int8 byte at ~23 B/clk/SM
  * is more than the 128 FMA/clk an SM has), so the two contractions run on the tensor cores with
  * warp-level MMA.  Every byte of the cache is read from global memory once.  At hd 128 and 256 every warp (or, with more
- * than 8 query heads per kv head, two warps that share it) owns a ring of 16-position tiles in shared memory, up to four
+ * than 8 query heads per kv head, two warps that share it) owns a ring of 16-position tiles in shared memory, two to four
  * deep, filled with asynchronous copies of whole rows or records; in a dense scan of the native q8_0 store at hd 128 a
  * tile is one contiguous span and one 4352-byte bulk copy (cp.async.bulk, completion on the stage's mbarrier).  That
  * layout's warps unload a stage into MMA fragments (ldmatrix for the K rows, transposing ldmatrix for the V rows),
- * refill it at once with the tile four ahead and compute from registers; the others read fragments from the stage as the
+ * refill it at once with the tile two ahead and compute from registers; the others read fragments from the stage as the
  * products need them and refill it then.  No block barrier in the main loop.  Queries are requested coalesced ahead of
- * the copies and passed to the fragments as fp16 through a stage that is not filled yet.  Head sizes 32 and 64, and
+ * the copies and passed to the fragments as fp16 through shared memory (a stage that is not filled yet, or behind the rings).  Head sizes 32 and 64, and
  * caches that are not aligned for the copies, load fragments straight into registers.
  *
  * Launches overlap (programmatic dependent launch): what the host knows to be complete -- positions, and in a dense scan
@@ -96,6 +96,7 @@ struct DecParams {
                                    * meeting at a cluster barrier */
     uint32_t hybrid;              /* host side: cluster size wanted for a grid merge */
     uint32_t direct;              /* host side: the cache is not aligned for asynchronous copies */
+    uint32_t deep;                /* host side: four blocks per SM */
     uint32_t bulk_runs;           /* whole tiles of a dense scan come in by one bulk copy each (else by cp.async) */
 };
 
@@ -857,7 +858,11 @@ __global__ void __launch_bounds__(DEC_THREADS) q4_xchg_merge_k(const Q4XchgDev *
 
 
 /* ---- the kernel ---------------------------------------------------------------------------- */
-constexpr int RING_STAGES = 4;
+constexpr size_t DEC_HALF_SM = 110000;                      /* bytes that leave room for two blocks per SM */
+/* Two tiles in flight per warp, and the one in its registers.  With four, a launch's first copies asked for 27 MB at once, and no
+ * warp had its first tile before most of them were in: us per launch, 64 sessions' lists 25.3 / 23.2 (three 24.2, one 23.0), 32 17.2 /
+ * 15.0, 777 dense rows x 12 71.7 / 69.6, 262 144 380 / 369; three and two differ by up to 2 % either way with a few lists. */
+constexpr int RING_STAGES = 2;
 /* A stage holds the 16 records of a tile as they lie in the store: row r at r * 272 = K codes | V codes | K and V
  * block scales.  Rows 272 bytes apart put the eight 16-byte row pieces of one 8x8 ldmatrix block into eight
  * different bank groups ((17 r + c) mod 8), so no swizzle is needed, and a tile whose 16 positions are
@@ -886,12 +891,12 @@ struct DecTile {
     static constexpr int V_OFF = REC ? HD : 16 * K_PITCH;
     static constexpr int BYTES = 16 * (K_PITCH + V_PITCH);
 };
-constexpr int dec_stages(int groups_bytes) {   /* as many, up to 4, as leave room for 3 blocks per SM */
-    return groups_bytes * 4 <= 73728 ? 4 : groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 73728 ? 2 : 1;
-}
-/* LIST: positions from a list (else a dense range; with DIRECT, where there is no list).  DIRECT: fragments are loaded straight
+/* Two, or what leaves room for 3 blocks per SM (with up to four 24 / 2 heads of 256 took 17.0 us over 16 384 rows of q8_0, now 14.9,
+ * 47.4 over 120 000, now 40.9; one 45.6) */
+constexpr int dec_stages(int groups_bytes, int most) { return most > 2 && groups_bytes * 3 <= 73728 ? 3 : groups_bytes * 2 <= 73728 ? 2 : 1; }
+/* LIST: positions from a list (else a dense range; with DIRECT, where there is no list), 2: and four blocks per SM.  DIRECT: fragments are loaded straight
  * into registers, from caches whose base is not aligned for the asynchronous copies (reference ABI only) and in long fp32 scans */
-template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
+template <int LAY, int HD, int NHT, bool DIRECT, int LIST>
 struct DecCfg {
     static constexpr bool STAGED = (LAY == LAY_Q8P && HD == 128);
     static constexpr bool STAGED2 = !STAGED && !DIRECT && HD >= 128;
@@ -901,16 +906,17 @@ struct DecCfg {
     static constexpr int REC = HD + 4;          /* acc[HD], m, l, 2 pad: 16-byte aligned records */
     static constexpr size_t EPI_BYTES = (size_t)NPG * HEADS * REC * sizeof(float);
     static constexpr int TILE2 = STAGED2 ? DecTile<LAY, (HD < 128 ? 128 : HD)>::BYTES : 16;
-    static constexpr int ST2 = dec_stages(NPG * TILE2);
-    static constexpr size_t RING_BYTES = STAGED ? (size_t)DEC_WARPS * RING_STAGES * RING_STAGE_BYTES + RING_BAR_BYTES
-                                       : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 : 0;
+    static constexpr int ST2 = dec_stages(NPG * TILE2, LAY == LAY_F16 && HD == 128 ? 3 : 2);
+    static constexpr size_t RING_BYTES = STAGED ? (size_t)DEC_WARPS * RING_STAGES * RING_STAGE_BYTES : STAGED2 ? (size_t)NPG * ST2 * TILE2 + DEC_WARPS * ST2 * 4 : 0;
     static constexpr size_t REC_BYTES = (size_t)HEADS * REC * sizeof(float);   /* the block's merged record */
     static constexpr size_t TAIL_BYTES = EPI_BYTES + REC_BYTES + MERGE_SCRATCH_FLOATS * sizeof(float);   /* after the loop */
-    static constexpr size_t SMEM = ((TAIL_BYTES > RING_BYTES ? TAIL_BYTES : RING_BYTES) + 15) / 16 * 16;
-    static constexpr int MIN_BLOCKS = STAGED ? (NHT == 1 ? 3 : 2) : STAGED2 ? (SMEM <= 74752 ? 3 : SMEM <= 113664 ? 2 : 1) : (HD * NHT <= 128 ? 3 : 1);
+    /* STAGED: the stages' barriers and the queries (as fp16) lie behind what the epilogue uses again */
+    static constexpr size_t BARS_AT = ((TAIL_BYTES > RING_BYTES ? TAIL_BYTES : RING_BYTES) + 15) / 16 * 16, Q_AT = BARS_AT + RING_BAR_BYTES, Q_PITCH = 2 * HD + 16;
+    static constexpr size_t SMEM = STAGED ? Q_AT + HEADS * Q_PITCH : BARS_AT;
+    static constexpr int MIN_BLOCKS = STAGED ? (LIST == 2 ? 4 : NHT == 1 ? 3 : 2) : STAGED2 ? (SMEM <= 74752 ? 3 : SMEM <= 113664 ? 2 : 1) : (HD * NHT <= 128 ? 3 : 1);
 };
 
-template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
+template <int LAY, int HD, int NHT, bool DIRECT, int LIST>
 __global__ void __launch_bounds__(DEC_THREADS, (DecCfg<LAY, HD, NHT, DIRECT, LIST>::MIN_BLOCKS))
 q4_decode_k(const DecParams P) {
     using Cfg = DecCfg<LAY, HD, NHT, DIRECT, LIST>;
@@ -1254,8 +1260,7 @@ q4_decode_k(const DecParams P) {
             moff[b] = (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8) * RING_ROW + (uint32_t)(2 * b + (lane >> 4)) * 16;
         /* one mbarrier per stage for the bulk copies, behind the rings of all warps (the epilogue never reaches
          * them); par: the phase each stage's barrier completes next */
-        const uint32_t bars = (uint32_t)__cvta_generic_to_shared(smem_raw) + DEC_WARPS * RING_STAGES * RING_STAGE_BYTES +
-                              (uint32_t)warp * RING_STAGES * 8;
+        const uint32_t bars = (uint32_t)__cvta_generic_to_shared(smem_raw) + (uint32_t)Cfg::BARS_AT + (uint32_t)warp * RING_STAGES * 8;
         uint32_t par = 0;
         bool ring_dead = false;   /* a bulk copy never arrived within the probe limit: the block reports it and stops computing */
         if (P.bulk_runs) {
@@ -1315,10 +1320,9 @@ q4_decode_k(const DecParams P) {
             cp_async_commit();   /* one group per tile, empty or not, keeps the wait count uniform */
         };
         /* ---- queries: requested coalesced, next to the list entries, and passed on as fp16 (exact for bf16 queries; scale *
-         * log2(e) multiplies the scores in fp32 later) through warp 0's last stage before that is filled */
-        constexpr int QV = HEADS * HD / 4 / DEC_THREADS, Q_PITCH = 2 * HD + 16;
-        static_assert(HEADS * Q_PITCH <= RING_STAGE_BYTES, "the queries fit a stage");
-        const uint32_t q_at = (uint32_t)__cvta_generic_to_shared(smem_raw) + (RING_STAGES - 1) * RING_STAGE_BYTES;
+         * log2(e) multiplies the scores in fp32 later) through shared memory of their own */
+        constexpr int QV = HEADS * HD / 4 / DEC_THREADS, Q_PITCH = (int)Cfg::Q_PITCH;
+        const uint32_t q_at = (uint32_t)__cvta_generic_to_shared(smem_raw) + (uint32_t)Cfg::Q_AT;
         uint4 qv[QV];
         auto request_q = [&]() {
 #pragma unroll
@@ -1336,28 +1340,32 @@ q4_decode_k(const DecParams P) {
                 }
             }
         };
-        int32_t pa, pb, pc, pd, pn0, pn1, pn2;
+        int32_t pf[RING_STAGES], pn0, pn1, pn2;
         bool hold = false;
         auto first_positions = [&]() {
-            pa = my_pos(0); pb = my_pos(1); pc = my_pos(2); pd = my_pos(3);
-            pn0 = my_pos(4); pn1 = my_pos(5); pn2 = my_pos(6);
-            if (P.new_k) {
-                const int32_t nw = (int32_t)newest;
-                hold = __any_sync(0xffffffffu, pa == nw || pb == nw || pc == nw || pd == nw);
+            bool names = false;
+#pragma unroll
+            for (int i = 0; i < RING_STAGES; i++) {
+                pf[i] = my_pos(i);
+                names = names || pf[i] == (int32_t)newest;
             }
+            pn0 = my_pos(RING_STAGES); pn1 = my_pos(RING_STAGES + 1); pn2 = my_pos(RING_STAGES + 2);
+            if (P.new_k) hold = __any_sync(0xffffffffu, names);
         };
-        auto fill = [&]() {   /* all stages but the last; rolled: the kernel's image is fetched anew by every launch */
+        auto fill = [&]() {   /* rolled: the kernel's image is fetched anew by every launch */
+            int32_t p = pf[0];
+            static_assert(RING_STAGES == 2, "positions by stage");
 #pragma unroll 1
-            for (uint32_t i = 0; i < RING_STAGES - 1; i++) {
-                issue(i, pa);
-                pa = pb; pb = pc;
+            for (uint32_t i = 0; i < RING_STAGES; i++) {
+                issue(i, p);
+                p = pf[1];
             }
         };
         if (!early) request_q();
         first_positions();
         /* ---- fused append, second half.  Over a list every split of the unit quantises and stores the unit's newest row
          * (identical bytes from every split, so no block depends on another having written), in a dense scan the split
-         * that reads it; a block's own store is ordered before its later reads by the barrier.  A warp whose first four tiles do not name the
+         * that reads it; a block's own store is ordered before its later reads by the barrier.  A warp whose first tiles do not name the
          * newest row fills its ring before that, so the append runs under the first copies. */
         if (!hold) fill();
         if (early) {
@@ -1413,9 +1421,6 @@ q4_decode_k(const DecParams P) {
                 qcorr[nt][b][1] = -1152.f * __shfl_sync(0xffffffffu, v, (2 * t + 1) * 4);
             }
         }
-
-        __syncthreads();         /* the queries have been read */
-        issue(RING_STAGES - 1, pd);
 
         for (uint32_t it = 0; it < n_my; it++) {
             cp_async_wait<RING_STAGES - 1>();    /* all but the newest RING_STAGES - 1 tiles have landed: tile `it` is in, if gathered */
@@ -2138,10 +2143,11 @@ __global__ void q4_lse_merge_k(const float *parts, uint32_t n_parts, uint32_t n_
     }
 }
 
-template <int LAY, int HD, int NHT, bool DIRECT, bool LIST>
+template <int LAY, int HD, int NHT, bool DIRECT, int LIST>
 bool launch(const DecParams &p_in, dim3 grid) {
     constexpr size_t smem_base = DecCfg<LAY, HD, NHT, DIRECT, LIST>::SMEM;
-    constexpr size_t SMEM_LIMIT = smem_base + 2u * DEC_CLUSTER_MAX * (HD + 4) * sizeof(float) + 16u;   /* ring / epilogue + the largest receive area of the push merge */
+    constexpr size_t SMEM_NEED = smem_base + 2u * DEC_CLUSTER_MAX * (HD + 4) * sizeof(float) + 16u;   /* ring / epilogue + the largest receive area of the push merge */
+    constexpr size_t SMEM_LIMIT = SMEM_NEED > DEC_HALF_SM ? SMEM_NEED : DEC_HALF_SM;
     static bool attr_done = false;
     if (!attr_done) {
         if (!q4i_check(cudaFuncSetAttribute(q4_decode_k<LAY, HD, NHT, DIRECT, LIST>,
@@ -2213,7 +2219,10 @@ bool launch(const DecParams &p_in, dim3 grid) {
         }
         if (n_blocks() > (uint64_t)occ * (uint64_t)g_q4.sm_count) p.gridmerge = 0;
     }
-    const size_t smem = smem_base + p.push_bytes;
+    size_t smem = smem_base + p.push_bytes;
+    /* A few lists' clusters are spread two blocks deep at most, by asking for half of an SM's shared memory, where all are resident
+     * at once so too (8 sessions 9.3 -> 8.6 us per launch, 10 9.8 -> 8.8; of 12, not: 10.2 -> 14.5). */
+    if (LIST && Cfg::STAGED && p.cluster && smem < DEC_HALF_SM && n_blocks() <= 2u * (uint64_t)g_q4.sm_count && resident_clusters(DEC_HALF_SM) * p.cluster >= n_blocks()) smem = DEC_HALF_SM;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;
@@ -2256,6 +2265,9 @@ bool launch_nht(const DecParams &p, dim3 grid) {
     }
     if constexpr (HD >= 128 && (LAY == LAY_Q8R || LAY == LAY_F16)) {
         if (p.direct) return p.gqa <= 8 ? launch<LAY, HD, 1, true, LIST>(p, grid) : launch<LAY, HD, 2, true, LIST>(p, grid);
+    }
+    if constexpr (LIST && LAY == LAY_Q8P && HD == 128) {
+        if (p.deep) return launch<LAY, HD, 1, false, 2>(p, grid);
     }
     return p.gqa <= 8 ? launch<LAY, HD, 1, false, LIST>(p, grid) : launch<LAY, HD, 2, false, LIST>(p, grid);
 }
@@ -2438,6 +2450,11 @@ bool q4i_decode(const Q4DecodeArgs &a) {
                    "decode: fused append needs both rows and a store at hd 128 or 256");
     p.direct = !a.many && (((uintptr_t)a.one.k | (uintptr_t)a.one.v) & (a.layout == LAY_Q8R && a.hd == 128 ? 7u : 15u)) != 0 ? 1u : 0u;
     if (!a.new_k && q4i_f32_direct(a.layout == LAY_F32 ? Q4K_F32 : -1, a.hd, a.n_head, a.n_kvh, a.n_units, rows)) p.direct = 1u;
+    /* Whole lists, a block each, in more than one wave: four blocks per SM, compiled for 128 registers, where they take a wave less
+     * than three: lists of 2051, 16 / 2 heads, 512 tokens 118 -> 108 us, 296 78.5 -> 63.3, 230 74 -> 63 (in as many waves slower: 200
+     * 51 -> 63, 400 94 -> 96). */
+    const uint32_t sms = (uint32_t)g_q4.sm_count;
+    p.deep = a.idx && a.layout == LAY_Q8P && a.hd == 128 && gqa <= 8 && S == 1u && !a.xchg && (units + 4u * sms - 1u) / (4u * sms) < (units + 3u * sms - 1u) / (3u * sms) ? 1u : 0u;
     dim3 grid(S, a.n_kvh, a.n_units);
     Q4Touch t = {};
     if (!a.many && !a.xchg && !a.scratch_part) {

@@ -661,3 +661,29 @@ def test_dense_scans_with_sixteen_heads_per_kv_head(oracle, kind, max_kv, rows):
     """two resident blocks per SM for q8_0 records (one wave of them), two warps to a tile for the others; a short store is one
     block's"""
     test_dense_at_the_position_word_in_larger_stores(oracle, kind, 32, 128, max_kv, rows)
+
+
+@pytest.mark.parametrize("n_head,n_kvh,n_tok", [(16, 2, 222), (16, 2, 223), (16, 2, 296), (16, 2, 297), (3, 1, 450), (16, 2, 450), (32, 2, 230)])
+def test_lists_of_many_tokens_on_both_sides_of_a_wave(n_head, n_kvh, n_tok):
+    """a block per token and kv head, three or four per SM (sixteen heads per kv head: two); ragged lists with padding, against the same
+    lists a few tokens at a time, which are other launches, each within the tolerance of the oracle's tests"""
+    L = lib()
+    hd, ctx, width = 128, 9000, 333
+    g = torch.Generator(device="cuda").manual_seed(n_tok)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    st = q4gpu.KVStore(1, n_kvh, hd, ctx, 2)
+    st.append(0, rn(ctx, n_kvh * hd), rn(ctx, n_kvh * hd), 0, ctx)
+    q, out = rn(n_tok, n_head, hd), torch.full((n_tok + 1, n_head, hd), 7.0, device="cuda")
+    idx = torch.randint(0, ctx, (n_tok, width), device="cuda", generator=g, dtype=torch.int32)
+    idx[torch.rand(n_tok, width, device="cuda", generator=g) < 0.1] = -1
+    idx[::7, :40] = torch.arange(40, device="cuda", dtype=torch.int32)
+    idx[3] = -1
+    ref = torch.empty(n_tok, n_head, hd, device="cuda")
+    for _ in range(2):
+        st.decode_idx_n(0, q, out, n_head, 0.0884, idx, width, n_tok, width)
+    for t in range(0, n_tok, 20):
+        m = min(20, n_tok - t)
+        st.decode_idx_n(0, q[t:], ref[t:], n_head, 0.0884, idx[t:], width, m, width)
+    assert_close(host(out[:n_tok]), host(ref), "lists of %d tokens" % n_tok)
+    assert (out[n_tok] == 7.0).all() and (out[3] == 0).all() and L.q4_gpu_last_error() == 0
+    st.close()
