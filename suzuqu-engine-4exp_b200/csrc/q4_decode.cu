@@ -89,7 +89,7 @@ struct DecParams {
     uint32_t pdl;                 /* launched with programmatic stream serialization */
     uint32_t gridmerge;           /* long scans: every split's record goes to scratch, the unit's blocks meet at a counter,
                                    * and (head, 32-dim) slices of the merge are shared out among them */
-    uint32_t mid_steps, mid_splits;   /* with gridmerge: a unit of fewer tiles uses this many blocks at most */
+    uint32_t few;                 /* > 0, with gridmerge: a unit uses no more blocks than its tiles per warp need, or this many; in clusters this many at most */
     uint32_t small_steps;         /* with gridmerge and clusters: a unit of at most this many tiles is left to its first cluster */
     uint32_t push_bytes;          /* > 0: the launch carries this much extra shared memory and merges by pushing */
     uint32_t push_async;          /* pushes complete an mbarrier of the receiving block (its last 16 bytes) instead of
@@ -973,8 +973,16 @@ q4_decode_k(const DecParams P) {
     const int32_t *list = LIST && (!DIRECT || P.idx) ? P.idx + (size_t)u * P.idx_unit_stride + (size_t)kh * P.idx_kvh_stride : nullptr;
     const uint32_t n_pos = list ? P.width : n_kv;
     const uint32_t steps = (n_pos + 15u) >> 4;
-    /* a launch sized for the store's capacity (position from the device) uses as many of its blocks as the context needs */
-    uint32_t S_act = P.gridmerge ? (steps <= 4u * DEC_WARPS ? 1u : min(steps < P.mid_steps ? P.mid_splits : S, (steps + DEC_WARPS - 1u) / DEC_WARPS)) : S;
+    /* A launch sized for the store's capacity (position from the device) uses as many of its blocks as the context needs. */
+    uint32_t S_act = P.gridmerge ? (steps <= 4u * DEC_WARPS ? 1u : min(S, (steps + DEC_WARPS - 1u) / DEC_WARPS)) : S;
+    if (P.few && S_act > 1u) {
+        if (P.cluster) {
+            S_act = min(S_act, P.few);
+        } else if (steps > S * Cfg::NPG && steps <= 5u * S * Cfg::NPG) {
+            const uint32_t tiles = (steps + S * Cfg::NPG - 1u) / (S * Cfg::NPG) * Cfg::NPG;   /* of a block */
+            S_act = max((steps + tiles - 1u) / tiles, min(S_act, P.few));
+        }
+    }
     const bool hybrid = P.gridmerge && P.cluster;
     const bool in_cluster = P.cluster && (!hybrid || steps <= P.small_steps);   /* the unit's splits are one cluster */
     if (hybrid) S_act = in_cluster ? P.cluster : (S_act + P.cluster - 1u) / P.cluster * P.cluster;
@@ -2202,7 +2210,6 @@ bool launch(const DecParams &p_in, dim3 grid) {
             p.push_async = 1u;
             grid.x = min(grid.x / p.cluster * p.cluster, fit);
             p.S = grid.x;
-            p.mid_splits = min(p.mid_splits, p.S);
             p.small_steps = (LAY == LAY_F32 ? 3u : 4u) * p.cluster * DEC_WARPS;
         } else {
             p.cluster = p.push_bytes = 0;
@@ -2415,16 +2422,14 @@ bool q4i_decode(const Q4DecodeArgs &a) {
         if (gm < 0) { const char *e = getenv("Q4_DEC_GRIDMERGE"); gm = e ? atoi(e) : 1; }
         p.gridmerge = (gm && !cluster && S > DEC_GROUP && !a.xchg) ? 1u : 0u;
     }
-    /* A step's dense scan of one session, up to 65536 rows of q8_0 or 49152 of fp16: two blocks per SM do better than three, the
-     * next launch's blocks find room and fill their rings under this one's tail (append + scan of 16384 rows in a store of 65536
-     * 11.3 -> 10.5 us in q8_0, 10.4 -> 9.5 in fp16; 65536 rows 17.5 -> 17.1, but 19.4 -> 20.2 in fp16; 80000 rows 18.3 -> 18.9 in
-     * q8_0, 120000 21.7 -> 23.5).  Not where two warps share a tile (more than 8 heads), not for several sessions (3 of 65536
-     * rows 26.3 -> 32.7), not at head sizes without a ring (64: 65536 rows 13.7 -> 15.3), not where the host gives the row count,
-     * as for partial results (65536 rows 13.9 -> 14.8, fp16 14.4 -> 16.4); fp32 tiles leave no second stage (33.2 -> 37.0). */
-    p.mid_steps = gqa > 8 || a.layout == LAY_F32 || a.n_units > 1 || a.hd < 128 || !a.pos ? 0u : a.layout == LAY_F16 ? 3073u : 4097u;
-    p.mid_splits = (uint32_t)g_q4.sm_count * 2u / units;
-    if (p.mid_splits > S) p.mid_splits = S;
-    if (p.mid_splits < 1u) p.mid_splits = 1u;
+    /* A step's dense scan of one session: where all blocks would take up to five tiles per warp, as few of them as take no more
+     * (but two per SM), for the merge is shorter then and the next launch's blocks find room.  Append + scan in a larger store, all blocks / so: fp16
+     * 16384 rows 9.4 / 8.4 us, q8_0 24000 8.3 / 8.0, 65536 12.4 / 12.0 (148 blocks per kv head at rings of four tiles 14.7), but fp16
+     * 100003 rows, eight tiles, 23.3 / 24.2.  In clusters two blocks per SM at most (20000 rows of fp16 at hd 256 14.8, 15.9 by
+     * tiles).  Not where two warps share a tile (24 / 2 heads of 256, 24000 rows of q8_0 14.9 / 15.5), for two heads' worth of
+     * registers (32 / 2 heads of 128 9.97 / 10.3), in fp32 (16384 rows 13.6 / 13.8), for several sessions, at head sizes without a ring
+     * or where the host gives the row count. */
+    p.few = !p.gridmerge || gqa > 8 || a.layout == LAY_F32 || a.n_units > 1 || a.hd < 128 || !a.pos ? 0u : (uint32_t)g_q4.sm_count * 2u / units;
     /* Where the launch is sized for a capacity and the context may be short, a grid merge's blocks come in clusters of 8, of
      * which a short context uses the first alone, merging through distributed shared memory (777 rows in a store of 32768:
      * 5.4 against 7.0 us; 512 rows in one of 262144 5.3 against 7.5).  Long scans lose 3 to 10 % by it, the next launch's blocks

@@ -687,3 +687,29 @@ def test_lists_of_many_tokens_on_both_sides_of_a_wave(n_head, n_kvh, n_tok):
     assert_close(host(out[:n_tok]), host(ref), "lists of %d tokens" % n_tok)
     assert (out[n_tok] == 7.0).all() and (out[3] == 0).all() and L.q4_gpu_last_error() == 0
     st.close()
+
+
+@pytest.mark.parametrize("kind,n_head,n_kvh,hd,max_kv,rows", [
+    (2, 16, 2, 128, 65536, (14207, 14208, 14209, 14225, 28416, 28433, 64000)), (2, 16, 4, 128, 65536, (7104, 7120, 20000, 35536)), (2, 8, 1, 128, 262144, (16385, 70000, 82000)),
+    (1, 16, 2, 128, 65536, (14209, 16384, 49153)), (1, 16, 2, 256, 40000, (14209, 30001)), (2, 16, 2, 256, 32768, (20000, 32768))])
+def test_scans_that_use_as_few_blocks_as_their_tiles_need(oracle, kind, n_head, n_kvh, hd, max_kv, rows):
+    """dense scans at the position word in larger stores, around the row counts from which a warp takes another tile, up to five
+    tiles per warp and beyond, once right after the position was pushed and twice with everything settled"""
+    L = lib()
+    kvw, top, scale = n_kvh * hd, max(rows), float(1.0 / np.sqrt(hd))
+    g = torch.Generator(device="cuda").manual_seed(hd + kind)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    st = q4gpu.KVStore(1, n_kvh, hd, max_kv, kind)
+    q, k, v = rn(n_head, hd), rn(top, kvw), rn(top, kvw)
+    st.append(0, k, v, 0, top)
+    kc, vc = oracle.kv_write(host(k), kind), oracle.kv_write(host(v), kind)
+    for r in rows:
+        outs = [torch.full((n_head, hd), float("nan"), device="cuda") for _ in range(3)]
+        L.q4_hip_pos_push(r - 1)
+        for o in outs:
+            st.decode(0, q, o, n_head, scale)
+        ref = oracle.attn(host(q).reshape(1, n_head, hd), kc, vc, None, n_head, n_kvh, hd, 1, r - 1, max_kv, scale, kind, threads=8)[0]
+        for o in outs:
+            assert_close(host(o).reshape(ref.shape), ref, "%d of %d rows" % (r, max_kv))
+    assert L.q4_gpu_last_error() == 0
+    st.close()
