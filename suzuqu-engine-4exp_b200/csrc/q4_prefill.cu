@@ -1115,11 +1115,11 @@ int q4i_prefill(const Q4PrefillArgs &a) {
      * against 591; between 300 and 400 it depends on the depth. */
     const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
     const uint32_t prefix = a.kv_base / PF_BN;
-    const bool pair = groups * a.n_kvh >= 48u && (np == 2u ? prefix >= 4u : hd == 256u ? prefix >= 16u : nq == 2u && a.layout == LAY_Q8P && prefix >= 112u);
+    const bool pair = groups * a.n_kvh >= 48u && (np == 2u ? prefix >= (hd == 256u ? 4u : 12u) : hd == 256u ? prefix >= 16u : nq == 2u && a.layout == LAY_Q8P && prefix >= 112u);
     const uint32_t ctas = pair ? 2u : 1u, unit = pair ? (nq == 2u ? 6u : 7u) : 0u;
     /* Pairs of blocks behind a prefix: their products are the tensor core's 64 cycles per 128 x 128 x 16 where one block's wait for
      * shared memory, and meeting costs a microsecond.  us, one block / pairs.  Both images: 512 tokens over 512 at hd 256 39.5 / 37.8,
-     * 2048 over 4000 392 / 361, at hd 128 144 / 128 (2048 over none 120 / 121).  One image at hd 256: 512 over 512 24.8 / 25.4, 2048 over
+     * 2048 over 4000 392 / 361, at hd 128 144 / 128, 512 over 512 21.4 / 22.4, over 1536 27.7 / 27.5 (2048 over none at hd 256 120 / 121).  One image at hd 256: 512 over 512 24.8 / 25.4, 2048 over
      * 4000 227 / 212.  Two groups per block: 8192 over 5000 515 / 514, 16 384 1159 / 1130, 40 000 2463 / 2389; with marks 8192 over 8000
      * 758 / 760; one group at hd 128 600 over 16 384 115 / 121.  And not for a few blocks in ranges (100 over 4000 39.6 / 40.2). */
     const uint32_t n_groups = (groups + nq * ctas - 1u) / (nq * ctas), tok_per_group = tpc * nq * ctas, blocks = n_groups * a.n_kvh;

@@ -553,7 +553,7 @@ def test_last_wave_split_over_positions_of_a_callers_cache(kind, n_head, hd, n_t
 @pytest.mark.parametrize("kind,n_head,n_kvh,hd,n_tok,kv_base,blocks", [
     (2, 24, 2, 256, 241, 512, 52), (2, 24, 2, 256, 241, 511, 50),            # 25 groups of 10 tokens, the last pair's second one empty; one block each
     (2, 24, 2, 256, 250, 1000, 52), (2, 32, 2, 256, 199, 700, 52),           # full groups; 16 query heads per kv head
-    (2, 16, 2, 128, 391, 640, 52), (2, 16, 2, 128, 384, 5000, 48), (2, 9, 3, 128, 673, 513, 54), (2, 1, 1, 128, 6100, 512, 48),
+    (2, 16, 2, 128, 391, 1536, 52), (2, 16, 2, 128, 391, 1535, 50), (2, 16, 2, 128, 384, 5000, 48), (2, 9, 3, 128, 673, 1537, 54), (2, 1, 1, 128, 6100, 1700, 48),
     (1, 24, 2, 256, 241, 2048, 52), (1, 24, 2, 256, 241, 2047, 50), (0, 24, 2, 256, 250, 2100, 52), (0, 4, 1, 256, 1537, 2049, 50),
     (-1, 16, 2, 128, 3010, 14336, 192), (-1, 16, 2, 128, 3010, 14335, 190), (-1, 32, 2, 128, 1510, 15000, 192)])   # the library's store: two groups per block
 def test_pairs_of_blocks(kind, n_head, n_kvh, hd, n_tok, kv_base, blocks):
