@@ -2172,9 +2172,10 @@ bool launch(const DecParams &p_in, dim3 grid) {
     auto n_blocks = [&]() -> uint64_t { return (uint64_t)grid.x * grid.y * grid.z; };
     /* how many clusters of this shape can be resident at once with `bytes` of dynamic shared memory per block */
     auto resident_clusters = [&](size_t bytes) -> uint64_t {
-        static size_t c_bytes[4];
-        static uint32_t c_cluster[4];
-        static int c_n[4], c_used = 0;
+        constexpr int KEPT = 32;   /* up to 16 cluster sizes with two or three sizes of shared memory each */
+        static size_t c_bytes[KEPT];
+        static uint32_t c_cluster[KEPT];
+        static int c_n[KEPT], c_used = 0;
         for (int i = 0; i < c_used; i++)
             if (c_bytes[i] == bytes && c_cluster[i] == p.cluster) return (uint64_t)c_n[i];
         cudaLaunchConfig_t qc;
@@ -2194,7 +2195,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
             (void)cudaGetLastError();
             n = 0;
         }
-        const int slot = c_used < 4 ? c_used++ : 3;
+        const int slot = c_used < KEPT ? c_used++ : KEPT - 1;
         c_bytes[slot] = bytes; c_cluster[slot] = p.cluster; c_n[slot] = n;
         return (uint64_t)n;
     };

@@ -713,3 +713,43 @@ def test_scans_that_use_as_few_blocks_as_their_tiles_need(oracle, kind, n_head, 
             assert_close(host(o).reshape(ref.shape), ref, "%d of %d rows" % (r, max_kv))
     assert L.q4_gpu_last_error() == 0
     st.close()
+
+
+def test_lists_of_more_sessions_than_a_wave():
+    """231 sessions with appends and lists in one launch of whole lists, four blocks per SM, against one session at a time"""
+    L = lib()
+    n, n_head, n_kvh, hd, width = 231, 16, 2, 128, 70
+    kvw, scale = n_kvh * hd, 0.0884
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    rows = [30 + (7 * i) % 90 for i in range(n)]
+    k, v, q = rn(n, kvw), rn(n, kvw), rn(n, n_head, hd)
+    data = rn(120, kvw)
+    stores = [[q4gpu.KVStore(1, n_kvh, hd, 128, 2) for _ in range(n)] for _ in range(2)]
+    idx = torch.full((n, width), -1, dtype=torch.int32, device="cuda")
+    for i, r in enumerate(rows):
+        m = min(width, r + 1)
+        idx[i, :m] = torch.randperm(r + 1, device="cuda", generator=g)[:m].sort().values.to(torch.int32)
+        idx[i, m - 1] = r                                  # the row that the launch appends
+        for st in (stores[0][i], stores[1][i]):
+            st.append(0, data, data, 0, r)
+    out, ref = torch.empty(n, n_head, hd, device="cuda"), torch.empty(n, n_head, hd, device="cuda")
+    b = q4gpu.Batch(stores[0])
+    b.set_pos(rows)
+    b.append_decode(0, k, v, q, out, n_head, scale, idx=idx, width=width, idx_sess_stride=width)
+    for i, st in enumerate(stores[1]):
+        L.q4_hip_pos_push(rows[i])
+        st.append_decode_d(0, k[i], v[i], q[i], ref[i], n_head, scale, idx=idx[i], width=width)
+    assert_close(host(out), host(ref), "231 sessions")
+    raw = [torch.empty(120 * stores[0][0].token_bytes, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    for i in (0, 100, 230):
+        for which in (0, 1):
+            for j in range(2):
+                stores[j][i].export(0, which, 0, rows[i] + 1, raw[j])
+            m = (rows[i] + 1) * stores[0][i].token_bytes
+            assert torch.equal(raw[0][:m], raw[1][:m]), (i, which)
+    assert L.q4_gpu_last_error() == 0
+    b.close() if hasattr(b, "close") else None
+    for pair in stores:
+        for st in pair:
+            st.close()
