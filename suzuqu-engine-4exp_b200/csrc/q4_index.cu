@@ -691,7 +691,8 @@ bool score_launch(const float *q, const float *pool, float *score, uint32_t n_to
         done = true;
         const bool early = ix_pdl() && (!pp || q4i_settled(g_q4.pos_written));
         const uint32_t fill = (rows + 31u) / 32u, grid = fill < (uint32_t)g_q4.sm_count ? (fill ? fill : 1u) : (uint32_t)g_q4.sm_count;
-        const bool ahead = early && q4i_blocks_ahead(pool, (uint64_t)rows * IX_HD * 4u, ratio);
+        /* a position of the host's need not be the word's: what pooling writes there may be any of the blocks */
+        const bool ahead = early && q4i_blocks_ahead(pool, (uint64_t)rows * IX_HD * 4u, pp ? ratio : 0u);
         g_q4.n_ahead += ahead;
         return ix_start("qsa_score launch", q4_ix_score1_k, dim3(grid), SC1_WARPS * 32u, SC1_SMEM, 1u, q, pool, score, n_blocks, stride, n_head, pos0, ratio,
                         pp, early, ahead);

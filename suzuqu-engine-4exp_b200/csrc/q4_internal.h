@@ -127,9 +127,9 @@ inline bool q4i_settled(uint64_t written) { return g_q4.settled > written && g_q
  * Such a kernel lets its successor start at once, does its work, and waits for its predecessor before it ends
  * (q4d_apart_begin / _end): whoever waits for it has waited for everything before it, as ever. */
 bool q4i_apart(const Q4Touch &touch);
-/* Whether the next launch may read the pooled blocks (of `ratio` tokens each) at p before it waits for the ones before it, but for
- * the block that the position word completes: captured likewise, and nothing else in those bytes is written by any that may not
- * have finished when it starts. */
+/* Whether the next launch may read the pooled blocks at p before it waits for the ones before it, but for the block of `ratio`
+ * tokens that the position word completes (0: that one too, for a launch that has its position from elsewhere): captured likewise,
+ * and nothing else in those bytes is written by any that may not have finished when it starts. */
 bool q4i_blocks_ahead(const void *p, uint64_t bytes, uint32_t ratio);
 inline void q4i_kv_written(q4_gpu_kv *kv, uint32_t layer) { kv->writes->at[layer] = g_q4.launches; }
 bool q4i_scratch(size_t part_floats, size_t n_counters); /* grows outside capture, fails inside */

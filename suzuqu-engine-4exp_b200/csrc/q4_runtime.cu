@@ -134,7 +134,7 @@ bool q4i_blocks_ahead(const void *p, uint64_t bytes, uint32_t ratio) {
     return flight_clear([&](const Q4Touch &f) {
         for (uint32_t b = 0; b < f.n; b++) {
             const uintptr_t b0 = (uintptr_t)f.r[b].p;
-            if (!f.r[b].write || (f.r[b].p == p && f.r[b].newest == ratio)) continue;
+            if (!f.r[b].write || (ratio && f.r[b].p == p && f.r[b].newest == ratio)) continue;
             if ((uintptr_t)p < b0 + f.r[b].bytes && b0 < (uintptr_t)p + bytes) return false;
         }
         return true;

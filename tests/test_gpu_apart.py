@@ -289,6 +289,7 @@ def test_scores_that_read_their_blocks_ahead():
     other = p["arena"] + blocks * HD * 4
     pool = lambda to, ratio=4: lambda: L.q4_hip_qsa_pool_d(p["raw0"], to, p["wn"], HD, ratio, 64, 1e4, 1e-6)
     score = lambda: L.q4_hip_qsa_score_d(p["q0"], p["arena"], p["score"], blocks, 4, HD, 4)
+    at_host = lambda: L.q4_hip_qsa_score(p["q0"], p["arena"], p["score"], 1, blocks, blocks, 4, HD, 4 * blocks - 1, 4)
     norm = lambda x, heads: lambda: L.q4_hip_qsa_k_prep_d(x, p["wn"], heads, HD, 64, 1e4, 1e-6)
     many = lambda: L.q4_hip_qsa_pool(p["raw1"], p["arena"], p["wn"], HD, 4, 0, blocks, 64, 1e4, 1e-6)
     last = lambda: L.q4_hip_qsa_pool(p["raw1"], p["arena"], p["wn"], HD, 4, blocks - 1, blocks, 64, 1e4, 1e-6)
@@ -306,7 +307,9 @@ def test_scores_that_read_their_blocks_ahead():
                          ([norm(p["k0"], 2), row, score], 0),
                          ([row, norm(p["q0"], 4), score], 0),                             # the norm does not wait for the first
                          ([row, norm(p["q0"], 4), pool(p["arena"]), score], 1),           # pooling does: it writes there too
-                         ([row, norm(p["q0"], 4), score, pool(p["arena"]), score], 1)]):
+                         ([row, norm(p["q0"], 4), score, pool(p["arena"]), score], 1),
+                         ([norm(p["k0"], 2), pool(p["arena"]), at_host], 0),              # the word's block is not the host position's newest
+                         ([norm(p["k0"], 2), pool(other), at_host], 1)]):
         for pos in (4 * blocks - 1, 4 * blocks - 2, 4 * 8192 - 1, 3):
             b.reset()
             L.q4_hip_pos_push(pos)
