@@ -24,6 +24,8 @@
 #include <math_constants.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "q4_internal.h"
 
 namespace {
@@ -885,11 +887,19 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topk1_k(const float *scor
  *            threshold's bin against one another.  Two cluster meetings after the launch wait (one block: none).
  *   emit     every chosen key finds its place in the list from a bitmap of the block's keys.
  * With the first digit counted over all keys, the threshold bin's keys collected by ballots, and two more passes of ballots
- * over all keys for the list, a selection took 6.9 us of one block (8192 normal keys, a chain of such launches) and 9.5 of eight
- * (65 536); now 5.4 and 6.9.  Rows of ties (all zeros 8.1 and 10.9 us, now 8.1 and 10.5) are counted digit by digit as before. */
+ * over all keys for the list, a selection took 6.7 us of one block (8192 normal keys, a chain of such launches) and 9.4 of eight
+ * (65 536); now 5.3 and 6.7.
+ *   wide     where the pivot's digit is many keys': those above it are collected, and the blocks tell one another in the same
+ *            meeting how many are at it, the least and the largest of them and their next digits.  So rows of ties need no more
+ *            meetings (all zeros 8.1 and 10.8 us with every digit counted, now 5.3 and 6.9; a row whose 560 keys above zero are
+ *            enough 7.95 / 7.3; with the pivot and then every digit 15.9).  Keys that differ behind their first 12 bits are
+ *            collected by their first 24 (1000 +- 0.5: 6.8 / 7.6, 10.8 / 10.4), and only where 1500 share 24 are the last 8
+ *            counted (7.3 / 8.7, 11.3 / 11.4).
+ * What a row of the usual kind does not need stands behind the end of its list: 0.1 to 0.2 us of 6 are instruction fetches. */
 constexpr uint32_t TKC_KPT = 8, TKC_KEYS = IX_TK_THREADS * TKC_KPT, TKC_MAX_ROW = 8 * TKC_KEYS;
 constexpr uint32_t TK_BINS = 4096, TK_B1 = 20, TK_B2 = 8;   /* digits: bits 31..20, 19..8, 7..0 */
 constexpr uint32_t TK_B2F = 12;   /* bits of a bin of collected keys */
+constexpr uint32_t TKC_ROUNDS = 6;                         /* of telling, at most: twice by the pivot and by the threshold's digit, once by its next one and behind its last */
 constexpr uint32_t TKC_NEAR = 32;                          /* keys of the threshold's bin that are compared with one another */
 __device__ __forceinline__ uint32_t tkc_rank() {
     uint32_t r;
@@ -988,13 +998,14 @@ struct TkcShared {
     static constexpr uint32_t CAP = NB > 1 ? IX_TK_THREADS : 2u * IX_TK_THREADS;   /* collected keys of a block, at most */
     __align__(16) uint32_t ha[TK_BINS];   /* this block's counts of the first digit; cluster: the collected keys' */
     __align__(16) uint32_t hb[NB > 1 ? TK_BINS : 4];   /* the cluster's counts of the first digit */
-    __align__(16) uint32_t h2[TK_BINS];   /* one block: the collected keys' counts; cluster: its counts of the second digit (rows of ties) */
-    __align__(16) uint32_t h3[256];       /* its counts of the third */
+    __align__(16) uint32_t h2[TK_BINS];   /* one block: the collected keys' counts; cluster: its counts of the pivot's next digit */
+    __align__(16) uint32_t h3[256];       /* counts of the last digit */
     uint32_t bg[TKC_KEYS / 32], be[TKC_KEYS / 32], before[TKC_KEYS / 32];   /* this block's keys above / at the threshold, a bit each; those of earlier words */
     uint32_t tot[4][32];
     uint32_t cand[NB][CAP], idx[CAP];     /* the keys that each block has collected; this block's indices */
-    uint32_t ccnt[NB], gcnt[NB];          /* their counts; keys above the pivot's digit or the threshold (rows of ties) */
-    uint32_t n_own, n_near, n_above, low, n_tie;   /* low, n_tie: keys above (low half-word) and at the threshold of earlier blocks / of this one */
+    struct { uint32_t n[NB], lo[NB], hi[NB], next[NB]; } told[2];   /* of every block in this round: keys that it has to collect, those at the pivot << 16, the least and largest of them, the least above them */
+    struct { uint32_t n, lo, hi, next; } own[TKC_ROUNDS];   /* this block's, as they are counted */
+    uint32_t n_near, low;                 /* low: keys above (low half-word) and at the threshold, of earlier blocks */
     uint32_t near[TKC_NEAR], thr, n_gt;
     TkPick st[3];
 };
@@ -1027,7 +1038,11 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     reinterpret_cast<uint4 *>(S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
     if (NB > 1) reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
     if (tx < 256) S.h3[tx] = S.bg[tx] = S.be[tx] = 0u;
-    if (tx == 0) S.n_own = S.n_near = S.n_above = S.low = S.n_tie = 0u;
+    if (tx < TKC_ROUNDS) {
+        S.own[tx].n = S.own[tx].hi = 0u;
+        S.own[tx].lo = S.own[tx].next = 0xffffffffu;
+    }
+    if (tx == 0) S.n_near = S.low = 0u;
     /* the sums are zero before anyone adds to them; a cluster meets while the keys are on their way (8
      * sessions' step, met before the wait 416 us, so 411.5: its blocks find room late) */
     if (NB == 1) __syncthreads();
@@ -1088,35 +1103,91 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
     };
     if (NB > 1) spread(S.hb, TK_BINS);
     const TkPick p1 = tk_pick<IX_TK_THREADS>(NB > 1 ? S.hb : S.ha, need, S.tot[0], &S.st[0]);
-    const uint32_t digit = p1.digit, edge = digit << TK_B1;
-    /* Where so many threads' maxima reach the pivot the keys are ties, and more than there is room for: of 8 keys per thread an
-     * eighth (a quarter, one block) are some among 11 (15) threads of 16.  (And a pivot of 0 could not be told from no key.) */
-    bool fast = digit != 0u && (n_vis <= S.CAP || (p1.above + p1.cnt) * 16u < (n_vis / TKC_KEYS * IX_TK_THREADS + min(n_vis % TKC_KEYS, IX_TK_THREADS)) * (NB > 1 ? 11u : 15u));
-    if (fast) {
-        /* ---- collect, in any order: one add per warp */
+    /* The keys that are above the threshold or at it are found among those that reach a pivot, the digits `at` << shift.  Where a
+     * block has no room for them, or so many threads' maxima reach the pivot that it will have none (of 8 keys per thread an eighth,
+     * of one block a quarter, are some among 11, 15, threads of 16), many keys share its digits: then only those above it are
+     * collected, and the blocks tell one another what lies at it (wide).  Those above may be enough; or the keys at it are equal, as
+     * in rows of ties, and that is the threshold; or its next digit is counted. */
+    uint32_t at = p1.digit, shift = TK_B1, n_round = 0, n_own, above, edge;   /* above: keys that have been collected */
+    uint32_t thr = 0, n_gt = 0, low = 0;   /* the need-th largest key, keys above it: n_gt < need <= n_gt + ties; of earlier blocks, and their ties << 16 */
+    bool clean = NB > 1;   /* the sums of the pivot's next digit are zero */
+    /* Collects in any order, one add per warp.  Whether every block had room for its keys and they are enough: like all that
+     * follows, the same in all blocks. */
+    auto collect = [&](auto is_wide) -> bool {
+        constexpr bool wide = decltype(is_wide)::value;
+        edge = (wide ? at + 1u : at) << shift;
+        if (wide) {
+            if (!clean) {
+                reinterpret_cast<uint4 *>(NB > 1 ? S.h2 : S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
+                tkc_sync<NB>();
+            }
+            clean = false;
+        }
         uint32_t n = 0;
+        if (!wide) {
 #pragma unroll
-        for (uint32_t i = 0; i < TKC_KPT; i++) n += key[i] >= edge;
-        uint32_t at = n;
+            for (uint32_t i = 0; i < TKC_KPT; i++) n += key[i] >= edge;
+        } else {
+            uint32_t lo = 0xffffffffu, hi = 0u, next = 0xffffffffu;
+#pragma unroll
+            for (uint32_t i = 0; i < TKC_KPT; i++) {
+                const uint32_t d = key[i] >> TK_B1;
+                if (d > at) {
+                    n++;
+                    next = min(next, key[i]);
+                }
+                if (live(i) && d == at) {
+                    n += 1u << 16;
+                    lo = min(lo, key[i]);
+                    hi = max(hi, key[i]);
+                }
+            }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            next = __reduce_min_sync(0xffffffffu, next);
+            if (lane == 0) {
+                atomicMin(&S.own[n_round].lo, lo);
+                atomicMax(&S.own[n_round].hi, hi);
+                atomicMin(&S.own[n_round].next, next);
+            }
+        }
+        uint32_t slot = n;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= (uint32_t)o) at += y;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, slot, o);
+            if (lane >= (uint32_t)o) slot += y;
         }
-        uint32_t slot = 0;
-        if (lane == 31 && at) slot = atomicAdd(&S.n_own, at);
-        at += __shfl_sync(0xffffffffu, slot, 31) - n;
+        uint32_t first = 0;
+        if (lane == 31 && slot) first = atomicAdd(&S.own[n_round].n, slot);
+        slot += __shfl_sync(0xffffffffu, first, 31) - n;
+        if (wide) slot &= 0xffffu;
+        static_assert(TKC_KEYS < 65536, "two counts share a word");
+        if (!wide || (n & 0xffffu)) {
 #pragma unroll
-        for (uint32_t i = 0; i < TKC_KPT; i++)
-            if (key[i] >= edge) {
-                if (at < S.CAP) {
-                    S.cand[rank][at] = key[i];
-                    S.idx[at] = IX_TK_THREADS * i + tx;
+            for (uint32_t i = 0; i < TKC_KPT; i++)
+                if (key[i] >= edge) {
+                    if (slot < S.CAP) {
+                        S.cand[rank][slot] = key[i];
+                        S.idx[slot] = IX_TK_THREADS * i + tx;
+                    }
+                    slot++;
                 }
-                at++;
-            }
+        }
         __syncthreads();
-        const uint32_t n_own = S.n_own;
+        const uint32_t mine = S.own[n_round].n;
+        auto &told = S.told[n_round & 1u];
+        n_own = wide ? mine & 0xffffu : mine;
+        if (wide) {   /* the keys at the pivot by their next digit: one bin's where they are equal */
+            const uint32_t lo = S.own[n_round].lo;
+            if (lo < S.own[n_round].hi) {
+#pragma unroll
+                for (uint32_t i = 0; i < TKC_KPT; i++)
+                    if (live(i) && key[i] >> TK_B1 == at) atomicAdd(&S.ha[(key[i] >> TK_B2) & (TK_BINS - 1u)], 1u);
+            } else if (tx == 0 && mine >> 16) {
+                S.ha[(lo >> TK_B2) & (TK_BINS - 1u)] = mine >> 16;
+            }
+            __syncthreads();
+        }
         if (NB > 1) {
             if (tx < n_own && n_own <= S.CAP) {
                 const uint32_t k = S.cand[rank][tx];
@@ -1124,183 +1195,245 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
                 for (uint32_t r = 0; r < NB; r++)
                     if (r != rank) tkc_st(tkc_remote(&S.cand[rank][tx], r), k);
             }
-            if (tx < NB) tkc_st(tkc_remote(&S.ccnt[rank], tx), n_own);
-            tkc_sync<NB>();   /* the last access to another block's shared memory, but for rows of ties */
-            for (uint32_t r = 0; r < NB; r++) fast = fast && S.ccnt[r] <= S.CAP;   /* same decision in all blocks */
-        } else {
-            fast = n_own <= S.CAP;
+            if (tx < NB) {
+                tkc_st(tkc_remote(&told.n[rank], tx), mine);
+                if (wide) {
+                    tkc_st(tkc_remote(&told.lo[rank], tx), S.own[n_round].lo);
+                    tkc_st(tkc_remote(&told.hi[rank], tx), S.own[n_round].hi);
+                    tkc_st(tkc_remote(&told.next[rank], tx), S.own[n_round].next);
+                }
+            }
+            /* the last access to another block's shared memory, unless there is another round */
+            if (wide) spread(S.h2, TK_BINS);
+            else tkc_sync<NB>();
         }
-    }
-    uint32_t thr = 0, n_gt = 0, low = 0;   /* the need-th largest key, keys above it: n_gt < need <= n_gt + ties; of earlier blocks, and their ties << 16 */
-    if (fast) {
-        /* ---- finish: all collected keys, a warp's lanes at one block's; every block's begin at other warps, for they are a
-         * hundred or two each */
-        constexpr uint32_t CPT = NB > 1 ? NB : 2u;
+        n_round++;
+        if (NB == 1) {
+            above = n_own;
+            return n_own <= S.CAP && above >= need;
+        }
+        bool fits = true;
+        above = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < NB; r++) {
+            const uint32_t c = wide ? told.n[r] & 0xffffu : told.n[r];
+            fits = fits && c <= S.CAP;
+            if (wide) above += c;
+        }
+        return fits && (!wide || above >= need);   /* a pivot is chosen so that enough keys reach it */
+    };
+    /* The threshold and this block's share of the list, from all collected keys, a warp's lanes at one block's; every block's begin
+     * at other warps, for they are a hundred or two each.  Not where it lies beyond the bins, four times `edge` or more. */
+    constexpr uint32_t CPT = NB > 1 ? NB : 2u;
+    auto place = [&](uint32_t j) { return NB > 1 ? (tx - 128u * j) % IX_TK_THREADS : tx + j * IX_TK_THREADS; };
+    auto finish = [&]() -> bool {
+        const uint32_t *n = S.told[(n_round - 1u) & 1u].n;
         uint32_t ck[CPT];   /* 0: none */
-        auto place = [&](uint32_t j) { return NB > 1 ? (tx - 128u * j) % IX_TK_THREADS : tx + j * IX_TK_THREADS; };
 #pragma unroll
         for (uint32_t j = 0; j < CPT; j++) {
             const uint32_t c = place(j);
-            ck[j] = c < (NB > 1 ? S.ccnt[j % NB] : S.n_own) ? S.cand[j % NB][c] : 0u;
+            ck[j] = c < (NB > 1 ? n[j % NB] & 0xffffu : n_own) ? S.cand[j % NB][c] : 0u;
             if (ck[j]) atomicAdd(&hist[min((ck[j] - edge) >> TK_B2F, TK_BINS - 1u)], 1u);
         }
         __syncthreads();
         const TkPick p2 = tk_pick<IX_TK_THREADS>(hist, need, S.tot[1], &S.st[1]);
-        fast = p2.digit < TK_BINS - 1u;   /* else what reaches beyond the bins, four times the pivot */
-        if (!fast) n_gt = 0xffffffffu;
-        if (fast) {
-            const uint32_t left = need - p2.above;
-            if (p2.cnt <= TKC_NEAR) {   /* mostly one to three */
-#pragma unroll
-                for (uint32_t j = 0; j < CPT; j++)
-                    if (ck[j] && (ck[j] - edge) >> TK_B2F == p2.digit) S.near[atomicAdd(&S.n_near, 1u)] = ck[j];
-                __syncthreads();
-                if (tx < p2.cnt) {
-                    const uint32_t k = S.near[tx];
-                    uint32_t more = 0, same = 0;
-                    for (uint32_t j = 0; j < p2.cnt; j++) {
-                        more += S.near[j] > k;
-                        same += S.near[j] == k;
-                    }
-                    if (more < left && left <= more + same) {
-                        S.thr = k;
-                        S.n_gt = p2.above + more;
-                    }
-                }
-            } else {   /* many keys share 24 bits */
-                uint32_t *h = NB > 1 ? S.hb : S.ha;
-                reinterpret_cast<uint4 *>(h)[tx] = make_uint4(0u, 0u, 0u, 0u);
-                __syncthreads();
-#pragma unroll
-                for (uint32_t j = 0; j < CPT; j++)
-                    if (ck[j] && (ck[j] - edge) >> TK_B2F == p2.digit) atomicAdd(&h[(ck[j] - edge) & (TK_BINS - 1u)], 1u);
-                __syncthreads();
-                const TkPick p3 = tk_pick<IX_TK_THREADS>(h, left, S.tot[2], &S.st[2]);
-                if (tx == 0) {
-                    S.thr = edge + (p2.digit << TK_B2F) + p3.digit;
-                    S.n_gt = p2.above + p3.above;
-                }
-            }
-            __syncthreads();
-            thr = S.thr;
-            n_gt = S.n_gt;
+        if (p2.digit == TK_BINS - 1u) return false;
+        const uint32_t left = need - p2.above;
+        if (p2.cnt <= TKC_NEAR) {   /* mostly one to three */
 #pragma unroll
             for (uint32_t j = 0; j < CPT; j++)
-                if (ck[j] >= thr) {
-                    if (NB > 1 && j != rank) {
-                        if (j < rank) atomicAdd(&S.low, ck[j] > thr ? 1u : 1u << 16);
-                    } else {
-                        const uint32_t i = S.idx[place(j)];
-                        atomicOr(ck[j] > thr ? &S.bg[i >> 5] : &S.be[i >> 5], 1u << (i & 31u));
-                    }
+                if (ck[j] && (ck[j] - edge) >> TK_B2F == p2.digit) S.near[atomicAdd(&S.n_near, 1u)] = ck[j];
+            __syncthreads();
+            if (tx < p2.cnt) {
+                const uint32_t k = S.near[tx];
+                uint32_t more = 0, same = 0;
+                for (uint32_t j = 0; j < p2.cnt; j++) {
+                    more += S.near[j] > k;
+                    same += S.near[j] == k;
                 }
-            __syncthreads();
-            low = S.low;
-        }
-    }
-    if (!fast) {
-        /* ---- Rows of ties: thousands of keys reach the pivot.  Where fewer than `need` are above its digit, that is the
-         * threshold's: the second digit is counted while the blocks tell one another how many those are.  Else the first digit
-         * is counted over all keys, after a meeting to clear the sums.  Then the third. */
-        auto sum = [&](uint32_t v, uint32_t *to) -> uint32_t {   /* over the block */
-            v = __reduce_add_sync(0xffffffffu, v);
-            if (lane == 0 && v) atomicAdd(to, v);
-            __syncthreads();
-            return *to;
-        };
-        const bool counted = NB == 1 || n_gt == 0xffffffffu;   /* the counts are not zero */
-        uint32_t n = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < TKC_KPT; i++) n += (key[i] >> TK_B1) > digit;
-        uint32_t above = sum(n, &S.n_above), pre = digit, d = 1;
-        if (NB > 1 && tx < NB) tkc_st(tkc_remote(&S.gcnt[rank], tx), above);
-        bool first = true;
-#pragma unroll 1
-        while (d < 3) {
-            const uint32_t sh = d == 0 ? TK_B1 : d == 1 ? TK_B2 : 0u, bits = d < 2 ? 12u : 8u;
-            if (NB == 1 || (first && counted)) {   /* in a cluster they are left at zero */
-                __syncthreads();
-                reinterpret_cast<uint4 *>(S.ha)[tx] = make_uint4(0u, 0u, 0u, 0u);
-                __syncthreads();
-            }
-            if (NB > 1 && d == 0) {
-                reinterpret_cast<uint4 *>(S.hb)[tx] = make_uint4(0u, 0u, 0u, 0u);
-                reinterpret_cast<uint4 *>(S.h2)[tx] = make_uint4(0u, 0u, 0u, 0u);
-                tkc_sync<NB>();
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < TKC_KPT; i++)
-                if (live(i) && (d == 0 || (key[i] >> (sh + bits)) == pre)) atomicAdd(&S.ha[(key[i] >> sh) & ((1u << bits) - 1u)], 1u);
-            __syncthreads();
-            uint32_t *h = NB == 1 ? S.ha : d == 0 ? S.hb : d == 1 ? S.h2 : S.h3;
-            if (NB > 1) spread(h, 1u << bits);
-            if (first) {
-                first = false;
-                if (NB > 1) {
-                    above = 0;
-                    for (uint32_t r = 0; r < NB; r++) above += S.gcnt[r];
-                }
-                if (above >= need) {
-                    d = 0;
-                    above = 0;
-                    continue;
+                if (more < left && left <= more + same) {
+                    S.thr = k;
+                    S.n_gt = p2.above + more;
                 }
             }
-            const TkPick p = d == 2 ? tk_pick256(h, need - above) : tk_pick<IX_TK_THREADS>(h, need - above, S.tot[2], &S.st[2]);
-            pre = d == 0 ? p.digit : (pre << bits) | p.digit;
-            above += p.above;
-            d++;
-        }
-        thr = pre;
-        n_gt = above;
-        n = 0;
+        } else {   /* many keys share 24 bits */
+            uint32_t *h = NB > 1 ? S.hb : S.ha;
+            reinterpret_cast<uint4 *>(h)[tx] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
 #pragma unroll
-        for (uint32_t i = 0; i < TKC_KPT; i++) {
-            const bool gt = live(i) && key[i] > thr, eq = live(i) && key[i] == thr;
-            const uint32_t mg = __ballot_sync(0xffffffffu, gt), me = __ballot_sync(0xffffffffu, eq);
-            if (lane == 0) { S.bg[32u * i + warp] = mg; S.be[32u * i + warp] = me; }
-            n += gt ? 1u : eq ? 1u << 16 : 0u;
+            for (uint32_t j = 0; j < CPT; j++)
+                if (ck[j] && (ck[j] - edge) >> TK_B2F == p2.digit) atomicAdd(&h[(ck[j] - edge) & (TK_BINS - 1u)], 1u);
+            __syncthreads();
+            const TkPick p3 = tk_pick<IX_TK_THREADS>(h, left, S.tot[2], &S.st[2]);
+            if (tx == 0) {
+                S.thr = edge + (p2.digit << TK_B2F) + p3.digit;
+                S.n_gt = p2.above + p3.above;
+            }
         }
-        static_assert(TKC_KEYS < 65536, "two counts share a word");
-        n = sum(n, &S.n_tie);
-        if (NB > 1) {   /* every block tells the others its counts */
-            if (tx < NB) tkc_st(tkc_remote(&S.gcnt[rank], tx), n);
-            tkc_sync<NB>();
-            for (uint32_t r = 0; r < rank; r++) low += S.gcnt[r];
-        }
-    }
-    /* ---- ordered emit: above the threshold in index order, then ties until `need` is full */
-    if (tx < TKC_KEYS / 32u) {
-        const uint32_t v = __popc(S.bg[tx]) | __popc(S.be[tx]) << 16;
-        uint32_t at = v;
+        __syncthreads();
+        thr = S.thr;
+        n_gt = S.n_gt;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= (uint32_t)o) at += y;
-        }
-        if (lane == 31) S.tot[3][warp] = at;
-        asm volatile("bar.sync 1, %0;" ::"n"(TKC_KEYS / 32u) : "memory");
-        S.before[tx] = at - v + __reduce_add_sync(0xffffffffu, lane < warp ? S.tot[3][lane] : 0u);
-    }
-    __syncthreads();
-    auto put = [&](uint32_t k, uint32_t i) {   /* key i of the block's, which reaches the threshold */
-        const uint32_t w = i >> 5, below = (1u << (i & 31u)) - 1u, all = S.before[w] + low, b = rank * TKC_KEYS + i;
-        uint32_t at = k > thr ? all & 0xffffu : n_gt + (all >> 16);
-        if (at >= need) return;
-        at += __popc((k > thr ? S.bg[w] : S.be[w]) & below);
-        if (at < need)
-            for (uint32_t j = 0; j < ratio && at * ratio + j < width; j++) out[at * ratio + j] = (int32_t)(b * ratio + j);
+        for (uint32_t j = 0; j < CPT; j++)
+            if (ck[j] >= thr) {
+                if (NB > 1 && j != rank) {
+                    if ((int)j < (int)rank) atomicAdd(&S.low, ck[j] > thr ? 1u : 1u << 16);
+                } else {
+                    const uint32_t i = S.idx[place(j)];
+                    atomicOr(ck[j] > thr ? &S.bg[i >> 5] : &S.be[i >> 5], 1u << (i & 31u));
+                }
+            }
+        __syncthreads();
+        low = S.low;
+        return true;
     };
-    if (fast) {
+    /* ---- ordered emit: above the threshold in index order, then ties until `need` is full.  The bits' counts before every word: */
+    auto count_words = [&]() {
+        if (tx < TKC_KEYS / 32u) {
+            const uint32_t v = __popc(S.bg[tx]) | __popc(S.be[tx]) << 16;
+            uint32_t sum = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= (uint32_t)o) sum += y;
+            }
+            if (lane == 31) S.tot[3][warp] = sum;
+            asm volatile("bar.sync 1, %0;" ::"n"(TKC_KEYS / 32u) : "memory");
+            S.before[tx] = sum - v + __reduce_add_sync(0xffffffffu, lane < warp ? S.tot[3][lane] : 0u);
+        }
+        __syncthreads();
+    };
+    auto put = [&](uint32_t w, uint32_t i) {   /* the w-th of the list: key i of the block's */
+        const uint32_t b = rank * TKC_KEYS + i;
+        for (uint32_t j = 0; j < ratio && w * ratio + j < width; j++) out[w * ratio + j] = (int32_t)(b * ratio + j);
+    };
+    auto emit = [&]() {
+        count_words();
 #pragma unroll
         for (uint32_t j = 0; j < S.CAP / IX_TK_THREADS; j++) {
             const uint32_t c = tx + j * IX_TK_THREADS;
-            if (c < S.n_own && S.cand[rank][c] >= thr) put(S.cand[rank][c], S.idx[c]);
+            if (c < n_own && S.cand[rank][c] >= thr) {
+                const bool gt = S.cand[rank][c] > thr;
+                const uint32_t i = S.idx[c], all = S.before[i >> 5] + low;
+                uint32_t w = gt ? all & 0xffffu : n_gt + (all >> 16);
+                if (w < need) {
+                    w += __popc((gt ? S.bg[i >> 5] : S.be[i >> 5]) & ((1u << (i & 31u)) - 1u));
+                    if (w < need) put(w, i);
+                }
+            }
         }
-    } else {
+    };
+    constexpr uint32_t ROOM = NB * S.CAP / 4u * 3u;   /* of all blocks, where their shares differ a little */
+    bool wide = at == 0u || (n_vis > S.CAP && (p1.above + p1.cnt) * 16u >= (n_vis / TKC_KEYS * IX_TK_THREADS + min(n_vis % TKC_KEYS, IX_TK_THREADS)) * (NB > 1 ? 11u : 15u));
+    bool over = false;   /* the threshold is above the pivot */
+    if (!wide) {
+        if (collect(std::false_type())) {
+            if (finish()) {
+                emit();
+                return;
+            }
+            over = true;
+        }
+        wide = true;
+    }
+    bool known = true;   /* `low` is */
+#pragma unroll 1
+    while (true) {
+        if (!over) {
+            if (wide ? collect(std::true_type()) : collect(std::false_type())) {
+                if (wide) {   /* they may begin far above the pivot */
+                    uint32_t next = S.own[n_round - 1u].next;
+                    for (uint32_t r = 0; NB > 1 && r < NB; r++) next = min(next, S.told[(n_round - 1u) & 1u].next[r]);
+                    edge = next >> TK_B1 << TK_B1;
+                }
+                if (finish()) {
+                    emit();
+                    return;
+                }
+                over = true;
+            } else if (wide) {
+                over = above >= need;
+            } else if (shift == TK_B1) {
+                wide = true;
+                continue;
+            }
+        }
+        uint32_t *sums = NB > 1 ? S.h2 : S.ha;
+        if (over) {   /* the first digit, of all keys */
+            reinterpret_cast<uint4 *>(hist)[tx] = make_uint4(0u, 0u, 0u, 0u);   /* may have been counted into */
+            reinterpret_cast<uint4 *>(sums)[tx] = make_uint4(0u, 0u, 0u, 0u);
+            clean = false;
+            tkc_sync<NB>();
+#pragma unroll
+            for (uint32_t i = 0; i < TKC_KPT; i++)
+                if (live(i)) atomicAdd(&S.ha[key[i] >> TK_B1], 1u);
+            __syncthreads();
+            if (NB > 1) spread(sums, TK_BINS);
+            const TkPick p = tk_pick<IX_TK_THREADS>(sums, need, S.tot[2], &S.st[2]);
+            at = p.digit;
+            over = false;
+            wide = at == 0u || p.above + p.cnt > ROOM;
+            continue;
+        }
+        if (shift == TK_B1) {
+            const auto &told = S.told[(n_round - 1u) & 1u];
+            uint32_t lo = S.own[n_round - 1u].lo, hi = S.own[n_round - 1u].hi;
+            for (uint32_t r = 0; NB > 1 && r < NB; r++) {
+                lo = min(lo, told.lo[r]);
+                hi = max(hi, told.hi[r]);
+            }
+            n_gt = above;
+            if (lo == hi) {   /* as in rows of ties: the threshold */
+                thr = lo;
+                for (uint32_t r = 0; NB > 1 && r < rank; r++) low += told.n[r];
+                break;
+            }
+            const TkPick p = tk_pick<IX_TK_THREADS>(sums, need - n_gt, S.tot[2], &S.st[2]);
+            at = at << (TK_B1 - TK_B2) | p.digit;
+            shift = TK_B2;
+            n_gt += p.above;
+            wide = false;
+            if (at && n_gt + p.cnt <= ROOM) continue;
+        }
+        /* the last digit */
 #pragma unroll
         for (uint32_t i = 0; i < TKC_KPT; i++)
-            if (live(i) && key[i] >= thr) put(key[i], IX_TK_THREADS * i + tx);
+            if (live(i) && key[i] >> TK_B2 == at) atomicAdd(&(NB > 1 ? S.ha : S.h3)[key[i] & 255u], 1u);
+        __syncthreads();
+        if (NB > 1) spread(S.h3, 256u);
+        const TkPick p = tk_pick256(S.h3, need - n_gt);
+        thr = at << TK_B2 | p.digit;
+        n_gt += p.above;
+        known = NB == 1;
+        break;
+    }
+    /* the list of all keys that reach the threshold; a key that is not there is 0 */
+    uint32_t mg[TKC_KPT], me[TKC_KPT], all[TKC_KPT];
+#pragma unroll
+    for (uint32_t i = 0; i < TKC_KPT; i++) {
+        mg[i] = __ballot_sync(0xffffffffu, key[i] > thr);
+        me[i] = __ballot_sync(0xffffffffu, live(i) && key[i] == thr);
+        if (lane == 0) { S.bg[32u * i + warp] = mg[i]; S.be[32u * i + warp] = me[i]; }
+    }
+    if (!known) {   /* the blocks tell one another what they hold */
+        uint32_t n = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < TKC_KPT; i++) n += __popc(mg[i]) | __popc(me[i]) << 16;
+        if (lane == 0 && n) atomicAdd(&S.own[n_round].n, n);
+        __syncthreads();
+        if (tx < NB) tkc_st(tkc_remote(&S.told[n_round & 1u].n[rank], tx), S.own[n_round].n);
+        tkc_sync<NB>();
+        for (uint32_t r = 0; r < rank; r++) low += S.told[n_round & 1u].n[r];
+    }
+    __syncthreads();
+    count_words();
+#pragma unroll
+    for (uint32_t i = 0; i < TKC_KPT; i++) all[i] = S.before[32u * i + warp] + low;
+#pragma unroll
+    for (uint32_t i = 0; i < TKC_KPT; i++) {
+        const bool gt = (mg[i] >> lane) & 1u;
+        const uint32_t m = gt ? mg[i] : me[i], w = (gt ? all[i] & 0xffffu : n_gt + (all[i] >> 16)) + __popc(m & ((1u << lane) - 1u));
+        if (((m >> lane) & 1u) && w < need) put(w, IX_TK_THREADS * i + tx);
     }
 }
 

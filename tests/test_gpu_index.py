@@ -483,3 +483,42 @@ def test_selection_from_the_threads_maxima(oracle, n_vis):
     d, d_sel = torch.from_numpy(sc).cuda(), torch.full((kinds, width), -7, dtype=torch.int32, device="cuda")
     assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), kinds, n_vis, n_vis, k_blk, RATIO, pos0, width)
     assert np.array_equal(host(d_sel), got)
+
+
+@pytest.mark.parametrize("n_vis", [600, 2100, 8192, 8193, 12000, 24576, 40000, 65536])
+def test_selection_where_the_pivot_has_no_room(oracle, n_vis):
+    """more keys reach the pivot than a block collects: ties at it with enough keys above it, one too few, or none; keys that share
+    12, 24 or all bits with it; keys of a few threads far above it; the least and the largest key there is"""
+    L = lib()
+    k_blk = 512
+    rng = np.random.default_rng(n_vis)
+    i, some, x = np.arange(n_vis), rng.permutation(n_vis), rng.standard_normal(n_vis).astype(np.float32)
+
+    def over_zeros(n):
+        row = np.zeros(n_vis, np.float32)
+        row[some[:n]] = 2 + rng.random(min(n, n_vis))
+        return row
+
+    def near(v):   # one value's leading 24 bits, any last 8
+        return (v.astype(np.float32).view(np.uint32) & ~np.uint32(255) | rng.integers(0, 256, n_vis, dtype=np.uint32)).view(np.float32)
+    rows = [over_zeros(n) for n in (511, 512, 513, 560, 1500)]
+    rows += [np.round(x * q) / q for q in (1, 4, 16)]
+    rows += [1000 + x / 2, -1000 - np.abs(x), near(np.ones(n_vis)), near(np.where(some % 3 == 0, 1.0, 1.0001)), near(-np.ones(n_vis))]
+    rows += [np.where(x > c, 1.0, 0.0) for c in (1.0, 2.5)] + [np.where(x > 1, -1.0, -2.0)]
+    rows += [np.where(i % 1024 < c, 100 + np.abs(x), np.abs(x)) for c in (70, 300)] + [np.where(i % 1024 < 300, 100 + x / 64, np.abs(x))]
+    rows += [np.full(n_vis, v, np.uint32).view(np.float32) for v in (0xffffffff, 0x7fffffff)]
+    rows += [np.where(x > c, np.float32(np.inf), x) for c in (0.0, 2.0)]
+    tiny = over_zeros(300)
+    tiny[some[300:]] = np.full(n_vis - 300 if n_vis > 300 else 0, 0xffffffff, np.uint32).view(np.float32)
+    sc = np.stack([r.astype(np.float32) for r in rows] + [tiny])
+    kinds, width = len(sc), k_blk * RATIO + 3
+    pos0 = n_vis * RATIO - kinds
+    got = np.zeros((kinds, width), np.int32)
+    for t in range(kinds):
+        d, d_sel = torch.from_numpy(sc[t]).cuda(), torch.full((width,), -7, dtype=torch.int32, device="cuda")
+        assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), 1, n_vis, n_vis, k_blk, RATIO, pos0 + t, width)
+        got[t] = host(d_sel)
+        assert np.array_equal(got[t], oracle.ix_topk(sc[t:t + 1], 1, n_vis, k_blk, RATIO, pos0 + t, width)[0]), t
+    d, d_sel = torch.from_numpy(sc).cuda(), torch.full((kinds, width), -7, dtype=torch.int32, device="cuda")
+    assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), kinds, n_vis, n_vis, k_blk, RATIO, pos0, width)
+    assert np.array_equal(host(d_sel), got)
