@@ -326,16 +326,18 @@ __global__ void __launch_bounds__(SC1_WARPS * 32) q4_ix_score1_k(const float *q,
 /* ---- scores of many sessions, one token and one pool each.  The sessions' rows are counted through and every warp takes an equal
  * share of the whole, which may end in one session and begin in the next.  Bound by HBM as long as shared memory keeps up: a
  * 16-byte read costs four cycles of what it returns to a warp, so a lane walks two rows (six reads per 4 dims of 64 rows; with one
- * row per lane, 32-row tiles in two buffers and six warps per SM, ten, and 71 MB of pools took 16.7 us of a layer's 34).  A stage is
- * 64 rows x 32 dims, 128 bytes of each row, so that five can be in flight per warp behind the one that is read; chunk c of row r
- * lies at c ^ (r & 7).  Score + select, us, in two buffers / here: 8 sessions up to 131 072 22.1 / 20.6, of 262 144 59.3 / 54.7,
- * 64 up to 131 072 114.6 / 109.9, of 8000 19.3 / 17.8, 33 up to 30 000 19.8 / 19.8; 2 up to 131 072 13.5 / 14.0. */
-constexpr uint32_t SB_WARPS = 4, SB_STAGES = 6, SB_ROWS = 64, SB_CD = 32, SB_STAGE = SB_ROWS * SB_CD * 4u;
+ * row per lane ten), but one where a tile has no more than 32.  A stage is 64 rows x 32 dims, 128 bytes of each row, two in flight
+ * per warp behind the one that is read; chunk c of row r lies at c ^ (r & 7).  A few sessions are two to five tiles a warp, and
+ * with fewer warps and deeper rings the last, partial one came late.  us from HBM, this kernel alone, six warps of 32-row tiles in
+ * two buffers / four warps of six stages / so: 8 sessions up to 131 072 (74 MB) 19.4 / 20.5 / 18.4, of 131 072 27.8 / 27.0 / 26.3,
+ * 64 up to 131 072 98.5 / 93.1 / 89.9, of 8000 18.4 / 19.7 / 17.4, 33 up to 30 000 18.5 / 19.7 / 18.6, 12 up to 60 000 15.9 / 16.4 /
+ * 16.1, 2 up to 131 072 (16 MB) 9.6 / 10.8 / 10.0. */
+constexpr uint32_t SB_WARPS = 8, SB_STAGES = 3, SB_ROWS = 64, SB_CD = 32, SB_STAGE = SB_ROWS * SB_CD * 4u;
 constexpr uint32_t SB_SMEM = SB_WARPS * (SB_STAGES * SB_STAGE + IX_HD * (uint32_t)sizeof(float4));
 struct SbAt { uint32_t t, row, end, left; const float *pool; };   /* session, rows [row, end) of it, rows of later sessions */
 __global__ void __launch_bounds__(SB_WARPS * 32, 1) q4_ix_score_batch_k(const float *q, float *score, uint32_t stride, uint32_t n_head, uint32_t ratio,
                                                                         const float *const *pools, const int32_t *pos_arr, uint32_t n_sess) {
-    extern __shared__ __align__(128) uint8_t sc_smem[];
+    extern __shared__ __align__(16) uint8_t sc_smem[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t buf = (uint32_t)__cvta_generic_to_shared(sc_smem) + warp * (SB_STAGES * SB_STAGE);
     float4 *qs = reinterpret_cast<float4 *>(sc_smem + SB_WARPS * SB_STAGES * SB_STAGE) + warp * IX_HD;   /* [dim] = the 4 heads' values */
@@ -413,52 +415,57 @@ __global__ void __launch_bounds__(SB_WARPS * 32, 1) q4_ix_score_batch_k(const fl
             for (uint32_t d = lane; d < IX_HD; d += 32u)
                 qs[d] = make_float4(qt[d], n_head > 1 ? qt[IX_HD + d] : 0.f, n_head > 2 ? qt[2 * IX_HD + d] : 0.f, n_head > 3 ? qt[3 * IX_HD + d] : 0.f);
         }
-        float d[2][4];
+        auto walk = [&](auto r) {
+            constexpr int R = decltype(r)::value;   /* rows per lane */
+            float d[R][4];
 #pragma unroll
-        for (int u = 0; u < 2; u++) d[u][0] = d[u][1] = d[u][2] = d[u][3] = 0.f;
+            for (int u = 0; u < R; u++) d[u][0] = d[u][1] = d[u][2] = d[u][3] = 0.f;
 #pragma unroll 1
-        for (uint32_t c = 0; c < IX_HD / SB_CD; c++) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(SB_STAGES - 2u) : "memory");
-            __syncwarp();   /* this stage has landed, and every lane is done with the one before, which is filled again */
-            fetch();
-            const uint32_t row = buf + stage * SB_STAGE + lane * (SB_CD * 4u), x = lane & 7u;
-            if (++stage == SB_STAGES) stage = 0;
-            auto read = [&](uint32_t i, float4 (&k)[2]) {   /* rows lane, lane + 32; stale bytes behind the end are walked and not stored */
+            for (uint32_t c = 0; c < IX_HD / SB_CD; c++) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(SB_STAGES - 2u) : "memory");
+                __syncwarp();   /* this stage has landed, and every lane is done with the one before, which is filled again */
+                fetch();
+                const uint32_t row = buf + stage * SB_STAGE + lane * (SB_CD * 4u), x = lane & 7u;
+                if (++stage == SB_STAGES) stage = 0;
+                auto read = [&](uint32_t i, float4 (&k)[R]) {   /* rows lane, lane + 32; stale bytes behind the end are walked and not stored */
 #pragma unroll
-                for (int u = 0; u < 2; u++)
-                    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(k[u].x), "=f"(k[u].y), "=f"(k[u].z), "=f"(k[u].w)
-                                 : "r"(row + ((i ^ x) << 4) + u * (32u * SB_CD * 4u)));   /* no clobber: the query's reads may go ahead */
-            };
-            float4 k[3][2];
-            read(0, k[0]);
-            read(1, k[1]);
-            const float4 *qc = qs + c * SB_CD;
-#pragma unroll
-            for (uint32_t i = 0; i < SB_CD / 4u; i++) {
-                if (i + 2u < SB_CD / 4u) read(i + 2u, k[(i + 2u) % 3u]);
-                const float4 q0 = qc[4 * i], q1 = qc[4 * i + 1], q2 = qc[4 * i + 2], q3 = qc[4 * i + 3];
-                auto step = [&](const float4 qd, float kd, float (&a)[4]) {
-                    a[0] = __fmaf_rn(qd.x, kd, a[0]); a[1] = __fmaf_rn(qd.y, kd, a[1]); a[2] = __fmaf_rn(qd.z, kd, a[2]); a[3] = __fmaf_rn(qd.w, kd, a[3]);
+                    for (int u = 0; u < R; u++)
+                        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(k[u].x), "=f"(k[u].y), "=f"(k[u].z), "=f"(k[u].w)
+                                     : "r"(row + ((i ^ x) << 4) + u * (32u * SB_CD * 4u)));   /* no clobber: the query's reads may go ahead */
                 };
+                float4 k[3][R];
+                read(0, k[0]);
+                read(1, k[1]);
+                const float4 *qc = qs + c * SB_CD;
 #pragma unroll
-                for (int u = 0; u < 2; u++) step(q0, k[i % 3u][u].x, d[u]);
+                for (uint32_t i = 0; i < SB_CD / 4u; i++) {
+                    if (i + 2u < SB_CD / 4u) read(i + 2u, k[(i + 2u) % 3u]);
+                    const float4 q0 = qc[4 * i], q1 = qc[4 * i + 1], q2 = qc[4 * i + 2], q3 = qc[4 * i + 3];
+                    auto step = [&](const float4 qd, float kd, float (&a)[4]) {
+                        a[0] = __fmaf_rn(qd.x, kd, a[0]); a[1] = __fmaf_rn(qd.y, kd, a[1]); a[2] = __fmaf_rn(qd.z, kd, a[2]); a[3] = __fmaf_rn(qd.w, kd, a[3]);
+                    };
 #pragma unroll
-                for (int u = 0; u < 2; u++) step(q1, k[i % 3u][u].y, d[u]);
+                    for (int u = 0; u < R; u++) step(q0, k[i % 3u][u].x, d[u]);
 #pragma unroll
-                for (int u = 0; u < 2; u++) step(q2, k[i % 3u][u].z, d[u]);
+                    for (int u = 0; u < R; u++) step(q1, k[i % 3u][u].y, d[u]);
 #pragma unroll
-                for (int u = 0; u < 2; u++) step(q3, k[i % 3u][u].w, d[u]);
+                    for (int u = 0; u < R; u++) step(q2, k[i % 3u][u].z, d[u]);
+#pragma unroll
+                    for (int u = 0; u < R; u++) step(q3, k[i % 3u][u].w, d[u]);
+                }
             }
-        }
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            float sc = __fadd_rn(0.f, fmaxf(d[u][0], 0.f));          /* s = 0; s += relu(dot_h) in head order */
-            if (n_head > 1) sc = __fadd_rn(sc, fmaxf(d[u][1], 0.f));
-            if (n_head > 2) sc = __fadd_rn(sc, fmaxf(d[u][2], 0.f));
-            if (n_head > 3) sc = __fadd_rn(sc, fmaxf(d[u][3], 0.f));
-            const uint32_t b = at.row + lane + 32u * u;
-            if (b < at.end) score[(size_t)at.t * stride + b] = sc;
-        }
+            for (int u = 0; u < R; u++) {
+                float sc = __fadd_rn(0.f, fmaxf(d[u][0], 0.f));          /* s = 0; s += relu(dot_h) in head order */
+                if (n_head > 1) sc = __fadd_rn(sc, fmaxf(d[u][1], 0.f));
+                if (n_head > 2) sc = __fadd_rn(sc, fmaxf(d[u][2], 0.f));
+                if (n_head > 3) sc = __fadd_rn(sc, fmaxf(d[u][3], 0.f));
+                const uint32_t b = at.row + lane + 32u * u;
+                if (b < at.end) score[(size_t)at.t * stride + b] = sc;
+            }
+        };
+        if (at.end - at.row > 32u) walk(std::integral_constant<int, 2>());
+        else walk(std::integral_constant<int, 1>());
         next(at);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -1277,7 +1284,7 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         for (uint32_t j = 0; j < CPT; j++)
             if (ck[j] >= thr) {
                 if (NB > 1 && j != rank) {
-                    if ((int)j < (int)rank) atomicAdd(&S.low, ck[j] > thr ? 1u : 1u << 16);
+                    if (j < rank) atomicAdd(&S.low, ck[j] > thr ? 1u : 1u << 16);
                 } else {
                     const uint32_t i = S.idx[place(j)];
                     atomicOr(ck[j] > thr ? &S.bg[i >> 5] : &S.be[i >> 5], 1u << (i & 31u));
@@ -1423,7 +1430,7 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         __syncthreads();
         if (tx < NB) tkc_st(tkc_remote(&S.told[n_round & 1u].n[rank], tx), S.own[n_round].n);
         tkc_sync<NB>();
-        for (uint32_t r = 0; r < rank; r++) low += S.told[n_round & 1u].n[r];
+        for (uint32_t r = 0; NB > 1 && r < rank; r++) low += S.told[n_round & 1u].n[r];
     }
     __syncthreads();
     count_words();

@@ -522,3 +522,30 @@ def test_selection_where_the_pivot_has_no_room(oracle, n_vis):
     d, d_sel = torch.from_numpy(sc).cuda(), torch.full((kinds, width), -7, dtype=torch.int32, device="cuda")
     assert L.q4_hip_qsa_topk(d.data_ptr(), d_sel.data_ptr(), kinds, n_vis, n_vis, k_blk, RATIO, pos0, width)
     assert np.array_equal(host(d_sel), got)
+
+
+@pytest.mark.parametrize("n_head", [1, 2, 3, 4])
+def test_batched_scores_in_equal_shares(oracle, n_head):
+    """sessions whose rows begin and end inside a warp's share, which is many tiles here (8 warps on each SM): tiles of 1 to 64 rows on
+    both sides of 32, empty sessions between long ones; and shares of a few rows, of none"""
+    L = lib()
+    rng = np.random.default_rng(n_head)
+    for blocks in ([40001, 0, 1, 33, 0, 65000, 64, 20007, 0, 31, 50003], [700, 0, 33, 1]):
+        n, stride = len(blocks), 65001 if blocks[0] > 700 else 33000
+        positions = [max(b * RATIO - 1 + i % 2 * 3, 0) for i, b in enumerate(blocks)]
+        q = rng.standard_normal((n, n_head, 128)).astype(np.float32)
+        pools = [rng.standard_normal((max(b, 1) + 1, 128)).astype(np.float32) for b in blocks]
+        d_pools = [dev(p) for p in pools]
+        ptrs = torch.tensor([t.data_ptr() for t in d_pools], dtype=torch.int64, device="cuda")
+        d_pos = torch.tensor(positions, dtype=torch.int32, device="cuda")
+        d_score = torch.full((n, stride), 7.0, device="cuda")
+        d_sel = torch.zeros(n, 67, dtype=torch.int32, device="cuda")
+        assert L.q4_gpu_qsa_select_batch(ptrs.data_ptr(), d_pos.data_ptr(), dev(q).data_ptr(), d_score.data_ptr(), d_sel.data_ptr(), n, stride, n_head,
+                                         128, 16, RATIO, 67)
+        got, sel = host(d_score), host(d_sel)
+        for t, pos in enumerate(positions):
+            nb = (pos + 1) // RATIO
+            want = oracle.ix_score(q[t:t + 1], pools[t], 1, nb, stride, n_head, pos, RATIO) if nb else np.zeros((1, stride), np.float32)
+            assert np.array_equal(got[t, :nb].view(np.uint32), want[0, :nb].view(np.uint32)), t
+            assert (got[t, nb:] == 7.0).all(), t
+            assert np.array_equal(sel[t], oracle.ix_topk(want, 1, stride, 16, RATIO, pos, 67)[0]), t
