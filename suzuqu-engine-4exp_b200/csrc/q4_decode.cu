@@ -2199,9 +2199,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
         c_bytes[slot] = bytes; c_cluster[slot] = p.cluster; c_n[slot] = n;
         return (uint64_t)n;
     };
-    /* The push merge needs extra shared memory; it is used only if that leaves the grid in one wave.
-     * (Asking for still more shared memory, so that a shallow grid spreads one or two blocks deep over all
-     * SMs instead of three deep over some, was measured: no gain at 1-8 sessions, 3 us slower at 16.) */
+    /* The push merge needs extra shared memory; it is used only if that leaves the grid in one wave. */
     if (p.gridmerge && p.hybrid) {
         p.cluster = p.hybrid;
         p.push_bytes = (p.gqa + p.cluster - 1u) / p.cluster * p.cluster * (HD + 4u) * (uint32_t)sizeof(float) + 16u;
@@ -2231,8 +2229,9 @@ bool launch(const DecParams &p_in, dim3 grid) {
     }
     size_t smem = smem_base + p.push_bytes;
     /* A few lists' clusters are spread two blocks deep at most, by asking for half of an SM's shared memory, where all are resident
-     * at once so too (8 sessions 9.3 -> 8.6 us per launch, 10 9.8 -> 8.8; of 12, not: 10.2 -> 14.5). */
-    if (LIST && Cfg::STAGED && p.cluster && smem < DEC_HALF_SM && n_blocks() <= 2u * (uint64_t)g_q4.sm_count && resident_clusters(DEC_HALF_SM) * p.cluster >= n_blocks()) smem = DEC_HALF_SM;
+     * at once so too (8 sessions 9.3 -> 8.6 us per launch, 10 9.8 -> 8.8; of 12, not: 10.2 -> 14.5).  Two warps to a tile: as rings
+     * of four tiles did by their size (8 sessions of 24 / 2 heads of 256 in q8_0 15.6 -> 12.6, 32 / 2 of 128 in fp16 10.3 -> 8.8). */
+    if (LIST && (Cfg::STAGED || Cfg::WPT == 2) && p.cluster && smem < DEC_HALF_SM && n_blocks() <= 2u * (uint64_t)g_q4.sm_count && resident_clusters(DEC_HALF_SM) * p.cluster >= n_blocks()) smem = DEC_HALF_SM;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;

@@ -689,6 +689,28 @@ def test_lists_of_many_tokens_on_both_sides_of_a_wave(n_head, n_kvh, n_tok):
     st.close()
 
 
+@pytest.mark.parametrize("kind,n_head,hd", [(2, 24, 256), (1, 32, 128), (2, 16, 128), (1, 24, 256)])
+@pytest.mark.parametrize("n_tok,width", [(7, 2051), (8, 2051), (11, 2051), (12, 2051), (16, 515), (17, 515)])
+def test_lists_of_a_few_tokens_spread_over_the_sms(kind, n_head, hd, n_tok, width):
+    """clusters of lists, two blocks per SM at most and more, one and two warps to a tile: against the same lists one at a time, each
+    within the tolerance of the oracle's tests"""
+    L = lib()
+    ctx, n_kvh, scale = 3000, 2, float(1 / np.sqrt(hd))
+    g = torch.Generator(device="cuda").manual_seed(n_tok + hd)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    st = q4gpu.KVStore(1, n_kvh, hd, ctx, kind)
+    st.append(0, rn(ctx, n_kvh * hd), rn(ctx, n_kvh * hd), 0, ctx)
+    q, out, ref = rn(n_tok, n_head, hd), torch.empty(n_tok, n_head, hd, device="cuda"), torch.empty(n_tok, n_head, hd, device="cuda")
+    idx = torch.rand(n_tok, ctx, device="cuda", generator=g).topk(width).indices.sort().values.int()
+    idx[1::3, -200:] = -1
+    st.decode_idx_n(0, q, out, n_head, scale, idx, width, n_tok, width)
+    for t in range(n_tok):
+        st.decode_idx_n(0, q[t:], ref[t:], n_head, scale, idx[t:], width, 1, width)
+    assert_close(host(out), host(ref), "%d lists of %d" % (n_tok, width))
+    assert L.q4_gpu_last_error() == 0
+    st.close()
+
+
 @pytest.mark.parametrize("kind,n_head,n_kvh,hd,max_kv,rows", [
     (2, 16, 2, 128, 65536, (14207, 14208, 14209, 14225, 28416, 28433, 64000)), (2, 16, 4, 128, 65536, (7104, 7120, 20000, 35536)), (2, 8, 1, 128, 262144, (16385, 70000, 82000)),
     (1, 16, 2, 128, 65536, (14209, 16384, 49153)), (1, 16, 2, 256, 40000, (14209, 30001)), (2, 16, 2, 256, 32768, (20000, 32768))])
