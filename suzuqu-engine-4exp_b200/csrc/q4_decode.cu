@@ -2225,7 +2225,7 @@ bool launch(const DecParams &p_in, dim3 grid) {
             (void)cudaGetLastError();
             occ = 0;
         }
-        if (n_blocks() > (uint64_t)occ * (uint64_t)g_q4.sm_count) p.gridmerge = 0;
+        if (n_blocks() > (uint64_t)occ * (uint64_t)g_q4.sm_count) p.gridmerge = p.few = 0;   /* the merge in two levels is one of all splits */
     }
     size_t smem = smem_base + p.push_bytes;
     /* A few lists' clusters are spread two blocks deep at most, by asking for half of an SM's shared memory, where all are resident
