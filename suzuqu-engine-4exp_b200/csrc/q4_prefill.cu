@@ -34,8 +34,12 @@
  *     scores, weights and outputs of its own and half of every K and V image, which the tensor cores read from both.  The first
  *     block issues; the second tells it what has landed.  Half the images' traffic from L2, and Q . K^T at the tensor core's
  *     pace: 128 positions of hd 256 with both images 4650 -> 4130 cycles (4096 of products), of two groups at hd 128 3370 -> 3170.
- *     What is told across is an arrival without cluster scope (1000 cycles each with it, and slower than one block): the data
- *     are the asynchronous proxy's or the tensor core's, ordered by the barriers of the block they lie in.
+ *     What orders the two blocks.  Weights, scores and outputs lie in tensor memory: tcgen05 fences before an arrival and behind a
+ *     wait, both relaxed at cluster scope.  Images: a warp of the second block waits for its halves (acquire), and
+ *     arrives behind a release that is restricted to shared memory, which the first block's wait acquires.  A full release takes
+ *     1000 cycles: one for each image, slower than one block; one for all that has landed meanwhile, 0.8 us per block (512 tokens
+ *     over 640 rows of 24 / 2 heads of 256 38.9 -> 39.9 us); restricted it is not to be seen.  A copy by tensor map can count
+ *     its bytes on the other block's barrier, but fetching the map cost the reference host's 2048-token chunk 2674 -> 2751 us.
  *  3. Where the last wave of blocks leaves much of the SMs idle, the positions of its blocks, or of all, are split over
  *     several; those write (O, m, l) and q4_pf_merge_k combines them.
  *
@@ -191,20 +195,44 @@ __device__ __forceinline__ void umma_commit(uint32_t el, uint32_t bar) {
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-/* one probe of a phase; the callers bound the number of probes */
+/* One probe of a phase; the callers bound the number of probes.  What the arrivals order: OWN, what the block itself does; of either
+ * block of a pair PAIR_TENSOR, accesses of tensor memory, between tcgen05 fences, and PAIR_BYTES, what lies in shared memory */
+enum { OWN, PAIR_TENSOR, PAIR_BYTES };
+template <int WHAT>
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     uint32_t done;
+    if constexpr (WHAT == PAIR_TENSOR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    else if constexpr (WHAT == PAIR_BYTES)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0u;
+}
+/* a probe that returns at once */
+__device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
+    uint32_t done;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0u;
 }
-/* on the barrier at that place in the first block of the pair */
+/* on the barrier at that place in the first block of the pair; what comes before it is ordered by a fence, of tcgen05 or release_shared */
 __device__ __forceinline__ void mbar_arrive_first(uint32_t bar) {
-    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [a];\n\t}"
                  ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void release_shared() { asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -404,9 +432,10 @@ __global__ void __launch_bounds__(256) q4_pf_stage_k(const Q4Cache C, uint32_t l
 
 /* the rest of a wait whose first test found the phase incomplete: at most two seconds from the block's start, and no
  * longer than every other thread of the block; out of line, so that the loops around it stay short */
+template <int WHAT>
 __device__ __noinline__ bool pf_wait(uint32_t bar, uint32_t parity, uint32_t s_abort, unsigned long long t_start) {
     for (uint32_t i = 0; i < PF_SPIN_LIMIT; i++) {
-        if (mbar_test(bar, parity)) return true;
+        if (mbar_test<WHAT>(bar, parity)) return true;
         if ((i & 63u) == 63u) {
             uint32_t a;
             asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(a) : "r"(s_abort) : "memory");
@@ -545,11 +574,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
     constexpr uint32_t IDESC_QK = (1u << 4) | ((uint32_t)(UN >> 3) << 17) | ((uint32_t)(PF_ROWS * CTAS >> 4) << 24);
     constexpr uint32_t IDESC_PV = (1u << 4) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(PF_ROWS * CTAS >> 4) << 24);
     const unsigned long long t_start = global_ns();
-    auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_test(bar, parity) || pf_wait(bar, parity, s_abort, t_start); };
+    constexpr int BYTES = PAIR ? PAIR_BYTES : OWN, TENSOR = PAIR ? PAIR_TENSOR : OWN;
+    auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return mbar_test<TENSOR>(bar, parity) || pf_wait<TENSOR>(bar, parity, s_abort, t_start); };
     /* by a whole warp, which goes on as one; the test that succeeds at once stays in line */
     auto all_wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        if (__builtin_expect(__all_sync(0xffffffffu, mbar_test(bar, parity)), 1)) return true;
-        return __all_sync(0xffffffffu, pf_wait(bar, parity, s_abort, t_start));
+        if (__builtin_expect(__all_sync(0xffffffffu, mbar_test<TENSOR>(bar, parity)), 1)) return true;
+        return __all_sync(0xffffffffu, pf_wait<TENSOR>(bar, parity, s_abort, t_start));
+    };
+    auto all_landed = [&](uint32_t bar, uint32_t parity) -> bool {
+        if (__builtin_expect(__all_sync(0xffffffffu, mbar_test<BYTES>(bar, parity)), 1)) return true;
+        return __all_sync(0xffffffffu, pf_wait<BYTES>(bar, parity, s_abort, t_start));
     };
     /* order of the images in the ring, that of their first use: K0 V0 K1 V1 .. where two groups share a tile, K0 K1 V0 K2
      * V1 .. V(n-1) where units are tiles (the scores run a tile and two tiles ahead of P . V) */
@@ -562,7 +596,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
             auto load = [&](const uint8_t *src, uint32_t chunks) {
                 for (uint32_t c = 0; c < chunks && ok; c++, at++) {
                     const uint32_t s = at % SLOTS, use = at / SLOTS;
-                    if (use > 0) ok = wait(empty + 8 * s, (use - 1u) & 1u);
+                    if (use > 0) ok = mbar_test<BYTES>(empty + 8 * s, (use - 1u) & 1u) || pf_wait<BYTES>(empty + 8 * s, (use - 1u) & 1u, s_abort, t_start);
                     if (ok) {
                         mbar_expect_tx(full + 8 * s, PIECE);
                         bulk_load(sR + s * PIECE, src + (size_t)c * PF_CHUNK + rank * PIECE, PIECE, full + 8 * s);
@@ -582,16 +616,25 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
              * (bounded again; these probes ignore the abort flag; phases that completed long ago answer at once). */
             if (!ok)
                 for (uint32_t t = at > SLOTS ? at - SLOTS : 0; t < at; t++)
-                    for (uint32_t i = 0; i < 4096u && !mbar_test(full + 8 * (t % SLOTS), (t / SLOTS) & 1u); i++) {}
+                    for (uint32_t i = 0; i < 4096u && !mbar_test<BYTES>(full + 8 * (t % SLOTS), (t / SLOTS) & 1u); i++) {}
         }
     } else if (PAIR && warp == SW && rank != 0u) {
         /* ================= second block of a pair: the products are issued in the first, which learns here what has landed ====== */
-        if (lane == 0)
-            for (uint32_t at = 0; at < n_tiles * (CK + CV); at++) {
-                ok = wait(full + 8 * (at % SLOTS), (at / SLOTS) & 1u);
+        /* All that has landed at once (one by one the reference host's chunk takes 2683 us, so 2671).  A slot's next image is not
+         * requested before this one has been told and used: the phases that are looked at are the present ones. */
+        for (uint32_t at = 0, n = n_tiles * (CK + CV); at < n;) {
+            const uint32_t i = at + lane;
+            const uint32_t here = __ballot_sync(0xffffffffu, lane < SLOTS && i < n && mbar_peek(full + 8 * (i % SLOTS), (i / SLOTS) & 1u));
+            const uint32_t k = (uint32_t)__ffs((int)~here) - 1u;
+            if (k == 0u) {
+                ok = all_landed(full + 8 * (at % SLOTS), (at / SLOTS) & 1u);
                 if (!ok) break;
-                mbar_arrive_first(full + 8 * (at % SLOTS));
+                continue;
             }
+            release_shared();
+            if (lane < k) mbar_arrive_first(full + 8 * (i % SLOTS));
+            at += k;
+        }
     } else if (warp == SW) {
         /* ================= tensor-core issuer: a converged warp, one elected lane ================= */
         if (n_tiles > 0) {
@@ -600,7 +643,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
             uint32_t slot = 0, phase = 0;
             auto take = [&]() -> uint32_t {
                 const uint32_t s = slot;
-                ok = ok && all_wait(full + 8 * s, phase);
+                ok = ok && all_landed(full + 8 * s, phase);
                 if (++slot == SLOTS) { slot = 0; phase ^= 1u; }
                 return s;
             };
