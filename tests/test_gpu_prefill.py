@@ -159,7 +159,8 @@ def test_prefill_large_magnitude_queries(oracle, mode):
 @pytest.mark.parametrize("kind", [2, 1, 0])
 @pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base,max_kv", [
     (24, 2, 256, 40, 0, 40), (24, 2, 256, 23, 1000, 1023), (4, 4, 256, 130, 127, 257), (16, 1, 256, 9, 640, 640),
-    (16, 2, 128, 300, 500, 800), (16, 2, 128, 8, 2000, 2008), (3, 1, 128, 129, 0, 129), (16, 2, 128, 100, 30, 90), (64, 4, 128, 301, 200, 501)])
+    (16, 2, 128, 300, 500, 800), (16, 2, 128, 8, 2000, 2008), (3, 1, 128, 129, 0, 129), (16, 2, 128, 100, 30, 90), (64, 4, 128, 301, 200, 501),
+    (24, 2, 256, 250, 2100, 2300), (24, 2, 256, 250, 2100, 2112)])   # pairs of blocks
 def test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, n_head, n_kvh, hd, n_tok, kv_base, max_kv):
     """q4_hip_qsa_decode_n with a prompt's slice on caches in the reference layout: every kind at both head sizes, group
     sizes that do not divide the 128-row tiles, tile edges, position ranges split over several blocks (few tokens
@@ -322,7 +323,8 @@ def test_first_token_of_a_reference_abi_chunk_is_its_value_row(oracle, n_head, n
 
 
 @pytest.mark.parametrize("kind,big", [(2, 900.0), (0, 1.0e5)])
-@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base", [(24, 2, 256, 7, 300), (24, 2, 256, 40, 300), (16, 2, 128, 7, 300), (16, 2, 128, 140, 300)])
+@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base", [(24, 2, 256, 7, 300), (24, 2, 256, 40, 300), (16, 2, 128, 7, 300), (16, 2, 128, 140, 300),
+                                                        (24, 2, 256, 250, 2100), (16, 2, 128, 391, 1600)])   # pairs of blocks
 def test_reference_abi_chunk_of_rows_beyond_fp16(oracle, kind, big, n_head, n_kvh, hd, n_tok, kv_base):
     """values beyond 65504 in some rows of K and of V (q8_0: a block scale of 900 is a legal fp16; fp32: magnitudes of 1e5, in
     one dim that the queries leave out, since the decode form rounds fp32 rows to fp16): finite and right for few tokens and for
@@ -356,13 +358,14 @@ def test_reference_abi_chunk_of_rows_beyond_fp16(oracle, kind, big, n_head, n_kv
 
 
 @pytest.mark.parametrize("kind", [2, 1, 0])
-@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok", [(24, 2, 256, 40), (16, 2, 128, 140)])
-def test_reference_abi_chunk_with_value_rows_that_are_not_finite(oracle, kind, n_head, n_kvh, hd, n_tok):
+@pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base,at", [(24, 2, 256, 40, 200, 17), (16, 2, 128, 140, 200, 17),
+                                                                (24, 2, 256, 250, 2100, 75), (24, 2, 256, 250, 2100, 76), (16, 2, 128, 391, 1600, 64)])   # pairs of blocks, both sides of a tile
+def test_reference_abi_chunk_with_value_rows_that_are_not_finite(oracle, kind, n_head, n_kvh, hd, n_tok, kv_base, at):
     """a token's output depends on the rows up to its own: those before a row with an infinity or NaN in V stay as they are, the
     others get NaN"""
     from gpu_util import assert_close
     L = lib()
-    kv_base, at, kvw = 200, 17, n_kvh * hd
+    kvw = n_kvh * hd
     n = kv_base + n_tok
     k, v = oracle.normal(61, 0, n * kvw).reshape(n, kvw), oracle.normal(61, 1, n * kvw).reshape(n, kvw).copy()
     q, g = oracle.normal(61, 2, n_tok * n_head * hd).reshape(n_tok, n_head, hd), oracle.normal(61, 3, n_tok * n_head * hd).reshape(n_tok, n_head, hd)
@@ -554,11 +557,12 @@ def test_last_wave_split_over_positions_of_a_callers_cache(kind, n_head, hd, n_t
     (2, 24, 2, 256, 241, 512, 52), (2, 24, 2, 256, 241, 511, 50),            # 25 groups of 10 tokens, the last pair's second one empty; one block each
     (2, 24, 2, 256, 250, 1000, 52), (2, 32, 2, 256, 199, 700, 52),           # full groups; 16 query heads per kv head
     (2, 16, 2, 128, 391, 1536, 52), (2, 16, 2, 128, 391, 1535, 50), (2, 16, 2, 128, 384, 5000, 48), (2, 9, 3, 128, 673, 1537, 54), (2, 1, 1, 128, 6100, 1700, 48),
+    (2, 24, 2, 256, 512, 512, 104), (2, 24, 2, 256, 512, 1000, 104), (1, 24, 2, 256, 512, 4000, 104), (0, 24, 2, 256, 512, 4000, 104),   # whole: nothing to merge
     (1, 24, 2, 256, 241, 2048, 52), (1, 24, 2, 256, 241, 2047, 50), (0, 24, 2, 256, 250, 2100, 52), (0, 4, 1, 256, 1537, 2049, 50),
     (-1, 16, 2, 128, 3010, 14336, 192), (-1, 16, 2, 128, 3010, 14335, 190), (-1, 32, 2, 128, 1510, 15000, 192)])   # the library's store: two groups per block
 def test_pairs_of_blocks(kind, n_head, n_kvh, hd, n_tok, kv_base, blocks):
-    """chunks behind a prefix on both sides of the line from which two blocks form one product: all tokens against 64 bits, twice the
-    same, nothing written behind the output, and the number of blocks (of a pair both count)"""
+    """chunks behind a prefix on both sides of the line from which two blocks form one product: all tokens against 64 bits, twice and
+    captured the same, nothing written behind the output, and the number of blocks (of a pair both count); one wave of pairs is not split"""
     from gpu_util import assert_close
     L = lib()
     ctx = kv_base + n_tok
@@ -592,10 +596,20 @@ def test_pairs_of_blocks(kind, n_head, n_kvh, hd, n_tok, kv_base, blocks):
     for _ in range(2):
         out = torch.full((n_tok + 64, n_head, hd), 7.0, dtype=dtype, device="cuda")
         run(out)
-        whole, late, _ = layout(L)
-        assert whole + late == blocks
+        whole, late, ranges = layout(L)
+        assert whole + late == blocks and (ranges == 1 or blocks != 104)
         outs.append(out)
     assert torch.equal(outs[0], outs[1]) and (outs[0][n_tok:] == 7.0).all()
+    torch.cuda.synchronize()
+    assert L.q4_gpu_set_stream(None) and L.q4_hip_graph_begin() == 1   # the library's own stream: the default one is not captured
+    run(outs[1])
+    graph = L.q4_hip_graph_end()
+    outs[1].fill_(7.0)
+    torch.cuda.synchronize()
+    assert graph and L.q4_hip_graph_launch(graph) and L.q4_hip_stream_sync()
+    assert torch.equal(outs[0], outs[1]) and layout(L)[0] + layout(L)[1] == blocks
+    L.q4_hip_graph_free(graph)
+    q4gpu.use_torch_stream()
     k, v = (rows_of(r, ctx, n_kvh, hd, 2 if kind < 0 else kind) for r in raw)
     ref = exact_attention(q, k, v, gate, n_head, n_kvh, kv_base, scale)
     (check if kind < 0 else assert_close)(host(outs[0][:n_tok].float()), ref, "%d over %d" % (n_tok, kv_base))
