@@ -1101,34 +1101,45 @@ bool stage(const Q4PrefillArgs &a, uint32_t n, uint32_t tiles, uint32_t unit, ui
  * 1.2 us, 0.2 per range, and 7 KB per ns.  600 tokens over 16 384 (76 blocks): 146 us in one range, 112 in three.
  * Two groups per block: a tile 1.8 us, a block 5.  There, and with more blocks than SMs, only those of the last wave are split,
  * the shortest of the chunk: 8192 tokens over 16 384 are 512 blocks, 444 and 68 x 2. */
-struct PfSplit { uint32_t whole, ranges; };
+struct PfSplit { uint32_t whole, ranges; uint64_t ns; };   /* ns: the estimate, to compare single blocks and pairs by */
 PfSplit best_split(uint32_t groups, uint32_t n_kvh, uint32_t sms, uint32_t kv_base, uint32_t tok_per_group, uint32_t tiles, uint64_t rows, uint32_t rows_per_group, uint32_t hd,
-                   uint32_t np, uint32_t nq) {
+                   uint32_t np, uint32_t nq, bool pair) {
     const uint32_t blocks = groups * n_kvh, waves = blocks / sms, rest = blocks % sms;
-    const uint64_t tile = nq == 2 ? 1800u : 640u + 190u * (hd / 128u) * 2u * np, block = nq == 2 ? 5000u : 2000u + 2000u * (hd / 128u);
+    uint64_t tile = nq == 2 ? 1800u : 640u + 190u * (hd / 128u) * 2u * np, block = nq == 2 ? 5000u : 2000u + 2000u * (hd / 128u);
     auto merge = [&](uint64_t n, uint32_t s) -> uint64_t { return 1200u + 200u * s + n * hd * s * 8u / 7000u; };
-    PfSplit r = {blocks, 1u};
-    const uint64_t whole = (waves + (rest != 0u)) * (tiles * tile + block);
+    /* The last wave's blocks are the last kv head's first tokens. */
+    const uint32_t seen = (kv_base + (rest < groups ? rest : groups) * tok_per_group + PF_BN - 1u) / PF_BN, n = seen < tiles ? seen : tiles;
+    auto all_in = [&](uint32_t s) -> uint64_t { return ((uint64_t)blocks * s + sms - 1u) / sms * ((tiles + s - 1u) / s * tile + block) + (s > 1u ? merge(rows, s) : 0u); };
+    auto rest_in = [&](uint32_t s) -> uint64_t { return waves * (tiles * tile + block) + (n + s - 1u) / s * tile + block + merge((uint64_t)rest * rows_per_group, s); };
+    PfSplit r = {blocks, 1u, 0u};
+    const uint64_t whole = all_in(1u);
     uint64_t best = whole - whole / 16u;   /* whole blocks need no merge: left for a clear gain only (causal chunks have less work) */
     for (uint32_t s = 2; s <= 16u && s <= tiles; s++) {
         if (nq == 1) {
-            const uint64_t t = ((uint64_t)blocks * s + sms - 1u) / sms * ((tiles + s - 1u) / s * tile + block) + merge(rows, s);
+            const uint64_t t = all_in(s);
             if (t < best) {
                 best = t;
-                r = {0u, s};
+                r = {0u, s, 0u};
             }
         }
-        /* The last wave's blocks are the last kv head's first tokens.  Where they are much shorter than the chunk's last tokens', as
-         * without a prefix, the blocks before them end so far apart that they fill the gaps (8192 tokens over none 240 us, split 255). */
-        const uint32_t seen = (kv_base + (rest < groups ? rest : groups) * tok_per_group + PF_BN - 1u) / PF_BN, n = seen < tiles ? seen : tiles;
+        /* Where they are much shorter than the chunk's last tokens', as without a prefix, the blocks before them end so far apart that
+         * they fill the gaps (8192 tokens over none 240 us, split 255). */
         if (waves && rest && rest * s <= sms && n >= 2u * (tiles - kv_base / PF_BN)) {
-            const uint64_t t = waves * (tiles * tile + block) + (n + s - 1u) / s * tile + block + merge((uint64_t)rest * rows_per_group, s), now = waves * (tiles * tile + block) + n * tile + block;
+            const uint64_t t = rest_in(s), now = waves * (tiles * tile + block) + n * tile + block;
             if (t < best && t < now) {
                 best = t;
-                r = {blocks - rest, s};
+                r = {blocks - rest, s, 0u};
             }
         }
     }
+    /* Pairs: their products are the tensor core's 64 cycles per 128 x 128 x 16 where one block's wait for shared memory, and meeting
+     * costs a microsecond. */
+    if (pair) {
+        tile = tile * (np == 2 ? 89u : nq == 2 ? 97u : 93u) / 100u;
+        block += 1000u;
+    }
+    r.ns = r.ranges == 1u ? all_in(1u) : r.whole ? rest_in(r.ranges) : all_in(r.ranges);
+    if (r.ranges == 1u) r.ns -= r.ns / 32u;
     return r;
 }
 
@@ -1158,20 +1169,33 @@ int q4i_prefill(const Q4PrefillArgs &a) {
      * against 591; between 300 and 400 it depends on the depth. */
     const uint32_t nq = hd == 128 && np == 1u && groups * a.n_kvh * 2u > sms * 5u ? 2u : 1u;
     const uint32_t prefix = a.kv_base / PF_BN;
-    const bool pair = groups * a.n_kvh >= 48u && (np == 2u ? prefix >= (hd == 256u ? 4u : 12u) : hd == 256u ? prefix >= 16u : nq == 2u && a.layout == LAY_Q8P && prefix >= 112u);
-    const uint32_t ctas = pair ? 2u : 1u, unit = pair ? (nq == 2u ? 6u : 7u) : 0u;
-    /* Pairs of blocks behind a prefix: their products are the tensor core's 64 cycles per 128 x 128 x 16 where one block's wait for
-     * shared memory, and meeting costs a microsecond.  us, one block / pairs.  Both images: 512 tokens over 512 at hd 256 39.5 / 37.8,
-     * 2048 over 4000 392 / 361, at hd 128 144 / 128, 512 over 512 21.4 / 22.4, over 1536 27.7 / 27.5 (2048 over none at hd 256 120 / 121).  One image at hd 256: 512 over 512 24.8 / 25.4, 2048 over
-     * 4000 227 / 212.  Two groups per block: 8192 over 5000 515 / 514, 16 384 1159 / 1130, 40 000 2463 / 2389; with marks 8192 over 8000
-     * 758 / 760; one group at hd 128 600 over 16 384 115 / 121.  And not for a few blocks in ranges (100 over 4000 39.6 / 40.2). */
-    const uint32_t n_groups = (groups + nq * ctas - 1u) / (nq * ctas), tok_per_group = tpc * nq * ctas, blocks = n_groups * a.n_kvh;
+    /* Pairs of blocks behind a prefix, where they are estimated to take 1.5 % less.  How many pairs fill the places of a wave, and how
+     * many ranges fit, moves a chunk by up to 20 % either way: 24 / 2 heads of 256 over 2048 rows of fp16, 350 tokens 1 % more in
+     * pairs, 380 2 % less; one kv head with 8 heads of 256 over 2048 rows of q8_0, 850 tokens 4 % less, but 770, 25 pairs in two ranges
+     * instead of 49 blocks in three, 10 % more; 32 / 2 heads, 290 tokens 35 % more.  us, one block / pairs.  Both images: 512 tokens over
+     * 512 at hd 256 39.5 / 37.8, 2048 over 4000 392 / 361, at hd 128 144 / 128, 512 over 512 21.4 / 22.4, over 1536 27.7 / 27.5 (2048
+     * over none at hd 256 120 / 121).  One image at hd 256: 512 over 512 24.8 / 25.4, 2048 over 4000 227 / 212.  Two groups per block:
+     * 8192 over 5000 515 / 514, 16 384 1159 / 1130, 40 000 2463 / 2389 (as long up to 12 000 rows, 1 % less over 14 336 and 20 000);
+     * with marks 8192 over 8000 758 / 760; one group at hd 128 600 over 16 384 115 / 121.  And not for a few blocks in ranges (100 over
+     * 4000 39.6 / 40.2). */
     const size_t k_bytes = (size_t)a.n_kvh * tiles * np * (hd / 128u) * PF_CHUNK, v_bytes = k_bytes, m_bytes = (size_t)a.n_kvh * tiles * (PF_BN / 32u) * (sizeof(PfMark) + 4u);   /* marks, flags (two bytes used per mark) */
-    PfSplit sp = best_split(n_groups, a.n_kvh, sms / ctas, a.kv_base, tok_per_group, tiles, (uint64_t)a.n_tok * a.n_head, tok_per_group * gqa, hd, np, nq);
+    auto layout = [&](uint32_t ctas) -> PfSplit {
+        const uint32_t per = tpc * nq * ctas;
+        return best_split((groups + nq * ctas - 1u) / (nq * ctas), a.n_kvh, sms / ctas, a.kv_base, per, tiles, (uint64_t)a.n_tok * a.n_head, per * gqa, hd, np, nq, ctas == 2u);
+    };
+    PfSplit sp = layout(1u);
+    bool pair = groups * a.n_kvh >= 48u && (np == 2u ? prefix >= (hd == 256u ? 4u : 12u) : hd == 256u ? prefix >= 16u : nq == 2u && a.layout == LAY_Q8P && prefix >= 112u);
+    if (pair) {
+        const PfSplit two = layout(2u);
+        pair = two.ns * 1000u < sp.ns * 985u;
+        if (pair) sp = two;
+    }
+    const uint32_t ctas = pair ? 2u : 1u, unit = pair ? (nq == 2u ? 6u : 7u) : 0u;
+    const uint32_t n_groups = (groups + nq * ctas - 1u) / (nq * ctas), tok_per_group = tpc * nq * ctas, blocks = n_groups * a.n_kvh;
     uint32_t part_tok;
     size_t rows, part_bytes;
     int room;
-    for (;; sp = {blocks, 1u}) {
+    for (;; sp = {blocks, 1u, 0u}) {
         /* tokens that parts are kept for: those of the groups at the end of the order */
         const uint32_t late = blocks - sp.whole;
         const uint64_t late_tok = (uint64_t)(late < n_groups ? late : n_groups) * tok_per_group;

@@ -160,7 +160,7 @@ def test_prefill_large_magnitude_queries(oracle, mode):
 @pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base,max_kv", [
     (24, 2, 256, 40, 0, 40), (24, 2, 256, 23, 1000, 1023), (4, 4, 256, 130, 127, 257), (16, 1, 256, 9, 640, 640),
     (16, 2, 128, 300, 500, 800), (16, 2, 128, 8, 2000, 2008), (3, 1, 128, 129, 0, 129), (16, 2, 128, 100, 30, 90), (64, 4, 128, 301, 200, 501),
-    (24, 2, 256, 250, 2100, 2300), (24, 2, 256, 250, 2100, 2112)])   # pairs of blocks
+    (24, 2, 256, 385, 2100, 2400), (24, 2, 256, 385, 2100, 2112)])   # pairs of blocks
 def test_reference_abi_chunks_on_the_tensor_cores(oracle, kind, n_head, n_kvh, hd, n_tok, kv_base, max_kv):
     """q4_hip_qsa_decode_n with a prompt's slice on caches in the reference layout: every kind at both head sizes, group
     sizes that do not divide the 128-row tiles, tile edges, position ranges split over several blocks (few tokens
@@ -324,7 +324,7 @@ def test_first_token_of_a_reference_abi_chunk_is_its_value_row(oracle, n_head, n
 
 @pytest.mark.parametrize("kind,big", [(2, 900.0), (0, 1.0e5)])
 @pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base", [(24, 2, 256, 7, 300), (24, 2, 256, 40, 300), (16, 2, 128, 7, 300), (16, 2, 128, 140, 300),
-                                                        (24, 2, 256, 250, 2100), (16, 2, 128, 391, 1600)])   # pairs of blocks
+                                                        (24, 2, 256, 385, 2100), (16, 2, 128, 610, 1600)])   # pairs of blocks
 def test_reference_abi_chunk_of_rows_beyond_fp16(oracle, kind, big, n_head, n_kvh, hd, n_tok, kv_base):
     """values beyond 65504 in some rows of K and of V (q8_0: a block scale of 900 is a legal fp16; fp32: magnitudes of 1e5, in
     one dim that the queries leave out, since the decode form rounds fp32 rows to fp16): finite and right for few tokens and for
@@ -359,7 +359,7 @@ def test_reference_abi_chunk_of_rows_beyond_fp16(oracle, kind, big, n_head, n_kv
 
 @pytest.mark.parametrize("kind", [2, 1, 0])
 @pytest.mark.parametrize("n_head,n_kvh,hd,n_tok,kv_base,at", [(24, 2, 256, 40, 200, 17), (16, 2, 128, 140, 200, 17),
-                                                                (24, 2, 256, 250, 2100, 75), (24, 2, 256, 250, 2100, 76), (16, 2, 128, 391, 1600, 64)])   # pairs of blocks, both sides of a tile
+                                                                (24, 2, 256, 385, 2100, 75), (24, 2, 256, 385, 2100, 76), (16, 2, 128, 610, 1600, 64)])   # pairs of blocks, both sides of a tile
 def test_reference_abi_chunk_with_value_rows_that_are_not_finite(oracle, kind, n_head, n_kvh, hd, n_tok, kv_base, at):
     """a token's output depends on the rows up to its own: those before a row with an infinity or NaN in V stay as they are, the
     others get NaN"""
@@ -553,12 +553,17 @@ def test_last_wave_split_over_positions_of_a_callers_cache(kind, n_head, hd, n_t
     assert L.q4_gpu_last_error() == 0
 
 
+@on_148_sms
 @pytest.mark.parametrize("kind,n_head,n_kvh,hd,n_tok,kv_base,blocks", [
-    (2, 24, 2, 256, 241, 512, 52), (2, 24, 2, 256, 241, 511, 50),            # 25 groups of 10 tokens, the last pair's second one empty; one block each
-    (2, 24, 2, 256, 250, 1000, 52), (2, 32, 2, 256, 199, 700, 52),           # full groups; 16 query heads per kv head
-    (2, 16, 2, 128, 391, 1536, 52), (2, 16, 2, 128, 391, 1535, 50), (2, 16, 2, 128, 384, 5000, 48), (2, 9, 3, 128, 673, 1537, 54), (2, 1, 1, 128, 6100, 1700, 48),
+    (2, 24, 2, 256, 241, 512, 50), (2, 24, 2, 256, 241, 511, 50),            # 25 groups of 10 tokens in two ranges: one block each
+    (2, 24, 2, 256, 381, 512, 80), (2, 24, 2, 256, 381, 511, 78),            # 39 groups, the last pair's second one empty; one block each
+    (2, 24, 2, 256, 250, 1000, 50), (2, 32, 2, 256, 199, 700, 50), (2, 24, 2, 256, 241, 3000, 52), (2, 32, 2, 256, 199, 2500, 52),   # pairs in ranges; 16 query heads per kv head
+    (2, 16, 2, 128, 391, 1536, 50), (2, 16, 2, 128, 391, 1535, 50), (2, 16, 2, 128, 610, 1536, 80), (2, 16, 2, 128, 610, 1535, 78), (2, 16, 2, 128, 391, 2500, 52),
+    (2, 16, 2, 128, 384, 5000, 48), (2, 9, 3, 128, 673, 1537, 54), (2, 1, 1, 128, 6100, 1700, 48),
     (2, 24, 2, 256, 512, 512, 104), (2, 24, 2, 256, 512, 1000, 104), (1, 24, 2, 256, 512, 4000, 104), (0, 24, 2, 256, 512, 4000, 104),   # whole: nothing to merge
-    (1, 24, 2, 256, 241, 2048, 52), (1, 24, 2, 256, 241, 2047, 50), (0, 24, 2, 256, 250, 2100, 52), (0, 4, 1, 256, 1537, 2049, 50),
+    (1, 24, 2, 256, 241, 2048, 50), (1, 24, 2, 256, 241, 2047, 50), (1, 24, 2, 256, 381, 2048, 80), (1, 24, 2, 256, 381, 2047, 78),
+    (0, 24, 2, 256, 250, 2100, 50), (0, 24, 2, 256, 250, 5000, 52), (0, 4, 1, 256, 1537, 2049, 49), (0, 4, 1, 256, 1601, 5000, 52),
+    (2, 8, 1, 256, 770, 2048, 49), (2, 8, 1, 256, 850, 2048, 54), (2, 32, 2, 256, 290, 2048, 74),                # pairs would fill fewer places
     (-1, 16, 2, 128, 3010, 14336, 192), (-1, 16, 2, 128, 3010, 14335, 190), (-1, 32, 2, 128, 1510, 15000, 192)])   # the library's store: two groups per block
 def test_pairs_of_blocks(kind, n_head, n_kvh, hd, n_tok, kv_base, blocks):
     """chunks behind a prefix on both sides of the line from which two blocks form one product: all tokens against 64 bits, twice and
