@@ -11,9 +11,9 @@
  * scalar FMA pipe cannot keep up with B200's memory system (8 FMA per int8 byte at ~23 B/clk/SM
  * is more than the 128 FMA/clk an SM has), so the two contractions run on the tensor cores with
  * warp-level MMA.  Every byte of the cache is read from global memory once.  At hd 128 and 256 every warp (or, with more
- * than 8 query heads per kv head, two warps that share it) owns a ring of 16-position tiles in shared memory, two to four
- * deep, filled with asynchronous copies of whole rows or records; in a dense scan of the native q8_0 store at hd 128 a
- * tile is one contiguous span and one 4352-byte bulk copy (cp.async.bulk, completion on the stage's mbarrier).  That
+ * than 8 query heads per kv head, two warps that share it) owns a ring of 16-position tiles in shared memory, two deep (where
+ * two do not fit one, up to three in fp16 at hd 128), filled with asynchronous copies of whole rows or records; in a dense scan of
+ * the native q8_0 store at hd 128 a tile is one contiguous span and one 4352-byte bulk copy (cp.async.bulk, completion on the stage's mbarrier).  That
  * layout's warps unload a stage into MMA fragments (ldmatrix for the K rows, transposing ldmatrix for the V rows),
  * refill it at once with the tile two ahead and compute from registers; the others read fragments from the stage as the
  * products need them and refill it then.  No block barrier in the main loop.  Queries are requested coalesced ahead of

@@ -142,8 +142,8 @@ constexpr uint32_t SC_ROW_FLOATS = IX_HD + 4, SC_WARPS = 2;
 constexpr uint32_t SC_TILE_BYTES = 32u * SC_ROW_FLOATS * sizeof(float);
 constexpr uint32_t SC_SMEM = SC_WARPS * 2u * SC_TILE_BYTES + IX_HD * sizeof(float4);
 /* SC_EACH: sessions with a pool and a position of their own, while there is room for a block per two tiles of every session; more
- * rows share the blocks (q4_ix_score_batch_k), which costs some counting (select of 2 sessions of 512 blocks, shared out 7.6 us,
- * 5.5 so). */
+ * rows share the blocks (q4_ix_score_batch_k), which costs some counting (score + select, shared out / so: 2 sessions of 512 blocks
+ * 6.2 / 4.2 us, of 14 000, almost all the room, 11.7 / 10.7; 8 of 3500 10.5 / 9.6). */
 enum { SC_ONE, SC_EACH };
 template <int FORM>
 __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, const float *pool, float *score,
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(SC_WARPS * 32) q4_ix_score_k(const float *q, c
  * that would not fit.  Eight steps in line, not 32: the kernel's image is fetched anew by every launch.
  * us, the form above / here: 64 rows 2.57 / 2.4, 4096 2.66 / 2.14, 16 384 4.28 / 4.1, 32 768 6.66 / 5.2, 65 536 9.3 / 8.5.
  * ahead: all blocks but the newest are requested before the wait (q4i_blocks_ahead), under whatever this launch's pooling still
- * waits for: a 262144-token select step 298.5 -> 255 us, the reference host's token 361 -> 345. */
+ * waits for: a 262144-token select step 298.5 -> 255 to 272 us from one card to another, the reference host's token 361 -> 340 to 350. */
 constexpr uint32_t SC1_WARPS = 7, SC1_ROWS = SC1_WARPS * 64, SC1_SHORT = 128, SC1_SMEM = IX_HD * (uint32_t)sizeof(float4) + SC1_ROWS * IX_HD * (uint32_t)sizeof(float);
 /* rows at .. at + 32 R - 1, below r1, by one warp */
 template <int R>
@@ -1036,8 +1036,8 @@ __global__ void __launch_bounds__(IX_TK_THREADS) q4_ix_topkc_k(const float *scor
         n_vis = (pos + 1u) / ratio;
         if (pp) n_read = min(stride, n_vis);
     }
-    /* The block's own shared memory is prepared, and the cluster has met once, before the launch waits for
-     * the previous kernel: with programmatic dependent launch this part runs under that kernel's tail. */
+    /* The block's own shared memory is prepared before the launch waits for the previous kernel: with programmatic dependent
+     * launch this part runs under that kernel's tail. */
     constexpr uint32_t BPT = TK_BINS / IX_TK_THREADS;   /* bins per thread */
     static_assert(BPT == 4, "one 16-byte word of counts per thread");
     uint32_t *hist = NB > 1 ? S.ha : S.h2;
@@ -1709,8 +1709,9 @@ bool topkm_start(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stri
                     ratio, pos0, width, words, pp, pos_arr);
 }
 /* Which form: rows of up to 8192 keys need one block either way, which keeps them in registers.  Longer rows take the
- * cluster form while all clusters are resident at once (two blocks of 1024 threads per SM), the streaming form beyond
- * (512 tokens x 32 768 keys), and the single block that re-reads the row behind 65 536 keys. */
+ * cluster form up to two blocks per SM, which are two or three waves, for a block of 1024 threads fills an SM's registers (us, the
+ * last so / the next one streamed: 37 / 38 tokens of 65 536 keys 21.7 / 27.6, 74 / 75 of 32 768 18.9 / 17.4, 148 / 149 of 16 384 13.1 /
+ * 14.5), the streaming form beyond (512 tokens x 32 768 keys), and the single block that re-reads the row behind 65 536 keys. */
 bool launch_topk(const float *score, int32_t *sel, uint32_t n_tok, uint32_t stride, uint32_t k_blk, uint32_t ratio,
                  uint32_t pos0, uint32_t width, const int32_t *pp, const int32_t *pos_arr = nullptr) {
     if (stride > TKC_MAX_ROW) {

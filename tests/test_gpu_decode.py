@@ -771,7 +771,7 @@ def test_lists_of_more_sessions_than_a_wave():
             m = (rows[i] + 1) * stores[0][i].token_bytes
             assert torch.equal(raw[0][:m], raw[1][:m]), (i, which)
     assert L.q4_gpu_last_error() == 0
-    b.close() if hasattr(b, "close") else None
+    b.close()
     for pair in stores:
         for st in pair:
             st.close()
