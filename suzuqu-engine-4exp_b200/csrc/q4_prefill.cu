@@ -612,6 +612,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) q4_prefill_k(const std::conditi
                 load(vs + (size_t)j * CV * PF_CHUNK, CV);
                 if (j + (3u - NQ) < n_tiles) load(ks + (size_t)(j + (3u - NQ)) * CK * PF_CHUNK, CK);
             }
+            /* A pair: the last images' slots have been told free before either block leaves, or that would reach shared memory that is
+             * another block's by then.  (Of two groups the last tile's V is not, where only its first half is needed.) */
+            if (PAIR && ok)
+                for (uint32_t t = at > SLOTS ? at - SLOTS : 0, end = at - (NQ == 2 ? n_seq & 1u : 0u); t < end && ok; t++)
+                    ok = mbar_test<BYTES>(empty + 8 * (t % SLOTS), (t / SLOTS) & 1u) || pf_wait<BYTES>(empty + 8 * (t % SLOTS), (t / SLOTS) & 1u, s_abort, t_start);
             /* Gave up somewhere: copies still in flight must land before the block's shared memory is released
              * (bounded again; these probes ignore the abort flag; phases that completed long ago answer at once). */
             if (!ok)
