@@ -2228,10 +2228,12 @@ bool launch(const DecParams &p_in, dim3 grid) {
         if (n_blocks() > (uint64_t)occ * (uint64_t)g_q4.sm_count) p.gridmerge = p.few = 0;   /* the merge in two levels is one of all splits */
     }
     size_t smem = smem_base + p.push_bytes;
-    /* A few lists' clusters are spread two blocks deep at most, by asking for half of an SM's shared memory, where all are resident
-     * at once so too (8 sessions 9.3 -> 8.6 us per launch, 10 9.8 -> 8.8; of 12, not: 10.2 -> 14.5).  Two warps to a tile: as rings
-     * of four tiles did by their size (8 sessions of 24 / 2 heads of 256 in q8_0 15.6 -> 12.6, 32 / 2 of 128 in fp16 10.3 -> 8.8). */
-    if (LIST && (Cfg::STAGED || Cfg::WPT == 2) && p.cluster && smem < DEC_HALF_SM && n_blocks() <= 2u * (uint64_t)g_q4.sm_count && resident_clusters(DEC_HALF_SM) * p.cluster >= n_blocks()) smem = DEC_HALF_SM;
+    /* A few units' clusters are spread two blocks deep at most, by asking for half of an SM's shared memory, where all are resident
+     * at once so too (lists of 8 sessions 9.3 -> 8.6 us per launch, 10 9.8 -> 8.8; of 12, not: 10.2 -> 14.5).  Two warps to a tile: as
+     * rings of four tiles did by their size (lists of 8 sessions of 24 / 2 heads of 256 in q8_0 15.6 -> 12.6, 32 / 2 of 128 in fp16 10.3 ->
+     * 8.8).  Dense scans of batches likewise (8 sessions up to 4000 rows, 24 / 2 / 256 22.1 -> 19.9, 16 / 2 / 128 9.5 -> 9.0), but not
+     * the clusters of a grid merge, which are to leave room for the next launch's (8192 rows in a store of 32768 7.3 -> 8.0). */
+    if ((Cfg::STAGED || Cfg::WPT == 2) && p.cluster && !p.gridmerge && smem < DEC_HALF_SM && n_blocks() <= 2u * (uint64_t)g_q4.sm_count && resident_clusters(DEC_HALF_SM) * p.cluster >= n_blocks()) smem = DEC_HALF_SM;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;

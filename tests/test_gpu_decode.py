@@ -711,6 +711,36 @@ def test_lists_of_a_few_tokens_spread_over_the_sms(kind, n_head, hd, n_tok, widt
     st.close()
 
 
+@pytest.mark.parametrize("kind,n_head,hd", [(2, 24, 256), (1, 32, 128), (2, 16, 128)])
+@pytest.mark.parametrize("n,top", [(2, 1500), (8, 2000), (24, 600), (25, 600)])
+def test_dense_batches_of_a_few_sessions_spread_over_the_sms(kind, n_head, hd, n, top):
+    """clusters of dense scans, two blocks per SM at most and more, one and two warps to a tile, with appends: against one session at a
+    time, which are other launches, each within the tolerance of the oracle's tests"""
+    L = lib()
+    n_kvh, scale = 2, float(1 / np.sqrt(hd))
+    g = torch.Generator(device="cuda").manual_seed(n + hd)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    rows = [top - 1 - (37 * i * i) % (top // 2) for i in range(n)]
+    data, k, v, q = rn(top, n_kvh * hd), rn(n, n_kvh * hd), rn(n, n_kvh * hd), rn(n, n_head, hd)
+    out, ref = torch.empty(n, n_head, hd, device="cuda"), torch.empty(n, n_head, hd, device="cuda")
+    stores = [[q4gpu.KVStore(1, n_kvh, hd, r + 1, kind) for r in rows] for _ in range(2)]
+    for pair in stores:
+        for st, r in zip(pair, rows):
+            st.append(0, data, data, 0, r)
+    b = q4gpu.Batch(stores[0])
+    b.set_pos(rows)
+    b.append_decode(0, k, v, q, out, n_head, scale)
+    for i, st in enumerate(stores[1]):
+        L.q4_hip_pos_push(rows[i])
+        st.append_decode_d(0, k[i], v[i], q[i], ref[i], n_head, scale)
+    assert_close(host(out), host(ref), "%d sessions up to %d rows" % (n, top))
+    assert L.q4_gpu_last_error() == 0
+    b.close()
+    for pair in stores:
+        for st in pair:
+            st.close()
+
+
 @pytest.mark.parametrize("kind,n_head,n_kvh,hd,max_kv,rows", [
     (2, 16, 2, 128, 65536, (14207, 14208, 14209, 14225, 28416, 28433, 64000)), (2, 16, 4, 128, 65536, (7104, 7120, 20000, 35536)), (2, 8, 1, 128, 262144, (16385, 70000, 82000)),
     (1, 16, 2, 128, 65536, (14209, 16384, 49153)), (1, 16, 2, 256, 40000, (14209, 30001)), (2, 16, 2, 256, 32768, (20000, 32768))])
